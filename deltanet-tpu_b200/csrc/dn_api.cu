@@ -136,9 +136,7 @@ int dn_residual_carve(const dn_shape* s, void* block, dn_residuals* out) {
 
 // ---- scratch accounting -------------------------------------------------------------------
 static size_t fwd_kernel_scratch(const Geo& g) {
-  size_t items = (size_t)g.B * g.H * g.NC;
-  size_t ctas = items < (size_t)sm_count() ? items : (size_t)sm_count();
-  return align_up(ctas * prepass_fwd_scratch_per_cta(g) * sizeof(float));
+  return align_up(prepass_fwd_scratch_floats(g) * sizeof(float));
 }
 static size_t bwd_kernel_scratch(const Geo& g) {
   size_t items = (size_t)g.B * g.H * g.NC;
@@ -358,20 +356,17 @@ int dn_chunk_fwd(const dn_shape* s, const void* q, const void* k, const void* v,
     std::lock_guard<std::mutex> lock(ov->enqueue);
     cudaStream_t st = (cudaStream_t)stream;
     float* carry = reinterpret_cast<float*>(p);
-    p += carry_bytes(g);
-    float* sc = reinterpret_cast<float*>(p);
-    const size_t scf = (size_t)(end - p) / sizeof(float);
     StateArgs a{};
     a.g = g; a.res = *res; a.seg = seg; a.init_state = (g.flags & DN_HAS_INIT) ? init_state : nullptr;
     a.out = out; a.final_state = final_state; a.states = res->states; a.carry = carry;
-    if ((rc = launch_prepass_fwd_tc(g, q, k, v, g_, b, w, seg, *res, sc, scf, st, 0, cut))) return rc;
+    if ((rc = launch_prepass_fwd_tc(g, q, k, v, g_, b, w, seg, *res, st, 0, cut))) return rc;
     if (cudaEventRecord(ov->ev[0], st) != cudaSuccess || cudaStreamWaitEvent(ov->side, ov->ev[0], 0) != cudaSuccess)
       return DN_ERR_CUDA_LAUNCH;
     // forked: whatever fails from here on, the side stream is joined back before returning
     a.c_begin = 0; a.c_end = cut;
     const int rc_side = launch_state_fwd_tc(a, ov->side);
     const cudaError_t e1 = cudaEventRecord(ov->ev[1], ov->side);
-    const int rc_main = launch_prepass_fwd_tc(g, q, k, v, g_, b, w, seg, *res, sc, scf, st, cut, g.NC);
+    const int rc_main = launch_prepass_fwd_tc(g, q, k, v, g_, b, w, seg, *res, st, cut, g.NC);
     const cudaError_t e2 = cudaStreamWaitEvent(st, ov->ev[1], 0);
     if (rc_side) return rc_side;
     if (rc_main) return rc_main;

@@ -29,7 +29,7 @@ struct InCfg {
   static constexpr int qkv_dt = MODE == 1 ? DN_F32 : DN_BF16;
 };
 inline int input_mode(const Geo& g) {
-  if (g.gate_dt != DN_F32 || (g.flags & (DN_FUSE_PROLOGUE | DN_STABILITY_GUARD))) return 2;
+  if (g.K != K || g.gate_dt != DN_F32 || (g.flags & (DN_FUSE_PROLOGUE | DN_STABILITY_GUARD))) return 2;
   if (g.gC == g.K && g.bC == g.K && g.wC == g.V) return g.qkv_dt == DN_BF16 ? 0 : 1;
   if (g.gC == 1 && g.bC == 1 && g.wC == 1 && g.qkv_dt == DN_BF16) return 3;
   if (g.gC == g.K && g.bC == 1 && g.wC == 1 && g.qkv_dt == DN_BF16) return 4;
@@ -46,6 +46,7 @@ struct Rows {
   size_t b_row0, b_pitch;
   int gC, bC;            // channels per row of g / b: 1 or K
   int rows_valid;        // tokens of the chunk that exist
+  int kp;                // 8-channel pieces of q, k, g, b that exist (K / 8); the rest of the 128-wide tile is zeros
   bool l2, fuse, guard, round_in;
   float scale;
   const float *rq, *rk;  // per-row normalisers (shared memory), 1 when l2 is off
@@ -70,13 +71,13 @@ __device__ __forceinline__ void zero8(float (&x)[8]) {
 // is unconditional (a row past the end reads row 0 and is zeroed afterwards), so that a caller's
 // loads can all be in flight together.
 __device__ __forceinline__ void raw_q8(const Rows& r, int x, int p, float (&o)[8]) {
-  const bool live = x < r.rows_valid;
-  load8(r.q, r.qk_row0 + (size_t)(live ? x : 0) * r.qk_pitch + 8 * p, r.qkv_dt, o);
+  const bool live = x < r.rows_valid && p < r.kp;
+  load8(r.q, r.qk_row0 + (live ? (size_t)x * r.qk_pitch + 8 * p : 0), r.qkv_dt, o);
   if (!live) zero8(o);
 }
 __device__ __forceinline__ void raw_k8(const Rows& r, int x, int p, float (&o)[8]) {
-  const bool live = x < r.rows_valid;
-  load8(r.k, r.qk_row0 + (size_t)(live ? x : 0) * r.qk_pitch + 8 * p, r.qkv_dt, o);
+  const bool live = x < r.rows_valid && p < r.kp;
+  load8(r.k, r.qk_row0 + (live ? (size_t)x * r.qk_pitch + 8 * p : 0), r.qkv_dt, o);
   if (!live) zero8(o);
 }
 // q_hat = l2norm(q) * scale, k_hat = l2norm(k), each rounded to the input dtype when the
@@ -107,8 +108,8 @@ __device__ __forceinline__ void raw_gate8(const void* base, size_t row0, size_t 
 }
 // activated erase gate b
 __device__ __forceinline__ void bact8(const Rows& r, int x, int p, float (&o)[8]) {
-  const bool live = x < r.rows_valid;
-  raw_gate8(r.b, r.b_row0, r.b_pitch, r.bC, r.gate_dt, live ? x : 0, p, o);
+  const bool live = x < r.rows_valid && p < r.kp;
+  raw_gate8(r.b, r.b_row0, r.b_pitch, r.bC, r.gate_dt, live ? x : 0, live ? p : 0, o);
   if (r.fuse) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) o[i] = 1.f / (1.f + expf(-o[i]));
@@ -120,8 +121,8 @@ __device__ __forceinline__ void bact8(const Rows& r, int x, int p, float (&o)[8]
 }
 // activated log-decay g (<= 0)
 __device__ __forceinline__ void gact8(const Rows& r, int x, int p, float (&o)[8]) {
-  const bool live = x < r.rows_valid;
-  raw_gate8(r.gg, r.g_row0, r.g_pitch, r.gC, r.gate_dt, live ? x : 0, p, o);
+  const bool live = x < r.rows_valid && p < r.kp;
+  raw_gate8(r.gg, r.g_row0, r.g_pitch, r.gC, r.gate_dt, live ? x : 0, live ? p : 0, o);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     if (r.fuse) { o[i] = -expf(fminf(o[i], 5.f)); if (r.guard) o[i] = fminf(o[i], -1e-6f); }
@@ -172,8 +173,8 @@ __device__ __forceinline__ void lambda_scan_512(const Rows& r, const int* seg_s,
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
     const int x = x0 + i;
-    const bool live = x < r.rows_valid;
-    float gv = ldf_ro(r.gg, r.g_row0 + (size_t)(live ? x : 0) * r.g_pitch + gcol, r.gate_dt);
+    const bool live = x < r.rows_valid && c < 8 * r.kp;
+    float gv = ldf_ro(r.gg, r.g_row0 + (live ? (size_t)x * r.g_pitch + gcol : 0), r.gate_dt);
     if (r.fuse) { gv = -expf(fminf(gv, 5.f)); if (r.guard) gv = fminf(gv, -1e-6f); }
     else { gv = gv <= 0.f ? gv : 0.f; if (r.guard) gv = fminf(gv, -1e-6f); }
     v[i] = live ? gv : 0.f;
@@ -269,8 +270,9 @@ __device__ __forceinline__ Rows make_rows(const Geo& g, const void* q, const voi
   r.qkv_dt = CF::fixed ? CF::qkv_dt : g.qkv_dt;
   r.gate_dt = CF::fixed ? DN_F32 : g.gate_dt;
   const size_t tok0 = (size_t)bidx * g.L + t0;
-  r.qk_pitch = (size_t)g.Hk * K;
-  r.qk_row0 = tok0 * r.qk_pitch + (size_t)(h / g.qk_div) * K;
+  r.qk_pitch = (size_t)g.Hk * g.K;
+  r.qk_row0 = tok0 * r.qk_pitch + (size_t)(h / g.qk_div) * g.K;
+  r.kp = CF::fixed ? K / 8 : g.K / 8;
   r.gC = CF::fixed ? (CF::scalar_gates ? 1 : K) : g.gC;
   r.bC = CF::fixed ? (CF::scalar_bw ? 1 : K) : g.bC;
   r.g_pitch = (size_t)g.gH * g.gC;

@@ -73,17 +73,16 @@ struct PrepassBwdArgs {
 int launch_status();
 long long launches_total();
 
-size_t prepass_fwd_scratch_per_cta(const Geo& g);
+size_t prepass_fwd_scratch_floats(const Geo& g);
 size_t prepass_bwd_scratch_per_cta(const Geo& g);
 
 int launch_prepass_fwd(const Geo& g, const void* q, const void* k, const void* v, const void* gg,
                        const void* b, const void* w, const int32_t* seg, const dn_residuals& res,
                        float* scratch, size_t scratch_floats, cudaStream_t st);
 bool prepass_fwd_tc_eligible(const Geo& g);
-size_t prepass_fwd_tc_scratch_per_cta();
 int launch_prepass_fwd_tc(const Geo& g, const void* q, const void* k, const void* v, const void* gg,
                           const void* b, const void* w, const int32_t* seg, const dn_residuals& res,
-                          float* scratch, size_t scratch_floats, cudaStream_t st, int c_begin = 0, int c_end = -1);
+                          cudaStream_t st, int c_begin = 0, int c_end = -1);
 int launch_state_fwd(const StateArgs& a, cudaStream_t st);
 // tensor-core (tcgen05) variants of the chain kernels, used when state_tc_eligible()
 bool state_tc_eligible(const Geo& g);

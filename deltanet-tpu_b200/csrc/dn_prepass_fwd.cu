@@ -277,17 +277,22 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_fwd_kernel(PrepassFwdAr
   }
 }
 
-size_t prepass_fwd_scratch_per_cta(const Geo& g) { return (size_t)5 * g.C * g.K + (size_t)g.C * g.Vw; }
+static size_t scratch_per_cta(const Geo& g) { return (size_t)5 * g.C * g.K + (size_t)g.C * g.Vw; }
+size_t prepass_fwd_scratch_floats(const Geo& g) {
+  if (prepass_fwd_tc_eligible(g)) return 0;
+  const size_t items = (size_t)g.B * g.H * g.NC, ctas = items < (size_t)sm_count() ? items : (size_t)sm_count();
+  return ctas * scratch_per_cta(g);
+}
 
 int launch_prepass_fwd(const Geo& g, const void* q, const void* k, const void* v, const void* gg,
                        const void* b, const void* w, const int32_t* seg, const dn_residuals& res,
                        float* scratch, size_t scratch_floats, cudaStream_t st) {
   if (prepass_fwd_tc_eligible(g))
-    return launch_prepass_fwd_tc(g, q, k, v, gg, b, w, seg, res, scratch, scratch_floats, st);
-  PrepassFwdArgs a;
+    return launch_prepass_fwd_tc(g, q, k, v, gg, b, w, seg, res, st);
+  PrepassFwdArgs a{};
   a.g = g; a.q = q; a.k = k; a.v = v; a.gg = gg; a.b = b; a.w = w; a.seg = seg; a.res = res;
   a.items = g.B * g.H * g.NC;
-  a.scratch_per_cta = prepass_fwd_scratch_per_cta(g);
+  a.scratch_per_cta = scratch_per_cta(g);
   int grid = a.items < sm_count() ? a.items : sm_count();
   if (scratch_floats < (size_t)grid * a.scratch_per_cta) return DN_ERR_SCRATCH_TOO_SMALL;
   a.scratch = scratch;

@@ -1,753 +1,884 @@
-// Prepass forward on the tcgen05 tensor cores (bf16 precision, chunk = K = 128, value width
-// 128 or 256).  Produces the same outputs as the fp32 formulation in dn_prepass_fwd.cu
-// (reference body: src/deltanet_tpu/gdn2.py:115-240), with the bf16 tiles W, U, M, qe, ke written
-// as tensor-core operand images ([col / 8][row][8], see Geo::img).
+// Forward prepass on the tcgen05 tensor cores (bf16 precision, 128-row tiles).
+// Same outputs as the fp32 formulation in dn_prepass_fwd.cu (reference body:
+// src/deltanet_tpu/gdn2.py:115-240); W, U, M, qe, ke are written as operand images, [col / 8][row][8].
 //
-// A and M.  A_ij = sum_c beta_ic exp(Lam_ic - Lam_jc) k_jc cannot in general be one matrix product
-// because the decay couples i, j and the channel c.  Two cases reduce to plain products and are taken
-// when they apply: one scalar decay per (token, head), where exp(lam_i - lam_j) is applied entry-wise
-// to the Gram products beta k k^T and q k^T while they drain; and channel-wise decay that stays
-// within e^{+-32} of each document's midpoint over the chunk (tested per chunk on the device),
-// where with f = exp(Lam - midpoint) the images k / f, q f, beta k f give A and M by one product
-// each.  Otherwise it is built hierarchically: at level s in {16,32,64}
-// the chunk is cut into pairs of adjacent s-row blocks, and for a pair with rows I (lower block),
-// columns J (upper block) and reference row r = first row of I
-//     A[I,J] = (beta_I * exp(Lam_I - Lam_r)) (k_J * exp(Lam_r - Lam_J))^T ,
-// with both scale factors <= 1 (the cumulative decay is monotone inside a document), so nothing
-// can overflow however strong the decay.  In one level every row is either a row of its pair
-// (lower block) or a column (upper block), so two images suffice: KR holds the beta-images on lower
-// rows and the k-images on upper rows, QK the q-images and the k-images, and
-//     level part of A = KR KR^T,   level part of M = QK KR^T       (one 128^3 MMA each);
-// entries outside the level's blocks are finite garbage that the drain ignores (entry (i,j) belongs
-// to the level of the highest bit in which i>>4 and j>>4 differ).  A level's drain shares a barrier
-// interval with the next level's image build (the images are free once the level's products have
-// completed).  The 16x16 diagonal blocks are evaluated exactly, pair by pair, on the CUDA cores;
-// when k_hat and q_hat are exactly bf16 this pass runs first and parks k_hat | q_hat (two bf16 per
-// column) and beta in tensor memory, from where the qe / ke / X pass and all level images are built
-// without touching global memory again.  The reference does the same with 32-row blocks and one
-// reference per block row (gdn2.py:162-197).
+// A and M are one matrix product each when the decay factors:
+//   * scalar decay per (token, head):  A_ij = beta_i e^{lam_i - lam_j} (k_i . k_j), M_ij = e^{lam_i - lam_j} (q_i . k_j):
+//     Gram products of the plain images, the decay applied per entry while they drain (prepass_fwd_scalar_kernel);
+//   * decay per channel that stays within e^{+-32} of each document's midpoint m over the tile: with
+//     f = e^{Lam - m},  A = (beta f) (k / f)^T,  M = (q f) (k / f)^T  (prepass_fwd_channel_kernel).
+// A tile with a stronger channel-wise decay takes the hierarchical factorisation (strong_route), decided per tile.
 //
-// T = (I+A)^-1 is obtained as in the fp32 formulation (substitution on 16x16 blocks + block
-// merges, fp32 in shared memory); W = T X and U = T Y are tcgen05 MMAs on bf16 operands, which
-// is also where the reference rounds to bf16 (gdn2.py:226-230).
-//
-// 512 threads per CTA, one CTA per SM, looping over (batch, exec head, chunk) items.  Phases that
-// read the operator's row-major tensors let a warp cover 8 rows x 4 pieces of 8 channels (row =
-// 8 * warp + (lane & 7) fixed per thread) with every load issued unconditionally; phases that drain
-// tensor memory own one row per thread, which the image layout of the outputs (and the panel
-// layout [col / 4][row][4] of the fp32 scratch that carries A to the inverse) turns into stores of
-// 512 contiguous bytes per warp.
-#ifdef DN_PHASE_TIMING
-#include <cstdio>
-#endif
+// What bounds an item is neither bytes nor tensor work but the length of its dependent phases (load, norms and
+// decay, products, inverse, products, store).  So a CTA takes 109 KB of shared memory and 256 columns of tensor
+// memory, half an SM, and two CTAs in different phases share each SM.  The footprint comes from three
+// choices: A and T share one block-packed fp32 triangle that is inverted in place (dn_tri_inverse.cuh), the
+// channel-wise kernel walks the channels in four groups of 32 whose images are double buffered under the
+// products of the previous group, and A goes from tensor memory straight into the triangle.
+#include <type_traits>
+
 #include "dn_chunkprep.cuh"
 #include "dn_kernels.cuh"
+#include "dn_tri_inverse.cuh"
 
 namespace dn {
 namespace {
 
 using namespace prep;
 constexpr int NT = 512;
-constexpr int AP = 132;                              // row pitch (floats) of A, T in shared memory
-constexpr int OFF_IMG = C * LP * 4;                  // level images / k cache / A start after Lambda
-constexpr int OFF_TM = OFF_IMG + C * AP * 4;         // merge scratch (16 KB)
-constexpr int OFF_XI = 160 * 1024;                   // X image: survives the inverse
-constexpr int OFF_TI = 192 * 1024;                   // T image
-constexpr int SMEM_BYTES = 224 * 1024;
-static_assert(OFF_TM + 16384 <= OFF_XI, "merge scratch below the X image");
-static_assert(OFF_IMG + 2 * 32768 <= OFF_XI, "level images below the X image");
+constexpr int PP = 130;                               // uint4 per panel of the images that threads write from rows of the
+constexpr uint32_t PB = PP * 16;                      //   operator's tensors (see row_of), in bytes
+constexpr int OFF_X = 0;                              // X image (scalar kernel: k_hat image first)
+constexpr int OFF_T = 16 * PB;                        // packed triangle A / T, then the Y image of the first half
+constexpr int OFF_TI = OFF_T + tri::BYTES;            // T image (merge scratch before it; scalar kernel: q_hat image first)
+constexpr int SMEM_BYTES = OFF_TI + 16 * PB;
+constexpr int LQ = 36;                                // row pitch (floats) of a 32-channel group of Lambda
+constexpr int OFF_LAM = OFF_T;                        // channel kernel, before the triangle: Lambda group,
+constexpr int OFF_TOT = OFF_LAM + C * LQ * 4;         //   the scan's 16 x 32 partial sums,
+constexpr int OFF_EDGE = OFF_TOT + 16 * 32 * 4;       //   each warp's copy of the two edge factors per channel (and zeros),
+constexpr int OFF_GI = OFF_EDGE + 16 * 96 * 4;        //   and two sets of three 128 x 32 images
+static_assert(tri::TMP_BYTES <= 32768, "merge scratch inside the T image");
+static_assert(OFF_GI + 2 * 3 * 4 * PB <= SMEM_BYTES, "channel group buffers");
+static_assert(16 * PB <= tri::BYTES && 3 * 64 * LQ * 4 <= 16 * PB, "Y over the triangle, diagonal-pass caches over X");
+static_assert(SMEM_BYTES <= 113 * 1024 - 2560, "two CTAs per SM, with the static arrays");
 
-__device__ __forceinline__ int p4v(int row, int col) { return ((col >> 2) << 7) + row; }
-__device__ __forceinline__ int p4f(int row, int col) { return ((((col >> 2) << 7) + row) << 2) + (col & 3); }
+// Thread mapping wherever rows of the operator's tensors are read: a warp covers 8 rows x 4 pieces of 16 bytes with
+// the pieces of a row in neighbouring lanes.  A 16-byte load is looked up in L1 eight lanes at a time; eight lanes in
+// eight rows cost 32 lookups per load instead of 8, and the data stage of L1 was the busiest unit of these kernels.
+__device__ __forceinline__ int row_of(int tid) { return tid >> 2; }
+__device__ __forceinline__ int piece_of(int tid) { return tid & 3; }
 
-// One merge level of the inverse: for every pair of adjacent S-row blocks (lower rows I, upper rows J)
-//   T[I,J] = -T[I,I] (A[I,J] T[J,J]).
-// 512 threads = (row pair of I) x (16 column groups of S/16 columns) x pairs; a thread owns a
-// 2 x (S/16) tile of outputs, so one step of the contraction costs two scalar loads and one
-// vector load from shared memory for 2 * S/16 multiply-adds.
-template <int S>
-__device__ __forceinline__ void merge_level(const float* As, float* Ts, float* Tm) {
-  constexpr int NJ = S / 16;
-  const int cg = threadIdx.x & 15, rest = threadIdx.x >> 4;     // rest = pair * (S/2) + row pair in I
-  const int p = rest / (S / 2), il = 2 * (rest - p * (S / 2));
-  const int i = 2 * p * S + S + il, j0 = 2 * p * S + cg * NJ, m0 = 2 * p * S;
-  float acc0[NJ], acc1[NJ];
+// 1 / (1 + e^-x) on the special-function unit (relative error a few 2^-23; the products it enters are rounded to bf16)
+__device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 1.f + umma::ex2_fast(-x * DN_LOG2E)); }
+
+// After the products: the 16-column pieces of A (already masked and scaled by `fix`) into the triangle, of M into
+// its image.  fix(row, col, a[16], m[16]) applies masks and decay.
+template <class FIX>
+__device__ __forceinline__ void drain_am(const umma::Ctx& cx, float* Tp, uint4* Mimg, FIX fix) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int quarter = warp & 3, group = warp >> 2, row = quarter * 32 + lane;
+  const uint32_t tbase = cx.tmem + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll 1
+  for (int cc = 0; cc < 32; cc += 16) {
+    const int col = group * 32 + cc;
+    float va[16], vm[16];
+    if (!cx.dead && col <= quarter * 32 + 31) {        // warp-uniform: a piece wholly above the warp's rows is zeros
+      umma::tmem_ld16(tbase + col, va);
+      umma::tmem_ld16(tbase + 128 + col, vm);
+      fix(row, col, va, vm);
+    } else {
 #pragma unroll
-  for (int u = 0; u < NJ; ++u) acc0[u] = acc1[u] = 0.f;
-#pragma unroll 4
-  for (int m = 0; m < S; ++m) {
-    const float a0 = As[i * AP + m0 + m], a1 = As[(i + 1) * AP + m0 + m];
-    const float* t = Ts + (m0 + m) * AP + j0;
+      for (int i = 0; i < 16; ++i) va[i] = vm[i] = 0.f;
+    }
+    if ((col >> 4) <= (row >> 4)) {
+      float4* d = reinterpret_cast<float4*>(tri::blk(Tp, row >> 4, col >> 4) + (row & 15) * tri::BP);
 #pragma unroll
-    for (int u = 0; u < NJ; ++u) { acc0[u] = fmaf(a0, t[u], acc0[u]); acc1[u] = fmaf(a1, t[u], acc1[u]); }
+      for (int i = 0; i < 4; ++i) d[i] = make_float4(va[4 * i], va[4 * i + 1], va[4 * i + 2], va[4 * i + 3]);
+    }
+    Mimg[(col / 8) * 128 + row] = umma::pack8p(vm);
+    Mimg[(col / 8 + 1) * 128 + row] = umma::pack8p(vm + 8);
   }
+  umma::tc_fence_before();
+}
+
+// Eight consecutive elements as loaded (bf16: the first vector only); converted where they are used, so that a load
+// can be in flight across a barrier without its converted values taking registers.
+struct Raw8 { uint4 a, b; };
+__device__ __forceinline__ Raw8 ldraw(const uint8_t* row, int p, int dt) {
+  Raw8 r;
+  r.b = make_uint4(0, 0, 0, 0);
+  if (dt == DN_BF16) r.a = __ldg(reinterpret_cast<const uint4*>(row) + p);
+  else { r.a = __ldg(reinterpret_cast<const uint4*>(row) + 2 * p); r.b = __ldg(reinterpret_cast<const uint4*>(row) + 2 * p + 1); }
+  return r;
+}
+__device__ __forceinline__ void cvraw(const Raw8& r, int dt, float (&x)[8]) {
+  if (dt == DN_BF16) umma::unpack8(r.a, x);
+  else {
+    x[0] = __uint_as_float(r.a.x); x[1] = __uint_as_float(r.a.y); x[2] = __uint_as_float(r.a.z); x[3] = __uint_as_float(r.a.w);
+    x[4] = __uint_as_float(r.b.x); x[5] = __uint_as_float(r.b.y); x[6] = __uint_as_float(r.b.z); x[7] = __uint_as_float(r.b.w);
+  }
+}
+
+// L2 requests made by threads 128 .. 511 while the first four warps are in the substitution: this tile's rows of v
+// and w, read right after the inverse, and the next tile's rows of k, q and g / b.  (One line per lane: the bulk form of
+// this request is issued lane by lane, about 80 cycles each, and took longer than what it hid.)
+__device__ __forceinline__ void prefetch_row(const void* p, uint32_t bytes) {
+  for (uint32_t o = 0; o < bytes; o += 128)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t*>(p) + o));
+}
+template <int VW>
+__device__ __forceinline__ void prefetch_rows(const PrepassFwdArgs& a, int h, int b, int t0, int next, int wC) {
+  const Geo& g = a.g;
+  const int x = threadIdx.x & 127, part = threadIdx.x >> 7;
+  const uint32_t qe = (uint32_t)dt_size(g.qkv_dt), ge = (uint32_t)dt_size(g.gate_dt);
+  if (part < 3) {
+    if (t0 + x < g.L) {
+      const size_t tok = (size_t)b * g.L + t0 + x;
+      if (part == 1) prefetch_row(reinterpret_cast<const uint8_t*>(a.v) + (tok * g.Hv * g.V + (size_t)h * VW) * qe, VW * qe);
+      else if (wC == g.V && g.wH == g.Hv)
+        prefetch_row(reinterpret_cast<const uint8_t*>(a.w) + (tok * g.Hv * g.V + (size_t)h * VW) * ge, VW * ge);
+    }
+  } else if (next < a.items) {
+    const int bh = next % (g.B * g.H), t = (a.c_begin + next / (g.B * g.H)) * C + x;
+    const int hn = bh % g.H;
+    if (t < g.L) {
+      const size_t tok = (size_t)(bh / g.H) * g.L + t, qk = (tok * g.Hk + hn / g.qk_div) * g.K;
+      prefetch_row(reinterpret_cast<const uint8_t*>(a.k) + qk * qe, g.K * qe);
+      prefetch_row(reinterpret_cast<const uint8_t*>(a.q) + qk * qe, g.K * qe);
+      if (g.gC > 1) prefetch_row(reinterpret_cast<const uint8_t*>(a.gg) + (tok * g.gH + g.gate_head(hn, g.gH)) * g.gC * ge, g.gC * ge);
+      if (g.bC > 1) prefetch_row(reinterpret_cast<const uint8_t*>(a.b) + (tok * g.bH + g.gate_head(hn, g.bH)) * g.bC * ge, g.bC * ge);
+    }
+  }
+}
+
+// T = (I + A)^-1, then W = T X and U = T (w v).  X image and A visible to all threads on entry.
+template <int VW>
+__device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm, const PrepassFwdArgs& a, int h, int b, int t0,
+                                                     size_t ibase, int next, int qdt, int gdt, int wC, bool fuse) {
+  constexpr int HW = VW < 128 ? VW : 128, NH = VW / HW, NP = HW / 32;
+  const Geo& g = a.g;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int x = row_of(tid), lgrp = piece_of(tid);
+  float* Tp = reinterpret_cast<float*>(sm + OFF_T);
+  uint4* XI = reinterpret_cast<uint4*>(sm + OFF_X);
+  uint4* TI = reinterpret_cast<uint4*>(sm + OFF_TI);
+  uint4* Y0 = reinterpret_cast<uint4*>(sm + OFF_T);
+  uint4* Wimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.W) + ibase * C * K);
+  uint4* Uimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.U) + ibase * C * VW);
+  const bool live = t0 + x < g.L;
+  const size_t tokr = (size_t)b * g.L + (live ? t0 + x : t0);
+  const uint8_t* vrow = reinterpret_cast<const uint8_t*>(a.v) + (tokr * g.Hv * g.V + (size_t)h * VW) * dt_size(qdt);
+  uint4 vr[NP];                                         // a half's pieces of v (bf16), requested ahead of use
+  auto request_v = [&](int half) {
+    if (qdt == DN_BF16) {
 #pragma unroll
-  for (int u = 0; u < NJ; ++u) {
-    Tm[(p * S + il) * S + cg * NJ + u] = acc0[u];
-    Tm[(p * S + il + 1) * S + cg * NJ + u] = acc1[u];
+      for (int it = 0; it < NP; ++it) vr[it] = __ldg(reinterpret_cast<const uint4*>(vrow) + half * (HW / 8) + it * 4 + lgrp);
+    }
+  };
+  auto build_y = [&](uint4* Y, int half) {              // Y = w v of the half's columns
+#pragma unroll
+    for (int it = 0; it < NP; ++it) {
+      const int p = it * 4 + lgrp;
+      const int col0 = half * HW + 8 * p, hv = (h * VW + col0) / g.V, cv = h * VW + col0 - hv * g.V;
+      float vv[8], ww[8];
+      if (wC == 1) {
+        const float w1 = ldf_ro(a.w, tokr * g.wH + g.w_head(hv), gdt);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ww[i] = w1;
+      } else {
+        load8(a.w, (tokr * g.wH + g.w_head(hv)) * wC + cv, gdt, ww);
+      }
+      if (qdt == DN_BF16) umma::unpack8(vr[it], vv);
+      else { const Raw8 r = ldraw(vrow, half * (HW / 8) + p, qdt); cvraw(r, qdt, vv); }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) vv[i] = live ? (fuse ? sigmoid_fast(ww[i]) : ww[i]) * vv[i] : 0.f;
+      Y[p * PP + x] = umma::pack8(vv);
+    }
+  };
+  tri::invert(Tp, reinterpret_cast<float*>(TI), [&]() { prefetch_rows<VW>(a, h, b, t0, next, wC); });
+  request_v(0);
+  tri::image(Tp, TI);
+  __syncthreads();                                      // T has been read: its place takes Y
+  build_y(Y0, 0);
+  umma::pre_issue_sync();
+  umma::issue_pitched<128, false, true>(cx, TI, 2048, XI, PB, C, 0, false);
+  umma::issue_pitched<HW, false, true>(cx, TI, 2048, Y0, PB, C, 128, false);
+  if (tid == 0 && !cx.dead) umma::mma_commit(cx.bar);
+  if (NH == 2) request_v(1);
+  if (a.res.T) {                                        // the image of T, for the backward
+    uint4* Tg = reinterpret_cast<uint4*>(a.res.T + ibase * C * C);
+#pragma unroll
+    for (int it = 0; it < 4; ++it) Tg[it * NT + tid] = TI[it * NT + tid];
+  }
+  umma::commit_wait_cta(cx);
+  if (NH == 2) {                                        // X has been consumed
+    build_y(XI, 1);
+    umma::fence_async_smem();                           // (ahead of the stores below: it would wait for them)
+  }
+  umma::drain<NT, 128>(cx, 0, [&](int row, int col, const float (&v)[16]) {
+    Wimg[(col / 8) * 128 + row] = umma::pack8p(v);
+    Wimg[(col / 8 + 1) * 128 + row] = umma::pack8p(v + 8);
+  });
+  if (NH == 2) {                                        // the second half goes where W was
+    __syncthreads();
+    umma::tc_fence_after();
+    umma::issue_pitched<HW, false, true>(cx, TI, 2048, XI, PB, C, 0, false);
+    if (tid == 0 && !cx.dead) umma::mma_commit(cx.bar);
+  }
+  umma::drain<NT, HW>(cx, 128, [&](int row, int col, const float (&v)[16]) {
+    Uimg[(col / 8) * 128 + row] = umma::pack8p(v);
+    Uimg[(col / 8 + 1) * 128 + row] = umma::pack8p(v + 8);
+  });
+  if (NH == 2) {
+    umma::commit_wait_cta(cx);
+    umma::drain<NT, HW>(cx, 0, [&](int row, int col, const float (&v)[16]) {
+      Uimg[2048 + (col / 8) * 128 + row] = umma::pack8p(v);
+      Uimg[2048 + (col / 8 + 1) * 128 + row] = umma::pack8p(v + 8);
+    });
   }
   __syncthreads();
+}
+
+__device__ __forceinline__ umma::Ctx setup(uint64_t* bar, uint32_t* base, int* err) {
+  if (threadIdx.x == 0) { umma::mbar_init(bar, 1); umma::fence_mbar_init(); }
+  if (threadIdx.x < 32) umma::tmem_alloc(base, 256);
+  umma::tc_fence_before();
+  __syncthreads();
+  umma::tc_fence_after();
+  return umma::Ctx{*base, bar, 0u, err, false};
+}
+__device__ __forceinline__ void teardown(uint32_t base) {
+  umma::tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x < 32) umma::tmem_dealloc(base, 256);
+}
+
+// ------------------------------------------------------------------------------- scalar decay, scalar erase gate
+// One load of q and k serves norms, images, qe and ke: a thread keeps its four 8-channel pieces of both in
+// registers while the row sums meet by shuffles and four warps scan the decay.
+template <int VW>
+__global__ void __launch_bounds__(NT, 2) prepass_fwd_scalar_kernel(const __grid_constant__ PrepassFwdArgs a, int* err) {
+  extern __shared__ __align__(128) uint8_t sm[];
+  __shared__ uint64_t bar;
+  __shared__ uint32_t tbase;
+  __shared__ int seg_s[C];
+  __shared__ float lam_s[C], bet_s[C], tot_s[4];
+  __shared__ int rst_s[4];
+  const Geo& g = a.g;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int x = row_of(tid), lgrp = piece_of(tid);
+  uint4* KI = reinterpret_cast<uint4*>(sm + OFF_X);
+  uint4* QI = reinterpret_cast<uint4*>(sm + OFF_TI);
+  umma::Ctx cx = setup(&bar, &tbase, err);
+  const bool guard = g.flags & DN_STABILITY_GUARD, l2 = g.flags & DN_QK_L2NORM;
+
+  for (int e_item = blockIdx.x; e_item < a.items; e_item += gridDim.x) {
+    const int bh = e_item % (g.B * g.H), c_idx = a.c_begin + e_item / (g.B * g.H);
+    const int h = bh % g.H, b = bh / g.H, t0 = c_idx * C;
+    const size_t ibase = (size_t)bh * g.NC + c_idx, tok0 = (size_t)b * g.L + t0;
+    const int rows = g.L - t0 < C ? g.L - t0 : C;
+    const bool live = x < rows;
+    uint4 kr[4], qr[4];
+    {
+      const uint4* kp = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.k) + ((tok0 + (live ? x : 0)) * g.Hk + h / g.qk_div) * g.K);
+      const uint4* qp = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.q) + ((tok0 + (live ? x : 0)) * g.Hk + h / g.qk_div) * g.K);
 #pragma unroll
-  for (int u = 0; u < NJ; ++u) acc0[u] = acc1[u] = 0.f;
-#pragma unroll 4
-  for (int m = 0; m < S; ++m) {
-    const float t0 = Ts[i * AP + m0 + S + m], t1 = Ts[(i + 1) * AP + m0 + S + m];
-    const float* t = Tm + (p * S + m) * S + cg * NJ;
+      for (int it = 0; it < 4; ++it) {
+        const int p = it * 4 + lgrp;
+        const bool on = live && 8 * p < g.K;
+        kr[it] = on ? __ldg(kp + p) : make_uint4(0, 0, 0, 0);
+        qr[it] = on ? __ldg(qp + p) : make_uint4(0, 0, 0, 0);
+      }
+    }
+    if (tid < C) {                                      // decay: a document-restarting scan over the rows, one row per thread
+      const int t = tid;
+      const int sg = seg_at(a.seg, b, t0 + t, g.L), sp = t ? seg_at(a.seg, b, t0 + t - 1, g.L) : sg;
+      float gv = 0.f, bv = 0.f;
+      if (t < rows) {
+        gv = ldf_ro(a.gg, (tok0 + t) * g.gH + g.gate_head(h, g.gH), g.gate_dt);
+        bv = ldf_ro(a.b, (tok0 + t) * g.bH + g.gate_head(h, g.bH), g.gate_dt);
+        gv = gv <= 0.f ? gv : 0.f;
+        if (guard) { bv = fmaxf(bv, 0.f); gv = fminf(gv, -1e-6f); }
+      }
+      bool cut = sg != sp;
 #pragma unroll
-    for (int u = 0; u < NJ; ++u) { acc0[u] = fmaf(t0, t[u], acc0[u]); acc1[u] = fmaf(t1, t[u], acc1[u]); }
+      for (int o = 1; o < 32; o <<= 1) {
+        const float up = __shfl_up_sync(0xffffffffu, gv, o);
+        const bool uc = __shfl_up_sync(0xffffffffu, (int)cut, o);
+        if (lane >= o) { if (!cut) gv += up; cut |= uc; }
+      }
+      seg_s[t] = sg;
+      bet_s[t] = bv;
+      if (lane == 31) { tot_s[warp] = gv; rst_s[warp] = cut; }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      float carry = 0.f;
+      for (int w2 = warp - 1; w2 >= 0; --w2) { carry += tot_s[w2]; if (rst_s[w2]) break; }
+      lam_s[t] = gv + (cut ? 0.f : carry);
+    }
+    float rq = 1.f, rk = 1.f;
+    if (l2) {
+      float sq = 0.f, sk = 0.f;
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        float f[8];
+        umma::unpack8(qr[it], f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sq = fmaf(f[i], f[i], sq);
+        umma::unpack8(kr[it], f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sk = fmaf(f[i], f[i], sk);
+      }
+      sq += __shfl_xor_sync(0xffffffffu, sq, 1);  sk += __shfl_xor_sync(0xffffffffu, sk, 1);
+      sq += __shfl_xor_sync(0xffffffffu, sq, 2); sk += __shfl_xor_sync(0xffffffffu, sk, 2);
+      rq = rsqrtf(sq + 1e-6f);
+      rk = rsqrtf(sk + 1e-6f);
+    }
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {                    // k_hat, q_hat; rounded to bf16 by the packing
+      float f[8];
+      umma::unpack8(kr[it], f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] *= rk;
+      kr[it] = umma::pack8(f);
+      umma::unpack8(qr[it], f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = (f[i] * rq) * g.scale;
+      qr[it] = umma::pack8(f);
+      const int p = it * 4 + lgrp;
+      KI[p * PP + x] = kr[it];
+      QI[p * PP + x] = qr[it];
+    }
+    umma::pre_issue_sync();
+    umma::issue_pitched<128, false, false>(cx, KI, PB, KI, PB, K, 0, false);             // k_hat k_hat^T
+    umma::issue_pitched<128, false, false>(cx, QI, PB, KI, PB, K, 128, false);           // q_hat k_hat^T
+    if (tid == 0 && !cx.dead) umma::mma_commit(cx.bar);
+    const float lam = lam_s[x], lend = lam_s[C - 1], el = umma::exp_neg(fminf(lam, 0.f)), eke = umma::exp_neg(fminf(lend - lam, 0.f));
+    const bool first = seg_s[x] == seg_s[0], last = seg_s[x] == seg_s[C - 1];
+    {                                                   // qe, ke while the products run
+      uint4* QE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.qe) + ibase * C * K);
+      uint4* KE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.ke) + ibase * C * K);
+      const float fq = first ? el : 0.f, fk = last ? eke : 0.f;
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int p = it * 4 + lgrp;
+        float f[8];
+        umma::unpack8(qr[it], f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] *= fq;
+        QE[p * 128 + x] = umma::pack8(f);
+        umma::unpack8(kr[it], f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] *= fk;
+        KE[p * 128 + x] = umma::pack8(f);
+      }
+      if (tid < K) a.res.lam_end[ibase * K + tid] = lend;
+    }
+    umma::commit_wait_cta(cx);
+    {                                                   // X = [first document] beta e^lam k_hat, over the k_hat image
+      const float bx = bet_s[x];
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        float f[8];
+        umma::unpack8(kr[it], f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = first ? (bx * f[i]) * el : 0.f;
+        KI[(it * 4 + lgrp) * PP + x] = umma::pack8(f);
+      }
+    }
+    {
+      const int row = (warp & 3) * 32 + lane;
+      const float lrow = lam_s[row] * DN_LOG2E, brow = bet_s[row];
+      const int srow = seg_s[row];
+      uint4* Mimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.M) + ibase * C * C);
+      drain_am(cx, reinterpret_cast<float*>(sm + OFF_T), Mimg, [&](int rw, int col, float (&va)[16], float (&vm)[16]) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int j = col + i;
+          const bool same = srow == seg_s[j];
+          const float f = umma::ex2_fast(fminf(lrow - lam_s[j] * DN_LOG2E, 0.f));
+          va[i] = (same && j < rw) ? brow * f * va[i] : 0.f;
+          vm[i] = (same && j <= rw) ? f * vm[i] : 0.f;
+        }
+      });
+    }
+    __syncthreads();
+    inverse_and_products<VW>(cx, sm, a, h, b, t0, ibase, e_item + gridDim.x, DN_BF16, g.gate_dt, g.wC, false);
   }
+  teardown(tbase);
+}
+
+// ------------------------------------------------------------------------------------------- decay per channel
+// The decay of one group of 32 channels: thread (channel lane, rows 8 warp .. 8 warp + 7) loads and activates its rows...
+__device__ __forceinline__ void load_decay(const Rows& r, int grp, int warp, int lane, float (&gv)[8]) {
+  const int c = 32 * grp + lane;
 #pragma unroll
-  for (int u = 0; u < NJ; ++u) { Ts[i * AP + j0 + u] = -acc0[u]; Ts[(i + 1) * AP + j0 + u] = -acc1[u]; }
+  for (int i = 0; i < 8; ++i) {
+    const int row = warp * 8 + i;
+    const bool on = row < r.rows_valid && (r.gC == 1 || c < r.gC);
+    gv[i] = on ? ldf_ro(r.gg, r.g_row0 + (size_t)row * r.g_pitch + (r.gC == 1 ? 0 : c), r.gate_dt) : 0.f;
+    if (on) {
+      if (r.fuse) { gv[i] = -expf(fminf(gv[i], 5.f)); if (r.guard) gv[i] = fminf(gv[i], -1e-6f); }
+      else { gv[i] = gv[i] <= 0.f ? gv[i] : 0.f; if (r.guard) gv[i] = fminf(gv[i], -1e-6f); }
+    }
+  }
+}
+// ... scans them in registers, restarting at document changes, ...
+__device__ __forceinline__ int scan_rows(const int* seg_s, int warp, int lane, float (&gv)[8], float* TOT, int* rst_s) {
+  float run = 0.f;
+  int nr = 8;                                           // first of the thread's rows that starts a document
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int row = warp * 8 + i;
+    if (row > 0 && seg_s[row] != seg_s[row - 1]) { run = 0.f; if (nr == 8) nr = i; }
+    run += gv[i];
+    gv[i] = run;
+  }
+  TOT[warp * 32 + lane] = run;
+  if (lane == 0) rst_s[warp] = nr < 8;
+  return nr;
+}
+// ... and after a barrier adds what the rows above hand on.
+__device__ __forceinline__ void chain_rows(int warp, int lane, const float (&gv)[8], int nr, const float* TOT, const int* rst_s, float* LAM) {
+  float carry = 0.f;
+  for (int w2 = warp - 1; w2 >= 0; --w2) { carry += TOT[w2 * 32 + lane]; if (rst_s[w2]) break; }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) LAM[(warp * 8 + i) * LQ + lane] = gv[i] + (i < nr ? carry : 0.f);
+}
+
+// Decay of any strength: the hierarchical factorisation.  At level s in {16, 32, 64} the tile is cut into pairs of
+// adjacent s-row blocks; for a pair with rows I (lower block), columns J (upper block) and reference row r = first of I
+//     A[I,J] = (beta_I e^{Lam_I - Lam_r}) (k_J e^{Lam_r - Lam_J})^T,   M[I,J] = (q_I e^{Lam_I - Lam_r}) (k_J e^{Lam_r - Lam_J})^T
+// with every factor <= 1.  A row is either a row or a column of its level, so two images suffice: KR (beta on lower
+// rows, k on upper rows) and QK (q, k); A = KR KR^T, M = QK KR^T, of which the drain keeps the blocks that the level
+// owns.  The 16 x 16 diagonal blocks are evaluated pair by pair.  (The reference: 32-row blocks, one reference row
+// per block row, gdn2.py:162-197.)  Five walks over the channel groups -- diagonal, three levels, X -- because the
+// footprint of the common route is kept: about 1.6 times the common route's time per tile, paid by such tiles only.
+template <int MODE>
+__device__ __noinline__ void strong_route(const PrepassFwdArgs& a, int b, int h, int t0, size_t ibase, const float* rq_s, const float* rk_s,
+                                          const int* seg_s, int* rst_s, uint8_t* sm, umma::Ctx& cx) {
+  const Rows r = make_rows<InCfg<MODE>>(a.g, a.q, a.k, a.gg, a.b, b, h, t0, rq_s, rk_s);
+  __nv_bfloat16* M = reinterpret_cast<__nv_bfloat16*>(a.res.M) + ibase * C * C;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, x = row_of(tid), lgrp = piece_of(tid);
+  float* Tp = reinterpret_cast<float*>(sm + OFF_T);
+  float* LAM = reinterpret_cast<float*>(sm + OFF_TI);
+  float* TOT = LAM + C * LQ;
+  float* KC = reinterpret_cast<float*>(sm + OFF_X);     // diagonal pass: k_hat, q_hat, beta of 64 rows, fp32
+  float* QC = KC + 64 * LQ;
+  float* BC = QC + 64 * LQ;
+  uint4* Mimg = reinterpret_cast<uint4*>(M);
+  auto decay = [&](int grp) {                           // Lambda of the group; begins and ends with a barrier
+    float gv[8];
+    load_decay(r, grp, warp, lane, gv);
+    __syncthreads();
+    const int nr = scan_rows(seg_s, warp, lane, gv, TOT, rst_s);
+    __syncthreads();
+    chain_rows(warp, lane, gv, nr, TOT, rst_s, LAM);
+    __syncthreads();
+  };
+  // ---- diagonal blocks: threads 0 .. 479 own a pair (i > j) of one of four blocks per half, threads 0 .. 63 also M_ii
+  int di = 1, dj = tid % 120;
+  while (dj >= di) { dj -= di; ++di; }
+  const int dblk = tid / 120;
+  float accA[2] = {0.f, 0.f}, accM[2] = {0.f, 0.f}, accD[2] = {0.f, 0.f};
+#pragma unroll 1
+  for (int grp = 0; grp < 4; ++grp) {
+    decay(grp);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      if (tid < 256) {
+        const int xr = tid >> 2, xx = half * 64 + xr, p = grp * 4 + (tid & 3), o = xr * LQ + 8 * (tid & 3);
+        float kh[8], qh[8], be[8];
+        khat8(r, xx, p, kh);
+        qhat8(r, xx, p, qh);
+        bact8(r, xx, p, be);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { KC[o + i] = kh[i]; QC[o + i] = qh[i]; BC[o + i] = be[i] * kh[i]; }
+      }
+      __syncthreads();
+      if (dblk < 4) {
+        const int ri = dblk * 16 + di, rj = dblk * 16 + dj;
+        const float* li = LAM + (half * 64 + ri) * LQ;
+        const float* lj = LAM + (half * 64 + rj) * LQ;
+        float sa = 0.f, sm_ = 0.f;
+#pragma unroll 4
+        for (int c = 0; c < 32; ++c) {
+          const float e = KC[rj * LQ + c] * umma::ex2_fast(fminf(li[c] - lj[c], 0.f) * DN_LOG2E);
+          sa = fmaf(BC[ri * LQ + c], e, sa);
+          sm_ = fmaf(QC[ri * LQ + c], e, sm_);
+        }
+        accA[half] += sa;
+        accM[half] += sm_;
+      }
+      if (tid < 64) {
+        float s = 0.f;
+#pragma unroll 4
+        for (int c = 0; c < 32; ++c) s = fmaf(QC[tid * LQ + c], KC[tid * LQ + c], s);
+        accD[half] += s;
+      }
+      __syncthreads();
+    }
+  }
+  {                                                     // zeros on and above the diagonal, then the pairs
+    const int row = tid & 127, q = tid >> 7, b = row >> 4;
+    *reinterpret_cast<float4*>(tri::blk(Tp, b, b) + (row & 15) * tri::BP + 4 * q) = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int p = 2 * b + q; p < 16; p += 4) Mimg[p * 128 + row] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      if (dblk < 4) {
+        const int b2 = half * 4 + dblk, ri = b2 * 16 + di, rj = b2 * 16 + dj;
+        const bool same = seg_s[ri] == seg_s[rj];
+        tri::blk(Tp, b2, b2)[di * tri::BP + dj] = same ? accA[half] : 0.f;
+        M[rix(true, ri, rj, C)] = __float2bfloat16_rn(same ? accM[half] : 0.f);
+      }
+      if (tid < 64) M[rix(true, half * 64 + tid, half * 64 + tid, C)] = __float2bfloat16_rn(accD[half]);
+    }
+  }
+  // ---- the three levels; images of 32 channels in the place of X, one set at a time
+  uint4* KR = reinterpret_cast<uint4*>(sm + OFF_X);
+  uint4* QK = KR + 4 * PP;
+#pragma unroll 1
+  for (int lv = 0; lv < 3; ++lv) {
+#pragma unroll 1
+    for (int grp = 0; grp < 4; ++grp) {
+      decay(grp);
+      const int p = grp * 4 + lgrp, s = 16 << lv, ref = level_ref(x, s);
+      const bool lower = x >= ref;
+      float kh[8], qh[8], be[8], f[8];
+      khat8(r, x, p, kh);
+      qhat8(r, x, p, qh);
+      bact8(r, x, p, be);
+      decay8(LAM + (lower ? x : ref) * LQ + 8 * lgrp, LAM + (lower ? ref : x) * LQ + 8 * lgrp, f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float kf = kh[i] * f[i];
+        be[i] = lower ? be[i] * kh[i] * f[i] : kf;
+        qh[i] = lower ? qh[i] * f[i] : kf;
+      }
+      KR[lgrp * PP + x] = umma::pack8(be);
+      QK[lgrp * PP + x] = umma::pack8(qh);
+      umma::pre_issue_sync();
+      umma::issue_pitched<128, false, false>(cx, KR, PB, KR, PB, 32, 0, grp > 0);
+      umma::issue_pitched<128, false, false>(cx, QK, PB, KR, PB, 32, 128, grp > 0);
+      umma::commit_wait(cx);
+    }
+    const int quarter = warp & 3, group = warp >> 2, row = quarter * 32 + lane, bi = row >> 4;
+    const uint32_t tbase = cx.tmem + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll 1
+    for (int cc = 0; cc < 32; cc += 16) {
+      const int col = group * 32 + cc, bj = col >> 4;
+      float va[16], vm[16];
+      if (!cx.dead) {
+        umma::tmem_ld16(tbase + col, va);
+        umma::tmem_ld16(tbase + 128 + col, vm);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) va[i] = vm[i] = 0.f;
+      }
+      if (bj >= bi || owner_level(bi, bj) != lv) continue;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const bool same = seg_s[row] == seg_s[col + i];
+        va[i] = same ? va[i] : 0.f;
+        vm[i] = same ? vm[i] : 0.f;
+      }
+      float4* d = reinterpret_cast<float4*>(tri::blk(Tp, bi, bj) + (row & 15) * tri::BP);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) d[i] = make_float4(va[4 * i], va[4 * i + 1], va[4 * i + 2], va[4 * i + 3]);
+      Mimg[(col / 8) * 128 + row] = umma::pack8p(vm);
+      Mimg[(col / 8 + 1) * 128 + row] = umma::pack8p(vm + 8);
+    }
+    umma::tc_fence_before();
+  }
+  // ---- X again (its place was taken), and qe, ke from factors that cannot overflow
+  uint4* XI = reinterpret_cast<uint4*>(sm + OFF_X);
+  uint4* QE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.qe) + ibase * C * K);
+  uint4* KE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.ke) + ibase * C * K);
+  const bool first = seg_s[x] == seg_s[0], last = seg_s[x] == seg_s[C - 1];
+#pragma unroll 1
+  for (int grp = 0; grp < 4; ++grp) {
+    decay(grp);
+    const int p = grp * 4 + lgrp;
+    float kh[8], qh[8], be[8];
+    khat8(r, x, p, kh);
+    qhat8(r, x, p, qh);
+    bact8(r, x, p, be);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float lam = LAM[x * LQ + 8 * lgrp + i], lend = LAM[(C - 1) * LQ + 8 * lgrp + i];
+      const float el = first ? umma::exp_neg(fminf(lam, 0.f)) : 0.f;
+      be[i] = be[i] * kh[i] * el;
+      qh[i] *= el;
+      kh[i] = last ? kh[i] * umma::exp_neg(fminf(lend - lam, 0.f)) : 0.f;
+    }
+    XI[p * PP + x] = umma::pack8(be);
+    QE[p * 128 + x] = umma::pack8(qh);
+    KE[p * 128 + x] = umma::pack8(kh);
+  }
   __syncthreads();
 }
 
 template <int VW, int MODE>
-__global__ void __launch_bounds__(NT, 1) prepass_fwd_tc_kernel(PrepassFwdArgs a, int* err) {
+__global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid_constant__ PrepassFwdArgs a, int* err) {
   using CF = InCfg<MODE>;
-  extern __shared__ __align__(128) uint8_t smraw[];
-  __shared__ uint64_t mma_bar;
-  __shared__ uint32_t tmem_base;
+  extern __shared__ __align__(128) uint8_t sm[];
+  __shared__ uint64_t bar, gbar[2];                     // one barrier per set of group images: a barrier must not run two phases ahead of its waiters
+  __shared__ uint32_t tbase;
   __shared__ int seg_s[C];
-  __shared__ int reset_s[4];
-  __shared__ float rq_s[C], rk_s[C], bsc_s[C];
-  __shared__ uint8_t ds_s[C], de_s[C];                  // first / last row of each row's document inside the chunk
+  __shared__ int rst_s[16];
+  __shared__ float rq_s[C], rk_s[C];
+  __shared__ uint8_t ds_s[C], de_s[C];                  // first / last row of each row's document inside the tile
   const Geo& g = a.g;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int myrow = warp * 8 + (lane & 7), lgrp = lane >> 3;
-  float* LAM = reinterpret_cast<float*>(smraw);
-  uint4* KR = reinterpret_cast<uint4*>(smraw + OFF_IMG);
-  uint4* QK = KR + IMG;
-  float* KHs = reinterpret_cast<float*>(smraw + OFF_IMG);          // k_hat cache (pitch AP), diagonal pass
-  float* TOTL = reinterpret_cast<float*>(smraw + OFF_IMG);         // partial sums of the decay scan
-  uint4* XI = reinterpret_cast<uint4*>(smraw + OFF_XI);
-  float* Ts = reinterpret_cast<float*>(smraw);                     // inverse: T over Lambda,
-  float* As = reinterpret_cast<float*>(smraw + OFF_IMG);           //          A over the images / cache
-  float* Tm = reinterpret_cast<float*>(smraw + OFF_TM);
-  uint4* TI = reinterpret_cast<uint4*>(smraw + OFF_TI);
-  uint4* YI = reinterpret_cast<uint4*>(smraw + OFF_IMG);           // Y image over A, after the inverse
+  const int x = row_of(tid), lgrp = piece_of(tid);
+  float* LAM = reinterpret_cast<float*>(sm + OFF_LAM);
+  float* TOT = reinterpret_cast<float*>(sm + OFF_TOT);
+  float* EDGE = reinterpret_cast<float*>(sm + OFF_EDGE) + warp * 96;
+  uint4* XI = reinterpret_cast<uint4*>(sm + OFF_X);
+  if (tid == 0) { umma::mbar_init(&gbar[0], 1); umma::mbar_init(&gbar[1], 1); }
+  umma::Ctx cx = setup(&bar, &tbase, err);
+  uint32_t gph[2] = {0u, 0u};
+  auto group_wait = [&](int set) {                      // one warp polls; a barrier follows every use
+    bool ok = true;
+    if (warp == 0 && !cx.dead) ok = umma::mbar_wait(&gbar[set], gph[set]);
+    gph[set] ^= 1u;
+    return ok;
+  };
+  const bool fuse = CF::fixed ? false : (g.flags & DN_FUSE_PROLOGUE) != 0, guard = CF::fixed ? false : (g.flags & DN_STABILITY_GUARD) != 0;
+  const bool l2 = g.flags & DN_QK_L2NORM;
+  const int qdt = CF::fixed ? CF::qkv_dt : g.qkv_dt, gdt = CF::fixed ? DN_F32 : g.gate_dt;
+  const bool round_in = !fuse && qdt == DN_BF16;
+  const int kp = CF::fixed ? 16 : g.K / 8, gC = CF::fixed ? K : g.gC, bC = CF::fixed ? (CF::scalar_bw ? 1 : K) : g.bC;
+  const int wC = CF::fixed ? (CF::scalar_bw ? 1 : g.V) : g.wC;
+  const uint32_t qes = qdt == DN_BF16 ? 2 : 4, ges = gdt == DN_BF16 ? 2 : 4;
+  constexpr float FAST_HALF_RANGE = 32.f;
 
-  float* Ag = a.scratch + (size_t)blockIdx.x * a.scratch_per_cta;     // A (fp32, masked), panel layout
-  float4* Ag4 = reinterpret_cast<float4*>(Ag);
-
-  if (tid == 0) { umma::mbar_init(&mma_bar, 1); umma::fence_mbar_init(); }
-  if (warp == 0) umma::tmem_alloc(&tmem_base, 512);
-  umma::tc_fence_before();
-  __syncthreads();
-  umma::tc_fence_after();
-  umma::Ctx cx{tmem_base, &mma_bar, 0u, err, false};
-
-  const bool fuse = CF::fixed ? false : (g.flags & DN_FUSE_PROLOGUE) != 0;     // the fixed modes have no fused prologue
-  // tensor-memory columns: level products at [0, 256); operand cache at [256, 384) (k_hat | q_hat, two
-  // bf16 per column) and [384, 512) (beta, fp32)
-  constexpr uint32_t COL_KQ = 256, COL_BE = 384;
-
-  // work items in chunk-major order inside the chunk range: all heads of chunk c_begin first
   for (int e_item = blockIdx.x; e_item < a.items; e_item += gridDim.x) {
     const int bh = e_item % (g.B * g.H), c_idx = a.c_begin + e_item / (g.B * g.H);
-    const int h = bh % g.H, b = bh / g.H;
-    const int item = bh * g.NC + c_idx;
-    const int t0 = c_idx * C;
-    const size_t ibase = (size_t)item;
-    uint4* Wimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.W) + ibase * C * K);
-    uint4* Uimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.U) + ibase * C * VW);
-    uint4* Mimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.M) + ibase * C * C);
-    __nv_bfloat16* Mel = reinterpret_cast<__nv_bfloat16*>(a.res.M) + ibase * C * C;
-    uint4* QEimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.qe) + ibase * C * K);
-    uint4* KEimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.ke) + ibase * C * K);
-
-    DN_MARK(0);
-    for (int i = tid; i < C; i += NT) seg_s[i] = seg_at(a.seg, b, t0 + i, g.L);
-    const Rows r = make_rows<CF>(g, a.q, a.k, a.gg, a.b, b, h, t0, rq_s, rk_s);
-    const int qdt = r.qkv_dt, gdt = r.gate_dt;           // compile-time constants in the fixed modes
-    const int wC = CF::fixed ? (CF::scalar_bw ? 1 : g.V) : g.wC;
-    const bool tm_cache = r.round_in;                    // k_hat, q_hat exactly bf16: they can be packed two per column
-    __syncthreads();
-    const int seg0 = seg_s[0], segL = seg_s[C - 1];
-    row_norms_8x4(r, myrow, lgrp, rq_s, rk_s);             // no barrier in between: the loads of q, k and g
-    lambda_scan_512(r, seg_s, LAM, TOTL, reset_s);         // are all in flight together
-    __syncthreads();
-
-    // ---- 16x16 diagonal blocks, exact.  k_hat, q_hat and beta of 64 rows at a time are cached in
-    //      shared memory (fp32; one global round trip per half); four warps per block take every
-    //      fourth row i, lanes own 4 channels, and every pair (i, j <= i) is one warp reduction.
-    const uint32_t tm_lane = cx.tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    auto diag_pass = [&]() {
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-      float* QHs = KHs + 64 * AP;                                       // q_hat (pitch AP)
-      float* BEs = reinterpret_cast<float*>(smraw + OFF_TI);            // beta (pitch 128)
+    const int h = bh % g.H, b = bh / g.H, t0 = c_idx * C;
+    const size_t ibase = (size_t)bh * g.NC + c_idx;
+    const int rows = g.L - t0 < C ? g.L - t0 : C;
+    const bool live = x < rows;                         // rows past the end read row 0 and are zeroed
+    const size_t tok = (size_t)b * g.L + t0 + (live ? x : 0);
+    const uint8_t* krow = reinterpret_cast<const uint8_t*>(a.k) + (tok * g.Hk + h / g.qk_div) * g.K * qes;
+    const uint8_t* qrow = reinterpret_cast<const uint8_t*>(a.q) + (tok * g.Hk + h / g.qk_div) * g.K * qes;
+    const uint8_t* brow = reinterpret_cast<const uint8_t*>(a.b) + (tok * g.bH + g.gate_head(h, g.bH)) * bC * ges;
+    // decay of a group of 32 channels: thread (channel = lane, rows 8 warp .. 8 warp + 7)
+    const uint32_t gpitch = (uint32_t)(g.gH * gC) * ges;
+    const uint8_t* grow = reinterpret_cast<const uint8_t*>(a.gg) +
+        (((size_t)b * g.L + t0 + (warp * 8 < rows ? warp * 8 : 0)) * g.gH + g.gate_head(h, g.gH)) * gC * ges + (gC == 1 ? 0 : lane) * ges;
+    float gv[8];
+    auto load_g = [&](int grp) {
+      const bool cin = gC == 1 || CF::fixed || 32 * grp < gC;
+      const uint8_t* gp = grow + (gC == 1 ? 0 : 32 * grp * ges);
+      if (rows == C && cin) {
 #pragma unroll
-      for (int it = 0; it < 2; ++it) {
-        const int w = it * 16 + warp, xr = (w & 7) * 8 + (lane & 7), p = (w >> 3) * 4 + lgrp, x = half * 64 + xr;
-        float kh[8], qh[8], ba[8];
-        khat8(r, x, p, kh);
-        qhat8(r, x, p, qh);
-        bact8(r, x, p, ba);
+        for (int i = 0; i < 8; ++i) gv[i] = ldf_ro(gp + i * gpitch, 0, gdt);
+      } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) ba[i] *= kh[i];
-        *reinterpret_cast<float4*>(KHs + xr * AP + 8 * p) = make_float4(kh[0], kh[1], kh[2], kh[3]);
-        *reinterpret_cast<float4*>(KHs + xr * AP + 8 * p + 4) = make_float4(kh[4], kh[5], kh[6], kh[7]);
-        *reinterpret_cast<float4*>(QHs + xr * AP + 8 * p) = make_float4(qh[0], qh[1], qh[2], qh[3]);
-        *reinterpret_cast<float4*>(QHs + xr * AP + 8 * p + 4) = make_float4(qh[4], qh[5], qh[6], qh[7]);
-        *reinterpret_cast<float4*>(BEs + xr * 128 + 8 * p) = make_float4(ba[0], ba[1], ba[2], ba[3]);
-        *reinterpret_cast<float4*>(BEs + xr * 128 + 8 * p + 4) = make_float4(ba[4], ba[5], ba[6], ba[7]);
+        for (int i = 0; i < 8; ++i) gv[i] = cin && warp * 8 + i < rows ? ldf_ro(gp + i * gpitch, 0, gdt) : (fuse ? -INFINITY : 0.f);
       }
-      __syncthreads();
-      DN_MARK(20 + 3 * half);
-      if (tm_cache && ((warp & 3) >> 1) == half) {
-        // every later pass (qe / ke / X, the three levels) reads k_hat, q_hat and beta from tensor
-        // memory: thread = row (its own lane), the four warps of a lane quarter take 32 channels each
-        const int xr = (warp & 3) * 32 + lane - 64 * half, cg0 = (warp >> 2) * 32;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int c0 = cg0 + 8 * j;
-          float kq[8], be8[8];
-          const float4 k0 = *reinterpret_cast<const float4*>(KHs + xr * AP + c0), k1 = *reinterpret_cast<const float4*>(KHs + xr * AP + c0 + 4);
-          const float4 q0 = *reinterpret_cast<const float4*>(QHs + xr * AP + c0), q1 = *reinterpret_cast<const float4*>(QHs + xr * AP + c0 + 4);
-          const float4 b0 = *reinterpret_cast<const float4*>(BEs + xr * 128 + c0), b1 = *reinterpret_cast<const float4*>(BEs + xr * 128 + c0 + 4);
-          const float kk[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w}, qq[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-#pragma unroll
-          for (int i = 0; i < 8; ++i)                   // both are exactly representable in bf16 here
-            kq[i] = __uint_as_float((__float_as_uint(kk[i]) >> 16) | (__float_as_uint(qq[i]) & 0xffff0000u));
-          be8[0] = b0.x; be8[1] = b0.y; be8[2] = b0.z; be8[3] = b0.w; be8[4] = b1.x; be8[5] = b1.y; be8[6] = b1.z; be8[7] = b1.w;
-          umma::tmem_st8(tm_lane + COL_KQ + c0, kq);
-          umma::tmem_st8(tm_lane + COL_BE + c0, be8);
-        }
-        umma::tmem_wait_st();
-      }
-      const int lb = warp >> 2, r0 = (half * 4 + lb) * 16, c0 = lb * 16;   // block rows in the chunk / in the caches
-#pragma unroll 1
-      for (int i = warp & 3; i < 16; i += 4) {
-        const int ri = r0 + i;
-        const float4 q4 = *reinterpret_cast<const float4*>(QHs + (c0 + i) * AP + 4 * lane);
-        const float4 b4 = *reinterpret_cast<const float4*>(BEs + (c0 + i) * 128 + 4 * lane);
-        const float4 li = *reinterpret_cast<const float4*>(LAM + ri * LP + 4 * lane);
-        const float qi[4] = {q4.x, q4.y, q4.z, q4.w}, bi4[4] = {b4.x, b4.y, b4.z, b4.w};
-        float arow = 0.f, mrow = 0.f;                  // lane j (< 16) keeps entry (ri, r0 + j)
-        const bool hi16 = lane & 16, hi8 = lane & 8, hi4 = lane & 4;
-#pragma unroll 1
-        for (int j = 0; j <= i; j += 4) {              // four columns per step, reduced together (see below)
-          float v[8];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int cj = j + u < 16 ? j + u : 15;    // (a column past the block is computed and dropped)
-            const float4 kk = *reinterpret_cast<const float4*>(KHs + (c0 + cj) * AP + 4 * lane);
-            const float4 ll = *reinterpret_cast<const float4*>(LAM + (r0 + cj) * LP + 4 * lane);
-            const float e0 = kk.x * umma::ex2_fast(fminf(li.x - ll.x, 0.f) * DN_LOG2E), e1 = kk.y * umma::ex2_fast(fminf(li.y - ll.y, 0.f) * DN_LOG2E);
-            const float e2 = kk.z * umma::ex2_fast(fminf(li.z - ll.z, 0.f) * DN_LOG2E), e3 = kk.w * umma::ex2_fast(fminf(li.w - ll.w, 0.f) * DN_LOG2E);
-            v[2 * u] = bi4[0] * e0 + bi4[1] * e1 + bi4[2] * e2 + bi4[3] * e3;
-            v[2 * u + 1] = qi[0] * e0 + qi[1] * e1 + qi[2] * e2 + qi[3] * e3;
-          }
-          // eight sums over the 32 lanes in 9 shuffles: at each of the first three steps a lane hands
-          // over the half it drops and adds what it receives to the half it keeps
-          float w4[4], u2[2], z;
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            const float got = __shfl_xor_sync(0xffffffffu, hi16 ? v[t] : v[4 + t], 16);
-            w4[t] = (hi16 ? v[4 + t] : v[t]) + got;
-          }
-#pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            const float got = __shfl_xor_sync(0xffffffffu, hi8 ? w4[t] : w4[2 + t], 8);
-            u2[t] = (hi8 ? w4[2 + t] : w4[t]) + got;
-          }
-          {
-            const float got = __shfl_xor_sync(0xffffffffu, hi4 ? u2[0] : u2[1], 4);
-            z = (hi4 ? u2[1] : u2[0]) + got;
-          }
-          z += __shfl_xor_sync(0xffffffffu, z, 2);
-          z += __shfl_xor_sync(0xffffffffu, z, 1);
-          // lane 16*(u>>1) + 8*(u&1) + 4*t now holds column j+u's sum of kind t (0: A, 1: M)
-          const int u = lane - j;                      // the column this lane keeps, if 0 <= u < 4
-          const int src = (u >= 0 && u < 4) ? 16 * (u >> 1) + 8 * (u & 1) : 0;
-          const float pa = __shfl_sync(0xffffffffu, z, src), pm = __shfl_sync(0xffffffffu, z, src + 4);
-          if (u >= 0 && u < 4 && lane <= i) {
-            const bool same = seg_s[ri] == seg_s[r0 + lane];
-            arow = (lane < i && same) ? pa : 0.f;
-            mrow = same ? pm : 0.f;
-          }
-        }
-        if (lane < 16) {
-          umma::st_keep1(Ag + p4f(ri, r0 + lane), arow);
-          Mel[rix(true, ri, r0 + lane, C)] = __float2bfloat16_rn(mrow);
-        }
-      }
-      DN_MARK(21 + 3 * half);
-      __syncthreads();
-      DN_MARK(22 + 3 * half);
-    }
     };
-
-    // ---- qe, ke, the X = [first doc] beta e^Lam operand image and the images of the first level for
-    //      one piece (row x, channels 8p..8p+7), from k_hat, q_hat and beta = b_act * k_hat
-    auto xi_piece = [&](int x, int p, const float (&kh)[8], const float (&qh)[8], const float (&be)[8]) {
-      const bool first = seg_s[x] == seg0, last = seg_s[x] == segL;
-      float lam[8], lend[8], o[8], el[8];
-      *reinterpret_cast<float4*>(lam) = *reinterpret_cast<const float4*>(LAM + x * LP + 8 * p);
-      *reinterpret_cast<float4*>(lam + 4) = *reinterpret_cast<const float4*>(LAM + x * LP + 8 * p + 4);
-      *reinterpret_cast<float4*>(lend) = *reinterpret_cast<const float4*>(LAM + (C - 1) * LP + 8 * p);
-      *reinterpret_cast<float4*>(lend + 4) = *reinterpret_cast<const float4*>(LAM + (C - 1) * LP + 8 * p + 4);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) el[i] = umma::exp_neg(fminf(lam[i], 0.f));
-#pragma unroll
-      for (int i = 0; i < 8; ++i) o[i] = first ? qh[i] * el[i] : 0.f;
-      QEimg[p * 128 + x] = umma::pack8(o);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) o[i] = last ? kh[i] * umma::exp_neg(fminf(lend[i] - lam[i], 0.f)) : 0.f;
-      KEimg[p * 128 + x] = umma::pack8(o);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) o[i] = first ? be[i] * el[i] : 0.f;
-      XI[p * 128 + x] = umma::pack8(o);
-      build_level_from_beta(kh, be, qh, LAM, 16, x, p, KR, QK);
-    };
-    // the cached operands of row x = this thread's tensor-memory lane, piece p
-    auto cached_piece = [&](int p, float (&kh)[8], float (&qh)[8], float (&be)[8]) {
-      float kq[8];
-      umma::tmem_ld8(tm_lane + COL_KQ + 8 * p, kq);
-      umma::tmem_ld8(tm_lane + COL_BE + 8 * p, be);
+    auto act_g = [&]() {                                // the activated decay (rows past the end: 0)
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        kh[i] = __uint_as_float(__float_as_uint(kq[i]) << 16);
-        qh[i] = __uint_as_float(__float_as_uint(kq[i]) & 0xffff0000u);
+        if (fuse) { const bool off = gv[i] == -INFINITY; gv[i] = off ? 0.f : -umma::ex2_fast(fminf(gv[i], 5.f) * DN_LOG2E); if (guard && !off) gv[i] = fminf(gv[i], -1e-6f); }
+        else { gv[i] = gv[i] <= 0.f ? gv[i] : 0.f; if (guard && warp * 8 + i < rows) gv[i] = fminf(gv[i], -1e-6f); }
       }
     };
-    auto xi_pass = [&]() {
-      if (tm_cache) {
-        const int x = (warp & 3) * 32 + lane;
-#pragma unroll 2
-        for (int j = 0; j < 4; ++j) {
-          const int p = (warp >> 2) * 4 + j;
-          float kh[8], qh[8], be[8];
-          cached_piece(p, kh, qh, be);
-          xi_piece(x, p, kh, qh, be);
-        }
-      } else {
-#pragma unroll 2
-        for (int it = 0; it < 4; ++it) {
-          const int p = it * 4 + lgrp;
-          float qh[8], kh[8], be[8];
-          qhat8(r, myrow, p, qh);
-          khat8(r, myrow, p, kh);
-          bact8(r, myrow, p, be);
+    load_g(0);
+    if (tid < C) seg_s[tid] = seg_at(a.seg, b, t0 + tid, g.L);
+    float rq = 1.f, rk = 1.f;
+    if (l2) {
+      float sq = 0.f, sk = 0.f;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) be[i] *= kh[i];
-          xi_piece(myrow, p, kh, qh, be);
+      for (int it = 0; it < 4; ++it) {
+        const int p = it * 4 + lgrp;
+        if (CF::fixed || p < kp) {
+          float f[8];
+          cvraw(ldraw(qrow, p, qdt), qdt, f);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) sq = fmaf(f[i], f[i], sq);
+          cvraw(ldraw(krow, p, qdt), qdt, f);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) sk = fmaf(f[i], f[i], sk);
         }
       }
-      if (tid < K) a.res.lam_end[ibase * K + tid] = LAM[(C - 1) * LP + tid];
+      sq += __shfl_xor_sync(0xffffffffu, sq, 1);  sk += __shfl_xor_sync(0xffffffffu, sk, 1);
+      sq += __shfl_xor_sync(0xffffffffu, sq, 2); sk += __shfl_xor_sync(0xffffffffu, sk, 2);
+      rq = rsqrtf(sq + 1e-6f);
+      rk = rsqrtf(sk + 1e-6f);
+    }
+    const float rqs = rq * g.scale;
+    if (lgrp == 0) { rq_s[x] = rq; rk_s[x] = rk; }      // (for the hierarchical route)
+    Raw8 kr, qr, br;                                    // this thread's piece of the group about to be built
+    float b1 = 0.f;
+    auto load_kqb = [&](int grp) {
+      const int p = grp * 4 + lgrp, pc = CF::fixed || p < kp ? p : 0;
+      kr = ldraw(krow, pc, qdt);
+      qr = ldraw(qrow, pc, qdt);
+      if (bC != 1) br = ldraw(brow, pc, gdt);
     };
-
-    if constexpr (CF::scalar_gates) {
-      // ---- one scalar decay and one scalar beta per (token, head): the decay leaves the channel sum,
-      //      A_ij = beta_i e^{lam_i - lam_j} (k_i . k_j),  M_ij = e^{lam_i - lam_j} (q_i . k_j),
-      //      so A and M are two Gram products on the plain bf16 images of k_hat and q_hat, and the decay
-      //      (exact, <= 1) is applied per entry by the drain.  No levels, no diagonal pass.
-      DN_MARK(1);
-      {
-        const int x = myrow;
-        const bool first = seg_s[x] == seg0, last = seg_s[x] == segL;
-        const bool live = x < r.rows_valid;
-        const float lam = LAM[x * LP], lend = LAM[(C - 1) * LP];
-        const float el = umma::exp_neg(fminf(lam, 0.f)), eke = umma::exp_neg(fminf(lend - lam, 0.f));
-        const float bx = live ? ldf_ro(r.b, r.b_row0 + (size_t)x * r.b_pitch, DN_F32) : 0.f;
-#pragma unroll 2
-        for (int it = 0; it < 4; ++it) {
-          const int p = it * 4 + lgrp;
-          float qh[8], kh[8], o[8];
-          qhat8(r, x, p, qh);
-          khat8(r, x, p, kh);
-          KR[p * 128 + x] = umma::pack8(kh);
-          QK[p * 128 + x] = umma::pack8(qh);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] = first ? qh[i] * el : 0.f;
-          QEimg[p * 128 + x] = umma::pack8(o);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] = last ? kh[i] * eke : 0.f;
-          KEimg[p * 128 + x] = umma::pack8(o);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] = first ? (bx * kh[i]) * el : 0.f;
-          XI[p * 128 + x] = umma::pack8(o);
-        }
-        if (lgrp == 0) bsc_s[x] = bx;
-        if (tid < K) a.res.lam_end[ibase * K + tid] = lend;
-      }
-      DN_MARK(2);
-      umma::pre_issue_sync();
-      umma::issue<128, false, false>(cx, KR, KR, K, 0, false);             // k_hat k_hat^T
-      umma::issue<128, false, false>(cx, QK, KR, K, 128, false);           // q_hat k_hat^T
-      umma::commit_wait(cx);
-      DN_MARK(3);
-      {
-        const int quarter = warp & 3, group = warp >> 2;
-        const int row = quarter * 32 + lane;
-        const uint32_t tbase = cx.tmem + ((uint32_t)(quarter * 32) << 16);
-        const float lrow = LAM[row * LP] * DN_LOG2E, brow = bsc_s[row];
-        const int srow = seg_s[row];
-#pragma unroll 1
-        for (int cc = 0; cc < 32; cc += 16) {
-          const int col = group * 32 + cc;
-          float va[16], vm[16];
-          if (!cx.dead && col <= quarter * 32 + 31) {    // warp-uniform: a piece wholly above the warp's rows is zeros
-            umma::tmem_ld16(tbase + col, va);
-            umma::tmem_ld16(tbase + 128 + col, vm);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) va[i] = vm[i] = 0.f;
-          }
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int j = col + i;
-            const bool same = srow == seg_s[j];
-            const float f = umma::ex2_fast(fminf(lrow - LAM[j * LP] * DN_LOG2E, 0.f));
-            va[i] = (same && j < row) ? brow * f * va[i] : 0.f;
-            vm[i] = (same && j <= row) ? f * vm[i] : 0.f;
-          }
-#pragma unroll
-          for (int i = 0; i < 4; ++i) umma::st_keep4(Ag4 + p4v(row, col + 4 * i), make_float4(va[4 * i], va[4 * i + 1], va[4 * i + 2], va[4 * i + 3]));
-          Mimg[(col / 8) * 128 + row] = umma::pack8p(vm);
-          Mimg[(col / 8 + 1) * 128 + row] = umma::pack8p(vm + 8);
-        }
-        umma::tc_fence_before();
-      }
-      __syncthreads();
-      DN_MARK(6);
-    } else {
-    // ---- Channel-wise decay.  When the decay of every document inside the chunk is moderate in every
-    //      channel, A and M are single Gram products as well: with m_c the midpoint of a document's
-    //      cumulative decay in channel c and f_ic = e^{Lam_ic - m_c},
-    //        A_ij = sum_c (beta_ic f_ic) (k_jc / f_jc),   M_ij = sum_c (q_ic f_ic) (k_jc / f_jc)
-    //      for i, j in one document, and every factor stays within e^{+-FAST_HALF_RANGE}: nothing can
-    //      overflow, and bf16 keeps its relative precision at any magnitude.  Chunks with a stronger decay
-    //      (half range above the bound in some channel of some document) take the hierarchical
-    //      factorisation below, whose factors never exceed 1 whatever the decay.
-    constexpr float FAST_HALF_RANGE = 32.f;
-    if (tid < C) {                              // first and last row of each row's document inside the chunk
+    load_kqb(0);
+    if (bC == 1) b1 = ldf_ro(brow, 0, gdt);
+    __syncthreads();
+    if (tid < C) {                                      // seg_s is non-decreasing: binary searches
       const int sx = seg_s[tid];
-      int lo = 0, hi = tid;                     // seg_s is non-decreasing: binary searches
+      int lo = 0, hi = tid;
       while (lo < hi) { const int mid = (lo + hi) >> 1; if (seg_s[mid] < sx) lo = mid + 1; else hi = mid; }
       ds_s[tid] = (uint8_t)lo;
       lo = tid; hi = C - 1;
       while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (seg_s[mid] > sx) hi = mid - 1; else lo = mid; }
       de_s[tid] = (uint8_t)lo;
     }
-    __syncthreads();
-    // one test per document and channel, at the document's last row: threads (row x, channel quarter)
+    // which of this warp's 8 rows start a document
+    const uint32_t cuts = __ballot_sync(0xffffffffu, lane < 8 && warp * 8 + lane > 0 && seg_s[warp * 8 + lane] != seg_s[warp * 8 + lane - (warp * 8 + lane > 0)]);
+    const int nr = cuts ? __ffs(cuts) - 1 : 8;
+    if (lane == 0) rst_s[warp] = cuts != 0;
+    EDGE[64 + lane] = 0.f;
     bool strong = false;
-    {
-      const int x = tid & 127;
-      if (de_s[x] == x) {
-        const float* ls = LAM + ds_s[x] * LP + (tid >> 7) * 32;
-        const float* le = LAM + x * LP + (tid >> 7) * 32;
-#pragma unroll 8
-        for (int c = 0; c < 32; ++c) strong |= 0.5f * (ls[c] - le[c]) > FAST_HALF_RANGE;
-      }
-    }
-    const bool fast = !__syncthreads_or(strong);
-    if (fast) {
-      DN_MARK(1);
-      uint4* BT = reinterpret_cast<uint4*>(smraw + OFF_TI);      // third image (beta f); the T image is built later
-      {
-        const int x = myrow;
-        const bool first = seg_s[x] == seg0, last = seg_s[x] == segL;
-        const float* lam_s = LAM + ds_s[x] * LP;
-        const float* lam_e = LAM + de_s[x] * LP;
-#pragma unroll 2
-        for (int it = 0; it < 4; ++it) {
-          const int p = it * 4 + lgrp;
-          float qh[8], kh[8], be[8], lam[8], ls[8], le[8], lend[8], o1[8], o2[8], o3[8];
-          qhat8(r, x, p, qh);
-          khat8(r, x, p, kh);
-          bact8(r, x, p, be);
-          *reinterpret_cast<float4*>(lam) = *reinterpret_cast<const float4*>(LAM + x * LP + 8 * p);
-          *reinterpret_cast<float4*>(lam + 4) = *reinterpret_cast<const float4*>(LAM + x * LP + 8 * p + 4);
-          *reinterpret_cast<float4*>(ls) = *reinterpret_cast<const float4*>(lam_s + 8 * p);
-          *reinterpret_cast<float4*>(ls + 4) = *reinterpret_cast<const float4*>(lam_s + 8 * p + 4);
-          *reinterpret_cast<float4*>(le) = *reinterpret_cast<const float4*>(lam_e + 8 * p);
-          *reinterpret_cast<float4*>(le + 4) = *reinterpret_cast<const float4*>(lam_e + 8 * p + 4);
-          *reinterpret_cast<float4*>(lend) = *reinterpret_cast<const float4*>(LAM + (C - 1) * LP + 8 * p);
-          *reinterpret_cast<float4*>(lend + 4) = *reinterpret_cast<const float4*>(LAM + (C - 1) * LP + 8 * p + 4);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            be[i] *= kh[i];                                             // beta = b_act * k_hat
-            const float d = (lam[i] - 0.5f * (ls[i] + le[i])) * DN_LOG2E;      // log2 f, |d| <= FAST_HALF_RANGE * log2 e
-            const float f = umma::ex2_fast(d), fi = umma::ex2_fast(-d);
-            o1[i] = kh[i] * fi;
-            o2[i] = qh[i] * f;
-            o3[i] = be[i] * f;
-          }
-          KR[p * 128 + x] = umma::pack8(o1);
-          QK[p * 128 + x] = umma::pack8(o2);
-          BT[p * 128 + x] = umma::pack8(o3);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float el = umma::exp_neg(fminf(lam[i], 0.f));
-            o1[i] = first ? qh[i] * el : 0.f;
-            o2[i] = last ? kh[i] * umma::exp_neg(fminf(lend[i] - lam[i], 0.f)) : 0.f;
-            o3[i] = first ? be[i] * el : 0.f;
-          }
-          QEimg[p * 128 + x] = umma::pack8(o1);
-          KEimg[p * 128 + x] = umma::pack8(o2);
-          XI[p * 128 + x] = umma::pack8(o3);
-        }
-        if (tid < K) a.res.lam_end[ibase * K + tid] = LAM[(C - 1) * LP + tid];
-      }
-      DN_MARK(2);
-      umma::pre_issue_sync();
-      umma::issue<128, false, false>(cx, BT, KR, K, 0, false);             // A = (beta f) (k / f)^T
-      umma::issue<128, false, false>(cx, QK, KR, K, 128, false);           // M = (q f) (k / f)^T
-      umma::commit_wait(cx);
-      DN_MARK(3);
-      {
-        const int quarter = warp & 3, group = warp >> 2;
-        const int row = quarter * 32 + lane;
-        const uint32_t tbase = cx.tmem + ((uint32_t)(quarter * 32) << 16);
-        const int srow = seg_s[row];
+    const bool first = seg_s[x] == seg_s[0], last = seg_s[x] == seg_s[C - 1];
 #pragma unroll 1
-        for (int cc = 0; cc < 32; cc += 16) {
-          const int col = group * 32 + cc;
-          float va[16], vm[16];
-          if (!cx.dead && col <= quarter * 32 + 31) {    // warp-uniform: a piece wholly above the warp's rows is zeros
-            umma::tmem_ld16(tbase + col, va);
-            umma::tmem_ld16(tbase + 128 + col, vm);
-          } else {
+    for (int grp = 0; grp < 4; ++grp) {
+      act_g();
+      if (cuts == 0) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) va[i] = vm[i] = 0.f;
-          }
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int j = col + i;
-            const bool same = srow == seg_s[j];
-            va[i] = (same && j < row) ? va[i] : 0.f;
-            vm[i] = (same && j <= row) ? vm[i] : 0.f;
-          }
-#pragma unroll
-          for (int i = 0; i < 4; ++i) umma::st_keep4(Ag4 + p4v(row, col + 4 * i), make_float4(va[4 * i], va[4 * i + 1], va[4 * i + 2], va[4 * i + 3]));
-          Mimg[(col / 8) * 128 + row] = umma::pack8p(vm);
-          Mimg[(col / 8 + 1) * 128 + row] = umma::pack8p(vm + 8);
-        }
-        umma::tc_fence_before();
-      }
-      __syncthreads();
-      DN_MARK(6);
-    } else {
-    DN_MARK(1);
-    if (tm_cache) diag_pass();                 // first: it also fills the tensor-memory operand cache
-    xi_pass();
-
-    DN_MARK(2);
-    // ---- A and M, level by level: two images, two MMAs, one predicated drain per level
-    auto build = [&](int lv) {
-      if (tm_cache) {
-        const int x = (warp & 3) * 32 + lane;
-#pragma unroll 2
-        for (int j = 0; j < 4; ++j) {
-          const int p = (warp >> 2) * 4 + j;
-          float kh[8], qh[8], be[8];
-          cached_piece(p, kh, qh, be);
-          build_level_from_beta(kh, be, qh, LAM, 16 << lv, x, p, KR, QK);
-        }
+        for (int i = 1; i < 8; ++i) gv[i] += gv[i - 1];
       } else {
-#pragma unroll 2
-        for (int it = 0; it < 4; ++it) build_level_piece(r, LAM, 16 << lv, myrow, it * 4 + lgrp, KR, QK);
-      }
-    };
-    auto drain_level = [&](int lv) {
-      const int quarter = warp & 3, group = warp >> 2;
-      const int row = quarter * 32 + lane, bi = row >> 4, bi0 = quarter * 2;
-      const uint32_t tbase = cx.tmem + ((uint32_t)(quarter * 32) << 16);
-#pragma unroll 1
-      for (int cc = 0; cc < 32; cc += 16) {
-        const int col = group * 32 + cc, bj = col >> 4;
-        // warp-uniform skip: neither of the warp's two row blocks has this piece at this level
-        const bool own0 = bj < bi0 && owner_level(bi0, bj) == lv, own1 = bj < bi0 + 1 && owner_level(bi0 + 1, bj) == lv;
-        const bool upper = lv == 0 && bj > bi0;                  // zero fill, once
-        if (!own0 && !own1 && !upper) continue;
-        float va[16], vm[16];
-        if (!cx.dead && (own0 || own1)) {
-          umma::tmem_ld16(tbase + col, va);
-          umma::tmem_ld16(tbase + 128 + col, vm);
-        } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) va[i] = vm[i] = 0.f;
+        for (int i = 1; i < 8; ++i) gv[i] += (cuts >> i) & 1 ? 0.f : gv[i - 1];
+      }
+      TOT[warp * 32 + lane] = gv[7];
+      __syncthreads();
+      // rows above hand on the sums back to the last warp in which a document starts
+      const uint32_t above = __ballot_sync(0xffffffffu, lane < warp && rst_s[lane & 15]);
+      float carry = 0.f;
+      for (int w2 = warp - 1, lo = above ? 31 - __clz(above) : 0; w2 >= lo; --w2) carry += TOT[w2 * 32 + lane];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {                     // kept in units of log 2
+        if (i < nr) gv[i] += carry;
+        LAM[(warp * 8 + i) * LQ + lane] = gv[i] * DN_LOG2E;
+      }
+      const float lam_last = gv[7];
+      bool ok = true;
+      if (grp >= 2) ok = group_wait(grp & 1);           // the set this group writes was read by the products of group - 2
+      if (__syncthreads_or(!ok)) { cx.dead = true; umma::report_timeout(err); }
+      uint4* KF = reinterpret_cast<uint4*>(sm + OFF_GI + (grp & 1) * 3 * 4 * PB);
+      uint4* QF = KF + 4 * PP;
+      uint4* BF = QF + 4 * PP;
+      // e^Lam = f e^{mid} and e^{Lam_end - Lam} = f^-1 e^{Lam_end - mid}, and they are only wanted in the first and the
+      // last document: two factors per channel, formed once per warp (lane = channel) instead of two exponentials per element
+      {
+        const float l9 = LAM[(C - 1) * LQ + lane];
+        EDGE[lane] = umma::ex2_fast(0.5f * (LAM[lane] + LAM[de_s[0] * LQ + lane]));
+        EDGE[32 + lane] = umma::ex2_fast(0.5f * (l9 - LAM[ds_s[C - 1] * LQ + lane]));
+        __syncwarp();
+      }
+      const int p = grp * 4 + lgrp;
+      const bool on = live && (CF::fixed || p < kp);
+      if (!on) kr.a = kr.b = qr.a = qr.b = make_uint4(0, 0, 0, 0);
+      float qh[8], kh[8], be[8], d8[8];
+      cvraw(kr, qdt, kh);
+      cvraw(qr, qdt, qh);
+      if (bC == 1) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) be[i] = b1;
+      } else cvraw(br, gdt, be);
+      {
+        const float* lx = LAM + x * LQ + 8 * lgrp;
+        const float* ls = LAM + ds_s[x] * LQ + 8 * lgrp;
+        const float* le = LAM + de_s[x] * LQ + 8 * lgrp;
+#pragma unroll
+        for (int i = 0; i < 8; i += 4) {
+          const float4 u0 = *reinterpret_cast<const float4*>(lx + i), u1 = *reinterpret_cast<const float4*>(ls + i), u2 = *reinterpret_cast<const float4*>(le + i);
+          d8[i] = fmaf(-0.5f, u1.x + u2.x, u0.x); d8[i + 1] = fmaf(-0.5f, u1.y + u2.y, u0.y);
+          d8[i + 2] = fmaf(-0.5f, u1.z + u2.z, u0.z); d8[i + 3] = fmaf(-0.5f, u1.w + u2.w, u0.w);
         }
-        const bool mine = bj < bi && owner_level(bi, bj) == lv;
-        const bool zero_fill = lv == 0 && bj > bi;
-        if (!mine && !zero_fill) continue;
+      }
+      float o1[8], o2[8], o3[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { kh[i] *= rk; qh[i] *= rqs; }
+      if (round_in) {
+        const uint4 pk = umma::pack8(kh), pq = umma::pack8(qh);
+        umma::unpack8(pk, kh);
+        umma::unpack8(pq, qh);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (fuse) be[i] = sigmoid_fast(be[i]); else if (guard) be[i] = fmaxf(be[i], 0.f);
+        be[i] *= kh[i];                                               // beta = b_act * k_hat
+        // log2 f; the decay is monotone inside a document, so the largest |log2 f| is half its range
+        strong |= fabsf(d8[i]) > FAST_HALF_RANGE * DN_LOG2E;
+        const float f = umma::ex2_fast(d8[i]), fi = umma::ex2_fast(-d8[i]);
+        o1[i] = kh[i] * fi;
+        o2[i] = qh[i] * f;
+        o3[i] = be[i] * f;
+      }
+      KF[lgrp * PP + x] = umma::pack8(o1);
+      QF[lgrp * PP + x] = umma::pack8(o2);
+      BF[lgrp * PP + x] = umma::pack8(o3);
+      umma::pre_issue_sync();
+      umma::issue_pitched<128, false, false>(cx, BF, PB, KF, PB, 32, 0, grp > 0);        // A += (beta f) (k / f)^T
+      umma::issue_pitched<128, false, false>(cx, QF, PB, KF, PB, 32, 128, grp > 0);      // M += (q f) (k / f)^T
+      if (tid == 0 && !cx.dead) umma::mma_commit(&gbar[grp & 1]);
+      // global stores and the next group's loads come behind the proxy fence, which waits for what precedes it
+      {
+        uint4* QE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.qe) + ibase * C * K);
+        uint4* KE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.ke) + ibase * C * K);
+        const float* pf = EDGE + (first ? 0 : 64) + 8 * lgrp;
+        const float* pl = EDGE + (last ? 32 : 64) + 8 * lgrp;
+#pragma unroll
+        for (int i = 0; i < 8; i += 4) {
+          const float4 u = *reinterpret_cast<const float4*>(pf + i), w = *reinterpret_cast<const float4*>(pl + i);
+          o2[i] *= u.x; o2[i + 1] *= u.y; o2[i + 2] *= u.z; o2[i + 3] *= u.w;
+          o3[i] *= u.x; o3[i + 1] *= u.y; o3[i + 2] *= u.z; o3[i + 3] *= u.w;
+          o1[i] *= w.x; o1[i + 1] *= w.y; o1[i + 2] *= w.z; o1[i + 3] *= w.w;
+        }
+        QE[p * 128 + x] = umma::pack8(o2);
+        KE[p * 128 + x] = umma::pack8(o1);
+        XI[p * PP + x] = umma::pack8(o3);
+        if (warp == 15) a.res.lam_end[ibase * K + 32 * grp + lane] = lam_last;
+      }
+      if (grp < 3) { load_g(grp + 1); load_kqb(grp + 1); }
+    }
+    const bool ok0 = group_wait(0), ok1 = group_wait(1);
+    if (__syncthreads_or(!(ok0 && ok1))) { cx.dead = true; umma::report_timeout(err); }
+    umma::tc_fence_after();
+    if (__syncthreads_or(strong)) {
+      umma::Ctx c2 = cx;
+      strong_route<MODE>(a, b, h, t0, ibase, rq_s, rk_s, seg_s, rst_s, sm, c2);
+      cx.phase = c2.phase;
+      cx.dead = c2.dead;
+    } else {
+      const int srow = seg_s[(warp & 3) * 32 + lane];
+      uint4* Mimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.M) + ibase * C * C);
+      drain_am(cx, reinterpret_cast<float*>(sm + OFF_T), Mimg, [&](int rw, int col, float (&va)[16], float (&vm)[16]) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const bool keep = mine && seg_s[row] == seg_s[col + i];
-          va[i] = keep ? va[i] : 0.f;
-          vm[i] = keep ? vm[i] : 0.f;
+          const bool same = srow == seg_s[col + i];
+          va[i] = (same && col + i < rw) ? va[i] : 0.f;
+          vm[i] = (same && col + i <= rw) ? vm[i] : 0.f;
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) umma::st_keep4(Ag4 + p4v(row, col + 4 * i), make_float4(va[4 * i], va[4 * i + 1], va[4 * i + 2], va[4 * i + 3]));
-        Mimg[(col / 8) * 128 + row] = umma::pack8p(vm);
-        Mimg[(col / 8 + 1) * 128 + row] = umma::pack8p(vm + 8);
-      }
-      umma::tc_fence_before();
-    };
-#pragma unroll 1
-    for (int lv = 0; lv < 3; ++lv) {                       // (the images of level 0 were built above)
-      const uint32_t tcol = 0;                             // the drain of level lv is over before level lv + 1 is issued
-      umma::pre_issue_sync();
-      umma::issue<128, false, false>(cx, KR, KR, K, tcol, false);          // A: KR KR^T
-      umma::issue<128, false, false>(cx, QK, KR, K, tcol + 128, false);    // M: QK KR^T
-      umma::commit_wait(cx);
-      DN_MARK(3 + lv);
-      if (lv < 2) build(lv + 1);
-      drain_level(lv);
+      });
+      __syncthreads();
     }
-    __syncthreads();
-
-    DN_MARK(6);
-    if (!tm_cache) diag_pass();
-    }
-    }
-
-    DN_MARK(7);
-    // The inverse below works out of shared memory for a while: ask for this item's rows of v and w (read
-    // right after it, for the first time) to be brought into L2 meanwhile.
-    if (tid < r.rows_valid) {
-      const size_t tok = (size_t)b * g.L + t0 + tid;
-      const uint32_t qe = (uint32_t)dt_size(qdt), ge = (uint32_t)dt_size(gdt);
-      umma::prefetch_l2(reinterpret_cast<const uint8_t*>(a.v) + (tok * g.Hv * g.V + (size_t)h * VW) * qe, VW * qe);
-      if (wC == g.V && g.wH == g.Hv)
-        umma::prefetch_l2(reinterpret_cast<const uint8_t*>(a.w) + (tok * g.Hv * g.V + (size_t)h * VW) * ge, VW * ge);
-    }
-    // ---- T = (I + A)^-1 in fp32: substitution on the diagonal blocks, then block merges
-    {
-      float4* As4 = reinterpret_cast<float4*>(As);
-      float4* Ts4 = reinterpret_cast<float4*>(Ts);
-#pragma unroll 4
-      for (int e = tid; e < 32 * C; e += NT) {
-        const int q = e >> 7, i = e & 127;
-        As4[i * (AP / 4) + q] = umma::ld_keep4(Ag4 + e);
-      }
-      for (int e = tid; e < C * AP / 4; e += NT) Ts4[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    __syncthreads();
-    if (tid < C) {
-      const int j = tid, blk0 = j & ~15, jl = j & 15;
-      float col[16];
-#pragma unroll
-      for (int m = 0; m < 16; ++m) col[m] = m == jl ? 1.f : 0.f;
-#pragma unroll
-      for (int i = 1; i < 16; ++i) {
-        float av[16];
-#pragma unroll
-        for (int u = 0; u < (i + 3) / 4; ++u)
-          *reinterpret_cast<float4*>(av + 4 * u) = *reinterpret_cast<const float4*>(As + (blk0 + i) * AP + blk0 + 4 * u);
-        float s = 0.f;
-#pragma unroll
-        for (int m = 0; m < i; ++m) s = fmaf(av[m], col[m], s);
-        if (i > jl) col[i] = -s;
-      }
-#pragma unroll
-      for (int i = 0; i < 16; ++i) Ts[(blk0 + i) * AP + j] = col[i];
-    }
-    __syncthreads();
-    DN_MARK(8);
-    merge_level<16>(As, Ts, Tm);
-    merge_level<32>(As, Ts, Tm);
-    merge_level<64>(As, Ts, Tm);
-    DN_MARK(9);
-    // ---- W = T X, U = T Y on the tensor cores
-    {
-      // T as K-major A: piece (p = j/8, x = i).  The same image is the residual the backward reads
-      // (bf16, in the first half of T's fp32-sized slot): it rounds T to bf16 there anyway.
-      uint4* Tg = a.res.T ? reinterpret_cast<uint4*>(a.res.T + ibase * C * C) : nullptr;
-      for (int e = tid; e < IMG; e += NT) {
-        const int p = e >> 7, x = e & 127;
-        const uint4 v = umma::ld8_f32(Ts + x * AP + 8 * p);
-        TI[e] = v;
-        if (Tg) Tg[e] = v;
-      }
-    }
-    {                                                           // Y = w*v as MN-major B
-      const int x = myrow, t = t0 + x;
-      const bool live = t < g.L;
-      const size_t tokr = (size_t)b * g.L + (live ? t : t0);
-#pragma unroll 4
-      for (int it = 0; it < VW / 32; ++it) {
-        const int p = it * 4 + lgrp;
-        const int col0 = h * VW + 8 * p, hv = col0 / g.V, cv = col0 - hv * g.V;
-        float vv[8], ww[8], f[8];
-        load8(a.v, tokr * g.Hv * g.V + col0, qdt, vv);
-        if (wC == 1) {
-          const float w1 = ldf_ro(a.w, tokr * g.wH + g.w_head(hv), gdt);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) ww[i] = w1;
-        } else {
-          load8(a.w, (tokr * g.wH + g.w_head(hv)) * wC + cv, gdt, ww);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float wa = fuse ? 1.f / (1.f + expf(-ww[i])) : ww[i];
-          f[i] = live ? wa * vv[i] : 0.f;
-        }
-        YI[p * 128 + x] = umma::pack8(f);
-      }
-    }
-    umma::pre_issue_sync();
-    umma::issue<128, false, true>(cx, TI, XI, C, 0, false);
-    umma::issue<VW, false, true>(cx, TI, YI, C, 128, false);
-    umma::commit_wait(cx);
-    DN_MARK(10);
-    umma::drain<NT, 128>(cx, 0, [&](int row, int col, const float (&v)[16]) {
-      Wimg[(col / 8) * 128 + row] = umma::pack8p(v);
-      Wimg[(col / 8 + 1) * 128 + row] = umma::pack8p(v + 8);
-    });
-    umma::drain<NT, VW>(cx, 128, [&](int row, int col, const float (&v)[16]) {
-      Uimg[(col / 8) * 128 + row] = umma::pack8p(v);
-      Uimg[(col / 8 + 1) * 128 + row] = umma::pack8p(v + 8);
-    });
-    __syncthreads();
-#ifdef DN_PHASE_TIMING
-    DN_MARK(11);
-    if (blockIdx.x == 0 && tid == 0 && e_item == 0) {
-      for (int i = 1; i < 12; ++i) printf("fwd mark %d -> %d: %lld\n", i - 1, i, g_phase_marks[i] - g_phase_marks[i - 1]);
-      printf("fwd item total %lld\n", g_phase_marks[11] - g_phase_marks[0]);
-      printf("fwd D: stage0 %lld compute0(warp0) %lld wait0 %lld stage1 %lld compute1 %lld wait1 %lld\n", g_phase_marks[20] - g_phase_marks[6],
-             g_phase_marks[21] - g_phase_marks[20], g_phase_marks[22] - g_phase_marks[21], g_phase_marks[23] - g_phase_marks[22],
-             g_phase_marks[24] - g_phase_marks[23], g_phase_marks[25] - g_phase_marks[24]);
-    }
-#endif
+    inverse_and_products<VW>(cx, sm, a, h, b, t0, ibase, e_item + gridDim.x, qdt, gdt, wC, fuse);
   }
-  umma::tc_fence_before();
-  __syncthreads();
-  if (warp == 0) umma::tmem_dealloc(tmem_base, 512);
+  teardown(tbase);
 }
 
 }  // namespace
 
 bool prepass_fwd_tc_eligible(const Geo& g) { return g.img; }
 
-size_t prepass_fwd_tc_scratch_per_cta() { return (size_t)C * C; }
-
 int launch_prepass_fwd_tc(const Geo& g, const void* q, const void* k, const void* v, const void* gg,
                           const void* b, const void* w, const int32_t* seg, const dn_residuals& res,
-                          float* scratch, size_t scratch_floats, cudaStream_t st, int c_begin, int c_end) {
-  PrepassFwdArgs a;
+                          cudaStream_t st, int c_begin, int c_end) {
+  PrepassFwdArgs a{};
   a.g = g; a.q = q; a.k = k; a.v = v; a.gg = gg; a.b = b; a.w = w; a.seg = seg; a.res = res;
   a.c_begin = c_begin; a.c_end = c_end < 0 ? g.NC : c_end;
   a.items = g.B * g.H * (a.c_end - a.c_begin);
   if (a.items <= 0) return DN_OK;
-  a.scratch_per_cta = prepass_fwd_tc_scratch_per_cta();
-  a.smem_tile_off = 0;
-  const int grid = a.items < sm_count() ? a.items : sm_count();
-  if (scratch_floats < (size_t)grid * a.scratch_per_cta) return DN_ERR_SCRATCH_TOO_SMALL;
-  a.scratch = scratch;
+  // k_hat and q_hat are rounded to bf16 ahead of their use here, which the fused prologue does not do
+  const bool scalar = g.gC == 1 && g.bC == 1 && g.qkv_dt == DN_BF16 && !(g.flags & DN_FUSE_PROLOGUE);
+  const int grid = a.items < 2 * sm_count() ? a.items : 2 * sm_count();
   int* err = device_error_ptr();
   auto go = [&](auto kernel) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     kernel<<<grid, NT, SMEM_BYTES, st>>>(a, err);
   };
-  const int mode = input_mode(g);
-  if (g.Vw == 256) {
-    if (mode == 0) go(prepass_fwd_tc_kernel<256, 0>); else if (mode == 1) go(prepass_fwd_tc_kernel<256, 1>); else if (mode == 3) go(prepass_fwd_tc_kernel<256, 3>); else if (mode == 4) go(prepass_fwd_tc_kernel<256, 4>); else go(prepass_fwd_tc_kernel<256, 2>);
-  } else {
-    if (mode == 0) go(prepass_fwd_tc_kernel<128, 0>); else if (mode == 1) go(prepass_fwd_tc_kernel<128, 1>); else if (mode == 3) go(prepass_fwd_tc_kernel<128, 3>); else if (mode == 4) go(prepass_fwd_tc_kernel<128, 4>); else go(prepass_fwd_tc_kernel<128, 2>);
-  }
+  auto pick = [&](auto vw) {
+    constexpr int VW = decltype(vw)::value;
+    if (scalar) { go(prepass_fwd_scalar_kernel<VW>); return; }
+    switch (input_mode(g)) {
+      case 0: go(prepass_fwd_channel_kernel<VW, 0>); break;
+      case 1: go(prepass_fwd_channel_kernel<VW, 1>); break;
+      case 4: go(prepass_fwd_channel_kernel<VW, 4>); break;
+      default: go(prepass_fwd_channel_kernel<VW, 2>); break;
+    }
+  };
+  if (g.Vw == 256) pick(std::integral_constant<int, 256>{});
+  else pick(std::integral_constant<int, 128>{});
   return launch_status();
 }
 

@@ -291,25 +291,53 @@ __device__ __forceinline__ void pre_issue_sync() {
   tc_fence_after();
 }
 
-// Issue (one thread) the MMAs of D[128 x N] (+)= A[128 x Kc] B[N x Kc]^T on staged operands.
+// Issue (one thread) the MMAs of D[128 x N] (+)= A[128 x Kc] B[N x Kc]^T on staged operands whose panels lie
+// a_pitch / b_pitch bytes apart (panels written by threads that hold several pieces of one row are kept 32 bytes
+// further apart than they are long: the pieces then fall into different banks).
+template <int N, bool A_MN, bool B_MN>
+__device__ __forceinline__ void issue_pitched(const Ctx& cx, const void* sA, uint32_t a_pitch, const void* sB, uint32_t b_pitch, int Kc,
+                                              uint32_t tmem_col, bool accumulate) {
+  if (threadIdx.x != 0 || cx.dead) return;
+  constexpr uint32_t idesc = instr_desc(N, A_MN ? 1 : 0, B_MN ? 1 : 0);
+  uint64_t ad = smem_desc(smem_u32(sA), A_MN ? 128u : a_pitch, A_MN ? a_pitch : 128u);
+  uint64_t bd = smem_desc(smem_u32(sB), B_MN ? 128u : b_pitch, B_MN ? b_pitch : 128u);
+  const uint32_t a_step = (A_MN ? 256u : 2u * a_pitch) >> 4, b_step = (B_MN ? 256u : 2u * b_pitch) >> 4;
+#pragma unroll 4
+  for (int ks = 0; ks < Kc / 16; ++ks) {
+    mma_bf16(cx.tmem + tmem_col, ad, bd, idesc, (accumulate || ks > 0) ? 1u : 0u);
+    ad += a_step;
+    bd += b_step;
+  }
+}
+// the same on images without padding
 template <int N, bool A_MN, bool B_MN>
 __device__ __forceinline__ void issue(const Ctx& cx, const void* sA, const void* sB, int Kc, uint32_t tmem_col,
                                       bool accumulate) {
-  if (threadIdx.x != 0 || cx.dead) return;
-  const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
-  constexpr uint32_t idesc = instr_desc(N, A_MN ? 1 : 0, B_MN ? 1 : 0);
-  const uint32_t a_lbo = A_MN ? 128u : 128u * 16u, a_sbo = A_MN ? (uint32_t)Kc * 16u : 128u;
-  const uint32_t b_lbo = B_MN ? 128u : (uint32_t)N * 16u, b_sbo = B_MN ? (uint32_t)Kc * 16u : 128u;
-  const uint32_t a_step = A_MN ? 256u : 2u * 128u * 16u, b_step = B_MN ? 256u : 2u * (uint32_t)N * 16u;
-  for (int ks = 0; ks < Kc / 16; ++ks)
-    mma_bf16(cx.tmem + tmem_col, smem_desc(a0 + ks * a_step, a_lbo, a_sbo), smem_desc(b0 + ks * b_step, b_lbo, b_sbo),
-             idesc, (accumulate || ks > 0) ? 1u : 0u);
+  issue_pitched<N, A_MN, B_MN>(cx, sA, A_MN ? (uint32_t)Kc * 16u : 2048u, sB, B_MN ? (uint32_t)Kc * 16u : (uint32_t)N * 16u, Kc, tmem_col,
+                               accumulate);
 }
 
+// Make every thread wait, boundedly, for a commit that has been issued already.
+__device__ __forceinline__ void commit_wait_only(Ctx& cx) {
+  if (!cx.dead && !mbar_wait(cx.bar, cx.phase)) {
+    cx.dead = true;
+    report_timeout(cx.err);
+  }
+  cx.phase ^= 1u;
+  tc_fence_after();
+}
 // Commit everything issued so far (one thread) and make every thread wait for it, boundedly.
 __device__ __forceinline__ void commit_wait(Ctx& cx) {
   if (threadIdx.x == 0 && !cx.dead) mma_commit(cx.bar);
-  if (!cx.dead && !mbar_wait(cx.bar, cx.phase)) {
+  commit_wait_only(cx);
+}
+
+// The same with one warp polling and the others parked at the CTA's barrier: every polling warp takes issue slots
+// from whatever else runs on the SM.  Also a barrier among the CTA's threads.
+__device__ __forceinline__ void commit_wait_cta(Ctx& cx) {
+  bool bad = false;
+  if (threadIdx.x < 32 && !cx.dead) bad = !mbar_wait(cx.bar, cx.phase);
+  if (__syncthreads_or(bad)) {
     cx.dead = true;
     report_timeout(cx.err);
   }
