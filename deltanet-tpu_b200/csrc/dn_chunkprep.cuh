@@ -67,6 +67,24 @@ __device__ __forceinline__ void zero8(float (&x)[8]) {
   for (int i = 0; i < 8; ++i) x[i] = 0.f;
 }
 
+// Eight consecutive elements as loaded (bf16: the first vector only); converted where they are used, so that a load
+// can be in flight across a barrier without its converted values taking registers.
+struct Raw8 { uint4 a, b; };
+__device__ __forceinline__ Raw8 ldraw(const uint8_t* row, int p, int dt) {
+  Raw8 r;
+  r.b = make_uint4(0, 0, 0, 0);
+  if (dt == DN_BF16) r.a = __ldg(reinterpret_cast<const uint4*>(row) + p);
+  else { r.a = __ldg(reinterpret_cast<const uint4*>(row) + 2 * p); r.b = __ldg(reinterpret_cast<const uint4*>(row) + 2 * p + 1); }
+  return r;
+}
+__device__ __forceinline__ void cvraw(const Raw8& r, int dt, float (&x)[8]) {
+  if (dt == DN_BF16) umma::unpack8(r.a, x);
+  else {
+    x[0] = __uint_as_float(r.a.x); x[1] = __uint_as_float(r.a.y); x[2] = __uint_as_float(r.a.z); x[3] = __uint_as_float(r.a.w);
+    x[4] = __uint_as_float(r.b.x); x[5] = __uint_as_float(r.b.y); x[6] = __uint_as_float(r.b.z); x[7] = __uint_as_float(r.b.w);
+  }
+}
+
 // raw q / k piece (channels 8p..8p+7 of chunk row x), zero on rows past the end.  The load itself
 // is unconditional (a row past the end reads row 0 and is zeroed afterwards), so that a caller's
 // loads can all be in flight together.

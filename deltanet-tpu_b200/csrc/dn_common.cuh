@@ -102,6 +102,13 @@ __host__ __device__ __forceinline__ float* dlend_part(const Geo& g, float* dH) {
   return dH + (size_t)g.B * g.H * g.NC * g.K * g.Vw / 2;
 }
 
+// T's slot holds a bf16 image in its first half; the first word of the second half tells the backward that the decay of
+// this tile is strong (channel-wise decay only)
+__host__ __device__ __forceinline__ int* strong_flag_ptr(const dn_residuals& res, size_t tile) {
+  return reinterpret_cast<int*>(res.T + tile * 128 * 128 + 128 * 64);
+}
+__device__ __forceinline__ bool strong_flag(const dn_residuals& res, size_t tile) { return *strong_flag_ptr(res, tile) != 0; }
+
 // element index of (row, col) in a residual tile of 128 rows (image layout) or `ncols` columns (row-major)
 __host__ __device__ __forceinline__ size_t rix(bool img, int row, int col, int ncols) {
   return img ? ((size_t)((col >> 3) * 128 + row) << 3) + (col & 7) : (size_t)row * ncols + col;

@@ -98,6 +98,9 @@ int launch_state_bwd(const StateArgs& a, cudaStream_t st);
 int launch_prepass_bwd(PrepassBwdArgs& a, size_t scratch_floats, cudaStream_t st);
 int launch_prepass_bwd_tc(PrepassBwdArgs& a, size_t scratch_floats, cudaStream_t st);
 bool prepass_bwd_tc_eligible(const Geo& g);
+// the kernel for all tiles but those marked for strong decay, and whether none can be (scalar gates)
+int launch_prepass_bwd_fast(const PrepassBwdArgs& a, cudaStream_t st);
+bool prepass_bwd_scalar_route(const Geo& g);
 size_t prepass_bwd_tc_scratch_per_cta(const Geo& g);
 int launch_canonical_segments(const int32_t* raw, const int32_t* first_is_new, int32_t* out,
                               int B, int L, cudaStream_t st);

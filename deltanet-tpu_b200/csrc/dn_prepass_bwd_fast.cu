@@ -1,0 +1,1013 @@
+// Chunk-parallel backward on the tcgen05 tensor cores, single-Gram routes (bf16 precision, 128-row tiles): the adjoint
+// of the state step's value-width contractions and of the prepass (reference: src/deltanet_tpu/gdn2.py:243-493,
+// 750-762) and of the fused prologue (558-575).  Tiles whose channel-wise decay is strong (marked by the forward
+// prepass in the unused half of T's slot) are left to dn_prepass_bwd_tc.cu, launched behind this kernel.
+//
+// With f_i = e^{Lam_i - mid} (mid: the document's midpoint; f = 1 and a decay f_ij applied per entry when the decay is one
+// scalar per token), dA = -(dX W^T + dY U^T), dM = dO V_new^T (masked):
+//     T1 = dA (k / f)   + [first doc] e^{Lam} / f  dX         d beta = f T1
+//     T2 = dM (k / f)   + [first doc] e^{Lam} / f  dqe        d q    = f T2   (+ dM_ii k_i)
+//     T3 = dA^T (beta f) + dM^T (q f) + [last doc] e^{Lam_end - Lam} f  dke       d k    = T3 / f (+ dM_ii q_i + d beta b)
+// Nothing of this leaves the SM: dqe, dke and dX stay in the tensor-memory columns where their products put them, are
+// scaled there (e^{Lam} / f and e^{Lam_end - Lam} f are constants of the channel), and T1, T2, T3 accumulate on
+// top; dA and dM go from tensor memory into their operand images.  The earlier form carried all eight 64 KB fp32
+// matrices through an L2 scratch and was bound by that and by the L1 data stage: 16-byte accesses with a
+// row per lane cost 32 lookups each.  Here rows of the operator's tensors are always read and written with the pieces of a
+// row in neighbouring lanes, staged through shared memory where the arithmetic wants a row per lane.
+// The decay gradient needs one array only: with dLam = beta dbeta + q dq - k dk (without the dM_ii terms),
+//     dg_t = sum_{i >= t, same doc} dLam_i + [last doc] (dLam_end + sum_i ke_i dke_i) .
+//
+// 512 threads, one CTA per SM, six shared-memory slots that operand images pass through, 512 tensor-memory columns:
+// dqe / T2 | dke / T3 | dX / T1 | temporary.
+#include <type_traits>
+
+#include "dn_chunkprep.cuh"
+#include "dn_kernels.cuh"
+
+namespace dn {
+namespace {
+
+using namespace prep;
+constexpr int NT = 512;
+constexpr int PP = 130;                               // uint4 per panel of images written from rows (bank spread)
+constexpr uint32_t PB = PP * 16;
+constexpr int SLOT = 16 * PB;
+constexpr int LPF = 132;                              // row pitch (floats) of Lambda, which takes slots 0 and 1 after the products
+constexpr int OFF_GI = C * LPF * 4;                   // then: two sets of three 128 x 32 images (k / f, q f, beta f), and later
+constexpr int OFF_RK = OFF_GI, OFF_RQ = OFF_RK + SLOT, OFF_RB = OFF_RQ + SLOT;      // the raw k, q and b
+constexpr int OFF_MISC = OFF_RB + 2 * SLOT;           // partial sums
+constexpr int MISC_FLOATS = 512 + 256 + 4 * 512 + 512;
+constexpr int SMEM_BYTES = OFF_MISC + MISC_FLOATS * 4;
+constexpr uint32_t T_Q = 0, T_K = 128, T_B = 256, T_TMP = 384;
+constexpr uint32_t IMGB = 32768;
+static_assert(OFF_GI + 2 * 3 * 4 * (int)PB <= 4 * SLOT && OFF_MISC >= 6 * SLOT, "regions");
+static_assert(SMEM_BYTES + 6 * 1024 <= 227 * 1024, "with the static arrays");
+
+__device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 1.f + umma::ex2_fast(-x * DN_LOG2E)); }
+
+struct Slots {
+  uint8_t* sm;
+  uint64_t* bars;          // one per slot
+  uint32_t phases;
+  int* err;
+  __device__ __forceinline__ uint4* at(int s) const { return reinterpret_cast<uint4*>(sm + s * SLOT); }
+  // one contiguous 32 KB operand image; ordinary accesses to the slot must lie before a barrier
+  __device__ __forceinline__ void load(int s, const __nv_bfloat16* src) {
+    if (threadIdx.x == 0) {
+      umma::fence_async_smem();
+      umma::mbar_expect_tx(bars + s, IMGB);
+      umma::bulk_load(at(s), src, IMGB, bars + s);
+    }
+  }
+  __device__ __forceinline__ void wait(int s) {
+    if (!umma::mbar_wait(bars + s, (phases >> s) & 1u)) umma::report_timeout(err);
+    phases ^= 1u << s;
+  }
+};
+
+// this thread's row (32 (warp & 3) + lane) and 32 columns (32 (warp >> 2)) of a 128-column block of tensor memory
+__device__ __forceinline__ void ld32(const umma::Ctx& cx, uint32_t addr, float (&v)[32]) {
+  if (!cx.dead) {
+    umma::tmem_ld32_nowait(addr, v);
+    umma::tmem_wait_ld();
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = 0.f;
+  }
+}
+__device__ __forceinline__ void st32(uint32_t addr, const float (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) umma::tmem_st8(addr + 8 * j, *reinterpret_cast<const float(*)[8]>(v + 8 * j));
+}
+__device__ __forceinline__ void image32(uint4* img, int pitch, int row, int group, const float (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) img[(4 * group + j) * pitch + row] = umma::pack8p(v + 8 * j);
+}
+// One step of summing 32 values per lane over the warp's lanes, all at once: a lane hands over the half it drops; after
+// the steps 16, 8, 4, 2, 1 lane c holds the sum of value c.
+template <int O>
+__device__ __forceinline__ void fold(float (&v)[32], int lane) {
+  const bool up = lane & O;
+#pragma unroll
+  for (int i = 0; i < O; ++i) {
+    const float got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + O], O);
+    v[i] = (up ? v[i + O] : v[i]) + got;
+  }
+}
+__device__ __forceinline__ void commit(const umma::Ctx& cx) {
+  if (threadIdx.x == 0 && !cx.dead) umma::mma_commit(cx.bar);
+}
+// eight elements of a row of one of the operator's tensors, piece p
+__device__ __forceinline__ void ldrow8(const uint8_t* row, int p, int dt, float (&x)[8]) { load8(row, 8 * p, dt, x); }
+__device__ __forceinline__ void strow8(void* base, size_t off, int dt, const float (&v)[8]) {
+  if (dt == DN_BF16) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(base) + off) = umma::pack8(v);
+  else {
+    float4* d = reinterpret_cast<float4*>(reinterpret_cast<float*>(base) + off);
+    d[0] = make_float4(v[0], v[1], v[2], v[3]);
+    d[1] = make_float4(v[4], v[5], v[6], v[7]);
+  }
+}
+
+// dO of one 128-column half (or less) into a padded image, rows past the end and columns past `width` as zeros
+__device__ __forceinline__ void stage_dO(uint4* dst, const void* d_out, size_t off, size_t pitch, int rows, int pieces, int dt) {
+  const int x = threadIdx.x >> 2, pp = threadIdx.x & 3;
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int p = it * 4 + pp;
+    if (x < rows && p < pieces) {
+      if (dt == DN_BF16) umma::cp_async16(dst + p * PP + x, reinterpret_cast<const __nv_bfloat16*>(d_out) + off + (size_t)x * pitch + 8 * p);
+      else dst[p * PP + x] = umma::ld8_f32_ro(reinterpret_cast<const float*>(d_out) + off + (size_t)x * pitch + 8 * p);
+    } else dst[p * PP + x] = make_uint4(0, 0, 0, 0);
+  }
+  umma::cp_async_commit();
+}
+
+template <int VW, int MODE, bool SC>
+__global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_constant__ PrepassBwdArgs a) {
+  using CF = InCfg<MODE>;
+  constexpr int NH = VW / 128;
+  extern __shared__ __align__(128) uint8_t sm[];
+  __shared__ uint64_t mma_bar, slot_bar[6], gbar[2];
+  __shared__ uint32_t tmem_base;
+  __shared__ int seg_s[C];
+  __shared__ int cut_s[8];
+  __shared__ uint8_t ds_s[C], de_s[C];                  // first / last row of each row's document inside the tile
+  __shared__ float rq_s[C], rk_s[C], dmi_s[C], dlend_s[C];
+  __shared__ float lam_s[C], bet_s[C];                  // scalar gates
+  const Geo& g = a.g;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int quarter = warp & 3, group = warp >> 2, row = quarter * 32 + lane;     // tensor-memory mapping
+  const int rx = tid >> 2, rp = tid & 3;                                           // row mapping: row, piece within four
+  float* MISC = reinterpret_cast<float*>(sm + OFF_MISC);
+  float* TOT = MISC;                                    // 4 x 128: the decay scan
+  float* EDGE = MISC + 512;                             // e^{mid} of the first document | e^{Lam_end - mid} of the last, per channel
+  float* SUM = MISC + 768;                              // 4 x 512: sums over channel groups / row quarters
+  float* PS = SUM + 2048;                               // 4 x 128: sum_i ke_i dke_i per row quarter
+  float* LAM = reinterpret_cast<float*>(sm);            // cumulative decay in units of log 2, later its cotangent
+  if (tid == 0) {
+    umma::mbar_init(&mma_bar, 1);
+    for (int i = 0; i < 6; ++i) umma::mbar_init(&slot_bar[i], 1);
+    umma::mbar_init(&gbar[0], 1);
+    umma::mbar_init(&gbar[1], 1);
+    umma::fence_mbar_init();
+  }
+  if (warp == 0) umma::tmem_alloc(&tmem_base, 512);
+  umma::tc_fence_before();
+  __syncthreads();
+  umma::tc_fence_after();
+  umma::Ctx cx{tmem_base, &mma_bar, 0u, a.err, false};
+  Slots sl{sm, slot_bar, 0u, a.err};
+  uint32_t gph = 0u;
+  const uint32_t tb = cx.tmem + ((uint32_t)(quarter * 32) << 16) + group * 32;
+
+  const bool l2 = g.flags & DN_QK_L2NORM, trunc = g.flags & DN_TRUNC_DT_BF16;
+  const bool fuse = CF::fixed ? false : (g.flags & DN_FUSE_PROLOGUE) != 0, guard = CF::fixed ? false : (g.flags & DN_STABILITY_GUARD) != 0;
+  const int qdt = CF::fixed ? CF::qkv_dt : g.qkv_dt, gdt = CF::fixed ? DN_F32 : g.gate_dt;
+  const bool round_in = !fuse && qdt == DN_BF16;
+  const int kp = CF::fixed && !SC ? 16 : g.K / 8, gC = SC ? 1 : (CF::fixed ? K : g.gC), bC = SC ? 1 : (CF::fixed ? (CF::scalar_bw ? 1 : K) : g.bC);
+  const int wC = CF::fixed && !SC ? (CF::scalar_bw ? 1 : g.V) : g.wC;
+  const uint32_t qes = qdt == DN_BF16 ? 2 : 4, ges = gdt == DN_BF16 ? 2 : 4;
+  const int vr = g.G * g.V;                             // value columns that exist
+
+  for (int e_item = blockIdx.x; e_item < a.items; e_item += gridDim.x) {
+    const int bh = e_item % (g.B * g.H), c_idx = a.c_begin + e_item / (g.B * g.H);
+    const int h = bh % g.H, b = bh / g.H, t0 = c_idx * C;
+    const size_t ibase = (size_t)bh * g.NC + c_idx;
+    if (!SC && strong_flag(a.res, ibase)) continue;     // uniform over the CTA
+    const int rows = g.L - t0 < C ? g.L - t0 : C;
+    const size_t tok0 = (size_t)b * g.L + t0;
+    const __nv_bfloat16* Wg = reinterpret_cast<const __nv_bfloat16*>(a.res.W) + ibase * C * K;
+    const __nv_bfloat16* Ug = reinterpret_cast<const __nv_bfloat16*>(a.res.U) + ibase * C * VW;
+    const __nv_bfloat16* Sg = states_img(g, a.res.states) + ibase * K * VW;
+    const __nv_bfloat16* dHg = reinterpret_cast<const __nv_bfloat16*>(a.dH) + ibase * K * VW;
+    const __nv_bfloat16* dVg = reinterpret_cast<const __nv_bfloat16*>(a.dV) + ibase * C * VW;
+    const __nv_bfloat16* Tg = reinterpret_cast<const __nv_bfloat16*>(a.res.T + ibase * C * C);
+    const size_t dO_off = tok0 * g.Hv * g.V + (size_t)h * vr, dO_pitch = (size_t)g.Hv * g.V;
+    constexpr int HN = C * 128;                         // elements of one half's image
+
+    // ---- products over the value width
+    sl.load(0, Wg);
+    sl.load(1, Sg);
+    sl.load(2, Ug);
+    if (NH == 1) {
+      sl.load(3, dVg);
+      sl.load(4, dHg);
+      stage_dO(sl.at(5), a.d_out, dO_off, dO_pitch, rows, vr / 8, qdt);
+    } else {
+      sl.load(3, Sg + HN);
+      sl.load(4, Ug + HN);
+      stage_dO(sl.at(5), a.d_out, dO_off, dO_pitch, rows, 16, qdt);
+    }
+    bool is_new, all_same;
+    chunk_flags(a.seg, g, b, c_idx, is_new, all_same);
+    if (tid < C) {
+      const int sg = seg_at(a.seg, b, t0 + tid, g.L);
+      seg_s[tid] = sg;
+      // dLambda_end = [one document] e^{Lambda_end} sum_v dH S (gdn2.py:759-762) from the reverse chain's per-slice sums
+      float acc = 0.f;
+      const float* part = dlend_part(g, const_cast<float*>(a.dH)) + ibase * (VW / 32) * K + tid;
+      for (int s2 = 0; s2 < VW / 32; ++s2) acc += __ldg(part + s2 * K);
+      dlend_s[tid] = all_same ? acc * expf(fminf(__ldg(a.res.lam_end + ibase * K + tid), 0.f)) : 0.f;
+      if (SC) {                                         // decay and erase gate: one row per thread, document-restarting scan
+        const int sp = tid ? seg_at(a.seg, b, t0 + tid - 1, g.L) : sg;
+        float gv = 0.f, bv = 0.f;
+        if (tid < rows) {
+          gv = ldf_ro(a.gg, (tok0 + tid) * g.gH + g.gate_head(h, g.gH), g.gate_dt);
+          bv = ldf_ro(a.b, (tok0 + tid) * g.bH + g.gate_head(h, g.bH), g.gate_dt);
+          gv = gv <= 0.f ? gv : 0.f;
+          if (guard) { bv = fmaxf(bv, 0.f); gv = fminf(gv, -1e-6f); }
+        }
+        bool cut = sg != sp;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const float up = __shfl_up_sync(0xffffffffu, gv, o);
+          const bool uc = __shfl_up_sync(0xffffffffu, (int)cut, o);
+          if (lane >= o) { if (!cut) gv += up; cut |= uc; }
+        }
+        if (lane == 31) { SUM[warp] = gv; cut_s[warp] = cut; }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        float carry = 0.f;
+        for (int w2 = warp - 1; w2 >= 0; --w2) { carry += SUM[w2]; if (cut_s[w2]) break; }
+        lam_s[tid] = gv + (cut ? 0.f : carry);
+        bet_s[tid] = bv;
+      }
+    }
+    // V_new = U - W S, in the place of U
+    auto vnew = [&](int slot, uint32_t col) {
+      float v[32];
+      ld32(cx, tb + col, v);
+      uint4* img = sl.at(slot);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float u[8];
+        umma::unpack8(img[(4 * group + j) * 128 + row], u);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) u[i] -= v[8 * j + i];
+        img[(4 * group + j) * 128 + row] = umma::pack8(u);
+      }
+    };
+    auto drain_dM = [&](int slot) {                     // masked (scalar gates: decayed) dM as an operand image; its diagonal apart
+      float v[32];
+      ld32(cx, tb + T_TMP, v);
+      const int sr = seg_s[row];
+      const float lr = SC ? lam_s[row] * DN_LOG2E : 0.f;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const int j = group * 32 + i;
+        if (j == row) dmi_s[row] = v[i];
+        float f = 1.f;
+        if (SC) f = umma::ex2_fast(fminf(lr - lam_s[j] * DN_LOG2E, 0.f));
+        v[i] = (j < row && sr == seg_s[j]) ? v[i] * f : 0.f;
+      }
+      image32(sl.at(slot), 128, row, group, v);
+    };
+    auto drain_neg = [&](int slot, uint32_t col) {
+      float v[32];
+      ld32(cx, tb + col, v);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = -v[i];
+      image32(sl.at(slot), 128, row, group, v);
+    };
+    sl.wait(0);
+    sl.wait(1);
+    sl.wait(2);
+    if constexpr (NH == 1) {
+      umma::pre_issue_sync();
+      umma::issue<128, false, true>(cx, sl.at(0), sl.at(1), K, T_TMP, false);                      // W S
+      commit(cx);
+      umma::cp_async_wait<0>();                         // dO
+      umma::commit_wait_cta(cx);
+      sl.load(0, Tg);
+      vnew(2, T_TMP);
+      sl.wait(3);
+      sl.wait(4);
+      umma::pre_issue_sync();
+      umma::issue_pitched<128, false, false>(cx, sl.at(5), PB, sl.at(2), 2048, 128, T_TMP, false); // dM  = dO V_new^T
+      umma::issue_pitched<128, false, false>(cx, sl.at(5), PB, sl.at(1), 2048, 128, T_Q, false);   // dqe = dO S^T
+      commit(cx);
+      umma::commit_wait_cta(cx);
+      umma::issue<128, false, false>(cx, sl.at(3), sl.at(1), 128, T_B, false);                     // -dW = dV S^T
+      umma::issue<128, false, false>(cx, sl.at(2), sl.at(4), 128, T_K, false);                     // dke = V_new dH^T
+      commit(cx);
+      drain_dM(5);
+      umma::commit_wait_cta(cx);
+      sl.load(2, Wg);
+      sl.load(4, Ug);
+      drain_neg(1, T_B);                                // dW
+      sl.wait(0);
+      umma::pre_issue_sync();
+      umma::issue<128, true, true>(cx, sl.at(0), sl.at(1), C, T_B, false);                         // dX = T^T dW
+      umma::issue<128, true, true>(cx, sl.at(0), sl.at(3), C, T_TMP, false);                       // dY = T^T dV
+      commit(cx);
+      umma::commit_wait_cta(cx);
+    } else {
+      sl.wait(3);
+      sl.wait(4);
+      umma::pre_issue_sync();
+      umma::issue<128, false, true>(cx, sl.at(0), sl.at(1), K, T_TMP, false);                      // W S, both halves
+      umma::issue<128, false, true>(cx, sl.at(0), sl.at(3), K, T_B, false);
+      commit(cx);
+      umma::cp_async_wait<0>();
+      umma::commit_wait_cta(cx);
+      sl.load(0, dVg);
+      vnew(2, T_TMP);
+      vnew(4, T_B);
+      umma::pre_issue_sync();
+      umma::issue_pitched<128, false, false>(cx, sl.at(5), PB, sl.at(2), 2048, 128, T_TMP, false); // dM, dqe: first half
+      umma::issue_pitched<128, false, false>(cx, sl.at(5), PB, sl.at(1), 2048, 128, T_Q, false);
+      commit(cx);
+      umma::commit_wait_cta(cx);
+      stage_dO(sl.at(5), a.d_out, dO_off + 128, dO_pitch, rows, 16, qdt);
+      sl.wait(0);
+      umma::issue<128, false, false>(cx, sl.at(0), sl.at(1), 128, T_B, false);                     // -dW: first half
+      commit(cx);
+      umma::cp_async_wait<0>();
+      umma::commit_wait_cta(cx);
+      sl.load(0, dVg + HN);
+      sl.load(1, dHg);
+      umma::pre_issue_sync();
+      umma::issue_pitched<128, false, false>(cx, sl.at(5), PB, sl.at(4), 2048, 128, T_TMP, true);  // second half
+      umma::issue_pitched<128, false, false>(cx, sl.at(5), PB, sl.at(3), 2048, 128, T_Q, true);
+      commit(cx);
+      umma::commit_wait_cta(cx);
+      sl.wait(0);
+      sl.wait(1);
+      umma::issue<128, false, false>(cx, sl.at(0), sl.at(3), 128, T_B, true);
+      umma::issue<128, false, false>(cx, sl.at(2), sl.at(1), 128, T_K, false);                     // dke: first half
+      commit(cx);
+      drain_dM(5);
+      umma::commit_wait_cta(cx);
+      sl.load(1, dHg + HN);                             // (slot 0 keeps the second half of dV)
+      sl.load(2, Tg);
+      drain_neg(3, T_B);                                // dW
+      sl.wait(1);
+      sl.wait(2);
+      umma::pre_issue_sync();
+      umma::issue<128, false, false>(cx, sl.at(4), sl.at(1), 128, T_K, true);                      // dke: second half
+      umma::issue<128, true, true>(cx, sl.at(2), sl.at(3), C, T_B, false);                         // dX = T^T dW
+      umma::issue<128, true, true>(cx, sl.at(2), sl.at(0), C, T_TMP, false);                       // dY: second half
+      commit(cx);
+      umma::commit_wait_cta(cx);
+    }
+    auto drain_dX = [&](int slot) {                     // as operand image; the accumulator itself stays for T1
+      float v[32];
+      ld32(cx, tb + T_B, v);
+      if (trunc) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = bf16r(v[i]);
+        st32(tb + T_B, v);
+        umma::tmem_wait_st();
+      }
+      image32(sl.at(slot), 128, row, group, v);
+    };
+    auto drain_dY = [&](int slot) {
+      float v[32];
+      ld32(cx, tb + T_TMP, v);
+      image32(sl.at(slot), PP, row, group, v);
+    };
+    // dv = dY w_act, dw = dY v (+ sigmoid adjoint; summed over a value head's columns when w is one scalar per head)
+    auto vphase = [&](int slot, int half) {
+      const uint4* img = sl.at(slot);
+      const bool live = rx < rows;
+      const size_t tok = tok0 + (live ? rx : 0);
+      const int steps_per_head = g.V / 32;
+      float sw = 0.f;
+#pragma unroll 2
+      for (int it = 0; it < 4; ++it) {
+        const int p = it * 4 + rp, col = half * 128 + 8 * p;
+        if (col - 8 * rp >= vr) break;                  // (uniform: value widths are multiples of 32)
+        const int hv = h * g.G + col / g.V, cv = col % g.V;
+        const size_t vo = (tok * g.Hv + hv) * g.V + cv;
+        float vv[8], ww[8], dy[8], dv8[8], dw8[8];
+        load8(a.v, vo, qdt, vv);
+        if (wC == 1) {
+          const float w1 = ldf_ro(a.w, tok * g.wH + g.w_head(hv), gdt);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) ww[i] = w1;
+        } else {
+          load8(a.w, (tok * g.wH + g.w_head(hv)) * wC + cv, gdt, ww);
+        }
+        umma::unpack8(img[p * PP + rx], dy);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          float wa = ww[i], dwv = dy[i] * vv[i];
+          if (fuse) { wa = sigmoid_fast(ww[i]); dwv *= wa * (1.f - wa); }
+          dv8[i] = dy[i] * wa;
+          dw8[i] = dwv;
+          sw += dwv;
+        }
+        if (live) {
+          strow8(a.dv, vo, qdt, dv8);
+          if (wC != 1) strow8(a.dw, (tok * g.Hv + hv) * wC + cv, a.dw_dt, dw8);
+        }
+        if (wC == 1 && (it + 1) % steps_per_head == 0) {
+          sw += __shfl_xor_sync(0xffffffffu, sw, 1);
+          sw += __shfl_xor_sync(0xffffffffu, sw, 2);
+          if (live && rp == 0) stf(a.dw, tok * g.Hv + hv, sw, a.dw_dt);
+          sw = 0.f;
+        }
+      }
+    };
+    if constexpr (NH == 1) {
+      drain_dX(0);
+      drain_dY(1);
+      sl.wait(2);
+      sl.wait(4);
+      umma::pre_issue_sync();
+      umma::issue<128, false, false>(cx, sl.at(0), sl.at(2), 128, T_TMP, false);                   // -dA = dX W^T + dY U^T
+      umma::issue_pitched<128, false, false>(cx, sl.at(1), PB, sl.at(4), 2048, 128, T_TMP, true);
+      commit(cx);
+      vphase(1, 0);
+      umma::commit_wait_cta(cx);
+    } else {
+      sl.load(0, dVg);
+      sl.load(1, Wg);
+      drain_dX(3);
+      drain_dY(4);
+      sl.wait(0);
+      umma::pre_issue_sync();
+      umma::issue<128, true, true>(cx, sl.at(2), sl.at(0), C, T_TMP, false);                       // dY: first half
+      commit(cx);
+      umma::commit_wait_cta(cx);
+      sl.load(0, Ug);
+      drain_dY(2);
+      sl.wait(0);
+      sl.wait(1);
+      umma::pre_issue_sync();
+      umma::issue<128, false, false>(cx, sl.at(3), sl.at(1), 128, T_TMP, false);                   // -dA = dX W^T + dY U^T
+      umma::issue_pitched<128, false, false>(cx, sl.at(2), PB, sl.at(0), 2048, 128, T_TMP, true);
+      commit(cx);
+      umma::commit_wait_cta(cx);
+      sl.load(0, Ug + HN);
+      vphase(2, 0);
+      sl.wait(0);
+      umma::issue_pitched<128, false, false>(cx, sl.at(4), PB, sl.at(0), 2048, 128, T_TMP, true);
+      commit(cx);
+      vphase(4, 1);
+      umma::commit_wait_cta(cx);
+    }
+    // ---- dA into slot 4 (dM is in slot 5); slots 0 .. 3 are free
+    {
+      float v[32];
+      ld32(cx, tb + T_TMP, v);
+      const int sr = seg_s[row];
+      const float lr = SC ? lam_s[row] * DN_LOG2E : 0.f;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const int j = group * 32 + i;
+        float f = 1.f;
+        if (SC) f = umma::ex2_fast(fminf(lr - lam_s[j] * DN_LOG2E, 0.f));
+        v[i] = (j < row && sr == seg_s[j]) ? -v[i] * f : 0.f;
+      }
+      image32(sl.at(4), 128, row, group, v);
+    }
+
+    // ---- key side: rows of q, k, b in the row mapping
+    const bool live = rx < rows;
+    const size_t tokx = tok0 + (live ? rx : 0);
+    const uint8_t* krow = reinterpret_cast<const uint8_t*>(a.k) + (tokx * g.Hk + h / g.qk_div) * g.K * qes;
+    const uint8_t* qrow = reinterpret_cast<const uint8_t*>(a.q) + (tokx * g.Hk + h / g.qk_div) * g.K * qes;
+    const uint8_t* brow = reinterpret_cast<const uint8_t*>(a.b) + (tokx * g.bH + g.gate_head(h, g.bH)) * bC * ges;
+    float rq = 1.f, rk = 1.f;
+    if (l2) {
+      float sq = 0.f, sk = 0.f;
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int p = it * 4 + rp;
+        if (p < kp) {
+          float f[8];
+          ldrow8(qrow, p, qdt, f);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) sq = fmaf(f[i], f[i], sq);
+          ldrow8(krow, p, qdt, f);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) sk = fmaf(f[i], f[i], sk);
+        }
+      }
+      sq += __shfl_xor_sync(0xffffffffu, sq, 1); sk += __shfl_xor_sync(0xffffffffu, sk, 1);
+      sq += __shfl_xor_sync(0xffffffffu, sq, 2); sk += __shfl_xor_sync(0xffffffffu, sk, 2);
+      rq = live ? rsqrtf(sq + 1e-6f) : 1.f;
+      rk = live ? rsqrtf(sk + 1e-6f) : 1.f;
+    }
+    if (rp == 0) { rq_s[rx] = rq; rk_s[rx] = rk; }
+    // the pieces of row rx as loaded, and activated: k_hat, q_hat, beta = b k_hat
+    Raw8 rawk, rawq, rawb;
+    float b1 = 0.f;
+    if (SC) b1 = bet_s[rx];
+    else if (bC == 1) {
+      b1 = ldf_ro(brow, 0, gdt);
+      if (fuse) b1 = sigmoid_fast(b1); else if (guard) b1 = fmaxf(b1, 0.f);
+      if (rp == 0) bet_s[rx] = live ? b1 : 0.f;
+    }
+    auto load_pieces = [&](int p) {
+      const int pc = p < kp ? p : 0;
+      rawk = ldraw(krow, pc, qdt);
+      rawq = ldraw(qrow, pc, qdt);
+      if (bC != 1) rawb = ldraw(brow, pc, gdt);
+    };
+    auto pieces = [&](int p, float (&kh)[8], float (&qh)[8], float (&be)[8]) {
+      const bool on = live && p < kp;
+      cvraw(rawk, qdt, kh);
+      cvraw(rawq, qdt, qh);
+      const float rqs = rq * g.scale;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { kh[i] = on ? kh[i] * rk : 0.f; qh[i] = on ? qh[i] * rqs : 0.f; }
+      if (round_in) {
+        const uint4 pk = umma::pack8(kh), pq = umma::pack8(qh);
+        umma::unpack8(pk, kh);
+        umma::unpack8(pq, qh);
+      }
+      if (bC == 1) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) be[i] = b1 * kh[i];
+      } else {
+        cvraw(rawb, gdt, be);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (fuse) be[i] = sigmoid_fast(be[i]); else if (guard) be[i] = fmaxf(be[i], 0.f);
+          be[i] *= kh[i];
+        }
+      }
+    };
+
+    // ---- the decay of all channels: thread (channel, 32 rows), scanned in registers, restarting at document changes
+    if constexpr (!SC) {
+      if (tid < C) {                                    // seg_s is non-decreasing: binary searches
+        const int sx = seg_s[tid];
+        int lo = 0, hi = tid;
+        while (lo < hi) { const int mid = (lo + hi) >> 1; if (seg_s[mid] < sx) lo = mid + 1; else hi = mid; }
+        ds_s[tid] = (uint8_t)lo;
+        lo = tid; hi = C - 1;
+        while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (seg_s[mid] > sx) hi = mid - 1; else lo = mid; }
+        de_s[tid] = (uint8_t)lo;
+      }
+      const int c = tid & 127, qd = tid >> 7, x0 = qd * 32;
+      const uint32_t gpitch = (uint32_t)(g.gH * gC) * ges;
+      const uint8_t* gp = reinterpret_cast<const uint8_t*>(a.gg) + (tok0 * g.gH + g.gate_head(h, g.gH)) * gC * ges + (gC == 1 ? 0 : c) * ges;
+      const bool cin = gC == 1 || c < gC;
+      float v[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const bool on = cin && x0 + i < rows;
+        float gv = ldf_ro(gp + (on ? (size_t)(x0 + i) * gpitch : 0) - (cin ? 0 : (size_t)c * ges), 0, gdt);
+        if (fuse) gv = -umma::ex2_fast(fminf(gv, 5.f) * DN_LOG2E); else gv = gv <= 0.f ? gv : 0.f;
+        if (guard) gv = fminf(gv, -1e-6f);
+        v[i] = on ? gv : 0.f;
+      }
+      const uint32_t cuts = __ballot_sync(0xffffffffu, x0 + lane > 0 && seg_s[x0 + lane] != seg_s[x0 + lane - (x0 + lane > 0)]);
+#pragma unroll
+      for (int i = 1; i < 32; ++i) v[i] += (cuts >> i) & 1 ? 0.f : v[i - 1];
+      TOT[qd * 128 + c] = v[31];
+      if (c == 0) cut_s[qd] = cuts != 0;
+      __syncthreads();
+      float carry = 0.f;
+      for (int q2 = qd - 1; q2 >= 0; --q2) { carry += TOT[q2 * 128 + c]; if (cut_s[q2]) break; }
+      const int nr = cuts ? __ffs(cuts) - 1 : 32;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) LAM[(x0 + i) * LPF + c] = (v[i] + (i < nr ? carry : 0.f)) * DN_LOG2E;
+      __syncthreads();
+      if (tid < C) {
+        EDGE[tid] = umma::ex2_fast(0.5f * (LAM[tid] + LAM[de_s[0] * LPF + tid]));
+        EDGE[128 + tid] = umma::ex2_fast(0.5f * (LAM[(C - 1) * LPF + tid] - LAM[ds_s[C - 1] * LPF + tid]));
+      }
+    }
+    __syncthreads();
+    // ---- dqe, dX, dke scaled where they lie; the column sums of ke dke
+    {
+      const bool first = seg_s[row] == seg_s[0], last = seg_s[row] == seg_s[C - 1];
+      float v[32];
+      const float el = SC ? (first ? umma::exp_neg(fminf(lam_s[row], 0.f)) : 0.f) : 0.f;
+      auto scale_first = [&](uint32_t col) {
+        ld32(cx, tb + col, v);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] *= SC ? el : (first ? EDGE[group * 32 + i] : 0.f);
+        st32(tb + col, v);
+      };
+      scale_first(T_Q);
+      scale_first(T_B);
+      ld32(cx, tb + T_K, v);
+      const bool on = last && row < rows;
+      const float eks = SC ? umma::exp_neg(fminf(lam_s[C - 1] - lam_s[row], 0.f)) : 0.f;
+      const uint8_t* kr = reinterpret_cast<const uint8_t*>(a.k) + ((tok0 + (row < rows ? row : 0)) * g.Hk + h / g.qk_div) * g.K * qes;
+      float od[32];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int p = group * 4 + j;
+        float kh[8];
+        ldrow8(kr, p < kp ? p : 0, qdt, kh);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int c = group * 32 + 8 * j + i;
+          kh[i] *= rk_s[row];
+          if (round_in) kh[i] = bf16r(kh[i]);
+          const float e = SC ? eks : umma::ex2_fast(fminf(LAM[(C - 1) * LPF + c] - LAM[row * LPF + c], 0.f));
+          od[8 * j + i] = on && p < kp ? v[8 * j + i] * (kh[i] * e) : 0.f;
+          v[8 * j + i] *= SC ? (last ? eks : 0.f) : (last ? EDGE[128 + c] : 0.f);
+        }
+      }
+      st32(tb + T_K, v);
+      if (SC) {
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) s += od[i];
+        s = warp_sum(s);
+        if (lane == 0) PS[warp] = s;
+      } else {
+        fold<16>(od, lane);
+        fold<8>(od, lane);
+        fold<4>(od, lane);
+        fold<2>(od, lane);
+        fold<1>(od, lane);
+        PS[quarter * 128 + group * 32 + lane] = od[0];
+      }
+      umma::tmem_wait_st();
+    }
+    // ---- T1, T2, T3 on top of them
+    if constexpr (SC) {
+      uint4 *KI = sl.at(0), *QI = sl.at(1), *BI = sl.at(2);
+#pragma unroll 2
+      for (int it = 0; it < 4; ++it) {
+        const int p = it * 4 + rp;
+        float kh[8], qh[8], be[8];
+        load_pieces(p);
+        pieces(p, kh, qh, be);
+        KI[p * PP + rx] = umma::pack8(kh);
+        QI[p * PP + rx] = umma::pack8(qh);
+        BI[p * PP + rx] = umma::pack8(be);
+      }
+      umma::pre_issue_sync();
+      umma::issue_pitched<128, false, true>(cx, sl.at(4), 2048, KI, PB, C, T_B, true);       // (dA f)   k_hat
+      umma::issue_pitched<128, false, true>(cx, sl.at(5), 2048, KI, PB, C, T_Q, true);       // (dM f)   k_hat
+      umma::issue_pitched<128, true, true>(cx, sl.at(4), 2048, BI, PB, C, T_K, true);        // (dA f)^T (b k_hat)
+      umma::issue_pitched<128, true, true>(cx, sl.at(5), 2048, QI, PB, C, T_K, true);        // (dM f)^T q_hat
+      commit(cx);
+      umma::commit_wait_cta(cx);
+    } else {
+      load_pieces(rp);
+#pragma unroll 1
+      for (int grp = 0; grp < 4; ++grp) {
+        const int p = grp * 4 + rp;
+        uint4* KF = reinterpret_cast<uint4*>(sm + OFF_GI + (grp & 1) * 3 * 4 * PB);
+        uint4* QF = KF + 4 * PP;
+        uint4* BF = QF + 4 * PP;
+        float kh[8], qh[8], be[8];
+        pieces(p, kh, qh, be);
+        const float* lx = LAM + rx * LPF + 8 * p;
+        const float* ls = LAM + ds_s[rx] * LPF + 8 * p;
+        const float* le = LAM + de_s[rx] * LPF + 8 * p;
+#pragma unroll
+        for (int i = 0; i < 8; i += 4) {
+          const float4 u0 = *reinterpret_cast<const float4*>(lx + i), u1 = *reinterpret_cast<const float4*>(ls + i), u2 = *reinterpret_cast<const float4*>(le + i);
+          const float d[4] = {fmaf(-0.5f, u1.x + u2.x, u0.x), fmaf(-0.5f, u1.y + u2.y, u0.y), fmaf(-0.5f, u1.z + u2.z, u0.z), fmaf(-0.5f, u1.w + u2.w, u0.w)};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float f = umma::ex2_fast(d[u]), fi = umma::ex2_fast(-d[u]);
+            kh[i + u] *= fi;
+            qh[i + u] *= f;
+            be[i + u] *= f;
+          }
+        }
+        if (grp >= 2) {                                 // the set was read by the products of group - 2
+          bool ok = true;
+          if (warp == 0 && !cx.dead) ok = umma::mbar_wait(&gbar[grp & 1], (gph >> (grp & 1)) & 1u);
+          gph ^= 1u << (grp & 1);
+          if (__syncthreads_or(!ok)) { cx.dead = true; umma::report_timeout(a.err); }
+        }
+        KF[rp * PP + rx] = umma::pack8(kh);
+        QF[rp * PP + rx] = umma::pack8(qh);
+        BF[rp * PP + rx] = umma::pack8(be);
+        umma::pre_issue_sync();
+        umma::issue_pitched<32, false, true>(cx, sl.at(4), 2048, KF, PB, C, T_B + 32 * grp, true);       // dA (k / f)
+        umma::issue_pitched<32, false, true>(cx, sl.at(5), 2048, KF, PB, C, T_Q + 32 * grp, true);       // dM (k / f)
+        umma::issue_pitched<32, true, true>(cx, sl.at(4), 2048, BF, PB, C, T_K + 32 * grp, true);        // dA^T (beta f)
+        umma::issue_pitched<32, true, true>(cx, sl.at(5), 2048, QF, PB, C, T_K + 32 * grp, true);        // dM^T (q f)
+        if (tid == 0 && !cx.dead) umma::mma_commit(&gbar[grp & 1]);
+        if (grp < 3) load_pieces((grp + 1) * 4 + rp);
+      }
+      bool ok = true;
+      if (warp == 0 && !cx.dead) ok = umma::mbar_wait(&gbar[0], gph & 1u) && umma::mbar_wait(&gbar[1], (gph >> 1) & 1u);
+      gph ^= 3u;
+      if (__syncthreads_or(!ok)) { cx.dead = true; umma::report_timeout(a.err); }
+      umma::tc_fence_after();
+    }
+    if (tid == 0 && e_item + (int)gridDim.x < a.items) {      // the next tile's images on their way into L2
+      const int nx = e_item + gridDim.x;
+      const size_t nb = (size_t)(nx % (g.B * g.H)) * g.NC + a.c_begin + nx / (g.B * g.H);
+      umma::prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(a.res.W) + nb * C * K, IMGB);
+      umma::prefetch_l2(states_img(g, a.res.states) + nb * K * VW, IMGB * NH);
+      umma::prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(a.res.U) + nb * C * VW, IMGB * NH);
+      umma::prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(a.dV) + nb * C * VW, IMGB * NH);
+      umma::prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(a.dH) + nb * K * VW, IMGB * NH);
+      umma::prefetch_l2(a.res.T + nb * C * C, IMGB);
+    }
+    // ---- raw k, q and b, turned from the row mapping into a row per lane
+    uint4* const RK = reinterpret_cast<uint4*>(sm + OFF_RK);
+    uint4* const RQ = reinterpret_cast<uint4*>(sm + OFF_RQ);
+    uint4* const RB = reinterpret_cast<uint4*>(sm + OFF_RB);
+    const bool staged = qdt == DN_BF16;                 // fp32 q, k are read and written a row per lane
+    if (staged) {
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int p = it * 4 + rp;
+        if (live && p < kp) {
+          umma::cp_async16(RK + p * PP + rx, krow + 16 * p);
+          umma::cp_async16(RQ + p * PP + rx, qrow + 16 * p);
+        } else RK[p * PP + rx] = RQ[p * PP + rx] = make_uint4(0, 0, 0, 0);
+      }
+    }
+    if (bC != 1) {
+      const int nv = gdt == DN_BF16 ? 16 : 32, have = kp * (gdt == DN_BF16 ? 1 : 2);
+#pragma unroll 4
+      for (int it = 0; it < nv / 4; ++it) {
+        const int p = it * 4 + rp;
+        if (live && p < have) umma::cp_async16(RB + p * PP + rx, brow + 16 * p);
+        else RB[p * PP + rx] = make_uint4(0, 0, 0, 0);
+      }
+    }
+    umma::cp_async_commit();
+    umma::cp_async_wait<0>();
+    __syncthreads();
+    // ---- combination, a row per lane, 32 channels per warp.  d q_n, d k_n and dLambda wait in the columns just read for the
+    //      row sums of the l2norm adjoint.
+    {
+      const bool rlive = row < rows;
+      const float dmii = dmi_s[row], rqr = rq_s[row], rkr = rk_s[row];
+      const size_t tokr = tok0 + (rlive ? row : 0);
+      const uint8_t* kg = reinterpret_cast<const uint8_t*>(a.k) + (tokr * g.Hk + h / g.qk_div) * g.K * qes;
+      const uint8_t* qg = reinterpret_cast<const uint8_t*>(a.q) + (tokr * g.Hk + h / g.qk_div) * g.K * qes;
+      auto raw_kq = [&](int p, float (&kr)[8], float (&qr)[8]) {
+        if (staged) {
+          umma::unpack8(RK[p * PP + row], kr);
+          umma::unpack8(RQ[p * PP + row], qr);
+        } else {
+          const bool on = rlive && p < kp;
+          ldrow8(kg, p < kp ? p : 0, qdt, kr);
+          ldrow8(qg, p < kp ? p : 0, qdt, qr);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) { kr[i] = on ? kr[i] : 0.f; qr[i] = on ? qr[i] : 0.f; }
+        }
+      };
+      float dq_dot = 0.f, dk_dot = 0.f, sb = 0.f, slam = 0.f;
+#pragma unroll 1
+      for (int it = 0; it < 4; ++it) {
+        const int p = group * 4 + it;
+        float dbp[8], dqp[8], dkp[8], kr[8], qr[8], ba[8], od[8];
+        if (!cx.dead) {
+          umma::tmem_ld8(tb + T_B + it * 8, dbp);
+          umma::tmem_ld8(tb + T_Q + it * 8, dqp);
+          umma::tmem_ld8(tb + T_K + it * 8, dkp);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) dbp[i] = dqp[i] = dkp[i] = 0.f;
+        }
+        raw_kq(p, kr, qr);
+        uint32_t bpos = 0, bzero = 0;                   // stability_guard: which raw b are above / at zero
+        if (bC == 1) {
+          const float b2 = bet_s[row];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) ba[i] = b2;
+        } else {
+          if (gdt == DN_BF16) umma::unpack8(RB[p * PP + row], ba);
+          else {
+            *reinterpret_cast<uint4*>(ba) = RB[2 * p * PP + row];
+            *reinterpret_cast<uint4*>(ba + 4) = RB[(2 * p + 1) * PP + row];
+          }
+          if (fuse) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ba[i] = rlive ? sigmoid_fast(ba[i]) : 0.f;
+          } else if (guard) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              bpos |= ba[i] > 0.f ? 1u << i : 0u;
+              bzero |= ba[i] == 0.f ? 1u << i : 0u;
+              ba[i] = fmaxf(ba[i], 0.f);
+            }
+          }
+        }
+        if constexpr (!SC) {
+          const float* lx = LAM + row * LPF + 8 * p;
+          const float* ls = LAM + ds_s[row] * LPF + 8 * p;
+          const float* le = LAM + de_s[row] * LPF + 8 * p;
+#pragma unroll
+          for (int i = 0; i < 8; i += 4) {
+            const float4 u0 = *reinterpret_cast<const float4*>(lx + i), u1 = *reinterpret_cast<const float4*>(ls + i), u2 = *reinterpret_cast<const float4*>(le + i);
+            const float d[4] = {fmaf(-0.5f, u1.x + u2.x, u0.x), fmaf(-0.5f, u1.y + u2.y, u0.y), fmaf(-0.5f, u1.z + u2.z, u0.z), fmaf(-0.5f, u1.w + u2.w, u0.w)};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const float f = umma::ex2_fast(d[u]);
+              dbp[i + u] *= f;
+              dqp[i + u] *= f;
+              dkp[i + u] *= umma::ex2_fast(-d[u]);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float qn = qr[i] * rqr, kn = kr[i] * rkr;
+          float qh = qn * g.scale, kh = kn;
+          if (round_in) { qh = bf16r(qh); kh = bf16r(kh); }
+          const float be = ba[i] * kh, dbeta = dbp[i];
+          od[i] = be * dbeta + qh * dqp[i] - kh * dkp[i];
+          slam += od[i];
+          const float dq = (dqp[i] + dmii * kh) * g.scale, dk = dkp[i] + dmii * qh + dbeta * ba[i];
+          float dbv = dbeta * kh;                       // d b_act
+          if (fuse) dbv *= ba[i] * (1.f - ba[i]);       // through the sigmoid
+          else if (guard && bC != 1) dbv *= (bpos >> i) & 1 ? 1.f : ((bzero >> i) & 1 ? 0.5f : 0.f);       // through max(b, 0)
+          sb += dbv;
+          dbp[i] = dbv;
+          dqp[i] = dq;                                  // d q_n, d k_n before the l2norm adjoint
+          dkp[i] = dk;
+          dq_dot = fmaf(qn, dq, dq_dot);
+          dk_dot = fmaf(kn, dk, dk_dot);
+        }
+        umma::tmem_st8(tb + T_Q + it * 8, dqp);
+        umma::tmem_st8(tb + T_K + it * 8, dkp);
+        if (!SC) umma::tmem_st8(tb + T_B + it * 8, od);
+        if (bC != 1) {                                  // d b in the place of b, when it has b's type
+          if (a.db_dt != gdt) { if (rlive && p < kp) strow8(a.db, ((tok0 + row) * g.H + h) * bC + 8 * p, a.db_dt, dbp); }
+          else if (gdt == DN_BF16) RB[p * PP + row] = umma::pack8(dbp);
+          else {
+            RB[2 * p * PP + row] = *reinterpret_cast<const uint4*>(dbp);
+            RB[(2 * p + 1) * PP + row] = *reinterpret_cast<const uint4*>(dbp + 4);
+          }
+        }
+      }
+      SUM[group * 128 + row] = dq_dot;
+      SUM[512 + group * 128 + row] = dk_dot;
+      SUM[1024 + group * 128 + row] = sb;
+      SUM[1536 + group * 128 + row] = slam;
+      umma::tmem_wait_st();
+      __syncthreads();
+      dq_dot = (SUM[row] + SUM[128 + row]) + (SUM[256 + row] + SUM[384 + row]);
+      dk_dot = (SUM[512 + row] + SUM[640 + row]) + (SUM[768 + row] + SUM[896 + row]);
+      if (bC == 1 && group == 0 && rlive) {
+        float s = (SUM[1024 + row] + SUM[1152 + row]) + (SUM[1280 + row] + SUM[1408 + row]);
+        if (guard && !fuse) {                           // through max(b, 0)
+          const float braw = ldf_ro(a.b, (tok0 + row) * g.bH + g.gate_head(h, g.bH), gdt);
+          s *= braw > 0.f ? 1.f : (braw == 0.f ? 0.5f : 0.f);
+        }
+        stf(a.db, (tok0 + row) * g.H + h, s, a.db_dt);
+      }
+      const bool inplace = staged && a.dq_dt == DN_BF16;
+#pragma unroll 2
+      for (int it = 0; it < 4; ++it) {
+        const int p = group * 4 + it;
+        float dqn[8], dkn[8], kr[8], qr[8];
+        umma::tmem_ld8(tb + T_Q + it * 8, dqn);
+        umma::tmem_ld8(tb + T_K + it * 8, dkn);
+        if (l2) {
+          raw_kq(p, kr, qr);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            dqn[i] = rqr * (dqn[i] - qr[i] * rqr * dq_dot);
+            dkn[i] = rkr * (dkn[i] - kr[i] * rkr * dk_dot);
+          }
+        }
+        if (inplace) {
+          RQ[p * PP + row] = umma::pack8(dqn);
+          RK[p * PP + row] = umma::pack8(dkn);
+        } else if (rlive && p < kp) {
+          const size_t o = ((tok0 + row) * g.H + h) * g.K + 8 * p;
+          strow8(a.dq, o, a.dq_dt, dqn);
+          strow8(a.dk, o, a.dq_dt, dkn);
+        }
+        if constexpr (!SC) {                            // dLambda over Lambda, which nobody needs any more
+          float od[8];
+          umma::tmem_ld8(tb + T_B + it * 8, od);
+          *reinterpret_cast<float4*>(LAM + row * LPF + 8 * p) = make_float4(od[0], od[1], od[2], od[3]);
+          *reinterpret_cast<float4*>(LAM + row * LPF + 8 * p + 4) = make_float4(od[4], od[5], od[6], od[7]);
+        }
+      }
+      umma::tc_fence_before();
+      __syncthreads();
+      if (inplace && live) {
+        const size_t o = ((tok0 + rx) * g.H + h) * g.K;
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+          const int p = it * 4 + rp;
+          if (p < kp) {
+            reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.dq) + o)[p] = RQ[p * PP + rx];
+            reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.dk) + o)[p] = RK[p * PP + rx];
+          }
+        }
+      }
+      if (bC != 1 && a.db_dt == gdt && live) {
+        uint4* d = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(a.db) + ((tok0 + rx) * g.H + h) * bC * ges);
+        const int have = kp * (gdt == DN_BF16 ? 1 : 2);
+        for (int p = rp; p < have; p += 4) d[p] = RB[p * PP + rx];
+      }
+    }
+    // ---- dg_t = sum_{i >= t, same doc} dLambda_i, and in the last document the Lambda_end path
+    const int segL = seg_s[C - 1], hg = g.gate_head(h, g.gH);
+    auto g_adjoint = [&](float d, float graw) {
+      if (fuse) {
+        const float gexp = -umma::ex2_fast(fminf(graw, 5.f) * DN_LOG2E);
+        return graw <= 5.f && (!guard || gexp < -1e-6f) ? d * gexp : 0.f;
+      }
+      return (guard ? graw < -1e-6f : graw <= 0.f) ? d : 0.f;               // through min(min(g, 0), -1e-6)
+    };
+    if constexpr (SC) {
+      if (tid < C) {
+        float v = (SUM[1536 + tid] + SUM[1664 + tid]) + (SUM[1792 + tid] + SUM[1920 + tid]);
+        bool cut = tid < C - 1 && seg_s[tid] != seg_s[tid + 1];             // a document ends behind this row
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const float dn = __shfl_down_sync(0xffffffffu, v, o);
+          const bool dc = __shfl_down_sync(0xffffffffu, (int)cut, o);
+          if (lane + o < 32) { if (!cut) v += dn; cut |= dc; }
+        }
+        if (lane == 0) { TOT[warp] = v; cut_s[warp] = cut; }
+        float e = dlend_s[lane] + dlend_s[32 + lane] + dlend_s[64 + lane] + dlend_s[96 + lane] + (lane < 16 ? PS[lane] : 0.f);
+        e = warp_sum(e);
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        float carry = 0.f;
+        for (int w2 = warp + 1; w2 < 4; ++w2) { carry += TOT[w2]; if (cut_s[w2]) break; }
+        if (!cut) v += carry;
+        if (seg_s[tid] == segL) v += e;
+        if (tid < rows) stf(a.dg, (tok0 + tid) * g.H + h, g_adjoint(v, ldf_ro(a.gg, (tok0 + tid) * g.gH + hg, gdt)), a.dg_dt);
+      }
+    } else {
+      const int c = tid & 127, qd = tid >> 7, x0 = qd * 32;
+      float v[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = LAM[(x0 + i) * LPF + c];
+      // documents that end behind a row of this quarter
+      const uint32_t ends = __ballot_sync(0xffffffffu, x0 + lane < C - 1 && seg_s[x0 + lane] != seg_s[x0 + lane + (x0 + lane < C - 1)]);
+#pragma unroll
+      for (int i = 30; i >= 0; --i) v[i] += (ends >> i) & 1 ? 0.f : v[i + 1];
+      TOT[qd * 128 + c] = v[0];
+      if (c == 0) cut_s[4 + qd] = ends != 0;
+      __syncthreads();
+      float carry = 0.f;
+      if (!(ends >> 31))                                // (the last row's own end cuts the quarter off from what follows)
+        for (int q2 = qd + 1; q2 < 4; ++q2) { carry += TOT[q2 * 128 + c]; if (cut_s[4 + q2]) break; }
+      const int lastcut = ends ? 31 - __clz(ends) : -1; // rows behind it take the carry
+      const float e = dlend_s[c] + (PS[c] + PS[128 + c]) + (PS[256 + c] + PS[384 + c]);
+      float sg[32];
+      const bool cin = gC == 1 || c < gC;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const int x = x0 + i;
+        float o = v[i] + (i > lastcut ? carry : 0.f);
+        if (seg_s[x] == segL) o += e;
+        sg[i] = o;
+      }
+      if (gC != 1) {
+#pragma unroll 8
+        for (int i = 0; i < 32; ++i) {
+          const int x = x0 + i;
+          if (x < rows && cin) {
+            const float gr = ldf_ro(a.gg, ((tok0 + x) * g.gH + hg) * gC + c, gdt);
+            stf(a.dg, ((tok0 + x) * g.H + h) * gC + c, g_adjoint(sg[i], gr), a.dg_dt);
+          }
+        }
+      } else {                                          // one decay per row: the sum over the channels
+#pragma unroll
+        for (int i = 0; i < 32; ++i) sg[i] = warp_sum(c < g.K ? sg[i] : 0.f);
+        if (lane == 0) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) SUM[(c >> 5) * 128 + x0 + i] = sg[i];
+        }
+        __syncthreads();
+        if (tid < rows) {
+          const float s = (SUM[tid] + SUM[128 + tid]) + (SUM[256 + tid] + SUM[384 + tid]);
+          stf(a.dg, (tok0 + tid) * g.H + h, g_adjoint(s, ldf_ro(a.gg, (tok0 + tid) * g.gH + hg, gdt)), a.dg_dt);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  umma::tc_fence_before();
+  __syncthreads();
+  if (warp == 0) umma::tmem_dealloc(tmem_base, 512);
+}
+
+}  // namespace
+
+bool prepass_bwd_scalar_route(const Geo& g) {
+  return g.gC == 1 && g.bC == 1 && g.qkv_dt == DN_BF16 && !(g.flags & DN_FUSE_PROLOGUE);
+}
+
+int launch_prepass_bwd_fast(const PrepassBwdArgs& a, cudaStream_t st) {
+  const Geo& g = a.g;
+  const int grid = a.items < sm_count() ? a.items : sm_count();
+  auto go = [&](auto kernel) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    kernel<<<grid, NT, SMEM_BYTES, st>>>(a);
+  };
+  auto pick = [&](auto vw) {
+    constexpr int VW = decltype(vw)::value;
+    if (prepass_bwd_scalar_route(g)) { go(prepass_bwd_fast_kernel<VW, 2, true>); return; }
+    switch (input_mode(g)) {
+      case 0: go(prepass_bwd_fast_kernel<VW, 0, false>); break;
+      case 1: go(prepass_bwd_fast_kernel<VW, 1, false>); break;
+      case 4: go(prepass_bwd_fast_kernel<VW, 4, false>); break;
+      default: go(prepass_bwd_fast_kernel<VW, 2, false>); break;
+    }
+  };
+  if (g.Vw == 256) pick(std::integral_constant<int, 256>{});
+  else pick(std::integral_constant<int, 128>{});
+  return launch_status();
+}
+
+}  // namespace dn

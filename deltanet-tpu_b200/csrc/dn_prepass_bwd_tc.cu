@@ -36,9 +36,8 @@
 // pieces of 8 channels (row = 8 * warp + (lane & 7) is fixed per thread); phases that drain or use
 // tensor memory own one row per thread (row = the thread's lane of its warp's lane quarter) and use
 // the panel layout of the scratch (see the header).
-#ifdef DN_PHASE_TIMING
-#include <cstdio>
-#endif
+#include <type_traits>
+
 #include "dn_chunkprep.cuh"
 #include "dn_kernels.cuh"
 #include "dn_prepass_bwd_tc.cuh"
@@ -95,8 +94,8 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
   __shared__ uint32_t tmem_base;
   __shared__ int seg_s[C];
   __shared__ int reset_s[8];                 // per 32-row quarter: a document starts inside it
-  __shared__ uint8_t ds_s[C], de_s[C];       // first / last row of each row's document inside the chunk
-  __shared__ float rq_s[C], rk_s[C], dlend_s[K], dlend_b_s[C];     // dlend_b_s: the activated scalar erase gate per row (scalar-gate path)
+  __shared__ float rq_s[C], rk_s[C], dlend_s[K];
+  __shared__ uint32_t todo_s[NT / 32];       // which of the next NT tiles of this CTA are marked
   const Geo& g = a.g;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int myrow = warp * 8 + (lane & 7), lgrp = lane >> 3;      // the 8 rows x 4 pieces mapping
@@ -125,6 +124,19 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
   const float4* DQE4 = reinterpret_cast<const float4*>(DQE);
   const float4* DKE4 = reinterpret_cast<const float4*>(DKE);
 
+  // Tiles are looked up NT at a time, so that a launch that finds nothing marked (the usual case) ends after
+  // one load per thread, without touching tensor memory.
+  auto look_up = [&](int base) {
+    const int e = base + tid * gridDim.x;
+    const bool on = e < a.items && strong_flag(a.res, (size_t)(e % (g.B * g.H)) * g.NC + a.c_begin + e / (g.B * g.H));
+    const uint32_t m = __ballot_sync(0xffffffffu, on);
+    if (lane == 0) todo_s[warp] = m;
+    return __syncthreads_or(on) != 0;
+  };
+  int base = blockIdx.x;
+  while (base < a.items && !look_up(base)) base += gridDim.x * NT;
+  if (base >= a.items) return;
+
   if (tid == 0) { umma::mbar_init(&mma_bar, 1); umma::mbar_init(&v_bar, 1); umma::mbar_init(&g_bar, 1); umma::fence_mbar_init(); }
   uint32_t v_phase = 0;
   ImgLoader imgld{&g_bar, 0u, a.err};
@@ -144,13 +156,15 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
   const bool trunc = g.flags & DN_TRUNC_DT_BF16;
 
   // work items in chunk-major order inside the chunk range: all heads of chunk c_begin first
-  for (int e_item = blockIdx.x; e_item < a.items; e_item += gridDim.x) {
+  for (;;) {
+  for (int tw = 0; tw < NT / 32; ++tw)
+  for (uint32_t tm = todo_s[tw]; tm; tm &= tm - 1) {
+    const int e_item = base + (tw * 32 + __ffs(tm) - 1) * gridDim.x;
     const int bh = e_item % (g.B * g.H), c_idx = a.c_begin + e_item / (g.B * g.H);
     const int h = bh % g.H, b = bh / g.H;
     const int item = bh * g.NC + c_idx;
     const int t0 = c_idx * C;
     const size_t ibase = (size_t)item;
-    DN_MARK(0);
     for (int i = tid; i < C; i += NT) seg_s[i] = seg_at(a.seg, b, t0 + i, g.L);
     bool is_new, all_same;
     chunk_flags(a.seg, g, b, c_idx, is_new, all_same);
@@ -292,7 +306,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
     }
     __syncthreads();
 
-    DN_MARK(7);
     // ---- L. rows, normalisers, cumulative decay
     row_norms_8x4(r, myrow, lgrp, rq_s, rk_s);
     lambda_scan_512(r, seg_s, LAM, TOTL, reset_s);
@@ -302,176 +315,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
       __syncthreads();
     }
 
-    // where phase E finds dbeta', dq', dk': 0 = fp32 panels in the scratch; 1 = the accumulators T1 | T2 | T3 in tensor
-    // memory, still to be scaled by f, f, 1/f; 2 = the same unscaled
-    int tm_src = 0;
-    if constexpr (CF::scalar_gates) {
-      // ---- D + H for one scalar decay and one scalar beta per (token, head).  With f_ij = e^{lam_i - lam_j}
-      //      (exact, <= 1 on the entries that survive the masks) and b_i the activated erase gate,
-      //        dbeta'_i = sum_j (dA_ij f_ij) k_j            dq'_i = sum_{j<i} (dM_ij f_ij) k_j
-      //        dk'_j    = sum_i (dA_ij f_ij b_i) k_i + sum_{i>j} (dM_ij f_ij) q_i
-      //      i.e. four products on the plain bf16 images of k_hat and q_hat: no levels, no diagonal pass.
-      //      The image of dA f is used twice, the second time with its rows scaled by b_i.
-      DN_MARK(8);
-      {
-        const int x = myrow;
-        const bool live = x < r.rows_valid;
-        if (lgrp == 0) dlend_b_s[x] = live ? ldf_ro(r.b, r.b_row0 + (size_t)x * r.b_pitch, DN_F32) : 0.f;
-#pragma unroll 2
-        for (int it = 0; it < 4; ++it) {
-          const int p = it * 4 + lgrp;
-          float qh[8], kh[8];
-          qhat8(r, x, p, qh);
-          khat8(r, x, p, kh);
-          I_KR[p * 128 + x] = umma::pack8(kh);
-          I_QK[p * 128 + x] = umma::pack8(qh);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {                    // images of dA f and dM f (strictly lower; the diagonal of dM goes through E)
-        const int e = u * NT + tid, p = e >> 7, x = e & 127;
-        const bool any = 8 * p < x;                    // the piece has entries below the diagonal
-        const float4 a0 = umma::ld_keep4_pred(DA4 + p4v(x, 8 * p), any), a1 = umma::ld_keep4_pred(DA4 + p4v(x, 8 * p + 4), any);
-        const float4 m0 = umma::ld_keep4_pred(DM4 + p4v(x, 8 * p), any), m1 = umma::ld_keep4_pred(DM4 + p4v(x, 8 * p + 4), any);
-        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, mv[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
-        const float lx = LAM[x * LP] * DN_LOG2E;
-        float oa[8], om[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int j = 8 * p + i;
-          const float f = umma::ex2_fast(fminf(lx - LAM[j * LP] * DN_LOG2E, 0.f));
-          oa[i] = av[i] * f;                           // (dA is zero on and above the diagonal and across documents)
-          om[i] = j < x ? mv[i] * f : 0.f;
-        }
-        I_DA[e] = umma::pack8(oa);
-        I_DM[e] = umma::pack8(om);
-      }
-      umma::pre_issue_sync();
-      umma::issue<128, false, true>(cx, I_DA, I_KR, C, 0, false);          // (dA f)   k_hat
-      umma::issue<128, false, true>(cx, I_DM, I_KR, C, 128, false);        // (dM f)   k_hat
-      umma::commit_wait(cx);
-      DN_MARK(9);
-      // T1, T2 stay in tensor memory (columns [0, 256)): phase E reads them there
-      umma::tc_fence_before();
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {                    // rows of the dA f image scaled by b_i
-        const int e = u * NT + tid, x = e & 127;
-        float v8[8];
-        umma::unpack8(I_DA[e], v8);
-        const float bx = dlend_b_s[x];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v8[i] *= bx;
-        I_DA[e] = umma::pack8(v8);
-      }
-      umma::pre_issue_sync();
-      umma::issue<128, true, true>(cx, I_DA, I_KR, C, 256, false);         // (dA f b)^T k_hat
-      umma::issue<128, true, true>(cx, I_DM, I_QK, C, 256, true);          // + (dM f)^T q_hat
-      umma::commit_wait(cx);
-      DN_MARK(10);
-      tm_src = 2;                                      // T3 at columns [256, 384), no scaling
-      umma::tc_fence_before();
-      __syncthreads();
-    } else {
-    // ---- Channel-wise decay, moderate in every channel of every document of the chunk (the same test as
-    //      in the forward prepass): D + H collapse to four products as in the scalar case.  With m_c the
-    //      midpoint of a document's cumulative decay and f_ic = e^{Lam_ic - m_c}, all within
-    //      e^{+-FAST_HALF_RANGE},
-    //        dbeta'_i = f_i * sum_j dA_ij (k_j / f_j)          dq'_i = f_i * sum_{j<i} dM_ij (k_j / f_j)
-    //        dk'_j    = (1 / f_j) * sum_i (dA_ij (beta_i f_i) + [i>j] dM_ij (q_i f_i))
-    constexpr float FAST_HALF_RANGE = 32.f;
-    if (tid < C) {                              // first and last row of each row's document inside the chunk
-      const int sx = seg_s[tid];
-      int lo = 0, hi = tid;                     // seg_s is non-decreasing: binary searches
-      while (lo < hi) { const int mid = (lo + hi) >> 1; if (seg_s[mid] < sx) lo = mid + 1; else hi = mid; }
-      ds_s[tid] = (uint8_t)lo;
-      lo = tid; hi = C - 1;
-      while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (seg_s[mid] > sx) hi = mid - 1; else lo = mid; }
-      de_s[tid] = (uint8_t)lo;
-    }
-    __syncthreads();
-    // one test per document and channel, at the document's last row: threads (row x, channel quarter)
-    bool strong = false;
-    {
-      const int x = tid & 127;
-      if (de_s[x] == x) {
-        const float* ls = LAM + ds_s[x] * LP + (tid >> 7) * 32;
-        const float* le = LAM + x * LP + (tid >> 7) * 32;
-#pragma unroll 8
-        for (int c = 0; c < 32; ++c) strong |= 0.5f * (ls[c] - le[c]) > FAST_HALF_RANGE;
-      }
-    }
-    const bool fast = !__syncthreads_or(strong);
-    if (fast) {
-      DN_MARK(8);
-      // log2 of f for (row x, channels 8p..8p+7)
-      auto log2f8 = [&](int x, int p, float (&d)[8]) {
-        const float* lx = LAM + x * LP + 8 * p;
-        const float* ls = LAM + ds_s[x] * LP + 8 * p;
-        const float* le = LAM + de_s[x] * LP + 8 * p;
-        const float4 a0 = *reinterpret_cast<const float4*>(lx), a1 = *reinterpret_cast<const float4*>(lx + 4);
-        const float4 s0 = *reinterpret_cast<const float4*>(ls), s1 = *reinterpret_cast<const float4*>(ls + 4);
-        const float4 e0 = *reinterpret_cast<const float4*>(le), e1 = *reinterpret_cast<const float4*>(le + 4);
-        const float l8[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-        const float m8[8] = {s0.x + e0.x, s0.y + e0.y, s0.z + e0.z, s0.w + e0.w, s1.x + e1.x, s1.y + e1.y, s1.z + e1.z, s1.w + e1.w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i) d[i] = (l8[i] - 0.5f * m8[i]) * DN_LOG2E;
-      };
-      uint4 bt[4];                                     // this thread's pieces of the beta f image, for the second round
-      {
-        const int x = myrow;
-#pragma unroll
-        for (int it = 0; it < 4; ++it) {               // images of k / f (slot KR) and q f (slot QK)
-          const int p = it * 4 + lgrp;
-          float qh[8], kh[8], ba[8], d[8];
-          qhat8(r, x, p, qh);
-          khat8(r, x, p, kh);
-          bact8(r, x, p, ba);
-          log2f8(x, p, d);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float f = umma::ex2_fast(d[i]);
-            ba[i] = (ba[i] * kh[i]) * f;
-            kh[i] *= umma::ex2_fast(-d[i]);
-            qh[i] *= f;
-          }
-          I_KR[p * 128 + x] = umma::pack8(kh);
-          I_QK[p * 128 + x] = umma::pack8(qh);
-          bt[it] = umma::pack8(ba);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {                    // images of dA and of the strictly lower part of dM
-        const int e = u * NT + tid, p = e >> 7, x = e & 127;
-        const bool any = 8 * p < x;
-        const float4 a0 = umma::ld_keep4_pred(DA4 + p4v(x, 8 * p), any), a1 = umma::ld_keep4_pred(DA4 + p4v(x, 8 * p + 4), any);
-        const float4 m0 = umma::ld_keep4_pred(DM4 + p4v(x, 8 * p), any), m1 = umma::ld_keep4_pred(DM4 + p4v(x, 8 * p + 4), any);
-        const float mv[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
-        float om[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) om[i] = 8 * p + i < x ? mv[i] : 0.f;
-        I_DA[e] = make_uint4(umma::pack2(a0.x, a0.y), umma::pack2(a0.z, a0.w), umma::pack2(a1.x, a1.y), umma::pack2(a1.z, a1.w));
-        I_DM[e] = umma::pack8(om);
-      }
-      umma::pre_issue_sync();
-      umma::issue<128, false, true>(cx, I_DA, I_KR, C, 0, false);          // dA (k / f)
-      umma::issue<128, false, true>(cx, I_DM, I_KR, C, 128, false);        // dM (k / f)
-      umma::commit_wait(cx);
-      DN_MARK(9);
-      // the k / f image has been consumed: beta f takes its slot for the second pair of products
-#pragma unroll
-      for (int it = 0; it < 4; ++it) I_KR[(it * 4 + lgrp) * 128 + myrow] = bt[it];
-      // f T1 = dbeta', f T2 = dq' are read from tensor memory by phase E (columns [0, 256))
-      umma::tc_fence_before();
-      umma::pre_issue_sync();
-      umma::issue<128, true, true>(cx, I_DA, I_KR, C, 256, false);         // dA^T (beta f)
-      umma::issue<128, true, true>(cx, I_DM, I_QK, C, 256, true);          // + dM^T (q f)
-      umma::commit_wait(cx);
-      DN_MARK(10);
-      tm_src = 1;                                      // T3 / f = dk' at columns [256, 384)
-      umma::tc_fence_before();
-      __syncthreads();
-    } else {
-    DN_MARK(8);
     // ---- D. diagonal 16x16 blocks, exact.  The blocks of dA and dM are staged in shared memory
     //         (all lanes of a warp read the same entry), and so are k_hat, q_hat and beta of 64 rows
     //         at a time (fp32, one global round trip per half); one thread per (block, channel)
@@ -508,7 +351,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
           *reinterpret_cast<float4*>(BC + xr * CP + 8 * p + 4) = make_float4(ba[4], ba[5], ba[6], ba[7]);
         }
         __syncthreads();
-        DN_MARK(20 + 3 * half);
         if (tm_cache && ((warp & 3) >> 1) == half) {
           // the level sweep reads k_hat, q_hat and beta from tensor memory instead of global memory:
           // thread = row (its own lane), the four warps of a lane quarter take 32 channels each
@@ -565,13 +407,10 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
 #pragma unroll
           for (int j = 0; j < 16; ++j) umma::st_keep1(DKP + p4f(r0 + j, c), sk[j]);
         }
-        DN_MARK(21 + 3 * half);
         __syncthreads();
-        DN_MARK(22 + 3 * half);
       }
     }
 
-    DN_MARK(9);
     // ---- H. three levels
     auto build = [&](int lv) {
       const int s = 16 << lv;
@@ -673,14 +512,10 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
         umma::issue<128, false, true>(cx, I_DM, I_QK, C, 128, false);      // dM_s   QK
         umma::issue<128, true, true>(cx, I_DM, I_QK, C, 128, true);        // dM_s^T QK
         umma::commit_wait(cx);
-        DN_MARK(10 + lv);
       }
     }
     __syncthreads();
-    }
-    }
 
-    DN_MARK(13);
     // ---- E. combination.  Thread mapping of a tensor-memory drain: warp w owns rows 32 (w % 4) + lane
     //         and the 32 channels [32 (w / 4), +32), walked in four pieces of 8.  dbeta', dq', dk' come
     //         straight from the accumulators of the two product rounds when the chunk took a single-Gram
@@ -701,7 +536,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
       const size_t tok = (size_t)b * g.L + t;
       const size_t outb = (tok * g.H + h) * r.bC;
       const size_t outqk = (tok * g.H + h) * K;
-      const bool tm_live = tm_src != 0 && !cx.dead;
       float dq_dot = 0.f, dk_dot = 0.f, sb2 = 0.f;
 #pragma unroll 1
       for (int it = 0; it < 4; ++it) {
@@ -711,20 +545,9 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
         raw_k8(r, x, p, kr);
         bact8(r, x, p, ba);
         if (!fuse && guard) raw_gate8(r.b, r.b_row0, r.b_pitch, r.bC, r.gate_dt, live ? x : 0, p, braw);
-        if (tm_src != 0) {
-          if (tm_live) {
-            umma::tmem_ld8(tb + it * 8, dbp);
-            umma::tmem_ld8(tb + 128 + it * 8, dqp);
-            umma::tmem_ld8(tb + 256 + it * 8, dkp);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) dbp[i] = dqp[i] = dkp[i] = 0.f;
-          }
-        } else {
           ld2x4(DBP4 + p4v(x, 8 * p), dbp);
           ld2x4(DQP4 + p4v(x, 8 * p), dqp);
           ld2x4(DKP4 + p4v(x, 8 * p), dkp);
-        }
         ld2x4(DX4 + p4v(x, 8 * p), dx);
         ld2x4(DQE4 + p4v(x, 8 * p), dqe);
         ld2x4(DKE4 + p4v(x, 8 * p), dke);
@@ -733,19 +556,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
         *reinterpret_cast<float4*>(lam + 4) = *reinterpret_cast<const float4*>(LAM + x * LP + 8 * p + 4);
         *reinterpret_cast<float4*>(lend) = *reinterpret_cast<const float4*>(LAM + (C - 1) * LP + 8 * p);
         *reinterpret_cast<float4*>(lend + 4) = *reinterpret_cast<const float4*>(LAM + (C - 1) * LP + 8 * p + 4);
-        if (tm_src == 1) {                                       // f = e^{Lambda - the document's midpoint}
-          const float* ls = LAM + ds_s[x] * LP + 8 * p;
-          const float* le = LAM + de_s[x] * LP + 8 * p;
-          const float4 s0 = *reinterpret_cast<const float4*>(ls), s1 = *reinterpret_cast<const float4*>(ls + 4);
-          const float4 e0 = *reinterpret_cast<const float4*>(le), e1 = *reinterpret_cast<const float4*>(le + 4);
-          const float m8[8] = {s0.x + e0.x, s0.y + e0.y, s0.z + e0.z, s0.w + e0.w, s1.x + e1.x, s1.y + e1.y, s1.z + e1.z, s1.w + e1.w};
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float d = (lam[i] - 0.5f * m8[i]) * DN_LOG2E;
-            const float f = umma::ex2_fast(d);
-            dbp[i] *= f; dqp[i] *= f; dkp[i] *= umma::ex2_fast(-d);
-          }
-        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           float qh = (qr[i] * rq) * r.scale, kh = kr[i];
@@ -815,7 +625,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
     }
     __syncthreads();
 
-    DN_MARK(14);
     // ---- R. dg_t = sum_{i >= t, same doc} dLambda_i + the Lambda_end path (prefix sum of dke*ke over
     //         earlier rows of the last document, plus the carried-state term).  Thread (channel c,
     //         quarter qd) scans 32 rows in registers; the quarters are chained through shared memory.
@@ -855,7 +664,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
     }
     __syncthreads();
 
-    DN_MARK(15);
     // ---- dg: one warp per row, 4 channels per lane
     {
       const int hg = g.gate_head(h, g.gH);
@@ -897,18 +705,11 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
       }
     }
 
-    DN_MARK(16);
     __syncthreads();
-#ifdef DN_PHASE_TIMING
-    DN_MARK(17);
-    if (blockIdx.x == 0 && tid == 0 && e_item == 0) {
-      for (int i = 1; i < 18; ++i) printf("mark %d -> %d: %lld\n", i - 1, i, g_phase_marks[i] - g_phase_marks[i - 1]);
-      printf("item total %lld\n", g_phase_marks[17] - g_phase_marks[0]);
-      printf("D: stage0 %lld compute0(warp0) %lld wait0 %lld stage1 %lld compute1 %lld wait1 %lld\n", g_phase_marks[20] - g_phase_marks[8],
-             g_phase_marks[21] - g_phase_marks[20], g_phase_marks[22] - g_phase_marks[21], g_phase_marks[23] - g_phase_marks[22],
-             g_phase_marks[24] - g_phase_marks[23], g_phase_marks[25] - g_phase_marks[24]);
-    }
-#endif
+  }
+  __syncthreads();
+  do base += gridDim.x * NT; while (base < a.items && !look_up(base));
+  if (base >= a.items) break;
   }
   umma::tc_fence_before();
   __syncthreads();
@@ -926,6 +727,8 @@ int launch_prepass_bwd_tc(PrepassBwdArgs& a, size_t scratch_floats, cudaStream_t
   if (a.items <= 0) return DN_OK;
   a.scratch_per_cta = prepass_bwd_tc_scratch_per_cta(g);
   a.err = device_error_ptr();
+  int rc = launch_prepass_bwd_fast(a, st);
+  if (rc || prepass_bwd_scalar_route(g)) return rc;
   const int grid = a.items < sm_count() ? a.items : sm_count();
   if (scratch_floats < (size_t)grid * a.scratch_per_cta) return DN_ERR_SCRATCH_TOO_SMALL;
   const size_t lam_phase = (size_t)C * LP * 4 + 4 * 32768;
@@ -939,11 +742,17 @@ int launch_prepass_bwd_tc(PrepassBwdArgs& a, size_t scratch_floats, cudaStream_t
   const int mode = input_mode(g);
   auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   a.bulk_v = mode == 0 && g.V == 128 && a.dw_dt == DN_F32 && al16(a.v) && al16(a.w) && al16(a.dv) && al16(a.dw);
-  if (g.Vw == 256) {
-    if (mode == 0) go(prepass_bwd_tc_kernel<256, 0>); else if (mode == 1) go(prepass_bwd_tc_kernel<256, 1>); else if (mode == 3) go(prepass_bwd_tc_kernel<256, 3>); else if (mode == 4) go(prepass_bwd_tc_kernel<256, 4>); else go(prepass_bwd_tc_kernel<256, 2>);
-  } else {
-    if (mode == 0) go(prepass_bwd_tc_kernel<128, 0>); else if (mode == 1) go(prepass_bwd_tc_kernel<128, 1>); else if (mode == 3) go(prepass_bwd_tc_kernel<128, 3>); else if (mode == 4) go(prepass_bwd_tc_kernel<128, 4>); else go(prepass_bwd_tc_kernel<128, 2>);
-  }
+  auto pick = [&](auto vw) {
+    constexpr int VW = decltype(vw)::value;
+    switch (mode) {
+      case 0: go(prepass_bwd_tc_kernel<VW, 0>); break;
+      case 1: go(prepass_bwd_tc_kernel<VW, 1>); break;
+      case 4: go(prepass_bwd_tc_kernel<VW, 4>); break;
+      default: go(prepass_bwd_tc_kernel<VW, 2>); break;
+    }
+  };
+  if (g.Vw == 256) pick(std::integral_constant<int, 256>{});
+  else pick(std::integral_constant<int, 128>{});
   return launch_status();
 }
 

@@ -101,7 +101,6 @@ __device__ __forceinline__ void bwd_gemms_tc(umma::Ctx& cx, uint8_t* img, const 
   float4* DM4 = reinterpret_cast<float4*>(io.DM);
   float4* DA4 = reinterpret_cast<float4*>(io.DA);
 
-  DN_MARK(1);
   // ---- 1. V_new = U - W S: the product in tensor memory, U taken from its image by the drain
   constexpr uint32_t B_KK = 128 * 128 * 2, B_KV = 128 * VW * 2;     // bytes of a (128,128) / (128,VW) image
   ld.expect(B_KK + 2 * B_KV);
@@ -130,7 +129,6 @@ __device__ __forceinline__ void bwd_gemms_tc(umma::Ctx& cx, uint8_t* img, const 
   });
   __syncthreads();                                // every row of U has been read before dO overwrites Z
 
-  DN_MARK(2);
   // ---- 2. dqe = dO S^T, dM = dO V_new^T
   if (io.qkv_dt == DN_BF16) {
 #pragma unroll
@@ -173,7 +171,6 @@ __device__ __forceinline__ void bwd_gemms_tc(umma::Ctx& cx, uint8_t* img, const 
     for (int i = 0; i < 4; ++i) umma::st_keep4(DM4 + p4v(row, col + 4 * i), make_float4(m[4 * i], m[4 * i + 1], m[4 * i + 2], m[4 * i + 3]));
   });
 
-  DN_MARK(3);
   // ---- 3. dW = -dV S^T (kept only as the operand image of step 5)
   ld.wait();
   umma::pre_issue_sync();
@@ -189,7 +186,6 @@ __device__ __forceinline__ void bwd_gemms_tc(umma::Ctx& cx, uint8_t* img, const 
     P[(col / 8 + 1) * 128 + row] = umma::pack8p(n + 8);
   });
 
-  DN_MARK(4);
   // ---- 4. dke = V_new dH^T
   ld.wait();
   umma::pre_issue_sync();
@@ -202,7 +198,6 @@ __device__ __forceinline__ void bwd_gemms_tc(umma::Ctx& cx, uint8_t* img, const 
     for (int i = 0; i < 4; ++i) umma::st_keep4(DKE4 + p4v(row, col + 4 * i), make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
   });
 
-  DN_MARK(5);
   // ---- 5. dX = T^T dW, dY = T^T dV
   ld.wait();
   umma::pre_issue_sync();
@@ -227,7 +222,6 @@ __device__ __forceinline__ void bwd_gemms_tc(umma::Ctx& cx, uint8_t* img, const 
     X[(col / 8 + 1) * 128 + row] = umma::pack8p(v + 8);
   });
 
-  DN_MARK(6);
   // ---- 6. dA = -(dX W^T + dY U^T), strictly lower and same document
   ld.wait();
   umma::pre_issue_sync();

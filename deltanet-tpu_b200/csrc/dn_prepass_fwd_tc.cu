@@ -81,24 +81,6 @@ __device__ __forceinline__ void drain_am(const umma::Ctx& cx, float* Tp, uint4* 
   umma::tc_fence_before();
 }
 
-// Eight consecutive elements as loaded (bf16: the first vector only); converted where they are used, so that a load
-// can be in flight across a barrier without its converted values taking registers.
-struct Raw8 { uint4 a, b; };
-__device__ __forceinline__ Raw8 ldraw(const uint8_t* row, int p, int dt) {
-  Raw8 r;
-  r.b = make_uint4(0, 0, 0, 0);
-  if (dt == DN_BF16) r.a = __ldg(reinterpret_cast<const uint4*>(row) + p);
-  else { r.a = __ldg(reinterpret_cast<const uint4*>(row) + 2 * p); r.b = __ldg(reinterpret_cast<const uint4*>(row) + 2 * p + 1); }
-  return r;
-}
-__device__ __forceinline__ void cvraw(const Raw8& r, int dt, float (&x)[8]) {
-  if (dt == DN_BF16) umma::unpack8(r.a, x);
-  else {
-    x[0] = __uint_as_float(r.a.x); x[1] = __uint_as_float(r.a.y); x[2] = __uint_as_float(r.a.z); x[3] = __uint_as_float(r.a.w);
-    x[4] = __uint_as_float(r.b.x); x[5] = __uint_as_float(r.b.y); x[6] = __uint_as_float(r.b.z); x[7] = __uint_as_float(r.b.w);
-  }
-}
-
 // L2 requests made by threads 128 .. 511 while the first four warps are in the substitution: this tile's rows of v
 // and w, read right after the inverse, and the next tile's rows of k, q and g / b.  (One line per lane: the bulk form of
 // this request is issued lane by lane, about 80 cycles each, and took longer than what it hid.)
@@ -137,7 +119,7 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
                                                      size_t ibase, int next, int qdt, int gdt, int wC, bool fuse) {
   constexpr int HW = VW < 128 ? VW : 128, NH = VW / HW, NP = HW / 32;
   const Geo& g = a.g;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x;
   const int x = row_of(tid), lgrp = piece_of(tid);
   float* Tp = reinterpret_cast<float*>(sm + OFF_T);
   uint4* XI = reinterpret_cast<uint4*>(sm + OFF_X);
@@ -824,7 +806,9 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
     const bool ok0 = group_wait(0), ok1 = group_wait(1);
     if (__syncthreads_or(!(ok0 && ok1))) { cx.dead = true; umma::report_timeout(err); }
     umma::tc_fence_after();
-    if (__syncthreads_or(strong)) {
+    const bool any_strong = __syncthreads_or(strong);
+    if (a.res.T && tid == 0) *strong_flag_ptr(a.res, ibase) = any_strong;        // the backward takes the same route
+    if (any_strong) {
       umma::Ctx c2 = cx;
       strong_route<MODE>(a, b, h, t0, ibase, rq_s, rk_s, seg_s, rst_s, sm, c2);
       cx.phase = c2.phase;
