@@ -59,7 +59,7 @@ int overlap_cut(const Geo& g) {
   const int cut = ((rounds - 1) * sms) / per_chunk;
   return (cut >= 1 && cut < g.NC) ? cut : 0;
 }
-size_t carry_bytes(const Geo& g) { return align_up((size_t)g.B * g.H * g.K * g.Vw * sizeof(float)); }
+size_t carry_bytes(const Geo& g) { return align_up((size_t)g.B * g.H * g.Kt * g.Vw * sizeof(float)); }
 }  // namespace
 
 extern "C" {
@@ -98,14 +98,14 @@ int dn_exec_view(const dn_shape* s, dn_exec* out) {
 static void residual_sizes(const Geo& g, size_t sz[8]) {
   const size_t n = (size_t)g.B * g.H * g.NC, ps = dt_size(g.pre_dt);
   const bool keep = !(g.flags & DN_INFERENCE);
-  sz[0] = n * g.C * g.K * ps;
+  sz[0] = n * g.C * g.Kt * ps;
   sz[1] = n * g.C * g.Vw * ps;
   sz[2] = n * g.C * g.C * ps;
   sz[3] = sz[0];
   sz[4] = sz[0];
-  sz[5] = n * g.K * sizeof(float);
+  sz[5] = n * g.Kt * sizeof(float);
   sz[6] = keep ? n * g.C * g.C * sizeof(float) : 0;
-  sz[7] = keep ? n * g.K * g.Vw * (g.img ? 2 : sizeof(float)) : 0;            // image path: a bf16 operand image (states_img)
+  sz[7] = keep ? n * g.Kt * g.Vw * (g.img ? 2 : sizeof(float)) : 0;            // image path: a bf16 operand image (states_img)
 }
 
 size_t dn_residual_bytes(const dn_shape* s) {
@@ -168,7 +168,7 @@ size_t dn_scratch_bytes(const dn_shape* s, int for_backward, int recompute) {
   }
   size_t tot = bwd_kernel_scratch(g) > fwd_kernel_scratch(g) ? bwd_kernel_scratch(g) : fwd_kernel_scratch(g);
   tot += align_up(n * g.C * g.Vw * sizeof(float));   // dV
-  tot += align_up(n * g.K * g.Vw * sizeof(float));   // dH
+  tot += align_up(n * g.Kt * g.Vw * sizeof(float));   // dH
   tot += staging_bytes(g);
   tot += carry_bytes(g);
   if (recompute) tot += align_up(full_residual_bytes(s));
@@ -397,7 +397,7 @@ int dn_chunk_bwd(const dn_shape* s, const void* q, const void* k, const void* v,
   const size_t n = (size_t)g.B * g.H * g.NC;
   auto take = [&](size_t bytes) { char* r = p; p += align_up(bytes); return r; };
   float* dV = reinterpret_cast<float*>(take(n * g.C * g.Vw * sizeof(float)));
-  float* dH = reinterpret_cast<float*>(take(n * g.K * g.Vw * sizeof(float)));
+  float* dH = reinterpret_cast<float*>(take(n * g.Kt * g.Vw * sizeof(float)));
   if (p > end) return DN_ERR_SCRATCH_TOO_SMALL;
   dn_residuals local;
   if (!res) {
@@ -460,7 +460,7 @@ int dn_sp_transition(const dn_shape* s, const dn_residuals* res, const int32_t* 
   if (peek_device_error()) return DN_ERR_DEVICE_WAIT;
   if (!res || !identity || !P) return DN_ERR_NULL_POINTER;
   Geo t = g;                       // same chunks and heads, value width K, one "value head" per exec head
-  t.Hv = g.H; t.G = 1; t.V = g.K; t.Vw = g.K; t.qk_div = 1;
+  t.Hv = g.H; t.G = 1; t.V = g.K; t.Vw = g.Kt; t.qk_div = 1;
   t.flags |= DN_HAS_INIT;
   StateArgs a{};
   a.g = t; a.res = *res; a.res.U = nullptr; a.res.states = nullptr; a.seg = seg;

@@ -21,7 +21,8 @@ int sm_count();
 // Everything a kernel needs to know about where a (batch, exec head, chunk) lives.
 struct Geo {
   int B, L, Hk, Hv, K, V, C, NC;
-  int H, Vw, G;          // exec heads, value width, value heads per exec head
+  int H, Vw, G;          // exec heads, value width of the tiles, value heads per exec head (G V columns of Vw exist)
+  int Kt;                // key width of the tiles: 128 on the tensor-core path (K columns exist), else K
   int qk_div;            // q/k head of exec head h is h / qk_div
   int gH, gC, bH, bC, wH, wC;
   int qkv_dt, gate_dt, pre_dt, prec;
@@ -62,44 +63,45 @@ inline int make_geo(const dn_shape* s, Geo* g) {
   if (s->precision != DN_PREC_FP32 && s->precision != DN_PREC_BF16) return DN_ERR_BAD_DTYPE;
   g->B = s->B; g->L = s->L; g->Hk = s->Hk; g->Hv = s->Hv; g->K = s->K; g->V = s->V;
   bool at_hv = (s->Hk < s->Hv) && (s->g_heads == s->Hv || s->b_heads == s->Hv);
-  // More than two value heads per key head would make a tile wider than the tensor-core kernels take
-  // (G V > 256): such calls use the per-value-head view too (the key-side work is repeated per value head,
-  // the key-side gradients are summed over the group as for gates given per value head).
-  if (s->Hk < s->Hv && s->precision == DN_PREC_BF16 && !(s->flags & DN_STATE_FP32_MM) && s->K == 128 && s->V == 128 &&
-      (s->Hv / s->Hk) * s->V > 256 && !force_simt())
-    at_hv = true;
+  // More than 256 value columns per key head would make a tile wider than the tensor-core kernels take: such calls
+  // use the per-value-head view too (the key-side work is repeated per value head, the key-side gradients are
+  // summed over the group as for gates given per value head).
+  const bool tc = s->precision == DN_PREC_BF16 && !(s->flags & DN_STATE_FP32_MM) && !force_simt();
+  if (tc && s->Hk < s->Hv && (s->Hv / s->Hk) * s->V > 256) at_hv = true;
   if (at_hv) { g->H = s->Hv; g->Vw = s->V; g->G = 1; g->qk_div = s->Hv / s->Hk; }
   else       { g->H = s->Hk; g->G = s->Hv / s->Hk; g->Vw = g->G * s->V; g->qk_div = 1; }
   if (g->Vw > 1024) return DN_ERR_BAD_SHAPE;
-  // Rows per tile.  The tensor-core kernels work on 128-row tiles (the M of a tcgen05.mma), so in
-  // bf16 precision a request for chunk 64 is run with two requested chunks merged into one tile:
-  // the chunked form is an exact regrouping of the token recurrence, results differ only in where
-  // the state is rounded to bf16 (every 128 tokens instead of every 64).  dn_exec_view reports the
-  // tile height actually used; every buffer size follows from it.
-  const bool tc_shape = s->precision == DN_PREC_BF16 && !(s->flags & DN_STATE_FP32_MM) && s->K == 128 &&
-                        (g->Vw == 128 || g->Vw == 256) && !force_simt();
-  g->C = (tc_shape && s->chunk == 64) ? 128 : s->chunk;
+  // The tensor-core kernels work on tiles of 128 rows (the M of a tcgen05.mma), 128 key columns and 128 or 256 value
+  // columns.  In bf16 precision a request for chunk 64 is run with two requested chunks merged into one tile: the
+  // chunked form is an exact regrouping of the token recurrence, results differ only in where the state is
+  // rounded to bf16 (every 128 tokens instead of every 64).  Narrower heads (K or V = 64) are run in the same
+  // tiles with the missing columns zero: even at K = V = 64 with one value head, where three quarters of the products are
+  // zeros, that is several times faster than the CUDA-core kernels.  dn_exec_view reports the tile height and value
+  // width actually used; every buffer size follows from them.
+  g->C = tc ? 128 : s->chunk;
+  g->Kt = tc ? 128 : s->K;
+  if (tc) g->Vw = g->Vw <= 128 ? 128 : 256;
   g->NC = (s->L + g->C - 1) / g->C;
   g->gH = s->g_heads; g->gC = s->g_cols; g->bH = s->b_heads; g->bC = s->b_cols;
   g->wH = s->w_heads; g->wC = s->w_cols;
   g->qkv_dt = s->qkv_dtype; g->gate_dt = s->gate_dtype; g->prec = s->precision;
   g->pre_dt = s->precision == DN_PREC_BF16 ? DN_BF16 : DN_F32;
   g->flags = s->flags; g->scale = s->scale;
-  g->img = tc_shape;
+  g->img = tc;
   return DN_OK;
 }
 
 // On the image path three more arrays are kept as bf16 operand images, [col / 8][128 rows][8]:
 //   * the chunk-entry states (the only copy on this path: the `states` slot holds the image): states_img();
 //   * T, in the first half of its fp32-sized slot;
-//   * dV and dH, in the first half of their fp32-sized buffers; the second half of the dH buffer
-//     carries the partial sums of dLambda_end, (item, column slice of 32, K) fp32: dlend_part().
+//   * dV and dH, in the first half of their fp32-sized buffers (dH: all of it when K = 64); the second half of the dV
+//     buffer carries the partial sums of dLambda_end, (item, column slice of 32, 128) fp32: dlend_part().
 __host__ __device__ __forceinline__ const __nv_bfloat16* states_img(const Geo& g, const float* states) {
   (void)g;
   return reinterpret_cast<const __nv_bfloat16*>(states);
 }
-__host__ __device__ __forceinline__ float* dlend_part(const Geo& g, float* dH) {
-  return dH + (size_t)g.B * g.H * g.NC * g.K * g.Vw / 2;
+__host__ __device__ __forceinline__ float* dlend_part(const Geo& g, float* dV) {
+  return dV + (size_t)g.B * g.H * g.NC * 128 * g.Vw / 2;
 }
 
 // T's slot holds a bf16 image in its first half; the first word of the second half tells the backward that the decay of

@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       seg_s[tid] = sg;
       // dLambda_end = [one document] e^{Lambda_end} sum_v dH S (gdn2.py:759-762) from the reverse chain's per-slice sums
       float acc = 0.f;
-      const float* part = dlend_part(g, const_cast<float*>(a.dH)) + ibase * (VW / 32) * K + tid;
+      const float* part = dlend_part(g, const_cast<float*>(a.dV)) + ibase * (VW / 32) * K + tid;
       for (int s2 = 0; s2 < VW / 32; ++s2) acc += __ldg(part + s2 * K);
       dlend_s[tid] = all_same ? acc * expf(fminf(__ldg(a.res.lam_end + ibase * K + tid), 0.f)) : 0.f;
       if (SC) {                                         // decay and erase gate: one row per thread, document-restarting scan
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       umma::issue_pitched<128, false, false>(cx, sl.at(5), PB, sl.at(1), 2048, 128, T_Q, false);
       commit(cx);
       umma::commit_wait_cta(cx);
-      stage_dO(sl.at(5), a.d_out, dO_off + 128, dO_pitch, rows, 16, qdt);
+      stage_dO(sl.at(5), a.d_out, dO_off + 128, dO_pitch, rows, vr / 8 - 16, qdt);
       sl.wait(0);
       umma::issue<128, false, false>(cx, sl.at(0), sl.at(1), 128, T_B, false);                     // -dW: first half
       commit(cx);

@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
     const Rows r = make_rows<CF>(g, a.q, a.k, a.gg, a.b, b, h, t0, rq_s, rk_s);
     const int qdt = r.qkv_dt, gdt = r.gate_dt;           // compile-time constants in the fixed modes
     const int wC = CF::fixed ? (CF::scalar_bw ? 1 : g.V) : g.wC;
+    const int vr = g.G * g.V;                            // value columns that exist
     const bool tm_cache = r.round_in;                    // k_hat, q_hat exactly bf16: they can be packed two per column
 
     // staging rows of phase V (headline mode): v as bf16 and w as fp32, one row per token, padded pitches
@@ -201,10 +202,11 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
       io.dV = reinterpret_cast<const __nv_bfloat16*>(a.dV) + ibase * CV;
       io.T = reinterpret_cast<const __nv_bfloat16*>(a.res.T + ibase * CC);
       io.slices = VW / 32;
-      io.dlend_part = dlend_part(g, const_cast<float*>(a.dH)) + ibase * (VW / 32) * K;
+      io.dlend_part = dlend_part(g, const_cast<float*>(a.dV)) + ibase * (VW / 32) * K;
       io.lam_end = a.res.lam_end + ibase * K;
       io.d_out = a.d_out; io.qkv_dt = CF::fixed ? CF::qkv_dt : g.qkv_dt;
-      io.dO_off = ((size_t)b * g.L + t0) * g.Hv * g.V + (size_t)h * VW;
+      io.dO_off = ((size_t)b * g.L + t0) * g.Hv * g.V + (size_t)h * vr;
+      io.dO_pieces = vr / 8;
       io.dO_pitch = (size_t)g.Hv * g.V;
       io.rows_valid = g.L - t0 < C ? g.L - t0 : C;
       io.DQE = DQE; io.DKE = DKE; io.DX = DX; io.DM = DM; io.DA = DA;
@@ -272,7 +274,8 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
 #pragma unroll 4
       for (int it = 0; it < PV / 4; ++it) {
         const int p = it * 4 + lgrp;
-        const int col0 = h * VW + 8 * p, hv = col0 / g.V, cv = col0 - hv * g.V;
+        if (32 * it >= vr) break;
+        const int col0 = h * vr + 8 * p, hv = col0 / g.V, cv = col0 - hv * g.V;
         float vv[8], ww[8], dy[8], dv8[8], dw8[8];
         load8(a.v, tokr * g.Hv * g.V + col0, qdt, vv);
         if (wC == 1) {
@@ -535,7 +538,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
       const float rq = rq_s[x], rk = rk_s[x];
       const size_t tok = (size_t)b * g.L + t;
       const size_t outb = (tok * g.H + h) * r.bC;
-      const size_t outqk = (tok * g.H + h) * K;
+      const size_t outqk = (tok * g.H + h) * g.K;
       float dq_dot = 0.f, dk_dot = 0.f, sb2 = 0.f;
 #pragma unroll 1
       for (int it = 0; it < 4; ++it) {
@@ -544,7 +547,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
         raw_q8(r, x, p, qr);
         raw_k8(r, x, p, kr);
         bact8(r, x, p, ba);
-        if (!fuse && guard) raw_gate8(r.b, r.b_row0, r.b_pitch, r.bC, r.gate_dt, live ? x : 0, p, braw);
+        if (!fuse && guard) raw_gate8(r.b, r.b_row0, r.b_pitch, r.bC, r.gate_dt, live ? x : 0, p < r.kp ? p : 0, braw);
           ld2x4(DBP4 + p4v(x, 8 * p), dbp);
           ld2x4(DQP4 + p4v(x, 8 * p), dqp);
           ld2x4(DKP4 + p4v(x, 8 * p), dkp);
@@ -589,7 +592,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
         *reinterpret_cast<float4*>(DLs + x * LP + 8 * p + 4) = make_float4(odl[4], odl[5], odl[6], odl[7]);
         *reinterpret_cast<float4*>(DKs + x * LP + 8 * p) = make_float4(odk[0], odk[1], odk[2], odk[3]);
         *reinterpret_cast<float4*>(DKs + x * LP + 8 * p + 4) = make_float4(odk[4], odk[5], odk[6], odk[7]);
-        if (live && r.bC != 1) out8(a.db, outb + 8 * p, a.db_dt, odb);
+        if (live && r.bC != 1 && p < r.kp) out8(a.db, outb + 8 * p, a.db_dt, odb);
       }
       // the four channel groups of a row meet here (added in a fixed order)
       TOT[fg * 128 + x] = dq_dot;
@@ -616,7 +619,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
             dkn[i] = rk * (dkn[i] - kn[i] * dk_dot);
           }
         }
-        if (live) {
+        if (live && p < r.kp) {
           out8(a.dq, outqk + 8 * p, a.dq_dt, dqn);
           out8(a.dk, outqk + 8 * p, a.dq_dt, dkn);
         }
@@ -673,15 +676,17 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
         const int t = live ? t0 + i : t0;              // a row past the end reads row 0 and writes nothing
         const size_t tok = (size_t)b * g.L + t;
         const size_t rowg = (tok * g.gH + hg) * r.gC, outg = (tok * g.H + h) * r.gC;
+        const bool cin = 4 * lane < 8 * r.kp;          // the lane's channels exist
+        const int gc = cin ? 4 * lane : 0;
         const float4 dl = *reinterpret_cast<const float4*>(DLs + i * LP + 4 * lane);
         float dgv[4] = {dl.x, dl.y, dl.z, dl.w}, gr[4];
         if (r.gC == 1) { gr[0] = gr[1] = gr[2] = gr[3] = ldf_ro(a.gg, rowg, gdt); }
         else if (gdt == DN_BF16) {
-          const uint2 u = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(a.gg) + rowg + 4 * lane));
+          const uint2 u = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(a.gg) + rowg + gc));
           gr[0] = __uint_as_float(u.x << 16); gr[1] = __uint_as_float(u.x & 0xffff0000u);
           gr[2] = __uint_as_float(u.y << 16); gr[3] = __uint_as_float(u.y & 0xffff0000u);
         } else {
-          const float4 u = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.gg) + rowg + 4 * lane));
+          const float4 u = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.gg) + rowg + gc));
           gr[0] = u.x; gr[1] = u.y; gr[2] = u.z; gr[3] = u.w;
         }
         float sg = 0.f;
@@ -697,7 +702,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
           sg += dgv[u];
         }
         if (r.gC == 1) { sg = warp_sum(sg); if (lane == 0 && live) stf(a.dg, outg, sg, a.dg_dt); }
-        else if (!live) { }
+        else if (!live || !cin) { }
         else if (a.dg_dt == DN_BF16)
           *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(a.dg) + outg + 4 * lane) = make_uint2(umma::pack2(dgv[0], dgv[1]), umma::pack2(dgv[2], dgv[3]));
         else

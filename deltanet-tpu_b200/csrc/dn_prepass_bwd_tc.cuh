@@ -44,6 +44,7 @@ struct BwdTcIo {
   int qkv_dt;
   size_t dO_off;                       // element offset of (row 0, column 0) of this item's dO block
   size_t dO_pitch;                     // elements between token rows
+  int dO_pieces;                       // 8-column pieces that exist (others read as 0)
   int rows_valid;                      // rows of the chunk that exist (others read as 0)
   float *DQE, *DKE, *DX, *DM, *DA;       // fp32 results in scratch, panel layout
   float* dlend_s;                      // out (shared, 128): [one doc] exp(lam_end) * sum_v dH * S
@@ -135,7 +136,7 @@ __device__ __forceinline__ void bwd_gemms_tc(umma::Ctx& cx, uint8_t* img, const 
     for (int it = 0; it < PV * 128 / NT; ++it) {
       int p, x;
       stage_coords<128>(it * NT + threadIdx.x, p, x);
-      if (x < io.rows_valid)
+      if (x < io.rows_valid && p < io.dO_pieces)
         umma::cp_async16(Z + p * 128 + x, reinterpret_cast<const __nv_bfloat16*>(io.d_out) + io.dO_off + (size_t)x * io.dO_pitch + 8 * p);
       else
         Z[p * 128 + x] = make_uint4(0, 0, 0, 0);
@@ -147,8 +148,8 @@ __device__ __forceinline__ void bwd_gemms_tc(umma::Ctx& cx, uint8_t* img, const 
     for (int it = 0; it < PV * 128 / NT; ++it) {
       int p, x;
       stage_coords<128>(it * NT + threadIdx.x, p, x);
-      const bool live = x < io.rows_valid;
-      uint4 val = umma::ld8_f32_ro(reinterpret_cast<const float*>(io.d_out) + io.dO_off + (size_t)(live ? x : 0) * io.dO_pitch + 8 * p);
+      const bool live = x < io.rows_valid && p < io.dO_pieces;
+      uint4 val = umma::ld8_f32_ro(reinterpret_cast<const float*>(io.d_out) + io.dO_off + (live ? (size_t)x * io.dO_pitch + 8 * p : 0));
       if (!live) val = make_uint4(0, 0, 0, 0);
       Z[p * 128 + x] = val;
     }

@@ -88,17 +88,16 @@ __device__ __forceinline__ void prefetch_row(const void* p, uint32_t bytes) {
   for (uint32_t o = 0; o < bytes; o += 128)
     asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t*>(p) + o));
 }
-template <int VW>
 __device__ __forceinline__ void prefetch_rows(const PrepassFwdArgs& a, int h, int b, int t0, int next, int wC) {
   const Geo& g = a.g;
-  const int x = threadIdx.x & 127, part = threadIdx.x >> 7;
+  const int x = threadIdx.x & 127, part = threadIdx.x >> 7, vr = g.G * g.V;
   const uint32_t qe = (uint32_t)dt_size(g.qkv_dt), ge = (uint32_t)dt_size(g.gate_dt);
   if (part < 3) {
     if (t0 + x < g.L) {
       const size_t tok = (size_t)b * g.L + t0 + x;
-      if (part == 1) prefetch_row(reinterpret_cast<const uint8_t*>(a.v) + (tok * g.Hv * g.V + (size_t)h * VW) * qe, VW * qe);
+      if (part == 1) prefetch_row(reinterpret_cast<const uint8_t*>(a.v) + (tok * g.Hv * g.V + (size_t)h * vr) * qe, vr * qe);
       else if (wC == g.V && g.wH == g.Hv)
-        prefetch_row(reinterpret_cast<const uint8_t*>(a.w) + (tok * g.Hv * g.V + (size_t)h * VW) * ge, VW * ge);
+        prefetch_row(reinterpret_cast<const uint8_t*>(a.w) + (tok * g.Hv * g.V + (size_t)h * vr) * ge, vr * ge);
     }
   } else if (next < a.items) {
     const int bh = next % (g.B * g.H), t = (a.c_begin + next / (g.B * g.H)) * C + x;
@@ -114,7 +113,7 @@ __device__ __forceinline__ void prefetch_rows(const PrepassFwdArgs& a, int h, in
 }
 
 // T = (I + A)^-1, then W = T X and U = T (w v).  X image and A visible to all threads on entry.
-template <int VW>
+template <int VW, bool PREFETCH>
 __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm, const PrepassFwdArgs& a, int h, int b, int t0,
                                                      size_t ibase, int next, int qdt, int gdt, int wC, bool fuse) {
   constexpr int HW = VW < 128 ? VW : 128, NH = VW / HW, NP = HW / 32;
@@ -127,21 +126,23 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
   uint4* Y0 = reinterpret_cast<uint4*>(sm + OFF_T);
   uint4* Wimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.W) + ibase * C * K);
   uint4* Uimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.U) + ibase * C * VW);
+  const int vr = g.G * g.V;                             // value columns that exist
   const bool live = t0 + x < g.L;
   const size_t tokr = (size_t)b * g.L + (live ? t0 + x : t0);
-  const uint8_t* vrow = reinterpret_cast<const uint8_t*>(a.v) + (tokr * g.Hv * g.V + (size_t)h * VW) * dt_size(qdt);
-  uint4 vr[NP];                                         // a half's pieces of v (bf16), requested ahead of use
+  const uint8_t* vrow = reinterpret_cast<const uint8_t*>(a.v) + (tokr * g.Hv * g.V + (size_t)h * vr) * dt_size(qdt);
+  uint4 vraw[NP];                                         // a half's pieces of v (bf16), requested ahead of use
   auto request_v = [&](int half) {
     if (qdt == DN_BF16) {
 #pragma unroll
-      for (int it = 0; it < NP; ++it) vr[it] = __ldg(reinterpret_cast<const uint4*>(vrow) + half * (HW / 8) + it * 4 + lgrp);
+      for (int it = 0; it < NP; ++it) vraw[it] = half * HW + 32 * it < vr ? __ldg(reinterpret_cast<const uint4*>(vrow) + half * (HW / 8) + it * 4 + lgrp) : make_uint4(0, 0, 0, 0);
     }
   };
   auto build_y = [&](uint4* Y, int half) {              // Y = w v of the half's columns
 #pragma unroll
     for (int it = 0; it < NP; ++it) {
       const int p = it * 4 + lgrp;
-      const int col0 = half * HW + 8 * p, hv = (h * VW + col0) / g.V, cv = h * VW + col0 - hv * g.V;
+      const int col0 = half * HW + 8 * p, hv = (h * vr + col0) / g.V, cv = h * vr + col0 - hv * g.V;
+      if (col0 - 8 * lgrp >= vr) { Y[p * PP + x] = make_uint4(0, 0, 0, 0); continue; }
       float vv[8], ww[8];
       if (wC == 1) {
         const float w1 = ldf_ro(a.w, tokr * g.wH + g.w_head(hv), gdt);
@@ -150,14 +151,18 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
       } else {
         load8(a.w, (tokr * g.wH + g.w_head(hv)) * wC + cv, gdt, ww);
       }
-      if (qdt == DN_BF16) umma::unpack8(vr[it], vv);
+      if (qdt == DN_BF16) umma::unpack8(vraw[it], vv);
       else { const Raw8 r = ldraw(vrow, half * (HW / 8) + p, qdt); cvraw(r, qdt, vv); }
 #pragma unroll
       for (int i = 0; i < 8; ++i) vv[i] = live ? (fuse ? sigmoid_fast(ww[i]) : ww[i]) * vv[i] : 0.f;
       Y[p * PP + x] = umma::pack8(vv);
     }
   };
-  tri::invert(Tp, reinterpret_cast<float*>(TI), [&]() { prefetch_rows<VW>(a, h, b, t0, next, wC); });
+  tri::invert(Tp, reinterpret_cast<float*>(TI), [&]() {
+    // (scalar gates: 779 -> 741 us at B=4 L=8192 Hv=32.  With decay per channel the requests cost more than they hide,
+    // 761 -> 819 us at L=20011: that kernel reads q, k, b, g in groups and has other tiles to switch to.)
+    if (PREFETCH) prefetch_rows(a, h, b, t0, next, wC);
+  });
   request_v(0);
   tri::image(Tp, TI);
   __syncthreads();                                      // T has been read: its place takes Y
@@ -364,7 +369,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_scalar_kernel(const __grid_
       });
     }
     __syncthreads();
-    inverse_and_products<VW>(cx, sm, a, h, b, t0, ibase, e_item + gridDim.x, DN_BF16, g.gate_dt, g.wC, false);
+    inverse_and_products<VW, true>(cx, sm, a, h, b, t0, ibase, e_item + gridDim.x, DN_BF16, g.gate_dt, g.wC, false);
   }
   teardown(tbase);
 }
@@ -826,7 +831,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       });
       __syncthreads();
     }
-    inverse_and_products<VW>(cx, sm, a, h, b, t0, ibase, e_item + gridDim.x, qdt, gdt, wC, fuse);
+    inverse_and_products<VW, false>(cx, sm, a, h, b, t0, ibase, e_item + gridDim.x, qdt, gdt, wC, fuse);
   }
   teardown(tbase);
 }

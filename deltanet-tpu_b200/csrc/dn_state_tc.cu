@@ -1,20 +1,24 @@
-// Inter-chunk recurrence on the tcgen05 tensor cores (bf16 precision, chunk = K = 128).
+// Inter-chunk recurrence on the tcgen05 tensor cores (bf16 precision, 128-row tiles).
 //
-// Same math and same CTA decomposition as the fp32 formulation in dn_state.cu: one CTA carries
-// a (128 x VS) column slice of the state of one (batch, exec head) through all chunks.  Here
-//   * the fp32 master copy of the slice lives in registers, one state row per thread
-//     (128 threads), and a bf16 copy in shared memory is the MMA operand -- the reference rounds
-//     the state to bf16 for these products as well (src/deltanet_tpu/gdn2.py:627-632);
-//   * the four 128x128 bf16 tiles of a chunk (W, qe, M, ke) are operand images in global memory and
-//     arrive one chunk ahead by one bulk copy each (mbarrier completion), each buffer refilled as
-//     soon as the MMA reading it has completed (row-major tiles of the fp32-residual layout: 16-byte
-//     cp.async copies); passes that need no outputs fetch W and ke only;
-//   * every product is a 128 x VS x 128 tcgen05.mma with the accumulator in tensor memory,
-//     read back one row per thread.  A 128x128 tile image in shared memory serves both as the
-//     operand (K-major descriptor) and as its transpose (MN-major descriptor), so ke^T, M^T,
-//     qe^T and W^T need no data movement.
-// Every wait on the MMA barrier is bounded; on a timeout the CTA stops issuing tensor work,
+// Same math as the fp32 formulation in dn_state.cu (reference: src/deltanet_tpu/gdn2.py:585-769): one CTA carries a
+// (128 x VS) column slice of the state of one (batch, exec head) through all chunks.  A chunk step is two dependent
+// products with a drain of tensor memory behind each,
+//     forward:  P = W S;  V = U - P;   S' = dec S + ke^T V          (off the chain: O = qe S + M V)
+//     reverse:  dV = M^T dO + ke dH;   dH' = dec dH + qe^T dO - W^T dV
+// and nothing else belongs on the serial path.  So the CTA is specialised by warp:
+//   * state warps (row of the state per lane, 32 columns per warp) hold the fp32 master in registers, turn
+//     accumulators into bf16 operands in shared memory and touch global memory only before and after the walk;
+//   * one thread issues every product, in an order that puts the products off the chain into the time in
+//     which the state warps drain;
+//   * one thread streams the chunk's tiles (W, qe, ke, M: operand images of 32 KB) through a ring of slots in the
+//     order of use, one brings the rows (U or the entry state, and Lambda_end), one stores what the
+//     state warps staged (entry states; dH, dV and the partial sums of dLambda_end), all by bulk copies;
+//   * four warps write the outputs from a second accumulator, or stage dO ahead (reverse).
+// Every hand-over is an mbarrier with one phase per use of the buffer it guards, so that no barrier can run two
+// phases ahead of a slow waiter.  Every wait is bounded; after one that gave up a thread skips the rest of its waits,
 // raises the library's error word and runs to its end.
+//
+// With narrow heads (K = 64 or value width 64) rows and columns past the end are zeros.
 #include "dn_kernels.cuh"
 #include "dn_umma.cuh"
 
@@ -22,581 +26,682 @@ namespace dn {
 
 namespace {
 
-constexpr int TILE_U4 = 128 * 16;   // a 128x128 bf16 tile in 16-byte units
+constexpr uint32_t TILE_B = 32768;                    // a 128 x 128 bf16 operand image
+constexpr int C = 128, KT = 128;
 
-__device__ __forceinline__ size_t native_state_index_tc(const Geo& g, int b, int h, int k, int jj) {
-  const int hv = h * g.G + jj / g.V, cv = jj % g.V;
-  return (((size_t)b * g.Hv + hv) * g.K + k) * g.V + cv;
+template <int VS, bool BWD>
+struct Plan {
+  static constexpr int NG = VS / 32;                  // state warps: 4 NG
+  static constexpr int ST = 128 * NG;                 // state threads; then 128 threads for O / dO; then four single-thread roles
+  static constexpr int NT = ST + 128 + 128;
+  static constexpr uint32_t SL = VS * 256;            // bytes of a (128 x VS) operand
+  static constexpr int DO_BUF = 2;                    // reverse: copies of dO
+  static constexpr int ROWS = BWD ? 2 : 3;            // buffers of the row loader
+  // forward: S, V (U arrives in V's place); reverse: dO, dH, dV, S rows
+  static constexpr int OPS = BWD ? DO_BUF + 2 + ROWS : 1 + ROWS;
+  static constexpr int SLOTS = VS == 32 ? (BWD ? 5 : 6) : (BWD ? 4 : 5);
+  static constexpr uint32_t SMEM = SLOTS * TILE_B + OPS * SL + ROWS * 512 + (BWD ? NG * 512 : 0);
+  static constexpr uint32_t TMEM = 4 * VS;
+  static_assert(SMEM + 512 <= 227 * 1024, "shared memory, with the static arrays");
+};
+
+__device__ __forceinline__ void arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smem_u32(bar)) : "memory");
 }
-
-// Thread `row` copies its share of a (128,128) bf16 tile into the panel image: its 256-byte row of
-// a row-major tile, or (img) piece `row` of each of the 16 panels of a tile that already lies in
-// global memory as the image -- then a warp's 32 copies are 512 contiguous bytes.
-__device__ __forceinline__ void copy_tile_async(uint4* dst, const __nv_bfloat16* src, int row, bool img) {
-  if (img) {
-    const uint4* s = reinterpret_cast<const uint4*>(src) + row;
+// one arrival per warp, behind the shared-memory and tensor-memory accesses of all its lanes
+__device__ __forceinline__ void warp_arrive(uint64_t* bar) {
+  umma::fence_async_smem();
+  umma::tc_fence_before();
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) arrive(bar);
+}
+struct Waiter {
+  int* err;
+  bool dead;
+  __device__ __forceinline__ void operator()(uint64_t* bar, uint32_t parity) {
+    if (dead) return;
+    if (!umma::mbar_wait(bar, parity)) { dead = true; umma::report_timeout(err); }
+  }
+};
+// D[128 x N] (+)= A B over a contraction of 128, by a converged warp; operands are images of 128-row panels
+template <bool MN>
+__device__ __forceinline__ uint64_t operand(const void* p) {
+  return umma::smem_desc(umma::smem_u32(p), MN ? 128u : 2048u, MN ? 2048u : 128u);
+}
+template <int N, bool A_MN, bool B_MN>
+__device__ __forceinline__ void product(uint32_t d, uint64_t ad, uint64_t bd, bool accumulate) {
+  constexpr uint32_t idesc = umma::instr_desc(N, A_MN ? 1 : 0, B_MN ? 1 : 0);
 #pragma unroll
-    for (int p = 0; p < 16; ++p) umma::cp_async16(dst + p * 128 + row, s + p * 128);
+  for (int k = 0; k < 8; ++k) {
+    umma::mma_bf16_warp(d, ad, bd, idesc, (accumulate || k > 0) ? 1u : 0u);
+    ad += (A_MN ? 256u : 4096u) >> 4;
+    bd += (B_MN ? 256u : 4096u) >> 4;
+  }
+}
+// Position in a ring of N buffers: index and the parity of the current use
+template <int N>
+struct Ring {
+  uint32_t at = 0, parity = 0;
+  __device__ __forceinline__ void next() {
+    if (++at == N) { at = 0; parity ^= 1u; }
+  }
+};
+__device__ __forceinline__ void ld32(bool dead, uint32_t addr, float (&v)[32]) {
+  if (!dead) {
+    umma::tmem_ld32_nowait(addr, v);
+    umma::tmem_wait_ld();
   } else {
-    const uint4* s = reinterpret_cast<const uint4*>(src + (size_t)row * 128);
 #pragma unroll
-    for (int p = 0; p < 16; ++p) umma::cp_async16(dst + p * 128 + row, s + p);
+    for (int i = 0; i < 32; ++i) v[i] = 0.f;
   }
 }
-
-// A (128,128) bf16 tile that lies in global memory as its operand image: one bulk copy, issued by
-// one thread, completion counted on an mbarrier (image layout only).
-__device__ __forceinline__ void bulk_tile(uint4* dst, const __nv_bfloat16* src, uint64_t* bar) {
-  umma::bulk_load(dst, src, TILE_U4 * 16, bar);
+__device__ __forceinline__ void image32(uint4* img, int row, const float (&v)[32]) {
+#pragma unroll
+  for (int p = 0; p < 4; ++p) img[p * 128 + row] = umma::pack8p(v + 8 * p);
 }
 
-template <int VS>
-__device__ __forceinline__ void stage_rows(uint4* dst, int row, const float (&x)[VS], float sign = 1.f) {
-#pragma unroll
-  for (int p = 0; p < VS / 8; ++p) {
-    float t[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) t[i] = sign * x[p * 8 + i];
-    dst[p * 128 + row] = umma::pack8(t);
+// Document flags of the chunks a chain walks, 32 at a time as bit masks a warp keeps in registers: bit i is chunk
+// top + dir * i.  (is_new: the chunk starts a document; all_same: the chunk is one document.)
+struct Flags {
+  uint32_t is_new, all_same;
+  __device__ __forceinline__ void fill(const int32_t* seg, const Geo& g, int b, int top, int dir, int lo, int hi) {
+    const int c = top + dir * (int)(threadIdx.x & 31);
+    bool n = false, s = false;
+    if (c >= lo && c < hi) chunk_flags(seg, g, b, c, n, s);
+    is_new = __ballot_sync(0xffffffffu, n);
+    all_same = __ballot_sync(0xffffffffu, s);
   }
+  __device__ __forceinline__ void next() { is_new >>= 1; all_same >>= 1; }
+};
+// 32 columns of one row of a native (B, Hv, K, V) state: offset, or none where the row or the columns do not exist
+__device__ __forceinline__ bool native_row(const Geo& g, int b, int h, int k, int col, size_t& off) {
+  off = (((size_t)b * g.Hv + h * g.G + col / g.V) * g.K + k) * g.V + col % g.V;
+  return k < g.K && col < g.G * g.V;
 }
-
-// issue the loads of one accumulator row (VS columns) without waiting; read_wait() before use
-template <int VS>
-__device__ __forceinline__ void read_acc_nowait(const umma::Ctx& cx, uint32_t col, int warp, float (&x)[VS]) {
-  if (!cx.dead) {
+__device__ __forceinline__ void load32(const float* p, float (&v)[32]) {
+  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
 #pragma unroll
-    for (int c = 0; c < VS; c += 32) umma::tmem_ld32_nowait(cx.tmem + ((uint32_t)(warp * 32) << 16) + col + c, x + c);
-  } else {
-#pragma unroll
-    for (int i = 0; i < VS; ++i) x[i] = 0.f;
-  }
-}
-__device__ __forceinline__ void read_wait(const umma::Ctx& cx) { if (!cx.dead) umma::tmem_wait_ld(); }
-template <int VS>
-__device__ __forceinline__ void read_acc(const umma::Ctx& cx, uint32_t col, int warp, float (&x)[VS]) {
-  read_acc_nowait<VS>(cx, col, warp, x);
-  read_wait(cx);
-}
-
-// Document flags of the chunks a chain walks, kept in shared memory 128 chunks at a time (plus one of
-// look-ahead) so that no step of the chain waits for the segment ids: thread i fills entry i.
-// dir = +1: entry i is chunk top + i; dir = -1: chunk top - i.  Bit 0: the chunk starts a document; bit 1:
-// the chunk is one document.  Ends with a __syncthreads().
-__device__ __forceinline__ void fill_flags(uint8_t* fl, const int32_t* seg, const Geo& g, int b, int top, int dir,
-                                           int lo, int hi) {
-  for (int i = threadIdx.x; i < 129; i += blockDim.x) {
-    const int c = top + dir * i;
-    uint8_t f = 0;
-    if (c >= lo && c < hi) {
-      bool n, s;
-      chunk_flags(seg, g, b, c, n, s);
-      f = (n ? 1 : 0) | (s ? 2 : 0);
+    for (int j = 0; j < 32; j += 4) {
+      const float4 t = *reinterpret_cast<const float4*>(p + j);
+      v[j] = t.x; v[j + 1] = t.y; v[j + 2] = t.z; v[j + 3] = t.w;
     }
-    fl[i] = f;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = p[j];
   }
-  __syncthreads();
+}
+__device__ __forceinline__ void store32(float* p, const float (&v)[32]) {
+  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(p + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) p[j] = v[j];
+  }
 }
 
-__host__ __device__ constexpr uint32_t tmem_cols(int vs) { return 3 * vs <= 128 ? 128u : (3 * vs <= 256 ? 256u : 512u); }
-
-template <int VS, bool WITH_OUT>
-__global__ void __launch_bounds__(128, 1) state_fwd_tc_kernel(StateArgs a) {
+template <int VS>
+__global__ void __launch_bounds__(Plan<VS, false>::NT, 1) state_fwd_tc_kernel(const __grid_constant__ StateArgs a) {
+  using PL = Plan<VS, false>;
+  constexpr int ST = PL::ST, NG = PL::NG, SLOTS = PL::SLOTS;
   extern __shared__ __align__(128) uint8_t sm[];
-  __shared__ uint64_t bar, tb[2];                       // MMA completion; tile arrival: W | qe, M, ke
+  constexpr int ROWS = PL::ROWS;
+  __shared__ uint64_t full[SLOTS], empty[SLOTS], row_full[ROWS], row_empty[ROWS];
+  __shared__ uint64_t s_ready, v_ready, p_done, s_done, o_done[2], o_free[2], s_free, all_done;
   __shared__ uint32_t tmem_base;
-  __shared__ uint8_t fl_s[132];
+  __shared__ int stop_s;
   const Geo& g = a.g;
-  constexpr int C = 128, K = 128;
-  const int Vw = g.Vw, h = blockIdx.y, b = blockIdx.z;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // (warp: uniform for the compiler)
+  const int Vw = g.Vw, vr = g.G * g.V, h = blockIdx.y, b = blockIdx.z;
   // slices past the value width carry the transition columns (see StateArgs::P_out)
   const bool trans = (int)blockIdx.x * VS >= Vw;
   const int v0 = trans ? 0 : blockIdx.x * VS, p0 = trans ? blockIdx.x * VS - Vw : 0;
-  const int row = threadIdx.x, warp = row >> 5;
-  uint4* sW = reinterpret_cast<uint4*>(sm);
-  uint4* sQE = sW + TILE_U4;
-  uint4* sM = sQE + TILE_U4;
-  uint4* sKE = sM + TILE_U4;
-  uint4* sS = sKE + TILE_U4;
-  uint4* sVn = sS + (VS / 8) * 128;
-  if (row == 0) { umma::mbar_init(&bar, 1); umma::mbar_init(&tb[0], 1); umma::mbar_init(&tb[1], 1); umma::fence_mbar_init(); }
-  if (warp == 0) umma::tmem_alloc(&tmem_base, tmem_cols(VS));
+  uint8_t* tiles = sm;
+  uint8_t* sS = sm + SLOTS * TILE_B;
+  uint8_t* sV = sS + PL::SL;                            // ROWS buffers
+  float* lam_s = reinterpret_cast<float*>(sV + ROWS * PL::SL);
+  const int cb = a.c_begin;
+  int ce = a.c_end;
+  if (tid == 0) {
+    for (int i = 0; i < SLOTS; ++i) { umma::mbar_init(&full[i], 1); umma::mbar_init(&empty[i], 1); }
+    for (int i = 0; i < ROWS; ++i) { umma::mbar_init(&row_full[i], 1); umma::mbar_init(&row_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { umma::mbar_init(&o_done[i], 1); umma::mbar_init(&o_free[i], 4); }
+    umma::mbar_init(&s_ready, 4 * NG); umma::mbar_init(&v_ready, 4 * NG);
+    umma::mbar_init(&p_done, 1); umma::mbar_init(&s_done, 1); umma::mbar_init(&s_free, 1); umma::mbar_init(&all_done, 1);
+    umma::fence_mbar_init();
+    stop_s = ce;
+  }
+  if (warp == 0) umma::tmem_alloc(&tmem_base, PL::TMEM);
   umma::tc_fence_before();
   __syncthreads();
+  // the first chunk behind which nothing depends on the state that this launch starts from
+  if (a.until_independent || a.skip_provisional) {
+    for (int c = cb + tid; c < ce; c += PL::NT) {
+      bool n, s, n2 = false, s2;
+      chunk_flags(a.seg, g, b, c, n, s);
+      if (c + 1 < ce) chunk_flags(a.seg, g, b, c + 1, n2, s2);
+      if (!s || n2) { atomicMin(&stop_s, c); break; }
+    }
+    __syncthreads();
+  }
   umma::tc_fence_after();
-  umma::Ctx cx{tmem_base, &bar, 0u, a.err, false};
-  constexpr uint32_t colP = 0, colO = VS, colS = 2 * VS;
-  const bool img = g.img;
-  uint32_t tph[2] = {0u, 0u};
-  auto tile_wait = [&](int i) {                         // bounded, like every wait here
-    if (!umma::mbar_wait(&tb[i], tph[i])) umma::report_timeout(a.err);
-    tph[i] ^= 1u;
-  };
+  const int stop = stop_s;
+  if (a.until_independent && stop + 1 < ce) ce = stop + 1;
+  const int n = ce - cb;
+  // index of the first chunk whose outputs are wanted
+  const int o_from = (!a.out || trans) ? n : (a.skip_provisional ? (stop + 1 < ce ? stop + 1 - cb : n) : 0);
+  const uint32_t tm = tmem_base;
+  constexpr uint32_t colP = 0, colS = VS, colO = 2 * VS;
+  const size_t item0 = ((size_t)b * g.H + h) * g.NC + cb;
+  const bool keep_states = a.states && !trans;
+  const bool has_u = a.res.U && !trans;
+  Waiter wait{a.err, false};
 
-  const __nv_bfloat16* Wg = reinterpret_cast<const __nv_bfloat16*>(a.res.W);
-  const __nv_bfloat16* QEg = reinterpret_cast<const __nv_bfloat16*>(a.res.qe);
-  const __nv_bfloat16* KEg = reinterpret_cast<const __nv_bfloat16*>(a.res.ke);
-  const __nv_bfloat16* Mg = reinterpret_cast<const __nv_bfloat16*>(a.res.M);
-  const __nv_bfloat16* Ug = trans ? nullptr : reinterpret_cast<const __nv_bfloat16*>(a.res.U);
-  float* const states = trans ? nullptr : a.states;
-  const size_t item0 = ((size_t)b * g.H + h) * g.NC;
-
-  const int cb = a.c_begin, ce = a.c_end;               // chunk range of this launch
-  float* carry = a.carry ? a.carry + (((size_t)b * g.H + h) * K + row) * Vw + v0 : nullptr;
-  auto fetch_W = [&](size_t it_) {
-    if (img) {
-      if (row == 0) { umma::mbar_expect_tx(&tb[0], TILE_U4 * 16); bulk_tile(sW, Wg + it_ * C * K, &tb[0]); }
-    } else {
-      copy_tile_async(sW, Wg + it_ * C * K, row, false);
-    }
-    umma::cp_async_commit();
-  };
-  // (a pass without outputs needs neither qe nor M: half the bytes a chunk step pulls through L2, which
-  // is what bounds the step)
-  const bool need_out_tiles = WITH_OUT && !trans;
-  // With skip_provisional the outputs of the chunks that still depend on the state this launch started from
-  // are left to the pass that follows with the true state (it rewrites exactly those chunks): `indep` turns
-  // true after the first chunk that holds a document boundary or precedes one.  Uniform over the CTA.
-  bool indep = !a.skip_provisional;
-  auto fetch_QMK = [&](size_t it_, bool with_out) {
-    if (img) {
-      if (row == 0) {
-        umma::mbar_expect_tx(&tb[1], (with_out ? 3 : 1) * TILE_U4 * 16);
-        if (with_out) {
-          bulk_tile(sQE, QEg + it_ * C * K, &tb[1]);
-          bulk_tile(sM, Mg + it_ * C * C, &tb[1]);
-        }
-        bulk_tile(sKE, KEg + it_ * C * K, &tb[1]);
-      }
-    } else {
-      if (with_out) {
-        copy_tile_async(sQE, QEg + it_ * C * K, row, false);
-        copy_tile_async(sM, Mg + it_ * C * C, row, false);
-      }
-      copy_tile_async(sKE, KEg + it_ * C * K, row, false);
-    }
-    umma::cp_async_commit();
-  };
-  fetch_W(item0 + cb);
-  fetch_QMK(item0 + cb, need_out_tiles && indep);
-
-  float S[VS];
+  if (tid < ST) {
+    // ------------------------------------------------------------------------------------------ state warps
+    const int row = (warp & 3) * 32 + lane, ng = warp >> 2, col = v0 + 32 * ng;
+    const uint32_t tb = tm + ((uint32_t)((warp & 3) * 32) << 16) + 32 * ng;
+    uint4* S_img = reinterpret_cast<uint4*>(sS) + ng * 512;
+    float* carry = a.carry ? a.carry + (((size_t)b * g.H + h) * KT + row) * Vw + col : nullptr;
+    size_t noff;
+    const bool native = native_row(g, b, h, row, col, noff);
+    float S[32];
 #pragma unroll
-  for (int j = 0; j < VS; ++j) S[j] = cb > 0 ? carry[j] : 0.f;
-
-  // This thread's row of U (VS columns) and of Lambda_end for one chunk, fetched one chunk ahead of use
-  // (right after the previous chunk's copy has been consumed), so the chain never waits for them.
-  uint4 ureg[VS / 8];
-  float lam_cur;
-  auto fetch_row = [&](size_t it_) {
-    if (Ug) {
-      if (g.img) {
-        const uint4* up = reinterpret_cast<const uint4*>(Ug + it_ * C * Vw) + (size_t)(v0 / 8) * 128 + row;
+    for (int j = 0; j < 32; ++j) S[j] = 0.f;
+    if (cb > 0) load32(carry, S);
+    Flags fl;
+    fl.fill(a.seg, g, b, cb, 1, cb, ce);
+    if (cb == 0 && !(fl.is_new & 1u)) {
+      if (trans) {
 #pragma unroll
-        for (int p = 0; p < VS / 8; ++p) ureg[p] = __ldg(up + p * 128);
-      } else {
-        const uint4* up = reinterpret_cast<const uint4*>(Ug + it_ * C * Vw + (size_t)row * Vw + v0);
-#pragma unroll
-        for (int p = 0; p < VS / 8; ++p) ureg[p] = __ldg(up + p);
-      }
-    } else {                                            // transition columns / U == NULL: U = 0
-#pragma unroll
-      for (int p = 0; p < VS / 8; ++p) ureg[p] = make_uint4(0, 0, 0, 0);
-    }
-    lam_cur = __ldg(a.res.lam_end + it_ * K + row);
-  };
-  fetch_row(item0 + cb);
-
-  for (int c = cb; c < ce; ++c) {
-    const size_t item = item0 + c;
-    const int fo = (c - cb) & 127;
-    if (fo == 0) fill_flags(fl_s, a.seg, g, b, c, 1, cb, ce);
-    const bool is_new = fl_s[fo] & 1, all_same = fl_s[fo] & 2;
-    const bool nis_new = fl_s[fo + 1] & 1;              // (zero past the end of the range)
-    if (c == 0 && !is_new && trans) {
-#pragma unroll
-      for (int j = 0; j < VS; ++j) S[j] = row == p0 + j ? 1.f : 0.f;
-    } else if (c == 0 && !is_new && a.init_state) {
-#pragma unroll
-      for (int j = 0; j < VS; ++j) S[j] = a.init_state[native_state_index_tc(g, b, h, row, v0 + j)];
-    } else if (is_new) {
-#pragma unroll
-      for (int j = 0; j < VS; ++j) S[j] = 0.f;
-    }
-    if (states && !g.img) {
-      float4* dst = reinterpret_cast<float4*>(states + item * K * Vw + (size_t)row * Vw + v0);
-#pragma unroll
-      for (int j = 0; j < VS / 4; ++j) dst[j] = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
-    }
-    stage_rows<VS>(sS, row, S);
-    if (states && g.img) {                              // the same bf16 rows, as an operand image for the backward
-      uint4* simg = reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(states_img(g, states)) + item * K * Vw) + (size_t)(v0 / 8) * 128 + row;
-#pragma unroll
-      for (int p = 0; p < VS / 8; ++p) simg[p * 128] = sS[p * 128 + row];
-    }
-    const float dec = all_same ? expf(fminf(lam_cur, 0.f)) : 0.f;
-    // the last chunk this CTA walks: the end of the range, or (until_independent) the point after which
-    // nothing depends on the state the chain started from.  Uniform over the CTA (the flags depend on the
-    // chunk only).  Nothing is prefetched past it, so no copy is in flight when the CTA leaves.
-    const bool last = c + 1 >= ce || (a.until_independent && (!all_same || nis_new));
-
-    if (img) tile_wait(0); else umma::cp_async_wait<1>();      // this chunk's W has landed
-    umma::pre_issue_sync();
-    umma::issue<VS, false, true>(cx, sW, sS, K, colP, false);          // P = W S
-    umma::commit_wait(cx);
-    if (!last) fetch_W(item + 1); else umma::cp_async_commit();
-
-    float vn[VS];
-    read_acc<VS>(cx, colP, warp, vn);
-#pragma unroll
-    for (int p = 0; p < VS / 8; ++p) {
-      float u[8];
-      umma::unpack8(ureg[p], u);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) vn[p * 8 + i] = u[i] - vn[p * 8 + i];      // V_new = U - W S
-    }
-    if (!last) fetch_row(item + 1);
-    stage_rows<VS>(sVn, row, vn);
-
-    if (img) tile_wait(1); else umma::cp_async_wait<1>();      // this chunk's qe, M, ke have landed
-    umma::pre_issue_sync();
-    const bool outc = need_out_tiles && indep;                         // this chunk's outputs are wanted
-    indep = indep || !all_same || nis_new;                             // ... and the next chunk's
-    if (outc) {
-      umma::issue<VS, false, true>(cx, sQE, sS, K, colO, false);       // O  = qe S
-      umma::issue<VS, false, true>(cx, sM, sVn, C, colO, true);        //    + M V_new
-    }
-    umma::issue<VS, true, true>(cx, sKE, sVn, C, colS, false);         // ke^T V_new
-    umma::commit_wait(cx);
-    if (!last) fetch_QMK(item + 1, need_out_tiles && indep); else umma::cp_async_commit();
-
-    float sn[VS];
-    if (outc) {
-      float o[VS];
-      read_acc_nowait<VS>(cx, colO, warp, o);
-      read_acc_nowait<VS>(cx, colS, warp, sn);
-      read_wait(cx);
-      const int t = c * C + row;
-      if (t < g.L) {
-        const size_t off = ((size_t)b * g.L + t) * g.Hv * g.V + (size_t)h * Vw + v0;
-        if (g.qkv_dt == DN_BF16) {
-          uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.out) + off);
-#pragma unroll
-          for (int p = 0; p < VS / 8; ++p) {
-            float t8[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) t8[i] = o[p * 8 + i];
-            dst[p] = umma::pack8(t8);
-          }
-        } else {
-          float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + off);
-#pragma unroll
-          for (int j = 0; j < VS / 4; ++j) dst[j] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
-        }
+        for (int j = 0; j < 32; ++j) S[j] = row == p0 + 32 * ng + j ? 1.f : 0.f;
+      } else if (a.init_state && native) {
+        load32(a.init_state + noff, S);
       }
     }
-    if (!outc) read_acc<VS>(cx, colS, warp, sn);
+    if (fl.is_new & 1u) {
 #pragma unroll
-    for (int j = 0; j < VS; ++j) S[j] = fmaf(dec, S[j], sn[j]);       // S <- decay * S + ke^T V_new
+      for (int j = 0; j < 32; ++j) S[j] = 0.f;
+    }
+    Ring<ROWS> rows;
+    Ring<SLOTS> ring;                                   // follows the tiles the products take
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+      const bool outs = i >= o_from;
+      if (keep_states && i > 0) wait(&s_free, (i - 1) & 1);
+      image32(S_img, row, S);
+      warp_arrive(&s_ready);
+      // V = U - W S, over U
+      wait(&row_full[rows.at], rows.parity);
+      uint4* V_img = reinterpret_cast<uint4*>(sV + rows.at * PL::SL) + ng * 512;
+      uint4 u[4];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) u[p] = has_u ? V_img[p * 128 + row] : make_uint4(0, 0, 0, 0);
+      float dec = fl.all_same & 1u ? expf(fminf(lam_s[rows.at * 128 + row], 0.f)) : 0.f;
+      const uint32_t row_at = rows.at;
+      rows.next();
+      fl.next();
+      if ((i & 31) == 31) fl.fill(a.seg, g, b, cb + i + 1, 1, cb, ce);
+      // the next chunk starts a document: nothing of this one is handed on
+      const bool drop = fl.is_new & 1u;
+      float x[32];
+      wait(&p_done, i & 1);
+      umma::tc_fence_after();
+      ld32(wait.dead, tb + colP, x);
+      // (released by the threads that see a product complete: a commit of its own costs the issuing warp 67 cycles)
+      if (tid == 0) arrive(&empty[ring.at]);            // W
+      ring.next();
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        float t[8];
+        umma::unpack8(u[p], t);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) t[k] -= x[8 * p + k];
+        V_img[p * 128 + row] = umma::pack8(t);
+      }
+      warp_arrive(&v_ready);
+      wait(&s_done, i & 1);
+      umma::tc_fence_after();
+      ld32(wait.dead, tb + colS, x);
+      if (outs) {
+        if (tid == 32) arrive(&empty[ring.at]);         // qe
+        ring.next();
+      }
+      if (tid == 64) arrive(&empty[ring.at]);           // ke
+      ring.next();
+      if (outs) ring.next();                            // M: released by the output warps, with V
+      else if (tid == 96) arrive(&row_empty[row_at]);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) S[j] = fmaf(dec, S[j], x[j]);
+      if (drop) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) S[j] = 0.f;
+      }
+    }
     umma::tc_fence_before();
-    if (last) break;
+    if (a.until_independent) {
+      // nothing to hand on: the caller has the final state from the shard's affine summary
+    } else if (trans) {
+      if (row < g.K) store32(a.P_out + (((size_t)b * g.H + h) * g.K + row) * g.K + p0 + 32 * ng, S);
+    } else if (ce < g.NC) {
+      store32(carry, S);
+    } else if (a.final_state && native) {
+      store32(a.final_state + noff, S);
+    }
+  } else if (tid < ST + 128) {
+    // ------------------------------------------------------------------------------------------ outputs, a row per lane
+    const int q = warp & 3, row = q * 32 + lane;
+    Ring<ROWS> rows;
+    rows.at = o_from % ROWS;
+    uint32_t m_at = (2 * o_from + 3) % SLOTS;           // M's slot (two tiles per chunk without outputs, four with)
+#pragma unroll 1
+    for (int i = o_from; i < n; ++i) {
+      const int oi = i - o_from;
+      wait(&o_done[oi & 1], (oi >> 1) & 1);
+      umma::tc_fence_after();
+      if (q == 0 && lane == 0) arrive(&empty[m_at]);
+      if (q == 1 && lane == 0) arrive(&row_empty[rows.at]);
+      rows.next();
+      m_at = (m_at + 4) % SLOTS;
+      const int t = (cb + i) * C + row;
+      const size_t off = ((size_t)b * g.L + t) * g.Hv * g.V + (size_t)h * vr + v0;
+#pragma unroll 1
+      for (int ng = 0; ng < NG; ++ng) {
+        float o[32];
+        ld32(wait.dead, tm + ((uint32_t)(q * 32) << 16) + colO + (oi & 1) * VS + 32 * ng, o);
+        if (ng == NG - 1) {
+          umma::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) arrive(&o_free[oi & 1]);
+        }
+        if (t < g.L && v0 + 32 * ng < vr) {
+          if (g.qkv_dt == DN_BF16) {
+            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.out) + off + 32 * ng);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) dst[p] = umma::pack8p(o + 8 * p);
+          } else {
+            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + off + 32 * ng);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) dst[j] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+          }
+        }
+      }
+    }
+  } else {
+    const int role = warp - (ST + 128) / 32;
+    if (role == 0) {
+      // ---------------------------------------------------------------------------------------- products
+      Ring<SLOTS> ring;
+      Ring<ROWS> rows;
+      Ring<2> ob;
+      const uint64_t tk = operand<false>(tiles), tt = operand<true>(tiles), bS = operand<true>(sS), bV = operand<true>(sV);
+#pragma unroll 1
+      for (int i = 0; i < n; ++i) {
+        const bool outs = i >= o_from;
+        const uint32_t colOi = tm + colO + ob.at * VS;
+        const uint64_t bVi = bV + rows.at * (PL::SL >> 4);
+        wait(&full[ring.at], ring.parity);
+        wait(&s_ready, i & 1);
+        umma::tc_fence_after();
+        product<VS, false, true>(tm + colP, tk + ring.at * (TILE_B >> 4), bS, false);            // P = W S
+        umma::mma_commit_warp(&p_done);
+        ring.next();
+        if (outs) {
+          wait(&full[ring.at], ring.parity);
+          if (i - o_from >= 2) { wait(&o_free[ob.at], ob.parity ^ 1u); umma::tc_fence_after(); }
+          product<VS, false, true>(colOi, tk + ring.at * (TILE_B >> 4), bS, false);              // O  = qe S
+          ring.next();
+        }
+        wait(&full[ring.at], ring.parity);
+        wait(&v_ready, i & 1);
+        umma::tc_fence_after();
+        product<VS, true, true>(tm + colS, tt + ring.at * (TILE_B >> 4), bVi, false);            // ke^T V
+        umma::mma_commit_warp(&s_done);
+        ring.next();
+        if (outs) {
+          wait(&full[ring.at], ring.parity);
+          product<VS, false, true>(colOi, tk + ring.at * (TILE_B >> 4), bVi, true);              //    + M V
+          umma::mma_commit_warp(&o_done[ob.at]);
+          ring.next();
+          ob.next();
+        }
+        rows.next();
+      }
+      umma::mma_commit_warp(&all_done);                 // every arrival above has happened before the CTA leaves
+      wait(&all_done, 0);
+    } else if (role == 1 && lane == 0) {
+      // ---------------------------------------------------------------------------------------- tiles, in the order of use
+      Ring<SLOTS> ring;
+      bool again = false;                               // the slot has been used before
+      auto load = [&](const void* base, size_t item) {
+        if (again) wait(&empty[ring.at], ring.parity ^ 1u);
+        umma::mbar_expect_tx(&full[ring.at], TILE_B);
+        umma::bulk_load(tiles + ring.at * TILE_B, reinterpret_cast<const uint8_t*>(base) + item * TILE_B, TILE_B, &full[ring.at]);
+        ring.next();
+        again |= ring.at == 0;
+      };
+#pragma unroll 1
+      for (int i = 0; i < n && !wait.dead; ++i) {
+        const bool outs = i >= o_from;
+        load(a.res.W, item0 + i);
+        if (outs) load(a.res.qe, item0 + i);
+        load(a.res.ke, item0 + i);
+        if (outs) load(a.res.M, item0 + i);
+      }
+    } else if (role == 2 && lane == 0) {
+      // ---------------------------------------------------------------------------------------- rows: U, Lambda_end
+      Ring<ROWS> ring;
+#pragma unroll 1
+      for (int i = 0; i < n && !wait.dead; ++i, ring.next()) {
+        const uint32_t s = ring.at;
+        if (i >= ROWS) wait(&row_empty[s], ring.parity ^ 1u);
+        umma::mbar_expect_tx(&row_full[s], 512 + (has_u ? PL::SL : 0));
+        umma::bulk_load(lam_s + s * 128, a.res.lam_end + (item0 + i) * KT, 512, &row_full[s]);
+        if (has_u)
+          umma::bulk_load(sV + s * PL::SL, reinterpret_cast<const uint8_t*>(a.res.U) + ((item0 + i) * Vw + v0) * 256, PL::SL, &row_full[s]);
+      }
+    } else if (role == 3 && lane == 0 && keep_states) {
+      // ---------------------------------------------------------------------------------------- chunk-entry states
+      uint8_t* dst = reinterpret_cast<uint8_t*>(a.states);
+      for (int i = 0; i < n && !wait.dead; ++i) {
+        wait(&s_ready, i & 1);
+        umma::bulk_store(dst + ((item0 + i) * Vw + v0) * 256, sS, PL::SL);
+        umma::bulk_commit();
+        umma::bulk_wait_read<0>();
+        arrive(&s_free);
+      }
+      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
   }
-  if (a.until_independent) {
-    // nothing to hand on: the caller has the final state from the shard's affine summary
-  } else if (trans) {
-    float* dst = a.P_out + (((size_t)b * g.H + h) * K + row) * K + p0;
-#pragma unroll
-    for (int j = 0; j < VS; ++j) dst[j] = S[j];
-  } else if (ce < g.NC) {
-#pragma unroll
-    for (int j = 0; j < VS; ++j) carry[j] = S[j];
-  } else if (a.final_state) {
-#pragma unroll
-    for (int j = 0; j < VS; ++j) a.final_state[native_state_index_tc(g, b, h, row, v0 + j)] = S[j];
-  }
-  umma::cp_async_wait<0>();
   __syncthreads();
-  if (warp == 0) umma::tmem_dealloc(tmem_base, tmem_cols(VS));
+  if (warp == 0) umma::tmem_dealloc(tmem_base, PL::TMEM);
 }
 
 template <int VS>
-__global__ void __launch_bounds__(128, 1) state_bwd_tc_kernel(StateArgs a) {
+__global__ void __launch_bounds__(Plan<VS, true>::NT, 1) state_bwd_tc_kernel(const __grid_constant__ StateArgs a) {
+  using PL = Plan<VS, true>;
+  constexpr int ST = PL::ST, NG = PL::NG, SLOTS = PL::SLOTS, DB = PL::DO_BUF, ROWS = PL::ROWS;
   extern __shared__ __align__(128) uint8_t sm[];
-  __shared__ uint64_t bar, tb[2];                       // MMA completion; tile arrival: M, ke | qe, W
+  __shared__ uint64_t full[SLOTS], empty[SLOTS], row_full[ROWS], row_empty[ROWS], do_ready[DB], do_free[DB];
+  __shared__ uint64_t h_ready, v_ready, v_done, h_done, h_free, v_free, all_done;
   __shared__ uint32_t tmem_base;
-  __shared__ uint8_t fl_s[132];
+  __shared__ int stop_s;
   const Geo& g = a.g;
-  constexpr int C = 128, K = 128;
-  const int Vw = g.Vw, v0 = blockIdx.x * VS, h = blockIdx.y, b = blockIdx.z;
-  const int row = threadIdx.x, warp = row >> 5;
-  uint4* sM = reinterpret_cast<uint4*>(sm);
-  uint4* sKE = sM + TILE_U4;
-  uint4* sQE = sKE + TILE_U4;
-  uint4* sW = sQE + TILE_U4;
-  uint4* sdO = sW + TILE_U4;
-  uint4* sdH = sdO + (VS / 8) * 128;
-  uint4* sdV = sdH + (VS / 8) * 128;
-  uint4* sSl = sdV + (VS / 8) * 128 + row;              // this thread's row of S (image path, bf16): piece j at sSl[j * 128]
-  const bool img = g.img;
-  if (row == 0) { umma::mbar_init(&bar, 1); umma::mbar_init(&tb[0], 1); umma::mbar_init(&tb[1], 1); umma::fence_mbar_init(); }
-  uint32_t tph[2] = {0u, 0u};
-  auto tile_wait = [&](int i) {                         // bounded, like every wait here
-    if (!umma::mbar_wait(&tb[i], tph[i])) umma::report_timeout(a.err);
-    tph[i] ^= 1u;
-  };
-  if (warp == 0) umma::tmem_alloc(&tmem_base, tmem_cols(VS));
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // (warp: uniform for the compiler)
+  const int Vw = g.Vw, vr = g.G * g.V, v0 = blockIdx.x * VS, h = blockIdx.y, b = blockIdx.z;
+  uint8_t* tiles = sm;
+  uint8_t* sdO = sm + SLOTS * TILE_B;                   // DB buffers
+  uint8_t* sdH = sdO + DB * PL::SL;
+  uint8_t* sdV = sdH + PL::SL;
+  uint8_t* sR = sdV + PL::SL;                           // rows of S, ROWS buffers
+  float* lam_s = reinterpret_cast<float*>(sR + ROWS * PL::SL);
+  float* part_s = lam_s + ROWS * 128;                   // partial sums of dLambda_end: NG x 128
+  const int ce = a.c_end;
+  int cb = a.c_begin;
+  if (tid == 0) {
+    for (int i = 0; i < SLOTS; ++i) { umma::mbar_init(&full[i], 1); umma::mbar_init(&empty[i], 1); }
+    for (int i = 0; i < ROWS; ++i) { umma::mbar_init(&row_full[i], 1); umma::mbar_init(&row_empty[i], 1); }
+    for (int i = 0; i < DB; ++i) { umma::mbar_init(&do_ready[i], 4); umma::mbar_init(&do_free[i], 1); }
+    umma::mbar_init(&h_ready, 4 * NG); umma::mbar_init(&v_ready, 4 * NG);
+    umma::mbar_init(&v_done, 1); umma::mbar_init(&h_done, 1);
+    umma::mbar_init(&h_free, 1); umma::mbar_init(&v_free, 1); umma::mbar_init(&all_done, 1);
+    umma::fence_mbar_init();
+    stop_s = cb;
+  }
+  if (warp == 0) umma::tmem_alloc(&tmem_base, PL::TMEM);
   umma::tc_fence_before();
   __syncthreads();
+  if (a.until_independent) {                            // the last chunk whose results depend on the incoming cotangent
+    for (int c = ce - 1 - tid; c >= cb; c -= PL::NT) {
+      bool n, s;
+      chunk_flags(a.seg, g, b, c, n, s);
+      if (n || !s) { atomicMax(&stop_s, c); break; }
+    }
+    __syncthreads();
+  }
   umma::tc_fence_after();
-  umma::Ctx cx{tmem_base, &bar, 0u, a.err, false};
-  constexpr uint32_t colV = 0, colH = VS;
+  cb = stop_s;
+  const int n = ce - cb;
+  const uint32_t tm = tmem_base;
+  constexpr uint32_t colV = 0, colQ = VS, colW = 2 * VS;
+  const size_t last = ((size_t)b * g.H + h) * g.NC + ce - 1;      // item of step i: last - i
+  Waiter wait{a.err, false};
 
-  const __nv_bfloat16* Wg = reinterpret_cast<const __nv_bfloat16*>(a.res.W);
-  const __nv_bfloat16* QEg = reinterpret_cast<const __nv_bfloat16*>(a.res.qe);
-  const __nv_bfloat16* KEg = reinterpret_cast<const __nv_bfloat16*>(a.res.ke);
-  const __nv_bfloat16* Mg = reinterpret_cast<const __nv_bfloat16*>(a.res.M);
-  const size_t item0 = ((size_t)b * g.H + h) * g.NC;
-  const int cb = a.c_begin, ce = a.c_end;               // chunk range of this launch, walked from ce - 1 down
-  float* carry = a.carry ? a.carry + (((size_t)b * g.H + h) * K + row) * Vw + v0 : nullptr;
-  const size_t last = item0 + ce - 1;
-
-  // image path: the thread's own row of the chunk-entry state (its bf16 image, the only copy kept)
-  // travels with M and ke, one chunk ahead, into a private strip of shared memory; it is needed for
-  // dLambda_end = sum_v dH * S
-  auto copy_S_row = [&](size_t it_) {
-    const uint4* src = reinterpret_cast<const uint4*>(states_img(g, a.res.states) + it_ * K * Vw) + (size_t)(v0 / 8) * 128 + row;
+  if (tid < ST) {
+    // ------------------------------------------------------------------------------------------ state warps
+    const int row = (warp & 3) * 32 + lane, ng = warp >> 2, col = v0 + 32 * ng;
+    const uint32_t tb = tm + ((uint32_t)((warp & 3) * 32) << 16) + 32 * ng;
+    uint4* H_img = reinterpret_cast<uint4*>(sdH) + ng * 512;
+    uint4* V_img = reinterpret_cast<uint4*>(sdV) + ng * 512;
+    float* carry = a.carry ? a.carry + (((size_t)b * g.H + h) * KT + row) * Vw + col : nullptr;
+    size_t noff;
+    const bool native = native_row(g, b, h, row, col, noff);
+    float dH[32];
 #pragma unroll
-    for (int j = 0; j < VS / 8; ++j) umma::cp_async16(sSl + j * 128, src + j * 128);
-  };
-  // image path: whole tiles by bulk copies on tb[], the S row by this thread's own cp.async group;
-  // otherwise everything by cp.async groups (two per chunk)
-  auto fetch_MK = [&](size_t it_) {
-    if (img) {
-      if (row == 0) {
-        umma::mbar_expect_tx(&tb[0], 2 * TILE_U4 * 16);
-        bulk_tile(sM, Mg + it_ * C * C, &tb[0]);
-        bulk_tile(sKE, KEg + it_ * C * K, &tb[0]);
-      }
-      copy_S_row(it_);
-    } else {
-      copy_tile_async(sM, Mg + it_ * C * C, row, false);
-      copy_tile_async(sKE, KEg + it_ * C * K, row, false);
-    }
-    umma::cp_async_commit();
-  };
-  auto fetch_QW = [&](size_t it_) {
-    if (img) {
-      if (row == 0) {
-        umma::mbar_expect_tx(&tb[1], 2 * TILE_U4 * 16);
-        bulk_tile(sQE, QEg + it_ * C * K, &tb[1]);
-        bulk_tile(sW, Wg + it_ * C * K, &tb[1]);
-      }
-    } else {
-      copy_tile_async(sQE, QEg + it_ * C * K, row, false);
-      copy_tile_async(sW, Wg + it_ * C * K, row, false);
-    }
-    umma::cp_async_commit();
-  };
-  fetch_MK(last);
-  fetch_QW(last);
-
-  float dH[VS];
-#pragma unroll
-  for (int j = 0; j < VS; ++j)
-    dH[j] = ce < g.NC ? carry[j] : (a.d_final ? a.d_final[native_state_index_tc(g, b, h, row, v0 + j)] : 0.f);
-
-  // This thread's row of dO of one chunk as raw 16-byte vectors (token c*C+row; zero past the end).
-  // They are fetched one chunk ahead so that the chain never waits for them.
-  constexpr int NV = VS / 8;                            // bf16 vectors per row slice; fp32 needs 2 * NV
-  uint4 raw[2 * NV];
-  const bool dobf = g.qkv_dt == DN_BF16;
-  auto fetch_dO = [&](int c) {
-    const int t = c * C + row;
-    const bool live = c >= cb && t < g.L;
-    const size_t off = ((size_t)b * g.L + (live ? t : 0)) * g.Hv * g.V + (size_t)h * Vw + v0;
-    if (dobf) {
-      const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.d_out) + off);
-#pragma unroll
-      for (int p = 0; p < NV; ++p) raw[p] = live ? __ldg(src + p) : make_uint4(0, 0, 0, 0);
-    } else {
-      const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(a.d_out) + off);
-#pragma unroll
-      for (int p = 0; p < 2 * NV; ++p) raw[p] = live ? __ldg(src + p) : make_uint4(0, 0, 0, 0);
-    }
-  };
-  fetch_dO(ce - 1);
-
-  for (int c = ce - 1; c >= cb; --c) {
-    const size_t item = item0 + c;
-    const int fo = (ce - 1 - c) & 127;
-    if (fo == 0) fill_flags(fl_s, a.seg, g, b, c, -1, cb, ce);
-    const bool is_new = fl_s[fo] & 1, all_same = fl_s[fo] & 2;
-    // dO of this chunk, rounded to bf16 as the reference does (gdn2.py:731)
-    float dO[VS];
-    if (dobf) {
-#pragma unroll
-      for (int p = 0; p < NV; ++p) {
-        float t8[8];
-        umma::unpack8(raw[p], t8);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) dO[p * 8 + i] = t8[i];
-      }
-    } else {
-#pragma unroll
-      for (int p = 0; p < 2 * NV; ++p) {
-        dO[4 * p] = __uint_as_float(raw[p].x); dO[4 * p + 1] = __uint_as_float(raw[p].y);
-        dO[4 * p + 2] = __uint_as_float(raw[p].z); dO[4 * p + 3] = __uint_as_float(raw[p].w);
-      }
-    }
-    // the last chunk this CTA walks: the start of the range, or (until_independent) the point below which
-    // nothing depends on the cotangent the chain started from.  Uniform over the CTA; nothing is
-    // prefetched past it.
-    const bool last = c <= cb || (a.until_independent && (is_new || !all_same));
-    fetch_dO(last ? cb - 1 : c - 1);                    // in flight during this chunk's products (zeros past the end)
-    stage_rows<VS>(sdO, row, dO);
-    stage_rows<VS>(sdH, row, dH);
-    if (img) {                                           // dH as a bf16 operand image
-      uint4* dst = reinterpret_cast<uint4*>(a.dH) + item * (K * Vw / 8) + (size_t)(v0 / 8) * 128 + row;
-#pragma unroll
-      for (int p = 0; p < VS / 8; ++p) dst[p * 128] = sdH[p * 128 + row];
-    } else {
-      float4* dst = reinterpret_cast<float4*>(a.dH + item * K * Vw + (size_t)row * Vw + v0);
-#pragma unroll
-      for (int j = 0; j < VS / 4; ++j) dst[j] = make_float4(dH[4 * j], dH[4 * j + 1], dH[4 * j + 2], dH[4 * j + 3]);
-    }
-    const float dec = all_same ? expf(fminf(__ldg(a.res.lam_end + item * K + row), 0.f)) : 0.f;
-
-    umma::cp_async_wait<1>();                           // M, ke of this chunk (cp.async path); the S row (image path)
-    if (img) tile_wait(0);
-    if (img) {                                          // partial sum of dLambda_end over this CTA's columns
+    for (int j = 0; j < 32; ++j) dH[j] = 0.f;
+    if (ce < g.NC) load32(carry, dH);
+    else if (a.d_final && native) load32(a.d_final + noff, dH);
+    Flags fl;
+    fl.fill(a.seg, g, b, ce - 1, -1, cb, ce);
+    Ring<ROWS> rows;
+    Ring<SLOTS> ring;                                   // follows the tiles the products take
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+      if (i > 0) wait(&h_free, (i - 1) & 1);
+      image32(H_img, row, dH);
+      warp_arrive(&h_ready);
+      // off the chain: this slice's share of dLambda_end = sum_v dH S, in fp32
+      wait(&row_full[rows.at], rows.parity);
+      const uint4* R_img = reinterpret_cast<const uint4*>(sR + rows.at * PL::SL) + ng * 512;
       float part = 0.f;
 #pragma unroll
-      for (int j = 0; j < VS / 8; ++j) {
-        float sv[8];
-        umma::unpack8(sSl[j * 128], sv);
+      for (int p = 0; p < 4; ++p) {
+        float s8[8];
+        umma::unpack8(R_img[p * 128 + row], s8);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) part = fmaf(dH[8 * j + i], sv[i], part);
+        for (int k = 0; k < 8; ++k) part = fmaf(dH[8 * p + k], s8[k], part);
       }
-      dlend_part(g, a.dH)[(item * gridDim.x + blockIdx.x) * K + row] = part;
-    }
-    umma::pre_issue_sync();
-    umma::issue<VS, true, true>(cx, sM, sdO, C, colV, false);          // dV  = M^T dO
-    umma::issue<VS, false, true>(cx, sKE, sdH, K, colV, true);         //     + ke dH
-    umma::commit_wait(cx);
-    if (!last) fetch_MK(item - 1); else umma::cp_async_commit();
-
-    float dv[VS];
-    read_acc<VS>(cx, colV, warp, dv);
-    if (img) {                                           // dV as a bf16 operand image
-      uint4* dst = reinterpret_cast<uint4*>(a.dV) + item * (C * Vw / 8) + (size_t)(v0 / 8) * 128 + row;
+      if (i > 0) wait(&v_free, (i - 1) & 1);            // dV and the sums of the step before have been read
+      part_s[ng * 128 + row] = part;
+      const float dec = fl.all_same & 1u ? expf(fminf(lam_s[rows.at * 128 + row], 0.f)) : 0.f;
+      const bool is_new = fl.is_new & 1u;
+      const uint32_t row_at = rows.at;
+      rows.next();
+      fl.next();
+      if ((i & 31) == 31) fl.fill(a.seg, g, b, ce - 2 - i, -1, cb, ce);
+      float x[32];
+      wait(&v_done, i & 1);
+      umma::tc_fence_after();
+      ld32(wait.dead, tb + colV, x);
+      // (released by the threads that see a product complete: a commit of its own costs the issuing warp 67 cycles)
+      if (tid == 0) arrive(&empty[ring.at]);            // M
+      ring.next();
+      if (tid == 32) arrive(&empty[ring.at]);           // ke
+      ring.next();
+      image32(V_img, row, x);
+      warp_arrive(&v_ready);
+      wait(&h_done, i & 1);
+      umma::tc_fence_after();
+      if (tid == 0) arrive(&empty[ring.at]);            // qe
+      ring.next();
+      if (tid == 32) arrive(&empty[ring.at]);           // W
+      ring.next();
+      if (tid == 64) arrive(&do_free[i & 1]);
+      if (tid == 96) arrive(&row_empty[row_at]);
+      if (is_new) {
 #pragma unroll
-      for (int p = 0; p < VS / 8; ++p) {
-        float t8[8];
+        for (int j = 0; j < 32; ++j) dH[j] = 0.f;
+      } else if (wait.dead) {
+        // nothing to add
+      } else {
+        float w[32];
+        umma::tmem_ld32_nowait(tb + colQ, x);
+        umma::tmem_ld32_nowait(tb + colW, w);
+        umma::tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) t8[i] = dv[p * 8 + i];
-        dst[p * 128] = umma::pack8(t8);
+        for (int j = 0; j < 32; ++j) dH[j] = fmaf(dec, dH[j], x[j] - w[j]);
       }
-    } else {
-      float4* dst = reinterpret_cast<float4*>(a.dV + item * C * Vw + (size_t)row * Vw + v0);
-#pragma unroll
-      for (int j = 0; j < VS / 4; ++j) dst[j] = make_float4(dv[4 * j], dv[4 * j + 1], dv[4 * j + 2], dv[4 * j + 3]);
     }
-    stage_rows<VS>(sdV, row, dv, -1.f);                 // staged negated: the product below is -W^T dV
-
-    if (img) tile_wait(1); else umma::cp_async_wait<1>();      // qe, W of this chunk
-    umma::pre_issue_sync();
-    umma::issue<VS, true, true>(cx, sQE, sdO, C, colH, false);         // qe^T dO
-    umma::issue<VS, true, true>(cx, sW, sdV, C, colH, true);           // - W^T dV
-    umma::commit_wait(cx);
-    if (!last) fetch_QW(item - 1); else umma::cp_async_commit();
-
-    float dn_[VS];
-    read_acc<VS>(cx, colH, warp, dn_);
-#pragma unroll
-    for (int j = 0; j < VS; ++j) dH[j] = is_new ? 0.f : fmaf(dec, dH[j], dn_[j]);
     umma::tc_fence_before();
-    if (last) break;
-  }
-  if (a.until_independent) {
-    // nothing to hand on: the caller has d_init from the shard's affine summary
-  } else if (cb > 0) {
+    if (a.until_independent) {
+      // nothing to hand on: the caller has d_init from the shard's affine summary
+    } else if (cb > 0) {
+      store32(carry, dH);
+    } else if (a.d_init && native) {
+      store32(a.d_init + noff, dH);
+    }
+  } else if (tid < ST + 128) {
+    // ------------------------------------------------------------------------------------------ dO, rounded to bf16 (gdn2.py:731)
+    const int row = (warp & 3) * 32 + lane;
+    for (int i = 0; i < n; ++i) {
+      const int t = (ce - 1 - i) * C + row;
+      const size_t off = ((size_t)b * g.L + (t < g.L ? t : 0)) * g.Hv * g.V + (size_t)h * vr + v0;
+      uint4 raw[4 * NG];
 #pragma unroll
-    for (int j = 0; j < VS; ++j) carry[j] = dH[j];
-  } else if (a.d_init) {
+      for (int p = 0; p < 4 * NG; ++p) {
+        const bool on = t < g.L && v0 + 8 * p < vr;
+        if (g.qkv_dt == DN_BF16) raw[p] = on ? __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.d_out) + off) + p) : make_uint4(0, 0, 0, 0);
+        else raw[p] = on ? umma::ld8_f32_ro(reinterpret_cast<const float*>(a.d_out) + off + 8 * p) : make_uint4(0, 0, 0, 0);
+      }
+      if (i >= DB) wait(&do_free[i % DB], (i / DB - 1) & 1);
+      uint4* img = reinterpret_cast<uint4*>(sdO + (i % DB) * PL::SL);
 #pragma unroll
-    for (int j = 0; j < VS; ++j) a.d_init[native_state_index_tc(g, b, h, row, v0 + j)] = dH[j];
+      for (int p = 0; p < 4 * NG; ++p) img[p * 128 + row] = raw[p];
+      warp_arrive(&do_ready[i % DB]);
+    }
+  } else {
+    const int role = warp - (ST + 128) / 32;
+    if (role == 0) {
+      // ---------------------------------------------------------------------------------------- products
+      Ring<SLOTS> ring;
+      Ring<DB> dos;
+      const uint64_t tk = operand<false>(tiles), tt = operand<true>(tiles), bO = operand<true>(sdO), bH = operand<true>(sdH), bV = operand<true>(sdV);
+#pragma unroll 1
+      for (int i = 0; i < n; ++i) {
+        const uint64_t bOi = bO + dos.at * (PL::SL >> 4);
+        wait(&full[ring.at], ring.parity);
+        wait(&do_ready[dos.at], dos.parity);
+        umma::tc_fence_after();
+        product<VS, true, true>(tm + colV, tt + ring.at * (TILE_B >> 4), bOi, false);            // dV  = M^T dO
+        ring.next();
+        wait(&full[ring.at], ring.parity);
+        wait(&h_ready, i & 1);
+        umma::tc_fence_after();
+        product<VS, false, true>(tm + colV, tk + ring.at * (TILE_B >> 4), bH, true);             //     + ke dH
+        umma::mma_commit_warp(&v_done);
+        ring.next();
+        wait(&full[ring.at], ring.parity);
+        product<VS, true, true>(tm + colQ, tt + ring.at * (TILE_B >> 4), bOi, false);            // qe^T dO
+        ring.next();
+        dos.next();
+        wait(&full[ring.at], ring.parity);
+        wait(&v_ready, i & 1);
+        umma::tc_fence_after();
+        product<VS, true, true>(tm + colW, tt + ring.at * (TILE_B >> 4), bV, false);             // W^T dV
+        umma::mma_commit_warp(&h_done);
+        ring.next();
+      }
+      umma::mma_commit_warp(&all_done);
+      wait(&all_done, 0);
+    } else if (role == 1 && lane == 0) {
+      // ---------------------------------------------------------------------------------------- tiles, in the order of use
+      Ring<SLOTS> ring;
+      bool again = false;                               // the slot has been used before
+      auto load = [&](const void* base, size_t item) {
+        if (again) wait(&empty[ring.at], ring.parity ^ 1u);
+        umma::mbar_expect_tx(&full[ring.at], TILE_B);
+        umma::bulk_load(tiles + ring.at * TILE_B, reinterpret_cast<const uint8_t*>(base) + item * TILE_B, TILE_B, &full[ring.at]);
+        ring.next();
+        again |= ring.at == 0;
+      };
+#pragma unroll 1
+      for (int i = 0; i < n && !wait.dead; ++i) {
+        load(a.res.M, last - i);
+        load(a.res.ke, last - i);
+        load(a.res.qe, last - i);
+        load(a.res.W, last - i);
+      }
+    } else if (role == 2 && lane == 0) {
+      // ---------------------------------------------------------------------------------------- rows: entry state, Lambda_end
+      Ring<ROWS> ring;
+#pragma unroll 1
+      for (int i = 0; i < n && !wait.dead; ++i, ring.next()) {
+        const uint32_t s = ring.at;
+        if (i >= ROWS) wait(&row_empty[s], ring.parity ^ 1u);
+        umma::mbar_expect_tx(&row_full[s], 512 + PL::SL);
+        umma::bulk_load(lam_s + s * 128, a.res.lam_end + (last - i) * KT, 512, &row_full[s]);
+        umma::bulk_load(sR + s * PL::SL, reinterpret_cast<const uint8_t*>(a.res.states) + ((last - i) * Vw + v0) * 256, PL::SL, &row_full[s]);
+      }
+    } else if (role == 3 && lane == 0) {
+      // ---------------------------------------------------------------------------------------- dH, dV, partial sums
+      float* parts = dlend_part(g, a.dV);
+      for (int i = 0; i < n && !wait.dead; ++i) {
+        wait(&h_ready, i & 1);
+        umma::bulk_store(reinterpret_cast<uint8_t*>(a.dH) + ((last - i) * Vw + v0) * 256, sdH, PL::SL);
+        umma::bulk_commit();
+        umma::bulk_wait_read<0>();
+        arrive(&h_free);
+        wait(&v_ready, i & 1);
+        umma::bulk_store(reinterpret_cast<uint8_t*>(a.dV) + ((last - i) * Vw + v0) * 256, sdV, PL::SL);
+        umma::bulk_store(parts + ((last - i) * (Vw / 32) + v0 / 32) * KT, part_s, NG * 512);
+        umma::bulk_commit();
+        umma::bulk_wait_read<0>();
+        arrive(&v_free);
+      }
+      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
   }
-  umma::cp_async_wait<0>();
   __syncthreads();
-  if (warp == 0) umma::tmem_dealloc(tmem_base, tmem_cols(VS));
+  if (warp == 0) umma::tmem_dealloc(tmem_base, PL::TMEM);
 }
 
-int pick_vs(const Geo& g) {
-  const int chains = g.B * g.H;
-  if (g.Vw % 64 == 0 && chains * (g.Vw / 64) >= sm_count()) return 64;
-  return 32;
-}
-
-template <int VS>
-size_t tc_smem(bool bwd) {
-  return (size_t)4 * TILE_U4 * 16 + (size_t)(bwd ? 3 : 2) * (VS / 8) * 128 * 16 + (bwd ? (size_t)128 * VS * 2 : 0);
+// Columns of the value width per CTA, 32 or 64.  What bounds a chunk step is shared memory: the products read their
+// operands at its full width (46 cycles per 128 x 32 x 16 MMA, 48 at 64 columns, 64 at 128: the tile, 4 KB of each, dominates),
+// the four tiles are written to it, and loads and stores of the threads wait their turn.  64 columns read the tiles half as
+// often and leave the step 2.0 us as against 1.9 (forward, storing entry states), 2.2 as against 3.2 (reverse); at 128 it was 4.4.
+// So: 64, except for forward passes that store entry states and fit the SMs at 32 (fused prologue L=6001, 96 CTAs:
+// 117 us against 139; the KDA pass over 131072 tokens with one launch of each kind: 3.92 ms against 4.18).
+int pick_vs_fwd(const StateArgs& a) {
+  if (a.P_out) return 64;                               // Vw + K columns of 32 heads in few enough CTAs for one wave
+  return a.states && a.g.B * a.g.H * (a.g.Vw / 32) <= sm_count() ? 32 : 64;
 }
 
 template <int VS>
 int launch_fwd_vs(const StateArgs& a, cudaStream_t st) {
-  dim3 grid((a.g.Vw + (a.P_out ? a.g.K : 0)) / VS, a.g.H, a.g.B);
-  const size_t smem = tc_smem<VS>(false);
-  if (a.out) {
-    cudaFuncSetAttribute(state_fwd_tc_kernel<VS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    state_fwd_tc_kernel<VS, true><<<grid, 128, smem, st>>>(a);
-  } else {
-    cudaFuncSetAttribute(state_fwd_tc_kernel<VS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    state_fwd_tc_kernel<VS, false><<<grid, 128, smem, st>>>(a);
-  }
+  using PL = Plan<VS, false>;
+  const dim3 grid((a.g.Vw + (a.P_out ? a.g.K : 0)) / VS, a.g.H, a.g.B);
+  cudaFuncSetAttribute(state_fwd_tc_kernel<VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL::SMEM);
+  state_fwd_tc_kernel<VS><<<grid, PL::NT, PL::SMEM, st>>>(a);
   return launch_status();
 }
-
 template <int VS>
 int launch_bwd_vs(const StateArgs& a, cudaStream_t st) {
-  dim3 grid(a.g.Vw / VS, a.g.H, a.g.B);
-  const size_t smem = tc_smem<VS>(true);
-  cudaFuncSetAttribute(state_bwd_tc_kernel<VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  state_bwd_tc_kernel<VS><<<grid, 128, smem, st>>>(a);
+  using PL = Plan<VS, true>;
+  const dim3 grid(a.g.Vw / VS, a.g.H, a.g.B);
+  cudaFuncSetAttribute(state_bwd_tc_kernel<VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL::SMEM);
+  state_bwd_tc_kernel<VS><<<grid, PL::NT, PL::SMEM, st>>>(a);
   return launch_status();
 }
 
-}  // namespace
-
-bool state_tc_eligible(const Geo& g) {
-  return g.prec == DN_PREC_BF16 && !(g.flags & DN_STATE_FP32_MM) && g.C == 128 && g.K == 128 && g.Vw % 32 == 0;
-}
-
-static StateArgs with_range(const StateArgs& in) {
+StateArgs with_range(const StateArgs& in) {
   StateArgs a = in;
   if (a.c_end <= 0) { a.c_begin = 0; a.c_end = a.g.NC; }
   a.err = device_error_ptr();
   return a;
 }
 
+}  // namespace
+
+bool state_tc_eligible(const Geo& g) { return g.img; }
+
 int launch_state_fwd_tc(const StateArgs& in, cudaStream_t st) {
   const StateArgs a = with_range(in);
-  // with the transition columns aboard, 64-column slices keep one (batch, head)'s Vw + K columns in few
-  // enough CTAs to run in one wave; the chain's time is its per-chunk latency, not the slice width
-  const int vs = (a.P_out && a.g.Vw % 64 == 0) ? 64 : pick_vs(a.g);
-  switch (vs) {
-    case 64: return launch_fwd_vs<64>(a, st);
-    default: return launch_fwd_vs<32>(a, st);
-  }
+  return pick_vs_fwd(a) == 64 ? launch_fwd_vs<64>(a, st) : launch_fwd_vs<32>(a, st);
 }
 
 int launch_state_bwd_tc(const StateArgs& in, cudaStream_t st) {
   const StateArgs a = with_range(in);
-  // image path: slices of 32 columns (the dLambda_end partial sums are laid out per slice of 32, and the
-  // S strip of a 64-column slice would not fit in shared memory)
-  switch (a.g.img ? 32 : pick_vs(a.g)) {
-    case 64: return launch_bwd_vs<64>(a, st);
-    default: return launch_bwd_vs<32>(a, st);
-  }
+  return launch_bwd_vs<64>(a, st);
 }
 
 }  // namespace dn
