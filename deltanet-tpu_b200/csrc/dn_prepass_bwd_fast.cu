@@ -45,6 +45,53 @@ static_assert(SMEM_BYTES + 6 * 1024 <= 227 * 1024, "with the static arrays");
 
 __device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 1.f + umma::ex2_fast(-x * DN_LOG2E)); }
 
+// The kernel's code runs once per tile and did not fit the instruction cache when every product, wait and drain was
+// expanded in place (160 to 270 KB): 16 warps then stalled on fetches, and a few instructions more in each wait were worth
+// 15 %.  So these are calls, and loops over the 32 columns a warp drains stay rolled in pieces of eight.
+__device__ __noinline__ void product_call(uint32_t d, uint64_t ad, uint64_t bd, uint32_t a_step, uint32_t b_step, uint32_t idesc, int n, uint32_t acc) {
+#pragma unroll 4
+  for (int k = 0; k < n; ++k) {
+    umma::mma_bf16_warp(d, ad, bd, idesc, acc);
+    acc = 1u;
+    ad += a_step;
+    bd += b_step;
+  }
+}
+// D[128 x N] (+)= A B, operands as images whose panels lie pa / pb bytes apart; Kc: length of the contraction
+template <int N, bool A_MN, bool B_MN>
+__device__ __forceinline__ void product(const umma::Ctx& cx, const void* A, uint32_t pa, const void* B, uint32_t pb, int Kc, uint32_t col, bool acc) {
+  if (threadIdx.x >= 32 || cx.dead) return;
+  product_call(cx.tmem + col, umma::smem_desc(umma::smem_u32(A), A_MN ? 128u : pa, A_MN ? pa : 128u),
+               umma::smem_desc(umma::smem_u32(B), B_MN ? 128u : pb, B_MN ? pb : 128u), (A_MN ? 256u : 2u * pa) >> 4, (B_MN ? 256u : 2u * pb) >> 4,
+               umma::instr_desc(N, A_MN ? 1 : 0, B_MN ? 1 : 0), Kc / 16, acc ? 1u : 0u);
+}
+__device__ __forceinline__ void commit(const umma::Ctx& cx) {
+  if (threadIdx.x < 32 && !cx.dead) umma::mma_commit_warp(cx.bar);
+}
+__device__ __noinline__ bool bar_wait_call(uint64_t* bar, uint32_t parity, int* err) {
+  if (umma::mbar_wait(bar, parity)) return true;
+  umma::report_timeout(err);
+  return false;
+}
+// one warp polls, the others wait at the barrier; also a barrier among the CTA's threads
+__device__ __noinline__ bool cta_wait_call(uint64_t* bar, uint32_t parity, int* err, bool dead) {
+  bool bad = false;
+  if (threadIdx.x < 32 && !dead) bad = !bar_wait_call(bar, parity, err);
+  dead |= __syncthreads_or(bad) != 0;
+  umma::tc_fence_after();
+  return dead;
+}
+__device__ __forceinline__ void finish(umma::Ctx& cx) {       // waits for what has been committed
+  cx.dead = cta_wait_call(cx.bar, cx.phase, cx.err, cx.dead);
+  cx.phase ^= 1u;
+}
+__device__ __noinline__ void slot_load_call(void* dst, const void* src, uint64_t* bar) {
+  if (threadIdx.x == 0) {
+    umma::fence_async_smem();
+    umma::mbar_expect_tx(bar, IMGB);
+    umma::bulk_load(dst, src, IMGB, bar);
+  }
+}
 struct Slots {
   uint8_t* sm;
   uint64_t* bars;          // one per slot
@@ -52,50 +99,92 @@ struct Slots {
   int* err;
   __device__ __forceinline__ uint4* at(int s) const { return reinterpret_cast<uint4*>(sm + s * SLOT); }
   // one contiguous 32 KB operand image; ordinary accesses to the slot must lie before a barrier
-  __device__ __forceinline__ void load(int s, const __nv_bfloat16* src) {
-    if (threadIdx.x == 0) {
-      umma::fence_async_smem();
-      umma::mbar_expect_tx(bars + s, IMGB);
-      umma::bulk_load(at(s), src, IMGB, bars + s);
-    }
-  }
+  __device__ __forceinline__ void load(int s, const __nv_bfloat16* src) { slot_load_call(at(s), src, bars + s); }
   __device__ __forceinline__ void wait(int s) {
-    if (!umma::mbar_wait(bars + s, (phases >> s) & 1u)) umma::report_timeout(err);
+    bar_wait_call(bars + s, (phases >> s) & 1u, err);
     phases ^= 1u << s;
   }
 };
 
-// this thread's row (32 (warp & 3) + lane) and 32 columns (32 (warp >> 2)) of a 128-column block of tensor memory
-__device__ __forceinline__ void ld32(const umma::Ctx& cx, uint32_t addr, float (&v)[32]) {
-  if (!cx.dead) {
-    umma::tmem_ld32_nowait(addr, v);
-    umma::tmem_wait_ld();
-  } else {
+__device__ __forceinline__ void ld8(bool dead, uint32_t addr, float (&v)[8]) {
+  if (!dead) umma::tmem_ld8(addr, v);
+  else {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = 0.f;
+    for (int i = 0; i < 8; ++i) v[i] = 0.f;
   }
 }
-__device__ __forceinline__ void st32(uint32_t addr, const float (&v)[32]) {
+__device__ __forceinline__ void ld16(bool dead, uint32_t addr, float (&v)[16]) {
+  if (!dead) umma::tmem_ld16(addr, v);
+  else {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) umma::tmem_st8(addr + 8 * j, *reinterpret_cast<const float(*)[8]>(v + 8 * j));
-}
-__device__ __forceinline__ void image32(uint4* img, int pitch, int row, int group, const float (&v)[32]) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) img[(4 * group + j) * pitch + row] = umma::pack8p(v + 8 * j);
-}
-// One step of summing 32 values per lane over the warp's lanes, all at once: a lane hands over the half it drops; after
-// the steps 16, 8, 4, 2, 1 lane c holds the sum of value c.
-template <int O>
-__device__ __forceinline__ void fold(float (&v)[32], int lane) {
-  const bool up = lane & O;
-#pragma unroll
-  for (int i = 0; i < O; ++i) {
-    const float got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + O], O);
-    v[i] = (up ? v[i + O] : v[i]) + got;
+    for (int i = 0; i < 16; ++i) v[i] = 0.f;
   }
 }
-__device__ __forceinline__ void commit(const umma::Ctx& cx) {
-  if (threadIdx.x == 0 && !cx.dead) umma::mma_commit(cx.bar);
+// Drains of 32 columns (32 group ..) of the thread's row of tensor memory into an operand image.  addr: row and group included.
+__device__ __noinline__ void drain_plain(bool dead, uint32_t addr, uint4* img, int pitch, int row, int group, float sign) {
+  img += 4 * group * pitch + row;
+#pragma unroll 1
+  for (int j = 0; j < 2; ++j, img += 2 * pitch) {
+    float v[16];
+    ld16(dead, addr + 16 * j, v);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] *= sign;
+    img[0] = umma::pack8p(v);
+    img[pitch] = umma::pack8p(v + 8);
+  }
+}
+__device__ __noinline__ void drain_sub(bool dead, uint32_t addr, uint4* img, int row, int group) {       // image - accumulator, in place
+  img += 4 * group * 128 + row;
+#pragma unroll 1
+  for (int j = 0; j < 2; ++j, img += 256) {
+    float v[16], u[8], t[8];
+    umma::unpack8(img[0], u);
+    umma::unpack8(img[128], t);
+    ld16(dead, addr + 16 * j, v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { u[i] -= v[i]; t[i] -= v[8 + i]; }
+    img[0] = umma::pack8(u);
+    img[128] = umma::pack8(t);
+  }
+}
+// strictly lower triangle inside a document, times the scalar decay when lam is given; the diagonal apart when diag is
+__device__ __noinline__ void drain_masked(bool dead, uint32_t addr, uint4* img, int row, int group, float sign, const int* seg, const float* lam, float* diag) {
+  const int sr = seg[row];
+  const float lr = lam ? lam[row] * DN_LOG2E : 0.f;
+  img += 4 * group * 128 + row;
+#pragma unroll 1
+  for (int j = 0; j < 2; ++j, img += 256) {
+    const int c0 = group * 32 + 16 * j;
+    if (c0 > (row | 31)) {                              // (uniform over the warp) nothing of this piece survives
+      img[0] = img[128] = make_uint4(0, 0, 0, 0);
+      continue;
+    }
+    float v[16];
+    ld16(dead, addr + 16 * j, v);
+    if (diag && (unsigned)(row - c0) < 16u) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (c0 + i == row) diag[row] = v[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = c0 + i < row && sr == seg[c0 + i] ? sign * v[i] : 0.f;
+    if (lam) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] *= umma::ex2_fast(fminf(lr - lam[c0 + i] * DN_LOG2E, 0.f));
+    }
+    img[0] = umma::pack8p(v);
+    img[128] = umma::pack8p(v + 8);
+  }
+}
+// One step of summing 8 values per lane over the warp's lanes, all at once: a lane hands over the N it drops
+template <int N, int LANES>
+__device__ __forceinline__ void fold(float (&v)[8], int lane) {
+  const bool up = lane & LANES;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + N], LANES);
+    v[i] = (up ? v[i + N] : v[i]) + got;
+  }
 }
 // eight elements of a row of one of the operator's tensors, piece p
 __device__ __forceinline__ void ldrow8(const uint8_t* row, int p, int dt, float (&x)[8]) { load8(row, 8 * p, dt, x); }
@@ -232,139 +321,106 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         bet_s[tid] = bv;
       }
     }
-    // V_new = U - W S, in the place of U
-    auto vnew = [&](int slot, uint32_t col) {
-      float v[32];
-      ld32(cx, tb + col, v);
-      uint4* img = sl.at(slot);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float u[8];
-        umma::unpack8(img[(4 * group + j) * 128 + row], u);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) u[i] -= v[8 * j + i];
-        img[(4 * group + j) * 128 + row] = umma::pack8(u);
-      }
-    };
-    auto drain_dM = [&](int slot) {                     // masked (scalar gates: decayed) dM as an operand image; its diagonal apart
-      float v[32];
-      ld32(cx, tb + T_TMP, v);
-      const int sr = seg_s[row];
-      const float lr = SC ? lam_s[row] * DN_LOG2E : 0.f;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int j = group * 32 + i;
-        if (j == row) dmi_s[row] = v[i];
-        float f = 1.f;
-        if (SC) f = umma::ex2_fast(fminf(lr - lam_s[j] * DN_LOG2E, 0.f));
-        v[i] = (j < row && sr == seg_s[j]) ? v[i] * f : 0.f;
-      }
-      image32(sl.at(slot), 128, row, group, v);
-    };
-    auto drain_neg = [&](int slot, uint32_t col) {
-      float v[32];
-      ld32(cx, tb + col, v);
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = -v[i];
-      image32(sl.at(slot), 128, row, group, v);
-    };
+    // V_new = U - W S, in the place of U; dM masked (scalar gates: decayed), its diagonal apart
+    auto vnew = [&](int slot, uint32_t col) { drain_sub(cx.dead, tb + col, sl.at(slot), row, group); };
+    auto drain_dM = [&](int slot) { drain_masked(cx.dead, tb + T_TMP, sl.at(slot), row, group, 1.f, seg_s, SC ? lam_s : nullptr, dmi_s); };
+    auto drain_neg = [&](int slot, uint32_t col) { drain_plain(cx.dead, tb + col, sl.at(slot), 128, row, group, -1.f); };
     sl.wait(0);
     sl.wait(1);
     sl.wait(2);
     if constexpr (NH == 1) {
       umma::pre_issue_sync();
-      umma::issue<128, false, true>(cx, sl.at(0), sl.at(1), K, T_TMP, false);                      // W S
+      product<128, false, true>(cx, sl.at(0), 2048, sl.at(1), 2048, K, T_TMP, false);                      // W S
       commit(cx);
       umma::cp_async_wait<0>();                         // dO
-      umma::commit_wait_cta(cx);
+      finish(cx);
       sl.load(0, Tg);
       vnew(2, T_TMP);
       sl.wait(3);
       sl.wait(4);
       umma::pre_issue_sync();
-      umma::issue_pitched<128, false, false>(cx, sl.at(5), PB, sl.at(2), 2048, 128, T_TMP, false); // dM  = dO V_new^T
-      umma::issue_pitched<128, false, false>(cx, sl.at(5), PB, sl.at(1), 2048, 128, T_Q, false);   // dqe = dO S^T
+      product<128, false, false>(cx, sl.at(5), PB, sl.at(2), 2048, 128, T_TMP, false); // dM  = dO V_new^T
+      product<128, false, false>(cx, sl.at(5), PB, sl.at(1), 2048, 128, T_Q, false);   // dqe = dO S^T
       commit(cx);
-      umma::commit_wait_cta(cx);
-      umma::issue<128, false, false>(cx, sl.at(3), sl.at(1), 128, T_B, false);                     // -dW = dV S^T
-      umma::issue<128, false, false>(cx, sl.at(2), sl.at(4), 128, T_K, false);                     // dke = V_new dH^T
+      finish(cx);
+      product<128, false, false>(cx, sl.at(3), 2048, sl.at(1), 2048, 128, T_B, false);                     // -dW = dV S^T
+      product<128, false, false>(cx, sl.at(2), 2048, sl.at(4), 2048, 128, T_K, false);                     // dke = V_new dH^T
       commit(cx);
       drain_dM(5);
-      umma::commit_wait_cta(cx);
+      finish(cx);
       sl.load(2, Wg);
       sl.load(4, Ug);
       drain_neg(1, T_B);                                // dW
       sl.wait(0);
       umma::pre_issue_sync();
-      umma::issue<128, true, true>(cx, sl.at(0), sl.at(1), C, T_B, false);                         // dX = T^T dW
-      umma::issue<128, true, true>(cx, sl.at(0), sl.at(3), C, T_TMP, false);                       // dY = T^T dV
+      product<128, true, true>(cx, sl.at(0), 2048, sl.at(1), 2048, C, T_B, false);                         // dX = T^T dW
+      product<128, true, true>(cx, sl.at(0), 2048, sl.at(3), 2048, C, T_TMP, false);                       // dY = T^T dV
       commit(cx);
-      umma::commit_wait_cta(cx);
+      finish(cx);
     } else {
       sl.wait(3);
       sl.wait(4);
       umma::pre_issue_sync();
-      umma::issue<128, false, true>(cx, sl.at(0), sl.at(1), K, T_TMP, false);                      // W S, both halves
-      umma::issue<128, false, true>(cx, sl.at(0), sl.at(3), K, T_B, false);
+      product<128, false, true>(cx, sl.at(0), 2048, sl.at(1), 2048, K, T_TMP, false);                      // W S, both halves
+      product<128, false, true>(cx, sl.at(0), 2048, sl.at(3), 2048, K, T_B, false);
       commit(cx);
       umma::cp_async_wait<0>();
-      umma::commit_wait_cta(cx);
+      finish(cx);
       sl.load(0, dVg);
       vnew(2, T_TMP);
       vnew(4, T_B);
       umma::pre_issue_sync();
-      umma::issue_pitched<128, false, false>(cx, sl.at(5), PB, sl.at(2), 2048, 128, T_TMP, false); // dM, dqe: first half
-      umma::issue_pitched<128, false, false>(cx, sl.at(5), PB, sl.at(1), 2048, 128, T_Q, false);
+      product<128, false, false>(cx, sl.at(5), PB, sl.at(2), 2048, 128, T_TMP, false); // dM, dqe: first half
+      product<128, false, false>(cx, sl.at(5), PB, sl.at(1), 2048, 128, T_Q, false);
       commit(cx);
-      umma::commit_wait_cta(cx);
+      finish(cx);
       stage_dO(sl.at(5), a.d_out, dO_off + 128, dO_pitch, rows, vr / 8 - 16, qdt);
       sl.wait(0);
-      umma::issue<128, false, false>(cx, sl.at(0), sl.at(1), 128, T_B, false);                     // -dW: first half
+      product<128, false, false>(cx, sl.at(0), 2048, sl.at(1), 2048, 128, T_B, false);                     // -dW: first half
       commit(cx);
       umma::cp_async_wait<0>();
-      umma::commit_wait_cta(cx);
+      finish(cx);
       sl.load(0, dVg + HN);
       sl.load(1, dHg);
       umma::pre_issue_sync();
-      umma::issue_pitched<128, false, false>(cx, sl.at(5), PB, sl.at(4), 2048, 128, T_TMP, true);  // second half
-      umma::issue_pitched<128, false, false>(cx, sl.at(5), PB, sl.at(3), 2048, 128, T_Q, true);
+      product<128, false, false>(cx, sl.at(5), PB, sl.at(4), 2048, 128, T_TMP, true);  // second half
+      product<128, false, false>(cx, sl.at(5), PB, sl.at(3), 2048, 128, T_Q, true);
       commit(cx);
-      umma::commit_wait_cta(cx);
+      finish(cx);
       sl.wait(0);
       sl.wait(1);
-      umma::issue<128, false, false>(cx, sl.at(0), sl.at(3), 128, T_B, true);
-      umma::issue<128, false, false>(cx, sl.at(2), sl.at(1), 128, T_K, false);                     // dke: first half
+      product<128, false, false>(cx, sl.at(0), 2048, sl.at(3), 2048, 128, T_B, true);
+      product<128, false, false>(cx, sl.at(2), 2048, sl.at(1), 2048, 128, T_K, false);                     // dke: first half
       commit(cx);
       drain_dM(5);
-      umma::commit_wait_cta(cx);
+      finish(cx);
       sl.load(1, dHg + HN);                             // (slot 0 keeps the second half of dV)
       sl.load(2, Tg);
       drain_neg(3, T_B);                                // dW
       sl.wait(1);
       sl.wait(2);
       umma::pre_issue_sync();
-      umma::issue<128, false, false>(cx, sl.at(4), sl.at(1), 128, T_K, true);                      // dke: second half
-      umma::issue<128, true, true>(cx, sl.at(2), sl.at(3), C, T_B, false);                         // dX = T^T dW
-      umma::issue<128, true, true>(cx, sl.at(2), sl.at(0), C, T_TMP, false);                       // dY: second half
+      product<128, false, false>(cx, sl.at(4), 2048, sl.at(1), 2048, 128, T_K, true);                      // dke: second half
+      product<128, true, true>(cx, sl.at(2), 2048, sl.at(3), 2048, C, T_B, false);                         // dX = T^T dW
+      product<128, true, true>(cx, sl.at(2), 2048, sl.at(0), 2048, C, T_TMP, false);                       // dY: second half
       commit(cx);
-      umma::commit_wait_cta(cx);
+      finish(cx);
     }
     auto drain_dX = [&](int slot) {                     // as operand image; the accumulator itself stays for T1
-      float v[32];
-      ld32(cx, tb + T_B, v);
       if (trunc) {
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+          float v[8];
+          ld8(cx.dead, tb + T_B + 8 * j, v);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = bf16r(v[i]);
-        st32(tb + T_B, v);
+          for (int i = 0; i < 8; ++i) v[i] = bf16r(v[i]);
+          umma::tmem_st8(tb + T_B + 8 * j, v);
+        }
         umma::tmem_wait_st();
       }
-      image32(sl.at(slot), 128, row, group, v);
+      drain_plain(cx.dead, tb + T_B, sl.at(slot), 128, row, group, 1.f);
     };
-    auto drain_dY = [&](int slot) {
-      float v[32];
-      ld32(cx, tb + T_TMP, v);
-      image32(sl.at(slot), PP, row, group, v);
-    };
+    auto drain_dY = [&](int slot) { drain_plain(cx.dead, tb + T_TMP, sl.at(slot), PP, row, group, 1.f); };
     // dv = dY w_act, dw = dY v (+ sigmoid adjoint; summed over a value head's columns when w is one scalar per head)
     auto vphase = [&](int slot, int half) {
       const uint4* img = sl.at(slot);
@@ -372,7 +428,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       const size_t tok = tok0 + (live ? rx : 0);
       const int steps_per_head = g.V / 32;
       float sw = 0.f;
-#pragma unroll 2
+#pragma unroll 1
       for (int it = 0; it < 4; ++it) {
         const int p = it * 4 + rp, col = half * 128 + 8 * p;
         if (col - 8 * rp >= vr) break;                  // (uniform: value widths are multiples of 32)
@@ -414,11 +470,11 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       sl.wait(2);
       sl.wait(4);
       umma::pre_issue_sync();
-      umma::issue<128, false, false>(cx, sl.at(0), sl.at(2), 128, T_TMP, false);                   // -dA = dX W^T + dY U^T
-      umma::issue_pitched<128, false, false>(cx, sl.at(1), PB, sl.at(4), 2048, 128, T_TMP, true);
+      product<128, false, false>(cx, sl.at(0), 2048, sl.at(2), 2048, 128, T_TMP, false);                   // -dA = dX W^T + dY U^T
+      product<128, false, false>(cx, sl.at(1), PB, sl.at(4), 2048, 128, T_TMP, true);
       commit(cx);
       vphase(1, 0);
-      umma::commit_wait_cta(cx);
+      finish(cx);
     } else {
       sl.load(0, dVg);
       sl.load(1, Wg);
@@ -426,41 +482,28 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       drain_dY(4);
       sl.wait(0);
       umma::pre_issue_sync();
-      umma::issue<128, true, true>(cx, sl.at(2), sl.at(0), C, T_TMP, false);                       // dY: first half
+      product<128, true, true>(cx, sl.at(2), 2048, sl.at(0), 2048, C, T_TMP, false);                       // dY: first half
       commit(cx);
-      umma::commit_wait_cta(cx);
+      finish(cx);
       sl.load(0, Ug);
       drain_dY(2);
       sl.wait(0);
       sl.wait(1);
       umma::pre_issue_sync();
-      umma::issue<128, false, false>(cx, sl.at(3), sl.at(1), 128, T_TMP, false);                   // -dA = dX W^T + dY U^T
-      umma::issue_pitched<128, false, false>(cx, sl.at(2), PB, sl.at(0), 2048, 128, T_TMP, true);
+      product<128, false, false>(cx, sl.at(3), 2048, sl.at(1), 2048, 128, T_TMP, false);                   // -dA = dX W^T + dY U^T
+      product<128, false, false>(cx, sl.at(2), PB, sl.at(0), 2048, 128, T_TMP, true);
       commit(cx);
-      umma::commit_wait_cta(cx);
+      finish(cx);
       sl.load(0, Ug + HN);
       vphase(2, 0);
       sl.wait(0);
-      umma::issue_pitched<128, false, false>(cx, sl.at(4), PB, sl.at(0), 2048, 128, T_TMP, true);
+      product<128, false, false>(cx, sl.at(4), PB, sl.at(0), 2048, 128, T_TMP, true);
       commit(cx);
       vphase(4, 1);
-      umma::commit_wait_cta(cx);
+      finish(cx);
     }
     // ---- dA into slot 4 (dM is in slot 5); slots 0 .. 3 are free
-    {
-      float v[32];
-      ld32(cx, tb + T_TMP, v);
-      const int sr = seg_s[row];
-      const float lr = SC ? lam_s[row] * DN_LOG2E : 0.f;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int j = group * 32 + i;
-        float f = 1.f;
-        if (SC) f = umma::ex2_fast(fminf(lr - lam_s[j] * DN_LOG2E, 0.f));
-        v[i] = (j < row && sr == seg_s[j]) ? -v[i] * f : 0.f;
-      }
-      image32(sl.at(4), 128, row, group, v);
-    }
+    drain_masked(cx.dead, tb + T_TMP, sl.at(4), row, group, -1.f, seg_s, SC ? lam_s : nullptr, nullptr);
 
     // ---- key side: rows of q, k, b in the row mapping
     const bool live = rx < rows;
@@ -575,50 +618,53 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     // ---- dqe, dX, dke scaled where they lie; the column sums of ke dke
     {
       const bool first = seg_s[row] == seg_s[0], last = seg_s[row] == seg_s[C - 1];
-      float v[32];
       const float el = SC ? (first ? umma::exp_neg(fminf(lam_s[row], 0.f)) : 0.f) : 0.f;
-      auto scale_first = [&](uint32_t col) {
-        ld32(cx, tb + col, v);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] *= SC ? el : (first ? EDGE[group * 32 + i] : 0.f);
-        st32(tb + col, v);
-      };
-      scale_first(T_Q);
-      scale_first(T_B);
-      ld32(cx, tb + T_K, v);
       const bool on = last && row < rows;
       const float eks = SC ? umma::exp_neg(fminf(lam_s[C - 1] - lam_s[row], 0.f)) : 0.f;
       const uint8_t* kr = reinterpret_cast<const uint8_t*>(a.k) + ((tok0 + (row < rows ? row : 0)) * g.Hk + h / g.qk_div) * g.K * qes;
-      float od[32];
-#pragma unroll
+      const float rkr = rk_s[row];
+      Raw8 knext = ldraw(kr, group * 4 < kp ? group * 4 : 0, qdt);
+      float pk = 0.f;
+#pragma unroll 1
       for (int j = 0; j < 4; ++j) {
-        const int p = group * 4 + j;
-        float kh[8];
-        ldrow8(kr, p < kp ? p : 0, qdt, kh);
+        const int p = group * 4 + j, c0 = group * 32 + 8 * j;
+        float v[8], w[8], x[8], kh[8], od[8];
+        const Raw8 kraw = knext;
+        if (j < 3) knext = ldraw(kr, p + 1 < kp ? p + 1 : 0, qdt);
+        ld8(cx.dead, tb + T_Q + 8 * j, v);
+        ld8(cx.dead, tb + T_B + 8 * j, w);
+        ld8(cx.dead, tb + T_K + 8 * j, x);
+        cvraw(kraw, qdt, kh);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int c = group * 32 + 8 * j + i;
-          kh[i] *= rk_s[row];
+          const float e1 = SC ? el : (first ? EDGE[c0 + i] : 0.f);
+          v[i] *= e1;
+          w[i] *= e1;
+          kh[i] *= rkr;
           if (round_in) kh[i] = bf16r(kh[i]);
-          const float e = SC ? eks : umma::ex2_fast(fminf(LAM[(C - 1) * LPF + c] - LAM[row * LPF + c], 0.f));
-          od[8 * j + i] = on && p < kp ? v[8 * j + i] * (kh[i] * e) : 0.f;
-          v[8 * j + i] *= SC ? (last ? eks : 0.f) : (last ? EDGE[128 + c] : 0.f);
+          const float e = SC ? eks : umma::ex2_fast(fminf(LAM[(C - 1) * LPF + c0 + i] - LAM[row * LPF + c0 + i], 0.f));
+          od[i] = on && p < kp ? x[i] * (kh[i] * e) : 0.f;
+          x[i] *= SC ? (last ? eks : 0.f) : (last ? EDGE[128 + c0 + i] : 0.f);
+        }
+        umma::tmem_st8(tb + T_Q + 8 * j, v);
+        umma::tmem_st8(tb + T_B + 8 * j, w);
+        umma::tmem_st8(tb + T_K + 8 * j, x);
+        if (SC) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) pk += od[i];
+        } else {
+          // sums over the warp's 32 rows: lane l ends with channel c0 + (l >> 2)'s
+          fold<4, 16>(od, lane);
+          fold<2, 8>(od, lane);
+          fold<1, 4>(od, lane);
+          od[0] += __shfl_xor_sync(0xffffffffu, od[0], 2);
+          od[0] += __shfl_xor_sync(0xffffffffu, od[0], 1);
+          if ((lane & 3) == 0) PS[quarter * 128 + c0 + (lane >> 2)] = od[0];
         }
       }
-      st32(tb + T_K, v);
       if (SC) {
-        float s = 0.f;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) s += od[i];
-        s = warp_sum(s);
-        if (lane == 0) PS[warp] = s;
-      } else {
-        fold<16>(od, lane);
-        fold<8>(od, lane);
-        fold<4>(od, lane);
-        fold<2>(od, lane);
-        fold<1>(od, lane);
-        PS[quarter * 128 + group * 32 + lane] = od[0];
+        pk = warp_sum(pk);
+        if (lane == 0) PS[warp] = pk;
       }
       umma::tmem_wait_st();
     }
@@ -636,12 +682,12 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         BI[p * PP + rx] = umma::pack8(be);
       }
       umma::pre_issue_sync();
-      umma::issue_pitched<128, false, true>(cx, sl.at(4), 2048, KI, PB, C, T_B, true);       // (dA f)   k_hat
-      umma::issue_pitched<128, false, true>(cx, sl.at(5), 2048, KI, PB, C, T_Q, true);       // (dM f)   k_hat
-      umma::issue_pitched<128, true, true>(cx, sl.at(4), 2048, BI, PB, C, T_K, true);        // (dA f)^T (b k_hat)
-      umma::issue_pitched<128, true, true>(cx, sl.at(5), 2048, QI, PB, C, T_K, true);        // (dM f)^T q_hat
+      product<128, false, true>(cx, sl.at(4), 2048, KI, PB, C, T_B, true);       // (dA f)   k_hat
+      product<128, false, true>(cx, sl.at(5), 2048, KI, PB, C, T_Q, true);       // (dM f)   k_hat
+      product<128, true, true>(cx, sl.at(4), 2048, BI, PB, C, T_K, true);        // (dA f)^T (b k_hat)
+      product<128, true, true>(cx, sl.at(5), 2048, QI, PB, C, T_K, true);        // (dM f)^T q_hat
       commit(cx);
-      umma::commit_wait_cta(cx);
+      finish(cx);
     } else {
       load_pieces(rp);
 #pragma unroll 1
@@ -668,27 +714,23 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
           }
         }
         if (grp >= 2) {                                 // the set was read by the products of group - 2
-          bool ok = true;
-          if (warp == 0 && !cx.dead) ok = umma::mbar_wait(&gbar[grp & 1], (gph >> (grp & 1)) & 1u);
+          cx.dead = cta_wait_call(&gbar[grp & 1], (gph >> (grp & 1)) & 1u, a.err, cx.dead);
           gph ^= 1u << (grp & 1);
-          if (__syncthreads_or(!ok)) { cx.dead = true; umma::report_timeout(a.err); }
         }
         KF[rp * PP + rx] = umma::pack8(kh);
         QF[rp * PP + rx] = umma::pack8(qh);
         BF[rp * PP + rx] = umma::pack8(be);
         umma::pre_issue_sync();
-        umma::issue_pitched<32, false, true>(cx, sl.at(4), 2048, KF, PB, C, T_B + 32 * grp, true);       // dA (k / f)
-        umma::issue_pitched<32, false, true>(cx, sl.at(5), 2048, KF, PB, C, T_Q + 32 * grp, true);       // dM (k / f)
-        umma::issue_pitched<32, true, true>(cx, sl.at(4), 2048, BF, PB, C, T_K + 32 * grp, true);        // dA^T (beta f)
-        umma::issue_pitched<32, true, true>(cx, sl.at(5), 2048, QF, PB, C, T_K + 32 * grp, true);        // dM^T (q f)
-        if (tid == 0 && !cx.dead) umma::mma_commit(&gbar[grp & 1]);
+        product<32, false, true>(cx, sl.at(4), 2048, KF, PB, C, T_B + 32 * grp, true);       // dA (k / f)
+        product<32, false, true>(cx, sl.at(5), 2048, KF, PB, C, T_Q + 32 * grp, true);       // dM (k / f)
+        product<32, true, true>(cx, sl.at(4), 2048, BF, PB, C, T_K + 32 * grp, true);        // dA^T (beta f)
+        product<32, true, true>(cx, sl.at(5), 2048, QF, PB, C, T_K + 32 * grp, true);        // dM^T (q f)
+        if (warp == 0 && !cx.dead) umma::mma_commit_warp(&gbar[grp & 1]);
         if (grp < 3) load_pieces((grp + 1) * 4 + rp);
       }
-      bool ok = true;
-      if (warp == 0 && !cx.dead) ok = umma::mbar_wait(&gbar[0], gph & 1u) && umma::mbar_wait(&gbar[1], (gph >> 1) & 1u);
+      cx.dead = cta_wait_call(&gbar[0], gph & 1u, a.err, cx.dead);
+      cx.dead = cta_wait_call(&gbar[1], (gph >> 1) & 1u, a.err, cx.dead);
       gph ^= 3u;
-      if (__syncthreads_or(!ok)) { cx.dead = true; umma::report_timeout(a.err); }
-      umma::tc_fence_after();
     }
     if (tid == 0 && e_item + (int)gridDim.x < a.items) {      // the next tile's images on their way into L2
       const int nx = e_item + gridDim.x;
