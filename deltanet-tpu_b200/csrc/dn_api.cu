@@ -146,7 +146,7 @@ static size_t bwd_kernel_scratch(const Geo& g) {
 static size_t staging_bytes(const Geo& g) {
   // f32 staging of gradients that must be summed over heads afterwards
   size_t rows = (size_t)g.B * g.L, tot = 0;
-  if (g.qk_div > 1) tot += 2 * align_up(rows * g.H * g.K * sizeof(float));
+  if (g.qk_div > 1 && prepass_bwd_group(g, g.NC) == 1) tot += 2 * align_up(rows * g.H * g.K * sizeof(float));
   if (g.gH != g.H) tot += align_up(rows * g.H * g.gC * sizeof(float));
   if (g.bH != g.H) tot += align_up(rows * g.H * g.bC * sizeof(float));
   if (g.wH != g.Hv) tot += align_up(rows * g.Hv * g.wC * sizeof(float));
@@ -269,7 +269,8 @@ int plan_prepass_bwd(const Geo& g, const void* q, const void* k, const void* v, 
   pl.dq = dq; pl.dk = dk; pl.dg = dg; pl.db = db; pl.dw = dw;
   a.dq_dt = g.qkv_dt; a.dg_dt = a.db_dt = a.dw_dt = g.gate_dt;
   auto take = [&](size_t nfl) { float* r = reinterpret_cast<float*>(p); p += align_up(nfl * sizeof(float)); return r; };
-  if (g.qk_div > 1) { pl.sq = take(rows * g.H * g.K); pl.sk = take(rows * g.H * g.K); a.dq = pl.sq; a.dk = pl.sk; a.dq_dt = DN_F32; }
+  a.group = prepass_bwd_group(g, g.NC);
+  if (g.qk_div > 1 && a.group == 1) { pl.sq = take(rows * g.H * g.K); pl.sk = take(rows * g.H * g.K); a.dq = pl.sq; a.dk = pl.sk; a.dq_dt = DN_F32; }
   if (g.gH != g.H) { pl.sg = take(rows * g.H * g.gC); a.dg = pl.sg; a.dg_dt = DN_F32; }
   if (g.bH != g.H) { pl.sb = take(rows * g.H * g.bC); a.db = pl.sb; a.db_dt = DN_F32; }
   if (g.wH != g.Hv) { pl.sw = take(rows * g.Hv * g.wC); a.dw = pl.sw; a.dw_dt = DN_F32; }
@@ -524,7 +525,7 @@ int dn_launch_count(const dn_shape* s, int backward, int recompute) {
   if (!backward) return split_f ? 4 : 2;
   int n = split_b ? 4 : 2;
   if (recompute) n += 2;
-  n += (g.qk_div > 1 ? 2 : 0) + (g.gH != g.H) + (g.bH != g.H) + (g.wH != g.Hv);   // head sums
+  n += (g.qk_div > 1 && prepass_bwd_group(g, g.NC) == 1 ? 2 : 0) + (g.gH != g.H) + (g.bH != g.H) + (g.wH != g.Hv);   // head sums
   return n;
 }
 

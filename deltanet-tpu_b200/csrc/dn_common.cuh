@@ -104,12 +104,11 @@ __host__ __device__ __forceinline__ float* dlend_part(const Geo& g, float* dV) {
   return dV + (size_t)g.B * g.H * g.NC * 128 * g.Vw / 2;
 }
 
-// T's slot holds a bf16 image in its first half; the first word of the second half tells the backward that the decay of
-// this tile is strong (channel-wise decay only)
-__host__ __device__ __forceinline__ int* strong_flag_ptr(const dn_residuals& res, size_t tile) {
-  return reinterpret_cast<int*>(res.T + tile * 128 * 128 + 128 * 64);
-}
-__device__ __forceinline__ bool strong_flag(const dn_residuals& res, size_t tile) { return *strong_flag_ptr(res, tile) != 0; }
+// T's slot holds a bf16 image in its first half.  In the second half the forward leaves for the backward: a word that
+// says whether the decay of the tile is strong (channel-wise decay only), and from float 128 on the 128 + 128 normalisers
+// of the rows of q and k.
+__host__ __device__ __forceinline__ float* tile_extra(const dn_residuals& res, size_t tile) { return res.T + tile * 128 * 128 + 128 * 64; }
+__device__ __forceinline__ bool strong_flag(const dn_residuals& res, size_t tile) { return *reinterpret_cast<const int*>(tile_extra(res, tile)) != 0; }
 
 // element index of (row, col) in a residual tile of 128 rows (image layout) or `ncols` columns (row-major)
 __host__ __device__ __forceinline__ size_t rix(bool img, int row, int col, int ncols) {

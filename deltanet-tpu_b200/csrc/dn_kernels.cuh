@@ -66,6 +66,7 @@ struct PrepassBwdArgs {
   int* err;                        // device error word (bounded waits report here)
   int c_begin, c_end;              // chunk range [c_begin, c_end) of every (batch, head); tensor-core path only
   bool bulk_v;                     // v, w, dv, dw move by bulk copies (set by the launcher)
+  int group;                       // heads one CTA takes in turn, summing their dq and dk (see prepass_bwd_group)
 };
 
 // Called right after every kernel launch of the library: DN_OK or DN_ERR_CUDA_LAUNCH from
@@ -101,6 +102,7 @@ bool prepass_bwd_tc_eligible(const Geo& g);
 // the kernel for all tiles but those marked for strong decay, and whether none can be (scalar gates)
 int launch_prepass_bwd_fast(const PrepassBwdArgs& a, cudaStream_t st);
 bool prepass_bwd_scalar_route(const Geo& g);
+int prepass_bwd_group(const Geo& g, int chunks);  // heads per CTA whose dq, dk it sums itself (1: they are staged)
 size_t prepass_bwd_tc_scratch_per_cta(const Geo& g);
 int launch_canonical_segments(const int32_t* raw, const int32_t* first_is_new, int32_t* out,
                               int B, int L, cudaStream_t st);

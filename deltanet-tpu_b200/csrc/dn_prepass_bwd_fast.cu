@@ -33,14 +33,14 @@ constexpr int PP = 130;                               // uint4 per panel of imag
 constexpr uint32_t PB = PP * 16;
 constexpr int SLOT = 16 * PB;
 constexpr int LPF = 132;                              // row pitch (floats) of Lambda, which takes slots 0 and 1 after the products
-constexpr int OFF_GI = C * LPF * 4;                   // then: two sets of three 128 x 32 images (k / f, q f, beta f), and later
+constexpr int OFF_GI = C * LPF * 4;                   // then: three 128 x 64 images (k / f, q f, beta f), and later
 constexpr int OFF_RK = OFF_GI, OFF_RQ = OFF_RK + SLOT, OFF_RB = OFF_RQ + SLOT;      // the raw k, q and b
 constexpr int OFF_MISC = OFF_RB + 2 * SLOT;           // partial sums
 constexpr int MISC_FLOATS = 512 + 256 + 4 * 512 + 512;
 constexpr int SMEM_BYTES = OFF_MISC + MISC_FLOATS * 4;
 constexpr uint32_t T_Q = 0, T_K = 128, T_B = 256, T_TMP = 384;
 constexpr uint32_t IMGB = 32768;
-static_assert(OFF_GI + 2 * 3 * 4 * (int)PB <= 4 * SLOT && OFF_MISC >= 6 * SLOT, "regions");
+static_assert(OFF_GI + 3 * 8 * (int)PB <= 4 * SLOT && OFF_MISC >= 6 * SLOT, "regions");
 static_assert(SMEM_BYTES + 6 * 1024 <= 227 * 1024, "with the static arrays");
 
 __device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 1.f + umma::ex2_fast(-x * DN_LOG2E)); }
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
   using CF = InCfg<MODE>;
   constexpr int NH = VW / 128;
   extern __shared__ __align__(128) uint8_t sm[];
-  __shared__ uint64_t mma_bar, slot_bar[6], gbar[2];
+  __shared__ uint64_t mma_bar, slot_bar[6];
   __shared__ uint32_t tmem_base;
   __shared__ int seg_s[C];
   __shared__ int cut_s[8];
@@ -236,8 +236,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
   if (tid == 0) {
     umma::mbar_init(&mma_bar, 1);
     for (int i = 0; i < 6; ++i) umma::mbar_init(&slot_bar[i], 1);
-    umma::mbar_init(&gbar[0], 1);
-    umma::mbar_init(&gbar[1], 1);
     umma::fence_mbar_init();
   }
   if (warp == 0) umma::tmem_alloc(&tmem_base, 512);
@@ -246,7 +244,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
   umma::tc_fence_after();
   umma::Ctx cx{tmem_base, &mma_bar, 0u, a.err, false};
   Slots sl{sm, slot_bar, 0u, a.err};
-  uint32_t gph = 0u;
   const uint32_t tb = cx.tmem + ((uint32_t)(quarter * 32) << 16) + group * 32;
 
   const bool l2 = g.flags & DN_QK_L2NORM, trunc = g.flags & DN_TRUNC_DT_BF16;
@@ -258,10 +255,14 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
   const uint32_t qes = qdt == DN_BF16 ? 2 : 4, ges = gdt == DN_BF16 ? 2 : 4;
   const int vr = g.G * g.V;                             // value columns that exist
 
-  for (int e_item = blockIdx.x; e_item < a.items; e_item += gridDim.x) {
-    const int bh = e_item % (g.B * g.H), c_idx = a.c_begin + e_item / (g.B * g.H);
-    const int h = bh % g.H, b = bh / g.H, t0 = c_idx * C;
-    const size_t ibase = (size_t)bh * g.NC + c_idx;
+  // A CTA takes the D heads that share a key head one after the other and adds up their dq and dk in its scratch (see
+  // prepass_bwd_grouped); otherwise D = 1.
+  const int D = SC ? a.group : 1, HG = g.H / D;
+  for (int e_item = blockIdx.x; e_item < a.items / D; e_item += gridDim.x)
+  for (int hd = 0; hd < D; ++hd) {
+    const int bg = e_item % (g.B * HG), c_idx = a.c_begin + e_item / (g.B * HG);
+    const int b = bg / HG, h = (bg - b * HG) * D + hd, t0 = c_idx * C;
+    const size_t ibase = (size_t)(b * g.H + h) * g.NC + c_idx;
     if (!SC && strong_flag(a.res, ibase)) continue;     // uniform over the CTA
     const int rows = g.L - t0 < C ? g.L - t0 : C;
     const size_t tok0 = (size_t)b * g.L + t0;
@@ -292,6 +293,8 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     if (tid < C) {
       const int sg = seg_at(a.seg, b, t0 + tid, g.L);
       seg_s[tid] = sg;
+      rq_s[tid] = __ldg(tile_extra(a.res, ibase) + 128 + tid);
+      rk_s[tid] = __ldg(tile_extra(a.res, ibase) + 256 + tid);
       // dLambda_end = [one document] e^{Lambda_end} sum_v dH S (gdn2.py:759-762) from the reverse chain's per-slice sums
       float acc = 0.f;
       const float* part = dlend_part(g, const_cast<float*>(a.dV)) + ibase * (VW / 32) * K + tid;
@@ -422,10 +425,18 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     };
     auto drain_dY = [&](int slot) { drain_plain(cx.dead, tb + T_TMP, sl.at(slot), PP, row, group, 1.f); };
     // dv = dY w_act, dw = dY v (+ sigmoid adjoint; summed over a value head's columns when w is one scalar per head)
+    // The rows of v and w are read one step ahead of their use.
+    const bool vlive = rx < rows;
+    const size_t vtok = tok0 + (vlive ? rx : 0);
+    Raw8 vraw, wraw;
+    auto v_load = [&](int col) {
+      const int cc = col < vr ? col : 0, hv = h * g.G + cc / g.V, cv = cc % g.V;
+      vraw = ldraw(reinterpret_cast<const uint8_t*>(a.v) + ((vtok * g.Hv + hv) * g.V + cv) * qes, 0, qdt);
+      if (wC == 1) wraw.a.x = __float_as_uint(ldf_ro(a.w, vtok * g.wH + g.w_head(hv), gdt));
+      else wraw = ldraw(reinterpret_cast<const uint8_t*>(a.w) + ((vtok * g.wH + g.w_head(hv)) * wC + cv) * ges, 0, gdt);
+    };
     auto vphase = [&](int slot, int half) {
       const uint4* img = sl.at(slot);
-      const bool live = rx < rows;
-      const size_t tok = tok0 + (live ? rx : 0);
       const int steps_per_head = g.V / 32;
       float sw = 0.f;
 #pragma unroll 1
@@ -433,16 +444,13 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         const int p = it * 4 + rp, col = half * 128 + 8 * p;
         if (col - 8 * rp >= vr) break;                  // (uniform: value widths are multiples of 32)
         const int hv = h * g.G + col / g.V, cv = col % g.V;
-        const size_t vo = (tok * g.Hv + hv) * g.V + cv;
         float vv[8], ww[8], dy[8], dv8[8], dw8[8];
-        load8(a.v, vo, qdt, vv);
+        cvraw(vraw, qdt, vv);
         if (wC == 1) {
-          const float w1 = ldf_ro(a.w, tok * g.wH + g.w_head(hv), gdt);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) ww[i] = w1;
-        } else {
-          load8(a.w, (tok * g.wH + g.w_head(hv)) * wC + cv, gdt, ww);
-        }
+          for (int i = 0; i < 8; ++i) ww[i] = __uint_as_float(wraw.a.x);
+        } else cvraw(wraw, gdt, ww);
+        if (it < 3) v_load(col + 32);
         umma::unpack8(img[p * PP + rx], dy);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -452,14 +460,14 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
           dw8[i] = dwv;
           sw += dwv;
         }
-        if (live) {
-          strow8(a.dv, vo, qdt, dv8);
-          if (wC != 1) strow8(a.dw, (tok * g.Hv + hv) * wC + cv, a.dw_dt, dw8);
+        if (vlive) {
+          strow8(a.dv, (vtok * g.Hv + hv) * g.V + cv, qdt, dv8);
+          if (wC != 1) strow8(a.dw, (vtok * g.Hv + hv) * wC + cv, a.dw_dt, dw8);
         }
         if (wC == 1 && (it + 1) % steps_per_head == 0) {
           sw += __shfl_xor_sync(0xffffffffu, sw, 1);
           sw += __shfl_xor_sync(0xffffffffu, sw, 2);
-          if (live && rp == 0) stf(a.dw, tok * g.Hv + hv, sw, a.dw_dt);
+          if (vlive && rp == 0) stf(a.dw, vtok * g.Hv + hv, sw, a.dw_dt);
           sw = 0.f;
         }
       }
@@ -473,6 +481,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       product<128, false, false>(cx, sl.at(0), 2048, sl.at(2), 2048, 128, T_TMP, false);                   // -dA = dX W^T + dY U^T
       product<128, false, false>(cx, sl.at(1), PB, sl.at(4), 2048, 128, T_TMP, true);
       commit(cx);
+      v_load(8 * rp);
       vphase(1, 0);
       finish(cx);
     } else {
@@ -493,9 +502,11 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       product<128, false, false>(cx, sl.at(3), 2048, sl.at(1), 2048, 128, T_TMP, false);                   // -dA = dX W^T + dY U^T
       product<128, false, false>(cx, sl.at(2), PB, sl.at(0), 2048, 128, T_TMP, true);
       commit(cx);
+      v_load(8 * rp);
       finish(cx);
       sl.load(0, Ug + HN);
       vphase(2, 0);
+      v_load(128 + 8 * rp);
       sl.wait(0);
       product<128, false, false>(cx, sl.at(4), PB, sl.at(0), 2048, 128, T_TMP, true);
       commit(cx);
@@ -511,28 +522,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     const uint8_t* krow = reinterpret_cast<const uint8_t*>(a.k) + (tokx * g.Hk + h / g.qk_div) * g.K * qes;
     const uint8_t* qrow = reinterpret_cast<const uint8_t*>(a.q) + (tokx * g.Hk + h / g.qk_div) * g.K * qes;
     const uint8_t* brow = reinterpret_cast<const uint8_t*>(a.b) + (tokx * g.bH + g.gate_head(h, g.bH)) * bC * ges;
-    float rq = 1.f, rk = 1.f;
-    if (l2) {
-      float sq = 0.f, sk = 0.f;
-#pragma unroll
-      for (int it = 0; it < 4; ++it) {
-        const int p = it * 4 + rp;
-        if (p < kp) {
-          float f[8];
-          ldrow8(qrow, p, qdt, f);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) sq = fmaf(f[i], f[i], sq);
-          ldrow8(krow, p, qdt, f);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) sk = fmaf(f[i], f[i], sk);
-        }
-      }
-      sq += __shfl_xor_sync(0xffffffffu, sq, 1); sk += __shfl_xor_sync(0xffffffffu, sk, 1);
-      sq += __shfl_xor_sync(0xffffffffu, sq, 2); sk += __shfl_xor_sync(0xffffffffu, sk, 2);
-      rq = live ? rsqrtf(sq + 1e-6f) : 1.f;
-      rk = live ? rsqrtf(sk + 1e-6f) : 1.f;
-    }
-    if (rp == 0) { rq_s[rx] = rq; rk_s[rx] = rk; }
+    const float rq = rq_s[rx], rk = rk_s[rx];
     // the pieces of row rx as loaded, and activated: k_hat, q_hat, beta = b k_hat
     Raw8 rawk, rawq, rawb;
     float b1 = 0.f;
@@ -573,6 +563,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       }
     };
 
+    uint32_t gpass = 0;                                 // which of the thread's 32 rows pass the gradient of g
     // ---- the decay of all channels: thread (channel, 32 rows), scanned in registers, restarting at document changes
     if constexpr (!SC) {
       if (tid < C) {                                    // seg_s is non-decreasing: binary searches
@@ -593,6 +584,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       for (int i = 0; i < 32; ++i) {
         const bool on = cin && x0 + i < rows;
         float gv = ldf_ro(gp + (on ? (size_t)(x0 + i) * gpitch : 0) - (cin ? 0 : (size_t)c * ges), 0, gdt);
+        gpass |= (guard ? gv < -1e-6f : gv <= 0.f) ? 1u << i : 0u;
         if (fuse) gv = -umma::ex2_fast(fminf(gv, 5.f) * DN_LOG2E); else gv = gv <= 0.f ? gv : 0.f;
         if (guard) gv = fminf(gv, -1e-6f);
         v[i] = on ? gv : 0.f;
@@ -689,58 +681,50 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       commit(cx);
       finish(cx);
     } else {
+      // Two rounds of 64 channels: what the images take beside Lambda, dA and dM.  (Four rounds of 32 with two sets of images
+      // overlapped building and products, but at 32 columns an MMA costs 46 cycles and at 64 it costs 48: 18.7 k cycles
+      // per tile against 11 k.)
+      uint4* KF = reinterpret_cast<uint4*>(sm + OFF_GI);
+      uint4* QF = KF + 8 * PP;
+      uint4* BF = QF + 8 * PP;
       load_pieces(rp);
 #pragma unroll 1
-      for (int grp = 0; grp < 4; ++grp) {
-        const int p = grp * 4 + rp;
-        uint4* KF = reinterpret_cast<uint4*>(sm + OFF_GI + (grp & 1) * 3 * 4 * PB);
-        uint4* QF = KF + 4 * PP;
-        uint4* BF = QF + 4 * PP;
-        float kh[8], qh[8], be[8];
-        pieces(p, kh, qh, be);
-        const float* lx = LAM + rx * LPF + 8 * p;
-        const float* ls = LAM + ds_s[rx] * LPF + 8 * p;
-        const float* le = LAM + de_s[rx] * LPF + 8 * p;
+      for (int rnd = 0; rnd < 2; ++rnd) {
+        if (rnd) finish(cx);                            // the images have been read
+#pragma unroll 1
+        for (int it = 0; it < 2; ++it) {
+          const int p = rnd * 8 + it * 4 + rp;
+          float kh[8], qh[8], be[8];
+          pieces(p, kh, qh, be);
+          if (p + 4 < 16) load_pieces(p + 4);
+          const float* lx = LAM + rx * LPF + 8 * p;
+          const float* ls = LAM + ds_s[rx] * LPF + 8 * p;
+          const float* le = LAM + de_s[rx] * LPF + 8 * p;
 #pragma unroll
-        for (int i = 0; i < 8; i += 4) {
-          const float4 u0 = *reinterpret_cast<const float4*>(lx + i), u1 = *reinterpret_cast<const float4*>(ls + i), u2 = *reinterpret_cast<const float4*>(le + i);
-          const float d[4] = {fmaf(-0.5f, u1.x + u2.x, u0.x), fmaf(-0.5f, u1.y + u2.y, u0.y), fmaf(-0.5f, u1.z + u2.z, u0.z), fmaf(-0.5f, u1.w + u2.w, u0.w)};
+          for (int i = 0; i < 8; i += 4) {
+            const float4 u0 = *reinterpret_cast<const float4*>(lx + i), u1 = *reinterpret_cast<const float4*>(ls + i), u2 = *reinterpret_cast<const float4*>(le + i);
+            const float d[4] = {fmaf(-0.5f, u1.x + u2.x, u0.x), fmaf(-0.5f, u1.y + u2.y, u0.y), fmaf(-0.5f, u1.z + u2.z, u0.z), fmaf(-0.5f, u1.w + u2.w, u0.w)};
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const float f = umma::ex2_fast(d[u]), fi = umma::ex2_fast(-d[u]);
-            kh[i + u] *= fi;
-            qh[i + u] *= f;
-            be[i + u] *= f;
+            for (int u = 0; u < 4; ++u) {
+              const float f = umma::ex2_fast(d[u]), fi = umma::ex2_fast(-d[u]);
+              kh[i + u] *= fi;
+              qh[i + u] *= f;
+              be[i + u] *= f;
+            }
           }
+          const int o = (it * 4 + rp) * PP + rx;
+          KF[o] = umma::pack8(kh);
+          QF[o] = umma::pack8(qh);
+          BF[o] = umma::pack8(be);
         }
-        if (grp >= 2) {                                 // the set was read by the products of group - 2
-          cx.dead = cta_wait_call(&gbar[grp & 1], (gph >> (grp & 1)) & 1u, a.err, cx.dead);
-          gph ^= 1u << (grp & 1);
-        }
-        KF[rp * PP + rx] = umma::pack8(kh);
-        QF[rp * PP + rx] = umma::pack8(qh);
-        BF[rp * PP + rx] = umma::pack8(be);
         umma::pre_issue_sync();
-        product<32, false, true>(cx, sl.at(4), 2048, KF, PB, C, T_B + 32 * grp, true);       // dA (k / f)
-        product<32, false, true>(cx, sl.at(5), 2048, KF, PB, C, T_Q + 32 * grp, true);       // dM (k / f)
-        product<32, true, true>(cx, sl.at(4), 2048, BF, PB, C, T_K + 32 * grp, true);        // dA^T (beta f)
-        product<32, true, true>(cx, sl.at(5), 2048, QF, PB, C, T_K + 32 * grp, true);        // dM^T (q f)
-        if (warp == 0 && !cx.dead) umma::mma_commit_warp(&gbar[grp & 1]);
-        if (grp < 3) load_pieces((grp + 1) * 4 + rp);
+        product<64, false, true>(cx, sl.at(4), 2048, KF, PB, C, T_B + 64 * rnd, true);       // dA (k / f)
+        product<64, false, true>(cx, sl.at(5), 2048, KF, PB, C, T_Q + 64 * rnd, true);       // dM (k / f)
+        product<64, true, true>(cx, sl.at(4), 2048, BF, PB, C, T_K + 64 * rnd, true);        // dA^T (beta f)
+        product<64, true, true>(cx, sl.at(5), 2048, QF, PB, C, T_K + 64 * rnd, true);        // dM^T (q f)
+        commit(cx);
       }
-      cx.dead = cta_wait_call(&gbar[0], gph & 1u, a.err, cx.dead);
-      cx.dead = cta_wait_call(&gbar[1], (gph >> 1) & 1u, a.err, cx.dead);
-      gph ^= 3u;
-    }
-    if (tid == 0 && e_item + (int)gridDim.x < a.items) {      // the next tile's images on their way into L2
-      const int nx = e_item + gridDim.x;
-      const size_t nb = (size_t)(nx % (g.B * g.H)) * g.NC + a.c_begin + nx / (g.B * g.H);
-      umma::prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(a.res.W) + nb * C * K, IMGB);
-      umma::prefetch_l2(states_img(g, a.res.states) + nb * K * VW, IMGB * NH);
-      umma::prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(a.res.U) + nb * C * VW, IMGB * NH);
-      umma::prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(a.dV) + nb * C * VW, IMGB * NH);
-      umma::prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(a.dH) + nb * K * VW, IMGB * NH);
-      umma::prefetch_l2(a.res.T + nb * C * C, IMGB);
+      finish(cx);
     }
     // ---- raw k, q and b, turned from the row mapping into a row per lane
     uint4* const RK = reinterpret_cast<uint4*>(sm + OFF_RK);
@@ -905,11 +889,27 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
             dkn[i] = rkr * (dkn[i] - kr[i] * rkr * dk_dot);
           }
         }
+        if (SC && D > 1) {                              // (the thread reads back what it wrote: no barrier)
+          float4* acc = reinterpret_cast<float4*>(a.scratch + (size_t)blockIdx.x * a.scratch_per_cta) + p * 512 + row;
+          float4* v4[4] = {reinterpret_cast<float4*>(dqn), reinterpret_cast<float4*>(dqn + 4), reinterpret_cast<float4*>(dkn), reinterpret_cast<float4*>(dkn + 4)};
+          if (hd > 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float4 t = umma::ld_keep4(acc + i * 128);
+              v4[i]->x += t.x; v4[i]->y += t.y; v4[i]->z += t.z; v4[i]->w += t.w;
+            }
+          }
+          if (hd < D - 1) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) umma::st_keep4(acc + i * 128, *v4[i]);
+            continue;
+          }
+        }
         if (inplace) {
           RQ[p * PP + row] = umma::pack8(dqn);
           RK[p * PP + row] = umma::pack8(dkn);
         } else if (rlive && p < kp) {
-          const size_t o = ((tok0 + row) * g.H + h) * g.K + 8 * p;
+          const size_t o = ((tok0 + row) * HG + h / D) * g.K + 8 * p;
           strow8(a.dq, o, a.dq_dt, dqn);
           strow8(a.dk, o, a.dq_dt, dkn);
         }
@@ -922,8 +922,8 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       }
       umma::tc_fence_before();
       __syncthreads();
-      if (inplace && live) {
-        const size_t o = ((tok0 + rx) * g.H + h) * g.K;
+      if (inplace && live && hd == D - 1) {
+        const size_t o = ((tok0 + rx) * HG + h / D) * g.K;
 #pragma unroll
         for (int it = 0; it < 4; ++it) {
           const int p = it * 4 + rp;
@@ -985,30 +985,43 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         for (int q2 = qd + 1; q2 < 4; ++q2) { carry += TOT[q2 * 128 + c]; if (cut_s[4 + q2]) break; }
       const int lastcut = ends ? 31 - __clz(ends) : -1; // rows behind it take the carry
       const float e = dlend_s[c] + (PS[c] + PS[128 + c]) + (PS[256 + c] + PS[384 + c]);
-      float sg[32];
       const bool cin = gC == 1 || c < gC;
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
-        const int x = x0 + i;
-        float o = v[i] + (i > lastcut ? carry : 0.f);
-        if (seg_s[x] == segL) o += e;
-        sg[i] = o;
+        if (i > lastcut) v[i] += carry;
+        if (seg_s[x0 + i] == segL) v[i] += e;
       }
       if (gC != 1) {
-#pragma unroll 8
-        for (int i = 0; i < 32; ++i) {
-          const int x = x0 + i;
-          if (x < rows && cin) {
-            const float gr = ldf_ro(a.gg, ((tok0 + x) * g.gH + hg) * gC + c, gdt);
-            stf(a.dg, ((tok0 + x) * g.H + h) * gC + c, g_adjoint(sg[i], gr), a.dg_dt);
+        const size_t o = ((tok0 + x0) * g.H + h) * gC + c, pitch = (size_t)g.H * gC;
+        if (fuse) {
+          const size_t gi = ((tok0 + x0) * g.gH + hg) * gC + c, gp = (size_t)g.gH * gC;
+#pragma unroll
+          for (int j = 0; j < 32; j += 16) {
+            float gr[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) gr[i] = x0 + j + i < rows && cin ? ldf_ro(a.gg, gi + (j + i) * gp, gdt) : 0.f;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[j + i] = g_adjoint(v[j + i], gr[i]);
           }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = (gpass >> i) & 1 ? v[i] : 0.f;
+        }
+        if (a.dg_dt == DN_BF16) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (x0 + i < rows && cin) reinterpret_cast<__nv_bfloat16*>(a.dg)[o + i * pitch] = __float2bfloat16_rn(v[i]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (x0 + i < rows && cin) reinterpret_cast<float*>(a.dg)[o + i * pitch] = v[i];
         }
       } else {                                          // one decay per row: the sum over the channels
 #pragma unroll
-        for (int i = 0; i < 32; ++i) sg[i] = warp_sum(c < g.K ? sg[i] : 0.f);
+        for (int i = 0; i < 32; ++i) v[i] = warp_sum(c < g.K ? v[i] : 0.f);
         if (lane == 0) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) SUM[(c >> 5) * 128 + x0 + i] = sg[i];
+          for (int i = 0; i < 32; ++i) SUM[(c >> 5) * 128 + x0 + i] = v[i];
         }
         __syncthreads();
         if (tid < rows) {
@@ -1026,13 +1039,25 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
 
 }  // namespace
 
+// Heads that share a key head (qk_div > 1) each have a dq and a dk, to be summed.  Taking them one after the other in one CTA
+// keeps the partial sums in L2 and writes the result once; staging them in fp32 and summing in a further kernel
+// moved 540 MB at B=2 L=4001 Hk=16 Hv=32, 187 us.  Only for scalar gates (with decay per channel some of the heads may be
+// left to the other kernel), and only where the coarser units cost no extra round of CTAs.
+int prepass_bwd_group(const Geo& g, int chunks) {
+  if (!prepass_bwd_tc_eligible(g) || !prepass_bwd_scalar_route(g) || g.qk_div <= 1) return 1;
+  const int sms = sm_count(), items = g.B * g.H * chunks, units = items / g.qk_div;
+  const int rounds = (items + sms - 1) / sms, coarse = (units + sms - 1) / sms * g.qk_div;
+  return coarse * 8 <= rounds * 9 ? g.qk_div : 1;
+}
+
 bool prepass_bwd_scalar_route(const Geo& g) {
   return g.gC == 1 && g.bC == 1 && g.qkv_dt == DN_BF16 && !(g.flags & DN_FUSE_PROLOGUE);
 }
 
 int launch_prepass_bwd_fast(const PrepassBwdArgs& a, cudaStream_t st) {
   const Geo& g = a.g;
-  const int grid = a.items < sm_count() ? a.items : sm_count();
+  const int units = a.items / (prepass_bwd_scalar_route(g) ? a.group : 1);
+  const int grid = units < sm_count() ? units : sm_count();
   auto go = [&](auto kernel) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     kernel<<<grid, NT, SMEM_BYTES, st>>>(a);

@@ -732,6 +732,7 @@ int launch_prepass_bwd_tc(PrepassBwdArgs& a, size_t scratch_floats, cudaStream_t
   if (a.items <= 0) return DN_OK;
   a.scratch_per_cta = prepass_bwd_tc_scratch_per_cta(g);
   a.err = device_error_ptr();
+  if (a.group > 1 && scratch_floats < (size_t)sm_count() * a.scratch_per_cta) return DN_ERR_SCRATCH_TOO_SMALL;
   int rc = launch_prepass_bwd_fast(a, st);
   if (rc || prepass_bwd_scalar_route(g)) return rc;
   const int grid = a.items < sm_count() ? a.items : sm_count();

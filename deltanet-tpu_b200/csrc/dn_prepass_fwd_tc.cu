@@ -339,6 +339,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_scalar_kernel(const __grid_
         KE[p * 128 + x] = umma::pack8(f);
       }
       if (tid < K) a.res.lam_end[ibase * K + tid] = lend;
+      if (a.res.T && lgrp == 0) { float* ex = tile_extra(a.res, ibase); ex[128 + x] = rq; ex[256 + x] = rk; }
     }
     umma::commit_wait_cta(cx);
     {                                                   // X = [first document] beta e^lam k_hat, over the k_hat image
@@ -677,7 +678,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       rk = rsqrtf(sk + 1e-6f);
     }
     const float rqs = rq * g.scale;
-    if (lgrp == 0) { rq_s[x] = rq; rk_s[x] = rk; }      // (for the hierarchical route)
+    if (lgrp == 0) { rq_s[x] = rq; rk_s[x] = rk; }      // (for the hierarchical route and the backward)
     Raw8 kr, qr, br;                                    // this thread's piece of the group about to be built
     float b1 = 0.f;
     auto load_kqb = [&](int grp) {
@@ -812,7 +813,11 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
     if (__syncthreads_or(!(ok0 && ok1))) { cx.dead = true; umma::report_timeout(err); }
     umma::tc_fence_after();
     const bool any_strong = __syncthreads_or(strong);
-    if (a.res.T && tid == 0) *strong_flag_ptr(a.res, ibase) = any_strong;        // the backward takes the same route
+    if (a.res.T) {                                      // the backward takes the same route
+      float* ex = tile_extra(a.res, ibase);
+      if (tid == 0) *reinterpret_cast<int*>(ex) = any_strong;
+      if (tid < C) { ex[128 + tid] = rq_s[tid]; ex[256 + tid] = rk_s[tid]; }
+    }
     if (any_strong) {
       umma::Ctx c2 = cx;
       strong_route<MODE>(a, b, h, t0, ibase, rq_s, rk_s, seg_s, rst_s, sm, c2);
