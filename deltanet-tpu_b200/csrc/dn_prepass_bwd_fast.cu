@@ -211,6 +211,65 @@ __device__ __forceinline__ void stage_dO(uint4* dst, const void* d_out, size_t o
   umma::cp_async_commit();
 }
 
+// dv = dY w_act, dw = dY v (+ sigmoid adjoint; summed over a value head's columns when w is one scalar per head) of 128
+// columns, dY from its image.  The rows of v are requested together where w is one scalar,
+// those of v and w one step ahead otherwise (less code).
+template <int MODE, bool SC>
+__device__ __noinline__ void v_phase_call(const PrepassBwdArgs& a, const uint4* img, int half, int h, size_t tok0, int rows, int wC) {
+  using CF = InCfg<MODE>;
+  const Geo& g = a.g;
+  const int rx = threadIdx.x >> 2, rp = threadIdx.x & 3, vr = g.G * g.V;
+  const int qdt = SC || MODE != 2 ? (SC ? DN_BF16 : CF::qkv_dt) : g.qkv_dt, gdt = CF::fixed ? DN_F32 : g.gate_dt;
+  const uint32_t qes = qdt == DN_BF16 ? 2 : 4, ges = gdt == DN_BF16 ? 2 : 4;
+  const bool fuse = CF::fixed || SC ? false : (g.flags & DN_FUSE_PROLOGUE) != 0;
+  const bool live = rx < rows;
+  const size_t tok = tok0 + (live ? rx : 0);
+  constexpr int VB = SC || CF::scalar_bw ? 4 : 1;
+  Raw8 vraw[VB], wraw[VB];
+  auto load = [&](int col, Raw8& vraw, Raw8& wraw) {
+    const int cc = col < vr ? col : 0, hv = h * g.G + cc / g.V, cv = cc % g.V;
+    vraw = ldraw(reinterpret_cast<const uint8_t*>(a.v) + ((tok * g.Hv + hv) * g.V + cv) * qes, 0, qdt);
+    if (wC == 1) wraw.a.x = __float_as_uint(ldf_ro(a.w, tok * g.wH + g.w_head(hv), gdt));
+    else wraw = ldraw(reinterpret_cast<const uint8_t*>(a.w) + ((tok * g.wH + g.w_head(hv)) * wC + cv) * ges, 0, gdt);
+  };
+  const int steps_per_head = g.V / 32;
+  float sw = 0.f;
+#pragma unroll
+  for (int i = 0; i < VB; ++i) load(half * 128 + 32 * i + 8 * rp, vraw[i], wraw[i]);
+#pragma unroll (VB)
+  for (int it = 0; it < 4; ++it) {
+    const int p = it * 4 + rp, col = half * 128 + 8 * p;
+    if (col - 8 * rp >= vr) break;                      // (uniform: value widths are multiples of 32)
+    const int hv = h * g.G + col / g.V, cv = col % g.V;
+    float vv[8], ww[8], dy[8], dv8[8], dw8[8];
+    cvraw(vraw[it % VB], qdt, vv);
+    if (wC == 1) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) ww[i] = __uint_as_float(wraw[it % VB].a.x);
+    } else cvraw(wraw[it % VB], gdt, ww);
+    if (VB == 1 && it < 3) load(col + 32, vraw[0], wraw[0]);
+    umma::unpack8(img[p * PP + rx], dy);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float wa = ww[i], dwv = dy[i] * vv[i];
+      if (fuse) { wa = sigmoid_fast(ww[i]); dwv *= wa * (1.f - wa); }
+      dv8[i] = dy[i] * wa;
+      dw8[i] = dwv;
+      sw += dwv;
+    }
+    if (live) {
+      strow8(a.dv, (tok * g.Hv + hv) * g.V + cv, qdt, dv8);
+      if (wC != 1) strow8(a.dw, (tok * g.Hv + hv) * wC + cv, a.dw_dt, dw8);
+    }
+    if (wC == 1 && (it + 1) % steps_per_head == 0) {
+      sw += __shfl_xor_sync(0xffffffffu, sw, 1);
+      sw += __shfl_xor_sync(0xffffffffu, sw, 2);
+      if (live && rp == 0) stf(a.dw, tok * g.Hv + hv, sw, a.dw_dt);
+      sw = 0.f;
+    }
+  }
+}
+
 template <int VW, int MODE, bool SC>
 __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_constant__ PrepassBwdArgs a) {
   using CF = InCfg<MODE>;
@@ -247,8 +306,8 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
   const uint32_t tb = cx.tmem + ((uint32_t)(quarter * 32) << 16) + group * 32;
 
   const bool l2 = g.flags & DN_QK_L2NORM, trunc = g.flags & DN_TRUNC_DT_BF16;
-  const bool fuse = CF::fixed ? false : (g.flags & DN_FUSE_PROLOGUE) != 0, guard = CF::fixed ? false : (g.flags & DN_STABILITY_GUARD) != 0;
-  const int qdt = CF::fixed ? CF::qkv_dt : g.qkv_dt, gdt = CF::fixed ? DN_F32 : g.gate_dt;
+  const bool fuse = CF::fixed || SC ? false : (g.flags & DN_FUSE_PROLOGUE) != 0, guard = CF::fixed ? false : (g.flags & DN_STABILITY_GUARD) != 0;
+  const int qdt = SC ? DN_BF16 : (CF::fixed ? CF::qkv_dt : g.qkv_dt), gdt = CF::fixed ? DN_F32 : g.gate_dt;
   const bool round_in = !fuse && qdt == DN_BF16;
   const int kp = CF::fixed && !SC ? 16 : g.K / 8, gC = SC ? 1 : (CF::fixed ? K : g.gC), bC = SC ? 1 : (CF::fixed ? (CF::scalar_bw ? 1 : K) : g.bC);
   const int wC = CF::fixed && !SC ? (CF::scalar_bw ? 1 : g.V) : g.wC;
@@ -424,54 +483,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       drain_plain(cx.dead, tb + T_B, sl.at(slot), 128, row, group, 1.f);
     };
     auto drain_dY = [&](int slot) { drain_plain(cx.dead, tb + T_TMP, sl.at(slot), PP, row, group, 1.f); };
-    // dv = dY w_act, dw = dY v (+ sigmoid adjoint; summed over a value head's columns when w is one scalar per head)
-    // The rows of v and w are read one step ahead of their use.
-    const bool vlive = rx < rows;
-    const size_t vtok = tok0 + (vlive ? rx : 0);
-    Raw8 vraw, wraw;
-    auto v_load = [&](int col) {
-      const int cc = col < vr ? col : 0, hv = h * g.G + cc / g.V, cv = cc % g.V;
-      vraw = ldraw(reinterpret_cast<const uint8_t*>(a.v) + ((vtok * g.Hv + hv) * g.V + cv) * qes, 0, qdt);
-      if (wC == 1) wraw.a.x = __float_as_uint(ldf_ro(a.w, vtok * g.wH + g.w_head(hv), gdt));
-      else wraw = ldraw(reinterpret_cast<const uint8_t*>(a.w) + ((vtok * g.wH + g.w_head(hv)) * wC + cv) * ges, 0, gdt);
-    };
-    auto vphase = [&](int slot, int half) {
-      const uint4* img = sl.at(slot);
-      const int steps_per_head = g.V / 32;
-      float sw = 0.f;
-#pragma unroll 1
-      for (int it = 0; it < 4; ++it) {
-        const int p = it * 4 + rp, col = half * 128 + 8 * p;
-        if (col - 8 * rp >= vr) break;                  // (uniform: value widths are multiples of 32)
-        const int hv = h * g.G + col / g.V, cv = col % g.V;
-        float vv[8], ww[8], dy[8], dv8[8], dw8[8];
-        cvraw(vraw, qdt, vv);
-        if (wC == 1) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) ww[i] = __uint_as_float(wraw.a.x);
-        } else cvraw(wraw, gdt, ww);
-        if (it < 3) v_load(col + 32);
-        umma::unpack8(img[p * PP + rx], dy);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          float wa = ww[i], dwv = dy[i] * vv[i];
-          if (fuse) { wa = sigmoid_fast(ww[i]); dwv *= wa * (1.f - wa); }
-          dv8[i] = dy[i] * wa;
-          dw8[i] = dwv;
-          sw += dwv;
-        }
-        if (vlive) {
-          strow8(a.dv, (vtok * g.Hv + hv) * g.V + cv, qdt, dv8);
-          if (wC != 1) strow8(a.dw, (vtok * g.Hv + hv) * wC + cv, a.dw_dt, dw8);
-        }
-        if (wC == 1 && (it + 1) % steps_per_head == 0) {
-          sw += __shfl_xor_sync(0xffffffffu, sw, 1);
-          sw += __shfl_xor_sync(0xffffffffu, sw, 2);
-          if (vlive && rp == 0) stf(a.dw, vtok * g.Hv + hv, sw, a.dw_dt);
-          sw = 0.f;
-        }
-      }
-    };
+    auto vphase = [&](int slot, int half) { v_phase_call<MODE, SC>(a, sl.at(slot), half, h, tok0, rows, wC); };
     if constexpr (NH == 1) {
       drain_dX(0);
       drain_dY(1);
@@ -481,7 +493,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       product<128, false, false>(cx, sl.at(0), 2048, sl.at(2), 2048, 128, T_TMP, false);                   // -dA = dX W^T + dY U^T
       product<128, false, false>(cx, sl.at(1), PB, sl.at(4), 2048, 128, T_TMP, true);
       commit(cx);
-      v_load(8 * rp);
       vphase(1, 0);
       finish(cx);
     } else {
@@ -502,11 +513,9 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       product<128, false, false>(cx, sl.at(3), 2048, sl.at(1), 2048, 128, T_TMP, false);                   // -dA = dX W^T + dY U^T
       product<128, false, false>(cx, sl.at(2), PB, sl.at(0), 2048, 128, T_TMP, true);
       commit(cx);
-      v_load(8 * rp);
       finish(cx);
       sl.load(0, Ug + HN);
       vphase(2, 0);
-      v_load(128 + 8 * rp);
       sl.wait(0);
       product<128, false, false>(cx, sl.at(4), PB, sl.at(0), 2048, 128, T_TMP, true);
       commit(cx);
@@ -577,29 +586,51 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       }
       const int c = tid & 127, qd = tid >> 7, x0 = qd * 32;
       const uint32_t gpitch = (uint32_t)(g.gH * gC) * ges;
-      const uint8_t* gp = reinterpret_cast<const uint8_t*>(a.gg) + (tok0 * g.gH + g.gate_head(h, g.gH)) * gC * ges + (gC == 1 ? 0 : c) * ges;
       const bool cin = gC == 1 || c < gC;
-      float v[32];
+      const uint8_t* gp = reinterpret_cast<const uint8_t*>(a.gg) + (tok0 * g.gH + g.gate_head(h, g.gH)) * gC * ges + (gC == 1 || !cin ? 0 : c) * ges;
+      constexpr int GB = MODE == 2 ? 8 : 32;            // rows requested together (code size against latency)
+      float nx[GB];
+      auto load_g = [&](int j) {                        // (rows past the end: row 0, dropped below)
+        const int x = x0 + GB * j;
+        if (gdt == DN_BF16) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const bool on = cin && x0 + i < rows;
-        float gv = ldf_ro(gp + (on ? (size_t)(x0 + i) * gpitch : 0) - (cin ? 0 : (size_t)c * ges), 0, gdt);
-        gpass |= (guard ? gv < -1e-6f : gv <= 0.f) ? 1u << i : 0u;
-        if (fuse) gv = -umma::ex2_fast(fminf(gv, 5.f) * DN_LOG2E); else gv = gv <= 0.f ? gv : 0.f;
-        if (guard) gv = fminf(gv, -1e-6f);
-        v[i] = on ? gv : 0.f;
-      }
+          for (int i = 0; i < GB; ++i) nx[i] = ldf_ro(gp + (x + i < rows ? (size_t)(x + i) * gpitch : 0), 0, DN_BF16);
+        } else {
+#pragma unroll
+          for (int i = 0; i < GB; ++i) nx[i] = ldf_ro(gp + (x + i < rows ? (size_t)(x + i) * gpitch : 0), 0, DN_F32);
+        }
+      };
+      load_g(0);
       const uint32_t cuts = __ballot_sync(0xffffffffu, x0 + lane > 0 && seg_s[x0 + lane] != seg_s[x0 + lane - (x0 + lane > 0)]);
+      float run = 0.f;
+      float* lp = LAM + x0 * LPF + c;
+#pragma unroll 1
+      for (int j = 0; j < 32 / GB; ++j) {
+        float v[GB];
 #pragma unroll
-      for (int i = 1; i < 32; ++i) v[i] += (cuts >> i) & 1 ? 0.f : v[i - 1];
-      TOT[qd * 128 + c] = v[31];
+        for (int i = 0; i < GB; ++i) v[i] = nx[i];
+        if (j < 32 / GB - 1) load_g(j + 1);
+#pragma unroll
+        for (int i = 0; i < GB; ++i) {
+          float gv = v[i];
+          gpass |= (guard ? gv < -1e-6f : gv <= 0.f) ? 1u << (GB * j + i) : 0u;
+          if (fuse) gv = -umma::ex2_fast(fminf(gv, 5.f) * DN_LOG2E); else gv = gv <= 0.f ? gv : 0.f;
+          if (guard) gv = fminf(gv, -1e-6f);
+          if (!(cin && x0 + GB * j + i < rows)) gv = 0.f;
+          run = ((cuts >> (GB * j + i)) & 1 ? 0.f : run) + gv * DN_LOG2E;      // kept in units of log 2
+          lp[(GB * j + i) * LPF] = run;
+        }
+      }
+      TOT[qd * 128 + c] = run;
       if (c == 0) cut_s[qd] = cuts != 0;
       __syncthreads();
       float carry = 0.f;
       for (int q2 = qd - 1; q2 >= 0; --q2) { carry += TOT[q2 * 128 + c]; if (cut_s[q2]) break; }
-      const int nr = cuts ? __ffs(cuts) - 1 : 32;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) LAM[(x0 + i) * LPF + c] = (v[i] + (i < nr ? carry : 0.f)) * DN_LOG2E;
+      if (qd > 0) {
+        const int nr = cuts ? __ffs(cuts) - 1 : 32;
+#pragma unroll 4
+        for (int i = 0; i < nr; ++i) lp[i * LPF] += carry;
+      }
       __syncthreads();
       if (tid < C) {
         EDGE[tid] = umma::ex2_fast(0.5f * (LAM[tid] + LAM[de_s[0] * LPF + tid]));
@@ -970,14 +1001,23 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       }
     } else {
       const int c = tid & 127, qd = tid >> 7, x0 = qd * 32;
-      float v[32];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = LAM[(x0 + i) * LPF + c];
       // documents that end behind a row of this quarter
       const uint32_t ends = __ballot_sync(0xffffffffu, x0 + lane < C - 1 && seg_s[x0 + lane] != seg_s[x0 + lane + (x0 + lane < C - 1)]);
+      const uint32_t lastdoc = __ballot_sync(0xffffffffu, seg_s[x0 + lane] == segL);
+      float* lp = LAM + x0 * LPF + c;
+      float run = 0.f;
+#pragma unroll 1
+      for (int j = 3; j >= 0; --j) {
+        float v[8];
 #pragma unroll
-      for (int i = 30; i >= 0; --i) v[i] += (ends >> i) & 1 ? 0.f : v[i + 1];
-      TOT[qd * 128 + c] = v[0];
+        for (int i = 0; i < 8; ++i) v[i] = lp[(8 * j + i) * LPF];
+#pragma unroll
+        for (int i = 7; i >= 0; --i) {
+          run = ((ends >> (8 * j + i)) & 1 ? 0.f : run) + v[i];
+          lp[(8 * j + i) * LPF] = run;
+        }
+      }
+      TOT[qd * 128 + c] = run;
       if (c == 0) cut_s[4 + qd] = ends != 0;
       __syncthreads();
       float carry = 0.f;
@@ -986,43 +1026,56 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       const int lastcut = ends ? 31 - __clz(ends) : -1; // rows behind it take the carry
       const float e = dlend_s[c] + (PS[c] + PS[128 + c]) + (PS[256 + c] + PS[384 + c]);
       const bool cin = gC == 1 || c < gC;
+      const size_t o = ((tok0 + x0) * g.H + h) * gC + c, pitch = (size_t)g.H * gC;
+      const size_t gi = ((tok0 + x0) * g.gH + hg) * gC + (cin && gC != 1 ? c : 0), gpit = (size_t)g.gH * gC;
+      float gr[8];
+      auto load_g = [&](int j) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        if (i > lastcut) v[i] += carry;
-        if (seg_s[x0 + i] == segL) v[i] += e;
-      }
-      if (gC != 1) {
-        const size_t o = ((tok0 + x0) * g.H + h) * gC + c, pitch = (size_t)g.H * gC;
-        if (fuse) {
-          const size_t gi = ((tok0 + x0) * g.gH + hg) * gC + c, gp = (size_t)g.gH * gC;
+        for (int i = 0; i < 8; ++i) {
+          const int x = 8 * j + i;
+          gr[i] = x0 + x < rows ? ldf_ro(a.gg, gi + x * gpit, gdt) : 0.f;
+        }
+      };
+      if (fuse && gC != 1) load_g(0);
+#pragma unroll 1
+      for (int j = 0; j < 4; ++j) {
+        float v[8];
 #pragma unroll
-          for (int j = 0; j < 32; j += 16) {
-            float gr[16];
+        for (int i = 0; i < 8; ++i) {
+          v[i] = lp[(8 * j + i) * LPF];
+          if (8 * j + i > lastcut) v[i] += carry;
+          if ((lastdoc >> (8 * j + i)) & 1) v[i] += e;
+        }
+        if (gC != 1) {
+          if (fuse) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) gr[i] = x0 + j + i < rows && cin ? ldf_ro(a.gg, gi + (j + i) * gp, gdt) : 0.f;
+            for (int i = 0; i < 8; ++i) v[i] = g_adjoint(v[i], gr[i]);
+            if (j < 3) load_g(j + 1);
+          } else {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[j + i] = g_adjoint(v[j + i], gr[i]);
+            for (int i = 0; i < 8; ++i) v[i] = (gpass >> (8 * j + i)) & 1 ? v[i] : 0.f;
           }
-        } else {
+          if (cin) {
+            const size_t oj = o + 8 * j * pitch;
+            if (a.dg_dt == DN_BF16) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = (gpass >> i) & 1 ? v[i] : 0.f;
+              for (int i = 0; i < 8; ++i)
+                if (x0 + 8 * j + i < rows) reinterpret_cast<__nv_bfloat16*>(a.dg)[oj + i * pitch] = __float2bfloat16_rn(v[i]);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                if (x0 + 8 * j + i < rows) reinterpret_cast<float*>(a.dg)[oj + i * pitch] = v[i];
+            }
+          }
+        } else {                                        // one decay per row: the sum over the channels
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float t = warp_sum(c < g.K ? v[i] : 0.f);
+            if (lane == 0) SUM[(c >> 5) * 128 + x0 + 8 * j + i] = t;
+          }
         }
-        if (a.dg_dt == DN_BF16) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (x0 + i < rows && cin) reinterpret_cast<__nv_bfloat16*>(a.dg)[o + i * pitch] = __float2bfloat16_rn(v[i]);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (x0 + i < rows && cin) reinterpret_cast<float*>(a.dg)[o + i * pitch] = v[i];
-        }
-      } else {                                          // one decay per row: the sum over the channels
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = warp_sum(c < g.K ? v[i] : 0.f);
-        if (lane == 0) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) SUM[(c >> 5) * 128 + x0 + i] = v[i];
-        }
+      }
+      if (gC == 1) {
         __syncthreads();
         if (tid < rows) {
           const float s = (SUM[tid] + SUM[128 + tid]) + (SUM[256 + tid] + SUM[384 + tid]);
