@@ -45,12 +45,18 @@ void err_setup() {
 }  // namespace
 
 int* device_error_ptr() {
+  static int* table[64] = {};                  // per device, once looked up
+  int dev = -1;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64)
+    if (int* known = __atomic_load_n(&table[dev], __ATOMIC_ACQUIRE)) return known;
   std::call_once(g_err_once, err_setup);
   int* p = nullptr;
-  if (g_err_mapped && cudaHostGetDevicePointer(reinterpret_cast<void**>(&p), g_err_page, 0) == cudaSuccess && p) return p;
-  cudaGetLastError();
-  p = nullptr;
-  cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_err_fallback);
+  if (!(g_err_mapped && cudaHostGetDevicePointer(reinterpret_cast<void**>(&p), g_err_page, 0) == cudaSuccess && p)) {
+    cudaGetLastError();
+    p = nullptr;
+    cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_err_fallback);
+  }
+  if (dev >= 0 && dev < 64) __atomic_store_n(&table[dev], p, __ATOMIC_RELEASE);
   return p;
 }
 

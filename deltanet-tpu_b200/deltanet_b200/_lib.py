@@ -90,6 +90,7 @@ _SIGNATURES = {
 EXPORTED = tuple(_SIGNATURES)
 
 _lib = None
+_host_mod = None
 
 
 def lib():
@@ -111,3 +112,22 @@ def lib():
 def check(status: int, what: str):
     if status != 0:
         raise RuntimeError(f"deltanet_b200: {what} failed: {lib().dn_status_string(status).decode()} (status {status})")
+
+
+_HOST_USES = ("dn_decode_step", "dn_chunk_fwd", "dn_chunk_bwd", "dn_residual_bytes", "dn_residual_carve", "dn_scratch_bytes",
+              "dn_canonical_segments", "dn_cu_seqlens_segments", "dn_status_string")
+
+
+def host():
+    """The operators' native host path (csrc/dn_torch.cpp), bound to the loaded library; raises if it is missing."""
+    global _host_mod
+    if _host_mod is None:
+        handle = lib()
+        try:
+            from . import _host as mod
+        except ImportError as e:
+            raise RuntimeError(f"deltanet_b200: the extension _host.so cannot be loaded ({e}); build it with "
+                               "deltanet-tpu_b200/csrc/build.sh.") from e
+        mod.bind({n: C.cast(getattr(handle, n), C.c_void_p).value for n in _HOST_USES})
+        _host_mod = mod
+    return _host_mod

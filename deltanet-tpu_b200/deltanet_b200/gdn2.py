@@ -5,8 +5,8 @@ the C-ABI library.
 Mirrors ``src/deltanet_tpu/gdn2.py`` of the reference: ``chunk_gdn2`` (1772-2286) and
 ``gdn2_decode_step`` (2289-2490).  Tensors are torch CUDA tensors; torch supplies device
 memory, streams and the autograd hook that plays the role of the reference's custom VJP
-(1446-1769).  All arithmetic on the path is in the CUDA library: the wrapper validates,
-describes layouts (gates are passed un-broadcast, lengths un-padded), and allocates.
+(1446-1769; csrc/dn_torch.cpp, which also takes plain calls whole).  All arithmetic on the path is in the CUDA
+library: the wrapper validates, describes layouts (gates are passed un-broadcast, lengths un-padded), and allocates.
 
 Deliberate supersets of the reference: ``chunk_size`` may be 64 or 128 and K, V may be
 64 or 128 (the reference accepts only 128/128/128, gdn2.py:1869-1870,1897-1898).
@@ -62,70 +62,8 @@ def _gate_layout(x: torch.Tensor, width: int):
     return (x.shape[2], 1) if x.dim() == 3 else (x.shape[2], x.shape[3])
 
 
-# --------------------------------------------------------------------------------------------
-class _ChunkOp(torch.autograd.Function):
-    """The differentiable operator boundary (reference: gdn2.py:1461-1766)."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, g, b, w, init_state, seg, shape, want_final, recompute, inference):
-        lib = L.lib()
-        B, Lq, Hv, V, K = shape.B, shape.L, shape.Hv, shape.V, shape.K
-        dev = q.device
-        out = torch.empty(B, Lq, Hv, V, dtype=q.dtype, device=dev)
-        final = torch.empty(B, Hv, K, V, dtype=torch.float32, device=dev) if want_final else None
-        needs_grad = (not inference) and any(ctx.needs_input_grad[:7])
-        keep = needs_grad and not recompute
-        res_block, res = None, None
-        if keep:
-            res_block = torch.empty(lib.dn_residual_bytes(shape), dtype=torch.uint8, device=dev)
-            res = L.Residuals()
-            L.check(lib.dn_residual_carve(shape, res_block.data_ptr(), res), "dn_residual_carve")
-        fshape = shape
-        if not keep:
-            fshape = L.Shape.from_buffer_copy(shape)
-            fshape.flags |= L.DN_INFERENCE
-        nbytes = lib.dn_scratch_bytes(fshape, 0, 0)
-        scratch = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=dev)
-        L.check(lib.dn_chunk_fwd(fshape, _ptr(q), _ptr(k), _ptr(v), _ptr(g), _ptr(b), _ptr(w), _ptr(seg),
-                                 _ptr(init_state), _ptr(out), _ptr(final), res if keep else None,
-                                 scratch.data_ptr(), scratch.numel(), _stream()), "dn_chunk_fwd")
-        ctx.shape, ctx.inference, ctx.recompute = shape, inference, recompute
-        ctx.res_block, ctx.want_final = res_block, want_final
-        ctx.has_init = init_state is not None
-        ctx.save_for_backward(q, k, v, g, b, w, init_state, seg)
-        ctx.set_materialize_grads(False)
-        if want_final:
-            return out, final
-        return out
-
-    @staticmethod
-    def backward(ctx, d_out, d_final=None):
-        if ctx.inference:
-            raise ValueError("chunk_gdn2: differentiation is not supported when is_inference=True; "
-                             "set is_inference=False for training.")
-        lib = L.lib()
-        q, k, v, g, b, w, init_state, seg = ctx.saved_tensors
-        shape = ctx.shape
-        dev = q.device
-        if d_out is None:
-            d_out = torch.zeros(shape.B, shape.L, shape.Hv, shape.V, dtype=q.dtype, device=dev)
-        d_out = d_out.to(q.dtype).contiguous()
-        if d_final is not None:
-            d_final = d_final.to(torch.float32).contiguous()
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        dg, db, dw = torch.empty_like(g), torch.empty_like(b), torch.empty_like(w)
-        d_init = torch.empty_like(init_state) if ctx.has_init else None
-        res = None
-        if ctx.res_block is not None:
-            res = L.Residuals()
-            L.check(lib.dn_residual_carve(shape, ctx.res_block.data_ptr(), res), "dn_residual_carve")
-        nbytes = lib.dn_scratch_bytes(shape, 1, 0 if res is not None else 1)
-        scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-        L.check(lib.dn_chunk_bwd(shape, _ptr(q), _ptr(k), _ptr(v), _ptr(g), _ptr(b), _ptr(w), _ptr(seg),
-                                 _ptr(init_state), res, _ptr(d_out), _ptr(d_final),
-                                 _ptr(dq), _ptr(dk), _ptr(dv), _ptr(dg), _ptr(db), _ptr(dw), _ptr(d_init),
-                                 scratch.data_ptr(), scratch.numel(), _stream()), "dn_chunk_bwd")
-        return dq, dk, dv, dg, db, dw, d_init, None, None, None, None, None
+_PLAIN_PRECISION = {"bf16": L.DN_PREC_BF16, "fp32": L.DN_PREC_FP32}
+_PLAIN_STATE = {None: False, "float32": False, "fp32": False, torch.float32: False, "bfloat16": True, "bf16": True, torch.bfloat16: True}
 
 
 def _segments(segment_ids, cu_seqlens, B, Lq, device, first_is_new):
@@ -214,6 +152,17 @@ def chunk_gdn2(
     ``mask_lambda_by_doc`` is always in effect (the kernels restart the cumulative decay at
     document changes, which is the more precise of the reference's two variants).
     """
+    # A plain call (CUDA tensors that need no conversion) is checked, laid out and enqueued in native code; it answers
+    # None when anything is out of the ordinary, and the checks below then say what.
+    if (initial_state_segment_id is None and not streaming_prefill and not stability_guard and (qk_l2norm or not fuse_prologue)
+            and (scale is None or type(scale) is float) and (chunk_size == 128 or chunk_size == 64) and type(chunk_size) is int
+            and type(precision) is str and precision in _PLAIN_PRECISION and isinstance(q, torch.Tensor) and q.is_cuda):
+        flags = ((L.DN_QK_L2NORM if qk_l2norm else 0) | (L.DN_FUSE_PROLOGUE if fuse_prologue else 0)
+                 | (L.DN_STATE_FP32_MM if state_fp32_matmul else 0) | (L.DN_TRUNC_DT_BF16 if truncate_bwd_dT_bf16 else 0))
+        r = L.host().chunk(q, k, v, g, b, w, segment_ids, cu_seqlens, initial_state, bool(output_final_state), chunk_size,
+                           _PLAIN_PRECISION[precision], scale, flags, bool(recompute_states), bool(is_inference))
+        if r is not None:
+            return r
     if fuse_prologue and not qk_l2norm:
         raise ValueError(
             "fuse_prologue=True requires qk_l2norm=True because L2-normalization is fused directly "
@@ -324,24 +273,26 @@ def chunk_gdn2(
     if is_inference and streaming_prefill and Lq > prefill_block_size:
         if prefill_block_size % chunk_size != 0:
             raise ValueError(f"prefill_block_size ({prefill_block_size}) must be a multiple of chunk_size ({chunk_size}).")
-        if seg is None:
-            seg = torch.zeros(B, Lq, dtype=torch.int32, device=q.device)
         outs, state = [], initial_state
+        out = torch.empty(B, Lq, Hv, V, dtype=qkv_dt, device=q.device) if B == 1 else None    # (a block of one row is contiguous)
         for sb in range(0, Lq, prefill_block_size):
             eb = min(sb + prefill_block_size, Lq)
-            seg_b = seg[:, sb:eb] if sb == 0 else seg[:, sb:eb] - seg[:, sb - 1:sb]
-            o_b, state = _ChunkOp.apply(
+            seg_b = None if seg is None else seg[:, sb:eb] if sb == 0 else seg[:, sb:eb] - seg[:, sb - 1:sb]
+            o_b, state = L.host().apply(
                 q[:, sb:eb].contiguous(), k[:, sb:eb].contiguous(), v[:, sb:eb].contiguous(),
                 g[:, sb:eb].contiguous(), b[:, sb:eb].contiguous(), w[:, sb:eb].contiguous(),
-                state, seg_b.contiguous(), make_shape(eb - sb, state is not None), True, False, True)
+                state, None if seg_b is None else seg_b.contiguous(), bytes(make_shape(eb - sb, state is not None)), True, False, True,
+                None if out is None else out[:, sb:eb])
             if stability_guard:
                 state = _cap_state(state, stability_tau)
             outs.append(o_b)
-        out = torch.cat(outs, dim=1).to(out_dtype)
+        if out is None or outs[0].requires_grad:
+            out = torch.cat(outs, dim=1)
+        out = out.to(out_dtype)
         return (out, state) if output_final_state else out
 
-    res = _ChunkOp.apply(q, k, v, g, b, w, initial_state, seg, make_shape(Lq, initial_state is not None),
-                         bool(output_final_state), bool(recompute_states), bool(is_inference))
+    res = L.host().apply(q, k, v, g, b, w, initial_state, seg, bytes(make_shape(Lq, initial_state is not None)),
+                         bool(output_final_state), bool(recompute_states), bool(is_inference), None)
     if output_final_state:
         out, final = res
         if stability_guard and is_inference:
@@ -387,6 +338,14 @@ def gdn2_decode_step(
     the buffer the new state is written to; passing ``state`` itself updates it in place when
     the dtypes match.
     """
+    if ((scale is None or type(scale) is float) and type(stability_tau) is float and (stability_tau > 0 or not stability_guard)
+            and (state_dtype is None or isinstance(state_dtype, (str, torch.dtype))) and state_dtype in _PLAIN_STATE
+            and isinstance(q, torch.Tensor) and q.is_cuda):
+        r = L.host().decode(q, k, v, g, b, w, state, reset, scale,
+                            (L.DN_QK_L2NORM if qk_l2norm else 0) | (L.DN_STABILITY_GUARD if stability_guard else 0),
+                            _PLAIN_STATE[state_dtype], stability_tau, out_state)
+        if r is not None:
+            return r
     if stability_guard and isinstance(stability_tau, (int, float)) and not stability_tau > 0:
         raise ValueError(f"stability_tau must be positive, got {stability_tau}.")
     nd = q.dim()
