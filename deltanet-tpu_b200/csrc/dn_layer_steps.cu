@@ -10,6 +10,8 @@
 // tokens with the stencil window in registers, so the halo is 3 rows per run) and writes each output
 // once.  Parameter gradients (conv weight, bias, A_log, dt_bias, norm weight) are reduced in a fixed
 // order through per-tile partial sums, so results are bit-reproducible.
+#include <cooperative_groups.h>
+
 #include "dn_kernels.cuh"
 #include "dn_umma.cuh"
 
@@ -446,34 +448,52 @@ __global__ void __launch_bounds__(256) gates_fwd_kernel(const void* a_, const vo
   beta[e] = 1.f / (1.f + expf(-ldf_ro(b_, e, dt)));
 }
 
-// da, db element-wise; dA_log[h] = sum dg * g, d dt_bias[h] = sum dg * dg/d(a): one CTA per head, fixed order
-__global__ void __launch_bounds__(256) gates_bwd_kernel(const void* a_, const void* b_, int dt, const float* A_log,
-                                                        const float* dt_bias, const float* dg, const float* dbeta,
-                                                        size_t tokens, int Hv, void* da, void* db, float* dA_log,
-                                                        float* d_dt_bias) {
-  const int h = blockIdx.x;
-  const float Ae = -expf(A_log[h]), bias = dt_bias[h];
+// da, db element-wise; dA_log[h] = sum dg * g, d dt_bias[h] = sum dg * dg/d(a).  A cluster of 8 CTAs takes 4 heads (so that a
+// thread's neighbours read next to it) and adds its partial sums in a fixed order through distributed shared memory:
+// 52 us -> 17 us at 8002 tokens x 32 heads, where one CTA per head walked the tokens alone.
+constexpr int GB_CTAS = 8, GB_HEADS = 4;
+__global__ void __cluster_dims__(GB_CTAS, 1, 1) __launch_bounds__(256)
+    gates_bwd_kernel(const void* a_, const void* b_, int dt, const float* A_log, const float* dt_bias, const float* dg, const float* dbeta,
+                     size_t tokens, int Hv, void* da, void* db, float* dA_log, float* d_dt_bias) {
+  __shared__ float red[2][256], sums[2][GB_HEADS];
+  const int rank = blockIdx.x % GB_CTAS, tid = threadIdx.x, hl = tid % GB_HEADS, h = blockIdx.x / GB_CTAS * GB_HEADS + hl;
   float sA = 0.f, sB = 0.f;
-  for (size_t t = threadIdx.x; t < tokens; t += 256) {
-    const size_t e = t * Hv + h;
-    const float x = ldf_ro(a_, e, dt) + bias;
-    const float sp = softplus(x), sg = 1.f / (1.f + expf(-x));
-    const float d = dg[e];
-    const float dx = d * Ae * sg;
-    stf(da, e, dx, dt);
-    const float be = 1.f / (1.f + expf(-ldf_ro(b_, e, dt)));
-    stf(db, e, dbeta[e] * be * (1.f - be), dt);
-    sA += d * Ae * sp;
-    sB += dx;
+  if (h < Hv) {
+    const float Ae = -expf(A_log[h]), bias = dt_bias[h];
+#pragma unroll 4
+    for (size_t t = rank * (256 / GB_HEADS) + tid / GB_HEADS; t < tokens; t += GB_CTAS * (256 / GB_HEADS)) {
+      const size_t e = t * Hv + h;
+      const float x = ldf_ro(a_, e, dt) + bias, braw = ldf_ro(b_, e, dt), d = __ldg(dg + e), dbe = __ldg(dbeta + e);
+      const float sp = softplus(x), sg = 1.f / (1.f + expf(-x));
+      const float dx = d * Ae * sg;
+      stf(da, e, dx, dt);
+      const float be = 1.f / (1.f + expf(-braw));
+      stf(db, e, dbe * be * (1.f - be), dt);
+      sA += d * Ae * sp;
+      sB += dx;
+    }
   }
-  __shared__ float red[2][256];
-  red[0][threadIdx.x] = sA; red[1][threadIdx.x] = sB;
+  red[0][tid] = sA;
+  red[1][tid] = sB;
   __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) { red[0][threadIdx.x] += red[0][threadIdx.x + o]; red[1][threadIdx.x] += red[1][threadIdx.x + o]; }
+  for (int o = 128; o >= GB_HEADS; o >>= 1) {
+    if (tid < o) { red[0][tid] += red[0][tid + o]; red[1][tid] += red[1][tid + o]; }
     __syncthreads();
   }
-  if (threadIdx.x == 0) { dA_log[h] = red[0][0]; d_dt_bias[h] = red[1][0]; }
+  if (tid < GB_HEADS) { sums[0][tid] = red[0][tid]; sums[1][tid] = red[1][tid]; }
+  auto cluster = cooperative_groups::this_cluster();
+  cluster.sync();
+  if (rank == 0 && tid < GB_HEADS && h < Hv) {
+    float tA = 0.f, tB = 0.f;
+    for (int r = 0; r < GB_CTAS; ++r) {
+      const float* peer = cluster.map_shared_rank(&sums[0][0], r);
+      tA += peer[tid];
+      tB += peer[GB_HEADS + tid];
+    }
+    dA_log[h] = tA;
+    d_dt_bias[h] = tB;
+  }
+  cluster.sync();                                        // the peers' shared memory has been read
 }
 
 // ---- gated RMSNorm -----------------------------------------------------------------------------------
@@ -724,7 +744,7 @@ int dn_gdn_gates_bwd(const void* a, const void* b, const float* A_log, const flo
   if (!a || !b || !A_log || !dt_bias || !dg || !dbeta || !da || !db || !dA_log || !d_dt_bias) return DN_ERR_NULL_POINTER;
   if (B < 1 || L < 1 || Hv < 1) return DN_ERR_BAD_SHAPE;
   if (dtype != DN_F32 && dtype != DN_BF16) return DN_ERR_BAD_DTYPE;
-  gates_bwd_kernel<<<Hv, 256, 0, (cudaStream_t)stream>>>(a, b, dtype, A_log, dt_bias, dg, dbeta, (size_t)B * L, Hv, da, db,
+  gates_bwd_kernel<<<(Hv + GB_HEADS - 1) / GB_HEADS * GB_CTAS, 256, 0, (cudaStream_t)stream>>>(a, b, dtype, A_log, dt_bias, dg, dbeta, (size_t)B * L, Hv, da, db,
                                                          dA_log, d_dt_bias);
   return launch_status();
 }

@@ -47,7 +47,7 @@ __device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 
 
 // The kernel's code runs once per tile and did not fit the instruction cache when every product, wait and drain was
 // expanded in place (160 to 270 KB): 16 warps then stalled on fetches, and a few instructions more in each wait were worth
-// 15 %.  So these are calls, and loops over the 32 columns a warp drains stay rolled in pieces of eight.
+// 15 %.  So these are calls, and loops over the 32 columns a warp drains stay rolled.
 __device__ __noinline__ void product_call(uint32_t d, uint64_t ad, uint64_t bd, uint32_t a_step, uint32_t b_step, uint32_t idesc, int n, uint32_t acc) {
 #pragma unroll 4
   for (int k = 0; k < n; ++k) {
@@ -64,9 +64,6 @@ __device__ __forceinline__ void product(const umma::Ctx& cx, const void* A, uint
   product_call(cx.tmem + col, umma::smem_desc(umma::smem_u32(A), A_MN ? 128u : pa, A_MN ? pa : 128u),
                umma::smem_desc(umma::smem_u32(B), B_MN ? 128u : pb, B_MN ? pb : 128u), (A_MN ? 256u : 2u * pa) >> 4, (B_MN ? 256u : 2u * pb) >> 4,
                umma::instr_desc(N, A_MN ? 1 : 0, B_MN ? 1 : 0), Kc / 16, acc ? 1u : 0u);
-}
-__device__ __forceinline__ void commit(const umma::Ctx& cx) {
-  if (threadIdx.x < 32 && !cx.dead) umma::mma_commit_warp(cx.bar);
 }
 __device__ __noinline__ bool bar_wait_call(uint64_t* bar, uint32_t parity, int* err) {
   if (umma::mbar_wait(bar, parity)) return true;

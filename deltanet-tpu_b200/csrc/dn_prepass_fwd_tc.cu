@@ -170,7 +170,7 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
   umma::pre_issue_sync();
   umma::issue_pitched<128, false, true>(cx, TI, 2048, XI, PB, C, 0, false);
   umma::issue_pitched<HW, false, true>(cx, TI, 2048, Y0, PB, C, 128, false);
-  if (tid == 0 && !cx.dead) umma::mma_commit(cx.bar);
+  umma::commit(cx);
   if (NH == 2) request_v(1);
   if (a.res.T) {                                        // the image of T, for the backward
     uint4* Tg = reinterpret_cast<uint4*>(a.res.T + ibase * C * C);
@@ -190,7 +190,7 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
     __syncthreads();
     umma::tc_fence_after();
     umma::issue_pitched<HW, false, true>(cx, TI, 2048, XI, PB, C, 0, false);
-    if (tid == 0 && !cx.dead) umma::mma_commit(cx.bar);
+    umma::commit(cx);
   }
   umma::drain<NT, HW>(cx, 128, [&](int row, int col, const float (&v)[16]) {
     Uimg[(col / 8) * 128 + row] = umma::pack8p(v);
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_scalar_kernel(const __grid_
     umma::pre_issue_sync();
     umma::issue_pitched<128, false, false>(cx, KI, PB, KI, PB, K, 0, false);             // k_hat k_hat^T
     umma::issue_pitched<128, false, false>(cx, QI, PB, KI, PB, K, 128, false);           // q_hat k_hat^T
-    if (tid == 0 && !cx.dead) umma::mma_commit(cx.bar);
+    umma::commit(cx);
     const float lam = lam_s[x], lend = lam_s[C - 1], el = umma::exp_neg(fminf(lam, 0.f)), eke = umma::exp_neg(fminf(lend - lam, 0.f));
     const bool first = seg_s[x] == seg_s[0], last = seg_s[x] == seg_s[C - 1];
     {                                                   // qe, ke while the products run
@@ -788,7 +788,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       umma::pre_issue_sync();
       umma::issue_pitched<128, false, false>(cx, BF, PB, KF, PB, 32, 0, grp > 0);        // A += (beta f) (k / f)^T
       umma::issue_pitched<128, false, false>(cx, QF, PB, KF, PB, 32, 128, grp > 0);      // M += (q f) (k / f)^T
-      if (tid == 0 && !cx.dead) umma::mma_commit(&gbar[grp & 1]);
+      if (tid < 32 && !cx.dead) umma::mma_commit_warp(&gbar[grp & 1]);
       // global stores and the next group's loads come behind the proxy fence, which waits for what precedes it
       {
         uint4* QE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.qe) + ibase * C * K);

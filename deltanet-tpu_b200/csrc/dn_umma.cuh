@@ -165,19 +165,8 @@ __host__ __device__ constexpr uint32_t instr_desc(int N, int a_mn, int b_mn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
          ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// The same two issued by one elected lane of a warp that runs converged: the descriptors then stay in uniform registers
-// and a product of eight MMAs is issued in 290 cycles; from a branch that a single thread takes, in 560.
+// One MMA, and the commit of all issued so far, by one elected lane of a warp that runs converged: the descriptors then stay in
+// uniform registers and a product of eight MMAs is issued in 290 cycles; from a branch that a single thread takes, in 560.
 __device__ __forceinline__ void mma_bf16_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
@@ -318,23 +307,27 @@ __device__ __forceinline__ void pre_issue_sync() {
   tc_fence_after();
 }
 
-// Issue (one thread) the MMAs of D[128 x N] (+)= A[128 x Kc] B[N x Kc]^T on staged operands whose panels lie
+// Issue (first warp, converged) the MMAs of D[128 x N] (+)= A[128 x Kc] B[N x Kc]^T on staged operands whose panels lie
 // a_pitch / b_pitch bytes apart (panels written by threads that hold several pieces of one row are kept 32 bytes
 // further apart than they are long: the pieces then fall into different banks).
 template <int N, bool A_MN, bool B_MN>
 __device__ __forceinline__ void issue_pitched(const Ctx& cx, const void* sA, uint32_t a_pitch, const void* sB, uint32_t b_pitch, int Kc,
                                               uint32_t tmem_col, bool accumulate) {
-  if (threadIdx.x != 0 || cx.dead) return;
+  if (threadIdx.x >= 32 || cx.dead) return;
   constexpr uint32_t idesc = instr_desc(N, A_MN ? 1 : 0, B_MN ? 1 : 0);
   uint64_t ad = smem_desc(smem_u32(sA), A_MN ? 128u : a_pitch, A_MN ? a_pitch : 128u);
   uint64_t bd = smem_desc(smem_u32(sB), B_MN ? 128u : b_pitch, B_MN ? b_pitch : 128u);
   const uint32_t a_step = (A_MN ? 256u : 2u * a_pitch) >> 4, b_step = (B_MN ? 256u : 2u * b_pitch) >> 4;
 #pragma unroll 4
   for (int ks = 0; ks < Kc / 16; ++ks) {
-    mma_bf16(cx.tmem + tmem_col, ad, bd, idesc, (accumulate || ks > 0) ? 1u : 0u);
+    mma_bf16_warp(cx.tmem + tmem_col, ad, bd, idesc, (accumulate || ks > 0) ? 1u : 0u);
     ad += a_step;
     bd += b_step;
   }
+}
+// Commit everything issued so far to the context's barrier
+__device__ __forceinline__ void commit(const Ctx& cx) {
+  if (threadIdx.x < 32 && !cx.dead) mma_commit_warp(cx.bar);
 }
 // the same on images without padding
 template <int N, bool A_MN, bool B_MN>
@@ -353,9 +346,9 @@ __device__ __forceinline__ void commit_wait_only(Ctx& cx) {
   cx.phase ^= 1u;
   tc_fence_after();
 }
-// Commit everything issued so far (one thread) and make every thread wait for it, boundedly.
+// Commit everything issued so far and make every thread wait for it, boundedly.
 __device__ __forceinline__ void commit_wait(Ctx& cx) {
-  if (threadIdx.x == 0 && !cx.dead) mma_commit(cx.bar);
+  commit(cx);
   commit_wait_only(cx);
 }
 
