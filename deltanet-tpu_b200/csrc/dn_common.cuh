@@ -170,65 +170,155 @@ __device__ __forceinline__ void chunk_flags(const int32_t* seg, const Geo& g, in
 }
 
 // --------------------------------------------------------------------------- CTA GEMM
+// The CTAs that share one item: one CTA, or (SPLIT) the cluster, a power of two of them.  Rows, elements, channels and output
+// tiles are dealt out over the team; what one member has written to global memory the others read behind sync().
+template <bool SPLIT>
+struct Team {
+  int rank = 0, ranks = 1, tiles = 0;
+  __device__ Team() {
+    if constexpr (SPLIT) {
+      asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+      asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+    }
+  }
+  __device__ void sync() const {
+    if constexpr (SPLIT)
+      asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    else
+      __syncthreads();
+  }
+  // takes the next output tile; is it this CTA's?
+  __device__ bool mine() { return !SPLIT || (tiles++ & (ranks - 1)) == rank; }
+  __device__ int row0() const { return rank * (DN_THREADS / 32) + (threadIdx.x >> 5); }   // this warp's first row
+  __device__ int rows() const { return ranks * (DN_THREADS / 32); }                       // ... and its stride
+  __device__ int elem0() const { return rank * DN_THREADS + threadIdx.x; }                // this thread's first element
+  __device__ int elems() const { return ranks * DN_THREADS; }
+};
+// CTAs an item for a job of `items`: as many as the chip has room for at one per SM, 8 (the portable cluster) at most.
+inline int team_size(int items, int most = 8) {
+  int ranks = 1;
+  while (ranks < most && items * ranks * 2 <= sm_count()) ranks *= 2;
+  return ranks;
+}
+template <class ARGS>
+inline void launch_team(void (*kernel)(ARGS), int items, int ranks, size_t smem, cudaStream_t st, const ARGS& a) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = ranks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(items * ranks);
+  cfg.blockDim = dim3(DN_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
 // C[M x N] = A[M x Kc] * B[Kc x N] with fa(i,k), fb(k,j) giving operand elements and
-// epi(i,j,acc) consuming results.  256 threads, 64x64 output tiles, fp32 FMA.  M, N, Kc
-// need not be multiples of the tile (out-of-range operand elements are read as 0 and
-// out-of-range results are not passed to epi).  A_KFAST / B_NFAST say which index of the
+// epi(i,j,acc) consuming results.  256 threads, 64 x GN output tiles (GN 64, or 16 where a call should be spread over more
+// CTAs), fp32 FMA.  M a multiple of 64, N of GN, Kc of 32.  A_KFAST / B_NFAST say which index of the
 // operand is contiguous in memory, which only steers the (coalesced) tile-load mapping.
-// `tile` is 2*16*68 floats of shared memory.  Ends with a __syncthreads().
-constexpr int GT = 64, GK = 16, GS = 68;
+// What bounds it at the sizes it is used for is the latency of the operand loads, not the multiply-adds: a step takes 32
+// values of the contraction, 8 loads per thread and operand in flight together, and the next step's loads travel
+// during this step's arithmetic.  (Steps of 16 without that: the backward kernel of a 64 x 64 chunk took 243 us,
+// with both 195.)  fa and fb may be called for a step while the one before is computed, never across tiles.
+// `tile` is GEMM_SMEM_FLOATS of shared memory.  Ends with a __syncthreads().
+constexpr int GT = 64, GK = 32, GS = 68;
 constexpr int GEMM_SMEM_FLOATS = 2 * GK * GS;
 
-template <bool A_KFAST, bool B_NFAST, class FA, class FB, class EPI>
-__device__ __forceinline__ void cta_gemm(int M, int N, int Kc, FA fa, FB fb, EPI epi, float* tile) {
+template <bool A_KFAST, bool B_NFAST, int GN = 64, class FA, class FB, class EPI, class TEAM = Team<false>>
+__device__ __forceinline__ void cta_gemm(int M, int N, int Kc, FA fa, FB fb, EPI epi, float* tile, TEAM&& team = TEAM{}) {
+  constexpr int NA = GT * GK / DN_THREADS, NB = GN * GK / DN_THREADS, NC = GN / 16, BS = GN + 4;
   float* As = tile;
   float* Bs = tile + GK * GS;
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+#pragma unroll 1
   for (int m0 = 0; m0 < M; m0 += GT) {
-    for (int n0 = 0; n0 < N; n0 += GT) {
-      float acc[4][4];
+#pragma unroll 1
+    for (int n0 = 0; n0 < N; n0 += GN) {
+      if (!team.mine()) continue;
+      float acc[4][NC], ra[NA], rb[NB];
+      auto load = [&](int k0) {
+#pragma unroll
+        for (int r = 0; r < NA; ++r) {
+          const int idx = tid + r * DN_THREADS;
+          const int kk = A_KFAST ? idx % GK : idx / GT, i = A_KFAST ? idx / GK : idx % GT;
+          ra[r] = fa(m0 + i, k0 + kk);
+        }
+#pragma unroll
+        for (int r = 0; r < NB; ++r) {
+          const int idx = tid + r * DN_THREADS;
+          const int j = B_NFAST ? idx % GN : idx / GK, kk = B_NFAST ? idx / GN : idx % GK;
+          rb[r] = fb(k0 + kk, n0 + j);
+        }
+      };
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
+        for (int c = 0; c < NC; ++c) acc[r][c] = 0.f;
+      load(0);
+#pragma unroll 1
       for (int k0 = 0; k0 < Kc; k0 += GK) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          int idx = tid + r * DN_THREADS;
-          int i, kk;
-          if (A_KFAST) { kk = idx & 15; i = idx >> 4; } else { i = idx & 63; kk = idx >> 6; }
-          float v = 0.f;
-          if (m0 + i < M && k0 + kk < Kc) v = fa(m0 + i, k0 + kk);
-          As[kk * GS + i] = v;
-          int j, k2;
-          if (B_NFAST) { j = idx & 63; k2 = idx >> 6; } else { k2 = idx & 15; j = idx >> 4; }
-          float u = 0.f;
-          if (n0 + j < N && k0 + k2 < Kc) u = fb(k0 + k2, n0 + j);
-          Bs[k2 * GS + j] = u;
+        for (int r = 0; r < NA; ++r) {
+          const int idx = tid + r * DN_THREADS;
+          As[(A_KFAST ? idx % GK : idx / GT) * GS + (A_KFAST ? idx / GK : idx % GT)] = ra[r];
+        }
+#pragma unroll
+        for (int r = 0; r < NB; ++r) {
+          const int idx = tid + r * DN_THREADS;
+          Bs[(B_NFAST ? idx / GN : idx % GK) * BS + (B_NFAST ? idx % GN : idx / GK)] = rb[r];
         }
         __syncthreads();
-#pragma unroll
+        if (k0 + GK < Kc) load(k0 + GK);
+#pragma unroll 8
         for (int kk = 0; kk < GK; ++kk) {
-          float4 a = *reinterpret_cast<const float4*>(&As[kk * GS + ty * 4]);
-          float4 b = *reinterpret_cast<const float4*>(&Bs[kk * GS + tx * 4]);
-          float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+          const float4 a = *reinterpret_cast<const float4*>(&As[kk * GS + ty * 4]);
+          const float av[4] = {a.x, a.y, a.z, a.w};
+          float bv[NC];
+          if constexpr (NC == 4) {
+            const float4 b = *reinterpret_cast<const float4*>(&Bs[kk * BS + tx * 4]);
+            bv[0] = b.x; bv[1] = b.y; bv[2] = b.z; bv[3] = b.w;
+          } else {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) bv[c] = Bs[kk * BS + tx * NC + c];
+          }
 #pragma unroll
           for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av[r], bv[c], acc[r][c]);
+            for (int c = 0; c < NC; ++c) acc[r][c] = fmaf(av[r], bv[c], acc[r][c]);
         }
         __syncthreads();
       }
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          int i = m0 + ty * 4 + r, j = n0 + tx * 4 + c;
-          if (i < M && j < N) epi(i, j, acc[r][c]);
-        }
+        for (int c = 0; c < NC; ++c) epi(m0 + ty * 4 + r, n0 + tx * NC + c, acc[r][c]);
     }
   }
   __syncthreads();
+}
+
+// Sums down C rows (pitch K) of one column of a scratch array, restarting where a document starts (forward) or ends
+// (reverse); in place.  Rows are read 16 at a time: the sum is serial, the loads need not be.
+template <bool REVERSE>
+__device__ __forceinline__ void column_scan(float* col, const int* seg, int C, int K) {
+  float run = 0.f;
+#pragma unroll 1
+  for (int i0 = 0; i0 < C; i0 += 16) {
+    float v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v[u] = col[(size_t)(REVERSE ? C - 1 - i0 - u : i0 + u) * K];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int i = REVERSE ? C - 1 - i0 - u : i0 + u, before = REVERSE ? i + 1 : i - 1;
+      if (i0 + u > 0 && seg[i] != seg[before]) run = 0.f;
+      run += v[u];
+      col[(size_t)i * K] = run;
+    }
+  }
 }
 
 }  // namespace dn

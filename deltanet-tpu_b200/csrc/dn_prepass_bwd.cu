@@ -19,22 +19,29 @@
 
 namespace dn {
 
-
 // fp32 SIMT products (the tensor-core variant lives in dn_prepass_bwd_tc.cu).
+// SPLIT: the CTAs of a cluster share an item, and its scratch: rows, columns and output tiles are dealt out, and the cluster's
+// barrier stands between the phases.  For jobs that leave most of the chip idle (launch_prepass_bwd), where one item is a
+// chain of latencies: 64 x 64 heads, chunks of 64, 8 items: 195 us with one CTA an item, 59 with eight.
+template <bool SPLIT>
 __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdArgs a) {
   extern __shared__ __align__(128) float smem[];
   const Geo& g = a.g;
   const int C = g.C, K = g.K, Vw = g.Vw;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  Team<SPLIT> team;
+  const int ranks = team.ranks, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int cols = K / ranks, col0 = team.rank * cols;      // this CTA's channels in the scans
+  constexpr int GN = SPLIT ? 16 : 64;
   float* tile = smem;                      // SIMT GEMM staging
   float* rq_s = tile + GEMM_SMEM_FLOATS;   // C
   float* rk_s = rq_s + C;                  // C
   float* dlend_s = rk_s + C;               // K
   int* seg_s = reinterpret_cast<int*>(dlend_s + K);   // C
   int* dstart_s = seg_s + C;               // C first row of the row's document inside the chunk
+  int* dend_s = dstart_s + C;              // C last row
 
   const size_t CK = (size_t)C * K, CV = (size_t)C * Vw, CC = (size_t)C * C;
-  float* sc = a.scratch + (size_t)blockIdx.x * a.scratch_per_cta;
+  float* sc = a.scratch + (size_t)(blockIdx.x / ranks) * a.scratch_per_cta;
   float* QH = sc;            float* KH = QH + CK;      float* LAM = KH + CK;
   float* GB = LAM + CK;      float* BA = GB + CK;      float* DW = BA + CK;
   float* DQE = DW + CK;      float* DKE = DQE + CK;    float* DX = DKE + CK;
@@ -48,7 +55,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
   const bool sbf = g.state_bf16(), ibf = g.bf16_mode(), trunc = ibf && (g.flags & DN_TRUNC_DT_BF16);
   const int pre = g.pre_dt;
 
-  for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
+  for (int item = blockIdx.x / ranks; item < a.items; item += gridDim.x / ranks) {
     const int c_idx = item % g.NC, h = (item / g.NC) % g.H, b = item / (g.NC * g.H);
     const int t0 = c_idx * C;
     const int hq = h / g.qk_div;
@@ -59,6 +66,9 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
       int s = tid;
       while (s > 0 && seg_s[s - 1] == seg_s[tid]) --s;
       dstart_s[tid] = s;
+      s = tid;
+      while (s < C - 1 && seg_s[s + 1] == seg_s[tid]) ++s;
+      dend_s[tid] = s;
     }
     const int seg0 = seg_s[0], segL = seg_s[C - 1];
     bool is_new, all_same;
@@ -72,7 +82,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
 
     // ---- prologue (as in the forward prepass), keeping the row norms and the activated b
     const int per = K / 32;
-    for (int i = warp; i < C; i += DN_THREADS / 32) {
+    for (int i = team.row0(); i < C; i += team.rows()) {
       const int t = t0 + i;
       const bool valid = t < g.L;
       const size_t rowqk = ((size_t)(b * (size_t)g.L + t) * g.Hk + hq) * K;
@@ -120,79 +130,71 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
         GB[i * K + c] = ba * kh;
       }
     }
-    __syncthreads();
-    if (tid < K) {
-      float run = 0.f;
-      int prev = seg_s[0];
-      for (int i = 0; i < C; ++i) {
-        const int s = seg_s[i];
-        if (s != prev) run = 0.f;
-        prev = s;
-        run += LAM[i * K + tid];
-        LAM[i * K + tid] = run;
-      }
-    }
+    team.sync();
+    if (tid < cols) column_scan<false>(LAM + col0 + tid, seg_s, C, K);
     // dLambda_end from the carried state: [one doc] sum_v dH*S*exp(Lambda_end)   (gdn2.py:759-762)
-    for (int kk = warp; kk < K; kk += DN_THREADS / 32) {
+    for (int kk = col0 + warp; kk < col0 + cols; kk += DN_THREADS / 32) {
       float s = 0.f;
       for (int j = lane; j < Vw; j += 32) s += dH[(size_t)kk * Vw + j] * S[(size_t)kk * Vw + j];
       s = warp_sum(s);
       if (lane == 0) dlend_s[kk] = all_same ? s * expf(fminf(a.res.lam_end[ibase * K + kk], 0.f)) : 0.f;
     }
-    __syncthreads();
-
     // ---- V_new = U - W S
-    cta_gemm<true, true>(C, Vw, K,
+    cta_gemm<true, true, GN>(C, Vw, K,
         [&](int i, int kk) { return ldf(a.res.W, bW + rix(g.img, i, kk, K), pre); },
         [&](int kk, int j) { float s = S[(size_t)kk * Vw + j]; return sbf ? bf16r(s) : s; },
         [&](int i, int j, float acc) { VN[i * Vw + j] = ldf(a.res.U, bU + rix(g.img, i, j, Vw), pre) - acc; },
-        tile);
+        tile, team);
     auto dO_at = [&](int i, int j) -> float {
       const int t = t0 + i;
       return t < g.L ? ldf(a.d_out, ((size_t)b * g.L + t) * g.Hv * g.V + (size_t)h * Vw + j, g.qkv_dt) : 0.f;
     };
-    // ---- dW = -dV S^T, dqe = dO S^T, dke = V_new dH^T, dM = dO V_new^T
-    cta_gemm<true, false>(C, K, Vw,
+    // ---- dW = -dV S^T, dqe = dO S^T, dY = T^T dV, then dke = V_new dH^T, dM = dO V_new^T
+    cta_gemm<true, false, GN>(C, K, Vw,
         [&](int i, int kk) { float x = dV[(size_t)i * Vw + kk]; return sbf ? bf16r(x) : x; },
         [&](int kk, int j) { float s = S[(size_t)j * Vw + kk]; return sbf ? bf16r(s) : s; },
-        [&](int i, int j, float acc) { DW[i * K + j] = -acc; }, tile);
-    cta_gemm<true, false>(C, K, Vw,
+        [&](int i, int j, float acc) { DW[i * K + j] = -acc; }, tile, team);
+    cta_gemm<true, false, GN>(C, K, Vw,
         [&](int i, int kk) { float x = dO_at(i, kk); return sbf ? bf16r(x) : x; },
         [&](int kk, int j) { float s = S[(size_t)j * Vw + kk]; return sbf ? bf16r(s) : s; },
-        [&](int i, int j, float acc) { DQE[i * K + j] = acc; }, tile);
-    cta_gemm<true, false>(C, K, Vw,
-        [&](int i, int kk) { float x = VN[i * Vw + kk]; return sbf ? bf16r(x) : x; },
-        [&](int kk, int j) { float x = dH[(size_t)j * Vw + kk]; return sbf ? bf16r(x) : x; },
-        [&](int i, int j, float acc) { DKE[i * K + j] = acc; }, tile);
-    cta_gemm<true, false>(C, C, Vw,
-        [&](int i, int kk) { float x = dO_at(i, kk); return ibf ? bf16r(x) : x; },
-        [&](int kk, int j) { float x = VN[j * Vw + kk]; return ibf ? bf16r(x) : x; },
-        [&](int i, int j, float acc) { DM[i * C + j] = (i >= j && seg_s[i] == seg_s[j]) ? acc : 0.f; }, tile);
-    // ---- dX = T^T dW, dY = T^T dV
-    cta_gemm<false, true>(C, K, C,
-        [&](int i, int kk) { float t = g.img ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(T)[rix(true, kk, i, C)]) : T[(size_t)kk * C + i]; return ibf ? bf16r(t) : t; },
-        [&](int kk, int j) { float x = DW[kk * K + j]; return ibf ? bf16r(x) : x; },
-        [&](int i, int j, float acc) { DX[i * K + j] = trunc ? bf16r(acc) : acc; }, tile);
-    cta_gemm<false, true>(C, Vw, C,
+        [&](int i, int j, float acc) { DQE[i * K + j] = acc; }, tile, team);
+    cta_gemm<false, true, GN>(C, Vw, C,
         [&](int i, int kk) { float t = g.img ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(T)[rix(true, kk, i, C)]) : T[(size_t)kk * C + i]; return ibf ? bf16r(t) : t; },
         [&](int kk, int j) { float x = dV[(size_t)kk * Vw + j]; return ibf ? bf16r(x) : x; },
-        [&](int i, int j, float acc) { DY[i * Vw + j] = trunc ? bf16r(acc) : acc; }, tile);
+        [&](int i, int j, float acc) { DY[i * Vw + j] = trunc ? bf16r(acc) : acc; }, tile, team);
+    if (SPLIT) team.sync();
+    cta_gemm<true, false, GN>(C, K, Vw,
+        [&](int i, int kk) { float x = VN[i * Vw + kk]; return sbf ? bf16r(x) : x; },
+        [&](int kk, int j) { float x = dH[(size_t)j * Vw + kk]; return sbf ? bf16r(x) : x; },
+        [&](int i, int j, float acc) { DKE[i * K + j] = acc; }, tile, team);
+    cta_gemm<true, false, GN>(C, C, Vw,
+        [&](int i, int kk) { float x = dO_at(i, kk); return ibf ? bf16r(x) : x; },
+        [&](int kk, int j) { float x = VN[j * Vw + kk]; return ibf ? bf16r(x) : x; },
+        [&](int i, int j, float acc) { DM[i * C + j] = (i >= j && seg_s[i] == seg_s[j]) ? acc : 0.f; }, tile, team);
+    // ---- dX = T^T dW
+    cta_gemm<false, true, GN>(C, K, C,
+        [&](int i, int kk) { float t = g.img ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(T)[rix(true, kk, i, C)]) : T[(size_t)kk * C + i]; return ibf ? bf16r(t) : t; },
+        [&](int kk, int j) { float x = DW[kk * K + j]; return ibf ? bf16r(x) : x; },
+        [&](int i, int j, float acc) { DX[i * K + j] = trunc ? bf16r(acc) : acc; }, tile, team);
+    if (SPLIT) team.sync();
     // ---- dA = -(dX W^T + dY U^T), strictly lower and same document
-    cta_gemm<true, false>(C, C, K + Vw,
+    cta_gemm<true, false, GN>(C, C, K + Vw,
         [&](int i, int kk) { return kk < K ? DX[i * K + kk] : DY[i * Vw + (kk - K)]; },
         [&](int kk, int j) {
           return kk < K ? ldf(a.res.W, bW + rix(g.img, j, kk, K), pre)
                         : ldf(a.res.U, bU + rix(g.img, j, kk - K, Vw), pre);
         },
-        [&](int i, int j, float acc) { DA[i * C + j] = (i > j && seg_s[i] == seg_s[j]) ? -acc : 0.f; }, tile);
+        [&](int i, int j, float acc) { DA[i * C + j] = (i > j && seg_s[i] == seg_s[j]) ? -acc : 0.f; }, tile, team);
 
+    if (SPLIT) team.sync();
     // ---- adjoints of A and M, pair by pair.  Row side: dbeta', dq'.  Column side: dk'.
     // The diagonal pair (i == i) has exponent 0: it feeds dq and dk but not dLambda, and is
     // kept out of the dLambda products so that they do not leave a rounding residue.
-    for (int e = tid; e < C * K; e += DN_THREADS) {
+    for (int e = team.elem0(); e < C * K; e += team.elems()) {
       const int i = e / K, c = e - i * K;
       const float li = LAM[e] * DN_LOG2E;
       float sb = 0.f, sq = 0.f;
+#pragma unroll 8
       for (int j = dstart_s[i]; j < i; ++j) {
         const float ek = KH[j * K + c] * exp2f(fminf(li - LAM[j * K + c] * DN_LOG2E, 0.f));
         sb = fmaf(DA[i * C + j], ek, sb);
@@ -202,21 +204,23 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
       DBP[e] = sb;
       DQP[e] = fmaf(DM[i * C + i], KH[e], sq);
     }
-    for (int e = tid; e < C * K; e += DN_THREADS) {
+    for (int e = team.elem0(); e < C * K; e += team.elems()) {
       const int j = e / K, c = e - j * K;
       const float lj = LAM[e] * DN_LOG2E;
       float sk = 0.f;
-      for (int i = j + 1; i < C && seg_s[i] == seg_s[j]; ++i) {
+      const int i_end = dend_s[j];
+#pragma unroll 8
+      for (int i = j + 1; i <= i_end; ++i) {
         const float ex = exp2f(fminf(LAM[i * K + c] * DN_LOG2E - lj, 0.f));
         sk = fmaf(fmaf(DA[i * C + j], GB[i * K + c], DM[i * C + j] * QH[i * K + c]), ex, sk);
       }
       DLAM[e] -= KH[e] * sk;
       DKP[e] = fmaf(DM[j * C + j], QH[e], sk);
     }
-    __syncthreads();
+    team.sync();
 
     // ---- combine: dLambda, d q_hat, d k_hat, d b_act  (in place over DLAM, DQP, DKP, DBP)
-    for (int e = tid; e < C * K; e += DN_THREADS) {
+    for (int e = team.elem0(); e < C * K; e += team.elems()) {
       const int i = e / K, c = e - i * K;
       const float lam = LAM[e], el = expf(fminf(lam, 0.f));
       const float eke = expf(fminf(LAM[(C - 1) * K + c] - lam, 0.f));
@@ -234,29 +238,31 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
       DKP[e] = dk;
       DBP[e] = dbeta * kh;        // d b_act
     }
-    __syncthreads();
+    team.sync();
     // ---- dg_t = sum_{i >= t, same doc} dLambda_i  +  the Lambda_end path.  A row i of the last
     // document reaches the chunk end through every later g, so the ke term adds the prefix sum
     // of dke*ke over EARLIER rows (the equivalent "-dke*ke at row i, +sum at the last row" form
     // cancels only up to rounding); the carried-state term dLambda_end reaches every row.
-    if (tid < K) {
-      const int c = tid;
-      float run = 0.f;
-      for (int i = C - 1; i >= 0; --i) {
-        if (i < C - 1 && seg_s[i] != seg_s[i + 1]) run = 0.f;
-        run += DLAM[i * K + c];
-        DLAM[i * K + c] = run;
-      }
+    if (tid < cols) {
+      const int c = col0 + tid;
+      column_scan<true>(DLAM + c, seg_s, C, K);
       float acc = dlend_s[c];              // zero unless the chunk is one document
-      for (int i = 0; i < C; ++i) {
-        if (seg_s[i] != segL) continue;
-        DLAM[i * K + c] += acc;
-        acc += DKE[i * K + c];
+#pragma unroll 1
+      for (int i0 = 0; i0 < C; i0 += 16) {
+        float dl[16], ke[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) { dl[u] = DLAM[(i0 + u) * K + c]; ke[u] = DKE[(i0 + u) * K + c]; }
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+          if (seg_s[i0 + u] != segL) continue;
+          DLAM[(i0 + u) * K + c] = dl[u] + acc;
+          acc += ke[u];
+        }
       }
     }
-    __syncthreads();
+    team.sync();
     // ---- write dg, db (per row: gate adjoints, optional channel reduction)
-    for (int i = warp; i < C; i += DN_THREADS / 32) {
+    for (int i = team.row0(); i < C; i += team.rows()) {
       const int t = t0 + i;
       if (t >= g.L) continue;
       const size_t rowg = ((size_t)(b * (size_t)g.L + t) * g.gH + hg) * g.gC;
@@ -318,7 +324,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
     }
     // ---- dv = dY * w_act, dw = dY * v (+ sigmoid adjoint, optional column reduction)
     const int nvh = Vw / g.V;      // value heads inside this exec head
-    for (int rv = warp; rv < C * nvh; rv += DN_THREADS / 32) {
+    for (int rv = team.row0(); rv < C * nvh; rv += team.rows()) {
       const int i = rv / nvh, vh = rv - i * nvh, t = t0 + i;
       if (t >= g.L) continue;
       const int hv = h * g.G + vh;
@@ -337,7 +343,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
       }
       if (g.wC == 1) { sw = warp_sum(sw); if (lane == 0) stf(a.dw, outw, sw, a.dw_dt); }
     }
-    __syncthreads();
+    team.sync();
   }
 }
 
@@ -357,8 +363,10 @@ int launch_prepass_bwd(PrepassBwdArgs& a, size_t scratch_floats, cudaStream_t st
   const int max_ctas = 2 * sm_count();
   int grid = a.items < max_ctas ? a.items : max_ctas;
   if (scratch_floats < (size_t)grid * a.scratch_per_cta) return DN_ERR_SCRATCH_TOO_SMALL;
-  const size_t smem = (GEMM_SMEM_FLOATS + (size_t)4 * g.C + g.K) * sizeof(float);
-  prepass_bwd_kernel<<<grid, DN_THREADS, smem, st>>>(a);
+  const size_t smem = (GEMM_SMEM_FLOATS + (size_t)5 * g.C + g.K) * sizeof(float);
+  const int ranks = team_size(a.items);
+  if (ranks > 1) launch_team(prepass_bwd_kernel<true>, a.items, ranks, smem, st, a);
+  else prepass_bwd_kernel<false><<<grid, DN_THREADS, smem, st>>>(a);
   return launch_status();
 }
 

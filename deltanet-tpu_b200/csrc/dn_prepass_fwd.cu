@@ -25,11 +25,17 @@ __device__ __forceinline__ void tri_unrank(int m, int& bi, int& bj) {
   bj = m - r * (r + 1) / 2;
 }
 
+// SPLIT: the CTAs of a cluster share an item (see Team).  Each makes the whole inverse for itself; everything else is dealt out.
+// 64 x 64 heads, chunks of 64, 8 items: 69 us with one CTA an item, 28 with eight.
+template <bool SPLIT>
 __global__ void __launch_bounds__(DN_THREADS, 1) prepass_fwd_kernel(PrepassFwdArgs a) {
   extern __shared__ __align__(16) float smem[];
   const Geo& g = a.g;
   const int C = g.C, K = g.K, Vw = g.Vw;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  Team<SPLIT> team;
+  const int ranks = team.ranks, tid = threadIdx.x, lane = tid & 31;
+  const int cols = K / ranks, col0 = team.rank * cols;      // this CTA's channels in the scan
+  constexpr int GN = SPLIT ? 16 : 64, MB = SPLIT ? 2 : 4;   // columns of an output tile; edge of a micro-block of pairs
   float* As = smem;                    // C*C
   float* Ts = As + C * C;              // C*C
   float* Tm = Ts + C * C;              // C*C (merge temporary); panels alias Ts/Tm
@@ -38,19 +44,20 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_fwd_kernel(PrepassFwdAr
   float* tile = smem + a.smem_tile_off;
   int* seg_s = reinterpret_cast<int*>(tile + GEMM_SMEM_FLOATS);
 
-  float* sc = a.scratch + (size_t)blockIdx.x * a.scratch_per_cta;
+  float* sc = a.scratch + (size_t)(blockIdx.x / ranks) * a.scratch_per_cta;
   float* QH = sc;
   float* KH = QH + C * K;
   float* LAM = KH + C * K;
   float* GB = LAM + C * K;
   float* X = GB + C * K;
   float* Y = X + C * K;
+  float* AG = Y + C * Vw;              // C*C: A on its way between the CTAs
 
   const bool l2 = g.flags & DN_QK_L2NORM, fuse = g.flags & DN_FUSE_PROLOGUE;
   const bool guard = g.flags & DN_STABILITY_GUARD;
   const bool round_in = !fuse && g.qkv_dt == DN_BF16;
 
-  for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
+  for (int item = blockIdx.x / ranks; item < a.items; item += gridDim.x / ranks) {
     const int c_idx = item % g.NC, h = (item / g.NC) % g.H, b = item / (g.NC * g.H);
     const int t0 = c_idx * C;
     const int hq = h / g.qk_div;
@@ -61,7 +68,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_fwd_kernel(PrepassFwdAr
 
     // ---- 1. prologue, one warp per row
     const int per = K / 32;
-    for (int i = warp; i < C; i += DN_THREADS / 32) {
+    for (int i = team.row0(); i < C; i += team.rows()) {
       const int t = t0 + i;
       const bool valid = t < g.L;
       const size_t rowqk = ((size_t)(b * (size_t)g.L + t) * g.Hk + hq) * K;
@@ -107,25 +114,15 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_fwd_kernel(PrepassFwdAr
         GB[i * K + c] = ba * kh;
       }
     }
-    __syncthreads();
+    team.sync();
 
     // ---- 2. cumulative log-decay down the rows, restarting at document changes
-    if (tid < K) {
-      float run = 0.f;
-      int prev = seg_s[0];
-      for (int i = 0; i < C; ++i) {
-        const int s = seg_s[i];
-        if (s != prev) run = 0.f;
-        prev = s;
-        run += LAM[i * K + tid];
-        LAM[i * K + tid] = run;
-      }
-    }
-    __syncthreads();
+    if (tid < cols) column_scan<false>(LAM + col0 + tid, seg_s, C, K);
+    team.sync();
 
     // ---- 3. masked factors: X = [first doc] beta e^Lam, qe, ke, Lambda_end, Y = w*v
     const size_t ibase = (size_t)item;
-    for (int e = tid; e < C * K; e += DN_THREADS) {
+    for (int e = team.elem0(); e < C * K; e += team.elems()) {
       const int i = e / K, c = e - i * K;
       const float lam = LAM[e], el = expf(fminf(lam, 0.f));
       const bool first = seg_s[i] == seg0, last = seg_s[i] == segL;
@@ -135,7 +132,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_fwd_kernel(PrepassFwdAr
       stf(a.res.ke, ibase * C * K + e, last ? KH[e] * expf(fminf(lend - lam, 0.f)) : 0.f, g.pre_dt);
       if (i == C - 1) a.res.lam_end[ibase * K + c] = lam;
     }
-    for (int e = tid; e < C * Vw; e += DN_THREADS) {
+    for (int e = team.elem0(); e < C * Vw; e += team.elems()) {
       const int i = e / Vw, j = e - i * Vw;
       const int t = t0 + i;
       float y = 0.f;
@@ -151,22 +148,22 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_fwd_kernel(PrepassFwdAr
     for (int e = tid; e < C * C; e += DN_THREADS) As[e] = 0.f;
     __syncthreads();
 
-    // ---- 4. A and M, pair by pair in 4x4 micro-blocks, channels in panels of 32
-    const int nb = C / 4, nmb = nb * (nb + 1) / 2;
+    // ---- 4. A and M, pair by pair in MB x MB micro-blocks, channels in panels of 32
+    const int nb = C / MB, nmb = nb * (nb + 1) / 2;
     float* pL = pan;
     float* pK = pL + C * PS;
     float* pB = pK + C * PS;
     float* pQ = pB + C * PS;
-    for (int slot = 0; slot * DN_THREADS < nmb; ++slot) {
-      const int m = tid + slot * DN_THREADS;
+    for (int slot = 0; slot * team.elems() < nmb; ++slot) {
+      const int m = tid * ranks + team.rank + slot * team.elems();
       int bi = 0, bj = 0;
       const bool act = m < nmb;
       if (act) tri_unrank(m, bi, bj);
-      float accA[4][4], accM[4][4];
+      float accA[MB][MB], accM[MB][MB];
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
+      for (int r = 0; r < MB; ++r)
 #pragma unroll
-        for (int s = 0; s < 4; ++s) accA[r][s] = accM[r][s] = 0.f;
+        for (int s = 0; s < MB; ++s) accA[r][s] = accM[r][s] = 0.f;
       for (int p = 0; p < K / 32; ++p) {
         __syncthreads();                    // As zero-fill / previous panel consumers done
         for (int e = tid; e < C * 32; e += DN_THREADS) {
@@ -178,20 +175,21 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_fwd_kernel(PrepassFwdAr
         }
         __syncthreads();
         if (act) {
+#pragma unroll 4
           for (int c = 0; c < 32; ++c) {
-            float Li[4], Bi[4], Qi[4], Lj[4], Kj[4];
+            float Li[MB], Bi[MB], Qi[MB], Lj[MB], Kj[MB];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-              Li[r] = pL[(4 * bi + r) * PS + c];
-              Bi[r] = pB[(4 * bi + r) * PS + c];
-              Qi[r] = pQ[(4 * bi + r) * PS + c];
-              Lj[r] = pL[(4 * bj + r) * PS + c];
-              Kj[r] = pK[(4 * bj + r) * PS + c];
+            for (int r = 0; r < MB; ++r) {
+              Li[r] = pL[(MB * bi + r) * PS + c];
+              Bi[r] = pB[(MB * bi + r) * PS + c];
+              Qi[r] = pQ[(MB * bi + r) * PS + c];
+              Lj[r] = pL[(MB * bj + r) * PS + c];
+              Kj[r] = pK[(MB * bj + r) * PS + c];
             }
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
+            for (int r = 0; r < MB; ++r)
 #pragma unroll
-              for (int s = 0; s < 4; ++s) {
+              for (int s = 0; s < MB; ++s) {
                 const float kk = Kj[s] * exp2f(fminf(Li[r] - Lj[s], 0.f));
                 accA[r][s] = fmaf(Bi[r], kk, accA[r][s]);
                 accM[r][s] = fmaf(Qi[r], kk, accM[r][s]);
@@ -202,32 +200,40 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_fwd_kernel(PrepassFwdAr
       __syncthreads();                      // panels (aliasing Ts/Tm) no longer read
       if (act) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
+        for (int r = 0; r < MB; ++r)
 #pragma unroll
-          for (int s = 0; s < 4; ++s) {
-            const int i = 4 * bi + r, j = 4 * bj + s;
+          for (int s = 0; s < MB; ++s) {
+            const int i = MB * bi + r, j = MB * bj + s;
             const bool same = seg_s[i] == seg_s[j];
-            As[i * C + j] = (i > j && same) ? accA[r][s] : 0.f;
+            (SPLIT ? AG : As)[i * C + j] = (i > j && same) ? accA[r][s] : 0.f;
             stf(a.res.M, ibase * C * C + i * C + j, (i >= j && same) ? accM[r][s] : 0.f, g.pre_dt);
           }
       }
     }
     // upper micro-blocks of M are zero
-    for (int e = tid; e < C * C; e += DN_THREADS) {
+    for (int e = team.elem0(); e < C * C; e += team.elems()) {
       const int i = e / C, j = e - i * C;
-      if ((j >> 2) > (i >> 2)) stf(a.res.M, ibase * C * C + e, 0.f, g.pre_dt);
+      if (j / MB > i / MB) stf(a.res.M, ibase * C * C + e, 0.f, g.pre_dt);
     }
     for (int e = tid; e < C * C; e += DN_THREADS) { Ts[e] = 0.f; }
-    __syncthreads();
+    team.sync();
+    if (SPLIT) {
+      for (int e = tid; e < C * C; e += DN_THREADS)
+        if (e % C < e / C) As[e] = AG[e];
+      __syncthreads();
+    }
 
     // ---- 5. T = (I + A)^-1: 16x16 diagonal blocks by substitution, then block merges
     if (tid < C) {
-      const int j = tid, blk0 = j & ~15;
-      Ts[j * C + j] = 1.f;
-      for (int i = j + 1; i < blk0 + 16; ++i) {
-        float s = 0.f;
-        for (int m = j; m < i; ++m) s = fmaf(As[i * C + m], Ts[m * C + j], s);
-        Ts[i * C + j] = -s;
+      const int j = tid & 15, blk0 = tid & ~15;      // column j of the block that starts at row blk0
+      float t[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        float s = i == j ? -1.f : 0.f;
+#pragma unroll
+        for (int m = 0; m < i; ++m) s = fmaf(As[(blk0 + i) * C + blk0 + m], t[m], s);
+        t[i] = -s;                                   // exactly 0 above the diagonal
+        if (i >= j) Ts[(blk0 + i) * C + tid] = -s;
       }
     }
     __syncthreads();
@@ -235,9 +241,10 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_fwd_kernel(PrepassFwdAr
       const int total = C * s / 2;
       for (int e = tid; e < total; e += DN_THREADS) {
         const int p = e / (s * s), rem = e - p * s * s, il = rem / s, jl = rem - il * s;
-        const int i = 2 * p * s + s + il, j = 2 * p * s + jl, mend = 2 * p * s + s;
+        const int i = 2 * p * s + s + il, j = 2 * p * s + jl, m0 = 2 * p * s;
         float acc = 0.f;
-        for (int m = j; m < mend; ++m) acc = fmaf(As[i * C + m], Ts[m * C + j], acc);
+#pragma unroll 16
+        for (int m = 0; m < s; ++m) acc = fmaf(As[i * C + m0 + m], Ts[(m0 + m) * C + j], acc);
         Tm[i * C + j] = acc;
       }
       __syncthreads();
@@ -245,13 +252,14 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_fwd_kernel(PrepassFwdAr
         const int p = e / (s * s), rem = e - p * s * s, il = rem / s, jl = rem - il * s;
         const int i = 2 * p * s + s + il, j = 2 * p * s + jl, m0 = 2 * p * s + s;
         float acc = 0.f;
-        for (int m = m0; m <= i; ++m) acc = fmaf(Ts[i * C + m], Tm[m * C + j], acc);
+#pragma unroll 16
+        for (int m = 0; m < s; ++m) acc = fmaf(Ts[i * C + m0 + m], Tm[(m0 + m) * C + j], acc);
         Ts[i * C + j] = -acc;
       }
       __syncthreads();
     }
     if (a.res.T)
-      for (int e = tid; e < C * C; e += DN_THREADS) a.res.T[ibase * C * C + e] = Ts[e];
+      for (int e = team.elem0(); e < C * C; e += team.elems()) a.res.T[ibase * C * C + e] = Ts[e];
 
     // ---- 6. W = T X, U = T Y (operands rounded to bf16 in bf16 precision, gdn2.py:226-230)
     const bool bf = g.bf16_mode();
@@ -259,25 +267,25 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_fwd_kernel(PrepassFwdAr
       void* Wd = a.res.W;
       const int pre = g.pre_dt;
       const size_t base = ibase * C * K;
-      cta_gemm<true, true>(C, K, C,
+      cta_gemm<true, true, GN>(C, K, C,
           [&](int i, int kk) { float t = Ts[i * C + kk]; return bf ? bf16r(t) : t; },
           [&](int kk, int j) { float x = X[kk * K + j]; return bf ? bf16r(x) : x; },
-          [&](int i, int j, float acc) { stf(Wd, base + (size_t)i * K + j, acc, pre); }, tile);
+          [&](int i, int j, float acc) { stf(Wd, base + (size_t)i * K + j, acc, pre); }, tile, team);
     }
     {
       void* Ud = a.res.U;
       const int pre = g.pre_dt;
       const size_t base = ibase * C * Vw;
-      cta_gemm<true, true>(C, Vw, C,
+      cta_gemm<true, true, GN>(C, Vw, C,
           [&](int i, int kk) { float t = Ts[i * C + kk]; return bf ? bf16r(t) : t; },
           [&](int kk, int j) { float y = Y[kk * Vw + j]; return bf ? bf16r(y) : y; },
-          [&](int i, int j, float acc) { stf(Ud, base + (size_t)i * Vw + j, acc, pre); }, tile);
+          [&](int i, int j, float acc) { stf(Ud, base + (size_t)i * Vw + j, acc, pre); }, tile, team);
     }
-    __syncthreads();
+    team.sync();
   }
 }
 
-static size_t scratch_per_cta(const Geo& g) { return (size_t)5 * g.C * g.K + (size_t)g.C * g.Vw; }
+static size_t scratch_per_cta(const Geo& g) { return (size_t)5 * g.C * g.K + (size_t)g.C * g.Vw + (size_t)g.C * g.C; }
 size_t prepass_fwd_scratch_floats(const Geo& g) {
   if (prepass_fwd_tc_eligible(g)) return 0;
   const size_t items = (size_t)g.B * g.H * g.NC, ctas = items < (size_t)sm_count() ? items : (size_t)sm_count();
@@ -299,8 +307,14 @@ int launch_prepass_fwd(const Geo& g, const void* q, const void* k, const void* v
   a.smem_tile_off = 3 * g.C * g.C;
   if (4 * g.C * 33 > 2 * g.C * g.C) a.smem_tile_off = g.C * g.C + 4 * g.C * 33;
   size_t smem = ((size_t)a.smem_tile_off + GEMM_SMEM_FLOATS + g.C) * sizeof(float);
-  cudaFuncSetAttribute(prepass_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  prepass_fwd_kernel<<<grid, DN_THREADS, smem, st>>>(a);
+  const int ranks = team_size(a.items);
+  if (ranks > 1) {
+    cudaFuncSetAttribute(prepass_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    launch_team(prepass_fwd_kernel<true>, a.items, ranks, smem, st, a);
+  } else {
+    cudaFuncSetAttribute(prepass_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    prepass_fwd_kernel<false><<<grid, DN_THREADS, smem, st>>>(a);
+  }
   return launch_status();
 }
 
