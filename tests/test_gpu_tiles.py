@@ -1,0 +1,129 @@
+"""The chunk kernels at the sizes where a tile, a route or a split of the work begins or ends, against the CPU oracle.
+
+Tolerances.  fp32: a value passes through at most six contractions of at most 256 products, each with a relative rounding
+error of about sqrt(256) * 2^-24 = 1e-6, and through the inverse of a unit triangular matrix whose entries stay below 10 for
+these inputs: under 1e-4, asserted at 2e-4.  bf16: each of about eight operands in a row is rounded to 8 bits, a relative
+error of 2^-9 / sqrt(3) = 1.1e-3 rms, and errors of the inverse reach the result about four times: 8e-3 to 1.3e-2, asserted at
+2e-2.  Whole numbers, and the same kernels called by another path, are equal.
+"""
+import pytest
+import torch
+
+from oracle import delta_oracle as O
+from test_gpu_tc_modes import compare, gdn_inputs
+
+pytestmark = pytest.mark.gpu
+
+BF16_TOL = 2e-2
+FP32_TOL = 2e-4
+
+
+@pytest.fixture(scope="module")
+def dn():
+    import deltanet_b200
+    return deltanet_b200
+
+
+def docs(B, L, *starts):
+    seg = torch.zeros(B, L, dtype=torch.int32)
+    for s in starts:
+        seg[:, s:] += 1
+    return seg
+
+
+# ---- fp32: an item per CTA or shared by a cluster, the chain with one or two staged chunks or none
+@pytest.mark.parametrize("C,K,V", [(64, 64, 64), (64, 128, 64), (128, 64, 128), (128, 128, 64)])
+@pytest.mark.parametrize("B,L", [(1, 1), (1, 257), (13, 130)])      # 8, 8 to 4 and 1 to 2 CTAs an item
+def test_fp32_splits(dn, C, K, V, B, L):
+    Hk, Hv = (1, 2) if B == 1 else (2, 4)
+    ins = O.make_inputs(31, B, L, Hk, Hv, K, V)[:6]
+    init = torch.randn(B, Hv, K, V, generator=torch.Generator().manual_seed(32)) * 0.1
+    seg = docs(B, L, 70, 128) if L > 128 else None
+    kw = dict(chunk_size=C, precision="fp32", qk_l2norm=True, output_final_state=True)
+    compare(lambda t, i: dn.chunk_gdn2(*t, segment_ids=None if seg is None else seg.cuda(), initial_state=i, **kw),
+            lambda t, i: O.chunk_gdn2(*t, segment_ids=seg, initial_state=i, **kw), list(ins), tol=FP32_TOL, init=init)
+
+
+# ---- bf16: key and value widths of 64 on padded tensor-core tiles
+@pytest.mark.parametrize("K,V,Hk,Hv", [(64, 64, 2, 2), (64, 64, 1, 2), (64, 64, 1, 3), (64, 64, 1, 4), (64, 128, 1, 2),
+                                       (128, 64, 2, 2), (128, 64, 1, 3)])
+@pytest.mark.parametrize("L,recompute", [(1, False), (127, False), (257, True)])
+def test_bf16_narrow_heads(dn, K, V, Hk, Hv, L, recompute):
+    ins = list(O.make_inputs(41, 1, L, Hk, Hv, K, V, qkv_dtype=torch.bfloat16)[:6])
+    ins[3] = ins[3].clone()
+    ins[3][:, L // 2:, :, ::7] *= 40.0                              # some channels decay to nothing inside a tile
+    init = torch.randn(1, Hv, K, V, generator=torch.Generator().manual_seed(42)) * 0.1
+    seg = docs(1, L, 60, 200) if L > 200 else None
+    kw = dict(chunk_size=128, precision="bf16", qk_l2norm=True, output_final_state=True)
+    compare(lambda t, i: dn.chunk_gdn2(*t, segment_ids=None if seg is None else seg.cuda(), initial_state=i,
+                                       recompute_states=recompute, **kw),
+            lambda t, i: O.chunk_gdn2(*t, segment_ids=seg, initial_state=i, **kw), ins, tol=BF16_TOL, init=init)
+
+
+# ---- scalar gates: heads of one key head taken in turn (288 items) or apart (144); the wide forward chain
+@pytest.mark.parametrize("B,L", [(18, 250), (18, 128)])
+def test_shared_key_heads(dn, B, L):
+    _, q, k, v, g, beta = gdn_inputs(51, B, L, 4, 8)
+    kw = dict(chunk_size=128, precision="bf16", qk_l2norm=True, output_final_state=True)
+    compare(lambda t, i: dn.chunk_gdn(*t, **kw), lambda t, i: O.chunk_gdn(*t, **kw), [q, k, v, g, beta], tol=BF16_TOL)
+
+
+# ---- segment ids in blocks: a run of equal ids may cross any number of them
+@pytest.mark.parametrize("L", [1, 255, 1024, 1025, 20011])
+def test_canonical_segments(dn, L):
+    from deltanet_b200 import _lib
+    gen = torch.Generator().manual_seed(61)
+    raw = torch.randint(-3, 3, (3, L), generator=gen, dtype=torch.int32)
+    raw[1] = 5                                                       # one document
+    raw[2, : L // 2] = raw[2, 0]                                     # one long document, then many short ones
+    new = torch.tensor([1, 0, 1], dtype=torch.int32)
+    ref = torch.zeros(3, L, dtype=torch.int64)
+    ref[:, 1:] = (raw[:, 1:] != raw[:, :-1]).long().cumsum(1)
+    lib = _lib.lib()
+    for first in (None, new):
+        out = torch.empty(3, L, dtype=torch.int32, device="cuda")
+        dev, fdev = raw.cuda(), None if first is None else first.cuda()
+        rc = lib.dn_canonical_segments(dev.data_ptr(), None if first is None else fdev.data_ptr(), out.data_ptr(), 3, L,
+                                       torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        assert torch.equal(out.cpu().long(), ref if first is None else ref + first[:, None])
+
+
+# ---- gate gradients: heads that do not fill a cluster's four, and tokens that do not fill its CTAs
+@pytest.mark.parametrize("B,L,Hv", [(1, 1, 1), (1, 3, 6), (2, 301, 5), (1, 64, 32)])
+def test_gate_gradients(dn, B, L, Hv):
+    gen = torch.Generator().manual_seed(71)
+    leaves = [torch.randn(B, L, Hv, generator=gen), torch.randn(B, L, Hv, generator=gen), torch.randn(Hv, generator=gen),
+              torch.randn(Hv, generator=gen)]
+    leaves = [t.requires_grad_() for t in leaves]
+    a, b, A_log, dt = leaves
+    ref = (-A_log.exp() * torch.nn.functional.softplus(a + dt), torch.sigmoid(b))
+    cot = [torch.randn(B, L, Hv, generator=gen) for _ in range(2)]
+    r = torch.autograd.grad(sum((x * c).sum() for x, c in zip(ref, cot)), leaves)
+    dev = [t.detach().cuda().requires_grad_() for t in leaves]
+    got = dn.gdn_gates(*dev)
+    s = torch.autograd.grad(sum((x * c.cuda()).sum() for x, c in zip(got, cot)), dev)
+    for x, y in zip(s, r):                                           # sums of at most 602 fp32 values: 602 * 2^-24 = 4e-5
+        assert O.rel_l2(x.cpu(), y) < 4e-5
+
+
+# ---- the operators' native host path and the general one launch the same kernels
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_host_paths_agree(dn, dtype):
+    B, L, H, K = 1, 300, 2, 64
+    ins = [t.cuda() for t in O.make_inputs(81, B, L, H, H, K, K, qkv_dtype=dtype)[:6]]
+    seg = docs(B, L, 111).cuda()
+    kw = dict(precision="fp32" if dtype == torch.float32 else "bf16", qk_l2norm=True, output_final_state=True)
+    strided = [torch.stack([t, t], -1)[..., 0] for t in ins]
+    res = []
+    for args, ids in ((ins, seg), (strided, seg.long())):
+        leaves = [t.detach().requires_grad_() for t in args]
+        o, s = dn.chunk_gdn2(*leaves, segment_ids=ids, **kw)
+        res.append((o, s) + torch.autograd.grad(o.float().sum() + s.sum(), leaves))
+    assert [torch.equal(x, y) for x, y in zip(*res)] == [True] * 8
+    st = torch.zeros(B, H, K, K, device="cuda")
+    tok, wide = [t[:, 0].contiguous() for t in ins], [t[:, 0] for t in strided]
+    for state_dtype in (torch.float32, torch.bfloat16):
+        one = dn.gdn2_decode_step(*tok, st.to(state_dtype), reset=torch.tensor([1], device="cuda", dtype=torch.int32))
+        two = dn.gdn2_decode_step(*wide, st.to(state_dtype), reset=torch.tensor([True], device="cuda"))
+        assert all(torch.equal(x, y) for x, y in zip(one, two))
