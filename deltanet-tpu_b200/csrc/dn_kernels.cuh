@@ -36,6 +36,7 @@ struct StateArgs {
   int c_begin, c_end;
   float* carry;
   int* err;                  // error word (bounded waits report here); set by the launchers
+  int parts;                 // walks the range may be cut into at document boundaries (tensor-core path; set by the launcher)
   // Sequence-sharded use.  P_out (B,H,K,K): the forward launch carries K extra "value" columns per
   // (batch, head) that start from the identity with U = 0 and end as the shard's transition matrix
   // (grid.x grows by K / VS slices; those slices write neither outputs nor chunk states).

@@ -140,7 +140,52 @@ __device__ __forceinline__ void store32(float* p, const float (&v)[32]) {
   }
 }
 
-template <int VS>
+// A document boundary cuts the chain: what a chunk that holds one, or starts with one, hands on does not depend on what it is
+// handed.  So the range [c_begin, c_end) is dealt out in `parts` equal parts.  The CTA of the first part starts where the
+// range does, that of any other at the first cut inside its part, and each ends where the next one starts; a part without a
+// cut has no walk and its CTA leaves.  Where the boundary lies inside a chunk, the new walk takes this chunk from zeros, for
+// what it hands on alone (`warm` = 1: it stores nothing of it).  Results are those of a single walk, bit for bit.
+// `found`: two words of shared memory.  Every thread calls; false: no walk.
+template <bool REVERSE, int NT>
+__device__ __forceinline__ bool find_walk(const StateArgs& a, int b, int part, int* found, int& lo, int& hi, int& warm) {
+  const int begin = a.c_begin, end = a.c_end, len = (end - begin + a.parts - 1) / a.parts, tid = threadIdx.x;
+  // the part, in the order of the walk: s0 its first chunk, s1 the first of the next part
+  const int s0 = REVERSE ? end - 1 - part * len : begin + part * len;
+  const int s1 = REVERSE ? max(begin - 1, s0 - len) : min(end, s0 + len);
+  constexpr int dir = REVERSE ? -1 : 1, none = REVERSE ? -1 : 0x7fffffff;
+  if (tid < 2) found[tid] = none;
+  __syncthreads();
+  auto search = [&](int from, int to, int* f) {
+    for (int c = from + dir * tid; dir * c < dir * to; c += dir * NT) {
+      bool n, s;
+      chunk_flags(a.seg, a.g, b, c, n, s);
+      // (a cut behind which nothing is left to walk is none)
+      if (REVERSE ? (n || !s) && c > begin : n || (!s && c + 1 < end)) {
+        const int v = 2 * c + (n ? 0 : 1);
+        if (REVERSE) atomicMax(f, v); else atomicMin(f, v);
+        break;
+      }
+    }
+  };
+  if (part > 0) search(s0, s1, &found[0]);
+  search(s1, REVERSE ? begin - 1 : end, &found[1]);
+  __syncthreads();
+  const int f0 = found[0], f1 = found[1];
+  if (part > 0 && f0 == none) return false;
+  warm = part > 0 ? f0 & 1 : 0;
+  if (REVERSE) {
+    hi = part > 0 ? (f0 >> 1) + warm : end;
+    lo = f1 == none ? begin : f1 >> 1;
+  } else {
+    lo = part > 0 ? f0 >> 1 : begin;
+    hi = f1 == none ? end : (f1 >> 1) + (f1 & 1);
+  }
+  return true;
+}
+
+// CUT: the range may be cut into several walks (find_walk).  An instance of its own, since bounds that are the launch's
+// parameters leave the uncut chain faster (by 17 us of 331 at 256 CTAs and 64 chunks).
+template <int VS, bool CUT>
 __global__ void __launch_bounds__(Plan<VS, false>::NT, 1) state_fwd_tc_kernel(const __grid_constant__ StateArgs a) {
   using PL = Plan<VS, false>;
   constexpr int ST = PL::ST, NG = PL::NG, SLOTS = PL::SLOTS;
@@ -152,7 +197,7 @@ __global__ void __launch_bounds__(Plan<VS, false>::NT, 1) state_fwd_tc_kernel(co
   __shared__ int stop_s;
   const Geo& g = a.g;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // (warp: uniform for the compiler)
-  const int Vw = g.Vw, vr = g.G * g.V, h = blockIdx.y, b = blockIdx.z;
+  const int Vw = g.Vw, vr = g.G * g.V, h = blockIdx.y, b = CUT ? blockIdx.z % g.B : blockIdx.z;
   // slices past the value width carry the transition columns (see StateArgs::P_out)
   const bool trans = (int)blockIdx.x * VS >= Vw;
   const int v0 = trans ? 0 : blockIdx.x * VS, p0 = trans ? blockIdx.x * VS - Vw : 0;
@@ -160,8 +205,10 @@ __global__ void __launch_bounds__(Plan<VS, false>::NT, 1) state_fwd_tc_kernel(co
   uint8_t* sS = sm + SLOTS * TILE_B;
   uint8_t* sV = sS + PL::SL;                            // ROWS buffers
   float* lam_s = reinterpret_cast<float*>(sV + ROWS * PL::SL);
-  const int cb = a.c_begin;
-  int ce = a.c_end;
+  int cb = a.c_begin, ce = a.c_end, warm = 0;
+  __shared__ int found_s[2];
+  if (CUT && !find_walk<false, PL::NT>(a, b, blockIdx.z / g.B, found_s, cb, ce, warm)) return;
+  const bool first_walk = !CUT || cb == a.c_begin, last_walk = !CUT || ce == a.c_end;
   if (tid == 0) {
     for (int i = 0; i < SLOTS; ++i) { umma::mbar_init(&full[i], 1); umma::mbar_init(&empty[i], 1); }
     for (int i = 0; i < ROWS; ++i) { umma::mbar_init(&row_full[i], 1); umma::mbar_init(&row_empty[i], 1); }
@@ -189,7 +236,7 @@ __global__ void __launch_bounds__(Plan<VS, false>::NT, 1) state_fwd_tc_kernel(co
   if (a.until_independent && stop + 1 < ce) ce = stop + 1;
   const int n = ce - cb;
   // index of the first chunk whose outputs are wanted
-  const int o_from = (!a.out || trans) ? n : (a.skip_provisional ? (stop + 1 < ce ? stop + 1 - cb : n) : 0);
+  const int o_from = (!a.out || trans) ? n : (a.skip_provisional ? (stop + 1 < ce ? stop + 1 - cb : n) : warm);
   const uint32_t tm = tmem_base;
   constexpr uint32_t colP = 0, colS = VS, colO = 2 * VS;
   const size_t item0 = ((size_t)b * g.H + h) * g.NC + cb;
@@ -208,7 +255,7 @@ __global__ void __launch_bounds__(Plan<VS, false>::NT, 1) state_fwd_tc_kernel(co
     float S[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) S[j] = 0.f;
-    if (cb > 0) load32(carry, S);
+    if (cb > 0 && first_walk) load32(carry, S);
     Flags fl;
     fl.fill(a.seg, g, b, cb, 1, cb, ce);
     if (cb == 0 && !(fl.is_new & 1u)) {
@@ -283,6 +330,8 @@ __global__ void __launch_bounds__(Plan<VS, false>::NT, 1) state_fwd_tc_kernel(co
       // nothing to hand on: the caller has the final state from the shard's affine summary
     } else if (trans) {
       if (row < g.K) store32(a.P_out + (((size_t)b * g.H + h) * g.K + row) * g.K + p0 + 32 * ng, S);
+    } else if (!last_walk) {
+      // the next walk does not need it
     } else if (ce < g.NC) {
       store32(carry, S);
     } else if (a.final_state && native) {
@@ -405,7 +454,7 @@ __global__ void __launch_bounds__(Plan<VS, false>::NT, 1) state_fwd_tc_kernel(co
       uint8_t* dst = reinterpret_cast<uint8_t*>(a.states);
       for (int i = 0; i < n && !wait.dead; ++i) {
         wait(&s_ready, i & 1);
-        umma::bulk_store(dst + ((item0 + i) * Vw + v0) * 256, sS, PL::SL);
+        if (!CUT || i >= warm) umma::bulk_store(dst + ((item0 + i) * Vw + v0) * 256, sS, PL::SL);
         umma::bulk_commit();
         umma::bulk_wait_read<0>();
         arrive(&s_free);
@@ -417,7 +466,7 @@ __global__ void __launch_bounds__(Plan<VS, false>::NT, 1) state_fwd_tc_kernel(co
   if (warp == 0) umma::tmem_dealloc(tmem_base, PL::TMEM);
 }
 
-template <int VS>
+template <int VS, bool CUT>
 __global__ void __launch_bounds__(Plan<VS, true>::NT, 1) state_bwd_tc_kernel(const __grid_constant__ StateArgs a) {
   using PL = Plan<VS, true>;
   constexpr int ST = PL::ST, NG = PL::NG, SLOTS = PL::SLOTS, DB = PL::DO_BUF, ROWS = PL::ROWS;
@@ -428,7 +477,7 @@ __global__ void __launch_bounds__(Plan<VS, true>::NT, 1) state_bwd_tc_kernel(con
   __shared__ int stop_s;
   const Geo& g = a.g;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // (warp: uniform for the compiler)
-  const int Vw = g.Vw, vr = g.G * g.V, v0 = blockIdx.x * VS, h = blockIdx.y, b = blockIdx.z;
+  const int Vw = g.Vw, vr = g.G * g.V, v0 = blockIdx.x * VS, h = blockIdx.y, b = CUT ? blockIdx.z % g.B : blockIdx.z;
   uint8_t* tiles = sm;
   uint8_t* sdO = sm + SLOTS * TILE_B;                   // DB buffers
   uint8_t* sdH = sdO + DB * PL::SL;
@@ -436,8 +485,10 @@ __global__ void __launch_bounds__(Plan<VS, true>::NT, 1) state_bwd_tc_kernel(con
   uint8_t* sR = sdV + PL::SL;                           // rows of S, ROWS buffers
   float* lam_s = reinterpret_cast<float*>(sR + ROWS * PL::SL);
   float* part_s = lam_s + ROWS * 128;                   // partial sums of dLambda_end: NG x 128
-  const int ce = a.c_end;
-  int cb = a.c_begin;
+  int cb = a.c_begin, ce = a.c_end, warm = 0;
+  __shared__ int found_s[2];
+  if (CUT && !find_walk<true, PL::NT>(a, b, blockIdx.z / g.B, found_s, cb, ce, warm)) return;
+  const bool first_walk = !CUT || ce == a.c_end, last_walk = !CUT || cb == a.c_begin;
   if (tid == 0) {
     for (int i = 0; i < SLOTS; ++i) { umma::mbar_init(&full[i], 1); umma::mbar_init(&empty[i], 1); }
     for (int i = 0; i < ROWS; ++i) { umma::mbar_init(&row_full[i], 1); umma::mbar_init(&row_empty[i], 1); }
@@ -479,7 +530,8 @@ __global__ void __launch_bounds__(Plan<VS, true>::NT, 1) state_bwd_tc_kernel(con
     float dH[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) dH[j] = 0.f;
-    if (ce < g.NC) load32(carry, dH);
+    if (!first_walk) { /* zeros */ }
+    else if (ce < g.NC) load32(carry, dH);
     else if (a.d_final && native) load32(a.d_final + noff, dH);
     Flags fl;
     fl.fill(a.seg, g, b, ce - 1, -1, cb, ce);
@@ -545,6 +597,8 @@ __global__ void __launch_bounds__(Plan<VS, true>::NT, 1) state_bwd_tc_kernel(con
     umma::tc_fence_before();
     if (a.until_independent) {
       // nothing to hand on: the caller has d_init from the shard's affine summary
+    } else if (!last_walk) {
+      // the next walk does not need it
     } else if (cb > 0) {
       store32(carry, dH);
     } else if (a.d_init && native) {
@@ -637,13 +691,15 @@ __global__ void __launch_bounds__(Plan<VS, true>::NT, 1) state_bwd_tc_kernel(con
       float* parts = dlend_part(g, a.dV);
       for (int i = 0; i < n && !wait.dead; ++i) {
         wait(&h_ready, i & 1);
-        umma::bulk_store(reinterpret_cast<uint8_t*>(a.dH) + ((last - i) * Vw + v0) * 256, sdH, PL::SL);
+        if (!CUT || i >= warm) umma::bulk_store(reinterpret_cast<uint8_t*>(a.dH) + ((last - i) * Vw + v0) * 256, sdH, PL::SL);
         umma::bulk_commit();
         umma::bulk_wait_read<0>();
         arrive(&h_free);
         wait(&v_ready, i & 1);
-        umma::bulk_store(reinterpret_cast<uint8_t*>(a.dV) + ((last - i) * Vw + v0) * 256, sdV, PL::SL);
-        umma::bulk_store(parts + ((last - i) * (Vw / 32) + v0 / 32) * KT, part_s, NG * 512);
+        if (!CUT || i >= warm) {
+          umma::bulk_store(reinterpret_cast<uint8_t*>(a.dV) + ((last - i) * Vw + v0) * 256, sdV, PL::SL);
+          umma::bulk_store(parts + ((last - i) * (Vw / 32) + v0 / 32) * KT, part_s, NG * 512);
+        }
         umma::bulk_commit();
         umma::bulk_wait_read<0>();
         arrive(&v_free);
@@ -655,31 +711,44 @@ __global__ void __launch_bounds__(Plan<VS, true>::NT, 1) state_bwd_tc_kernel(con
   if (warp == 0) umma::tmem_dealloc(tmem_base, PL::TMEM);
 }
 
+// Parts to cut the range into (find_walk): four times as many walks as SMs, where documents are given and one walk per column
+// slice leaves half of the chip idle.  A part is 4 chunks at least and the range 24, because a walk costs about two steps more than
+// its chunks.  32 heads, 1024 chunks in 8 documents: forward 2361 us -> 1185, with entry states 1587 -> 1185, reverse 2243 -> 1725;
+// 24 heads, 47 chunks in documents of 8 on average: forward 117 -> 75, reverse 105 -> 82; over 12 chunks it loses (51 -> 56).
+// (Twice the SMs: 73 and 81, but 2194 for the reverse above: documents that share a part are one walk.)
+int pick_parts(const StateArgs& a) {
+  const int ctas = a.g.B * a.g.H * (a.g.Vw / 64), chunks = a.c_end - a.c_begin;
+  if (!a.seg || a.P_out || a.until_independent || a.skip_provisional || ctas * 2 > sm_count() || chunks < 24) return 1;
+  const int want = 4 * sm_count() / ctas, most = chunks / 4;
+  return want < most ? want : most;
+}
+
 // Columns of the value width per CTA, 32 or 64.  What bounds a chunk step is shared memory: the products read their
 // operands at its full width (46 cycles per 128 x 32 x 16 MMA, 48 at 64 columns, 64 at 128: the tile, 4 KB of each, dominates),
 // the four tiles are written to it, and loads and stores of the threads wait their turn.  64 columns read the tiles half as
 // often and leave the step 2.0 us as against 1.9 (forward, storing entry states), 2.2 as against 3.2 (reverse); at 128 it was 4.4.
-// So: 64, except for forward passes that store entry states and fit the SMs at 32 (fused prologue L=6001, 96 CTAs:
+// So: 64, except for uncut forward passes that store entry states and fit the SMs at 32 (fused prologue L=6001, 96 CTAs:
 // 117 us against 139; the KDA pass over 131072 tokens with one launch of each kind: 3.92 ms against 4.18).
 int pick_vs_fwd(const StateArgs& a) {
   if (a.P_out) return 64;                               // Vw + K columns of 32 heads in few enough CTAs for one wave
   return a.states && a.g.B * a.g.H * (a.g.Vw / 32) <= sm_count() ? 32 : 64;
 }
 
-template <int VS>
-int launch_fwd_vs(const StateArgs& a, cudaStream_t st) {
+
+template <int VS, bool CUT>
+int launch_fwd(const StateArgs& a, cudaStream_t st) {
   using PL = Plan<VS, false>;
-  const dim3 grid((a.g.Vw + (a.P_out ? a.g.K : 0)) / VS, a.g.H, a.g.B);
-  cudaFuncSetAttribute(state_fwd_tc_kernel<VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL::SMEM);
-  state_fwd_tc_kernel<VS><<<grid, PL::NT, PL::SMEM, st>>>(a);
+  const dim3 grid((a.g.Vw + (a.P_out ? a.g.K : 0)) / VS, a.g.H, a.g.B * a.parts);
+  cudaFuncSetAttribute(state_fwd_tc_kernel<VS, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL::SMEM);
+  state_fwd_tc_kernel<VS, CUT><<<grid, PL::NT, PL::SMEM, st>>>(a);
   return launch_status();
 }
-template <int VS>
-int launch_bwd_vs(const StateArgs& a, cudaStream_t st) {
+template <int VS, bool CUT>
+int launch_bwd(const StateArgs& a, cudaStream_t st) {
   using PL = Plan<VS, true>;
-  const dim3 grid(a.g.Vw / VS, a.g.H, a.g.B);
-  cudaFuncSetAttribute(state_bwd_tc_kernel<VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL::SMEM);
-  state_bwd_tc_kernel<VS><<<grid, PL::NT, PL::SMEM, st>>>(a);
+  const dim3 grid(a.g.Vw / VS, a.g.H, a.g.B * a.parts);
+  cudaFuncSetAttribute(state_bwd_tc_kernel<VS, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL::SMEM);
+  state_bwd_tc_kernel<VS, CUT><<<grid, PL::NT, PL::SMEM, st>>>(a);
   return launch_status();
 }
 
@@ -687,6 +756,7 @@ StateArgs with_range(const StateArgs& in) {
   StateArgs a = in;
   if (a.c_end <= 0) { a.c_begin = 0; a.c_end = a.g.NC; }
   a.err = device_error_ptr();
+  a.parts = pick_parts(a);
   return a;
 }
 
@@ -696,12 +766,13 @@ bool state_tc_eligible(const Geo& g) { return g.img; }
 
 int launch_state_fwd_tc(const StateArgs& in, cudaStream_t st) {
   const StateArgs a = with_range(in);
-  return pick_vs_fwd(a) == 64 ? launch_fwd_vs<64>(a, st) : launch_fwd_vs<32>(a, st);
+  if (a.parts > 1) return launch_fwd<64, true>(a, st);
+  return pick_vs_fwd(a) == 64 ? launch_fwd<64, false>(a, st) : launch_fwd<32, false>(a, st);
 }
 
 int launch_state_bwd_tc(const StateArgs& in, cudaStream_t st) {
   const StateArgs a = with_range(in);
-  return launch_bwd_vs<64>(a, st);
+  return a.parts > 1 ? launch_bwd<64, true>(a, st) : launch_bwd<64, false>(a, st);
 }
 
 }  // namespace dn

@@ -68,6 +68,19 @@ def test_shared_key_heads(dn, B, L):
     compare(lambda t, i: dn.chunk_gdn(*t, **kw), lambda t, i: O.chunk_gdn(*t, **kw), [q, k, v, g, beta], tol=BF16_TOL)
 
 
+# ---- chains cut at document boundaries: inside a chunk, at its start, several in one part, in the last chunk, none at all
+@pytest.mark.parametrize("recompute", [False, True])
+def test_chains_cut_at_documents(dn, recompute):
+    B, L, Hk, Hv = 2, 26 * 128 + 5, 1, 2
+    ins = list(O.make_inputs(55, B, L, Hk, Hv, 64, 64, qkv_dtype=torch.bfloat16)[:6])
+    init = torch.randn(B, Hv, 64, 64, generator=torch.Generator().manual_seed(56)) * 0.1
+    seg = docs(B, L, 5 * 128, 7 * 128 + 1, 8 * 128 - 1, 8 * 128, 13 * 128 + 70, 13 * 128 + 90, 20 * 128 - 1, 26 * 128, 26 * 128 + 3)
+    seg[1] = 0
+    kw = dict(chunk_size=128, precision="bf16", qk_l2norm=True, output_final_state=True)
+    compare(lambda t, i: dn.chunk_gdn2(*t, segment_ids=seg.cuda(), initial_state=i, recompute_states=recompute, **kw),
+            lambda t, i: O.chunk_gdn2(*t, segment_ids=seg, initial_state=i, **kw), ins, tol=BF16_TOL, init=init)
+
+
 # ---- segment ids in blocks: a run of equal ids may cross any number of them
 @pytest.mark.parametrize("L", [1, 255, 1024, 1025, 20011])
 def test_canonical_segments(dn, L):
