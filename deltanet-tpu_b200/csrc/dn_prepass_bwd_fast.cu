@@ -208,43 +208,60 @@ __device__ __forceinline__ void stage_dO(uint4* dst, const void* d_out, size_t o
   umma::cp_async_commit();
 }
 
-// dv = dY w_act, dw = dY v (+ sigmoid adjoint; summed over a value head's columns when w is one scalar per head) of 128
-// columns, dY from its image.  The rows of v are requested together where w is one scalar,
-// those of v and w one step ahead otherwise (less code).
-template <int MODE, bool SC>
-__device__ __noinline__ void v_phase_call(const PrepassBwdArgs& a, const uint4* img, int half, int h, size_t tok0, int rows, int wC) {
-  using CF = InCfg<MODE>;
+// 16 bytes of an input tensor, issued where it stands: an ordinary load may be moved down to its use, past the branches between
+__device__ __forceinline__ uint4 ld16_now(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+template <bool BF>
+struct Piece {                                          // eight elements as loaded
+  uint4 a[BF ? 1 : 2];
+  __device__ __forceinline__ void load(const void* base, size_t off) {
+    const uint4* p = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(base) + off * (BF ? 2 : 4));
+    a[0] = ld16_now(p);
+    if (!BF) a[BF ? 0 : 1] = ld16_now(p + 1);
+  }
+  __device__ __forceinline__ void get(float (&x)[8]) const {
+    if (BF) umma::unpack8(a[0], x);
+    else {
+      const uint4 b = a[BF ? 0 : 1];
+      x[0] = __uint_as_float(a[0].x); x[1] = __uint_as_float(a[0].y); x[2] = __uint_as_float(a[0].z); x[3] = __uint_as_float(a[0].w);
+      x[4] = __uint_as_float(b.x); x[5] = __uint_as_float(b.y); x[6] = __uint_as_float(b.z); x[7] = __uint_as_float(b.w);
+    }
+  }
+};
+// dv = dY w_act, dw = dY v (+ sigmoid adjoint; summed over a value head's columns when w is one scalar per head, SW) of 128
+// columns, dY from its image.  Bound by the latency of the rows of v and w (2.2 to 3.2 k cycles with every SM here at once), so
+// all of them are requested together; one function per type, because only code that runs takes instruction cache.
+template <bool QBF, bool GBF, bool SW>
+__device__ __noinline__ void v_phase(const PrepassBwdArgs& a, const uint4* img, int half, int h, size_t tok0, int rows, bool fuse) {
   const Geo& g = a.g;
-  const int rx = threadIdx.x >> 2, rp = threadIdx.x & 3, vr = g.G * g.V;
-  const int qdt = SC || MODE != 2 ? (SC ? DN_BF16 : CF::qkv_dt) : g.qkv_dt, gdt = CF::fixed ? DN_F32 : g.gate_dt;
-  const uint32_t qes = qdt == DN_BF16 ? 2 : 4, ges = gdt == DN_BF16 ? 2 : 4;
-  const bool fuse = CF::fixed || SC ? false : (g.flags & DN_FUSE_PROLOGUE) != 0;
+  const int rx = threadIdx.x >> 2, rp = threadIdx.x & 3, vr = g.G * g.V, vsh = g.V == 128 ? 7 : 6;
   const bool live = rx < rows;
   const size_t tok = tok0 + (live ? rx : 0);
-  constexpr int VB = SC || CF::scalar_bw ? 4 : 1;
-  Raw8 vraw[VB], wraw[VB];
-  auto load = [&](int col, Raw8& vraw, Raw8& wraw) {
-    const int cc = col < vr ? col : 0, hv = h * g.G + cc / g.V, cv = cc % g.V;
-    vraw = ldraw(reinterpret_cast<const uint8_t*>(a.v) + ((tok * g.Hv + hv) * g.V + cv) * qes, 0, qdt);
-    if (wC == 1) wraw.a.x = __float_as_uint(ldf_ro(a.w, tok * g.wH + g.w_head(hv), gdt));
-    else wraw = ldraw(reinterpret_cast<const uint8_t*>(a.w) + ((tok * g.wH + g.w_head(hv)) * wC + cv) * ges, 0, gdt);
-  };
-  const int steps_per_head = g.V / 32;
+  Piece<QBF> vraw[4];
+  Piece<GBF> wraw[4];
+  float ws[4];
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int col = half * 128 + 32 * it + 8 * rp, cc = col < vr ? col : 0, hv = h * g.G + (cc >> vsh), cv = cc & (g.V - 1);
+    vraw[it].load(a.v, (tok * g.Hv + hv) * g.V + cv);
+    if (SW) ws[it] = ldf_ro(a.w, tok * g.wH + g.w_head(hv), GBF ? DN_BF16 : DN_F32);
+    else wraw[it].load(a.w, (tok * g.wH + g.w_head(hv)) * g.V + cv);
+  }
   float sw = 0.f;
 #pragma unroll
-  for (int i = 0; i < VB; ++i) load(half * 128 + 32 * i + 8 * rp, vraw[i], wraw[i]);
-#pragma unroll (VB)
   for (int it = 0; it < 4; ++it) {
     const int p = it * 4 + rp, col = half * 128 + 8 * p;
     if (col - 8 * rp >= vr) break;                      // (uniform: value widths are multiples of 32)
-    const int hv = h * g.G + col / g.V, cv = col % g.V;
+    const int hv = h * g.G + (col >> vsh), cv = col & (g.V - 1);
     float vv[8], ww[8], dy[8], dv8[8], dw8[8];
-    cvraw(vraw[it % VB], qdt, vv);
-    if (wC == 1) {
+    vraw[it].get(vv);
+    if (SW) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) ww[i] = __uint_as_float(wraw[it % VB].a.x);
-    } else cvraw(wraw[it % VB], gdt, ww);
-    if (VB == 1 && it < 3) load(col + 32, vraw[0], wraw[0]);
+      for (int i = 0; i < 8; ++i) ww[i] = ws[it];
+    } else wraw[it].get(ww);
     umma::unpack8(img[p * PP + rx], dy);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -255,10 +272,10 @@ __device__ __noinline__ void v_phase_call(const PrepassBwdArgs& a, const uint4* 
       sw += dwv;
     }
     if (live) {
-      strow8(a.dv, (tok * g.Hv + hv) * g.V + cv, qdt, dv8);
-      if (wC != 1) strow8(a.dw, (tok * g.Hv + hv) * wC + cv, a.dw_dt, dw8);
+      strow8(a.dv, (tok * g.Hv + hv) * g.V + cv, QBF ? DN_BF16 : DN_F32, dv8);
+      if (!SW) strow8(a.dw, (tok * g.Hv + hv) * g.V + cv, a.dw_dt, dw8);
     }
-    if (wC == 1 && (it + 1) % steps_per_head == 0) {
+    if (SW && ((col + 32) & (g.V - 1)) < 32) {          // the head's last step
       sw += __shfl_xor_sync(0xffffffffu, sw, 1);
       sw += __shfl_xor_sync(0xffffffffu, sw, 2);
       if (live && rp == 0) stf(a.dw, tok * g.Hv + hv, sw, a.dw_dt);
@@ -480,7 +497,20 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       drain_plain(cx.dead, tb + T_B, sl.at(slot), 128, row, group, 1.f);
     };
     auto drain_dY = [&](int slot) { drain_plain(cx.dead, tb + T_TMP, sl.at(slot), PP, row, group, 1.f); };
-    auto vphase = [&](int slot, int half) { v_phase_call<MODE, SC>(a, sl.at(slot), half, h, tok0, rows, wC); };
+    auto vphase = [&](int slot, int half) {
+      auto go = [&](auto qbf, auto gbf, auto scalar) {
+        v_phase<decltype(qbf)::value, decltype(gbf)::value, decltype(scalar)::value>(a, sl.at(slot), half, h, tok0, rows, fuse);
+      };
+      constexpr std::true_type yes{};
+      constexpr std::false_type no{};
+      if (qdt == DN_BF16) {
+        if (gdt == DN_BF16) { if (wC == 1) go(yes, yes, yes); else go(yes, yes, no); }
+        else { if (wC == 1) go(yes, no, yes); else go(yes, no, no); }
+      } else {
+        if (gdt == DN_BF16) { if (wC == 1) go(no, yes, yes); else go(no, yes, no); }
+        else { if (wC == 1) go(no, no, yes); else go(no, no, no); }
+      }
+    };
     if constexpr (NH == 1) {
       drain_dX(0);
       drain_dY(1);
