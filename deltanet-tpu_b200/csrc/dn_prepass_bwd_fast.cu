@@ -82,21 +82,24 @@ __device__ __forceinline__ void finish(umma::Ctx& cx) {       // waits for what 
   cx.dead = cta_wait_call(cx.bar, cx.phase, cx.err, cx.dead);
   cx.phase ^= 1u;
 }
-__device__ __noinline__ void slot_load_call(void* dst, const void* src, uint64_t* bar) {
-  if (threadIdx.x == 0) {
+__device__ __noinline__ void slot_load_call(void* dst, const void* src, uint64_t* bar, int who) {
+  if ((int)threadIdx.x == who) {
     umma::fence_async_smem();
     umma::mbar_expect_tx(bar, IMGB);
     umma::bulk_load(dst, src, IMGB, bar);
   }
 }
+// Slots 0, 1 and 2 (W, S and U at the start of a tile) lie where the raw k, q and b were, which are done with before the decay
+// gradient is: they are loaded for the next tile while that runs.
 struct Slots {
   uint8_t* sm;
   uint64_t* bars;          // one per slot
   uint32_t phases;
   int* err;
-  __device__ __forceinline__ uint4* at(int s) const { return reinterpret_cast<uint4*>(sm + s * SLOT); }
+  __device__ __forceinline__ uint4* region(int p) const { return reinterpret_cast<uint4*>(sm + (p < 2 ? p * SLOT : OFF_GI + (p - 2) * SLOT)); }
+  __device__ __forceinline__ uint4* at(int s) const { return region(s < 3 ? s + 2 : s < 5 ? s - 3 : 5); }
   // one contiguous 32 KB operand image; ordinary accesses to the slot must lie before a barrier
-  __device__ __forceinline__ void load(int s, const __nv_bfloat16* src) { slot_load_call(at(s), src, bars + s); }
+  __device__ __forceinline__ void load(int s, const __nv_bfloat16* src, int who = 0) { slot_load_call(at(s), src, bars + s, who); }
   __device__ __forceinline__ void wait(int s) {
     bar_wait_call(bars + s, (phases >> s) & 1u, err);
     phases ^= 1u << s;
@@ -293,6 +296,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
   __shared__ uint32_t tmem_base;
   __shared__ int seg_s[C];
   __shared__ int cut_s[8];
+  __shared__ int next_strong_s;
   __shared__ uint8_t ds_s[C], de_s[C];                  // first / last row of each row's document inside the tile
   __shared__ float rq_s[C], rk_s[C], dmi_s[C], dlend_s[C];
   __shared__ float lam_s[C], bet_s[C];                  // scalar gates
@@ -331,17 +335,28 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
   // A CTA takes the D heads that share a key head one after the other and adds up their dq and dk in its scratch (see
   // prepass_bwd_grouped); otherwise D = 1.
   const int D = SC ? a.group : 1, HG = g.H / D;
-  for (int e_item = blockIdx.x; e_item < a.items / D; e_item += gridDim.x)
-  for (int hd = 0; hd < D; ++hd) {
+  auto tile_of = [&](int e, int hd) {
+    const int bg = e % (g.B * HG), b = bg / HG, h = (bg - b * HG) * D + hd;
+    return (size_t)(b * g.H + h) * g.NC + a.c_begin + e / (g.B * HG);
+  };
+  const __nv_bfloat16* states = states_img(g, a.res.states);
+  auto load_first = [&](size_t ib, int who) {           // what the first product and its drain take
+    sl.load(0, reinterpret_cast<const __nv_bfloat16*>(a.res.W) + ib * C * K, who);
+    sl.load(1, states + ib * K * VW, who);
+    sl.load(2, reinterpret_cast<const __nv_bfloat16*>(a.res.U) + ib * C * VW, who);
+  };
+  bool loaded = false;                                  // load_first has been done during the tile before
+  for (int e_item = blockIdx.x, hd = 0; e_item < a.items / D; (hd = hd + 1 < D ? hd + 1 : 0) == 0 ? e_item += gridDim.x : 0) {
     const int bg = e_item % (g.B * HG), c_idx = a.c_begin + e_item / (g.B * HG);
     const int b = bg / HG, h = (bg - b * HG) * D + hd, t0 = c_idx * C;
     const size_t ibase = (size_t)(b * g.H + h) * g.NC + c_idx;
-    if (!SC && strong_flag(a.res, ibase)) continue;     // uniform over the CTA
+    if (!SC && !loaded && strong_flag(a.res, ibase)) continue;              // uniform over the CTA
+    if (!loaded) load_first(ibase, 0);
     const int rows = g.L - t0 < C ? g.L - t0 : C;
     const size_t tok0 = (size_t)b * g.L + t0;
     const __nv_bfloat16* Wg = reinterpret_cast<const __nv_bfloat16*>(a.res.W) + ibase * C * K;
     const __nv_bfloat16* Ug = reinterpret_cast<const __nv_bfloat16*>(a.res.U) + ibase * C * VW;
-    const __nv_bfloat16* Sg = states_img(g, a.res.states) + ibase * K * VW;
+    const __nv_bfloat16* Sg = states + ibase * K * VW;
     const __nv_bfloat16* dHg = reinterpret_cast<const __nv_bfloat16*>(a.dH) + ibase * K * VW;
     const __nv_bfloat16* dVg = reinterpret_cast<const __nv_bfloat16*>(a.dV) + ibase * C * VW;
     const __nv_bfloat16* Tg = reinterpret_cast<const __nv_bfloat16*>(a.res.T + ibase * C * C);
@@ -349,9 +364,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     constexpr int HN = C * 128;                         // elements of one half's image
 
     // ---- products over the value width
-    sl.load(0, Wg);
-    sl.load(1, Sg);
-    sl.load(2, Ug);
     if (NH == 1) {
       sl.load(3, dVg);
       sl.load(4, dHg);
@@ -361,24 +373,37 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       sl.load(4, Ug + HN);
       stage_dO(sl.at(5), a.d_out, dO_off, dO_pitch, rows, 16, qdt);
     }
-    bool is_new, all_same;
-    chunk_flags(a.seg, g, b, c_idx, is_new, all_same);
-    if (tid < C) {
-      const int sg = seg_at(a.seg, b, t0 + tid, g.L);
-      seg_s[tid] = sg;
-      rq_s[tid] = __ldg(tile_extra(a.res, ibase) + 128 + tid);
-      rk_s[tid] = __ldg(tile_extra(a.res, ibase) + 256 + tid);
+    // V_new = U - W S, in the place of U; dM masked (scalar gates: decayed), its diagonal apart
+    auto vnew = [&](int slot, uint32_t col) { drain_sub(cx.dead, tb + col, sl.at(slot), row, group); };
+    auto drain_dM = [&](int slot) { drain_masked(cx.dead, tb + T_TMP, sl.at(slot), row, group, 1.f, seg_s, SC ? lam_s : nullptr, dmi_s); };
+    auto drain_neg = [&](int slot, uint32_t col) { drain_plain(cx.dead, tb + col, sl.at(slot), 128, row, group, -1.f); };
+    sl.wait(0);
+    sl.wait(1);
+    umma::tc_fence_after();
+    product<128, false, true>(cx, sl.at(0), 2048, sl.at(1), 2048, K, T_TMP, false);                        // W S
+    // (beside the first product, which warp 0 issues)
+    if (const int x = tid - 256; x >= 0 && x < C) {
+      bool is_new, all_same;
+      chunk_flags(a.seg, g, b, c_idx, is_new, all_same);
+      const int sg = seg_at(a.seg, b, t0 + x, g.L);
+      seg_s[x] = sg;
+      rq_s[x] = __ldg(tile_extra(a.res, ibase) + 128 + x);
+      rk_s[x] = __ldg(tile_extra(a.res, ibase) + 256 + x);
       // dLambda_end = [one document] e^{Lambda_end} sum_v dH S (gdn2.py:759-762) from the reverse chain's per-slice sums
       float acc = 0.f;
-      const float* part = dlend_part(g, const_cast<float*>(a.dV)) + ibase * (VW / 32) * K + tid;
+      const float* part = dlend_part(g, const_cast<float*>(a.dV)) + ibase * (VW / 32) * K + x;
       for (int s2 = 0; s2 < VW / 32; ++s2) acc += __ldg(part + s2 * K);
-      dlend_s[tid] = all_same ? acc * expf(fminf(__ldg(a.res.lam_end + ibase * K + tid), 0.f)) : 0.f;
+      dlend_s[x] = all_same ? acc * expf(fminf(__ldg(a.res.lam_end + ibase * K + x), 0.f)) : 0.f;
+      if (!SC && x == 0) {                              // does the next tile belong to the other kernel?
+        const int ne = e_item + (int)gridDim.x;
+        next_strong_s = ne >= a.items || strong_flag(a.res, tile_of(ne, 0));
+      }
       if (SC) {                                         // decay and erase gate: one row per thread, document-restarting scan
-        const int sp = tid ? seg_at(a.seg, b, t0 + tid - 1, g.L) : sg;
+        const int sp = x ? seg_at(a.seg, b, t0 + x - 1, g.L) : sg;
         float gv = 0.f, bv = 0.f;
-        if (tid < rows) {
-          gv = ldf_ro(a.gg, (tok0 + tid) * g.gH + g.gate_head(h, g.gH), g.gate_dt);
-          bv = ldf_ro(a.b, (tok0 + tid) * g.bH + g.gate_head(h, g.bH), g.gate_dt);
+        if (x < rows) {
+          gv = ldf_ro(a.gg, (tok0 + x) * g.gH + g.gate_head(h, g.gH), g.gate_dt);
+          bv = ldf_ro(a.b, (tok0 + x) * g.bH + g.gate_head(h, g.bH), g.gate_dt);
           gv = gv <= 0.f ? gv : 0.f;
           if (guard) { bv = fmaxf(bv, 0.f); gv = fminf(gv, -1e-6f); }
         }
@@ -389,27 +414,23 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
           const bool uc = __shfl_up_sync(0xffffffffu, (int)cut, o);
           if (lane >= o) { if (!cut) gv += up; cut |= uc; }
         }
-        if (lane == 31) { SUM[warp] = gv; cut_s[warp] = cut; }
+        if (lane == 31) { SUM[warp - 8] = gv; cut_s[warp - 8] = cut; }
         asm volatile("bar.sync 1, 128;" ::: "memory");
         float carry = 0.f;
-        for (int w2 = warp - 1; w2 >= 0; --w2) { carry += SUM[w2]; if (cut_s[w2]) break; }
-        lam_s[tid] = gv + (cut ? 0.f : carry);
-        bet_s[tid] = bv;
+        for (int w2 = warp - 9; w2 >= 0; --w2) { carry += SUM[w2]; if (cut_s[w2]) break; }
+        lam_s[x] = gv + (cut ? 0.f : carry);
+        bet_s[x] = bv;
       }
     }
-    // V_new = U - W S, in the place of U; dM masked (scalar gates: decayed), its diagonal apart
-    auto vnew = [&](int slot, uint32_t col) { drain_sub(cx.dead, tb + col, sl.at(slot), row, group); };
-    auto drain_dM = [&](int slot) { drain_masked(cx.dead, tb + T_TMP, sl.at(slot), row, group, 1.f, seg_s, SC ? lam_s : nullptr, dmi_s); };
-    auto drain_neg = [&](int slot, uint32_t col) { drain_plain(cx.dead, tb + col, sl.at(slot), 128, row, group, -1.f); };
-    sl.wait(0);
-    sl.wait(1);
+    if (NH == 2) {
+      sl.wait(3);
+      product<128, false, true>(cx, sl.at(0), 2048, sl.at(3), 2048, K, T_B, false);
+    }
+    commit(cx);
     sl.wait(2);
+    umma::cp_async_wait<0>();                           // dO
+    finish(cx);
     if constexpr (NH == 1) {
-      umma::pre_issue_sync();
-      product<128, false, true>(cx, sl.at(0), 2048, sl.at(1), 2048, K, T_TMP, false);                      // W S
-      commit(cx);
-      umma::cp_async_wait<0>();                         // dO
-      finish(cx);
       sl.load(0, Tg);
       vnew(2, T_TMP);
       sl.wait(3);
@@ -434,15 +455,8 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       commit(cx);
       finish(cx);
     } else {
-      sl.wait(3);
-      sl.wait(4);
-      umma::pre_issue_sync();
-      product<128, false, true>(cx, sl.at(0), 2048, sl.at(1), 2048, K, T_TMP, false);                      // W S, both halves
-      product<128, false, true>(cx, sl.at(0), 2048, sl.at(3), 2048, K, T_B, false);
-      commit(cx);
-      umma::cp_async_wait<0>();
-      finish(cx);
       sl.load(0, dVg);
+      sl.wait(4);
       vnew(2, T_TMP);
       vnew(4, T_B);
       umma::pre_issue_sync();
@@ -549,8 +563,9 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       vphase(4, 1);
       finish(cx);
     }
-    // ---- dA into slot 4 (dM is in slot 5); slots 0 .. 3 are free
-    drain_masked(cx.dead, tb + T_TMP, sl.at(4), row, group, -1.f, seg_s, SC ? lam_s : nullptr, nullptr);
+    // ---- dA (dM is in slot 5); everything else is free
+    uint4 *const dAi = sl.region(4), *const dMi = sl.at(5);
+    drain_masked(cx.dead, tb + T_TMP, dAi, row, group, -1.f, seg_s, SC ? lam_s : nullptr, nullptr);
 
     // ---- key side: rows of q, k, b in the row mapping
     const bool live = rx < rows;
@@ -720,7 +735,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     }
     // ---- T1, T2, T3 on top of them
     if constexpr (SC) {
-      uint4 *KI = sl.at(0), *QI = sl.at(1), *BI = sl.at(2);
+      uint4 *KI = sl.region(0), *QI = sl.region(1), *BI = sl.region(2);
 #pragma unroll 2
       for (int it = 0; it < 4; ++it) {
         const int p = it * 4 + rp;
@@ -732,10 +747,10 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         BI[p * PP + rx] = umma::pack8(be);
       }
       umma::pre_issue_sync();
-      product<128, false, true>(cx, sl.at(4), 2048, KI, PB, C, T_B, true);       // (dA f)   k_hat
-      product<128, false, true>(cx, sl.at(5), 2048, KI, PB, C, T_Q, true);       // (dM f)   k_hat
-      product<128, true, true>(cx, sl.at(4), 2048, BI, PB, C, T_K, true);        // (dA f)^T (b k_hat)
-      product<128, true, true>(cx, sl.at(5), 2048, QI, PB, C, T_K, true);        // (dM f)^T q_hat
+      product<128, false, true>(cx, dAi, 2048, KI, PB, C, T_B, true);       // (dA f)   k_hat
+      product<128, false, true>(cx, dMi, 2048, KI, PB, C, T_Q, true);       // (dM f)   k_hat
+      product<128, true, true>(cx, dAi, 2048, BI, PB, C, T_K, true);        // (dA f)^T (b k_hat)
+      product<128, true, true>(cx, dMi, 2048, QI, PB, C, T_K, true);        // (dM f)^T q_hat
       commit(cx);
       finish(cx);
     } else {
@@ -776,10 +791,10 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
           BF[o] = umma::pack8(be);
         }
         umma::pre_issue_sync();
-        product<64, false, true>(cx, sl.at(4), 2048, KF, PB, C, T_B + 64 * rnd, true);       // dA (k / f)
-        product<64, false, true>(cx, sl.at(5), 2048, KF, PB, C, T_Q + 64 * rnd, true);       // dM (k / f)
-        product<64, true, true>(cx, sl.at(4), 2048, BF, PB, C, T_K + 64 * rnd, true);        // dA^T (beta f)
-        product<64, true, true>(cx, sl.at(5), 2048, QF, PB, C, T_K + 64 * rnd, true);        // dM^T (q f)
+        product<64, false, true>(cx, dAi, 2048, KF, PB, C, T_B + 64 * rnd, true);       // dA (k / f)
+        product<64, false, true>(cx, dMi, 2048, KF, PB, C, T_Q + 64 * rnd, true);       // dM (k / f)
+        product<64, true, true>(cx, dAi, 2048, BF, PB, C, T_K + 64 * rnd, true);        // dA^T (beta f)
+        product<64, true, true>(cx, dMi, 2048, QF, PB, C, T_K + 64 * rnd, true);        // dM^T (q f)
         commit(cx);
       }
       finish(cx);
@@ -1006,7 +1021,13 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       }
       return (guard ? graw < -1e-6f : graw <= 0.f) ? d : 0.f;               // through min(min(g, 0), -1e-6)
     };
+    // the next tile's first operands, where the raw rows were (asked for by a warp that has little left to do)
+    const int ne = hd + 1 < D ? e_item : e_item + (int)gridDim.x;
+    loaded = ne < a.items / D && (SC || next_strong_s == 0);
+    auto load_next = [&] { if (loaded) load_first(tile_of(ne, hd + 1 < D ? hd + 1 : 0), 480); };
     if constexpr (SC) {
+      __syncthreads();
+      load_next();
       if (tid < C) {
         float v = (SUM[1536 + tid] + SUM[1664 + tid]) + (SUM[1792 + tid] + SUM[1920 + tid]);
         bool cut = tid < C - 1 && seg_s[tid] != seg_s[tid + 1];             // a document ends behind this row
@@ -1047,6 +1068,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       TOT[qd * 128 + c] = run;
       if (c == 0) cut_s[4 + qd] = ends != 0;
       __syncthreads();
+      load_next();
       float carry = 0.f;
       if (!(ends >> 31))                                // (the last row's own end cuts the quarter off from what follows)
         for (int q2 = qd + 1; q2 < 4; ++q2) { carry += TOT[q2 * 128 + c]; if (cut_s[4 + q2]) break; }
