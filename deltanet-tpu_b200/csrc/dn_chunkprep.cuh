@@ -1,4 +1,4 @@
-// Per-chunk preparation shared by the tensor-core prepass kernels (chunk = K = 128):
+// Per-chunk preparation shared by the tensor-core prepass kernels (128-row tiles, channels padded to 128):
 // activated and normalised rows of q, k, b, g read straight from the user's tensors in
 // 8-element pieces, the cumulative log-decay in shared memory, and the bf16 operand images of
 // one level of the hierarchical A/M factorisation.
@@ -17,21 +17,18 @@ constexpr int LP = 132;                // row pitch (floats) of the shared-memor
 // What a kernel instantiation knows about its inputs at compile time.  MODE 0: q/k/v in bf16, gates
 // in fp32 and already activated (no fused prologue), every gate with one value per channel; MODE 1:
 // the same with q/k/v in fp32; MODE 2: nothing (dtypes, gate widths and the prologue are run-time
-// properties, every load sits behind a branch and both activation paths are compiled in); MODE 3:
-// bf16 q/k/v, fp32 activated gates with ONE value per head (Gated DeltaNet's scalar decay and beta);
+// properties, every load sits behind a branch and both activation paths are compiled in);
 // MODE 4: bf16 q/k/v, fp32 activated gates, the decay per channel and ONE erase / write gate value per head
 // (the KDA layout).
 template <int MODE>
 struct InCfg {
   static constexpr bool fixed = MODE != 2;
-  static constexpr bool scalar_gates = MODE == 3;                 // the decay is one scalar per (token, head)
-  static constexpr bool scalar_bw = MODE == 3 || MODE == 4;       // b and w are
+  static constexpr bool scalar_bw = MODE == 4;       // b and w are one scalar per (token, head)
   static constexpr int qkv_dt = MODE == 1 ? DN_F32 : DN_BF16;
 };
 inline int input_mode(const Geo& g) {
   if (g.K != K || g.gate_dt != DN_F32 || (g.flags & (DN_FUSE_PROLOGUE | DN_STABILITY_GUARD))) return 2;
   if (g.gC == g.K && g.bC == g.K && g.wC == g.V) return g.qkv_dt == DN_BF16 ? 0 : 1;
-  if (g.gC == 1 && g.bC == 1 && g.wC == 1 && g.qkv_dt == DN_BF16) return 3;
   if (g.gC == g.K && g.bC == 1 && g.wC == 1 && g.qkv_dt == DN_BF16) return 4;
   return 2;
 }
@@ -136,25 +133,6 @@ __device__ __forceinline__ void bact8(const Rows& r, int x, int p, float (&o)[8]
     for (int i = 0; i < 8; ++i) o[i] = fmaxf(o[i], 0.f);
   }
   if (!live) zero8(o);
-}
-// activated log-decay g (<= 0)
-__device__ __forceinline__ void gact8(const Rows& r, int x, int p, float (&o)[8]) {
-  const bool live = x < r.rows_valid && p < r.kp;
-  raw_gate8(r.gg, r.g_row0, r.g_pitch, r.gC, r.gate_dt, live ? x : 0, live ? p : 0, o);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    if (r.fuse) { o[i] = -expf(fminf(o[i], 5.f)); if (r.guard) o[i] = fminf(o[i], -1e-6f); }
-    else { o[i] = o[i] <= 0.f ? o[i] : 0.f; if (r.guard) o[i] = fminf(o[i], -1e-6f); }
-  }
-  if (!live) zero8(o);
-}
-// beta = b_act * k_hat
-__device__ __forceinline__ void beta8(const Rows& r, int x, int p, float (&o)[8]) {
-  float kk[8];
-  bact8(r, x, p, o);
-  khat8(r, x, p, kk);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) o[i] *= kk[i];
 }
 
 // Row normalisers, 512 threads, a warp covering 8 rows x 4 pieces: thread (myrow = 8*warp + (lane&7),
@@ -291,7 +269,7 @@ __device__ __forceinline__ Rows make_rows(const Geo& g, const void* q, const voi
   r.qk_pitch = (size_t)g.Hk * g.K;
   r.qk_row0 = tok0 * r.qk_pitch + (size_t)(h / g.qk_div) * g.K;
   r.kp = CF::fixed ? K / 8 : g.K / 8;
-  r.gC = CF::fixed ? (CF::scalar_gates ? 1 : K) : g.gC;
+  r.gC = CF::fixed ? K : g.gC;
   r.bC = CF::fixed ? (CF::scalar_bw ? 1 : K) : g.bC;
   r.g_pitch = (size_t)g.gH * g.gC;
   r.g_row0 = tok0 * r.g_pitch + (size_t)g.gate_head(h, g.gH) * g.gC;

@@ -19,7 +19,7 @@
 
 namespace dn {
 
-// fp32 SIMT products (the tensor-core variant lives in dn_prepass_bwd_tc.cu).
+// fp32 SIMT products, row-major tiles (the tensor-core variants are dn_prepass_bwd_fast.cu and dn_prepass_bwd_tc.cu).
 // SPLIT: the CTAs of a cluster share an item, and its scratch: rows, columns and output tiles are dealt out, and the cluster's
 // barrier stands between the phases.  For jobs that leave most of the chip idle (launch_prepass_bwd), where one item is a
 // chain of latencies: 64 x 64 heads, chunks of 64, 8 items: 195 us with one CTA an item, 59 with eight.
@@ -141,9 +141,9 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
     }
     // ---- V_new = U - W S
     cta_gemm<true, true, GN>(C, Vw, K,
-        [&](int i, int kk) { return ldf(a.res.W, bW + rix(g.img, i, kk, K), pre); },
+        [&](int i, int kk) { return ldf(a.res.W, bW + (size_t)i * K + kk, pre); },
         [&](int kk, int j) { float s = S[(size_t)kk * Vw + j]; return sbf ? bf16r(s) : s; },
-        [&](int i, int j, float acc) { VN[i * Vw + j] = ldf(a.res.U, bU + rix(g.img, i, j, Vw), pre) - acc; },
+        [&](int i, int j, float acc) { VN[i * Vw + j] = ldf(a.res.U, bU + (size_t)i * Vw + j, pre) - acc; },
         tile, team);
     auto dO_at = [&](int i, int j) -> float {
       const int t = t0 + i;
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
         [&](int kk, int j) { float s = S[(size_t)j * Vw + kk]; return sbf ? bf16r(s) : s; },
         [&](int i, int j, float acc) { DQE[i * K + j] = acc; }, tile, team);
     cta_gemm<false, true, GN>(C, Vw, C,
-        [&](int i, int kk) { float t = g.img ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(T)[rix(true, kk, i, C)]) : T[(size_t)kk * C + i]; return ibf ? bf16r(t) : t; },
+        [&](int i, int kk) { float t = T[(size_t)kk * C + i]; return ibf ? bf16r(t) : t; },
         [&](int kk, int j) { float x = dV[(size_t)kk * Vw + j]; return ibf ? bf16r(x) : x; },
         [&](int i, int j, float acc) { DY[i * Vw + j] = trunc ? bf16r(acc) : acc; }, tile, team);
     if (SPLIT) team.sync();
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
         [&](int i, int j, float acc) { DM[i * C + j] = (i >= j && seg_s[i] == seg_s[j]) ? acc : 0.f; }, tile, team);
     // ---- dX = T^T dW
     cta_gemm<false, true, GN>(C, K, C,
-        [&](int i, int kk) { float t = g.img ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(T)[rix(true, kk, i, C)]) : T[(size_t)kk * C + i]; return ibf ? bf16r(t) : t; },
+        [&](int i, int kk) { float t = T[(size_t)kk * C + i]; return ibf ? bf16r(t) : t; },
         [&](int kk, int j) { float x = DW[kk * K + j]; return ibf ? bf16r(x) : x; },
         [&](int i, int j, float acc) { DX[i * K + j] = trunc ? bf16r(acc) : acc; }, tile, team);
     if (SPLIT) team.sync();
@@ -181,8 +181,8 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
     cta_gemm<true, false, GN>(C, C, K + Vw,
         [&](int i, int kk) { return kk < K ? DX[i * K + kk] : DY[i * Vw + (kk - K)]; },
         [&](int kk, int j) {
-          return kk < K ? ldf(a.res.W, bW + rix(g.img, j, kk, K), pre)
-                        : ldf(a.res.U, bU + rix(g.img, j, kk - K, Vw), pre);
+          return kk < K ? ldf(a.res.W, bW + (size_t)j * K + kk, pre)
+                        : ldf(a.res.U, bU + (size_t)j * Vw + kk - K, pre);
         },
         [&](int i, int j, float acc) { DA[i * C + j] = (i > j && seg_s[i] == seg_s[j]) ? -acc : 0.f; }, tile, team);
 

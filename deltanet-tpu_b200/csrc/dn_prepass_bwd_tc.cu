@@ -1,6 +1,8 @@
-// Chunk-parallel backward on the tcgen05 tensor cores (bf16 precision, chunk = K = 128, value
-// width 128 or 256): the adjoint of the state step's value-width contractions, of the prepass
-// (reference: src/deltanet_tpu/gdn2.py:243-493, 750-762) and of the fused prologue (558-575).
+// Chunk-parallel backward of tiles with strong channel-wise decay (bf16 precision, 128-row tiles on the tcgen05 tensor
+// cores): the adjoint of the state step's value-width contractions, of the prepass (reference:
+// src/deltanet_tpu/gdn2.py:243-493, 750-762) and of the fused prologue (558-575).  The forward prepass marks the tiles whose
+// decay leaves e^{+-32} of a document's midpoint; all others are dn_prepass_bwd_fast.cu's.  Launched behind that kernel,
+// this one usually finds nothing marked and ends after one look.
 //
 // Per (batch, exec head, chunk), 512 threads, one CTA per SM, in this order:
 //   G. nine matrix products (bwd_gemms_tc): V_new, dqe, dM, dW, dke, dX, dY, dA.  Every operand is a
@@ -8,25 +10,18 @@
 //   V. dv and dw from the bf16 image of dY that G leaves in shared memory; in the headline mode the
 //      rows of v, w, dv, dw move by bulk copies through padded staging rows.
 //   L. row normalisers and the cumulative log-decay of the chunk in shared memory.
-//   D/H. adjoints of A and M, i.e. dbeta', dq', dk', by one of three routes:
-//      (a) one scalar decay per (token, head): with f_ij = e^{lam_i - lam_j} applied entry-wise to dA and dM,
-//          two rounds of two products on the plain images of k_hat and q_hat;
-//      (b) channel-wise decay that stays within e^{+-32} of each document's midpoint over the chunk (tested
-//          per chunk on the device): the same two rounds on images of k_hat / f, q_hat f, beta k_hat f with
-//          f = e^{Lam - midpoint}; the results are scaled by f, f, 1 / f when phase E reads them;
-//          on (a) and (b) the three accumulators stay in tensor memory for phase E;
-//      (c) otherwise: D. the 16x16 diagonal blocks of dA and dM, exact, one thread per (block, channel), from
-//          shared-memory caches of k_hat, q_hat, beta (64 rows at a time), which initialises dbeta', dq', dk'
-//          in the scratch and parks k_hat | q_hat (two bf16 per column) and beta in tensor memory; then
-//          H. the three-level factorisation of the forward: in one level every row is either a ROW of the
-//          level's entries (lower block of its pair) or a COLUMN (upper block), so with dA_s / dM_s the
-//          entries the level owns, KR the image holding beta-images on lower rows and k-images on upper
-//          rows, and QK holding q-images / k-images,
-//            T1 = (dA_s + dA_s^T) KR,   T2 = (dM_s + dM_s^T) QK        (four MMAs, one drain)
-//            lower rows:  dbeta' += rowfac * T1,  dq' += rowfac * T2
-//            upper rows:  dk'    += colfac * (T1 + T2)
-//          with the same exp(Lam - Lam_ref) factors (all <= 1) as the forward; a level's drain overlaps the
-//          next level's image build.
+//   D. adjoints of A and M, i.e. dbeta', dq', dk': the 16x16 diagonal blocks of dA and dM, exact, one thread per (block, channel), from
+//      shared-memory caches of k_hat, q_hat, beta (64 rows at a time), which initialises dbeta', dq', dk'
+//      in the scratch and parks k_hat | q_hat (two bf16 per column) and beta in tensor memory; then
+//      H. the three-level factorisation of the forward: in one level every row is either a ROW of the
+//      level's entries (lower block of its pair) or a COLUMN (upper block), so with dA_s / dM_s the
+//      entries the level owns, KR the image holding beta-images on lower rows and k-images on upper
+//      rows, and QK holding q-images / k-images,
+//        T1 = (dA_s + dA_s^T) KR,   T2 = (dM_s + dM_s^T) QK        (four MMAs, one drain)
+//        lower rows:  dbeta' += rowfac * T1,  dq' += rowfac * T2
+//        upper rows:  dk'    += colfac * (T1 + T2)
+//      with the same exp(Lam - Lam_ref) factors (all <= 1) as the forward; a level's drain overlaps the
+//      next level's image build.
 //   E. combination into dLambda, d q_hat, d k_hat, d b (written), the l2norm adjoint and dq, dk, in the
 //      thread mapping of a tensor-memory drain; the operands of the second half wait in tensor memory.
 //   R. dg by a within-document reverse cumulative sum plus the Lambda_end path; written with the

@@ -1,5 +1,5 @@
-// The nine matrix products of the chunk-parallel backward on the tcgen05 tensor cores
-// (bf16 precision, chunk = K = 128, value width VW in {128, 256}).
+// The nine matrix products of the chunk-parallel backward of strong-decay tiles on the tcgen05 tensor cores
+// (bf16 precision, 128-row tiles, channels padded to 128, value width to VW in {128, 256}).
 //
 // Operand images live in four shared-memory slots (X, Y, Z of 128 x VW bf16, P of 128 x 128)
 // that are refilled as the sequence advances; accumulators live in tensor memory (512 columns)

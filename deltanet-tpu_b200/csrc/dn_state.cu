@@ -62,10 +62,10 @@ __global__ void __launch_bounds__(DN_THREADS) state_fwd_kernel(StateArgs a) {
     const size_t bW = item * C * K, bU = item * C * Vw, bM = item * C * C;
     // V_new = U - W S
     cta_gemm<true, true, VS>(C, VS, K,
-        [&](int i, int kk) { return ldf(a.res.W, bW + rix(g.img, i, kk, K), pre); },
+        [&](int i, int kk) { return ldf(a.res.W, bW + (size_t)i * K + kk, pre); },
         [&](int kk, int j) { float s = S[kk * VS + j]; return sbf ? bf16r(s) : s; },
         [&](int i, int j, float acc) {
-          const float u = (a.res.U && !trans) ? ldf(a.res.U, bU + rix(g.img, i, v0 + j, Vw), pre) : 0.f;   // transition columns: U = 0
+          const float u = (a.res.U && !trans) ? ldf(a.res.U, bU + (size_t)i * Vw + v0 + j, pre) : 0.f;   // transition columns: U = 0
           Vn[i * VS + j] = u - acc;
         },
         tile);
@@ -73,8 +73,8 @@ __global__ void __launch_bounds__(DN_THREADS) state_fwd_kernel(StateArgs a) {
       // O = [qe | M] [S ; V_new]
       cta_gemm<true, true, VS>(C, VS, K + C,
           [&](int i, int kk) {
-            return kk < K ? ldf(a.res.qe, bW + rix(g.img, i, kk, K), pre)
-                          : ldf(a.res.M, bM + rix(g.img, i, kk - K, C), pre);
+            return kk < K ? ldf(a.res.qe, bW + (size_t)i * K + kk, pre)
+                          : ldf(a.res.M, bM + (size_t)i * C + kk - K, pre);
           },
           [&](int kk, int j) {
             if (kk < K) { float s = S[kk * VS + j]; return sbf ? bf16r(s) : s; }
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(DN_THREADS) state_fwd_kernel(StateArgs a) {
     }
     // S <- decay * S + ke^T V_new
     cta_gemm<false, true, VS>(K, VS, C,
-        [&](int i, int kk) { return ldf(a.res.ke, bW + rix(g.img, kk, i, K), pre); },
+        [&](int i, int kk) { return ldf(a.res.ke, bW + (size_t)kk * K + i, pre); },
         [&](int kk, int j) { float x = Vn[kk * VS + j]; return sbf ? bf16r(x) : x; },
         [&](int i, int j, float acc) {
           float carried = 0.f;
@@ -146,8 +146,8 @@ __global__ void __launch_bounds__(DN_THREADS) state_bwd_kernel(StateArgs a) {
     // dV = M^T dO + ke dH
     cta_gemm<false, true, VS>(C, VS, C + K,
         [&](int i, int kk) {
-          return kk < C ? ldf(a.res.M, bM + rix(g.img, kk, i, C), pre)
-                        : ldf(a.res.ke, bW + rix(g.img, i, kk - C, K), pre);
+          return kk < C ? ldf(a.res.M, bM + (size_t)kk * C + i, pre)
+                        : ldf(a.res.ke, bW + (size_t)i * K + kk - C, pre);
         },
         [&](int kk, int j) {
           if (kk < C) { float x = dOs[kk * VS + j]; return ibf ? bf16r(x) : x; }
@@ -162,8 +162,8 @@ __global__ void __launch_bounds__(DN_THREADS) state_bwd_kernel(StateArgs a) {
     // dH <- decay * dH + qe^T dO - W^T dV, cleared at a document start
     cta_gemm<false, true, VS>(K, VS, 2 * C,
         [&](int i, int kk) {
-          return kk < C ? ldf(a.res.qe, bW + rix(g.img, kk, i, K), pre)
-                        : -ldf(a.res.W, bW + rix(g.img, kk - C, i, K), pre);
+          return kk < C ? ldf(a.res.qe, bW + (size_t)kk * K + i, pre)
+                        : -ldf(a.res.W, bW + (size_t)(kk - C) * K + i, pre);
         },
         [&](int kk, int j) {
           float x = kk < C ? dOs[kk * VS + j] : dVs[(kk - C) * VS + j];
@@ -444,7 +444,7 @@ static int launch_bwd(const StateArgs& a, cudaStream_t st) {
 
 // fp32 residuals and products, and room for a chunk's factors (all but 128 x 128).
 static bool staged(const Geo& g) {
-  return g.pre_dt == DN_F32 && !g.img && !g.state_bf16() && !g.bf16_mode() && !(g.C == 128 && g.K == 128);
+  return g.pre_dt == DN_F32 && !g.state_bf16() && !g.bf16_mode() && !(g.C == 128 && g.K == 128);
 }
 template <int C, int K>
 static int launch_staged(const StateArgs& a, bool bwd, cudaStream_t st) {

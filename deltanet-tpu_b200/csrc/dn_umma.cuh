@@ -78,12 +78,6 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 
-// Asks the memory system to bring a contiguous global range into L2 (no destination, nothing to wait
-// for).  Skipped unless address and size are multiples of 16 bytes.
-__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
-  if (((reinterpret_cast<uintptr_t>(p) | bytes) & 15u) == 0 && bytes)
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
 
 // ---- fences ------------------------------------------------------------------------------
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -229,18 +223,6 @@ __device__ __forceinline__ float4 ld_keep4_pred(const float4* p, bool pred) {
   return v;
 }
 
-// ---- predicated loads ------------------------------------------------------------------------
-// 16-byte global load through L2 only, skipped (zeros returned) when `pred` is false: no branch, so
-// the loads of an unrolled group stay back to back
-__device__ __forceinline__ float4 ldcg_pred(const float4* p, bool pred) {
-  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
-      : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w) : "l"(p), "r"((int)pred) : "memory");
-  return v;
-}
 
 // ---- packing helpers ---------------------------------------------------------------------
 __device__ __forceinline__ uint32_t pack2(float a, float b) {

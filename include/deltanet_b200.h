@@ -90,11 +90,12 @@ typedef struct dn_shape {
 
 /* Exec-head view of a shape (what the residual layouts are expressed in). */
 typedef struct dn_exec {
-  int32_t H, Vw, G, NC;        /* exec heads, value width, value heads per exec head, chunks */
+  int32_t H, Vw, G, NC;        /* exec heads, value width (padded to 128 or 256 on the tensor-core path), value heads per
+                                  exec head, chunks */
   int32_t pre_dtype;           /* dtype of W,U,M,qe,ke: bf16 in bf16 precision else f32 (gdn2.py:1247) */
   int32_t chunk;               /* rows per tile the kernels use, the C of every layout below.  Equal to
-                                  dn_shape.chunk except on the tensor-core path (bf16 precision, K = 128,
-                                  Vw in {128,256}): there tiles are 128 rows, the M of a tcgen05.mma, and a
+                                  dn_shape.chunk except on the tensor-core path (bf16 precision without
+                                  DN_STATE_FP32_MM): there tiles are 128 rows, the M of a tcgen05.mma, and a
                                   request for 64 runs with pairs of requested chunks merged into one tile
                                   (the chunked form regroups the token recurrence exactly; only the points
                                   where the state is rounded to bf16 move).  NC = ceil(L / chunk).          */
@@ -107,12 +108,12 @@ int dn_exec_view(const dn_shape* s, dn_exec* out);
  *
  * The five pre_dtype tiles are opaque to the caller: only the library's own entry points read
  * them.  Each (batch, head, chunk) tile holds rows x cols elements, row-major in general; for shapes
- * that take the tensor-core path (precision bf16 without DN_STATE_FP32_MM, K = 128, Vw in {128,256},
- * DN_FORCE_SIMT unset) a tile is stored as the tensor cores' operand image, [col / 8][row][8 elements], so that
- * every kernel copies it into shared memory as it lies.  The sizes are the same in both layouts.
- * On that path T holds a bf16 image in the first half of its slot, and the chunk-entry states are kept
+ * that take the tensor-core path (precision bf16 without DN_STATE_FP32_MM,
+ * DN_FORCE_SIMT unset) a tile is stored as the tensor cores' operand image, [col / 8][row][8 elements], with K and Vw
+ * padded to 128 (Vw: or 256), so that every kernel copies it into shared memory as it lies; dn_residual_bytes accounts for it.
+ * On that path T holds a bf16 image in the first half of its slot and per-row factors of the tile in the second, and the chunk-entry states are kept
  * as a bf16 operand image only (half the bytes; dn_residual_bytes accounts for it).  The dV / dH
- * buffers that dn_state_bwd hands to dn_prepass_bwd are opaque in the same way (bf16 images plus the
+ * buffers that dn_state_bwd hands to dn_prepass_bwd are opaque in the same way (bf16 images, and behind dV's the
  * partial sums of the decay cotangent); a caller only sizes them (fp32 element counts) and passes
  * them on.
  */
@@ -262,8 +263,7 @@ int dn_sp_apply(const float* P, const float* S_in, const float* Q, float* S_out,
  * cudaFree or other allocating routine.
  *
  *  - Shapes whose prepass needs more scratch than the array return DN_ERR_STATIC_SCRATCH_EXCEEDED
- *    (the tensor-core path, bf16 precision with chunk = K = 128, needs 9.3 MiB and always fits;
- *    the fp32 path fits for chunk = K = V = 64).
+ *    (the tensor-core path, bf16 precision, needs none; the fp32 path fits for chunk = K = V = 64).
  *  - The first call on each device looks up the array's device address (with that device
  *    current).  Make that first call outside any stream capture.
  *  - All calls share the one array and it keeps the previous call's contents.  Nothing in it has
