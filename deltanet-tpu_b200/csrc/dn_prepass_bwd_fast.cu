@@ -147,16 +147,20 @@ __device__ __noinline__ void drain_sub(bool dead, uint32_t addr, uint4* img, int
     img[128] = umma::pack8(t);
   }
 }
-// strictly lower triangle inside a document, times the scalar decay when lam is given; the diagonal apart when diag is
-__device__ __noinline__ void drain_masked(bool dead, uint32_t addr, uint4* img, int row, int group, float sign, const int* seg, const float* lam, float* diag) {
+// strictly lower triangle inside a document, times the scalar decay when lam is given; the diagonal apart when diag is; a second
+// image, of the first one's rows times `by`, when there is one
+__device__ __noinline__ void drain_masked(bool dead, uint32_t addr, uint4* img, int row, int group, float sign, const int* seg, const float* lam, float* diag,
+                                           uint4* img2 = nullptr, float by = 0.f) {
   const int sr = seg[row];
   const float lr = lam ? lam[row] * DN_LOG2E : 0.f;
   img += 4 * group * 128 + row;
+  if (img2) img2 += 4 * group * 128 + row;
 #pragma unroll 1
   for (int j = 0; j < 2; ++j, img += 256) {
     const int c0 = group * 32 + 16 * j;
     if (c0 > (row | 31)) {                              // (uniform over the warp) nothing of this piece survives
       img[0] = img[128] = make_uint4(0, 0, 0, 0);
+      if (img2) img2[256 * j] = img2[256 * j + 128] = make_uint4(0, 0, 0, 0);
       continue;
     }
     float v[16];
@@ -172,8 +176,20 @@ __device__ __noinline__ void drain_masked(bool dead, uint32_t addr, uint4* img, 
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] *= umma::ex2_fast(fminf(lr - lam[c0 + i] * DN_LOG2E, 0.f));
     }
-    img[0] = umma::pack8p(v);
-    img[128] = umma::pack8p(v + 8);
+    const uint4 lo = umma::pack8p(v), hi = umma::pack8p(v + 8);
+    img[0] = lo;
+    img[128] = hi;
+    if (img2) {
+      float t[8];
+      umma::unpack8(lo, t);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) t[i] *= by;
+      img2[256 * j] = umma::pack8(t);
+      umma::unpack8(hi, t);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) t[i] *= by;
+      img2[256 * j + 128] = umma::pack8(t);
+    }
   }
 }
 // One step of summing 8 values per lane over the warp's lanes, all at once: a lane hands over the N it drops
@@ -564,8 +580,8 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       finish(cx);
     }
     // ---- dA (dM is in slot 5); everything else is free
-    uint4 *const dAi = sl.region(4), *const dMi = sl.at(5);
-    drain_masked(cx.dead, tb + T_TMP, dAi, row, group, -1.f, seg_s, SC ? lam_s : nullptr, nullptr);
+    uint4 *const dAi = sl.region(4), *const dMi = sl.at(5), *const dAb = SC ? sl.region(2) : nullptr;
+    drain_masked(cx.dead, tb + T_TMP, dAi, row, group, -1.f, seg_s, SC ? lam_s : nullptr, nullptr, dAb, SC ? bet_s[row] : 0.f);
 
     // ---- key side: rows of q, k, b in the row mapping
     const bool live = rx < rows;
@@ -735,7 +751,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     }
     // ---- T1, T2, T3 on top of them
     if constexpr (SC) {
-      uint4 *KI = sl.region(0), *QI = sl.region(1), *BI = sl.region(2);
+      uint4 *KI = sl.region(0), *QI = sl.region(1);
 #pragma unroll 2
       for (int it = 0; it < 4; ++it) {
         const int p = it * 4 + rp;
@@ -744,12 +760,11 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         pieces(p, kh, qh, be);
         KI[p * PP + rx] = umma::pack8(kh);
         QI[p * PP + rx] = umma::pack8(qh);
-        BI[p * PP + rx] = umma::pack8(be);
       }
       umma::pre_issue_sync();
       product<128, false, true>(cx, dAi, 2048, KI, PB, C, T_B, true);       // (dA f)   k_hat
       product<128, false, true>(cx, dMi, 2048, KI, PB, C, T_Q, true);       // (dM f)   k_hat
-      product<128, true, true>(cx, dAi, 2048, BI, PB, C, T_K, true);        // (dA f)^T (b k_hat)
+      product<128, true, true>(cx, dAb, 2048, KI, PB, C, T_K, true);        // (dA f b)^T k_hat: b goes with the rows of dA
       product<128, true, true>(cx, dMi, 2048, QI, PB, C, T_K, true);        // (dM f)^T q_hat
       commit(cx);
       finish(cx);
