@@ -1,5 +1,5 @@
 // The operators' host path in native code: a CPython extension that takes torch tensors, checks that a call is a plain one
-// (CUDA tensors, contiguous, one dtype for q/k/v and one for the gates, shapes as documented), allocates, and calls the
+// (CUDA tensors of one device, contiguous, one dtype for q/k/v and one for the gates, shapes as documented), allocates, and calls the
 // C ABI.  A call that is not plain is answered with None: the Python layer then validates it, with its error messages,
 // converts what has to be converted and comes back through `apply`.
 //
@@ -43,7 +43,8 @@ void check(int status, const char* what) {
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 const void* ptr(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nullptr; }
 int code(at::ScalarType t) { return t == at::kBFloat16 ? DN_BF16 : (t == at::kFloat ? DN_F32 : -1); }
-bool plain(const Tensor& t) { return t.is_cuda() && t.is_contiguous(); }
+// Can a kernel take the tensor as it is, beside `q`?  (What is not on q's device the general path moves or refuses.)
+bool plain(const Tensor& t, const Tensor& q) { return t.device() == q.device() && t.is_contiguous(); }
 
 // ------------------------------------------------------------------------------------------------ the chunked operator
 Tensor bytes_on(const Tensor& like, size_t n) {
@@ -161,8 +162,9 @@ PyObject* py_chunk(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (int i = 6; i < 9; ++i)
     if (a[i] != Py_None && !THPVariable_Check(a[i])) Py_RETURN_NONE;
   const Tensor ids = tensor_or_none(a[6]), cu = tensor_or_none(a[7]), init = tensor_or_none(a[8]);
+  if (!q.is_cuda()) Py_RETURN_NONE;
   for (const Tensor* t : {&q, &k, &v, &g, &b, &w})
-    if (!plain(*t)) Py_RETURN_NONE;
+    if (!plain(*t, q)) Py_RETURN_NONE;
   if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || q.sizes() != k.sizes()) Py_RETURN_NONE;
   const int64_t B = q.size(0), Lq = q.size(1), Hk = q.size(2), K = q.size(3), Hv = v.size(2), V = v.size(3);
   if (v.size(0) != B || v.size(1) != Lq || B < 1 || Lq < 1 || Hk < 1 || Hv < 1 || Hv % Hk) Py_RETURN_NONE;
@@ -175,13 +177,13 @@ PyObject* py_chunk(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!gate(g, 2, B, Lq, Hk, Hv, K, s.g_heads, s.g_cols) || !gate(b, 2, B, Lq, Hk, Hv, K, s.b_heads, s.b_cols) ||
       !gate(w, 2, B, Lq, Hk, Hv, V, s.w_heads, s.w_cols))
     Py_RETURN_NONE;
-  if (init.defined() && (!plain(init) || init.scalar_type() != at::kFloat || init.dim() != 4 || init.size(0) != B || init.size(1) != Hv ||
+  if (init.defined() && (!plain(init, q) || init.scalar_type() != at::kFloat || init.dim() != 4 || init.size(0) != B || init.size(1) != Hv ||
                          init.size(2) != K || init.size(3) != V))
     Py_RETURN_NONE;
-  if (ids.defined() && (cu.defined() || !plain(ids) || ids.scalar_type() != at::kInt || ids.numel() != B * Lq ||
+  if (ids.defined() && (cu.defined() || !plain(ids, q) || ids.scalar_type() != at::kInt || ids.numel() != B * Lq ||
                         !(ids.dim() == 2 ? ids.size(0) == B : ids.dim() == 1)))
     Py_RETURN_NONE;
-  if (cu.defined() && (!plain(cu) || cu.scalar_type() != at::kInt || cu.dim() != 1 || cu.numel() < 2)) Py_RETURN_NONE;
+  if (cu.defined() && (!plain(cu, q) || cu.scalar_type() != at::kInt || cu.dim() != 1 || cu.numel() < 2)) Py_RETURN_NONE;
   s.B = (int32_t)B; s.L = (int32_t)Lq; s.Hk = (int32_t)Hk; s.Hv = (int32_t)Hv; s.K = (int32_t)K; s.V = (int32_t)V;
   s.qkv_dtype = qdt;
   s.gate_dtype = gdt;
@@ -226,8 +228,9 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor g = THPVariable_Unpack(a[3]), b = THPVariable_Unpack(a[4]), w = THPVariable_Unpack(a[5]), state = THPVariable_Unpack(a[6]);
   const Tensor reset = tensor_or_none(a[7]);
   Tensor next = tensor_or_none(a[12]);
+  if (!q.is_cuda()) Py_RETURN_NONE;
   for (const Tensor* t : {&q, &k, &v, &g, &b, &w, &state})
-    if (!plain(*t)) Py_RETURN_NONE;
+    if (!plain(*t, q)) Py_RETURN_NONE;
   if (q.dim() != 3 || k.dim() != 3 || v.dim() != 3 || q.sizes() != k.sizes() || state.dim() != 4) Py_RETURN_NONE;
   const int64_t B = q.size(0), Hk = q.size(1), K = q.size(2), Hv = v.size(1), V = v.size(2);
   if (v.size(0) != B || B < 1 || Hk < 1 || Hv < 1 || Hv % Hk || (K != 64 && K != 128) || (V != 64 && V != 128)) Py_RETURN_NONE;
@@ -244,7 +247,7 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (t->dim() == 3 && t->size(1) == 1 && (t->size(2) == 1 || t->size(2) == Hk || t->size(2) == Hv)) Py_RETURN_NONE;
   s.flags = (uint32_t)PyLong_AsUnsignedLong(a[9]);
   if (reset.defined()) {
-    if (!plain(reset) || (reset.scalar_type() != at::kBool && reset.scalar_type() != at::kByte)) Py_RETURN_NONE;
+    if (!plain(reset, q) || (reset.scalar_type() != at::kBool && reset.scalar_type() != at::kByte)) Py_RETURN_NONE;
     if (reset.dim() == 2 && reset.size(0) == B && reset.size(1) == Hv && Hv > 1) s.flags |= DN_RESET_PER_HEAD;
     else if (reset.dim() != 1 || reset.size(0) != B) Py_RETURN_NONE;
   }
@@ -261,7 +264,7 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!next.defined()) {
     next = at::empty({B, Hv, K, V}, state.options().dtype(st).requires_grad(false));
     next_py = nullptr;
-  } else if (!plain(next) || next.scalar_type() != st || next.sizes() != state.sizes()) {
+  } else if (!plain(next, q) || next.scalar_type() != st || next.sizes() != state.sizes()) {
     Py_RETURN_NONE;
   }
   Tensor o = at::empty({B, Hv, V}, q.options().requires_grad(false));
@@ -272,6 +275,14 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(o));
   PyTuple_SET_ITEM(r, 1, next_py ? Py_NewRef(next_py) : THPVariable_Wrap(next));
   return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// plain(t, q): the test that every tensor of a call has to pass
+PyObject* py_plain(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK_VALUE(n == 2 && all_tensors(a, 2), "plain: two tensors");
+  return PyBool_FromLong(plain(THPVariable_Unpack(a[0]), THPVariable_Unpack(a[1])));
   END_HANDLE_TH_ERRORS
 }
 
@@ -300,6 +311,7 @@ PyMethodDef methods[] = {
     {"chunk", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_chunk)), METH_FASTCALL, nullptr},
     {"apply", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_apply)), METH_FASTCALL, nullptr},
     {"decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_decode)), METH_FASTCALL, nullptr},
+    {"plain", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_plain)), METH_FASTCALL, nullptr},
     {"bind", py_bind, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

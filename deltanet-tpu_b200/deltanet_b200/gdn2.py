@@ -45,9 +45,14 @@ def _precision_code(precision) -> int:
 
 
 def _require_cuda(*ts):
+    """All tensors (the first decides) on one CUDA device: a kernel gets their addresses as they are."""
     for t in ts:
-        if t is not None and not t.is_cuda:
+        if t is None:
+            continue
+        if not t.is_cuda:
             raise RuntimeError("deltanet_b200 runs on CUDA tensors only; there is no CPU path.")
+        if t.device != ts[0].device:
+            raise RuntimeError(f"deltanet_b200: all tensors of a call must be on one device, got {ts[0].device} and {t.device}.")
 
 
 def _common_dtype(ts: Sequence[torch.Tensor]) -> torch.dtype:
@@ -409,7 +414,7 @@ def gdn2_decode_step(
                 raise ValueError(f"reset shape {tuple(torch.as_tensor(reset).shape)} must broadcast over (B, Hv, 1, 1); "
                                  "per-element resets inside a (K, V) state are not supported.")
         reset_t = reset_t.to(torch.uint8).contiguous()
-    _require_cuda(q, k, v, g, b, w, state)
+    _require_cuda(q, k, v, g, b, w, state, out_state)
     if scale is None:
         scale = 1.0 / math.sqrt(K)
     out_dtype = v.dtype
