@@ -1,7 +1,10 @@
 // The operators' host path in native code: a CPython extension that takes torch tensors, checks that a call is a plain one
 // (CUDA tensors of one device, contiguous, one dtype for q/k/v and one for the gates, shapes as documented), allocates, and calls the
 // C ABI.  A call that is not plain is answered with None: the Python layer then validates it, with its error messages,
-// converts what has to be converted and comes back through `apply`.
+// converts what has to be converted and comes back through `forward`, inside a Python autograd function unless nothing
+// watches the call (`bare`).  What is left to that function: tangents (forward-mode AD), function transforms, tracing, and
+// dispatch modes.  They see a Python autograd function and either follow it or raise their own error, whereas addresses handed
+// over here would leave them with results that look like constants.
 //
 // Why: a decode step of one sequence takes 4.5 us on the GPU, its path through the interpreter (shape checks, seven
 // conversions that change nothing, ctypes structures) took 25; a short prompt 25 of 50.
@@ -9,9 +12,12 @@
 // Nothing of the CUDA library is linked: `bind` receives the addresses of the C-ABI functions from the module that has
 // loaded it (which may be an instrumented build).
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/graph_task.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 
 #include <cmath>
@@ -43,10 +49,26 @@ void check(int status, const char* what) {
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 const void* ptr(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nullptr; }
 int code(at::ScalarType t) { return t == at::kBFloat16 ? DN_BF16 : (t == at::kFloat ? DN_F32 : -1); }
+// A tensor with memory of its own behind it: not a wrapper of a function transform, a fake or a tensor that stands for
+// something else than what its memory holds.
+bool dense(const Tensor& t) {
+  constexpr c10::DispatchKeySet wrappers({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
+                                          c10::DispatchKey::Functionalize, c10::DispatchKey::Negative, c10::DispatchKey::Conjugate,
+                                          c10::DispatchKey::ZeroTensor});
+  return t.layout() == at::kStrided && !t.key_set().has_any(wrappers) && t.has_storage();
+}
 // Can a kernel take the tensor as it is, beside `q`?  (What is not on q's device the general path moves or refuses.)
-bool plain(const Tensor& t, const Tensor& q) { return t.device() == q.device() && t.is_contiguous(); }
+bool plain(const Tensor& t, const Tensor& q) { return dense(t) && t.device() == q.device() && t.is_contiguous(); }
+// Does something follow the calls of this thread that an address would escape?
+bool watched() { return torch::jit::tracer::isTracing() || c10::impl::TorchDispatchModeTLS::any_modes_set(); }
+bool tangent(const Tensor& t) { return t.defined() && t._fw_grad(0).defined(); }
 
 // ------------------------------------------------------------------------------------------------ the chunked operator
+void require_dense(std::initializer_list<const Tensor*> ts) {
+  for (const Tensor* t : ts)
+    TORCH_CHECK(!t->defined() || dense(*t),
+                "deltanet_b200: a tensor of this call has no memory of its own (a fake tensor, or the wrapper of a function transform)");
+}
 Tensor bytes_on(const Tensor& like, size_t n) {
   return at::empty({(int64_t)(n < 256 ? 256 : n)}, like.options().dtype(at::kByte));
 }
@@ -54,6 +76,7 @@ Tensor bytes_on(const Tensor& like, size_t n) {
 // the forward; keeps the residuals in *kept when asked
 variable_list forward(const dn_shape& shape, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& b,
                       const Tensor& w, const Tensor& init, const Tensor& seg, bool want_final, Tensor* kept, Tensor out = Tensor()) {
+  require_dense({&q, &k, &v, &g, &b, &w, &init, &seg});
   if (!out.defined()) out = at::empty({shape.B, shape.L, shape.Hv, shape.V}, q.options().requires_grad(false));
   Tensor fin;
   if (want_final) fin = at::empty({shape.B, shape.Hv, shape.K, shape.V}, q.options().dtype(at::kFloat).requires_grad(false));
@@ -61,11 +84,13 @@ variable_list forward(const dn_shape& shape, const Tensor& q, const Tensor& k, c
   dn_shape f = shape;
   if (kept) {
     *kept = bytes_on(q, abi.residual_bytes(&shape));
+    require_dense({kept});
     check(abi.residual_carve(&shape, kept->mutable_data_ptr(), &res), "dn_residual_carve");
   } else {
     f.flags |= DN_INFERENCE;
   }
   Tensor scratch = bytes_on(q, abi.scratch_bytes(&f, 0, 0));
+  require_dense({&out, &fin, &scratch});
   check(abi.chunk_fwd(&f, ptr(q), ptr(k), ptr(v), ptr(g), ptr(b), ptr(w), static_cast<const int32_t*>(ptr(seg)),
                       static_cast<const float*>(ptr(init)), out.mutable_data_ptr(), want_final ? fin.mutable_data_ptr<float>() : nullptr,
                       kept ? &res : nullptr, scratch.mutable_data_ptr(), scratch.numel(), stream()),
@@ -74,7 +99,31 @@ variable_list forward(const dn_shape& shape, const Tensor& q, const Tensor& k, c
   return {out};
 }
 
-// The differentiable operator boundary (reference: gdn2.py:1461-1766).
+// its adjoint: the gradients of q, k, v, g, b, w and the initial state
+variable_list backward(const dn_shape& shape, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& b,
+                       const Tensor& w, const Tensor& init, const Tensor& seg, const Tensor& kept, const Tensor& d_out_in, const Tensor& d_final_in) {
+  require_dense({&q, &k, &v, &g, &b, &w, &init, &seg, &kept});
+  Tensor d_out = d_out_in.defined() ? d_out_in.to(q.scalar_type()).resolve_neg().contiguous()
+                                    : at::zeros({shape.B, shape.L, shape.Hv, shape.V}, q.options().requires_grad(false));
+  Tensor d_final;
+  if (d_final_in.defined()) d_final = d_final_in.to(at::kFloat).resolve_neg().contiguous();
+  auto like = [](const Tensor& t) { return at::empty(t.sizes(), t.options().requires_grad(false)); };
+  Tensor dq = like(q), dk = like(k), dv = like(v), dg = like(g), db = like(b), dw = like(w), d_init;
+  if (init.defined()) d_init = like(init);
+  dn_residuals res;
+  if (kept.defined()) check(abi.residual_carve(&shape, const_cast<void*>(kept.const_data_ptr()), &res), "dn_residual_carve");
+  Tensor scratch = bytes_on(q, abi.scratch_bytes(&shape, 1, kept.defined() ? 0 : 1));
+  require_dense({&d_out, &d_final, &dq, &scratch});
+  check(abi.chunk_bwd(&shape, ptr(q), ptr(k), ptr(v), ptr(g), ptr(b), ptr(w), static_cast<const int32_t*>(ptr(seg)),
+                      static_cast<const float*>(ptr(init)), kept.defined() ? &res : nullptr, ptr(d_out),
+                      static_cast<const float*>(ptr(d_final)), dq.mutable_data_ptr(), dk.mutable_data_ptr(), dv.mutable_data_ptr(),
+                      dg.mutable_data_ptr(), db.mutable_data_ptr(), dw.mutable_data_ptr(),
+                      d_init.defined() ? d_init.mutable_data_ptr<float>() : nullptr, scratch.mutable_data_ptr(), scratch.numel(), stream()),
+        "dn_chunk_bwd");
+  return {dq, dk, dv, dg, db, dw, d_init};
+}
+
+// The differentiable operator boundary (reference: gdn2.py:1461-1766) of plain calls.
 struct ChunkOp : public torch::autograd::Function<ChunkOp> {
   static variable_list forward(AutogradContext* ctx, Variable q, Variable k, Variable v, Variable g, Variable b, Variable w,
                                std::optional<Tensor> init_in, std::optional<Tensor> seg_in, std::string shape_bytes, bool want_final,
@@ -86,7 +135,10 @@ struct ChunkOp : public torch::autograd::Function<ChunkOp> {
     variable_list r = ::forward(shape, q, k, v, g, b, w, init, seg, want_final, inference || recompute ? nullptr : &kept);
     ctx->saved_data["shape"] = shape_bytes;
     ctx->saved_data["inference"] = inference;
-    ctx->save_for_backward({q, k, v, g, b, w, init, seg, kept});
+    // The residuals are no tensor of the user's and do not pass through saved-tensor hooks: a hook that stores tensors in fewer
+    // bits would turn the block of bytes into others.
+    ctx->saved_data["kept"] = kept;
+    ctx->save_for_backward({q, k, v, g, b, w, init, seg});
     ctx->set_materialize_grads(false);
     return r;
   }
@@ -98,33 +150,24 @@ struct ChunkOp : public torch::autograd::Function<ChunkOp> {
     const std::string bytes = ctx->saved_data["shape"].toStringRef();
     std::memcpy(&shape, bytes.data(), sizeof(shape));
     const variable_list s = ctx->get_saved_variables();
-    const Tensor &q = s[0], &k = s[1], &v = s[2], &g = s[3], &b = s[4], &w = s[5], &init = s[6], &seg = s[7], &kept = s[8];
-    Tensor d_out = grads[0].defined() ? grads[0].to(q.scalar_type()).contiguous()
-                                      : at::zeros({shape.B, shape.L, shape.Hv, shape.V}, q.options().requires_grad(false));
-    Tensor d_final;
-    if (grads.size() > 1 && grads[1].defined()) d_final = grads[1].to(at::kFloat).contiguous();
-    auto like = [](const Tensor& t) { return at::empty(t.sizes(), t.options().requires_grad(false)); };
-    Tensor dq = like(q), dk = like(k), dv = like(v), dg = like(g), db = like(b), dw = like(w), d_init;
-    if (init.defined()) d_init = like(init);
-    dn_residuals res;
-    if (kept.defined()) check(abi.residual_carve(&shape, const_cast<void*>(kept.const_data_ptr()), &res), "dn_residual_carve");
-    Tensor scratch = bytes_on(q, abi.scratch_bytes(&shape, 1, kept.defined() ? 0 : 1));
-    check(abi.chunk_bwd(&shape, ptr(q), ptr(k), ptr(v), ptr(g), ptr(b), ptr(w), static_cast<const int32_t*>(ptr(seg)),
-                        static_cast<const float*>(ptr(init)), kept.defined() ? &res : nullptr, ptr(d_out),
-                        static_cast<const float*>(ptr(d_final)), dq.mutable_data_ptr(), dk.mutable_data_ptr(), dv.mutable_data_ptr(),
-                        dg.mutable_data_ptr(), db.mutable_data_ptr(), dw.mutable_data_ptr(),
-                        d_init.defined() ? d_init.mutable_data_ptr<float>() : nullptr, scratch.mutable_data_ptr(), scratch.numel(), stream()),
-          "dn_chunk_bwd");
-    return {dq, dk, dv, dg, db, dw, d_init, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    variable_list d = ::backward(shape, s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7], ctx->saved_data["kept"].toTensor(), grads[0],
+                                 grads.size() > 1 ? grads[1] : Tensor());
+    if (!torch::autograd::get_current_graph_task_keep_graph()) ctx->saved_data.erase("kept");      // goes when the saved tensors do
+    d.resize(12);
+    return d;
   }
 };
 
+bool wants_grad(std::initializer_list<const Tensor*> ts) {
+  if (!at::GradMode::is_enabled()) return false;
+  for (const Tensor* t : ts)
+    if (t->defined() && t->requires_grad()) return true;
+  return false;
+}
+
 variable_list run(const dn_shape& shape, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& b, const Tensor& w,
-                  const Tensor& init, const Tensor& seg, bool want_final, bool recompute, bool inference, Tensor out = Tensor()) {
-  const bool grad = at::GradMode::is_enabled() &&
-                    (q.requires_grad() || k.requires_grad() || v.requires_grad() || g.requires_grad() || b.requires_grad() ||
-                     w.requires_grad() || (init.defined() && init.requires_grad()));
-  if (!grad) return forward(shape, q, k, v, g, b, w, init, seg, want_final, nullptr, out);
+                  const Tensor& init, const Tensor& seg, bool want_final, bool recompute, bool inference) {
+  if (!wants_grad({&q, &k, &v, &g, &b, &w, &init})) return forward(shape, q, k, v, g, b, w, init, seg, want_final, nullptr);
   auto opt = [](const Tensor& t) { return t.defined() ? std::optional<Tensor>(t) : std::nullopt; };
   return ChunkOp::apply(q, k, v, g, b, w, opt(init), opt(seg), std::string(reinterpret_cast<const char*>(&shape), sizeof(shape)), want_final,
                         recompute, inference);
@@ -162,7 +205,7 @@ PyObject* py_chunk(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (int i = 6; i < 9; ++i)
     if (a[i] != Py_None && !THPVariable_Check(a[i])) Py_RETURN_NONE;
   const Tensor ids = tensor_or_none(a[6]), cu = tensor_or_none(a[7]), init = tensor_or_none(a[8]);
-  if (!q.is_cuda()) Py_RETURN_NONE;
+  if (!q.is_cuda() || watched()) Py_RETURN_NONE;
   for (const Tensor* t : {&q, &k, &v, &g, &b, &w})
     if (!plain(*t, q)) Py_RETURN_NONE;
   if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || q.sizes() != k.sizes()) Py_RETURN_NONE;
@@ -173,6 +216,8 @@ PyObject* py_chunk(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (qdt < 0 || gdt < 0 || code(k.scalar_type()) != qdt || code(v.scalar_type()) != qdt || code(b.scalar_type()) != gdt ||
       code(w.scalar_type()) != gdt)
     Py_RETURN_NONE;
+  for (const Tensor* t : {&q, &k, &v, &g, &b, &w, &init})
+    if (tangent(*t)) Py_RETURN_NONE;
   dn_shape s{};
   if (!gate(g, 2, B, Lq, Hk, Hv, K, s.g_heads, s.g_cols) || !gate(b, 2, B, Lq, Hk, Hv, K, s.b_heads, s.b_cols) ||
       !gate(w, 2, B, Lq, Hk, Hv, V, s.w_heads, s.w_cols))
@@ -205,16 +250,49 @@ PyObject* py_chunk(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// apply(q, k, v, g, b, w, initial_state, seg, shape bytes, want_final, recompute, inference, out): prepared tensors, canonical
-// ids; out: a contiguous tensor for the outputs, or None (not used where a gradient is wanted)
-PyObject* py_apply(PyObject*, PyObject* const* a, Py_ssize_t n) {
+// The two directions on prepared tensors and canonical ids, without autograd.
+bool shape_of(PyObject* o, dn_shape* s) {
+  if (!PyBytes_Check(o) || PyBytes_GET_SIZE(o) != (Py_ssize_t)sizeof(dn_shape)) return false;
+  std::memcpy(s, PyBytes_AS_STRING(o), sizeof(dn_shape));
+  return true;
+}
+PyObject* tuple_of(const variable_list& r) {                                     // (an undefined tensor is None)
+  PyObject* t = PyTuple_New((Py_ssize_t)r.size());
+  for (size_t i = 0; i < r.size(); ++i) PyTuple_SET_ITEM(t, (Py_ssize_t)i, THPVariable_Wrap(r[i]));
+  return t;
+}
+// forward(q, k, v, g, b, w, initial_state, seg, shape bytes, want_final, keep, out) -> (out, final | None, residuals | None);
+// out: a contiguous tensor for the outputs, or None
+PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  TORCH_CHECK_VALUE(n == 13 && all_tensors(a, 6) && PyBytes_Check(a[8]) && PyBytes_GET_SIZE(a[8]) == (Py_ssize_t)sizeof(dn_shape), "apply: bad arguments");
   dn_shape s;
-  std::memcpy(&s, PyBytes_AS_STRING(a[8]), sizeof(s));
-  return wrap(run(s, THPVariable_Unpack(a[0]), THPVariable_Unpack(a[1]), THPVariable_Unpack(a[2]), THPVariable_Unpack(a[3]),
-                  THPVariable_Unpack(a[4]), THPVariable_Unpack(a[5]), tensor_or_none(a[6]), tensor_or_none(a[7]), a[9] == Py_True,
-                  a[10] == Py_True, a[11] == Py_True, tensor_or_none(a[12])));
+  TORCH_CHECK_VALUE(n == 12 && all_tensors(a, 6) && shape_of(a[8], &s), "forward: bad arguments");
+  Tensor kept;
+  variable_list r = forward(s, THPVariable_Unpack(a[0]), THPVariable_Unpack(a[1]), THPVariable_Unpack(a[2]), THPVariable_Unpack(a[3]),
+                            THPVariable_Unpack(a[4]), THPVariable_Unpack(a[5]), tensor_or_none(a[6]), tensor_or_none(a[7]), a[9] == Py_True,
+                            a[10] == Py_True ? &kept : nullptr, tensor_or_none(a[11]));
+  return tuple_of({r[0], r.size() > 1 ? r[1] : Tensor(), kept});
+  END_HANDLE_TH_ERRORS
+}
+// backward(q, k, v, g, b, w, initial_state, seg, residuals, d_out, d_final, shape bytes) -> the seven gradients
+PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  dn_shape s;
+  TORCH_CHECK_VALUE(n == 12 && all_tensors(a, 6) && shape_of(a[11], &s), "backward: bad arguments");
+  return tuple_of(backward(s, THPVariable_Unpack(a[0]), THPVariable_Unpack(a[1]), THPVariable_Unpack(a[2]), THPVariable_Unpack(a[3]),
+                           THPVariable_Unpack(a[4]), THPVariable_Unpack(a[5]), tensor_or_none(a[6]), tensor_or_none(a[7]),
+                           tensor_or_none(a[8]), tensor_or_none(a[9]), tensor_or_none(a[10])));
+  END_HANDLE_TH_ERRORS
+}
+// bare(*tensors): may a call on them pass autograd by?  No gradient is wanted, and nothing follows it.
+PyObject* py_bare(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (watched()) Py_RETURN_FALSE;
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    const Tensor t = tensor_or_none(a[i]);
+    if (t.defined() && (!dense(t) || tangent(t) || wants_grad({&t}))) Py_RETURN_FALSE;
+  }
+  Py_RETURN_TRUE;
   END_HANDLE_TH_ERRORS
 }
 
@@ -228,7 +306,7 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor g = THPVariable_Unpack(a[3]), b = THPVariable_Unpack(a[4]), w = THPVariable_Unpack(a[5]), state = THPVariable_Unpack(a[6]);
   const Tensor reset = tensor_or_none(a[7]);
   Tensor next = tensor_or_none(a[12]);
-  if (!q.is_cuda()) Py_RETURN_NONE;
+  if (!q.is_cuda() || watched()) Py_RETURN_NONE;
   for (const Tensor* t : {&q, &k, &v, &g, &b, &w, &state})
     if (!plain(*t, q)) Py_RETURN_NONE;
   if (q.dim() != 3 || k.dim() != 3 || v.dim() != 3 || q.sizes() != k.sizes() || state.dim() != 4) Py_RETURN_NONE;
@@ -309,7 +387,9 @@ PyObject* py_bind(PyObject*, PyObject* d) {
 
 PyMethodDef methods[] = {
     {"chunk", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_chunk)), METH_FASTCALL, nullptr},
-    {"apply", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_apply)), METH_FASTCALL, nullptr},
+    {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_forward)), METH_FASTCALL, nullptr},
+    {"backward", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_backward)), METH_FASTCALL, nullptr},
+    {"bare", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_bare)), METH_FASTCALL, nullptr},
     {"decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_decode)), METH_FASTCALL, nullptr},
     {"plain", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_plain)), METH_FASTCALL, nullptr},
     {"bind", py_bind, METH_O, nullptr},

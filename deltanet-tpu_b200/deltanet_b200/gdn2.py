@@ -62,9 +62,45 @@ def _common_dtype(ts: Sequence[torch.Tensor]) -> torch.dtype:
     return torch.float32
 
 
+def _prepared(t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """The tensor as its memory is handed to the kernels: of `dtype`, contiguous, with the sign that it stands for."""
+    return t.to(dtype).resolve_neg().contiguous()
+
+
 def _gate_layout(x: torch.Tensor, width: int):
     """(heads, cols) of a gate given as (B,L,H) or (B,L,H,1|width)."""
     return (x.shape[2], 1) if x.dim() == 3 else (x.shape[2], x.shape[3])
+
+
+# --------------------------------------------------------------------------------------------
+class _ChunkOp(torch.autograd.Function):
+    """The differentiable operator boundary (reference: gdn2.py:1461-1766) of the calls that the native path leaves to the
+    general one; transforms, tracers and modes see this function."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, g, b, w, init_state, seg, shape, want_final, recompute, inference):
+        keep = not inference and not recompute and any(ctx.needs_input_grad[:7])
+        ctx.shape, ctx.inference = shape, inference
+        out, final, ctx.kept = L.host().forward(q, k, v, g, b, w, init_state, seg, shape, want_final, keep, None)
+        ctx.save_for_backward(q, k, v, g, b, w, init_state, seg)
+        ctx.set_materialize_grads(False)
+        return (out, final) if want_final else out
+
+    @staticmethod
+    def backward(ctx, d_out, d_final=None):
+        if ctx.inference:
+            raise ValueError("chunk_gdn2: differentiation is not supported when is_inference=True; "
+                             "set is_inference=False for training.")
+        q, k, v, g, b, w, init_state, seg = ctx.saved_tensors
+        return L.host().backward(q, k, v, g, b, w, init_state, seg, ctx.kept, d_out, d_final, ctx.shape) + (None,) * 5
+
+
+def _chunk(q, k, v, g, b, w, init_state, seg, shape, want_final, recompute, inference, out=None):
+    """(out, final | None) of prepared tensors; `out`, a contiguous tensor, takes the outputs where nothing follows the call."""
+    if L.host().bare(q, k, v, g, b, w, init_state):
+        return L.host().forward(q, k, v, g, b, w, init_state, seg, bytes(shape), want_final, False, out)[:2]
+    r = _ChunkOp.apply(q, k, v, g, b, w, init_state, seg, bytes(shape), want_final, recompute, inference)
+    return r if want_final else (r, None)
 
 
 _PLAIN_PRECISION = {"bf16": L.DN_PREC_BF16, "fp32": L.DN_PREC_FP32}
@@ -237,10 +273,10 @@ def chunk_gdn2(
     out_dtype = v.dtype
     qkv_dt = _common_dtype((q, k, v))
     gate_dt = _common_dtype((g, b, w))
-    q, k, v = (t.to(qkv_dt).contiguous() for t in (q, k, v))
-    g, b, w = (t.to(gate_dt).contiguous() for t in (g, b, w))
+    q, k, v = (_prepared(t, qkv_dt) for t in (q, k, v))
+    g, b, w = (_prepared(t, gate_dt) for t in (g, b, w))
     if initial_state is not None:
-        initial_state = initial_state.to(torch.float32).contiguous()
+        initial_state = _prepared(initial_state, torch.float32)
 
     first_is_new = None
     if initial_state is not None and initial_state_segment_id is not None:
@@ -283,27 +319,28 @@ def chunk_gdn2(
         for sb in range(0, Lq, prefill_block_size):
             eb = min(sb + prefill_block_size, Lq)
             seg_b = None if seg is None else seg[:, sb:eb] if sb == 0 else seg[:, sb:eb] - seg[:, sb - 1:sb]
-            o_b, state = L.host().apply(
+            block = None if out is None else out[:, sb:eb]
+            o_b, state = _chunk(
                 q[:, sb:eb].contiguous(), k[:, sb:eb].contiguous(), v[:, sb:eb].contiguous(),
                 g[:, sb:eb].contiguous(), b[:, sb:eb].contiguous(), w[:, sb:eb].contiguous(),
-                state, None if seg_b is None else seg_b.contiguous(), bytes(make_shape(eb - sb, state is not None)), True, False, True,
-                None if out is None else out[:, sb:eb])
+                state, None if seg_b is None else seg_b.contiguous(), make_shape(eb - sb, state is not None), True, False, True, block)
+            if o_b is not block:                        # a tensor of its own: joined at the end
+                out = None
             if stability_guard:
                 state = _cap_state(state, stability_tau)
             outs.append(o_b)
-        if out is None or outs[0].requires_grad:
+        if out is None:
             out = torch.cat(outs, dim=1)
         out = out.to(out_dtype)
         return (out, state) if output_final_state else out
 
-    res = L.host().apply(q, k, v, g, b, w, initial_state, seg, bytes(make_shape(Lq, initial_state is not None)),
-                         bool(output_final_state), bool(recompute_states), bool(is_inference), None)
+    out, final = _chunk(q, k, v, g, b, w, initial_state, seg, make_shape(Lq, initial_state is not None),
+                        bool(output_final_state), bool(recompute_states), bool(is_inference))
     if output_final_state:
-        out, final = res
         if stability_guard and is_inference:
             final = _cap_state(final, stability_tau)
         return out.to(out_dtype), final
-    return res.to(out_dtype)
+    return out.to(out_dtype)
 
 
 # --------------------------------------------------------------------------------------------
@@ -420,11 +457,9 @@ def gdn2_decode_step(
     out_dtype = v.dtype
     qkv_dt = _common_dtype((q, k, v))
     gate_dt = _common_dtype((g, b, w))
-    q, k, v = (t.to(qkv_dt).contiguous() for t in (q, k, v))
-    g, b, w = (t.to(gate_dt).contiguous() for t in (g, b, w))
-    if state.dtype not in _DT:
-        state = state.to(torch.float32)
-    state = state.contiguous()
+    q, k, v = (_prepared(t, qkv_dt) for t in (q, k, v))
+    g, b, w = (_prepared(t, gate_dt) for t in (g, b, w))
+    state = _prepared(state, state.dtype if state.dtype in _DT else torch.float32)
     lay = lambda x: (x.shape[1], 1) if x.dim() == 2 else (x.shape[1], x.shape[2])
     (gh, gc), (bh, bc), (wh, wc) = lay(g), lay(b), lay(w)
     flags = (L.DN_QK_L2NORM if qk_l2norm else 0) | (L.DN_STABILITY_GUARD if stability_guard else 0) | \
