@@ -2,6 +2,7 @@
 // and the order in which the kernels are enqueued.  Nothing here allocates device memory or
 // synchronises.
 #include <cstdlib>
+#include <initializer_list>
 #include <mutex>
 
 #include "dn_kernels.cuh"
@@ -59,6 +60,19 @@ int overlap_cut(const Geo& g) {
   const int cut = ((rounds - 1) * sms) / per_chunk;
   return (cut >= 1 && cut < g.NC) ? cut : 0;
 }
+// The tensor-core kernels move rows of the operator's tensors 16 bytes at a time, and images by bulk copies, which want the same.
+// (A gate of one value per head is read by elements.)
+bool aligned16(std::initializer_list<const void*> ps) {
+  uintptr_t bits = 0;
+  for (const void* p : ps) bits |= reinterpret_cast<uintptr_t>(p);
+  return (bits & 15) == 0;
+}
+bool rows_aligned(const Geo& g, const void* q, const void* k, const void* v, const void* g_, const void* b, const void* w) {
+  return !g.img || aligned16({q, k, v, g.gC > 1 ? g_ : nullptr, g.bC > 1 ? b : nullptr, g.wC > 1 ? w : nullptr});
+}
+bool images_aligned(const Geo& g, const dn_residuals& r) {
+  return !g.img || aligned16({r.W, r.U, r.M, r.qe, r.ke, r.lam_end, r.T, r.states});
+}
 size_t carry_bytes(const Geo& g) { return align_up((size_t)g.B * g.H * g.Kt * g.Vw * sizeof(float)); }
 }  // namespace
 
@@ -80,6 +94,7 @@ const char* dn_status_string(int st) {
     case DN_ERR_CUDA_LAUNCH: return "a CUDA kernel launch failed";
     case DN_ERR_UNSUPPORTED: return "unsupported combination of options";
     case DN_ERR_DEVICE_WAIT: return "an earlier kernel gave up a bounded wait (see dn_device_error / dn_device_error_reset)";
+    case DN_ERR_MISALIGNED: return "a buffer does not start at a multiple of 16 bytes, which the kernels for this shape need";
     case DN_ERR_STATIC_SCRATCH_EXCEEDED: return "this shape needs more scratch than the built-in static array (see dn_static_scratch_bytes)";
     default: return "unknown status";
   }
@@ -199,6 +214,7 @@ int dn_prepass_fwd(const dn_shape* s, const void* q, const void* k, const void* 
   if (peek_device_error()) return DN_ERR_DEVICE_WAIT;
   if (!q || !k || !v || !g_ || !b || !w || !res || !scratch) return DN_ERR_NULL_POINTER;
   if (!res->W || !res->U || !res->M || !res->qe || !res->ke || !res->lam_end) return DN_ERR_NULL_POINTER;
+  if (!rows_aligned(g, q, k, v, g_, b, w) || !images_aligned(g, *res)) return DN_ERR_MISALIGNED;
   return launch_prepass_fwd(g, q, k, v, g_, b, w, seg, *res, reinterpret_cast<float*>(scratch),
                             scratch_bytes / sizeof(float), (cudaStream_t)stream);
 }
@@ -211,6 +227,7 @@ int dn_state_fwd(const dn_shape* s, const dn_residuals* res, const int32_t* seg,
   if (peek_device_error()) return DN_ERR_DEVICE_WAIT;
   if (!res || (!out && !final_state && !res->states)) return DN_ERR_NULL_POINTER;
   if ((g.flags & DN_HAS_INIT) && !init_state) return DN_ERR_NULL_POINTER;
+  if (!images_aligned(g, *res) || (g.img && !aligned16({out}))) return DN_ERR_MISALIGNED;
   StateArgs a{};
   a.g = g; a.res = *res; a.seg = seg; a.init_state = (g.flags & DN_HAS_INIT) ? init_state : nullptr;
   a.out = out; a.final_state = final_state; a.states = res->states;
@@ -225,6 +242,7 @@ int dn_recompute_states(const dn_shape* s, const dn_residuals* res, const int32_
   if (peek_device_error()) return DN_ERR_DEVICE_WAIT;
   if (!res || !res->states) return DN_ERR_NULL_POINTER;
   if ((g.flags & DN_HAS_INIT) && !init_state) return DN_ERR_NULL_POINTER;
+  if (!images_aligned(g, *res)) return DN_ERR_MISALIGNED;
   StateArgs a{};
   a.g = g; a.res = *res; a.seg = seg; a.init_state = (g.flags & DN_HAS_INIT) ? init_state : nullptr;
   a.states = res->states;
@@ -240,6 +258,7 @@ int dn_state_bwd(const dn_shape* s, const dn_residuals* res, const int32_t* seg,
   if (peek_device_error()) return DN_ERR_DEVICE_WAIT;
   if (!res || !d_out || !dV || !dH) return DN_ERR_NULL_POINTER;
   if (g.img && !res->states) return DN_ERR_NULL_POINTER;      // dLambda_end is reduced in the reverse chain on this path
+  if (!images_aligned(g, *res) || (g.img && !aligned16({d_out, dV, dH}))) return DN_ERR_MISALIGNED;
   StateArgs a{};
   a.g = g; a.res = *res; a.seg = seg; a.d_out = d_out; a.d_final = d_final_state;
   a.dV = dV; a.dH = dH; a.d_init = (g.flags & DN_HAS_INIT) ? d_init : nullptr;
@@ -260,6 +279,9 @@ int plan_prepass_bwd(const Geo& g, const void* q, const void* k, const void* v, 
                      const void* d_out, const float* dV, const float* dH,
                      void* dq, void* dk, void* dv, void* dg, void* db, void* dw,
                      char* p, size_t bytes, BwdPlan& pl) {
+  if (!rows_aligned(g, q, k, v, g_, b, w) || !rows_aligned(g, dq, dk, dv, dg, db, dw) || !images_aligned(g, res) ||
+      (g.img && !aligned16({d_out, dV, dH, p})))
+    return DN_ERR_MISALIGNED;
   const size_t rows = (size_t)g.B * g.L;
   char* end = p + bytes;
   PrepassBwdArgs& a = pl.a;
@@ -336,6 +358,7 @@ int dn_chunk_fwd(const dn_shape* s, const void* q, const void* k, const void* v,
   if (peek_device_error()) return DN_ERR_DEVICE_WAIT;
   if (!q || !k || !v || !g_ || !b || !w || !out || !scratch) return DN_ERR_NULL_POINTER;
   if ((g.flags & DN_HAS_INIT) && !init_state) return DN_ERR_NULL_POINTER;
+  if (!rows_aligned(g, q, k, v, g_, b, w) || (res && !images_aligned(g, *res)) || (g.img && !aligned16({out, scratch}))) return DN_ERR_MISALIGNED;
   char* p = reinterpret_cast<char*>(scratch);
   char* end = p + scratch_bytes;
   dn_residuals local;
@@ -392,6 +415,9 @@ int dn_chunk_bwd(const dn_shape* s, const void* q, const void* k, const void* v,
   if (!q || !k || !v || !g_ || !b || !w || !d_out || !scratch) return DN_ERR_NULL_POINTER;
   if (!dq || !dk || !dv || !dg || !db || !dw) return DN_ERR_NULL_POINTER;
   if (g.flags & DN_INFERENCE) return DN_ERR_UNSUPPORTED;
+  if (!rows_aligned(g, q, k, v, g_, b, w) || !rows_aligned(g, dq, dk, dv, dg, db, dw) || (res && !images_aligned(g, *res)) ||
+      (g.img && !aligned16({d_out, scratch})))
+    return DN_ERR_MISALIGNED;
   cudaStream_t st = (cudaStream_t)stream;
   char* p = reinterpret_cast<char*>(scratch);
   char* end = p + scratch_bytes;
@@ -460,6 +486,7 @@ int dn_sp_transition(const dn_shape* s, const dn_residuals* res, const int32_t* 
   if (rc) return rc;
   if (peek_device_error()) return DN_ERR_DEVICE_WAIT;
   if (!res || !identity || !P) return DN_ERR_NULL_POINTER;
+  if (!images_aligned(g, *res)) return DN_ERR_MISALIGNED;
   Geo t = g;                       // same chunks and heads, value width K, one "value head" per exec head
   t.Hv = g.H; t.G = 1; t.V = g.K; t.Vw = g.Kt; t.qk_div = 1;
   t.flags |= DN_HAS_INIT;
@@ -480,6 +507,7 @@ int dn_sp_summary(const dn_shape* s, const dn_residuals* res, const int32_t* seg
   if (peek_device_error()) return DN_ERR_DEVICE_WAIT;
   if (!res || !Q || !P) return DN_ERR_NULL_POINTER;
   if (!res->W || !res->U || !res->ke || !res->lam_end || (out && (!res->M || !res->qe))) return DN_ERR_NULL_POINTER;
+  if (!images_aligned(g, *res) || (g.img && !aligned16({out}))) return DN_ERR_MISALIGNED;
   StateArgs a{};
   a.g = g; a.res = *res; a.seg = seg; a.init_state = nullptr;
   a.out = out; a.final_state = Q; a.states = res->states; a.P_out = P;
@@ -496,6 +524,7 @@ int dn_sp_correct_fwd(const dn_shape* s, const dn_residuals* res, const int32_t*
   if (peek_device_error()) return DN_ERR_DEVICE_WAIT;
   if (!res || !S_in || (!out && !res->states)) return DN_ERR_NULL_POINTER;
   if (!(g.flags & DN_HAS_INIT)) return DN_ERR_UNSUPPORTED;
+  if (!images_aligned(g, *res) || (g.img && !aligned16({out}))) return DN_ERR_MISALIGNED;
   StateArgs a{};
   a.g = g; a.res = *res; a.seg = seg; a.init_state = S_in;
   a.out = out; a.states = res->states; a.until_independent = true;
@@ -511,6 +540,7 @@ int dn_sp_correct_bwd(const dn_shape* s, const dn_residuals* res, const int32_t*
   if (peek_device_error()) return DN_ERR_DEVICE_WAIT;
   if (!res || !d_out || !d_final_state || !dV || !dH) return DN_ERR_NULL_POINTER;
   if (g.img && !res->states) return DN_ERR_NULL_POINTER;
+  if (!images_aligned(g, *res) || (g.img && !aligned16({d_out, dV, dH}))) return DN_ERR_MISALIGNED;
   StateArgs a{};
   a.g = g; a.res = *res; a.seg = seg; a.d_out = d_out; a.d_final = d_final_state;
   a.dV = dV; a.dH = dH; a.until_independent = true;
@@ -547,6 +577,7 @@ int dn_decode_step(const dn_decode_shape* s, const void* q, const void* k, const
   if (!okh(s->g_heads) || !okh(s->b_heads) || !okh(s->w_heads)) return DN_ERR_BAD_SHAPE;
   if ((s->g_cols != 1 && s->g_cols != s->K) || (s->b_cols != 1 && s->b_cols != s->K) ||
       (s->w_cols != 1 && s->w_cols != s->V)) return DN_ERR_BAD_SHAPE;
+  if (!aligned16({state_in, state_out})) return DN_ERR_MISALIGNED;
   if (state_in == state_out && s->state_in_dtype != s->state_out_dtype) return DN_ERR_UNSUPPORTED;
   if (peek_device_error()) return DN_ERR_DEVICE_WAIT;
   return launch_decode(*s, q, k, v, g_, b, w, state_in, reset, out, state_out, (cudaStream_t)stream);

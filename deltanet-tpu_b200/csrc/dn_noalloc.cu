@@ -49,6 +49,14 @@ int dn_prepass_fwd_static(const dn_shape* s, const void* q, const void* k, const
   if (dn::peek_device_error()) return DN_ERR_DEVICE_WAIT;
   if (!q || !k || !v || !g_ || !b || !w || !res) return DN_ERR_NULL_POINTER;
   if (!res->W || !res->U || !res->M || !res->qe || !res->ke || !res->lam_end) return DN_ERR_NULL_POINTER;
+  if (g.img) {                                    // as in dn_prepass_fwd: rows and images are moved 16 bytes at a time
+    uintptr_t bits = 0;
+    for (const void* p : {q, k, v, (const void*)(g.gC > 1 ? g_ : nullptr), (const void*)(g.bC > 1 ? b : nullptr), (const void*)(g.wC > 1 ? w : nullptr),
+                          (const void*)res->W, (const void*)res->U, (const void*)res->M, (const void*)res->qe, (const void*)res->ke,
+                          (const void*)res->lam_end, (const void*)res->T})
+      bits |= reinterpret_cast<uintptr_t>(p);
+    if (bits & 15) return DN_ERR_MISALIGNED;
+  }
   if (dn::prepass_fwd_scratch_floats(g) * sizeof(float) > DN_STATIC_SCRATCH_BYTES) return DN_ERR_STATIC_SCRATCH_EXCEEDED;
   void* scratch = nullptr;
   if ((rc = static_scratch(&scratch))) return rc;

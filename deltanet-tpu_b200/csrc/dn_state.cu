@@ -442,9 +442,13 @@ static int launch_bwd(const StateArgs& a, cudaStream_t st) {
   return launch_status();
 }
 
-// fp32 residuals and products, and room for a chunk's factors (all but 128 x 128).
-static bool staged(const Geo& g) {
-  return g.pre_dt == DN_F32 && !g.state_bf16() && !g.bf16_mode() && !(g.C == 128 && g.K == 128);
+// fp32 residuals and products, room for a chunk's factors (all but 128 x 128), and factors that 16-byte copies can fetch.
+static bool staged(const StateArgs& a) {
+  const Geo& g = a.g;
+  uintptr_t bits = 0;
+  for (const void* p : {(const void*)a.res.W, (const void*)a.res.qe, (const void*)a.res.ke, (const void*)a.res.M, (const void*)a.res.lam_end})
+    bits |= reinterpret_cast<uintptr_t>(p);
+  return g.pre_dt == DN_F32 && !g.state_bf16() && !g.bf16_mode() && !(g.C == 128 && g.K == 128) && (bits & 15) == 0;
 }
 template <int C, int K>
 static int launch_staged(const StateArgs& a, bool bwd, cudaStream_t st) {
@@ -461,13 +465,13 @@ static int launch_staged(const StateArgs& a, bool bwd, cudaStream_t st) {
 
 int launch_state_fwd(const StateArgs& a, cudaStream_t st) {
   if (state_tc_eligible(a.g) && !force_simt()) return launch_state_fwd_tc(a, st);
-  if (staged(a.g)) return launch_staged(a, false, st);
+  if (staged(a)) return launch_staged(a, false, st);
   return narrow(a.g) ? launch_fwd<16>(a, st) : launch_fwd<64>(a, st);
 }
 
 int launch_state_bwd(const StateArgs& a, cudaStream_t st) {
   if (state_tc_eligible(a.g) && !force_simt()) return launch_state_bwd_tc(a, st);
-  if (staged(a.g)) return launch_staged(a, true, st);
+  if (staged(a)) return launch_staged(a, true, st);
   return narrow(a.g) ? launch_bwd<16>(a, st) : launch_bwd<64>(a, st);
 }
 

@@ -59,6 +59,9 @@ bool dense(const Tensor& t) {
 }
 // Can a kernel take the tensor as it is, beside `q`?  (What is not on q's device the general path moves or refuses.)
 bool plain(const Tensor& t, const Tensor& q) { return dense(t) && t.device() == q.device() && t.is_contiguous(); }
+// The kernels read and write the operator's tensors 16 bytes at a time.  A view at an odd offset is copied first.
+bool at16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(ptr(t)) & 15) == 0; }
+Tensor aligned(const Tensor& t) { return !t.defined() || at16(t) ? t : t.clone(at::MemoryFormat::Contiguous); }
 // Does something follow the calls of this thread that an address would escape?
 bool watched() { return torch::jit::tracer::isTracing() || c10::impl::TorchDispatchModeTLS::any_modes_set(); }
 bool tangent(const Tensor& t) { return t.defined() && t._fw_grad(0).defined(); }
@@ -74,9 +77,10 @@ Tensor bytes_on(const Tensor& like, size_t n) {
 }
 
 // the forward; keeps the residuals in *kept when asked
-variable_list forward(const dn_shape& shape, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& b,
-                      const Tensor& w, const Tensor& init, const Tensor& seg, bool want_final, Tensor* kept, Tensor out = Tensor()) {
-  require_dense({&q, &k, &v, &g, &b, &w, &init, &seg});
+variable_list forward(const dn_shape& shape, const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const Tensor& g_in, const Tensor& b_in,
+                      const Tensor& w_in, const Tensor& init, const Tensor& seg, bool want_final, Tensor* kept, Tensor out = Tensor()) {
+  require_dense({&q_in, &k_in, &v_in, &g_in, &b_in, &w_in, &init, &seg});
+  const Tensor q = aligned(q_in), k = aligned(k_in), v = aligned(v_in), g = aligned(g_in), b = aligned(b_in), w = aligned(w_in);
   if (!out.defined()) out = at::empty({shape.B, shape.L, shape.Hv, shape.V}, q.options().requires_grad(false));
   Tensor fin;
   if (want_final) fin = at::empty({shape.B, shape.Hv, shape.K, shape.V}, q.options().dtype(at::kFloat).requires_grad(false));
@@ -100,10 +104,11 @@ variable_list forward(const dn_shape& shape, const Tensor& q, const Tensor& k, c
 }
 
 // its adjoint: the gradients of q, k, v, g, b, w and the initial state
-variable_list backward(const dn_shape& shape, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& b,
-                       const Tensor& w, const Tensor& init, const Tensor& seg, const Tensor& kept, const Tensor& d_out_in, const Tensor& d_final_in) {
-  require_dense({&q, &k, &v, &g, &b, &w, &init, &seg, &kept});
-  Tensor d_out = d_out_in.defined() ? d_out_in.to(q.scalar_type()).resolve_neg().contiguous()
+variable_list backward(const dn_shape& shape, const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const Tensor& g_in, const Tensor& b_in,
+                       const Tensor& w_in, const Tensor& init, const Tensor& seg, const Tensor& kept, const Tensor& d_out_in, const Tensor& d_final_in) {
+  require_dense({&q_in, &k_in, &v_in, &g_in, &b_in, &w_in, &init, &seg, &kept});
+  const Tensor q = aligned(q_in), k = aligned(k_in), v = aligned(v_in), g = aligned(g_in), b = aligned(b_in), w = aligned(w_in);
+  Tensor d_out = d_out_in.defined() ? aligned(d_out_in.to(q.scalar_type()).resolve_neg().contiguous())
                                     : at::zeros({shape.B, shape.L, shape.Hv, shape.V}, q.options().requires_grad(false));
   Tensor d_final;
   if (d_final_in.defined()) d_final = d_final_in.to(at::kFloat).resolve_neg().contiguous();
@@ -303,11 +308,12 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 13 || !all_tensors(a, 7)) Py_RETURN_NONE;
   if ((a[7] != Py_None && !THPVariable_Check(a[7])) || (a[12] != Py_None && !THPVariable_Check(a[12]))) Py_RETURN_NONE;
   const Tensor q = THPVariable_Unpack(a[0]), k = THPVariable_Unpack(a[1]), v = THPVariable_Unpack(a[2]);
-  const Tensor g = THPVariable_Unpack(a[3]), b = THPVariable_Unpack(a[4]), w = THPVariable_Unpack(a[5]), state = THPVariable_Unpack(a[6]);
+  const Tensor g = THPVariable_Unpack(a[3]), b = THPVariable_Unpack(a[4]), w = THPVariable_Unpack(a[5]);
+  Tensor state = THPVariable_Unpack(a[6]);
   const Tensor reset = tensor_or_none(a[7]);
   Tensor next = tensor_or_none(a[12]);
   if (!q.is_cuda() || watched()) Py_RETURN_NONE;
-  for (const Tensor* t : {&q, &k, &v, &g, &b, &w, &state})
+  for (const Tensor* t : std::initializer_list<const Tensor*>{&q, &k, &v, &g, &b, &w, &state})
     if (!plain(*t, q)) Py_RETURN_NONE;
   if (q.dim() != 3 || k.dim() != 3 || v.dim() != 3 || q.sizes() != k.sizes() || state.dim() != 4) Py_RETURN_NONE;
   const int64_t B = q.size(0), Hk = q.size(1), K = q.size(2), Hv = v.size(1), V = v.size(2);
@@ -342,9 +348,10 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!next.defined()) {
     next = at::empty({B, Hv, K, V}, state.options().dtype(st).requires_grad(false));
     next_py = nullptr;
-  } else if (!plain(next, q) || next.scalar_type() != st || next.sizes() != state.sizes()) {
+  } else if (!plain(next, q) || !at16(next) || next.scalar_type() != st || next.sizes() != state.sizes()) {
     Py_RETURN_NONE;
   }
+  state = aligned(state);
   Tensor o = at::empty({B, Hv, V}, q.options().requires_grad(false));
   check(abi.decode_step(&s, ptr(q), ptr(k), ptr(v), ptr(g), ptr(b), ptr(w), ptr(state), static_cast<const uint8_t*>(ptr(reset)),
                         o.mutable_data_ptr(), const_cast<void*>(next.const_data_ptr()), stream()),
@@ -361,6 +368,15 @@ PyObject* py_plain(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK_VALUE(n == 2 && all_tensors(a, 2), "plain: two tensors");
   return PyBool_FromLong(plain(THPVariable_Unpack(a[0]), THPVariable_Unpack(a[1])));
+  END_HANDLE_TH_ERRORS
+}
+
+// aligned(t): t itself, or a copy of it that starts at a multiple of 16 bytes
+PyObject* py_aligned(PyObject*, PyObject* o) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK_VALUE(THPVariable_Check(o), "aligned: a tensor");
+  const Tensor& t = THPVariable_Unpack(o);
+  return at16(t) ? Py_NewRef(o) : THPVariable_Wrap(aligned(t));
   END_HANDLE_TH_ERRORS
 }
 
@@ -392,6 +408,7 @@ PyMethodDef methods[] = {
     {"bare", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_bare)), METH_FASTCALL, nullptr},
     {"decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_decode)), METH_FASTCALL, nullptr},
     {"plain", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_plain)), METH_FASTCALL, nullptr},
+    {"aligned", py_aligned, METH_O, nullptr},
     {"bind", py_bind, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -67,6 +67,11 @@ def _prepared(t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     return t.to(dtype).resolve_neg().contiguous()
 
 
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """The tensor, or a copy where it starts at an odd offset: the kernels read 16 bytes at a time."""
+    return L.host().aligned(t)
+
+
 def _gate_layout(x: torch.Tensor, width: int):
     """(heads, cols) of a gate given as (B,L,H) or (B,L,H,1|width)."""
     return (x.shape[2], 1) if x.dim() == 3 else (x.shape[2], x.shape[3])
@@ -459,15 +464,15 @@ def gdn2_decode_step(
     gate_dt = _common_dtype((g, b, w))
     q, k, v = (_prepared(t, qkv_dt) for t in (q, k, v))
     g, b, w = (_prepared(t, gate_dt) for t in (g, b, w))
-    state = _prepared(state, state.dtype if state.dtype in _DT else torch.float32)
+    state = _aligned(_prepared(state, state.dtype if state.dtype in _DT else torch.float32))
     lay = lambda x: (x.shape[1], 1) if x.dim() == 2 else (x.shape[1], x.shape[2])
     (gh, gc), (bh, bc), (wh, wc) = lay(g), lay(b), lay(w)
     flags = (L.DN_QK_L2NORM if qk_l2norm else 0) | (L.DN_STABILITY_GUARD if stability_guard else 0) | \
         (L.DN_RESET_PER_HEAD if reset_per_head else 0)
     if out_state is None:
         out_state = torch.empty(B, Hv, K, V, dtype=tgt, device=q.device)
-    elif out_state.dtype != tgt or tuple(out_state.shape) != (B, Hv, K, V) or not out_state.is_contiguous():
-        raise ValueError("out_state must be a contiguous (B, Hv, K, V) tensor of the target state dtype.")
+    elif out_state.dtype != tgt or tuple(out_state.shape) != (B, Hv, K, V) or not out_state.is_contiguous() or out_state.data_ptr() % 16:
+        raise ValueError("out_state must be a contiguous (B, Hv, K, V) tensor of the target state dtype that starts at a multiple of 16 bytes.")
     o = torch.empty(B, Hv, V, dtype=qkv_dt, device=q.device)
     ds = L.DecodeShape(B=B, Hk=Hk, Hv=Hv, K=K, V=V, g_heads=gh, g_cols=gc, b_heads=bh, b_cols=bc,
                        w_heads=wh, w_cols=wc, qkv_dtype=_DT[qkv_dt], gate_dtype=_DT[gate_dt],

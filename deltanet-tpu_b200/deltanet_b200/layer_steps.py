@@ -15,7 +15,7 @@ from typing import Optional
 import torch
 
 from . import _lib as L
-from .gdn2 import _DT, _ptr, _require_cuda, _stream
+from .gdn2 import _DT, _aligned, _prepared, _ptr, _require_cuda, _stream
 
 
 def _f32(t):
@@ -28,7 +28,7 @@ class _Producer(torch.autograd.Function):
         lib = L.lib()
         B, Lq, D = mixed.shape
         W = conv_w.shape[-1]
-        mixed = mixed.contiguous()
+        mixed = _aligned(mixed.contiguous())
         w32, b32 = _f32(conv_w.reshape(D, W)), _f32(conv_b)
         q = torch.empty(B, Lq, Hk, K, dtype=mixed.dtype, device=mixed.device)
         k = torch.empty_like(q)
@@ -46,7 +46,7 @@ class _Producer(torch.autograd.Function):
         lib = L.lib()
         mixed, w32, b32, seg = ctx.saved_tensors
         B, Lq, Hk, Hv, K, V, W, D = ctx.dims
-        dq, dk, dv = (t.to(mixed.dtype).contiguous() for t in (dq, dk, dv))
+        dq, dk, dv = (_aligned(_prepared(t, mixed.dtype)) for t in (dq, dk, dv))
         d_mixed = torch.empty_like(mixed)
         dw = torch.empty(D, W, dtype=torch.float32, device=mixed.device)
         db = torch.empty(D, dtype=torch.float32, device=mixed.device) if b32 is not None else None
@@ -137,7 +137,7 @@ class _GatedNorm(torch.autograd.Function):
     def forward(ctx, o, z, weight, eps):
         lib = L.lib()
         V = o.shape[-1]
-        o_, z_ = o.contiguous(), z.to(o.dtype).contiguous()
+        o_, z_ = _aligned(o.contiguous()), _aligned(z.to(o.dtype).contiguous())
         w32 = _f32(weight)
         rows = o_.numel() // V
         y = torch.empty_like(o_)
@@ -153,7 +153,7 @@ class _GatedNorm(torch.autograd.Function):
         o_, z_, w32 = ctx.saved_tensors
         V = o_.shape[-1]
         rows = o_.numel() // V
-        dy = dy.to(o_.dtype).contiguous()
+        dy = _aligned(_prepared(dy, o_.dtype))
         d_o, d_z = torch.empty_like(o_), torch.empty_like(z_)
         dw = torch.empty_like(w32)
         n = lib.dn_gated_rmsnorm_scratch_bytes(rows, V)

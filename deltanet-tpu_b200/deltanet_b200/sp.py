@@ -186,8 +186,8 @@ class CudaOps:
         B, Lq, Hk, K = q.shape
         Hv, V = v.shape[2], v.shape[3]
         qkv_dt, gate_dt = _g._common_dtype((q, k, v)), _g._common_dtype((g, b, w))
-        q, k, v = (t.to(qkv_dt).contiguous() for t in (q, k, v))
-        g, b, w = (t.to(gate_dt).contiguous() for t in (g, b, w))
+        q, k, v = (_g._aligned(_g._prepared(t, qkv_dt)) for t in (q, k, v))
+        g, b, w = (_g._aligned(_g._prepared(t, gate_dt)) for t in (g, b, w))
         gh, gc = _g._gate_layout(g, K)
         bh, bc = _g._gate_layout(b, K)
         wh, wc = _g._gate_layout(w, V)
@@ -271,7 +271,7 @@ class CudaOps:
                                             _g._stream()), "dn_recompute_states")
         ex, dev = c["ex"], d_out.device
         items = B * ex.H * ex.NC
-        c["d_out"] = d_out.to(c["ins"][2].dtype).contiguous()
+        c["d_out"] = _g._aligned(_g._prepared(d_out, c["ins"][2].dtype))
         c["dV"] = torch.empty(items * ex.chunk * ex.Vw, device=dev)
         c["dH"] = torch.empty(items * K * ex.Vw, device=dev)
         d_init0 = torch.empty(B, Hv, K, V, device=dev)

@@ -71,6 +71,7 @@ enum {
   DN_ERR_CUDA_LAUNCH = 5,    /* cudaGetLastError() after a launch was not cudaSuccess  */
   DN_ERR_UNSUPPORTED = 6,
   DN_ERR_STATIC_SCRATCH_EXCEEDED = 7, /* dn_prepass_fwd_static: the shape needs more scratch than the built-in array */
+  DN_ERR_MISALIGNED = 9,     /* a buffer that is moved 16 bytes at a time does not start at a multiple of 16 (below) */
   DN_ERR_DEVICE_WAIT = 8     /* an EARLIER kernel gave up a bounded wait: results since then are not to be
                                 trusted; nothing was enqueued by this call (see dn_device_error_reset)  */
 };
@@ -87,6 +88,13 @@ typedef struct dn_shape {
   uint32_t flags;
   float scale;                 /* query scale (already resolved, gdn2.py:1978) */
 } dn_shape;
+
+/*
+ * Alignment.  On the tensor-core path (precision bf16 without DN_STATE_FP32_MM, DN_FORCE_SIMT unset) q, k, v, out, d_out, dq,
+ * dk, dv, every gate given per channel and its gradient, the residual tiles, dV, dH and scratch start at multiples of 16
+ * bytes; so do the states of dn_decode_step in either precision.  Other buffers start at a multiple of their element.  A call
+ * that breaks this returns DN_ERR_MISALIGNED and enqueues nothing.
+ */
 
 /* Exec-head view of a shape (what the residual layouts are expressed in). */
 typedef struct dn_exec {

@@ -137,3 +137,75 @@ def test_saved_tensor_hooks_see_the_inputs_only(fn):
 def test_sign_views(fn):
     t = _inputs(6)
     assert torch.equal(fn(torch._neg_view(t[0]), *t[1:]), fn(-t[0], *t[1:]))
+
+
+# ---- addresses: rows are moved 16 bytes at a time
+def test_odd_offsets_are_copied(host):
+    flat = torch.arange(33, dtype=torch.float32)
+    even, odd = flat[:32].view(4, 8), flat[1:].view(4, 8)
+    assert host.aligned(even) is even and host.plain(odd, even)
+    got = host.aligned(odd)
+    assert got.data_ptr() % 16 == 0 and torch.equal(got, odd)
+
+
+@pytest.mark.parametrize("K,V", [(64, 64), (128, 128)])
+def test_misaligned_buffers_get_a_status(K, V):
+    """No address here is ever read: the status comes before anything is enqueued."""
+    lib, at = _lib.lib(), 1 << 20
+    s = _lib.Shape(B=1, L=64, Hk=1, Hv=1, K=K, V=V, chunk=128, g_heads=1, g_cols=K, b_heads=1, b_cols=K, w_heads=1, w_cols=V,
+                   qkv_dtype=_lib.DN_BF16, gate_dtype=_lib.DN_F32, precision=_lib.DN_PREC_BF16, flags=0, scale=1.0)
+    res = _lib.Residuals()
+    for odd in range(8):
+        a = [at + (2 if i == odd else 0) for i in range(8)]
+        assert lib.dn_chunk_fwd(s, *a[:6], None, None, a[6], None, None, a[7], 1 << 30, None) == 9
+    assert lib.dn_residual_carve(s, at + 8, res) == 0
+    assert lib.dn_prepass_fwd(s, *[at] * 6, None, res, at, 1 << 30, None) == 9
+    assert lib.dn_prepass_fwd_static(s, *[at] * 6, None, res, None) == 9
+    assert lib.dn_state_bwd(s, res, None, at, None, at, at, None, None) == 9
+    for odd in range(14):
+        a = [at + (2 if i == odd else 0) for i in range(14)]
+        assert lib.dn_chunk_bwd(s, *a[:6], None, None, None, a[6], None, *a[7:13], None, a[13], 1 << 30, None) == 9
+    d = _lib.DecodeShape(B=1, Hk=1, Hv=1, K=K, V=V, g_heads=1, g_cols=1, b_heads=1, b_cols=1, w_heads=1, w_cols=1, qkv_dtype=_lib.DN_F32,
+                         gate_dtype=_lib.DN_F32, state_in_dtype=_lib.DN_F32, state_out_dtype=_lib.DN_F32, flags=0, scale=1.0, stability_tau=1.0)
+    for i, o in ((at + 4, at), (at, at + 8)):
+        assert lib.dn_decode_step(d, *[at] * 6, i, None, at, o, None) == 9
+
+
+def _offset(t):
+    return torch.cat([t.new_zeros(1), t.detach().reshape(-1)])[1:].view(t.shape)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K,V,dtype,precision", [(64, 64, torch.bfloat16, "bf16"), (128, 128, torch.bfloat16, "bf16"), (64, 64, torch.float32, "fp32")])
+def test_offset_views_give_the_same(K, V, dtype, precision):
+    import deltanet_b200 as dn
+    gen = torch.Generator().manual_seed(9)
+    r = lambda *s: torch.rand(*s, generator=gen)
+    t = [(r(1, 200, 2, n) - 0.5).to(dtype).cuda() for n in (K, K, V)] + [-r(1, 200, 2, K).cuda(), r(1, 200, 2, K).cuda(), r(1, 200, 2, V).cuda()]
+    cot = (r(1, 200, 2, V) - 0.5).to(dtype).cuda()
+    res = []
+    for leaves, d in ((t, cot), ([_offset(x) for x in t], _offset(cot))):
+        leaves = [x.detach().requires_grad_() for x in leaves]
+        out = dn.chunk_gdn2(*leaves, precision=precision, qk_l2norm=True)
+        res.append((out,) + torch.autograd.grad(out, leaves, d))
+    assert all(torch.equal(x, y) for x, y in zip(*res))
+    tok, state = [x[:, 0].contiguous() for x in t], r(1, 2, K, V).cuda()
+    one = dn.gdn2_decode_step(*tok, state)
+    two = dn.gdn2_decode_step(*tok, _offset(state))
+    assert all(torch.equal(x, y) for x, y in zip(one, two))
+    two = dn.gdn2_decode_step(*[_offset(x) for x in tok], state)          # the other decode kernel: sums of K in another order
+    for x, y in zip(one, two):                                            # (fp32, or one rounding of the outputs to bf16)
+        assert float((x.float() - y.float()).norm() / x.float().norm()) < (1e-2 if x.dtype == torch.bfloat16 else K * 2.0 ** -24)
+    with pytest.raises(ValueError, match="multiple of 16 bytes"):
+        dn.gdn2_decode_step(*tok, state, out_state=_offset(state))
+
+
+@pytest.mark.gpu
+def test_offset_views_of_the_layer_steps():
+    import deltanet_b200 as dn
+    gen = torch.Generator().manual_seed(10)
+    x, w = torch.randn(1, 50, 256, generator=gen).cuda(), torch.randn(256, 4, generator=gen).cuda()
+    o, z, n = torch.randn(1, 50, 2, 64, generator=gen).cuda(), torch.randn(1, 50, 2, 64, generator=gen).cuda(), torch.ones(64).cuda()
+    kw = dict(num_k_heads=1, num_v_heads=2, head_k_dim=64, head_v_dim=64)
+    assert all(torch.equal(a, b) for a, b in zip(dn.gdn_qkv_producer(x, w, **kw), dn.gdn_qkv_producer(_offset(x), w, **kw)))
+    assert torch.equal(dn.gated_rmsnorm(o, z, n), dn.gated_rmsnorm(_offset(o), _offset(z), n))
