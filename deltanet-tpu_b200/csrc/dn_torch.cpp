@@ -178,6 +178,17 @@ variable_list run(const dn_shape& shape, const Tensor& q, const Tensor& k, const
                         recompute, inference);
 }
 
+// Allocation and enqueueing go on without the interpreter's lock: a call that waits for room in the launch queue, or for
+// cudaMalloc, does not hold up the other Python threads.
+struct Free_gil {
+  PyThreadState* state = PyEval_SaveThread();
+  void back() {
+    if (state) PyEval_RestoreThread(state);
+    state = nullptr;
+  }
+  ~Free_gil() { back(); }
+};
+
 PyObject* wrap(const variable_list& r) {
   if (r.size() == 1) return THPVariable_Wrap(r[0]);
   return PyTuple_Pack(2, py::reinterpret_steal<py::object>(THPVariable_Wrap(r[0])).ptr(),
@@ -242,6 +253,9 @@ PyObject* py_chunk(PyObject*, PyObject* const* a, Py_ssize_t n) {
   s.scale = a[12] == Py_None ? (float)(1.0 / std::sqrt((double)K)) : (float)PyFloat_AsDouble(a[12]);
   s.flags = (uint32_t)PyLong_AsUnsignedLong(a[13]) | (init.defined() ? DN_HAS_INIT : 0u);
   if (PyErr_Occurred()) return nullptr;
+  const bool want_final = a[9] == Py_True, recompute = a[14] == Py_True, inference = a[15] == Py_True;
+  variable_list r;
+  Free_gil gil;
   Tensor seg;
   if (ids.defined() || cu.defined()) {
     seg = at::empty({B, Lq}, q.options().dtype(at::kInt).requires_grad(false));
@@ -251,10 +265,17 @@ PyObject* py_chunk(PyObject*, PyObject* const* a, Py_ssize_t n) {
     else
       check(abi.cu_seqlens_segments(cu.const_data_ptr<int32_t>(), (int32_t)cu.numel(), nullptr, out, s.B, s.L, stream()), "dn_cu_seqlens_segments");
   }
-  return wrap(run(s, q, k, v, g, b, w, init, seg, a[9] == Py_True, a[14] == Py_True, a[15] == Py_True));
+  r = run(s, q, k, v, g, b, w, init, seg, want_final, recompute, inference);
+  gil.back();
+  return wrap(r);
   END_HANDLE_TH_ERRORS
 }
 
+std::vector<Tensor> tensors(PyObject* const* a, int n) {
+  std::vector<Tensor> t;
+  for (int i = 0; i < n; ++i) t.push_back(tensor_or_none(a[i]));
+  return t;
+}
 // The two directions on prepared tensors and canonical ids, without autograd.
 bool shape_of(PyObject* o, dn_shape* s) {
   if (!PyBytes_Check(o) || PyBytes_GET_SIZE(o) != (Py_ssize_t)sizeof(dn_shape)) return false;
@@ -272,10 +293,13 @@ PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   dn_shape s;
   TORCH_CHECK_VALUE(n == 12 && all_tensors(a, 6) && shape_of(a[8], &s), "forward: bad arguments");
+  const std::vector<Tensor> t = tensors(a, 8);
+  const Tensor out = tensor_or_none(a[11]);
+  const bool want_final = a[9] == Py_True, keep = a[10] == Py_True;
   Tensor kept;
-  variable_list r = forward(s, THPVariable_Unpack(a[0]), THPVariable_Unpack(a[1]), THPVariable_Unpack(a[2]), THPVariable_Unpack(a[3]),
-                            THPVariable_Unpack(a[4]), THPVariable_Unpack(a[5]), tensor_or_none(a[6]), tensor_or_none(a[7]), a[9] == Py_True,
-                            a[10] == Py_True ? &kept : nullptr, tensor_or_none(a[11]));
+  Free_gil gil;
+  const variable_list r = forward(s, t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], want_final, keep ? &kept : nullptr, out);
+  gil.back();
   return tuple_of({r[0], r.size() > 1 ? r[1] : Tensor(), kept});
   END_HANDLE_TH_ERRORS
 }
@@ -284,9 +308,11 @@ PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   dn_shape s;
   TORCH_CHECK_VALUE(n == 12 && all_tensors(a, 6) && shape_of(a[11], &s), "backward: bad arguments");
-  return tuple_of(backward(s, THPVariable_Unpack(a[0]), THPVariable_Unpack(a[1]), THPVariable_Unpack(a[2]), THPVariable_Unpack(a[3]),
-                           THPVariable_Unpack(a[4]), THPVariable_Unpack(a[5]), tensor_or_none(a[6]), tensor_or_none(a[7]),
-                           tensor_or_none(a[8]), tensor_or_none(a[9]), tensor_or_none(a[10])));
+  const std::vector<Tensor> t = tensors(a, 11);
+  Free_gil gil;
+  const variable_list r = backward(s, t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], t[10]);
+  gil.back();
+  return tuple_of(r);
   END_HANDLE_TH_ERRORS
 }
 // bare(*tensors): may a call on them pass autograd by?  No gradient is wanted, and nothing follows it.
@@ -344,18 +370,16 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   s.stability_tau = (float)PyFloat_AsDouble(a[11]);
   if (PyErr_Occurred()) return nullptr;
   const at::ScalarType st = s.state_out_dtype == DN_BF16 ? at::kBFloat16 : at::kFloat;
-  PyObject* next_py = a[12];
-  if (!next.defined()) {
-    next = at::empty({B, Hv, K, V}, state.options().dtype(st).requires_grad(false));
-    next_py = nullptr;
-  } else if (!plain(next, q) || !at16(next) || next.scalar_type() != st || next.sizes() != state.sizes()) {
-    Py_RETURN_NONE;
-  }
+  PyObject* next_py = next.defined() ? a[12] : nullptr;
+  if (next_py && (!plain(next, q) || !at16(next) || next.scalar_type() != st || next.sizes() != state.sizes())) Py_RETURN_NONE;
+  Free_gil gil;
   state = aligned(state);
+  if (!next_py) next = at::empty({B, Hv, K, V}, state.options().dtype(st).requires_grad(false));
   Tensor o = at::empty({B, Hv, V}, q.options().requires_grad(false));
   check(abi.decode_step(&s, ptr(q), ptr(k), ptr(v), ptr(g), ptr(b), ptr(w), ptr(state), static_cast<const uint8_t*>(ptr(reset)),
                         o.mutable_data_ptr(), const_cast<void*>(next.const_data_ptr()), stream()),
         "dn_decode_step");
+  gil.back();
   PyObject* r = PyTuple_New(2);
   PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(o));
   PyTuple_SET_ITEM(r, 1, next_py ? Py_NewRef(next_py) : THPVariable_Wrap(next));

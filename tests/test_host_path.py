@@ -209,3 +209,22 @@ def test_offset_views_of_the_layer_steps():
     kw = dict(num_k_heads=1, num_v_heads=2, head_k_dim=64, head_v_dim=64)
     assert all(torch.equal(a, b) for a, b in zip(dn.gdn_qkv_producer(x, w, **kw), dn.gdn_qkv_producer(_offset(x), w, **kw)))
     assert torch.equal(dn.gated_rmsnorm(o, z, n), dn.gated_rmsnorm(_offset(o), _offset(z), n))
+
+
+# ---- other Python threads run while a call is enqueued
+@pytest.mark.gpu
+def test_calls_are_enqueued_without_the_interpreter_lock(host, fn):
+    """PyGILState_Check, 1 where the calling thread holds the lock, stands in for the entry points: its answer is their status."""
+    import ctypes as C
+    import deltanet_b200 as dn
+    lib, held = _lib.lib(), C.cast(C.pythonapi.PyGILState_Check, C.c_void_p).value
+    real = {n: C.cast(getattr(lib, n), C.c_void_p).value for n in _lib._HOST_USES}
+    t, token = _inputs(11, True), [x[:, 0].contiguous() for x in _inputs(12)]
+    host.bind(dict(real, dn_decode_step=held, dn_chunk_fwd=held, dn_chunk_bwd=held))
+    try:
+        dn.gdn2_decode_step(*token, torch.zeros(1, 2, 64, 64, device="cuda"))
+        torch.autograd.grad(fn(*t).sum(), t)
+        wide = [torch.stack([x, x], -1)[..., 0] for x in t]                 # the general path
+        torch.autograd.grad(fn(*wide).sum(), t)
+    finally:
+        host.bind(real)
