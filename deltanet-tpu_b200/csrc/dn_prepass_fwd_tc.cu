@@ -416,11 +416,20 @@ __device__ __forceinline__ void chain_rows(int warp, int lane, const float (&gv)
 // Decay of any strength: the hierarchical factorisation.  At level s in {16, 32, 64} the tile is cut into pairs of
 // adjacent s-row blocks; for a pair with rows I (lower block), columns J (upper block) and reference row r = first of I
 //     A[I,J] = (beta_I e^{Lam_I - Lam_r}) (k_J e^{Lam_r - Lam_J})^T,   M[I,J] = (q_I e^{Lam_I - Lam_r}) (k_J e^{Lam_r - Lam_J})^T
-// with every factor <= 1.  A row is either a row or a column of its level, so two images suffice: KR (beta on lower
-// rows, k on upper rows) and QK (q, k); A = KR KR^T, M = QK KR^T, of which the drain keeps the blocks that the level
-// owns.  The 16 x 16 diagonal blocks are evaluated pair by pair.  (The reference: 32-row blocks, one reference row
-// per block row, gdn2.py:162-197.)  Five walks over the channel groups -- diagonal, three levels, X -- because the
-// footprint of the common route is kept: about 1.6 times the common route's time per tile, paid by such tiles only.
+// with every factor <= 1.  Half of the tile's rows are lower rows of a level and half upper rows, so a level is ONE product of
+// 128 x 64: its lower rows' beta and q (64 each) against its upper rows' k, and the three levels' results fit 192 columns of
+// tensor memory together.  That lets one walk over the channel groups do everything -- decay, the three levels, X, qe, ke, and
+// beside the products the 16 x 16 diagonal blocks, pair by pair.  What bounds it is the length of a group's dependent steps
+// (load, scan, images, products), so walks count: with five of them (diagonal, a level each, X), and the common route's four
+// groups run to their end first, a prefill of 8192 tokens of 16 x 32 heads, every tile strong, took 981 us; with one walk, and
+// the common route left as soon as a group finds strong decay, 623; a kernel of its own with one CTA per SM took 676.
+// (The reference: 32-row blocks, one reference row per block row, gdn2.py:162-197.)
+constexpr int LV_B = 4 * PP;                            // a level's images: 4 panels of 128 rows, then 4 of 64 rows,
+constexpr int LV_PITCH = 66;                            //   66 pieces apart
+constexpr int LV_SIZE = LV_B + 4 * LV_PITCH;            // (in pieces of 16 bytes)
+constexpr int DP = 33;                                  // row pitch (floats) of the diagonal blocks' rows
+static_assert(3 * LV_SIZE * 16 <= tri::BYTES, "levels in the triangle's place");
+static_assert((C * LQ + 16 * 32 + 3 * 32 * DP) * 4 <= 16 * PB, "decay and diagonal rows in the place of the T image");
 template <int MODE>
 __device__ __noinline__ void strong_route(const PrepassFwdArgs& a, int b, int h, int t0, size_t ibase, const float* rq_s, const float* rk_s,
                                           const int* seg_s, int* rst_s, uint8_t* sm, umma::Ctx& cx) {
@@ -428,160 +437,152 @@ __device__ __noinline__ void strong_route(const PrepassFwdArgs& a, int b, int h,
   __nv_bfloat16* M = reinterpret_cast<__nv_bfloat16*>(a.res.M) + ibase * C * C;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, x = row_of(tid), lgrp = piece_of(tid);
   float* Tp = reinterpret_cast<float*>(sm + OFF_T);
+  uint4* XI = reinterpret_cast<uint4*>(sm + OFF_X);
+  uint4* LV = reinterpret_cast<uint4*>(sm + OFF_T);
   float* LAM = reinterpret_cast<float*>(sm + OFF_TI);
   float* TOT = LAM + C * LQ;
-  float* KC = reinterpret_cast<float*>(sm + OFF_X);     // diagonal pass: k_hat, q_hat, beta of 64 rows, fp32
-  float* QC = KC + 64 * LQ;
-  float* BC = QC + 64 * LQ;
+  float* KC = TOT + 16 * 32;                            // k_hat, q_hat, beta of 32 rows, fp32
+  float* QC = KC + 32 * DP;
+  float* BC = QC + 32 * DP;
   uint4* Mimg = reinterpret_cast<uint4*>(M);
-  auto decay = [&](int grp) {                           // Lambda of the group; begins and ends with a barrier
-    float gv[8];
+  uint4* QE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.qe) + ibase * C * K);
+  uint4* KE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.ke) + ibase * C * K);
+  const bool first = seg_s[x] == seg_s[0], last = seg_s[x] == seg_s[C - 1];
+  // diagonal blocks, 32 rows (two blocks) at a time: a thread takes a pair (i > j) and half of the group's channels
+  const int dblk = (tid >> 1) / 120, ch = 16 * (tid & 1);
+  int di = 1, dj = (tid >> 1) % 120;
+  while (dj >= di) { dj -= di; ++di; }
+  const int ri = dblk * 16 + di, rj = dblk * 16 + dj;
+  float accA[4] = {}, accM[4] = {}, accD = 0.f;
+#pragma unroll 1
+  for (int grp = 0; grp < 4; ++grp) {
+    const int p = grp * 4 + lgrp;
+    if (4 * grp >= r.kp) {                              // channels that do not exist
+      XI[p * PP + x] = QE[p * 128 + x] = KE[p * 128 + x] = make_uint4(0, 0, 0, 0);
+      if (warp == 15) a.res.lam_end[ibase * K + 32 * grp + lane] = 0.f;
+      continue;
+    }
+    float gv[8], kh[8], qh[8], be[8];
     load_decay(r, grp, warp, lane, gv);
+    khat8(r, x, p, kh);
+    qhat8(r, x, p, qh);
+    bact8(r, x, p, be);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { accD = fmaf(qh[i], kh[i], accD); be[i] *= kh[i]; }
     __syncthreads();
     const int nr = scan_rows(seg_s, warp, lane, gv, TOT, rst_s);
     __syncthreads();
     chain_rows(warp, lane, gv, nr, TOT, rst_s, LAM);
     __syncthreads();
-  };
-  // ---- diagonal blocks: threads 0 .. 479 own a pair (i > j) of one of four blocks per half, threads 0 .. 63 also M_ii
-  int di = 1, dj = tid % 120;
-  while (dj >= di) { dj -= di; ++di; }
-  const int dblk = tid / 120;
-  float accA[2] = {0.f, 0.f}, accM[2] = {0.f, 0.f}, accD[2] = {0.f, 0.f};
+    if (warp == 15) a.res.lam_end[ibase * K + 32 * grp + lane] = LAM[(C - 1) * LQ + lane];
 #pragma unroll 1
-  for (int grp = 0; grp < 4; ++grp) {
-    decay(grp);
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      if (tid < 256) {
-        const int xr = tid >> 2, xx = half * 64 + xr, p = grp * 4 + (tid & 3), o = xr * LQ + 8 * (tid & 3);
-        float kh[8], qh[8], be[8];
-        khat8(r, xx, p, kh);
-        qhat8(r, xx, p, qh);
-        bact8(r, xx, p, be);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { KC[o + i] = kh[i]; QC[o + i] = qh[i]; BC[o + i] = be[i] * kh[i]; }
-      }
-      __syncthreads();
-      if (dblk < 4) {
-        const int ri = dblk * 16 + di, rj = dblk * 16 + dj;
-        const float* li = LAM + (half * 64 + ri) * LQ;
-        const float* lj = LAM + (half * 64 + rj) * LQ;
-        float sa = 0.f, sm_ = 0.f;
-#pragma unroll 4
-        for (int c = 0; c < 32; ++c) {
-          const float e = KC[rj * LQ + c] * umma::ex2_fast(fminf(li[c] - lj[c], 0.f) * DN_LOG2E);
-          sa = fmaf(BC[ri * LQ + c], e, sa);
-          sm_ = fmaf(QC[ri * LQ + c], e, sm_);
-        }
-        accA[half] += sa;
-        accM[half] += sm_;
-      }
-      if (tid < 64) {
-        float s = 0.f;
-#pragma unroll 4
-        for (int c = 0; c < 32; ++c) s = fmaf(QC[tid * LQ + c], KC[tid * LQ + c], s);
-        accD[half] += s;
-      }
-      __syncthreads();
-    }
-  }
-  {                                                     // zeros on and above the diagonal, then the pairs
-    const int row = tid & 127, q = tid >> 7, b = row >> 4;
-    *reinterpret_cast<float4*>(tri::blk(Tp, b, b) + (row & 15) * tri::BP + 4 * q) = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int p = 2 * b + q; p < 16; p += 4) Mimg[p * 128 + row] = make_uint4(0, 0, 0, 0);
-    __syncthreads();
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      if (dblk < 4) {
-        const int b2 = half * 4 + dblk, ri = b2 * 16 + di, rj = b2 * 16 + dj;
-        const bool same = seg_s[ri] == seg_s[rj];
-        tri::blk(Tp, b2, b2)[di * tri::BP + dj] = same ? accA[half] : 0.f;
-        M[rix(true, ri, rj, C)] = __float2bfloat16_rn(same ? accM[half] : 0.f);
-      }
-      if (tid < 64) M[rix(true, half * 64 + tid, half * 64 + tid, C)] = __float2bfloat16_rn(accD[half]);
-    }
-  }
-  // ---- the three levels; images of 32 channels in the place of X, one set at a time
-  uint4* KR = reinterpret_cast<uint4*>(sm + OFF_X);
-  uint4* QK = KR + 4 * PP;
-#pragma unroll 1
-  for (int lv = 0; lv < 3; ++lv) {
-#pragma unroll 1
-    for (int grp = 0; grp < 4; ++grp) {
-      decay(grp);
-      const int p = grp * 4 + lgrp, s = 16 << lv, ref = level_ref(x, s);
+    for (int lv = 0; lv < 3; ++lv) {
+      const int s = 16 << lv, ref = level_ref(x, s), at = ((x >> (5 + lv)) << (4 + lv)) + (x & (s - 1));
       const bool lower = x >= ref;
-      float kh[8], qh[8], be[8], f[8];
-      khat8(r, x, p, kh);
-      qhat8(r, x, p, qh);
-      bact8(r, x, p, be);
+      uint4* I = LV + lv * LV_SIZE;
+      float f[8], o[8];
       decay8(LAM + (lower ? x : ref) * LQ + 8 * lgrp, LAM + (lower ? ref : x) * LQ + 8 * lgrp, f);
+      if (lower) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float kf = kh[i] * f[i];
-        be[i] = lower ? be[i] * kh[i] * f[i] : kf;
-        qh[i] = lower ? qh[i] * f[i] : kf;
-      }
-      KR[lgrp * PP + x] = umma::pack8(be);
-      QK[lgrp * PP + x] = umma::pack8(qh);
-      umma::pre_issue_sync();
-      umma::issue_pitched<128, false, false>(cx, KR, PB, KR, PB, 32, 0, grp > 0);
-      umma::issue_pitched<128, false, false>(cx, QK, PB, KR, PB, 32, 128, grp > 0);
-      umma::commit_wait(cx);
-    }
-    const int quarter = warp & 3, group = warp >> 2, row = quarter * 32 + lane, bi = row >> 4;
-    const uint32_t tbase = cx.tmem + ((uint32_t)(quarter * 32) << 16);
-#pragma unroll 1
-    for (int cc = 0; cc < 32; cc += 16) {
-      const int col = group * 32 + cc, bj = col >> 4;
-      float va[16], vm[16];
-      if (!cx.dead) {
-        umma::tmem_ld16(tbase + col, va);
-        umma::tmem_ld16(tbase + 128 + col, vm);
+        for (int i = 0; i < 8; ++i) o[i] = be[i] * f[i];
+        I[lgrp * PP + at] = umma::pack8(o);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] = qh[i] * f[i];
+        I[lgrp * PP + 64 + at] = umma::pack8(o);
       } else {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) va[i] = vm[i] = 0.f;
+        for (int i = 0; i < 8; ++i) o[i] = kh[i] * f[i];
+        I[LV_B + lgrp * LV_PITCH + at] = umma::pack8(o);
       }
-      if (bj >= bi || owner_level(bi, bj) != lv) continue;
+    }
+    {                                                   // X, qe, ke
+      float o[8];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const bool same = seg_s[row] == seg_s[col + i];
-        va[i] = same ? va[i] : 0.f;
-        vm[i] = same ? vm[i] : 0.f;
+      for (int i = 0; i < 8; ++i) o[i] = first ? be[i] * umma::exp_neg(fminf(LAM[x * LQ + 8 * lgrp + i], 0.f)) : 0.f;
+      XI[p * PP + x] = umma::pack8(o);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) o[i] = first ? qh[i] * umma::exp_neg(fminf(LAM[x * LQ + 8 * lgrp + i], 0.f)) : 0.f;
+      QE[p * 128 + x] = umma::pack8(o);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        o[i] = last ? kh[i] * umma::exp_neg(fminf(LAM[(C - 1) * LQ + 8 * lgrp + i] - LAM[x * LQ + 8 * lgrp + i], 0.f)) : 0.f;
+      KE[p * 128 + x] = umma::pack8(o);
+    }
+    umma::pre_issue_sync();
+#pragma unroll 1
+    for (int lv = 0; lv < 3; ++lv)
+      umma::issue_pitched<64, false, false>(cx, LV + lv * LV_SIZE, PB, LV + lv * LV_SIZE + LV_B, LV_PITCH * 16, 32, 64 * lv, grp > 0);
+    umma::commit(cx);
+#pragma unroll
+    for (int ps = 0; ps < 4; ++ps) {                    // diagonal blocks, beside the products
+      if ((warp >> 2) == ps) {
+        const int o = (x & 31) * DP + 8 * lgrp;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { KC[o + i] = kh[i]; QC[o + i] = qh[i]; BC[o + i] = be[i]; }
       }
-      float4* d = reinterpret_cast<float4*>(tri::blk(Tp, bi, bj) + (row & 15) * tri::BP);
+      __syncthreads();
+      if (dblk < 2) {
+        const float *li = LAM + (32 * ps + ri) * LQ + ch, *lj = LAM + (32 * ps + rj) * LQ + ch;
+        const float *kc = KC + rj * DP + ch, *qc = QC + ri * DP + ch, *bc = BC + ri * DP + ch;
+        float sa = 0.f, sq = 0.f;
+#pragma unroll 4
+        for (int c = 0; c < 16; ++c) {
+          const float e = kc[c] * umma::ex2_fast(fminf(li[c] - lj[c], 0.f) * DN_LOG2E);
+          sa = fmaf(bc[c], e, sa);
+          sq = fmaf(qc[c], e, sq);
+        }
+        accA[ps] += sa;
+        accM[ps] += sq;
+      }
+      __syncthreads();
+    }
+    umma::commit_wait_cta(cx);
+  }
+  // ---- zeros on and above the diagonal, then the diagonal blocks and the levels' blocks
+  {
+    const int row = tid & 127, q = tid >> 7, b2 = row >> 4;
+    *reinterpret_cast<float4*>(tri::blk(Tp, b2, b2) + (row & 15) * tri::BP + 4 * q) = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int p = 2 * b2 + q; p < 16; p += 4) Mimg[p * 128 + row] = make_uint4(0, 0, 0, 0);
+  }
+  __syncthreads();
 #pragma unroll
-      for (int i = 0; i < 4; ++i) d[i] = make_float4(va[4 * i], va[4 * i + 1], va[4 * i + 2], va[4 * i + 3]);
-      Mimg[(col / 8) * 128 + row] = umma::pack8p(vm);
-      Mimg[(col / 8 + 1) * 128 + row] = umma::pack8p(vm + 8);
+  for (int ps = 0; ps < 4; ++ps) {
+    const float sa = accA[ps] + __shfl_xor_sync(0xffffffffu, accA[ps], 1), sq = accM[ps] + __shfl_xor_sync(0xffffffffu, accM[ps], 1);
+    if (dblk < 2 && ch == 0) {
+      const int i = 32 * ps + ri, j = 32 * ps + rj;
+      const bool same = seg_s[i] == seg_s[j];
+      tri::blk(Tp, i >> 4, i >> 4)[di * tri::BP + dj] = same ? sa : 0.f;
+      M[rix(true, i, j, C)] = __float2bfloat16_rn(same ? sq : 0.f);
+    }
+  }
+  accD += __shfl_xor_sync(0xffffffffu, accD, 1);
+  accD += __shfl_xor_sync(0xffffffffu, accD, 2);
+  if (lgrp == 0) M[rix(true, x, x, C)] = __float2bfloat16_rn(accD);
+  {
+    const int quarter = warp & 3, u0 = 16 * (warp >> 2), at = (quarter & 1) * 32 + lane;      // lanes 0 .. 63: A's lower rows, 64 .. 127: M's
+    const uint32_t tbase = cx.tmem + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll 1
+    for (int lv = 0; lv < 3; ++lv) {
+      float v[16];
+      if (!cx.dead) umma::tmem_ld16(tbase + 64 * lv + u0, v);
+      else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.f;
+      }
+      if ((at >> (4 + lv)) != (u0 >> (4 + lv))) continue;       // rows and columns of different pairs
+      const int s = 16 << lv, row = ((at >> (4 + lv)) << (5 + lv)) + s + (at & (s - 1)), col = ((u0 >> (4 + lv)) << (5 + lv)) + (u0 & (s - 1));
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = seg_s[row] == seg_s[col + i] ? v[i] : 0.f;
+      if (quarter < 2) {
+        float4* d = reinterpret_cast<float4*>(tri::blk(Tp, row >> 4, col >> 4) + (row & 15) * tri::BP);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+      } else {
+        Mimg[(col / 8) * 128 + row] = umma::pack8p(v);
+        Mimg[(col / 8 + 1) * 128 + row] = umma::pack8p(v + 8);
+      }
     }
     umma::tc_fence_before();
-  }
-  // ---- X again (its place was taken), and qe, ke from factors that cannot overflow
-  uint4* XI = reinterpret_cast<uint4*>(sm + OFF_X);
-  uint4* QE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.qe) + ibase * C * K);
-  uint4* KE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.ke) + ibase * C * K);
-  const bool first = seg_s[x] == seg_s[0], last = seg_s[x] == seg_s[C - 1];
-#pragma unroll 1
-  for (int grp = 0; grp < 4; ++grp) {
-    decay(grp);
-    const int p = grp * 4 + lgrp;
-    float kh[8], qh[8], be[8];
-    khat8(r, x, p, kh);
-    qhat8(r, x, p, qh);
-    bact8(r, x, p, be);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float lam = LAM[x * LQ + 8 * lgrp + i], lend = LAM[(C - 1) * LQ + 8 * lgrp + i];
-      const float el = first ? umma::exp_neg(fminf(lam, 0.f)) : 0.f;
-      be[i] = be[i] * kh[i] * el;
-      qh[i] *= el;
-      kh[i] = last ? kh[i] * umma::exp_neg(fminf(lend - lam, 0.f)) : 0.f;
-    }
-    XI[p * PP + x] = umma::pack8(be);
-    QE[p * 128 + x] = umma::pack8(qh);
-    KE[p * 128 + x] = umma::pack8(kh);
   }
   __syncthreads();
 }
@@ -594,6 +595,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
   __shared__ uint32_t tbase;
   __shared__ int seg_s[C];
   __shared__ int rst_s[16];
+  __shared__ int strong_s;
   __shared__ float rq_s[C], rk_s[C];
   __shared__ uint8_t ds_s[C], de_s[C];                  // first / last row of each row's document inside the tile
   const Geo& g = a.g;
@@ -656,6 +658,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
     };
     load_g(0);
     if (tid < C) seg_s[tid] = seg_at(a.seg, b, t0 + tid, g.L);
+    if (tid == 0) strong_s = 0;
     float rq = 1.f, rk = 1.f;
     if (l2) {
       float sq = 0.f, sk = 0.f;
@@ -706,8 +709,9 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
     EDGE[64 + lane] = 0.f;
     bool strong = false;
     const bool first = seg_s[x] == seg_s[0], last = seg_s[x] == seg_s[C - 1];
+    int grp = 0;
 #pragma unroll 1
-    for (int grp = 0; grp < 4; ++grp) {
+    for (; grp < 4; ++grp) {
       act_g();
       if (cuts == 0) {
 #pragma unroll
@@ -718,6 +722,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       }
       TOT[warp * 32 + lane] = gv[7];
       __syncthreads();
+      if (strong_s) break;                              // found by the group before (nobody writes it between these two barriers)
       // rows above hand on the sums back to the last warp in which a document starts
       const uint32_t above = __ballot_sync(0xffffffffu, lane < warp && rst_s[lane & 15]);
       float carry = 0.f;
@@ -782,6 +787,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
         o2[i] = qh[i] * f;
         o3[i] = be[i] * f;
       }
+      if (strong) strong_s = 1;
       KF[lgrp * PP + x] = umma::pack8(o1);
       QF[lgrp * PP + x] = umma::pack8(o2);
       BF[lgrp * PP + x] = umma::pack8(o3);
@@ -809,8 +815,9 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       }
       if (grp < 3) { load_g(grp + 1); load_kqb(grp + 1); }
     }
-    const bool ok0 = group_wait(0), ok1 = group_wait(1);
-    if (__syncthreads_or(!(ok0 && ok1))) { cx.dead = true; umma::report_timeout(err); }
+    bool ok = group_wait((grp - 1) & 1);                 // the last two groups' products
+    if (grp > 1) ok = group_wait(grp & 1) && ok;
+    if (__syncthreads_or(!ok)) { cx.dead = true; umma::report_timeout(err); }
     umma::tc_fence_after();
     const bool any_strong = __syncthreads_or(strong);
     if (a.res.T) {                                      // the backward takes the same route

@@ -60,6 +60,22 @@ def test_bf16_narrow_heads(dn, K, V, Hk, Hv, L, recompute):
             lambda t, i: O.chunk_gdn2(*t, segment_ids=seg, initial_state=i, **kw), ins, tol=BF16_TOL, init=init)
 
 
+# ---- strong decay: seen in each of the four channel groups, in every channel, by one document of a tile only
+@pytest.mark.parametrize("channels", [slice(0, 1), slice(40, 41), slice(70, 71), slice(127, 128), slice(None)])
+@pytest.mark.parametrize("L", [33, 300])
+def test_strong_decay(dn, channels, L):
+    ins = list(O.make_inputs(45, 1, L, 1, 2, 128, 128, qkv_dtype=torch.bfloat16)[:6])
+    ins[3] = ins[3].clone()
+    ins[3][..., channels] *= 12.0
+    seg = docs(1, L, 70, 150, 256) if L > 256 else None
+    if seg is not None:
+        ins[3][:, 70:150] /= 12.0                                   # (a tile with moderate documents beside a strong one)
+    init = torch.randn(1, 2, 128, 128, generator=torch.Generator().manual_seed(46)) * 0.1
+    kw = dict(chunk_size=128, precision="bf16", qk_l2norm=True, output_final_state=True)
+    compare(lambda t, i: dn.chunk_gdn2(*t, segment_ids=None if seg is None else seg.cuda(), initial_state=i, **kw),
+            lambda t, i: O.chunk_gdn2(*t, segment_ids=seg, initial_state=i, **kw), ins, tol=BF16_TOL, init=init)
+
+
 # ---- scalar gates: heads of one key head taken in turn (288 items) or apart (144); the wide forward chain
 @pytest.mark.parametrize("B,L", [(18, 250), (18, 128)])
 def test_shared_key_heads(dn, B, L):
