@@ -48,3 +48,14 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "nope.so"))
     with pytest.raises(RuntimeError, match="no CPU or eager fallback"):
         _lib.lib()
+
+
+def test_the_c_library_builds_without_torch():
+    """What `make all` would run: nvcc only where PYTHON has no torch, and the extension too where it has."""
+    import subprocess
+    import sys
+    csrc = os.path.join(ROOT, "deltanet-tpu_b200", "csrc")
+    for python, host in ((os.path.join(ROOT, "no", "such", "python"), False), (sys.executable, True)):
+        r = subprocess.run(["make", "-C", csrc, "-n", "-B", "all", f"PYTHON={python}"], capture_output=True, text=True)
+        assert r.returncode == 0 and "dn_api.cu" in r.stdout
+        assert ("dn_torch.cpp" in r.stdout) == host
