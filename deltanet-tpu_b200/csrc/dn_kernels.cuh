@@ -75,7 +75,8 @@ struct PrepassBwdArgs {
 int launch_status();
 long long launches_total();
 
-size_t prepass_fwd_scratch_floats(const Geo& g);
+size_t prepass_fwd_scratch_floats(const Geo& g);  // what the forward prepass likes to have ...
+size_t prepass_fwd_scratch_least(const Geo& g);   // ... and what it can do with
 size_t prepass_bwd_scratch_per_cta(const Geo& g);
 
 int launch_prepass_fwd(const Geo& g, const void* q, const void* k, const void* v, const void* gg,

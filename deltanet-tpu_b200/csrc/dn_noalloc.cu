@@ -57,7 +57,7 @@ int dn_prepass_fwd_static(const dn_shape* s, const void* q, const void* k, const
       bits |= reinterpret_cast<uintptr_t>(p);
     if (bits & 15) return DN_ERR_MISALIGNED;
   }
-  if (dn::prepass_fwd_scratch_floats(g) * sizeof(float) > DN_STATIC_SCRATCH_BYTES) return DN_ERR_STATIC_SCRATCH_EXCEEDED;
+  if (dn::prepass_fwd_scratch_least(g) * sizeof(float) > DN_STATIC_SCRATCH_BYTES) return DN_ERR_STATIC_SCRATCH_EXCEEDED;
   void* scratch = nullptr;
   if ((rc = static_scratch(&scratch))) return rc;
   return dn::launch_prepass_fwd(g, q, k, v, g_, b, w, seg, *res, reinterpret_cast<float*>(scratch),

@@ -285,29 +285,34 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_fwd_kernel(PrepassFwdAr
   }
 }
 
-static size_t scratch_per_cta(const Geo& g) { return (size_t)5 * g.C * g.K + (size_t)g.C * g.Vw + (size_t)g.C * g.C; }
-size_t prepass_fwd_scratch_floats(const Geo& g) {
-  if (prepass_fwd_tc_eligible(g)) return 0;
+// Per CTA, or per cluster where the CTAs of one share an item: they also hand A round.
+static size_t scratch_per_cta(const Geo& g, bool shared) { return (size_t)5 * g.C * g.K + (size_t)g.C * g.Vw + (shared ? (size_t)g.C * g.C : 0); }
+static size_t scratch_floats(const Geo& g, bool shared) {
   const size_t items = (size_t)g.B * g.H * g.NC, ctas = items < (size_t)sm_count() ? items : (size_t)sm_count();
-  return ctas * scratch_per_cta(g);
+  return ctas * scratch_per_cta(g, shared);
 }
+size_t prepass_fwd_scratch_floats(const Geo& g) {
+  return prepass_fwd_tc_eligible(g) ? 0 : scratch_floats(g, team_size(g.B * g.H * g.NC) > 1);
+}
+size_t prepass_fwd_scratch_least(const Geo& g) { return prepass_fwd_tc_eligible(g) ? 0 : scratch_floats(g, false); }
 
 int launch_prepass_fwd(const Geo& g, const void* q, const void* k, const void* v, const void* gg,
                        const void* b, const void* w, const int32_t* seg, const dn_residuals& res,
-                       float* scratch, size_t scratch_floats, cudaStream_t st) {
+                       float* scratch, size_t floats, cudaStream_t st) {
   if (prepass_fwd_tc_eligible(g))
     return launch_prepass_fwd_tc(g, q, k, v, gg, b, w, seg, res, st);
   PrepassFwdArgs a{};
   a.g = g; a.q = q; a.k = k; a.v = v; a.gg = gg; a.b = b; a.w = w; a.seg = seg; a.res = res;
   a.items = g.B * g.H * g.NC;
-  a.scratch_per_cta = scratch_per_cta(g);
-  int grid = a.items < sm_count() ? a.items : sm_count();
-  if (scratch_floats < (size_t)grid * a.scratch_per_cta) return DN_ERR_SCRATCH_TOO_SMALL;
+  // A caller's scratch may hold an item per CTA and no more (a shape's share of the static array): one CTA an item then.
+  const int grid = a.items < sm_count() ? a.items : sm_count(), team = team_size(a.items);
+  const int ranks = team > 1 && floats >= (size_t)grid * scratch_per_cta(g, true) ? team : 1;
+  a.scratch_per_cta = scratch_per_cta(g, ranks > 1);
+  if (floats < (size_t)grid * a.scratch_per_cta) return DN_ERR_SCRATCH_TOO_SMALL;
   a.scratch = scratch;
   a.smem_tile_off = 3 * g.C * g.C;
   if (4 * g.C * 33 > 2 * g.C * g.C) a.smem_tile_off = g.C * g.C + 4 * g.C * 33;
   size_t smem = ((size_t)a.smem_tile_off + GEMM_SMEM_FLOATS + g.C) * sizeof(float);
-  const int ranks = team_size(a.items);
   if (ranks > 1) {
     cudaFuncSetAttribute(prepass_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     launch_team(prepass_fwd_kernel<true>, a.items, ranks, smem, st, a);

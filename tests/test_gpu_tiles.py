@@ -44,6 +44,27 @@ def test_fp32_splits(dn, C, K, V, B, L):
             lambda t, i: O.chunk_gdn2(*t, segment_ids=seg, initial_state=i, **kw), list(ins), tol=FP32_TOL, init=init)
 
 
+# ---- the forward prepass on the least scratch it can do with: one CTA an item where the CTAs of a cluster would share it
+@pytest.mark.parametrize("L,C,K,V,Hk,Hv", [(148 * 64, 128, 64, 64, 2, 2), (148 * 64, 64, 64, 64, 1, 8), (74 * 128, 128, 128, 64, 1, 3)])
+def test_static_scratch_shapes(dn, L, C, K, V, Hk, Hv):
+    from deltanet_b200 import _lib
+    lib = _lib.lib()
+    s = _lib.Shape(B=1, L=L, Hk=Hk, Hv=Hv, K=K, V=V, chunk=C, g_heads=Hk, g_cols=K, b_heads=Hk, b_cols=K, w_heads=Hv, w_cols=V,
+                   qkv_dtype=_lib.DN_F32, gate_dtype=_lib.DN_F32, precision=_lib.DN_PREC_FP32, flags=_lib.DN_QK_L2NORM, scale=1.0)
+    ins = [t.cuda() for t in O.make_inputs(33, 1, L, Hk, Hv, K, V)[:6]]
+    n, blocks = lib.dn_scratch_bytes(s, 0, 0), []
+    scratch = torch.empty(n, dtype=torch.uint8, device="cuda")
+    for static in (False, True):
+        block = torch.zeros(lib.dn_residual_bytes(s), dtype=torch.uint8, device="cuda")
+        res = _lib.Residuals()
+        assert lib.dn_residual_carve(s, block.data_ptr(), res) == 0
+        at = [t.data_ptr() for t in ins] + [None, res]
+        st = torch.cuda.current_stream().cuda_stream
+        assert (lib.dn_prepass_fwd_static(s, *at, st) if static else lib.dn_prepass_fwd(s, *at, scratch.data_ptr(), n, st)) == 0
+        blocks.append(block.view(torch.float32))
+    assert O.rel_l2(blocks[1], blocks[0]) < 128 * 2.0 ** -24         # the same sums of 128 terms, in another order where the team differs
+
+
 # ---- bf16: key and value widths of 64 on padded tensor-core tiles
 @pytest.mark.parametrize("K,V,Hk,Hv", [(64, 64, 2, 2), (64, 64, 1, 2), (64, 64, 1, 3), (64, 64, 1, 4), (64, 128, 1, 2),
                                        (128, 64, 2, 2), (128, 64, 1, 3)])
