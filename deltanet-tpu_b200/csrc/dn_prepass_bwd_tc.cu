@@ -727,11 +727,13 @@ int launch_prepass_bwd_tc(PrepassBwdArgs& a, size_t scratch_floats, cudaStream_t
   if (a.items <= 0) return DN_OK;
   a.scratch_per_cta = prepass_bwd_tc_scratch_per_cta(g);
   a.err = device_error_ptr();
-  if (a.group > 1 && scratch_floats < (size_t)sm_count() * a.scratch_per_cta) return DN_ERR_SCRATCH_TOO_SMALL;
-  int rc = launch_prepass_bwd_fast(a, st);
-  if (rc || prepass_bwd_scalar_route(g)) return rc;
+  // both kernels' needs, before either is enqueued: the sums over a key head's heads, the strong tiles' matrices
   const int grid = a.items < sm_count() ? a.items : sm_count();
-  if (scratch_floats < (size_t)grid * a.scratch_per_cta) return DN_ERR_SCRATCH_TOO_SMALL;
+  const bool scalar = prepass_bwd_scalar_route(g);
+  const size_t ctas = scalar ? (a.group > 1 ? sm_count() : 0) : grid;
+  if (scratch_floats < ctas * a.scratch_per_cta) return DN_ERR_SCRATCH_TOO_SMALL;
+  int rc = launch_prepass_bwd_fast(a, st);
+  if (rc || scalar) return rc;
   const size_t lam_phase = (size_t)C * LP * 4 + 4 * 32768;
   size_t smem = bwd_tc_image_bytes(g.Vw);
   if (smem < lam_phase) smem = lam_phase;

@@ -105,6 +105,31 @@ def test_shared_key_heads(dn, B, L):
     compare(lambda t, i: dn.chunk_gdn(*t, **kw), lambda t, i: O.chunk_gdn(*t, **kw), [q, k, v, g, beta], tol=BF16_TOL)
 
 
+# ---- too little scratch for the strong tiles' kernel: an error, and no gradient has been touched
+def test_scratch_is_checked_before_anything_is_enqueued(dn):
+    from deltanet_b200 import _lib
+    lib = _lib.lib()
+    L, H, K = 256, 2, 128
+    s = _lib.Shape(B=1, L=L, Hk=H, Hv=H, K=K, V=K, chunk=128, g_heads=H, g_cols=K, b_heads=H, b_cols=K, w_heads=H, w_cols=K,
+                   qkv_dtype=_lib.DN_BF16, gate_dtype=_lib.DN_F32, precision=_lib.DN_PREC_BF16, flags=_lib.DN_QK_L2NORM, scale=1.0)
+    ins = [t.cuda() for t in O.make_inputs(34, 1, L, H, H, K, K, qkv_dtype=torch.bfloat16)[:6]]
+    block = torch.zeros(lib.dn_residual_bytes(s), dtype=torch.uint8, device="cuda")
+    res = _lib.Residuals()
+    assert lib.dn_residual_carve(s, block.data_ptr(), res) == 0
+    scratch = torch.empty(lib.dn_scratch_bytes(s, 1, 0), dtype=torch.uint8, device="cuda")
+    out, dv, dh = (torch.zeros(1, L, H, K, device="cuda", dtype=t) for t in (torch.bfloat16, torch.float32, torch.float32))
+    st = torch.cuda.current_stream().cuda_stream
+    at = [t.data_ptr() for t in ins] + [None]
+    assert lib.dn_chunk_fwd(s, *at, None, out.data_ptr(), None, res, scratch.data_ptr(), scratch.numel(), st) == 0
+    grads = [torch.full_like(t, 7.0) for t in ins]
+    rest = [out.data_ptr(), dv.data_ptr(), dh.data_ptr()] + [t.data_ptr() for t in grads] + [scratch.data_ptr()]
+    assert lib.dn_state_bwd(s, res, None, out.data_ptr(), None, dv.data_ptr(), dh.data_ptr(), None, st) == 0
+    assert lib.dn_prepass_bwd(s, *at, res, *rest, 4096, st) == 4                     # DN_ERR_SCRATCH_TOO_SMALL
+    assert all(bool((t == 7.0).all()) for t in grads)
+    assert lib.dn_prepass_bwd(s, *at, res, *rest, scratch.numel(), st) == 0
+    assert not any(bool((t == 7.0).all()) for t in grads)
+
+
 # ---- chains cut at document boundaries: inside a chunk, at its start, several in one part, in the last chunk, none at all
 @pytest.mark.parametrize("recompute", [False, True])
 def test_chains_cut_at_documents(dn, recompute):
