@@ -86,12 +86,12 @@ bool force_simt() {
 // 343 us -> 35 us at L = 131072, 25 -> 7 at B = 4 L = 8192, where one CTA per row went through the row alone.
 constexpr int SEG_THREADS = 512;
 __global__ void __launch_bounds__(SEG_THREADS) canonical_segments_kernel(const int32_t* raw, const int32_t* first_is_new,
-                                                                          int32_t* out, int L, int per_cta) {
+                                                                          int32_t* out, int L, int per_cta, int per_row) {
   __shared__ int part[SEG_THREADS / 32], base_s;
-  const int b = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int b = blockIdx.x / per_row, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int32_t* r = raw + (size_t)b * L;
   int32_t* o = out + (size_t)b * L;
-  const int start = blockIdx.x * per_cta, end = min(L, start + per_cta);
+  const int start = (blockIdx.x % per_row) * per_cta, end = min(L, start + per_cta);
   int cnt = 0;
 #pragma unroll 8
   for (int t = 1 + tid; t < start; t += SEG_THREADS) cnt += __ldg(r + t) != __ldg(r + t - 1);
@@ -124,7 +124,8 @@ int launch_canonical_segments(const int32_t* raw, const int32_t* first_is_new, i
                               int B, int L, cudaStream_t st) {
   int per_cta = SEG_THREADS;                             // at most 256 CTAs per row: the counting is quadratic in their number
   while ((L + per_cta - 1) / per_cta > 256) per_cta *= 2;
-  canonical_segments_kernel<<<dim3((L + per_cta - 1) / per_cta, B), SEG_THREADS, 0, st>>>(raw, first_is_new, out, L, per_cta);
+  const int per_row = (L + per_cta - 1) / per_cta;       // (one dimension: any number of rows)
+  canonical_segments_kernel<<<B * per_row, SEG_THREADS, 0, st>>>(raw, first_is_new, out, L, per_cta, per_row);
   return launch_status();
 }
 

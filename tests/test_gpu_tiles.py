@@ -164,6 +164,18 @@ def test_canonical_segments(dn, L):
         assert torch.equal(out.cpu().long(), ref if first is None else ref + first[:, None])
 
 
+# ---- more rows than a launch has in its second dimension, and rows so long that their blocks grow
+@pytest.mark.parametrize("B,L", [(70000, 3), (2, 131072), (2, 131073), (1, 600001)])
+def test_canonical_segments_of_many_and_long_rows(dn, B, L):
+    from deltanet_b200 import _lib
+    raw = (torch.rand(B, L, generator=torch.Generator().manual_seed(62)) < 0.01).int().cumsum(1).int() % 3
+    ref = torch.zeros(B, L, dtype=torch.int64)
+    ref[:, 1:] = (raw[:, 1:] != raw[:, :-1]).long().cumsum(1)
+    dev, out = raw.cuda(), torch.full((B, L), -1, dtype=torch.int32, device="cuda")
+    assert _lib.lib().dn_canonical_segments(dev.data_ptr(), None, out.data_ptr(), B, L, torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(out.cpu().long(), ref)
+
+
 # ---- gate gradients: heads that do not fill a cluster's four, and tokens that do not fill its CTAs
 @pytest.mark.parametrize("B,L,Hv", [(1, 1, 1), (1, 3, 6), (2, 301, 5), (1, 64, 32)])
 def test_gate_gradients(dn, B, L, Hv):
