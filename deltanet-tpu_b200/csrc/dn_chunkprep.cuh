@@ -27,7 +27,7 @@ struct InCfg {
   static constexpr int qkv_dt = MODE == 1 ? DN_F32 : DN_BF16;
 };
 inline int input_mode(const Geo& g) {
-  if (g.K != K || g.gate_dt != DN_F32 || (g.flags & (DN_FUSE_PROLOGUE | DN_STABILITY_GUARD))) return 2;
+  if (g.fine || g.gate_dt != DN_F32 || (g.flags & (DN_FUSE_PROLOGUE | DN_STABILITY_GUARD))) return 2;
   if (g.gC == g.K && g.bC == g.K && g.wC == g.V) return g.qkv_dt == DN_BF16 ? 0 : 1;
   if (g.gC == g.K && g.bC == 1 && g.wC == 1 && g.qkv_dt == DN_BF16) return 4;
   return 2;
@@ -207,13 +207,16 @@ __device__ __forceinline__ void decay8(const float* la, const float* lb, float (
   for (int i = 0; i < 8; ++i) f[i] = umma::ex2_fast(fminf(d[i], 0.f) * DN_LOG2E);
 }
 
+// the second bf16 part of a value: what the first one leaves (together 16 bits)
+__device__ __forceinline__ float low_part(float x) { return x - bf16r(x); }
+
 // Operand images of level s (pairs of adjacent s-row blocks; reference row = first row of the
 // lower block).  Every row has one role per level: rows of the upper blocks (x < ref) carry
 // k_hat * exp(Lam_ref - Lam_x) in BOTH images; rows of the lower blocks carry
 // beta * exp(Lam_x - Lam_ref) in KR and q_hat * exp(Lam_x - Lam_ref) in QK.  All scale factors are
 // <= 1.  One piece (row x, channel group p) per call, stored at image[p*128 + x].
 __device__ __forceinline__ void build_level_from(const float (&kh)[8], const float (&ba)[8], const float (&qh)[8],
-                                                 const float* LAM, int s, int x, int p, uint4* KR, uint4* QK) {
+                                                 const float* LAM, int s, int x, int p, uint4* KR, uint4* QK, bool low = false) {
   const int ref = level_ref(x, s);
   const bool lower = x >= ref;
   float f[8], o1[8], o2[8];
@@ -224,12 +227,16 @@ __device__ __forceinline__ void build_level_from(const float (&kh)[8], const flo
     o1[i] = lower ? (ba[i] * kh[i]) * f[i] : kf;
     o2[i] = lower ? qh[i] * f[i] : kf;
   }
+  if (low) {                       // the images of the second parts
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { o1[i] = low_part(o1[i]); o2[i] = low_part(o2[i]); }
+  }
   KR[p * 128 + x] = umma::pack8(o1);
   QK[p * 128 + x] = umma::pack8(o2);
 }
 // The same from beta = b_act * k_hat already formed (operands cached on chip).
 __device__ __forceinline__ void build_level_from_beta(const float (&kh)[8], const float (&be)[8], const float (&qh)[8],
-                                                      const float* LAM, int s, int x, int p, uint4* KR, uint4* QK) {
+                                                      const float* LAM, int s, int x, int p, uint4* KR, uint4* QK, bool low = false) {
   const int ref = level_ref(x, s);
   const bool lower = x >= ref;
   float f[8], o1[8], o2[8];
@@ -240,15 +247,19 @@ __device__ __forceinline__ void build_level_from_beta(const float (&kh)[8], cons
     o1[i] = lower ? be[i] * f[i] : kf;
     o2[i] = lower ? qh[i] * f[i] : kf;
   }
+  if (low) {                       // the images of the second parts
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { o1[i] = low_part(o1[i]); o2[i] = low_part(o2[i]); }
+  }
   KR[p * 128 + x] = umma::pack8(o1);
   QK[p * 128 + x] = umma::pack8(o2);
 }
-__device__ __forceinline__ void build_level_piece(const Rows& r, const float* LAM, int s, int x, int p, uint4* KR, uint4* QK) {
+__device__ __forceinline__ void build_level_piece(const Rows& r, const float* LAM, int s, int x, int p, uint4* KR, uint4* QK, bool low = false) {
   float kh[8], ba[8], qh[8];
   khat8(r, x, p, kh);              // all three loads are issued before the role is looked at
   bact8(r, x, p, ba);
   qhat8(r, x, p, qh);
-  build_level_from(kh, ba, qh, LAM, s, x, p, KR, QK);
+  build_level_from(kh, ba, qh, LAM, s, x, p, KR, QK, low);
 }
 
 // Which level owns entry (row block bi, column block bj) of the strictly lower block triangle:

@@ -24,6 +24,7 @@ struct Geo {
   int H, Vw, G;          // exec heads, value width of the tiles, value heads per exec head (G V columns of Vw exist)
   int Kt;                // key width of the tiles: 128 on the tensor-core path (K columns exist), else K
   int qk_div;            // q/k head of exec head h is h / qk_div
+  bool fine;             // tensor-core path: factors and cotangents of the intra-chunk matrices in two bf16 parts (make_geo)
   int gH, gC, bH, bC, wH, wC;
   int qkv_dt, gate_dt, pre_dt, prec;
   uint32_t flags;
@@ -78,6 +79,11 @@ inline int make_geo(const dn_shape* s, Geo* g) {
   // tiles with the missing columns zero: even at K = V = 64 with one value head, where three quarters of the products are
   // zeros, that is several times faster than the CUDA-core kernels.  dn_exec_view reports the tile height and value
   // width actually used; every buffer size follows from them.
+  // What the CUDA-core kernels computed in fp32 stays that exact: they build A, M and their cotangents from fp32 factors, and
+  // in one bf16 part the tensor cores lose it (K = V = 64, channel-wise decay: dg 3.4e-3 off 64-bit results on the CUDA cores,
+  // 1.35e-2 with one part).  So the shapes that are new to these tiles take their factors and cotangents in two parts.  K = 128
+  // with 128 or 256 value columns has had one part from the beginning.
+  g->fine = tc && (s->K == 64 || (g->G * s->V != 128 && g->G * s->V != 256));
   g->C = tc ? 128 : s->chunk;
   g->Kt = tc ? 128 : s->K;
   if (tc) g->Vw = g->Vw <= 128 ? 128 : 256;

@@ -233,6 +233,49 @@ __device__ __forceinline__ uint4 ld16_now(const void* p) {
   asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
+// a piece of an image in the CTA's scratch
+__device__ __forceinline__ uint4 keep_piece(const float4* p) {
+  const float4 t = umma::ld_keep4(p);
+  return make_uint4(__float_as_uint(t.x), __float_as_uint(t.y), __float_as_uint(t.z), __float_as_uint(t.w));
+}
+__device__ __forceinline__ void keep_piece(float4* p, uint4 v) {
+  umma::st_keep4(p, make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)));
+}
+// Second parts of a drain's 32 columns, v - bf16(v), piece by piece to `put(piece, bits)`; for the masked kind v as drain_masked
+// forms it, and the second part of its rows times `by` to `put2`.
+template <class PUT>
+__device__ __forceinline__ void drain_low(bool dead, uint32_t addr, int group, PUT put) {
+#pragma unroll 1
+  for (int j = 0; j < 4; ++j) {
+    float v[8];
+    ld8(dead, addr + 8 * j, v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = low_part(v[i]);
+    put(4 * group + j, umma::pack8(v));
+  }
+}
+template <class PUT, class PUT2>
+__device__ __forceinline__ void drain_masked_low(bool dead, uint32_t addr, int row, int group, float sign, const int* seg, const float* lam, float by,
+                                                 PUT put, PUT2 put2) {
+  const int sr = seg[row];
+  const float lr = lam[row] * DN_LOG2E;
+#pragma unroll 1
+  for (int j = 0; j < 4; ++j) {
+    const int c0 = group * 32 + 8 * j;
+    float v[8], w[8];
+    ld8(dead, addr + 8 * j, v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[i] = c0 + i < row && sr == seg[c0 + i] ? sign * v[i] : 0.f;
+      v[i] *= umma::ex2_fast(fminf(lr - lam[c0 + i] * DN_LOG2E, 0.f));
+      const float hi = bf16r(v[i]);
+      w[i] = v[i] * by - bf16r(hi * by);
+      v[i] -= hi;
+    }
+    put(4 * group + j, umma::pack8(v));
+    put2(4 * group + j, umma::pack8(w));
+  }
+}
 template <bool BF>
 struct Piece {                                          // eight elements as loaded
   uint4 a[BF ? 1 : 2];
@@ -253,8 +296,9 @@ struct Piece {                                          // eight elements as loa
 // dv = dY w_act, dw = dY v (+ sigmoid adjoint; summed over a value head's columns when w is one scalar per head, SW) of 128
 // columns, dY from its image.  Bound by the latency of the rows of v and w (2.2 to 3.2 k cycles with every SM here at once), so
 // all of them are requested together; one function per type, because only code that runs takes instruction cache.
-template <bool QBF, bool GBF, bool SW>
-__device__ __noinline__ void v_phase(const PrepassBwdArgs& a, const uint4* img, int half, int h, size_t tok0, int rows, bool fuse) {
+// low (LOW): the second part of dY, an image in global memory.
+template <bool QBF, bool GBF, bool SW, bool LOW>
+__device__ __noinline__ void v_phase(const PrepassBwdArgs& a, const uint4* img, int half, int h, size_t tok0, int rows, bool fuse, const float4* low) {
   const Geo& g = a.g;
   const int rx = threadIdx.x >> 2, rp = threadIdx.x & 3, vr = g.G * g.V, vsh = g.V == 128 ? 7 : 6;
   const bool live = rx < rows;
@@ -282,6 +326,12 @@ __device__ __noinline__ void v_phase(const PrepassBwdArgs& a, const uint4* img, 
       for (int i = 0; i < 8; ++i) ww[i] = ws[it];
     } else wraw[it].get(ww);
     umma::unpack8(img[p * PP + rx], dy);
+    if (LOW) {
+      float lo[8];
+      umma::unpack8(keep_piece(low + p * 128 + rx), lo);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) dy[i] += lo[i];
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       float wa = ww[i], dwv = dy[i] * vv[i];
@@ -303,7 +353,8 @@ __device__ __noinline__ void v_phase(const PrepassBwdArgs& a, const uint4* img, 
   }
 }
 
-template <int VW, int MODE, bool SC>
+// FINE (scalar gates; see make_geo): dA, dM, dX and dY take part in two bf16 parts.  k_hat and q_hat have one.
+template <int VW, int MODE, bool SC, bool FINE = false>
 __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_constant__ PrepassBwdArgs a) {
   using CF = InCfg<MODE>;
   constexpr int NH = VW / 128;
@@ -347,6 +398,9 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
   const int wC = CF::fixed && !SC ? (CF::scalar_bw ? 1 : g.V) : g.wC;
   const uint32_t qes = qdt == DN_BF16 ? 2 : 4, ges = gdt == DN_BF16 ? 2 : 4;
   const int vr = g.G * g.V;                             // value columns that exist
+  // second parts that wait for their use (behind the sums of dq and dk): dM's, then those of the halves of dY
+  float4* const low_M = reinterpret_cast<float4*>(a.scratch + (size_t)blockIdx.x * a.scratch_per_cta) + 8192;
+  float4* const low_Y = low_M + 2048;
 
   // A CTA takes the D heads that share a key head one after the other and adds up their dq and dk in its scratch (see
   // prepass_bwd_grouped); otherwise D = 1.
@@ -391,7 +445,11 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     }
     // V_new = U - W S, in the place of U; dM masked (scalar gates: decayed), its diagonal apart
     auto vnew = [&](int slot, uint32_t col) { drain_sub(cx.dead, tb + col, sl.at(slot), row, group); };
-    auto drain_dM = [&](int slot) { drain_masked(cx.dead, tb + T_TMP, sl.at(slot), row, group, 1.f, seg_s, SC ? lam_s : nullptr, dmi_s); };
+    auto drain_dM = [&](int slot) {
+      drain_masked(cx.dead, tb + T_TMP, sl.at(slot), row, group, 1.f, seg_s, SC ? lam_s : nullptr, dmi_s);
+      if constexpr (FINE)
+        drain_masked_low(cx.dead, tb + T_TMP, row, group, 1.f, seg_s, lam_s, 0.f, [&](int p, uint4 v) { keep_piece(low_M + p * 128 + row, v); }, [](int, uint4) {});
+    };
     auto drain_neg = [&](int slot, uint32_t col) { drain_plain(cx.dead, tb + col, sl.at(slot), 128, row, group, -1.f); };
     sl.wait(0);
     sl.wait(1);
@@ -526,10 +584,20 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       }
       drain_plain(cx.dead, tb + T_B, sl.at(slot), 128, row, group, 1.f);
     };
-    auto drain_dY = [&](int slot) { drain_plain(cx.dead, tb + T_TMP, sl.at(slot), PP, row, group, 1.f); };
+    auto drain_dY = [&](int slot, int half) {
+      drain_plain(cx.dead, tb + T_TMP, sl.at(slot), PP, row, group, 1.f);
+      if constexpr (FINE)                               // (trunc: dY has one part)
+        drain_low(cx.dead, tb + T_TMP, group, [&](int p, uint4 v) { keep_piece(low_Y + half * 2048 + p * 128 + row, trunc ? make_uint4(0, 0, 0, 0) : v); });
+    };
+    // (the calls below put a barrier behind these; a thread reads back what it wrote)
+    auto low_dX = [&](int slot) { drain_low(cx.dead, tb + T_B, group, [&](int p, uint4 v) { sl.at(slot)[p * 128 + row] = v; }); };
+    auto low_dY = [&](int slot, int half) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sl.at(slot)[(4 * group + j) * 128 + row] = keep_piece(low_Y + half * 2048 + (4 * group + j) * 128 + row);
+    };
     auto vphase = [&](int slot, int half) {
       auto go = [&](auto qbf, auto gbf, auto scalar) {
-        v_phase<decltype(qbf)::value, decltype(gbf)::value, decltype(scalar)::value>(a, sl.at(slot), half, h, tok0, rows, fuse);
+        v_phase<decltype(qbf)::value, decltype(gbf)::value, decltype(scalar)::value, FINE>(a, sl.at(slot), half, h, tok0, rows, fuse, low_Y + half * 2048);
       };
       constexpr std::true_type yes{};
       constexpr std::false_type no{};
@@ -543,27 +611,36 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     };
     if constexpr (NH == 1) {
       drain_dX(0);
-      drain_dY(1);
+      drain_dY(1, 0);
+      if constexpr (FINE) low_dY(3, 0);
       sl.wait(2);
       sl.wait(4);
       umma::pre_issue_sync();
       product<128, false, false>(cx, sl.at(0), 2048, sl.at(2), 2048, 128, T_TMP, false);                   // -dA = dX W^T + dY U^T
       product<128, false, false>(cx, sl.at(1), PB, sl.at(4), 2048, 128, T_TMP, true);
+      if constexpr (FINE) product<128, false, false>(cx, sl.at(3), 2048, sl.at(4), 2048, 128, T_TMP, true);
       commit(cx);
       vphase(1, 0);
       finish(cx);
+      if constexpr (FINE) {
+        low_dX(0);
+        umma::pre_issue_sync();
+        product<128, false, false>(cx, sl.at(0), 2048, sl.at(2), 2048, 128, T_TMP, true);
+        commit(cx);
+        finish(cx);
+      }
     } else {
       sl.load(0, dVg);
       sl.load(1, Wg);
       drain_dX(3);
-      drain_dY(4);
+      drain_dY(4, 1);
       sl.wait(0);
       umma::pre_issue_sync();
       product<128, true, true>(cx, sl.at(2), 2048, sl.at(0), 2048, C, T_TMP, false);                       // dY: first half
       commit(cx);
       finish(cx);
       sl.load(0, Ug);
-      drain_dY(2);
+      drain_dY(2, 0);
       sl.wait(0);
       sl.wait(1);
       umma::pre_issue_sync();
@@ -571,6 +648,18 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       product<128, false, false>(cx, sl.at(2), PB, sl.at(0), 2048, 128, T_TMP, true);
       commit(cx);
       finish(cx);
+      if constexpr (FINE) {
+        low_dX(3);
+        umma::pre_issue_sync();
+        product<128, false, false>(cx, sl.at(3), 2048, sl.at(1), 2048, 128, T_TMP, true);
+        commit(cx);
+        finish(cx);
+        low_dY(1, 0);
+        umma::pre_issue_sync();
+        product<128, false, false>(cx, sl.at(1), 2048, sl.at(0), 2048, 128, T_TMP, true);
+        commit(cx);
+        finish(cx);
+      }
       sl.load(0, Ug + HN);
       vphase(2, 0);
       sl.wait(0);
@@ -578,6 +667,13 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       commit(cx);
       vphase(4, 1);
       finish(cx);
+      if constexpr (FINE) {
+        low_dY(1, 1);
+        umma::pre_issue_sync();
+        product<128, false, false>(cx, sl.at(1), 2048, sl.at(0), 2048, 128, T_TMP, true);
+        commit(cx);
+        finish(cx);
+      }
     }
     // ---- dA (dM is in slot 5); everything else is free
     uint4 *const dAi = sl.region(4), *const dMi = sl.at(5), *const dAb = SC ? sl.region(2) : nullptr;
@@ -768,6 +864,19 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       product<128, true, true>(cx, dMi, 2048, QI, PB, C, T_K, true);        // (dM f)^T q_hat
       commit(cx);
       finish(cx);
+      if constexpr (FINE) {                             // the same on the second parts
+        drain_masked_low(cx.dead, tb + T_TMP, row, group, -1.f, seg_s, lam_s, bet_s[row], [&](int p, uint4 v) { dAi[p * 128 + row] = v; },
+                         [&](int p, uint4 v) { dAb[p * 128 + row] = v; });
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dMi[(4 * group + j) * 128 + row] = keep_piece(low_M + (4 * group + j) * 128 + row);
+        umma::pre_issue_sync();
+        product<128, false, true>(cx, dAi, 2048, KI, PB, C, T_B, true);
+        product<128, false, true>(cx, dMi, 2048, KI, PB, C, T_Q, true);
+        product<128, true, true>(cx, dAb, 2048, KI, PB, C, T_K, true);
+        product<128, true, true>(cx, dMi, 2048, QI, PB, C, T_K, true);
+        commit(cx);
+        finish(cx);
+      }
     } else {
       // Two rounds of 64 channels: what the images take beside Lambda, dA and dM.  (Four rounds of 32 with two sets of images
       // overlapped building and products, but at 32 columns an MMA costs 46 cycles and at 64 it costs 48: 18.7 k cycles
@@ -1181,7 +1290,10 @@ int launch_prepass_bwd_fast(const PrepassBwdArgs& a, cudaStream_t st) {
   };
   auto pick = [&](auto vw) {
     constexpr int VW = decltype(vw)::value;
-    if (prepass_bwd_scalar_route(g)) { go(prepass_bwd_fast_kernel<VW, 2, true>); return; }
+    if (prepass_bwd_scalar_route(g)) {
+      if (g.fine) go(prepass_bwd_fast_kernel<VW, 2, true, true>); else go(prepass_bwd_fast_kernel<VW, 2, true>);
+      return;
+    }
     switch (input_mode(g)) {
       case 0: go(prepass_bwd_fast_kernel<VW, 0, false>); break;
       case 1: go(prepass_bwd_fast_kernel<VW, 1, false>); break;

@@ -187,6 +187,8 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
       }
     };
 
+    // second part of dY, for fine shapes: in the scratch that phase D begins with
+    float4* const dY_low = reinterpret_cast<float4*>(DBP);
     // ---- G. the matrix products (and dLambda_end from the carried state)
     {
       BwdTcIo io;
@@ -207,6 +209,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
       io.DQE = DQE; io.DKE = DKE; io.DX = DX; io.DM = DM; io.DA = DA;
       io.dlend_s = dlend_s; io.all_same = all_same;
       io.seg_s = seg_s; io.trunc = trunc;
+      io.dY_low = !CF::fixed && g.fine && !trunc ? dY_low : nullptr;
       // the rows of v and w of the first value head are requested as soon as the products are done: they
       // travel while the last accumulator drains (phase V below waits for them)
       bwd_gemms_tc<VW, NT>(cx, smraw, io, imgld, [&]() {
@@ -281,6 +284,13 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
           load8(a.w, (tokr * g.wH + g.w_head(hv)) * wC + cv, gdt, ww);
         }
         umma::unpack8(reinterpret_cast<const uint4*>(smraw)[p * 128 + x], dy);
+        if (!CF::fixed && g.fine && !trunc) {
+          const float4 t = umma::ld_keep4(dY_low + p * 128 + x);
+          float lo[8];
+          umma::unpack8(make_uint4(__float_as_uint(t.x), __float_as_uint(t.y), __float_as_uint(t.z), __float_as_uint(t.w)), lo);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) dy[i] += lo[i];
+        }
         if (live) {
           const size_t vrow = tok * g.Hv * g.V + col0;
 #pragma unroll
@@ -410,8 +420,8 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
     }
 
     // ---- H. three levels
-    auto build = [&](int lv) {
-      const int s = 16 << lv;
+    const bool fine = !CF::fixed && g.fine;              // factors and cotangents in two parts (see make_geo)
+    auto build_cotangents = [&](int lv, bool low) {
       static_assert(IMG == 4 * NT, "four pieces per thread");
 #pragma unroll
       for (int half = 0; half < 2; ++half) {           // dA_s, dM_s: the entries this level owns
@@ -428,12 +438,19 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const int e = (2 * half + u) * NT + tid;
+          if (low) {
+            auto rest = [](float4& v) { v = make_float4(low_part(v.x), low_part(v.y), low_part(v.z), low_part(v.w)); };
+            rest(a0[u]); rest(a1[u]); rest(m0[u]); rest(m1[u]);
+          }
           uint4 va = make_uint4(umma::pack2(a0[u].x, a0[u].y), umma::pack2(a0[u].z, a0[u].w), umma::pack2(a1[u].x, a1[u].y), umma::pack2(a1[u].z, a1[u].w));
           uint4 vm = make_uint4(umma::pack2(m0[u].x, m0[u].y), umma::pack2(m0[u].z, m0[u].w), umma::pack2(m1[u].x, m1[u].y), umma::pack2(m1[u].z, m1[u].w));
           I_DA[e] = va;
           I_DM[e] = vm;
         }
       }
+    };
+    auto build_factors = [&](int lv, bool low) {
+      const int s = 16 << lv;
       if (tm_cache) {
         const int x = (warp & 3) * 32 + lane;
         const uint32_t tl = cx.tmem + ((uint32_t)((warp & 3) * 32) << 16);
@@ -448,11 +465,11 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
             kh[i] = __uint_as_float(__float_as_uint(kq[i]) << 16);
             qh[i] = __uint_as_float(__float_as_uint(kq[i]) & 0xffff0000u);
           }
-          build_level_from_beta(kh, be8, qh, LAM, s, x, p, I_KR, I_QK);
+          build_level_from_beta(kh, be8, qh, LAM, s, x, p, I_KR, I_QK, low);
         }
       } else {
 #pragma unroll 2
-        for (int it = 0; it < 4; ++it) build_level_piece(r, LAM, s, myrow, it * 4 + lgrp, I_KR, I_QK);
+        for (int it = 0; it < 4; ++it) build_level_piece(r, LAM, s, myrow, it * 4 + lgrp, I_KR, I_QK, low);
       }
     };
     auto drain_level = [&](int lv) {
@@ -501,15 +518,21 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
     // images are free once the products of lv - 1 have completed), then the products of lv are issued
 #pragma unroll 1
     for (int lv = 0; lv <= 3; ++lv) {
-      if (lv < 3) build(lv);
+      if (lv < 3) { build_cotangents(lv, false); build_factors(lv, false); }
       if (lv > 0) drain_level(lv - 1);
       if (lv < 3) {
-        umma::pre_issue_sync();
-        umma::issue<128, false, true>(cx, I_DA, I_KR, C, 0, false);        // dA_s   KR
-        umma::issue<128, true, true>(cx, I_DA, I_KR, C, 0, true);          // dA_s^T KR
-        umma::issue<128, false, true>(cx, I_DM, I_QK, C, 128, false);      // dM_s   QK
-        umma::issue<128, true, true>(cx, I_DM, I_QK, C, 128, true);        // dM_s^T QK
-        umma::commit_wait(cx);
+        // (fine: first parts, then the factors' second parts, then the cotangents')
+#pragma unroll 1
+        for (int part = 0; part < (fine ? 3 : 1); ++part) {
+          if (part == 1) build_factors(lv, true);
+          if (part == 2) { build_cotangents(lv, true); build_factors(lv, false); }
+          umma::pre_issue_sync();
+          umma::issue<128, false, true>(cx, I_DA, I_KR, C, 0, part > 0);     // dA_s   KR
+          umma::issue<128, true, true>(cx, I_DA, I_KR, C, 0, true);          // dA_s^T KR
+          umma::issue<128, false, true>(cx, I_DM, I_QK, C, 128, part > 0);   // dM_s   QK
+          umma::issue<128, true, true>(cx, I_DM, I_QK, C, 128, true);        // dM_s^T QK
+          umma::commit_wait(cx);
+        }
       }
     }
     __syncthreads();
@@ -727,13 +750,15 @@ int launch_prepass_bwd_tc(PrepassBwdArgs& a, size_t scratch_floats, cudaStream_t
   if (a.items <= 0) return DN_OK;
   a.scratch_per_cta = prepass_bwd_tc_scratch_per_cta(g);
   a.err = device_error_ptr();
-  // both kernels' needs, before either is enqueued: the sums over a key head's heads, the strong tiles' matrices
+  // both kernels' needs, before either is enqueued: the sums over a key head's heads, second parts; the strong tiles' matrices
   const int grid = a.items < sm_count() ? a.items : sm_count();
   const bool scalar = prepass_bwd_scalar_route(g);
-  const size_t ctas = scalar ? (a.group > 1 ? sm_count() : 0) : grid;
+  const size_t ctas = scalar ? (a.group > 1 ? sm_count() : (g.fine ? grid : 0)) : grid;
   if (scratch_floats < ctas * a.scratch_per_cta) return DN_ERR_SCRATCH_TOO_SMALL;
-  int rc = launch_prepass_bwd_fast(a, st);
-  if (rc || scalar) return rc;
+  if (scalar || !g.fine) {                               // (fine, decay per channel: every tile is this file's)
+    int rc = launch_prepass_bwd_fast(a, st);
+    if (rc || scalar) return rc;
+  }
   const size_t lam_phase = (size_t)C * LP * 4 + 4 * 32768;
   size_t smem = bwd_tc_image_bytes(g.Vw);
   if (smem < lam_phase) smem = lam_phase;

@@ -51,6 +51,7 @@ struct BwdTcIo {
   bool all_same;
   const int* seg_s;
   bool trunc;
+  float4* dY_low;                      // fine shapes: where the second part of dY goes (image layout, global), else null
 };
 
 // dO staging.  A warp covers 8 rows x 4 panels per step: its 32 global loads fall in 8 row
@@ -217,10 +218,21 @@ __device__ __forceinline__ void bwd_gemms_tc(umma::Ctx& cx, uint8_t* img, const 
     Y2[(col / 8) * 128 + row] = umma::pack8p(r);
     Y2[(col / 8 + 1) * 128 + row] = umma::pack8p(r + 8);
   });
-  // dY is kept only as its bf16 image X: operand of step 6, and read again by the caller for dv, dw
+  // dY is kept only as its bf16 image X: operand of step 6, and read again by the caller for dv, dw (fine shapes: with what
+  // the image leaves)
   umma::drain<NT, VW>(cx, 256, [&](int row, int col, const float (&v)[16]) {
     X[(col / 8) * 128 + row] = umma::pack8p(v);
     X[(col / 8 + 1) * 128 + row] = umma::pack8p(v + 8);
+    if (io.dY_low) {
+      float lo[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) lo[i] = v[i] - bf16r(v[i]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint4 u = umma::pack8p(lo + 8 * h);
+        umma::st_keep4(io.dY_low + (col / 8 + h) * 128 + row, make_float4(__uint_as_float(u.x), __uint_as_float(u.y), __uint_as_float(u.z), __uint_as_float(u.w)));
+      }
+    }
   });
 
   // ---- 6. dA = -(dX W^T + dY U^T), strictly lower and same document
@@ -229,6 +241,35 @@ __device__ __forceinline__ void bwd_gemms_tc(umma::Ctx& cx, uint8_t* img, const 
   umma::issue<128, false, false>(cx, Y2, P, 128, 0, false);
   umma::issue<128, false, false>(cx, X, Z, VW, 0, true);
   umma::commit_wait(cx);
+  if (io.dY_low) {
+    // the second parts of dX, then of dY by halves of 128 columns (T's place holds one such image)
+    const int row = (threadIdx.x >> 5 & 3) * 32 + (threadIdx.x & 31), group = threadIdx.x >> 7;
+    constexpr int PER = 128 / (NT / 128);
+#pragma unroll 1
+    for (int c = 0; c < PER; c += 8) {
+      const int col = group * PER + c;
+      const float4 u0 = umma::ld_keep4(DX4 + p4v(row, col)), u1 = umma::ld_keep4(DX4 + p4v(row, col + 4));
+      float v[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] -= bf16r(v[i]);
+      Y2[(col / 8) * 128 + row] = umma::pack8(v);
+    }
+    umma::pre_issue_sync();
+    umma::issue<128, false, false>(cx, Y2, P, 128, 0, true);
+#pragma unroll 1
+    for (int h = 0; h < VW / 128; ++h) {
+      umma::drain<NT, 128>(cx, 256 + 128 * h, [&](int rw, int col, const float (&v)[16]) {
+        float lo[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) lo[i] = v[i] - bf16r(v[i]);
+        Y[(col / 8) * 128 + rw] = umma::pack8p(lo);
+        Y[(col / 8 + 1) * 128 + rw] = umma::pack8p(lo + 8);
+      });
+      umma::pre_issue_sync();
+      umma::issue<128, false, false>(cx, Y, Z + 2048 * h, 128, 0, true);
+      umma::commit_wait(cx);
+    }
+  }
   after_products();
   umma::drain<NT, 128>(cx, 0, [&](int row, int col, const float (&v)[16]) {
     float m[16];

@@ -447,7 +447,12 @@ __device__ __noinline__ void strong_route(const PrepassFwdArgs& a, int b, int h,
   uint4* Mimg = reinterpret_cast<uint4*>(M);
   uint4* QE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.qe) + ibase * C * K);
   uint4* KE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.ke) + ibase * C * K);
-  const bool first = seg_s[x] == seg_s[0], last = seg_s[x] == seg_s[C - 1];
+  const bool first = seg_s[x] == seg_s[0], last = seg_s[x] == seg_s[C - 1], live = x < r.rows_valid;     // (other rows read row 0)
+  const size_t x0 = live ? x : 0;
+  const uint8_t* krow = reinterpret_cast<const uint8_t*>(r.k) + (r.qk_row0 + x0 * r.qk_pitch) * dt_size(r.qkv_dt);
+  const uint8_t* qrow = reinterpret_cast<const uint8_t*>(r.q) + (r.qk_row0 + x0 * r.qk_pitch) * dt_size(r.qkv_dt);
+  const uint8_t* brow = reinterpret_cast<const uint8_t*>(r.b) + (r.b_row0 + x0 * r.b_pitch) * dt_size(r.gate_dt);
+  const float rq = rq_s[x], rk = rk_s[x], b1 = r.bC == 1 ? ldf_ro(brow, 0, r.gate_dt) : 0.f;
   // diagonal blocks, 32 rows (two blocks) at a time: a thread takes a pair (i > j) and half of the group's channels
   const int dblk = (tid >> 1) / 120, ch = 16 * (tid & 1);
   int di = 1, dj = (tid >> 1) % 120;
@@ -463,38 +468,67 @@ __device__ __noinline__ void strong_route(const PrepassFwdArgs& a, int b, int h,
       continue;
     }
     float gv[8], kh[8], qh[8], be[8];
+    const Raw8 kr = ldraw(krow, p, r.qkv_dt), qr = ldraw(qrow, p, r.qkv_dt);      // all of the group's loads together
+    Raw8 br;
+    if (r.bC != 1) br = ldraw(brow, p, r.gate_dt);
     load_decay(r, grp, warp, lane, gv);
-    khat8(r, x, p, kh);
-    qhat8(r, x, p, qh);
-    bact8(r, x, p, be);
+    if (4 * (grp + 1) < r.kp) {                         // the next group's lines of g and b: the next load of them is exposed
+      const int row = warp * 8 + (lane & 7), es = r.gate_dt == DN_BF16 ? 2 : 4;
+      const bool isg = lane < 8;
+      if (lane < 16 && row < r.rows_valid && (isg ? r.gC : r.bC) != 1)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t*>(isg ? r.gg : r.b) +
+                     ((isg ? r.g_row0 + row * r.g_pitch : r.b_row0 + row * r.b_pitch) + 32 * (grp + 1)) * es));
+    }
+    cvraw(kr, r.qkv_dt, kh);
+    cvraw(qr, r.qkv_dt, qh);
+    if (r.bC != 1) cvraw(br, r.gate_dt, be);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { accD = fmaf(qh[i], kh[i], accD); be[i] *= kh[i]; }
+    for (int i = 0; i < 8; ++i) {
+      kh[i] = live ? kh[i] * rk : 0.f;
+      qh[i] = live ? qh[i] * rq * r.scale : 0.f;
+      if (r.round_in) { kh[i] = bf16r(kh[i]); qh[i] = bf16r(qh[i]); }
+      if (r.bC == 1) be[i] = b1;
+      if (r.fuse) be[i] = 1.f / (1.f + expf(-be[i])); else if (r.guard) be[i] = fmaxf(be[i], 0.f);
+      be[i] *= kh[i];                                   // beta
+      accD = fmaf(qh[i], kh[i], accD);
+    }
     __syncthreads();
     const int nr = scan_rows(seg_s, warp, lane, gv, TOT, rst_s);
     __syncthreads();
     chain_rows(warp, lane, gv, nr, TOT, rst_s, LAM);
     __syncthreads();
     if (warp == 15) a.res.lam_end[ibase * K + 32 * grp + lane] = LAM[(C - 1) * LQ + lane];
+    // the images of a level: `rows` the lower rows' part of beta and q, `columns` the upper rows' of k (0, 1: first, second, -1: as it is)
+    auto levels = [&](int rows, int columns) {
 #pragma unroll 1
-    for (int lv = 0; lv < 3; ++lv) {
-      const int s = 16 << lv, ref = level_ref(x, s), at = ((x >> (5 + lv)) << (4 + lv)) + (x & (s - 1));
-      const bool lower = x >= ref;
-      uint4* I = LV + lv * LV_SIZE;
-      float f[8], o[8];
-      decay8(LAM + (lower ? x : ref) * LQ + 8 * lgrp, LAM + (lower ? ref : x) * LQ + 8 * lgrp, f);
-      if (lower) {
+      for (int lv = 0; lv < 3; ++lv) {
+        const int s = 16 << lv, ref = level_ref(x, s), at = ((x >> (5 + lv)) << (4 + lv)) + (x & (s - 1));
+        const bool lower = x >= ref;
+        uint4* I = LV + lv * LV_SIZE;
+        float f[8], o[8];
+        decay8(LAM + (lower ? x : ref) * LQ + 8 * lgrp, LAM + (lower ? ref : x) * LQ + 8 * lgrp, f);
+        if (lower && rows >= 0) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = be[i] * f[i];
-        I[lgrp * PP + at] = umma::pack8(o);
+          for (int i = 0; i < 8; ++i) { o[i] = be[i] * f[i]; if (rows) o[i] = low_part(o[i]); }
+          I[lgrp * PP + at] = umma::pack8(o);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = qh[i] * f[i];
-        I[lgrp * PP + 64 + at] = umma::pack8(o);
-      } else {
+          for (int i = 0; i < 8; ++i) { o[i] = qh[i] * f[i]; if (rows) o[i] = low_part(o[i]); }
+          I[lgrp * PP + 64 + at] = umma::pack8(o);
+        } else if (!lower && columns >= 0) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = kh[i] * f[i];
-        I[LV_B + lgrp * LV_PITCH + at] = umma::pack8(o);
+          for (int i = 0; i < 8; ++i) { o[i] = kh[i] * f[i]; if (columns) o[i] = low_part(o[i]); }
+          I[LV_B + lgrp * LV_PITCH + at] = umma::pack8(o);
+        }
       }
-    }
+    };
+    auto products = [&](bool accumulate) {
+      umma::pre_issue_sync();
+#pragma unroll
+      for (int lv = 0; lv < 3; ++lv)
+        umma::issue_pitched<64, false, false>(cx, LV + lv * LV_SIZE, PB, LV + lv * LV_SIZE + LV_B, LV_PITCH * 16, 32, 64 * lv, accumulate);
+      umma::commit(cx);
+    };
+    levels(0, 0);
     {                                                   // X, qe, ke
       float o[8];
 #pragma unroll
@@ -508,11 +542,7 @@ __device__ __noinline__ void strong_route(const PrepassFwdArgs& a, int b, int h,
         o[i] = last ? kh[i] * umma::exp_neg(fminf(LAM[(C - 1) * LQ + 8 * lgrp + i] - LAM[x * LQ + 8 * lgrp + i], 0.f)) : 0.f;
       KE[p * 128 + x] = umma::pack8(o);
     }
-    umma::pre_issue_sync();
-#pragma unroll 1
-    for (int lv = 0; lv < 3; ++lv)
-      umma::issue_pitched<64, false, false>(cx, LV + lv * LV_SIZE, PB, LV + lv * LV_SIZE + LV_B, LV_PITCH * 16, 32, 64 * lv, grp > 0);
-    umma::commit(cx);
+    products(grp > 0);
 #pragma unroll
     for (int ps = 0; ps < 4; ++ps) {                    // diagonal blocks, beside the products
       if ((warp >> 2) == ps) {
@@ -537,6 +567,14 @@ __device__ __noinline__ void strong_route(const PrepassFwdArgs& a, int b, int h,
       __syncthreads();
     }
     umma::commit_wait_cta(cx);
+    if (!InCfg<MODE>::fixed && a.g.fine) {              // second parts of the rows, then of the columns (see make_geo)
+      levels(1, -1);
+      products(true);
+      umma::commit_wait_cta(cx);
+      levels(0, 1);
+      products(true);
+      umma::commit_wait_cta(cx);
+    }
   }
   // ---- zeros on and above the diagonal, then the diagonal blocks and the levels' blocks
   {
@@ -595,7 +633,6 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
   __shared__ uint32_t tbase;
   __shared__ int seg_s[C];
   __shared__ int rst_s[16];
-  __shared__ int strong_s;
   __shared__ float rq_s[C], rk_s[C];
   __shared__ uint8_t ds_s[C], de_s[C];                  // first / last row of each row's document inside the tile
   const Geo& g = a.g;
@@ -658,7 +695,6 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
     };
     load_g(0);
     if (tid < C) seg_s[tid] = seg_at(a.seg, b, t0 + tid, g.L);
-    if (tid == 0) strong_s = 0;
     float rq = 1.f, rk = 1.f;
     if (l2) {
       float sq = 0.f, sk = 0.f;
@@ -707,11 +743,13 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
     const int nr = cuts ? __ffs(cuts) - 1 : 8;
     if (lane == 0) rst_s[warp] = cuts != 0;
     EDGE[64 + lane] = 0.f;
-    bool strong = false;
+    bool strong = false, any_strong = false;
     const bool first = seg_s[x] == seg_s[0], last = seg_s[x] == seg_s[C - 1];
     int grp = 0;
+    const bool fine = !CF::fixed && g.fine;              // the hierarchical route has an exact diagonal and factors in two parts
+    any_strong = fine;
 #pragma unroll 1
-    for (; grp < 4; ++grp) {
+    for (; grp < 4 && !fine; ++grp) {
       act_g();
       if (cuts == 0) {
 #pragma unroll
@@ -722,7 +760,6 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       }
       TOT[warp * 32 + lane] = gv[7];
       __syncthreads();
-      if (strong_s) break;                              // found by the group before (nobody writes it between these two barriers)
       // rows above hand on the sums back to the last warp in which a document starts
       const uint32_t above = __ballot_sync(0xffffffffu, lane < warp && rst_s[lane & 15]);
       float carry = 0.f;
@@ -787,11 +824,14 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
         o2[i] = qh[i] * f;
         o3[i] = be[i] * f;
       }
-      if (strong) strong_s = 1;
       KF[lgrp * PP + x] = umma::pack8(o1);
       QF[lgrp * PP + x] = umma::pack8(o2);
       BF[lgrp * PP + x] = umma::pack8(o3);
-      umma::pre_issue_sync();
+      umma::fence_async_smem();                         // umma::pre_issue_sync(), with a vote
+      umma::tc_fence_before();
+      any_strong = __syncthreads_or(strong) != 0;
+      umma::tc_fence_after();
+      if (any_strong) break;
       umma::issue_pitched<128, false, false>(cx, BF, PB, KF, PB, 32, 0, grp > 0);        // A += (beta f) (k / f)^T
       umma::issue_pitched<128, false, false>(cx, QF, PB, KF, PB, 32, 128, grp > 0);      // M += (q f) (k / f)^T
       if (tid < 32 && !cx.dead) umma::mma_commit_warp(&gbar[grp & 1]);
@@ -815,11 +855,10 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       }
       if (grp < 3) { load_g(grp + 1); load_kqb(grp + 1); }
     }
-    bool ok = group_wait((grp - 1) & 1);                 // the last two groups' products
-    if (grp > 1) ok = group_wait(grp & 1) && ok;
+    bool ok = grp == 0 || group_wait((grp - 1) & 1);     // the products nobody has waited for: the last two groups', or where
+    if (grp == 4) ok = group_wait(0) && ok;             //   the walk ended early the last group's
     if (__syncthreads_or(!ok)) { cx.dead = true; umma::report_timeout(err); }
     umma::tc_fence_after();
-    const bool any_strong = __syncthreads_or(strong);
     if (a.res.T) {                                      // the backward takes the same route
       float* ex = tile_extra(a.res, ibase);
       if (tid == 0) *reinterpret_cast<int*>(ex) = any_strong;

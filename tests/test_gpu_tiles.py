@@ -81,6 +81,31 @@ def test_bf16_narrow_heads(dn, K, V, Hk, Hv, L, recompute):
             lambda t, i: O.chunk_gdn2(*t, segment_ids=seg, initial_state=i, **kw), ins, tol=BF16_TOL, init=init)
 
 
+# ---- the same heads against 64-bit results.  W, U, V_new, the state, T and the cotangents enter products as bf16 on any path,
+# up to eight roundings of 2^-9 / sqrt(3) in a row, 3.2e-3; factors of the intra-chunk matrices and the cotangents of these matrices
+# are exact to 16 bits, so nothing is added to that.  (One bf16 part for those: dg 1.3e-2 for decay per channel.)
+@pytest.mark.parametrize("K,V,Hk,Hv,per_channel,strong,dtype",
+                         [(64, 64, 1, 2, True, 1.0, torch.bfloat16), (64, 64, 1, 2, True, 3.0, torch.bfloat16), (64, 128, 1, 2, True, 1.0, torch.float32),
+                          (128, 64, 1, 1, True, 1.0, torch.bfloat16), (128, 64, 1, 3, True, 1.0, torch.float32), (64, 64, 2, 2, False, 1.0, torch.float32),
+                          (64, 64, 1, 3, False, 1.0, torch.bfloat16), (128, 64, 2, 2, False, 1.0, torch.bfloat16), (64, 128, 1, 2, False, 1.0, torch.bfloat16)])
+@pytest.mark.parametrize("trunc", [False, True])
+def test_narrow_heads_against_64_bits(dn, K, V, Hk, Hv, per_channel, strong, dtype, trunc):
+    L = 300
+    ins = list(O.make_inputs(47, 1, L, Hk, Hv, K, V, qkv_dtype=dtype, gate_layout="channel" if per_channel else "scalar_hv")[:6])
+    ins[3] = ins[3] * strong
+    seg = docs(1, L, 90, 200)
+    exact = [t.double().requires_grad_() for t in ins]
+    ref = O.token_serial_gdn2(*exact, segment_ids=seg, qk_l2norm=True)
+    cot = torch.randn(ref.shape, generator=torch.Generator().manual_seed(48)).to(dtype)
+    ref = (ref,) + torch.autograd.grad(ref, exact, cot.double())
+    dev = [t.cuda().requires_grad_() for t in ins]
+    out = dn.chunk_gdn2(*dev, segment_ids=seg.cuda(), qk_l2norm=True, precision="bf16", truncate_bwd_dT_bf16=trunc)
+    got = (out,) + torch.autograd.grad(out, dev, cot.cuda())
+    errs = [O.rel_l2(x.float().cpu(), y) for x, y in zip(got, ref)]
+    # inputs, outputs and the l2-normalised rows in bf16 add a rounding each; dX and dY cut to bf16 where asked for add another
+    assert max(errs) < (5e-3 if not trunc else 7e-3), errs
+
+
 # ---- strong decay: seen in each of the four channel groups, in every channel, by one document of a tile only
 @pytest.mark.parametrize("channels", [slice(0, 1), slice(40, 41), slice(70, 71), slice(127, 128), slice(None)])
 @pytest.mark.parametrize("L", [33, 300])
