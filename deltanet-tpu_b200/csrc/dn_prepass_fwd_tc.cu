@@ -743,11 +743,9 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
     const int nr = cuts ? __ffs(cuts) - 1 : 8;
     if (lane == 0) rst_s[warp] = cuts != 0;
     EDGE[64 + lane] = 0.f;
-    bool strong = false, any_strong = false;
     const bool first = seg_s[x] == seg_s[0], last = seg_s[x] == seg_s[C - 1];
     int grp = 0;
     const bool fine = !CF::fixed && g.fine;              // the hierarchical route has an exact diagonal and factors in two parts
-    any_strong = fine;
 #pragma unroll 1
     for (; grp < 4 && !fine; ++grp) {
       act_g();
@@ -770,7 +768,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
         LAM[(warp * 8 + i) * LQ + lane] = gv[i] * DN_LOG2E;
       }
       const float lam_last = gv[7];
-      bool ok = true;
+      bool ok = true, strong = false;
       if (grp >= 2) ok = group_wait(grp & 1);           // the set this group writes was read by the products of group - 2
       if (__syncthreads_or(!ok)) { cx.dead = true; umma::report_timeout(err); }
       uint4* KF = reinterpret_cast<uint4*>(sm + OFF_GI + (grp & 1) * 3 * 4 * PB);
@@ -829,9 +827,9 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       BF[lgrp * PP + x] = umma::pack8(o3);
       umma::fence_async_smem();                         // umma::pre_issue_sync(), with a vote
       umma::tc_fence_before();
-      any_strong = __syncthreads_or(strong) != 0;
+      const bool stop = __syncthreads_or(strong) != 0;
       umma::tc_fence_after();
-      if (any_strong) break;
+      if (stop) break;
       umma::issue_pitched<128, false, false>(cx, BF, PB, KF, PB, 32, 0, grp > 0);        // A += (beta f) (k / f)^T
       umma::issue_pitched<128, false, false>(cx, QF, PB, KF, PB, 32, 128, grp > 0);      // M += (q f) (k / f)^T
       if (tid < 32 && !cx.dead) umma::mma_commit_warp(&gbar[grp & 1]);
@@ -859,6 +857,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
     if (grp == 4) ok = group_wait(0) && ok;             //   the walk ended early the last group's
     if (__syncthreads_or(!ok)) { cx.dead = true; umma::report_timeout(err); }
     umma::tc_fence_after();
+    const bool any_strong = grp < 4;
     if (a.res.T) {                                      // the backward takes the same route
       float* ex = tile_extra(a.res, ibase);
       if (tid == 0) *reinterpret_cast<int*>(ex) = any_strong;
