@@ -233,9 +233,29 @@ def test_host_paths_agree(dn, dtype):
         o, s = dn.chunk_gdn2(*leaves, segment_ids=ids, **kw)
         res.append((o, s) + torch.autograd.grad(o.float().sum() + s.sum(), leaves))
     assert [torch.equal(x, y) for x, y in zip(*res)] == [True] * 8
-    st = torch.zeros(B, H, K, K, device="cuda")
-    tok, wide = [t[:, 0].contiguous() for t in ins], [t[:, 0] for t in strided]
-    for state_dtype in (torch.float32, torch.bfloat16):
-        one = dn.gdn2_decode_step(*tok, st.to(state_dtype), reset=torch.tensor([1], device="cuda", dtype=torch.int32))
-        two = dn.gdn2_decode_step(*wide, st.to(state_dtype), reset=torch.tensor([True], device="cuda"))
-        assert all(torch.equal(x, y) for x, y in zip(one, two))
+
+
+# ---- the same for a decode step: the native path answers the plain call and leaves the strided one to the general path
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("state_dtype", [torch.float32, torch.bfloat16])
+def test_decode_host_paths_agree(dn, state_dtype, per_head):
+    from deltanet_b200 import _lib as L
+    B, H, K = 3, 2, 64
+    ins = [t[:, 0].contiguous().cuda() for t in O.make_inputs(82, B, 1, H, H, K, K, qkv_dtype=torch.bfloat16)[:6]]
+    state = torch.randn(B, H, K, K, generator=torch.Generator().manual_seed(83)).to(state_dtype).cuda()
+    reset = torch.tensor([[False, True], [True, True], [False, False]] if per_head else [False, True, False], device="cuda")
+    wide = [torch.stack([t, t], -1)[..., 0] for t in ins]
+    native = lambda t, s, out: L.host().decode(*t, s, reset, None, L.DN_QK_L2NORM, state_dtype == torch.bfloat16, 1000.0, out)
+    kw = dict(reset=reset, qk_l2norm=True, state_dtype=state_dtype)
+    assert native(wide, state, None) is None
+    one, two, three = native(ins, state, None), dn.gdn2_decode_step(*ins, state, **kw), dn.gdn2_decode_step(*wide, state, **kw)
+    assert one is not None
+    assert all(torch.equal(x, y) and torch.equal(x, z) for x, y, z in zip(one, two, three))
+    kept = (one[1].float() == 0).all(dim=(2, 3))                      # no state is zeros: each is decayed, or has been reset and rewritten
+    assert not bool(kept.any()) and not torch.equal(one[1], state)
+    for t, into in ((ins, state.clone()), (wide, state.clone())):     # in place
+        o, s = dn.gdn2_decode_step(*t, into, out_state=into, **kw)
+        assert s is into and torch.equal(o, one[0]) and torch.equal(into, one[1])
+    ref = O.decode_step(*[t.cpu() for t in ins], state.cpu(), reset=None if per_head else reset.cpu(), qk_l2norm=True, state_dtype=state_dtype)
+    if not per_head:                                                  # one rounding of outputs (and bf16 states)
+        assert O.rel_l2(one[0].float().cpu(), ref[0].float()) < 2.0 ** -8 and O.rel_l2(one[1].float().cpu(), ref[1].float()) < 2.0 ** -8
