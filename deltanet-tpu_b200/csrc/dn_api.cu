@@ -12,10 +12,13 @@ using namespace dn;
 static inline size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
 // ---- overlap of the chunk-parallel kernels with the chains ------------------------------------
-// The chunk-parallel kernels run one CTA per SM over B*H*NC work items; when that count leaves the
-// last round of CTAs mostly empty (192 items on 148 SMs), dn_chunk_fwd / dn_chunk_bwd cut the chunk
-// axis in two and run the chain of one part on a side stream next to the chunk-parallel kernel of
-// the other part.  The side stream forks from and joins back into the caller's stream through
+// The backward's chunk-parallel kernels run one CTA per SM over B*H*NC work items; when that count leaves the
+// last round of CTAs mostly empty (192 items on 148 SMs), dn_chunk_bwd cuts the chunk
+// axis in two and runs the chain of one part on a side stream next to the chunk-parallel kernel of
+// the other part: 164 us instead of about 190 at the headline shape.  dn_chunk_fwd cuts at the same place, although the
+// forward prepass holds two CTAs per SM.  Above 296 items that pays (300 items of 256 columns 187 us in one piece, 160 cut;
+// 314 items of few heads 470 and 418; 512 items of scalar gates 110 and 125, a loss); below, where everything fits one round of
+// 296 CTAs, it does not (192 items of 256 columns 122 us in one piece and 127 cut, 256 items of scalar gates 63 and 80).  The side stream forks from and joins back into the caller's stream through
 // events, so the caller still sees one stream-ordered operation.  The stream and its events are
 // created on the first such call per device (host objects; do that call outside stream capture).
 // DN_NO_OVERLAP=1 turns the split off.

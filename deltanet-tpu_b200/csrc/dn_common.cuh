@@ -32,8 +32,8 @@ struct Geo {
   // Layout of the bf16 residual tiles W, U, M, qe, ke.  false: row-major (rows x cols).  true: the
   // operand image of the tensor-core kernels, [col / 8][row][8] -- a tile is then copied into shared
   // memory as it lies, and a thread that owns one row writes 16 bytes next to its neighbours'.
-  // Chosen once per shape (prepass on the tensor cores <=> image layout); every kernel reading or
-  // writing these tiles goes through rix().
+  // Chosen once per shape (prepass on the tensor cores <=> image layout).  The image kernels index pieces of 16 bytes as
+  // [(col / 8) * 128 + row] where they stand: another layout means editing each of them.
   bool img;
   __host__ __device__ bool bf16_mode() const { return prec == DN_PREC_BF16; }
   __host__ __device__ bool state_bf16() const { return prec == DN_PREC_BF16 && !(flags & DN_STATE_FP32_MM); }
@@ -116,19 +116,8 @@ __host__ __device__ __forceinline__ float* dlend_part(const Geo& g, float* dV) {
 __host__ __device__ __forceinline__ float* tile_extra(const dn_residuals& res, size_t tile) { return res.T + tile * 128 * 128 + 128 * 64; }
 __device__ __forceinline__ bool strong_flag(const dn_residuals& res, size_t tile) { return *reinterpret_cast<const int*>(tile_extra(res, tile)) != 0; }
 
-// element index of (row, col) in a residual tile of 128 rows (image layout) or `ncols` columns (row-major)
-__host__ __device__ __forceinline__ size_t rix(bool img, int row, int col, int ncols) {
-  return img ? ((size_t)((col >> 3) * 128 + row) << 3) + (col & 7) : (size_t)row * ncols + col;
-}
-
-// Optional phase clock (compile with -DDN_PHASE_TIMING): CTA 0 records clock64 at marked points of
-// its first item and prints the differences.  Compiled out otherwise.
-#ifdef DN_PHASE_TIMING
-static __device__ long long g_phase_marks[48];
-#define DN_MARK(i) do { if (blockIdx.x == 0 && threadIdx.x == 0) g_phase_marks[i] = clock64(); } while (0)
-#else
-#define DN_MARK(i) do { } while (0)
-#endif
+// element index of (row, col) in an image of 128 rows
+__device__ __forceinline__ size_t image_index(int row, int col) { return ((size_t)((col >> 3) * 128 + row) << 3) + (col & 7); }
 
 // --------------------------------------------------------------------------- dtype helpers
 // A bounded wait gave up: raise the library's error word (a plain store; the word may live in

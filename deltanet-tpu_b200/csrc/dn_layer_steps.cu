@@ -500,24 +500,6 @@ __global__ void __cluster_dims__(GB_CTAS, 1, 1) __launch_bounds__(256)
 // One warp per row of V (64 or 128) elements, EPL = V / 32 per lane.  The normalised value is rounded to
 // the input dtype before the weight is applied, as the layer this mirrors does.
 template <int EPL>
-__device__ __forceinline__ void ld_row(const void* base, size_t off, int dt, float (&x)[EPL]) {
-  if (dt == DN_BF16) {
-    const __nv_bfloat16* p = reinterpret_cast<const __nv_bfloat16*>(base) + off;
-    if (EPL == 4) {
-      const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
-      x[0] = __uint_as_float(u.x << 16); x[1] = __uint_as_float(u.x & 0xffff0000u);
-      x[2] = __uint_as_float(u.y << 16); x[3] = __uint_as_float(u.y & 0xffff0000u);
-    } else {
-      const uint32_t u = __ldg(reinterpret_cast<const uint32_t*>(p));
-      x[0] = __uint_as_float(u << 16); x[1] = __uint_as_float(u & 0xffff0000u);
-    }
-  } else {
-    const float* p = reinterpret_cast<const float*>(base) + off;
-    if (EPL == 4) { const float4 u = __ldg(reinterpret_cast<const float4*>(p)); x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; }
-    else { const float2 u = __ldg(reinterpret_cast<const float2*>(p)); x[0] = u.x; x[1] = u.y; }
-  }
-}
-template <int EPL>
 __device__ __forceinline__ void st_row(void* base, size_t off, int dt, const float (&x)[EPL]) {
   if (dt == DN_BF16) {
     __nv_bfloat16* p = reinterpret_cast<__nv_bfloat16*>(base) + off;

@@ -3,6 +3,9 @@
 // src/deltanet_tpu/gdn2.py:243-493, 750-762) and of the fused prologue (558-575).  The forward prepass marks the tiles whose
 // decay leaves e^{+-32} of a document's midpoint; all others are dn_prepass_bwd_fast.cu's.  Launched behind that kernel,
 // this one usually finds nothing marked and ends after one look.
+// Fine shapes (make_geo: 64-wide heads and the like) with decay per channel are all this kernel's: its diagonal blocks, DX, DM and
+// DA are fp32, and it takes dX, dY, DA, DM and the levels' factors in two bf16 parts.  B=4 L=2048, 16 heads of 64: 1.69 ms a
+// training step, 11.1 on the CUDA cores; 0.70 with everything in one part, four times further off in dg.
 //
 // Per (batch, exec head, chunk), 512 threads, one CTA per SM, in this order:
 //   G. nine matrix products (bwd_gemms_tc): V_new, dqe, dM, dW, dke, dX, dY, dA.  Every operand is a
@@ -539,8 +542,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_tc_kernel(PrepassBwdArgs a)
 
     // ---- E. combination.  Thread mapping of a tensor-memory drain: warp w owns rows 32 (w % 4) + lane
     //         and the 32 channels [32 (w / 4), +32), walked in four pieces of 8.  dbeta', dq', dk' come
-    //         straight from the accumulators of the two product rounds when the chunk took a single-Gram
-    //         route (tm_src != 0), else from the scratch panels.  dLambda and dke*ke go to shared memory,
+    //         from the scratch panels.  dLambda and dke*ke go to shared memory,
     //         d b is written.  The l2norm adjoint needs each row's <q_n, dq_n> and <k_n, dk_n>, whose
     //         four partial sums sit in four warps: they meet in shared memory; until then a thread
     //         parks its d q_n, d k_n, q_n, k_n in the tensor-memory columns it has just read (and in

@@ -7,7 +7,8 @@
 //     Gram products of the plain images, the decay applied per entry while they drain (prepass_fwd_scalar_kernel);
 //   * decay per channel that stays within e^{+-32} of each document's midpoint m over the tile: with
 //     f = e^{Lam - m},  A = (beta f) (k / f)^T,  M = (q f) (k / f)^T  (prepass_fwd_channel_kernel).
-// A tile with a stronger channel-wise decay takes the hierarchical factorisation (strong_route), decided per tile.
+// A tile with a stronger channel-wise decay takes the hierarchical factorisation (strong_route), decided per tile; so do all
+// tiles of fine shapes (make_geo), for its exact diagonal, with factors in two bf16 parts.
 //
 // What bounds an item is neither bytes nor tensor work but the length of its dependent phases (load, norms and
 // decay, products, inverse, products, store).  So a CTA takes 109 KB of shared memory and 256 columns of tensor
@@ -590,12 +591,12 @@ __device__ __noinline__ void strong_route(const PrepassFwdArgs& a, int b, int h,
       const int i = 32 * ps + ri, j = 32 * ps + rj;
       const bool same = seg_s[i] == seg_s[j];
       tri::blk(Tp, i >> 4, i >> 4)[di * tri::BP + dj] = same ? sa : 0.f;
-      M[rix(true, i, j, C)] = __float2bfloat16_rn(same ? sq : 0.f);
+      M[image_index(i, j)] = __float2bfloat16_rn(same ? sq : 0.f);
     }
   }
   accD += __shfl_xor_sync(0xffffffffu, accD, 1);
   accD += __shfl_xor_sync(0xffffffffu, accD, 2);
-  if (lgrp == 0) M[rix(true, x, x, C)] = __float2bfloat16_rn(accD);
+  if (lgrp == 0) M[image_index(x, x)] = __float2bfloat16_rn(accD);
   {
     const int quarter = warp & 3, u0 = 16 * (warp >> 2), at = (quarter & 1) * 32 + lane;      // lanes 0 .. 63: A's lower rows, 64 .. 127: M's
     const uint32_t tbase = cx.tmem + ((uint32_t)(quarter * 32) << 16);

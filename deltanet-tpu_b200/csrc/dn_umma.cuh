@@ -1,8 +1,7 @@
 // tcgen05 (5th-gen tensor core) building blocks for sm_100a, in inline PTX:
-// TMEM allocation, shared-memory matrix descriptors, single-thread MMA issue, commit to an
-// mbarrier with a BOUNDED wait, TMEM loads, and on top of them `umma_gemm`, a CTA-wide
-// bf16 x bf16 -> fp32 GEMM whose operands are gathered by the CTA's threads into shared memory
-// and whose 128 x N result is handed to an epilogue functor straight from tensor memory.
+// TMEM allocation, shared-memory matrix descriptors, MMA issue by an elected lane of a converged warp, commit to an
+// mbarrier with a BOUNDED wait, TMEM loads and stores, and on top of them the issue of a whole product on staged
+// operands and the drain of its 128 x N result to an epilogue functor straight from tensor memory.
 //
 // Shared-memory operand layout (no swizzle, the "interleaved" canonical layout): an operand
 // tile is a sequence of PANELS; a panel is `inner` rows of 16 bytes (8 bf16 elements):

@@ -159,7 +159,7 @@ int dn_cu_seqlens_segments(const int32_t* cu_seqlens, int32_t n_cu, const int32_
  * outputs then live in scratch only.
  *
  * Streams: all work is ordered on `stream`.  For shapes whose B*H*NC work items leave the last
- * round of the one-CTA-per-SM kernels mostly empty, dn_chunk_fwd and dn_chunk_bwd cut the chunk
+ * round of one CTA per SM mostly empty, dn_chunk_fwd and dn_chunk_bwd cut the chunk
  * axis in two and run part of the inter-chunk chain on a library-owned side stream next to the
  * chunk-parallel kernel of the other part; the side stream forks from `stream` and joins back into
  * it through events before the call's last kernel, so the caller still sees one stream-ordered
