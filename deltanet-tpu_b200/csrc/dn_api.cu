@@ -558,7 +558,7 @@ int dn_launch_count(const dn_shape* s, int backward, int recompute) {
   if (!backward) return split_f ? 4 : 2;
   int n = split_b ? 4 : 2;
   if (recompute) n += 2;
-  if (prepass_bwd_tc_eligible(g) && !prepass_bwd_scalar_route(g) && !g.fine) n += split_b ? 2 : 1;       // strong-decay tiles
+  if (prepass_bwd_tc_eligible(g) && !prepass_bwd_scalar_route(g)) n += split_b ? 2 : 1;       // strong-decay tiles
   n += (g.qk_div > 1 && prepass_bwd_group(g, g.NC) == 1 ? 2 : 0) + (g.gH != g.H) + (g.bH != g.H) + (g.wH != g.Hv);   // head sums
   return n;
 }

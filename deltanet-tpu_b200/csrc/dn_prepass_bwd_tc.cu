@@ -3,9 +3,7 @@
 // src/deltanet_tpu/gdn2.py:243-493, 750-762) and of the fused prologue (558-575).  The forward prepass marks the tiles whose
 // decay leaves e^{+-32} of a document's midpoint; all others are dn_prepass_bwd_fast.cu's.  Launched behind that kernel,
 // this one usually finds nothing marked and ends after one look.
-// Fine shapes (make_geo: 64-wide heads and the like) with decay per channel are all this kernel's: its diagonal blocks, DX, DM and
-// DA are fp32, and it takes dX, dY, DA, DM and the levels' factors in two bf16 parts.  B=4 L=2048, 16 heads of 64: 1.69 ms a
-// training step, 11.1 on the CUDA cores; 0.70 with everything in one part, four times further off in dg.
+// Fine shapes (make_geo: 64-wide heads and the like): dX, dY, dA, dM and the levels' factors in two bf16 parts, like the fast kernel's.
 //
 // Per (batch, exec head, chunk), 512 threads, one CTA per SM, in this order:
 //   G. nine matrix products (bwd_gemms_tc): V_new, dqe, dM, dW, dke, dX, dY, dA.  Every operand is a
@@ -757,10 +755,8 @@ int launch_prepass_bwd_tc(PrepassBwdArgs& a, size_t scratch_floats, cudaStream_t
   const bool scalar = prepass_bwd_scalar_route(g);
   const size_t ctas = scalar ? (a.group > 1 ? sm_count() : (g.fine ? grid : 0)) : grid;
   if (scratch_floats < ctas * a.scratch_per_cta) return DN_ERR_SCRATCH_TOO_SMALL;
-  if (scalar || !g.fine) {                               // (fine, decay per channel: every tile is this file's)
-    int rc = launch_prepass_bwd_fast(a, st);
-    if (rc || scalar) return rc;
-  }
+  int rc = launch_prepass_bwd_fast(a, st);
+  if (rc || scalar) return rc;
   const size_t lam_phase = (size_t)C * LP * 4 + 4 * 32768;
   size_t smem = bwd_tc_image_bytes(g.Vw);
   if (smem < lam_phase) smem = lam_phase;

@@ -7,8 +7,8 @@
 //     Gram products of the plain images, the decay applied per entry while they drain (prepass_fwd_scalar_kernel);
 //   * decay per channel that stays within e^{+-32} of each document's midpoint m over the tile: with
 //     f = e^{Lam - m},  A = (beta f) (k / f)^T,  M = (q f) (k / f)^T  (prepass_fwd_channel_kernel).
-// A tile with a stronger channel-wise decay takes the hierarchical factorisation (strong_route), decided per tile; so do all
-// tiles of fine shapes (make_geo), for its exact diagonal, with factors in two bf16 parts.
+// A tile with a stronger channel-wise decay takes the hierarchical factorisation (strong_route), decided per tile.  Fine shapes
+// (make_geo) have factors in two bf16 parts on both routes.
 //
 // What bounds an item is neither bytes nor tensor work but the length of its dependent phases (load, norms and
 // decay, products, inverse, products, store).  So a CTA takes 109 KB of shared memory and 256 columns of tensor
@@ -626,7 +626,9 @@ __device__ __noinline__ void strong_route(const PrepassFwdArgs& a, int b, int h,
   __syncthreads();
 }
 
-template <int VW, int MODE>
+// FINE (see make_geo): the three factors in two bf16 parts, in the two sets of images, so that a group's products (first x first,
+// second x first, first x second) are waited for by the next group.
+template <int VW, int MODE, bool FINE = false>
 __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid_constant__ PrepassFwdArgs a, int* err) {
   using CF = InCfg<MODE>;
   extern __shared__ __align__(128) uint8_t sm[];
@@ -746,9 +748,8 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
     EDGE[64 + lane] = 0.f;
     const bool first = seg_s[x] == seg_s[0], last = seg_s[x] == seg_s[C - 1];
     int grp = 0;
-    const bool fine = !CF::fixed && g.fine;              // the hierarchical route has an exact diagonal and factors in two parts
 #pragma unroll 1
-    for (; grp < 4 && !fine; ++grp) {
+    for (; grp < 4; ++grp) {
       act_g();
       if (cuts == 0) {
 #pragma unroll
@@ -770,9 +771,9 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       }
       const float lam_last = gv[7];
       bool ok = true, strong = false;
-      if (grp >= 2) ok = group_wait(grp & 1);           // the set this group writes was read by the products of group - 2
+      if (FINE ? grp >= 1 : grp >= 2) ok = group_wait(FINE ? 0 : grp & 1);        // the set this group writes was read by the products of group - 2
       if (__syncthreads_or(!ok)) { cx.dead = true; umma::report_timeout(err); }
-      uint4* KF = reinterpret_cast<uint4*>(sm + OFF_GI + (grp & 1) * 3 * 4 * PB);
+      uint4* KF = reinterpret_cast<uint4*>(sm + OFF_GI + (FINE ? 0 : grp & 1) * 3 * 4 * PB);
       uint4* QF = KF + 4 * PP;
       uint4* BF = QF + 4 * PP;
       // e^Lam = f e^{mid} and e^{Lam_end - Lam} = f^-1 e^{Lam_end - mid}, and they are only wanted in the first and the
@@ -826,6 +827,18 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       KF[lgrp * PP + x] = umma::pack8(o1);
       QF[lgrp * PP + x] = umma::pack8(o2);
       BF[lgrp * PP + x] = umma::pack8(o3);
+      if constexpr (FINE) {
+        float l[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) l[i] = low_part(o1[i]);
+        KF[12 * PP + lgrp * PP + x] = umma::pack8(l);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) l[i] = low_part(o2[i]);
+        QF[12 * PP + lgrp * PP + x] = umma::pack8(l);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) l[i] = low_part(o3[i]);
+        BF[12 * PP + lgrp * PP + x] = umma::pack8(l);
+      }
       umma::fence_async_smem();                         // umma::pre_issue_sync(), with a vote
       umma::tc_fence_before();
       const bool stop = __syncthreads_or(strong) != 0;
@@ -833,7 +846,13 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       if (stop) break;
       umma::issue_pitched<128, false, false>(cx, BF, PB, KF, PB, 32, 0, grp > 0);        // A += (beta f) (k / f)^T
       umma::issue_pitched<128, false, false>(cx, QF, PB, KF, PB, 32, 128, grp > 0);      // M += (q f) (k / f)^T
-      if (tid < 32 && !cx.dead) umma::mma_commit_warp(&gbar[grp & 1]);
+      if constexpr (FINE) {
+        umma::issue_pitched<128, false, false>(cx, BF + 12 * PP, PB, KF, PB, 32, 0, true);
+        umma::issue_pitched<128, false, false>(cx, BF, PB, KF + 12 * PP, PB, 32, 0, true);
+        umma::issue_pitched<128, false, false>(cx, QF + 12 * PP, PB, KF, PB, 32, 128, true);
+        umma::issue_pitched<128, false, false>(cx, QF, PB, KF + 12 * PP, PB, 32, 128, true);
+      }
+      if (tid < 32 && !cx.dead) umma::mma_commit_warp(&gbar[FINE ? 0 : grp & 1]);
       // global stores and the next group's loads come behind the proxy fence, which waits for what precedes it
       {
         uint4* QE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.qe) + ibase * C * K);
@@ -854,8 +873,13 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       }
       if (grp < 3) { load_g(grp + 1); load_kqb(grp + 1); }
     }
-    bool ok = grp == 0 || group_wait((grp - 1) & 1);     // the products nobody has waited for: the last two groups', or where
-    if (grp == 4) ok = group_wait(0) && ok;             //   the walk ended early the last group's
+    bool ok = true;                                     // the products nobody has waited for: the last two groups', or where the
+    if (FINE) {                                         //   walk ended early the last group's (FINE: the last group's, or none)
+      if (grp == 4) ok = group_wait(0);
+    } else {
+      if (grp > 0) ok = group_wait((grp - 1) & 1);
+      if (grp == 4) ok = group_wait(0) && ok;
+    }
     if (__syncthreads_or(!ok)) { cx.dead = true; umma::report_timeout(err); }
     umma::tc_fence_after();
     const bool any_strong = grp < 4;
@@ -914,7 +938,7 @@ int launch_prepass_fwd_tc(const Geo& g, const void* q, const void* k, const void
       case 0: go(prepass_fwd_channel_kernel<VW, 0>); break;
       case 1: go(prepass_fwd_channel_kernel<VW, 1>); break;
       case 4: go(prepass_fwd_channel_kernel<VW, 4>); break;
-      default: go(prepass_fwd_channel_kernel<VW, 2>); break;
+      default: if (g.fine) go(prepass_fwd_channel_kernel<VW, 2, true>); else go(prepass_fwd_channel_kernel<VW, 2>); break;
     }
   };
   if (g.Vw == 256) pick(std::integral_constant<int, 256>{});
