@@ -259,3 +259,27 @@ def test_decode_host_paths_agree(dn, state_dtype, per_head):
     ref = O.decode_step(*[t.cpu() for t in ins], state.cpu(), reset=None if per_head else reset.cpu(), qk_l2norm=True, state_dtype=state_dtype)
     if not per_head:                                                  # one rounding of outputs (and bf16 states)
         assert O.rel_l2(one[0].float().cpu(), ref[0].float()) < 2.0 ** -8 and O.rel_l2(one[1].float().cpu(), ref[1].float()) < 2.0 ** -8
+
+
+# ---- narrow heads sharded by sequence: the transition columns and the buffers between the phases on padded tiles
+@pytest.mark.parametrize("n,K,V,recompute", [(2, 64, 64, False), (4, 64, 128, True), (2, 128, 64, False)])
+def test_sharded_narrow_heads(n, K, V, recompute):
+    import test_gpu_sp
+    test_gpu_sp.test_sharded_equals_unsharded(n, "bf16", 128, K, V, BF16_TOL, recompute)
+
+
+# ---- narrow heads in the forms that only the run-time input mode knows: bf16 gates, mixed widths, the guard, the prologue
+@pytest.mark.parametrize("gates", ["bf16", "mixed", "guard", "fused", "fused_scalar"])
+@pytest.mark.parametrize("K,V,Hk,Hv", [(64, 64, 1, 2), (128, 64, 2, 2)])
+def test_narrow_heads_gate_forms(dn, gates, K, V, Hk, Hv):
+    ins = list(O.make_inputs(49, 1, 200, Hk, Hv, K, V, qkv_dtype=torch.bfloat16)[:6])
+    kw = dict(chunk_size=128, precision="bf16", qk_l2norm=True, output_final_state=True)
+    if gates == "bf16": ins[3:] = [t.bfloat16() for t in ins[3:]]
+    if gates == "mixed": ins[4], ins[5] = ins[4][..., :1].contiguous(), ins[5][..., 0].contiguous()
+    if gates == "guard": ins[4], kw["stability_guard"] = ins[4] - 0.4, True
+    if gates.startswith("fused"):
+        kw["fuse_prologue"] = True
+        ins[3], ins[4], ins[5] = ins[3], ins[4] - 0.5, ins[5] - 0.5
+    if gates == "fused_scalar": ins[3:] = [t[..., 0].contiguous() for t in ins[3:]]
+    seg = docs(1, 200, 70, 130)
+    compare(lambda t, i: dn.chunk_gdn2(*t, segment_ids=seg.cuda(), **kw), lambda t, i: O.chunk_gdn2(*t, segment_ids=seg, **kw), ins, tol=BF16_TOL)
