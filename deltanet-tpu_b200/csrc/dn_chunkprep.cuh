@@ -278,14 +278,14 @@ __device__ __forceinline__ Rows make_rows(const Geo& g, const void* q, const voi
   r.gate_dt = CF::fixed ? DN_F32 : g.gate_dt;
   const size_t tok0 = (size_t)bidx * g.L + t0;
   r.qk_pitch = (size_t)g.Hk * g.K;
-  r.qk_row0 = tok0 * r.qk_pitch + (size_t)(h / g.qk_div) * g.K;
+  r.qk_row0 = tok0 * r.qk_pitch + (size_t)g.qk_head(h) * g.K;
   r.kp = CF::fixed ? K / 8 : g.K / 8;
   r.gC = CF::fixed ? K : g.gC;
   r.bC = CF::fixed ? (CF::scalar_bw ? 1 : K) : g.bC;
   r.g_pitch = (size_t)g.gH * g.gC;
-  r.g_row0 = tok0 * r.g_pitch + (size_t)g.gate_head(h, g.gH) * g.gC;
+  r.g_row0 = tok0 * r.g_pitch + (size_t)g.g_head(h) * g.gC;
   r.b_pitch = (size_t)g.bH * g.bC;
-  r.b_row0 = tok0 * r.b_pitch + (size_t)g.gate_head(h, g.bH) * g.bC;
+  r.b_row0 = tok0 * r.b_pitch + (size_t)g.b_head(h) * g.bC;
   r.rows_valid = g.L - t0 < C ? g.L - t0 : C;
   r.l2 = g.flags & DN_QK_L2NORM;
   r.fuse = CF::fixed ? false : (g.flags & DN_FUSE_PROLOGUE) != 0;

@@ -17,6 +17,26 @@ bool force_simt();
 // streaming multiprocessors of the current device (queried once per device)
 int sm_count();
 
+// Division by a divisor that the launch knows: n * ceil(2^64 / d) >> 64, exact for every 32-bit n (the excess of the reciprocal
+// over 1 / d is below 2^-64, so the error of the product stays below 1 / d).  Two multiplications; the compiler's division by an
+// unknown divisor is a chain of about 20 instructions through the special-function unit, and the kernels decode a tile's place
+// (batch, head, chunk, the heads that its gates and its keys have) by half a dozen of these in a row, 600 to 1000 cycles a tile.
+struct FastDiv {
+  int d;
+  uint32_t hi, lo;                     // ceil(2^64 / d), 0 for d = 1
+  void set(int divisor) {
+    d = divisor;
+    const uint64_t m = d > 1 ? ~0ull / (uint64_t)d + 1 : 0;
+    hi = (uint32_t)(m >> 32);
+    lo = (uint32_t)m;
+  }
+  __host__ __device__ __forceinline__ int div(int n) const {
+    const uint64_t t = (uint64_t)(uint32_t)n * hi + (((uint64_t)(uint32_t)n * lo) >> 32);
+    return d == 1 ? n : (int)(t >> 32);
+  }
+  __host__ __device__ __forceinline__ void divmod(int n, int& q, int& r) const { q = div(n); r = n - q * d; }
+};
+
 // --------------------------------------------------------------------------- geometry
 // Everything a kernel needs to know about where a (batch, exec head, chunk) lives.
 struct Geo {
@@ -35,6 +55,18 @@ struct Geo {
   // Chosen once per shape (prepass on the tensor cores <=> image layout).  The image kernels index pieces of 16 bytes as
   // [(col / 8) * 128 + row] where they stand: another layout means editing each of them.
   bool img;
+  FastDiv by_BH, by_H, by_q, by_g, by_b, by_w;           // B H, H, qk_div; exec heads per head of g and b, value heads per head of w
+  // tile `e` of the chunks from c_begin on, in the order chunk, batch, head
+  __host__ __device__ __forceinline__ void tile(int e, int c_begin, int& b, int& h, int& c) const {
+    int bh;
+    by_BH.divmod(e, c, bh);
+    c += c_begin;
+    by_H.divmod(bh, b, h);
+  }
+  __host__ __device__ __forceinline__ int qk_head(int h) const { return by_q.div(h); }
+  __host__ __device__ __forceinline__ int g_head(int h) const { return by_g.div(h); }      // gate_head(h, gH)
+  __host__ __device__ __forceinline__ int b_head(int h) const { return by_b.div(h); }      // gate_head(h, bH)
+  __host__ __device__ __forceinline__ int w_of(int hv) const { return by_w.div(hv); }      // w_head(hv)
   __host__ __device__ bool bf16_mode() const { return prec == DN_PREC_BF16; }
   __host__ __device__ bool state_bf16() const { return prec == DN_PREC_BF16 && !(flags & DN_STATE_FP32_MM); }
   // head of a gate tensor that exec head h (and, for w, value head hv) reads
@@ -94,6 +126,8 @@ inline int make_geo(const dn_shape* s, Geo* g) {
   g->pre_dt = s->precision == DN_PREC_BF16 ? DN_BF16 : DN_F32;
   g->flags = s->flags; g->scale = s->scale;
   g->img = tc;
+  g->by_BH.set(g->B * g->H); g->by_H.set(g->H); g->by_q.set(g->qk_div);
+  g->by_g.set(g->H / g->gH); g->by_b.set(g->H / g->bH); g->by_w.set(g->Hv / g->wH);
   return DN_OK;
 }
 
@@ -137,6 +171,12 @@ __device__ __forceinline__ float ldf_ro(const void* p, size_t i, int dt) {
   return dt == DN_BF16 ? __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(p) + i))
                        : __ldg(reinterpret_cast<const float*>(p) + i);
 }
+// The same in two steps, bits and value, where the type is known at run time only and several loads are to be in flight together: the
+// conversion of a bf16 element waits for its load, whichever type the call turns out to have.
+__device__ __forceinline__ uint32_t ldbits_ro(const void* p, size_t i, int dt) {
+  return dt == DN_BF16 ? (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(p) + i) : __ldg(reinterpret_cast<const uint32_t*>(p) + i);
+}
+__device__ __forceinline__ float bits_value(uint32_t u, int dt) { return __uint_as_float(dt == DN_BF16 ? u << 16 : u); }
 __device__ __forceinline__ void stf(void* p, size_t i, float v, int dt) {
   if (dt == DN_BF16) reinterpret_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(v);
   else reinterpret_cast<float*>(p)[i] = v;

@@ -68,6 +68,8 @@ struct PrepassBwdArgs {
   int c_begin, c_end;              // chunk range [c_begin, c_end) of every (batch, head); tensor-core path only
   bool bulk_v;                     // v, w, dv, dw move by bulk copies (set by the launcher)
   int group;                       // heads one CTA takes in turn, summing their dq and dk (see prepass_bwd_group)
+  int units;                       // items / group, and B H / group, H / group (set by the launcher)
+  FastDiv by_BHG, by_HG;
 };
 
 // Called right after every kernel launch of the library: DN_OK or DN_ERR_CUDA_LAUNCH from

@@ -310,8 +310,8 @@ __device__ __noinline__ void v_phase(const PrepassBwdArgs& a, const uint4* img, 
   for (int it = 0; it < 4; ++it) {
     const int col = half * 128 + 32 * it + 8 * rp, cc = col < vr ? col : 0, hv = h * g.G + (cc >> vsh), cv = cc & (g.V - 1);
     vraw[it].load(a.v, (tok * g.Hv + hv) * g.V + cv);
-    if (SW) ws[it] = ldf_ro(a.w, tok * g.wH + g.w_head(hv), GBF ? DN_BF16 : DN_F32);
-    else wraw[it].load(a.w, (tok * g.wH + g.w_head(hv)) * g.V + cv);
+    if (SW) ws[it] = ldf_ro(a.w, tok * g.wH + g.w_of(hv), GBF ? DN_BF16 : DN_F32);
+    else wraw[it].load(a.w, (tok * g.wH + g.w_of(hv)) * g.V + cv);
   }
   float sw = 0.f;
 #pragma unroll
@@ -406,10 +406,18 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
 
   // A CTA takes the D heads that share a key head one after the other and adds up their dq and dk in its scratch (see
   // prepass_bwd_grouped); otherwise D = 1.
-  const int D = SC ? a.group : 1, HG = g.H / D;
+  const int D = SC ? a.group : 1, HG = a.by_HG.d, units = a.units;
+  auto place = [&](int e, int hd, int& b, int& h, int& c) {
+    int bg;
+    a.by_BHG.divmod(e, c, bg);
+    c += a.c_begin;
+    a.by_HG.divmod(bg, b, h);
+    h = h * D + hd;
+  };
   auto tile_of = [&](int e, int hd) {
-    const int bg = e % (g.B * HG), b = bg / HG, h = (bg - b * HG) * D + hd;
-    return (size_t)(b * g.H + h) * g.NC + a.c_begin + e / (g.B * HG);
+    int b, h, c;
+    place(e, hd, b, h, c);
+    return (size_t)(b * g.H + h) * g.NC + c;
   };
   const __nv_bfloat16* states = states_img(g, a.res.states);
   auto load_first = [&](size_t ib, int who) {           // what the first product and its drain take
@@ -418,9 +426,11 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     sl.load(2, reinterpret_cast<const __nv_bfloat16*>(a.res.U) + ib * C * VW, who);
   };
   bool loaded = false;                                  // load_first has been done during the tile before
-  for (int e_item = blockIdx.x, hd = 0; e_item < a.items / D; (hd = hd + 1 < D ? hd + 1 : 0) == 0 ? e_item += gridDim.x : 0) {
-    const int bg = e_item % (g.B * HG), c_idx = a.c_begin + e_item / (g.B * HG);
-    const int b = bg / HG, h = (bg - b * HG) * D + hd, t0 = c_idx * C;
+  for (int e_item = blockIdx.x, hd = 0; e_item < units; (hd = hd + 1 < D ? hd + 1 : 0) == 0 ? e_item += gridDim.x : 0) {
+    int b, h, c_idx;
+    place(e_item, hd, b, h, c_idx);
+    const int t0 = c_idx * C;
+    const int hk = D > 1 ? g.qk_head(h) : h;              // head of dq and dk
     const size_t ibase = (size_t)(b * g.H + h) * g.NC + c_idx;
     if (!SC && !loaded && strong_flag(a.res, ibase)) continue;              // uniform over the CTA
     if (!loaded) load_first(ibase, 0);
@@ -478,8 +488,9 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         const int sp = x ? seg_at(a.seg, b, t0 + x - 1, g.L) : sg;
         float gv = 0.f, bv = 0.f;
         if (x < rows) {
-          gv = ldf_ro(a.gg, (tok0 + x) * g.gH + g.gate_head(h, g.gH), g.gate_dt);
-          bv = ldf_ro(a.b, (tok0 + x) * g.bH + g.gate_head(h, g.bH), g.gate_dt);
+          const uint32_t gu = ldbits_ro(a.gg, (tok0 + x) * g.gH + g.g_head(h), g.gate_dt), bu = ldbits_ro(a.b, (tok0 + x) * g.bH + g.b_head(h), g.gate_dt);
+          gv = bits_value(gu, g.gate_dt);
+          bv = bits_value(bu, g.gate_dt);
           gv = gv <= 0.f ? gv : 0.f;
           if (guard) { bv = fmaxf(bv, 0.f); gv = fminf(gv, -1e-6f); }
         }
@@ -684,9 +695,9 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     // ---- key side: rows of q, k, b in the row mapping
     const bool live = rx < rows;
     const size_t tokx = tok0 + (live ? rx : 0);
-    const uint8_t* krow = reinterpret_cast<const uint8_t*>(a.k) + (tokx * g.Hk + h / g.qk_div) * g.K * qes;
-    const uint8_t* qrow = reinterpret_cast<const uint8_t*>(a.q) + (tokx * g.Hk + h / g.qk_div) * g.K * qes;
-    const uint8_t* brow = reinterpret_cast<const uint8_t*>(a.b) + (tokx * g.bH + g.gate_head(h, g.bH)) * bC * ges;
+    const uint8_t* krow = reinterpret_cast<const uint8_t*>(a.k) + (tokx * g.Hk + g.qk_head(h)) * g.K * qes;
+    const uint8_t* qrow = reinterpret_cast<const uint8_t*>(a.q) + (tokx * g.Hk + g.qk_head(h)) * g.K * qes;
+    const uint8_t* brow = reinterpret_cast<const uint8_t*>(a.b) + (tokx * g.bH + g.b_head(h)) * bC * ges;
     const float rq = rq_s[rx], rk = rk_s[rx];
     // the pieces of row rx as loaded, and activated: k_hat, q_hat, beta = b k_hat
     Raw8 rawk, rawq, rawb;
@@ -743,18 +754,13 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       const int c = tid & 127, qd = tid >> 7, x0 = qd * 32;
       const uint32_t gpitch = (uint32_t)(g.gH * gC) * ges;
       const bool cin = gC == 1 || c < gC;
-      const uint8_t* gp = reinterpret_cast<const uint8_t*>(a.gg) + (tok0 * g.gH + g.gate_head(h, g.gH)) * gC * ges + (gC == 1 || !cin ? 0 : c) * ges;
+      const uint8_t* gp = reinterpret_cast<const uint8_t*>(a.gg) + (tok0 * g.gH + g.g_head(h)) * gC * ges + (gC == 1 || !cin ? 0 : c) * ges;
       constexpr int GB = MODE == 2 ? 8 : 32;            // rows requested together (code size against latency)
-      float nx[GB];
+      uint32_t nx[GB];
       auto load_g = [&](int j) {                        // (rows past the end: row 0, dropped below)
         const int x = x0 + GB * j;
-        if (gdt == DN_BF16) {
 #pragma unroll
-          for (int i = 0; i < GB; ++i) nx[i] = ldf_ro(gp + (x + i < rows ? (size_t)(x + i) * gpitch : 0), 0, DN_BF16);
-        } else {
-#pragma unroll
-          for (int i = 0; i < GB; ++i) nx[i] = ldf_ro(gp + (x + i < rows ? (size_t)(x + i) * gpitch : 0), 0, DN_F32);
-        }
+        for (int i = 0; i < GB; ++i) nx[i] = ldbits_ro(gp + (x + i < rows ? (size_t)(x + i) * gpitch : 0), 0, gdt);
       };
       load_g(0);
       const uint32_t cuts = __ballot_sync(0xffffffffu, x0 + lane > 0 && seg_s[x0 + lane] != seg_s[x0 + lane - (x0 + lane > 0)]);
@@ -764,7 +770,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       for (int j = 0; j < 32 / GB; ++j) {
         float v[GB];
 #pragma unroll
-        for (int i = 0; i < GB; ++i) v[i] = nx[i];
+        for (int i = 0; i < GB; ++i) v[i] = bits_value(nx[i], gdt);
         if (j < 32 / GB - 1) load_g(j + 1);
 #pragma unroll
         for (int i = 0; i < GB; ++i) {
@@ -800,7 +806,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       const float el = SC ? (first ? umma::exp_neg(fminf(lam_s[row], 0.f)) : 0.f) : 0.f;
       const bool on = last && row < rows;
       const float eks = SC ? umma::exp_neg(fminf(lam_s[C - 1] - lam_s[row], 0.f)) : 0.f;
-      const uint8_t* kr = reinterpret_cast<const uint8_t*>(a.k) + ((tok0 + (row < rows ? row : 0)) * g.Hk + h / g.qk_div) * g.K * qes;
+      const uint8_t* kr = reinterpret_cast<const uint8_t*>(a.k) + ((tok0 + (row < rows ? row : 0)) * g.Hk + g.qk_head(h)) * g.K * qes;
       const float rkr = rk_s[row];
       Raw8 knext = ldraw(kr, group * 4 < kp ? group * 4 : 0, qdt);
       float pk = 0.f;
@@ -971,8 +977,8 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       const bool rlive = row < rows;
       const float dmii = dmi_s[row], rqr = rq_s[row], rkr = rk_s[row];
       const size_t tokr = tok0 + (rlive ? row : 0);
-      const uint8_t* kg = reinterpret_cast<const uint8_t*>(a.k) + (tokr * g.Hk + h / g.qk_div) * g.K * qes;
-      const uint8_t* qg = reinterpret_cast<const uint8_t*>(a.q) + (tokr * g.Hk + h / g.qk_div) * g.K * qes;
+      const uint8_t* kg = reinterpret_cast<const uint8_t*>(a.k) + (tokr * g.Hk + g.qk_head(h)) * g.K * qes;
+      const uint8_t* qg = reinterpret_cast<const uint8_t*>(a.q) + (tokr * g.Hk + g.qk_head(h)) * g.K * qes;
       auto raw_kq = [&](int p, float (&kr)[8], float (&qr)[8]) {
         if (staged) {
           umma::unpack8(RK[p * PP + row], kr);
@@ -1081,7 +1087,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       if (bC == 1 && group == 0 && rlive) {
         float s = (SUM[1024 + row] + SUM[1152 + row]) + (SUM[1280 + row] + SUM[1408 + row]);
         if (guard && !fuse) {                           // through max(b, 0)
-          const float braw = ldf_ro(a.b, (tok0 + row) * g.bH + g.gate_head(h, g.bH), gdt);
+          const float braw = ldf_ro(a.b, (tok0 + row) * g.bH + g.b_head(h), gdt);
           s *= braw > 0.f ? 1.f : (braw == 0.f ? 0.5f : 0.f);
         }
         stf(a.db, (tok0 + row) * g.H + h, s, a.db_dt);
@@ -1121,7 +1127,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
           RQ[p * PP + row] = umma::pack8(dqn);
           RK[p * PP + row] = umma::pack8(dkn);
         } else if (rlive && p < kp) {
-          const size_t o = ((tok0 + row) * HG + h / D) * g.K + 8 * p;
+          const size_t o = ((tok0 + row) * HG + hk) * g.K + 8 * p;
           strow8(a.dq, o, a.dq_dt, dqn);
           strow8(a.dk, o, a.dq_dt, dkn);
         }
@@ -1135,7 +1141,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       umma::tc_fence_before();
       __syncthreads();
       if (inplace && live && hd == D - 1) {
-        const size_t o = ((tok0 + rx) * HG + h / D) * g.K;
+        const size_t o = ((tok0 + rx) * HG + hk) * g.K;
 #pragma unroll
         for (int it = 0; it < 4; ++it) {
           const int p = it * 4 + rp;
@@ -1152,7 +1158,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       }
     }
     // ---- dg_t = sum_{i >= t, same doc} dLambda_i, and in the last document the Lambda_end path
-    const int segL = seg_s[C - 1], hg = g.gate_head(h, g.gH);
+    const int segL = seg_s[C - 1], hg = g.g_head(h);
     auto g_adjoint = [&](float d, float graw) {
       if (fuse) {
         const float gexp = -umma::ex2_fast(fminf(graw, 5.f) * DN_LOG2E);
@@ -1162,7 +1168,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     };
     // the next tile's first operands, where the raw rows were (asked for by a warp that has little left to do)
     const int ne = hd + 1 < D ? e_item : e_item + (int)gridDim.x;
-    loaded = ne < a.items / D && (SC || next_strong_s == 0);
+    loaded = ne < units && (SC || next_strong_s == 0);
     auto load_next = [&] { if (loaded) load_first(tile_of(ne, hd + 1 < D ? hd + 1 : 0), 480); };
     if constexpr (SC) {
       __syncthreads();
@@ -1216,12 +1222,12 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       const bool cin = gC == 1 || c < gC;
       const size_t o = ((tok0 + x0) * g.H + h) * gC + c, pitch = (size_t)g.H * gC;
       const size_t gi = ((tok0 + x0) * g.gH + hg) * gC + (cin && gC != 1 ? c : 0), gpit = (size_t)g.gH * gC;
-      float gr[8];
+      uint32_t gr[8];
       auto load_g = [&](int j) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int x = 8 * j + i;
-          gr[i] = x0 + x < rows ? ldf_ro(a.gg, gi + x * gpit, gdt) : 0.f;
+          gr[i] = x0 + x < rows ? ldbits_ro(a.gg, gi + x * gpit, gdt) : 0u;
         }
       };
       if (fuse && gC != 1) load_g(0);
@@ -1237,7 +1243,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         if (gC != 1) {
           if (fuse) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = g_adjoint(v[i], gr[i]);
+            for (int i = 0; i < 8; ++i) v[i] = g_adjoint(v[i], bits_value(gr[i], gdt));
             if (j < 3) load_g(j + 1);
           } else {
 #pragma unroll
@@ -1295,9 +1301,12 @@ bool prepass_bwd_scalar_route(const Geo& g) {
   return g.gC == 1 && g.bC == 1 && g.qkv_dt == DN_BF16 && !(g.flags & DN_FUSE_PROLOGUE);
 }
 
-int launch_prepass_bwd_fast(const PrepassBwdArgs& a, cudaStream_t st) {
+int launch_prepass_bwd_fast(const PrepassBwdArgs& args, cudaStream_t st) {
+  PrepassBwdArgs a = args;
   const Geo& g = a.g;
-  const int units = a.items / (prepass_bwd_scalar_route(g) ? a.group : 1);
+  const int D = prepass_bwd_scalar_route(g) ? a.group : 1, units = a.units = a.items / D;
+  a.by_HG.set(g.H / D);
+  a.by_BHG.set(g.B * (g.H / D));
   const int grid = units < sm_count() ? units : sm_count();
   auto go = [&](auto kernel) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);

@@ -48,14 +48,22 @@ static_assert(SMEM_BYTES <= 113 * 1024 - 2560, "two CTAs per SM, with the static
 // eight rows cost 32 lookups per load instead of 8, and the data stage of L1 was the busiest unit of these kernels.
 __device__ __forceinline__ int row_of(int tid) { return tid >> 2; }
 __device__ __forceinline__ int piece_of(int tid) { return tid & 3; }
+// Where a row's 16 pieces are wanted at once, eight lanes take 128 bytes of a row: half the lookups again.  A thread then has the
+// pieces (tid & 7) and (tid & 7) + 8 of the rows tid >> 3 and (tid >> 3) + 64, piece `it` of four; panels of such images are
+// 129 pieces apart.
+constexpr int PQ = 129;
+constexpr uint32_t PQB = PQ * 16;
+__device__ __forceinline__ int row8_of(int tid, int it) { return (tid >> 3) + 64 * (it >> 1); }
+__device__ __forceinline__ int piece8_of(int tid, int it) { return (tid & 7) + 8 * (it & 1); }
 
 // 1 / (1 + e^-x) on the special-function unit (relative error a few 2^-23; the products it enters are rounded to bf16)
 __device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 1.f + umma::ex2_fast(-x * DN_LOG2E)); }
 
-// After the products: the 16-column pieces of A (already masked and scaled by `fix`) into the triangle, of M into
-// its image.  fix(row, col, a[16], m[16]) applies masks and decay.
+// After the products: the 16-column pieces of A into the triangle, of M into its image.  fix(col, a[16], m[16]) applies the
+// decay; the masks -- a column counts from the first row `ds` of the row's document up to the row, for A exclusively --
+// are skipped by warps that have nothing to mask in a piece.
 template <class FIX>
-__device__ __forceinline__ void drain_am(const umma::Ctx& cx, float* Tp, uint4* Mimg, FIX fix) {
+__device__ __forceinline__ void drain_am(const umma::Ctx& cx, float* Tp, uint4* Mimg, int ds, FIX fix) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int quarter = warp & 3, group = warp >> 2, row = quarter * 32 + lane;
   const uint32_t tbase = cx.tmem + ((uint32_t)(quarter * 32) << 16);
@@ -66,7 +74,15 @@ __device__ __forceinline__ void drain_am(const umma::Ctx& cx, float* Tp, uint4* 
     if (!cx.dead && col <= quarter * 32 + 31) {        // warp-uniform: a piece wholly above the warp's rows is zeros
       umma::tmem_ld16(tbase + col, va);
       umma::tmem_ld16(tbase + 128 + col, vm);
-      fix(row, col, va, vm);
+      fix(col, va, vm);
+      if (col + 15 >= quarter * 32 || !__all_sync(0xffffffffu, ds <= col)) {
+        const int from = ds - col, to = row - col;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          va[i] = (i >= from && i < to) ? va[i] : 0.f;
+          vm[i] = (i >= from && i <= to) ? vm[i] : 0.f;
+        }
+      }
     } else {
 #pragma unroll
       for (int i = 0; i < 16; ++i) va[i] = vm[i] = 0.f;
@@ -82,95 +98,94 @@ __device__ __forceinline__ void drain_am(const umma::Ctx& cx, float* Tp, uint4* 
   umma::tc_fence_before();
 }
 
-// L2 requests made by threads 128 .. 511 while the first four warps are in the substitution: this tile's rows of v
-// and w, read right after the inverse, and the next tile's rows of k, q and g / b.  (One line per lane: the bulk form of
-// this request is issued lane by lane, about 80 cycles each, and took longer than what it hid.)
+// L2 requests made by warps that wait for the substitution: this tile's rows of v and w, read right after the inverse, by warps
+// 4 to 7 (which join the inverse sooner), and the next tile's rows of k and q by warps 12 to 15.  (One line per lane: the bulk form
+// of this request is issued lane by lane, about 80 cycles each, and took longer than what it hid.)
 __device__ __forceinline__ void prefetch_row(const void* p, uint32_t bytes) {
   for (uint32_t o = 0; o < bytes; o += 128)
     asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t*>(p) + o));
 }
-__device__ __forceinline__ void prefetch_rows(const PrepassFwdArgs& a, int h, int b, int t0, int next, int wC) {
+__device__ __forceinline__ void prefetch_vw(const PrepassFwdArgs& a, int h, int b, int t0) {
   const Geo& g = a.g;
-  const int x = threadIdx.x & 127, part = threadIdx.x >> 7, vr = g.G * g.V;
+  const int x = threadIdx.x & 127, vr = g.G * g.V;
+  if (t0 + x >= g.L) return;
   const uint32_t qe = (uint32_t)dt_size(g.qkv_dt), ge = (uint32_t)dt_size(g.gate_dt);
-  if (part < 3) {
-    if (t0 + x < g.L) {
-      const size_t tok = (size_t)b * g.L + t0 + x;
-      if (part == 1) prefetch_row(reinterpret_cast<const uint8_t*>(a.v) + (tok * g.Hv * g.V + (size_t)h * vr) * qe, vr * qe);
-      else if (wC == g.V && g.wH == g.Hv)
-        prefetch_row(reinterpret_cast<const uint8_t*>(a.w) + (tok * g.Hv * g.V + (size_t)h * vr) * ge, vr * ge);
-    }
-  } else if (next < a.items) {
-    const int bh = next % (g.B * g.H), t = (a.c_begin + next / (g.B * g.H)) * C + x;
-    const int hn = bh % g.H;
-    if (t < g.L) {
-      const size_t tok = (size_t)(bh / g.H) * g.L + t, qk = (tok * g.Hk + hn / g.qk_div) * g.K;
-      prefetch_row(reinterpret_cast<const uint8_t*>(a.k) + qk * qe, g.K * qe);
-      prefetch_row(reinterpret_cast<const uint8_t*>(a.q) + qk * qe, g.K * qe);
-      if (g.gC > 1) prefetch_row(reinterpret_cast<const uint8_t*>(a.gg) + (tok * g.gH + g.gate_head(hn, g.gH)) * g.gC * ge, g.gC * ge);
-      if (g.bC > 1) prefetch_row(reinterpret_cast<const uint8_t*>(a.b) + (tok * g.bH + g.gate_head(hn, g.bH)) * g.bC * ge, g.bC * ge);
-    }
-  }
+  const size_t at = ((size_t)b * g.L + t0 + x) * g.Hv * g.V + (size_t)h * vr;
+  prefetch_row(reinterpret_cast<const uint8_t*>(a.v) + at * qe, vr * qe);
+  if (g.wC == g.V && g.wH == g.Hv) prefetch_row(reinterpret_cast<const uint8_t*>(a.w) + at * ge, vr * ge);
+}
+__device__ __forceinline__ void prefetch_kq(const PrepassFwdArgs& a, int e_item) {
+  const Geo& g = a.g;
+  if (e_item >= a.items) return;
+  int b, h, c;
+  g.tile(e_item, a.c_begin, b, h, c);
+  const int t = c * C + (threadIdx.x & 127);
+  if (t >= g.L) return;
+  const uint32_t qe = (uint32_t)dt_size(g.qkv_dt);
+  const size_t qk = (((size_t)b * g.L + t) * g.Hk + g.qk_head(h)) * g.K;
+  prefetch_row(reinterpret_cast<const uint8_t*>(a.k) + qk * qe, g.K * qe);
+  prefetch_row(reinterpret_cast<const uint8_t*>(a.q) + qk * qe, g.K * qe);
 }
 
 // T = (I + A)^-1, then W = T X and U = T (w v).  X image and A visible to all threads on entry.
-template <int VW, bool PREFETCH>
+// others(): run by warps that wait for the substitution (tri::invert); ahead(): run by all as soon as the products have read their
+// operands (the images of X and T are free then).
+template <int VW, class OTHERS, class AHEAD>
 __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm, const PrepassFwdArgs& a, int h, int b, int t0,
-                                                     size_t ibase, int next, int qdt, int gdt, int wC, bool fuse) {
-  constexpr int HW = VW < 128 ? VW : 128, NH = VW / HW, NP = HW / 32;
+                                                     size_t ibase, int qdt, int gdt, int wC, bool fuse, OTHERS others, AHEAD ahead) {
+  constexpr int NH = VW / 128;
   const Geo& g = a.g;
   const int tid = threadIdx.x;
-  const int x = row_of(tid), lgrp = piece_of(tid);
   float* Tp = reinterpret_cast<float*>(sm + OFF_T);
   uint4* XI = reinterpret_cast<uint4*>(sm + OFF_X);
   uint4* TI = reinterpret_cast<uint4*>(sm + OFF_TI);
   uint4* Y0 = reinterpret_cast<uint4*>(sm + OFF_T);
   uint4* Wimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.W) + ibase * C * K);
   uint4* Uimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.U) + ibase * C * VW);
-  const int vr = g.G * g.V;                             // value columns that exist
-  const bool live = t0 + x < g.L;
-  const size_t tokr = (size_t)b * g.L + (live ? t0 + x : t0);
-  const uint8_t* vrow = reinterpret_cast<const uint8_t*>(a.v) + (tokr * g.Hv * g.V + (size_t)h * vr) * dt_size(qdt);
-  uint4 vraw[NP];                                         // a half's pieces of v (bf16), requested ahead of use
+  const int vr = g.G * g.V, vsh = g.V == 128 ? 7 : 6;   // value columns that exist
+  uint4 vraw[4];                                          // a half's pieces of v (bf16) and scalar write gates, requested ahead of use
+  uint32_t w1[4];
+  auto row_at = [&](int it) { const int x = row8_of(tid, it); return (size_t)b * g.L + (t0 + x < g.L ? t0 + x : t0); };
   auto request_v = [&](int half) {
-    if (qdt == DN_BF16) {
 #pragma unroll
-      for (int it = 0; it < NP; ++it) vraw[it] = half * HW + 32 * it < vr ? __ldg(reinterpret_cast<const uint4*>(vrow) + half * (HW / 8) + it * 4 + lgrp) : make_uint4(0, 0, 0, 0);
+    for (int it = 0; it < 4; ++it) {
+      const int col0 = half * 128 + 8 * piece8_of(tid, it), cc = col0 < vr ? col0 : 0;
+      const size_t tok = row_at(it);
+      if (wC == 1) w1[it] = ldbits_ro(a.w, tok * g.wH + g.w_of(h * g.G + (cc >> vsh)), gdt);
+      if (qdt == DN_BF16)
+        vraw[it] = col0 < vr ? __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.v) + tok * g.Hv * g.V + (size_t)h * vr + col0)) : make_uint4(0, 0, 0, 0);
     }
   };
   auto build_y = [&](uint4* Y, int half) {              // Y = w v of the half's columns
 #pragma unroll
-    for (int it = 0; it < NP; ++it) {
-      const int p = it * 4 + lgrp;
-      const int col0 = half * HW + 8 * p, hv = (h * vr + col0) / g.V, cv = h * vr + col0 - hv * g.V;
-      if (col0 - 8 * lgrp >= vr) { Y[p * PP + x] = make_uint4(0, 0, 0, 0); continue; }
+    for (int it = 0; it < 4; ++it) {
+      const int x = row8_of(tid, it), p = piece8_of(tid, it);
+      const int col0 = half * 128 + 8 * p, cv = col0 & (g.V - 1);
+      if (col0 >= vr) { Y[p * PQ + x] = make_uint4(0, 0, 0, 0); continue; }
+      const size_t tok = row_at(it);
       float vv[8], ww[8];
       if (wC == 1) {
-        const float w1 = ldf_ro(a.w, tokr * g.wH + g.w_head(hv), gdt);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) ww[i] = w1;
+        for (int i = 0; i < 8; ++i) ww[i] = bits_value(w1[it], gdt);
       } else {
-        load8(a.w, (tokr * g.wH + g.w_head(hv)) * wC + cv, gdt, ww);
+        load8(a.w, (tok * g.wH + g.w_of(h * g.G + (col0 >> vsh))) * wC + cv, gdt, ww);
       }
       if (qdt == DN_BF16) umma::unpack8(vraw[it], vv);
-      else { const Raw8 r = ldraw(vrow, half * (HW / 8) + p, qdt); cvraw(r, qdt, vv); }
+      else load8(a.v, tok * g.Hv * g.V + (size_t)h * vr + col0, qdt, vv);
+      const bool live = t0 + x < g.L;
 #pragma unroll
       for (int i = 0; i < 8; ++i) vv[i] = live ? (fuse ? sigmoid_fast(ww[i]) : ww[i]) * vv[i] : 0.f;
-      Y[p * PP + x] = umma::pack8(vv);
+      Y[p * PQ + x] = umma::pack8(vv);
     }
   };
-  tri::invert(Tp, reinterpret_cast<float*>(TI), [&]() {
-    // (scalar gates: 779 -> 741 us at B=4 L=8192 Hv=32.  With decay per channel the requests cost more than they hide,
-    // 761 -> 819 us at L=20011: that kernel reads q, k, b, g in groups and has other tiles to switch to.)
-    if (PREFETCH) prefetch_rows(a, h, b, t0, next, wC);
-  });
+  tri::invert(Tp, reinterpret_cast<float*>(TI), others);
   request_v(0);
   tri::image(Tp, TI);
   __syncthreads();                                      // T has been read: its place takes Y
   build_y(Y0, 0);
   umma::pre_issue_sync();
   umma::issue_pitched<128, false, true>(cx, TI, 2048, XI, PB, C, 0, false);
-  umma::issue_pitched<HW, false, true>(cx, TI, 2048, Y0, PB, C, 128, false);
+  umma::issue_pitched<128, false, true>(cx, TI, 2048, Y0, PQB, C, 128, false);
   umma::commit(cx);
   if (NH == 2) request_v(1);
   if (a.res.T) {                                        // the image of T, for the backward
@@ -179,6 +194,7 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
     for (int it = 0; it < 4; ++it) Tg[it * NT + tid] = TI[it * NT + tid];
   }
   umma::commit_wait_cta(cx);
+  if (NH == 1) ahead();
   if (NH == 2) {                                        // X has been consumed
     build_y(XI, 1);
     umma::fence_async_smem();                           // (ahead of the stores below: it would wait for them)
@@ -190,16 +206,17 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
   if (NH == 2) {                                        // the second half goes where W was
     __syncthreads();
     umma::tc_fence_after();
-    umma::issue_pitched<HW, false, true>(cx, TI, 2048, XI, PB, C, 0, false);
+    umma::issue_pitched<128, false, true>(cx, TI, 2048, XI, PQB, C, 0, false);
     umma::commit(cx);
   }
-  umma::drain<NT, HW>(cx, 128, [&](int row, int col, const float (&v)[16]) {
+  umma::drain<NT, 128>(cx, 128, [&](int row, int col, const float (&v)[16]) {
     Uimg[(col / 8) * 128 + row] = umma::pack8p(v);
     Uimg[(col / 8 + 1) * 128 + row] = umma::pack8p(v + 8);
   });
   if (NH == 2) {
     umma::commit_wait_cta(cx);
-    umma::drain<NT, HW>(cx, 0, [&](int row, int col, const float (&v)[16]) {
+    ahead();
+    umma::drain<NT, 128>(cx, 0, [&](int row, int col, const float (&v)[16]) {
       Uimg[2048 + (col / 8) * 128 + row] = umma::pack8p(v);
       Uimg[2048 + (col / 8 + 1) * 128 + row] = umma::pack8p(v + 8);
     });
@@ -222,156 +239,191 @@ __device__ __forceinline__ void teardown(uint32_t base) {
 }
 
 // ------------------------------------------------------------------------------- scalar decay, scalar erase gate
-// One load of q and k serves norms, images, qe and ke: a thread keeps its four 8-channel pieces of both in
-// registers while the row sums meet by shuffles and four warps scan the decay.
+// The decay of a tile, by 128 threads (named barrier 1), a row per thread: cumulative over the rows, restarting at documents; the
+// erase gate; and the first row of each row's document.
+struct alignas(16) ScalarRows {
+  float lam[C], bet[C];
+  uint8_t ds[C];
+};
+__device__ __forceinline__ void scan_scalar(const PrepassFwdArgs& a, int e_item, int t, ScalarRows& out, float* tot_s, int* rst_s) {
+  const Geo& g = a.g;
+  int b, h, c;
+  g.tile(e_item, a.c_begin, b, h, c);
+  const int t0 = c * C;
+  const int lane = t & 31, w = t >> 5;
+  const size_t tok = (size_t)b * g.L + t0 + t;
+  const bool guard = g.flags & DN_STABILITY_GUARD;
+  const int sg = seg_at(a.seg, b, t0 + t, g.L), sp = t ? seg_at(a.seg, b, t0 + t - 1, g.L) : sg;
+  float gv = 0.f, bv = 0.f;
+  if (t0 + t < g.L) {
+    const uint32_t gu = ldbits_ro(a.gg, tok * g.gH + g.g_head(h), g.gate_dt), bu = ldbits_ro(a.b, tok * g.bH + g.b_head(h), g.gate_dt);
+    gv = bits_value(gu, g.gate_dt);
+    bv = bits_value(bu, g.gate_dt);
+    gv = gv <= 0.f ? gv : 0.f;
+    if (guard) { bv = fmaxf(bv, 0.f); gv = fminf(gv, -1e-6f); }
+  }
+  int start = sg != sp ? t : -1;                        // last document start up to this row, as far as has been seen
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float up = __shfl_up_sync(0xffffffffu, gv, o);
+    const int us = __shfl_up_sync(0xffffffffu, start, o);
+    if (lane >= o) { if (start < 0) gv += up; start = max(start, us); }
+  }
+  if (lane == 31) { tot_s[w] = gv; rst_s[w] = start; }
+  tri::bar_sync(1, 128);
+  float carry = 0.f;
+  int above = 0;
+  for (int w2 = w - 1; w2 >= 0; --w2) { carry += tot_s[w2]; if (rst_s[w2] >= 0) { above = rst_s[w2]; break; } }
+  out.lam[t] = gv + (start >= 0 ? 0.f : carry);
+  out.bet[t] = bv;
+  out.ds[t] = (uint8_t)(start >= 0 ? start : above);
+  tri::bar_sync(1, 128);                                // tot_s and rst_s may be written again
+}
+
+// q and k are read once, eight lanes a row; qe, ke and X come from the images of q_hat and k_hat, a row per lane, so that the
+// stores of a warp are 512 contiguous bytes.  What an item waits for is taken off its path: the next item's decay is scanned by warps
+// 8 to 11 beside the substitution (its loads come from HBM: 1 to 2 k cycles), its rows of k and q are asked into L2 there and into
+// shared memory beside the last drains.
 template <int VW>
 __global__ void __launch_bounds__(NT, 2) prepass_fwd_scalar_kernel(const __grid_constant__ PrepassFwdArgs a, int* err) {
   extern __shared__ __align__(128) uint8_t sm[];
   __shared__ uint64_t bar;
   __shared__ uint32_t tbase;
-  __shared__ int seg_s[C];
-  __shared__ float lam_s[C], bet_s[C], tot_s[4];
+  __shared__ ScalarRows rows_s[2];
+  __shared__ float tot_s[4];
   __shared__ int rst_s[4];
   const Geo& g = a.g;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int x = row_of(tid), lgrp = piece_of(tid);
+  const int tid = threadIdx.x, warp = tid >> 5, row = tid & 127, group = tid >> 7;
   uint4* KI = reinterpret_cast<uint4*>(sm + OFF_X);
   uint4* QI = reinterpret_cast<uint4*>(sm + OFF_TI);
   umma::Ctx cx = setup(&bar, &tbase, err);
-  const bool guard = g.flags & DN_STABILITY_GUARD, l2 = g.flags & DN_QK_L2NORM;
+  const bool l2 = g.flags & DN_QK_L2NORM;
+  auto load_kq = [&](int e_item) {                      // raw rows where their images are going to be; a thread reads back what it asked for
+    if (e_item >= a.items) return;
+    int b, h, c;
+    g.tile(e_item, a.c_begin, b, h, c);
+    const size_t row0 = (size_t)b * g.L * g.Hk + g.qk_head(h);
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int t = c * C + row8_of(tid, it), p = piece8_of(tid, it), o = p * PQ + row8_of(tid, it);
+      const bool on = t < g.L && 8 * p < g.K;
+      const size_t at = on ? (row0 + (size_t)t * g.Hk) * g.K + 8 * p : 0;
+      umma::cp_async16_or_zero(KI + o, reinterpret_cast<const __nv_bfloat16*>(a.k) + at, on);
+      umma::cp_async16_or_zero(QI + o, reinterpret_cast<const __nv_bfloat16*>(a.q) + at, on);
+    }
+    umma::cp_async_commit();
+  };
+  load_kq(blockIdx.x);
+  if (tid < C) scan_scalar(a, blockIdx.x, tid, rows_s[0], tot_s, rst_s);
 
-  for (int e_item = blockIdx.x; e_item < a.items; e_item += gridDim.x) {
-    const int bh = e_item % (g.B * g.H), c_idx = a.c_begin + e_item / (g.B * g.H);
-    const int h = bh % g.H, b = bh / g.H, t0 = c_idx * C;
-    const size_t ibase = (size_t)bh * g.NC + c_idx, tok0 = (size_t)b * g.L + t0;
-    const int rows = g.L - t0 < C ? g.L - t0 : C;
-    const bool live = x < rows;
-    uint4 kr[4], qr[4];
-    {
-      const uint4* kp = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.k) + ((tok0 + (live ? x : 0)) * g.Hk + h / g.qk_div) * g.K);
-      const uint4* qp = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.q) + ((tok0 + (live ? x : 0)) * g.Hk + h / g.qk_div) * g.K);
+  int set = 0;
+  for (int e_item = blockIdx.x; e_item < a.items; e_item += gridDim.x, set ^= 1) {
+    int b, h, c_idx;
+    g.tile(e_item, a.c_begin, b, h, c_idx);
+    const int t0 = c_idx * C;
+    const size_t ibase = ((size_t)b * g.H + h) * g.NC + c_idx;
+    const ScalarRows& R = rows_s[set];
+    umma::cp_async_wait<0>();
 #pragma unroll
-      for (int it = 0; it < 4; ++it) {
-        const int p = it * 4 + lgrp;
-        const bool on = live && 8 * p < g.K;
-        kr[it] = on ? __ldg(kp + p) : make_uint4(0, 0, 0, 0);
-        qr[it] = on ? __ldg(qp + p) : make_uint4(0, 0, 0, 0);
-      }
-    }
-    if (tid < C) {                                      // decay: a document-restarting scan over the rows, one row per thread
-      const int t = tid;
-      const int sg = seg_at(a.seg, b, t0 + t, g.L), sp = t ? seg_at(a.seg, b, t0 + t - 1, g.L) : sg;
-      float gv = 0.f, bv = 0.f;
-      if (t < rows) {
-        gv = ldf_ro(a.gg, (tok0 + t) * g.gH + g.gate_head(h, g.gH), g.gate_dt);
-        bv = ldf_ro(a.b, (tok0 + t) * g.bH + g.gate_head(h, g.bH), g.gate_dt);
-        gv = gv <= 0.f ? gv : 0.f;
-        if (guard) { bv = fmaxf(bv, 0.f); gv = fminf(gv, -1e-6f); }
-      }
-      bool cut = sg != sp;
+    for (int r = 0; r < 2; ++r) {                       // k_hat, q_hat of the thread's two rows; rounded to bf16 by the packing
+      uint4 kr[2], qr[2];
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const float up = __shfl_up_sync(0xffffffffu, gv, o);
-        const bool uc = __shfl_up_sync(0xffffffffu, (int)cut, o);
-        if (lane >= o) { if (!cut) gv += up; cut |= uc; }
+      for (int j = 0; j < 2; ++j) {
+        const int at = piece8_of(tid, 2 * r + j) * PQ + row8_of(tid, 2 * r + j);
+        kr[j] = KI[at];
+        qr[j] = QI[at];
       }
-      seg_s[t] = sg;
-      bet_s[t] = bv;
-      if (lane == 31) { tot_s[warp] = gv; rst_s[warp] = cut; }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      float carry = 0.f;
-      for (int w2 = warp - 1; w2 >= 0; --w2) { carry += tot_s[w2]; if (rst_s[w2]) break; }
-      lam_s[t] = gv + (cut ? 0.f : carry);
-    }
-    float rq = 1.f, rk = 1.f;
-    if (l2) {
-      float sq = 0.f, sk = 0.f;
+      float rq = 1.f, rk = 1.f;
+      if (l2) {
+        float sq = 0.f, sk = 0.f;
 #pragma unroll
-      for (int it = 0; it < 4; ++it) {
+        for (int j = 0; j < 2; ++j) {
+          float f[8];
+          umma::unpack8(qr[j], f);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) sq = fmaf(f[i], f[i], sq);
+          umma::unpack8(kr[j], f);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) sk = fmaf(f[i], f[i], sk);
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) { sq += __shfl_xor_sync(0xffffffffu, sq, o); sk += __shfl_xor_sync(0xffffffffu, sk, o); }
+        rq = rsqrtf(sq + 1e-6f);
+        rk = rsqrtf(sk + 1e-6f);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int at = piece8_of(tid, 2 * r + j) * PQ + row8_of(tid, 2 * r + j);
         float f[8];
-        umma::unpack8(qr[it], f);
+        umma::unpack8(kr[j], f);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) sq = fmaf(f[i], f[i], sq);
-        umma::unpack8(kr[it], f);
+        for (int i = 0; i < 8; ++i) f[i] *= rk;
+        KI[at] = umma::pack8(f);
+        umma::unpack8(qr[j], f);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) sk = fmaf(f[i], f[i], sk);
+        for (int i = 0; i < 8; ++i) f[i] = (f[i] * rq) * g.scale;
+        QI[at] = umma::pack8(f);
       }
-      sq += __shfl_xor_sync(0xffffffffu, sq, 1);  sk += __shfl_xor_sync(0xffffffffu, sk, 1);
-      sq += __shfl_xor_sync(0xffffffffu, sq, 2); sk += __shfl_xor_sync(0xffffffffu, sk, 2);
-      rq = rsqrtf(sq + 1e-6f);
-      rk = rsqrtf(sk + 1e-6f);
-    }
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {                    // k_hat, q_hat; rounded to bf16 by the packing
-      float f[8];
-      umma::unpack8(kr[it], f);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] *= rk;
-      kr[it] = umma::pack8(f);
-      umma::unpack8(qr[it], f);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] = (f[i] * rq) * g.scale;
-      qr[it] = umma::pack8(f);
-      const int p = it * 4 + lgrp;
-      KI[p * PP + x] = kr[it];
-      QI[p * PP + x] = qr[it];
+      if (a.res.T && (tid & 7) == 0) { float* ex = tile_extra(a.res, ibase); ex[128 + row8_of(tid, 2 * r)] = rq; ex[256 + row8_of(tid, 2 * r)] = rk; }
     }
     umma::pre_issue_sync();
-    umma::issue_pitched<128, false, false>(cx, KI, PB, KI, PB, K, 0, false);             // k_hat k_hat^T
-    umma::issue_pitched<128, false, false>(cx, QI, PB, KI, PB, K, 128, false);           // q_hat k_hat^T
+    umma::issue_pitched<128, false, false>(cx, KI, PQB, KI, PQB, K, 0, false);           // k_hat k_hat^T
+    umma::issue_pitched<128, false, false>(cx, QI, PQB, KI, PQB, K, 128, false);         // q_hat k_hat^T
     umma::commit(cx);
-    const float lam = lam_s[x], lend = lam_s[C - 1], el = umma::exp_neg(fminf(lam, 0.f)), eke = umma::exp_neg(fminf(lend - lam, 0.f));
-    const bool first = seg_s[x] == seg_s[0], last = seg_s[x] == seg_s[C - 1];
+    uint4 xr[4];                                        // X = [first document] beta e^lam k_hat
     {                                                   // qe, ke while the products run
+      const float lam = R.lam[row], lend = R.lam[C - 1], el = umma::exp_neg(fminf(lam, 0.f)), bx = R.bet[row];
+      const bool first = R.ds[row] == 0, last = R.ds[row] == R.ds[C - 1];
       uint4* QE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.qe) + ibase * C * K);
       uint4* KE = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.ke) + ibase * C * K);
-      const float fq = first ? el : 0.f, fk = last ? eke : 0.f;
+      const float fq = first ? el : 0.f, fk = last ? umma::exp_neg(fminf(lend - lam, 0.f)) : 0.f;
 #pragma unroll
       for (int it = 0; it < 4; ++it) {
-        const int p = it * 4 + lgrp;
-        float f[8];
-        umma::unpack8(qr[it], f);
+        const int p = it * 4 + group;
+        float f[8], o[8];
+        umma::unpack8(QI[p * PQ + row], f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] *= fq;
-        QE[p * 128 + x] = umma::pack8(f);
-        umma::unpack8(kr[it], f);
+        QE[p * 128 + row] = umma::pack8(f);
+        umma::unpack8(KI[p * PQ + row], f);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] *= fk;
-        KE[p * 128 + x] = umma::pack8(f);
+        for (int i = 0; i < 8; ++i) o[i] = f[i] * fk;
+        KE[p * 128 + row] = umma::pack8(o);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] = first ? (bx * f[i]) * el : 0.f;
+        xr[it] = umma::pack8(o);
       }
       if (tid < K) a.res.lam_end[ibase * K + tid] = lend;
-      if (a.res.T && lgrp == 0) { float* ex = tile_extra(a.res, ibase); ex[128 + x] = rq; ex[256 + x] = rk; }
     }
     umma::commit_wait_cta(cx);
-    {                                                   // X = [first document] beta e^lam k_hat, over the k_hat image
-      const float bx = bet_s[x];
 #pragma unroll
-      for (int it = 0; it < 4; ++it) {
-        float f[8];
-        umma::unpack8(kr[it], f);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] = first ? (bx * f[i]) * el : 0.f;
-        KI[(it * 4 + lgrp) * PP + x] = umma::pack8(f);
-      }
-    }
+    for (int it = 0; it < 4; ++it) KI[(it * 4 + group) * PP + row] = xr[it];             // over the k_hat image
     {
-      const int row = (warp & 3) * 32 + lane;
-      const float lrow = lam_s[row] * DN_LOG2E, brow = bet_s[row];
-      const int srow = seg_s[row];
+      const float lrow = R.lam[row] * DN_LOG2E, brow = R.bet[row];
       uint4* Mimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.M) + ibase * C * C);
-      drain_am(cx, reinterpret_cast<float*>(sm + OFF_T), Mimg, [&](int rw, int col, float (&va)[16], float (&vm)[16]) {
+      drain_am(cx, reinterpret_cast<float*>(sm + OFF_T), Mimg, R.ds[row], [&](int col, float (&va)[16], float (&vm)[16]) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int j = col + i;
-          const bool same = srow == seg_s[j];
-          const float f = umma::ex2_fast(fminf(lrow - lam_s[j] * DN_LOG2E, 0.f));
-          va[i] = (same && j < rw) ? brow * f * va[i] : 0.f;
-          vm[i] = (same && j <= rw) ? f * vm[i] : 0.f;
+        for (int i = 0; i < 16; i += 4) {
+          const float4 l4 = *reinterpret_cast<const float4*>(R.lam + col + i);
+          const float l[4] = {l4.x, l4.y, l4.z, l4.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float f = umma::ex2_fast(fminf(lrow - l[u] * DN_LOG2E, 0.f));
+            va[i + u] *= brow * f;
+            vm[i + u] *= f;
+          }
         }
       });
     }
     __syncthreads();
-    inverse_and_products<VW, true>(cx, sm, a, h, b, t0, ibase, e_item + gridDim.x, DN_BF16, g.gate_dt, g.wC, false);
+    const int next = e_item + gridDim.x;
+    inverse_and_products<VW>(cx, sm, a, h, b, t0, ibase, DN_BF16, g.gate_dt, g.wC, false, [&]() {
+      // (the requests: 779 -> 741 us at B=4 L=8192 Hv=32.  With decay per channel they cost more than they hide,
+      // 761 -> 819 us at L=20011: that kernel reads q, k, b, g in groups and has other tiles to switch to.)
+      if (warp < 8) prefetch_vw(a, h, b, t0);
+      else if (warp >= 12) prefetch_kq(a, next);
+      else if (next < a.items) scan_scalar(a, next, tid - 256, rows_s[set ^ 1], tot_s, rst_s);
+    }, [&]() { load_kq(next); });
   }
   teardown(tbase);
 }
@@ -664,34 +716,38 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
   constexpr float FAST_HALF_RANGE = 32.f;
 
   for (int e_item = blockIdx.x; e_item < a.items; e_item += gridDim.x) {
-    const int bh = e_item % (g.B * g.H), c_idx = a.c_begin + e_item / (g.B * g.H);
-    const int h = bh % g.H, b = bh / g.H, t0 = c_idx * C;
-    const size_t ibase = (size_t)bh * g.NC + c_idx;
+    int b, h, c_idx;
+    g.tile(e_item, a.c_begin, b, h, c_idx);
+    const int t0 = c_idx * C;
+    const size_t ibase = ((size_t)b * g.H + h) * g.NC + c_idx;
     const int rows = g.L - t0 < C ? g.L - t0 : C;
     const bool live = x < rows;                         // rows past the end read row 0 and are zeroed
     const size_t tok = (size_t)b * g.L + t0 + (live ? x : 0);
-    const uint8_t* krow = reinterpret_cast<const uint8_t*>(a.k) + (tok * g.Hk + h / g.qk_div) * g.K * qes;
-    const uint8_t* qrow = reinterpret_cast<const uint8_t*>(a.q) + (tok * g.Hk + h / g.qk_div) * g.K * qes;
-    const uint8_t* brow = reinterpret_cast<const uint8_t*>(a.b) + (tok * g.bH + g.gate_head(h, g.bH)) * bC * ges;
+    const uint8_t* krow = reinterpret_cast<const uint8_t*>(a.k) + (tok * g.Hk + g.qk_head(h)) * g.K * qes;
+    const uint8_t* qrow = reinterpret_cast<const uint8_t*>(a.q) + (tok * g.Hk + g.qk_head(h)) * g.K * qes;
+    const uint8_t* brow = reinterpret_cast<const uint8_t*>(a.b) + (tok * g.bH + g.b_head(h)) * bC * ges;
     // decay of a group of 32 channels: thread (channel = lane, rows 8 warp .. 8 warp + 7)
     const uint32_t gpitch = (uint32_t)(g.gH * gC) * ges;
     const uint8_t* grow = reinterpret_cast<const uint8_t*>(a.gg) +
-        (((size_t)b * g.L + t0 + (warp * 8 < rows ? warp * 8 : 0)) * g.gH + g.gate_head(h, g.gH)) * gC * ges + (gC == 1 ? 0 : lane) * ges;
+        (((size_t)b * g.L + t0 + (warp * 8 < rows ? warp * 8 : 0)) * g.gH + g.g_head(h)) * gC * ges + (gC == 1 ? 0 : lane) * ges;
     float gv[8];
+    uint32_t graw[8];
+    const uint32_t off_bits = gdt == DN_BF16 ? 0xff80u : 0xff800000u;      // -infinity
     auto load_g = [&](int grp) {
       const bool cin = gC == 1 || CF::fixed || 32 * grp < gC;
       const uint8_t* gp = grow + (gC == 1 ? 0 : 32 * grp * ges);
       if (rows == C && cin) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) gv[i] = ldf_ro(gp + i * gpitch, 0, gdt);
+        for (int i = 0; i < 8; ++i) graw[i] = ldbits_ro(gp + i * gpitch, 0, gdt);
       } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) gv[i] = cin && warp * 8 + i < rows ? ldf_ro(gp + i * gpitch, 0, gdt) : (fuse ? -INFINITY : 0.f);
+        for (int i = 0; i < 8; ++i) graw[i] = cin && warp * 8 + i < rows ? ldbits_ro(gp + i * gpitch, 0, gdt) : (fuse ? off_bits : 0u);
       }
     };
     auto act_g = [&]() {                                // the activated decay (rows past the end: 0)
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
+        gv[i] = bits_value(graw[i], gdt);
         if (fuse) { const bool off = gv[i] == -INFINITY; gv[i] = off ? 0.f : -umma::ex2_fast(fminf(gv[i], 5.f) * DN_LOG2E); if (guard && !off) gv[i] = fminf(gv[i], -1e-6f); }
         else { gv[i] = gv[i] <= 0.f ? gv[i] : 0.f; if (guard && warp * 8 + i < rows) gv[i] = fminf(gv[i], -1e-6f); }
       }
@@ -770,6 +826,9 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
         LAM[(warp * 8 + i) * LQ + lane] = gv[i] * DN_LOG2E;
       }
       const float lam_last = gv[7];
+      // (with one write and erase gate per head a group's loads are few enough to be waited for by the proxy fence below, and g, which is
+      // wanted first, is asked for ahead of it: 131072 tokens of 32 heads 10.08 -> 9.54 ms; with channel-wise gates 798 -> 812 us at L=20011)
+      if (CF::scalar_bw && grp < 3) load_g(grp + 1);
       bool ok = true, strong = false;
       if (FINE ? grp >= 1 : grp >= 2) ok = group_wait(FINE ? 0 : grp & 1);        // the set this group writes was read by the products of group - 2
       if (__syncthreads_or(!ok)) { cx.dead = true; umma::report_timeout(err); }
@@ -871,7 +930,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
         XI[p * PP + x] = umma::pack8(o3);
         if (warp == 15) a.res.lam_end[ibase * K + 32 * grp + lane] = lam_last;
       }
-      if (grp < 3) { load_g(grp + 1); load_kqb(grp + 1); }
+      if (grp < 3) { if (!CF::scalar_bw) load_g(grp + 1); load_kqb(grp + 1); }
     }
     bool ok = true;                                     // the products nobody has waited for: the last two groups', or where the
     if (FINE) {                                         //   walk ended early the last group's (FINE: the last group's, or none)
@@ -894,19 +953,11 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       cx.phase = c2.phase;
       cx.dead = c2.dead;
     } else {
-      const int srow = seg_s[(warp & 3) * 32 + lane];
       uint4* Mimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.M) + ibase * C * C);
-      drain_am(cx, reinterpret_cast<float*>(sm + OFF_T), Mimg, [&](int rw, int col, float (&va)[16], float (&vm)[16]) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const bool same = srow == seg_s[col + i];
-          va[i] = (same && col + i < rw) ? va[i] : 0.f;
-          vm[i] = (same && col + i <= rw) ? vm[i] : 0.f;
-        }
-      });
+      drain_am(cx, reinterpret_cast<float*>(sm + OFF_T), Mimg, ds_s[(warp & 3) * 32 + lane], [](int, float (&)[16], float (&)[16]) {});
       __syncthreads();
     }
-    inverse_and_products<VW, false>(cx, sm, a, h, b, t0, ibase, e_item + gridDim.x, qdt, gdt, wC, fuse);
+    inverse_and_products<VW>(cx, sm, a, h, b, t0, ibase, qdt, gdt, wC, fuse, [] {}, [] {});
   }
   teardown(tbase);
 }
