@@ -297,22 +297,31 @@ struct Piece {                                          // eight elements as loa
 // columns, dY from its image.  Bound by the latency of the rows of v and w (2.2 to 3.2 k cycles with every SM here at once), so
 // all of them are requested together; one function per type, because only code that runs takes instruction cache.
 // low (LOW): the second part of dY, an image in global memory.
+template <bool QBF, bool GBF, bool SW>
+struct VRows {
+  Piece<QBF> v[4];
+  Piece<GBF> w[SW ? 1 : 4];
+  uint32_t ws[SW ? 4 : 1];
+  __device__ __forceinline__ void request(const PrepassBwdArgs& a, int half, int h, size_t tok0, int rows) {
+    const Geo& g = a.g;
+    const int rx = threadIdx.x >> 2, rp = threadIdx.x & 3, vr = g.G * g.V, vsh = g.V == 128 ? 7 : 6;
+    const size_t tok = tok0 + (rx < rows ? rx : 0);
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int col = half * 128 + 32 * it + 8 * rp, cc = col < vr ? col : 0, hv = h * g.G + (cc >> vsh), cv = cc & (g.V - 1);
+      v[it].load(a.v, (tok * g.Hv + hv) * g.V + cv);
+      if (SW) ws[SW ? it : 0] = ldbits_ro(a.w, tok * g.wH + g.w_of(hv), GBF ? DN_BF16 : DN_F32);
+      else w[SW ? 0 : it].load(a.w, (tok * g.wH + g.w_of(hv)) * g.V + cv);
+    }
+  }
+};
 template <bool QBF, bool GBF, bool SW, bool LOW>
-__device__ __noinline__ void v_phase(const PrepassBwdArgs& a, const uint4* img, int half, int h, size_t tok0, int rows, bool fuse, const float4* low) {
+__device__ __forceinline__ void v_body(const VRows<QBF, GBF, SW>& in, const PrepassBwdArgs& a, const uint4* img, int half, int h, size_t tok0, int rows, bool fuse,
+                                       const float4* low) {
   const Geo& g = a.g;
   const int rx = threadIdx.x >> 2, rp = threadIdx.x & 3, vr = g.G * g.V, vsh = g.V == 128 ? 7 : 6;
   const bool live = rx < rows;
   const size_t tok = tok0 + (live ? rx : 0);
-  Piece<QBF> vraw[4];
-  Piece<GBF> wraw[4];
-  float ws[4];
-#pragma unroll
-  for (int it = 0; it < 4; ++it) {
-    const int col = half * 128 + 32 * it + 8 * rp, cc = col < vr ? col : 0, hv = h * g.G + (cc >> vsh), cv = cc & (g.V - 1);
-    vraw[it].load(a.v, (tok * g.Hv + hv) * g.V + cv);
-    if (SW) ws[it] = ldf_ro(a.w, tok * g.wH + g.w_of(hv), GBF ? DN_BF16 : DN_F32);
-    else wraw[it].load(a.w, (tok * g.wH + g.w_of(hv)) * g.V + cv);
-  }
   float sw = 0.f;
 #pragma unroll
   for (int it = 0; it < 4; ++it) {
@@ -320,11 +329,11 @@ __device__ __noinline__ void v_phase(const PrepassBwdArgs& a, const uint4* img, 
     if (col - 8 * rp >= vr) break;                      // (uniform: value widths are multiples of 32)
     const int hv = h * g.G + (col >> vsh), cv = col & (g.V - 1);
     float vv[8], ww[8], dy[8], dv8[8], dw8[8];
-    vraw[it].get(vv);
+    in.v[it].get(vv);
     if (SW) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) ww[i] = ws[it];
-    } else wraw[it].get(ww);
+      for (int i = 0; i < 8; ++i) ww[i] = bits_value(in.ws[SW ? it : 0], GBF ? DN_BF16 : DN_F32);
+    } else in.w[SW ? 0 : it].get(ww);
     umma::unpack8(img[p * PP + rx], dy);
     if (LOW) {
       float lo[8];
@@ -351,6 +360,12 @@ __device__ __noinline__ void v_phase(const PrepassBwdArgs& a, const uint4* img, 
       sw = 0.f;
     }
   }
+}
+template <bool QBF, bool GBF, bool SW, bool LOW>
+__device__ __noinline__ void v_phase(const PrepassBwdArgs& a, const uint4* img, int half, int h, size_t tok0, int rows, bool fuse, const float4* low) {
+  VRows<QBF, GBF, SW> in;
+  in.request(a, half, h, tok0, rows);
+  v_body<QBF, GBF, SW, LOW>(in, a, img, half, h, tok0, rows, fuse, low);
 }
 
 // FINE (see make_geo): dA, dM, dX and dY take part in two bf16 parts, and so do the factors where the decay is per channel (the
@@ -425,7 +440,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     sl.load(1, states + ib * K * VW, who);
     sl.load(2, reinterpret_cast<const __nv_bfloat16*>(a.res.U) + ib * C * VW, who);
   };
-  bool loaded = false;                                  // load_first has been done during the tile before
+  bool loaded = false, staged_dO = false;               // load_first, stage_dO have been done during the tile before
   for (int e_item = blockIdx.x, hd = 0; e_item < units; (hd = hd + 1 < D ? hd + 1 : 0) == 0 ? e_item += gridDim.x : 0) {
     int b, h, c_idx;
     place(e_item, hd, b, h, c_idx);
@@ -444,16 +459,21 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     const __nv_bfloat16* Tg = reinterpret_cast<const __nv_bfloat16*>(a.res.T + ibase * C * C);
     const size_t dO_off = tok0 * g.Hv * g.V + (size_t)h * vr, dO_pitch = (size_t)g.Hv * g.V;
     constexpr int HN = C * 128;                         // elements of one half's image
+    // One half, bf16 v and one fp32 write gate per head: the rows are few enough to wait in registers, and are asked for two products
+    // and two drains ahead of their use.
+    constexpr bool V_AHEAD = NH == 1 && (SC || CF::scalar_bw);
+    const bool v_ahead = V_AHEAD && qdt == DN_BF16 && gdt == DN_F32 && wC == 1;
+    VRows<true, false, true> vrows;
 
     // ---- products over the value width
     if (NH == 1) {
       sl.load(3, dVg);
       sl.load(4, dHg);
-      stage_dO(sl.at(5), a.d_out, dO_off, dO_pitch, rows, vr / 8, qdt);
+      if (!staged_dO) stage_dO(sl.at(5), a.d_out, dO_off, dO_pitch, rows, vr / 8, qdt);
     } else {
       sl.load(3, Sg + HN);
       sl.load(4, Ug + HN);
-      stage_dO(sl.at(5), a.d_out, dO_off, dO_pitch, rows, 16, qdt);
+      if (!staged_dO) stage_dO(sl.at(5), a.d_out, dO_off, dO_pitch, rows, 16, qdt);
     }
     // V_new = U - W S, in the place of U; dM masked (scalar gates: decayed), its diagonal apart
     auto vnew = [&](int slot, uint32_t col) { drain_sub(cx.dead, tb + col, sl.at(slot), row, group); };
@@ -540,6 +560,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       product<128, true, true>(cx, sl.at(0), 2048, sl.at(1), 2048, C, T_B, false);                         // dX = T^T dW
       product<128, true, true>(cx, sl.at(0), 2048, sl.at(3), 2048, C, T_TMP, false);                       // dY = T^T dV
       commit(cx);
+      if (v_ahead) vrows.request(a, 0, h, tok0, rows);
       finish(cx);
     } else {
       sl.load(0, dVg);
@@ -633,7 +654,8 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       product<128, false, false>(cx, sl.at(1), PB, sl.at(4), 2048, 128, T_TMP, true);
       if constexpr (FINE) product<128, false, false>(cx, sl.at(3), 2048, sl.at(4), 2048, 128, T_TMP, true);
       commit(cx);
-      vphase(1, 0);
+      if (v_ahead) v_body<true, false, true, FINE>(vrows, a, sl.at(1), 0, h, tok0, rows, fuse, low_Y);
+      else vphase(1, 0);
       finish(cx);
       if constexpr (FINE) {
         low_dX(0);
@@ -690,7 +712,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     }
     // ---- dA (dM is in slot 5); everything else is free
     uint4 *const dAi = sl.region(4), *const dMi = sl.at(5), *const dAb = SC ? sl.region(2) : nullptr;
-    drain_masked(cx.dead, tb + T_TMP, dAi, row, group, -1.f, seg_s, SC ? lam_s : nullptr, nullptr, dAb, SC ? bet_s[row] : 0.f);
+    if constexpr (!SC) drain_masked(cx.dead, tb + T_TMP, dAi, row, group, -1.f, seg_s, nullptr, nullptr);
 
     // ---- key side: rows of q, k, b in the row mapping
     const bool live = rx < rows;
@@ -799,6 +821,28 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         EDGE[128 + tid] = umma::ex2_fast(0.5f * (LAM[(C - 1) * LPF + tid] - LAM[ds_s[C - 1] * LPF + tid]));
       }
     }
+    // Scalar gates: the thread's pieces of k and q stay in registers until the combination wants the raw rows (reading them
+    // three times, once a row per lane, took 3 k cycles of a tile's 63)
+    uint4 kraw4[SC ? 4 : 1], qraw4[SC ? 4 : 1];
+    if constexpr (SC) {
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int p = it * 4 + rp, pc = p < kp ? p : 0;
+        kraw4[it] = ld16_now(krow + 16 * pc);
+        qraw4[it] = ld16_now(qrow + 16 * pc);
+      }
+      drain_masked(cx.dead, tb + T_TMP, dAi, row, group, -1.f, seg_s, lam_s, nullptr, dAb, bet_s[row]);
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int p = it * 4 + rp;
+        float kh[8], qh[8], be[8];
+        rawk.a = kraw4[it];
+        rawq.a = qraw4[it];
+        pieces(p, kh, qh, be);
+        sl.region(0)[p * PP + rx] = umma::pack8(kh);
+        sl.region(1)[p * PP + rx] = umma::pack8(qh);
+      }
+    }
     __syncthreads();
     // ---- dqe, dX, dke scaled where they lie; the column sums of ke dke
     {
@@ -808,25 +852,29 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       const float eks = SC ? umma::exp_neg(fminf(lam_s[C - 1] - lam_s[row], 0.f)) : 0.f;
       const uint8_t* kr = reinterpret_cast<const uint8_t*>(a.k) + ((tok0 + (row < rows ? row : 0)) * g.Hk + g.qk_head(h)) * g.K * qes;
       const float rkr = rk_s[row];
-      Raw8 knext = ldraw(kr, group * 4 < kp ? group * 4 : 0, qdt);
+      Raw8 knext;
+      if (!SC) knext = ldraw(kr, group * 4 < kp ? group * 4 : 0, qdt);
       float pk = 0.f;
 #pragma unroll 1
       for (int j = 0; j < 4; ++j) {
         const int p = group * 4 + j, c0 = group * 32 + 8 * j;
         float v[8], w[8], x[8], kh[8], od[8];
         const Raw8 kraw = knext;
-        if (j < 3) knext = ldraw(kr, p + 1 < kp ? p + 1 : 0, qdt);
+        if (!SC && j < 3) knext = ldraw(kr, p + 1 < kp ? p + 1 : 0, qdt);
         ld8(cx.dead, tb + T_Q + 8 * j, v);
         ld8(cx.dead, tb + T_B + 8 * j, w);
         ld8(cx.dead, tb + T_K + 8 * j, x);
-        cvraw(kraw, qdt, kh);
+        if constexpr (SC) umma::unpack8(sl.region(0)[p * PP + row], kh);
+        else cvraw(kraw, qdt, kh);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const float e1 = SC ? el : (first ? EDGE[c0 + i] : 0.f);
           v[i] *= e1;
           w[i] *= e1;
-          kh[i] *= rkr;
-          if (round_in) kh[i] = bf16r(kh[i]);
+          if (!SC) {
+            kh[i] *= rkr;
+            if (round_in) kh[i] = bf16r(kh[i]);
+          }
           const float e = SC ? eks : umma::ex2_fast(fminf(LAM[(C - 1) * LPF + c0 + i] - LAM[row * LPF + c0 + i], 0.f));
           od[i] = on && p < kp ? x[i] * (kh[i] * e) : 0.f;
           x[i] *= SC ? (last ? eks : 0.f) : (last ? EDGE[128 + c0 + i] : 0.f);
@@ -856,15 +904,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     // ---- T1, T2, T3 on top of them
     if constexpr (SC) {
       uint4 *KI = sl.region(0), *QI = sl.region(1);
-#pragma unroll 2
-      for (int it = 0; it < 4; ++it) {
-        const int p = it * 4 + rp;
-        float kh[8], qh[8], be[8];
-        load_pieces(p);
-        pieces(p, kh, qh, be);
-        KI[p * PP + rx] = umma::pack8(kh);
-        QI[p * PP + rx] = umma::pack8(qh);
-      }
       umma::pre_issue_sync();
       product<128, false, true>(cx, dAi, 2048, KI, PB, C, T_B, true);       // (dA f)   k_hat
       product<128, false, true>(cx, dMi, 2048, KI, PB, C, T_Q, true);       // (dM f)   k_hat
@@ -953,7 +992,11 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
 #pragma unroll
       for (int it = 0; it < 4; ++it) {
         const int p = it * 4 + rp;
-        if (live && p < kp) {
+        if constexpr (SC) {
+          const bool on = live && p < kp;
+          RK[p * PP + rx] = on ? kraw4[it] : make_uint4(0, 0, 0, 0);
+          RQ[p * PP + rx] = on ? qraw4[it] : make_uint4(0, 0, 0, 0);
+        } else if (live && p < kp) {
           umma::cp_async16(RK + p * PP + rx, krow + 16 * p);
           umma::cp_async16(RQ + p * PP + rx, qrow + 16 * p);
         } else RK[p * PP + rx] = RQ[p * PP + rx] = make_uint4(0, 0, 0, 0);
@@ -971,6 +1014,15 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     umma::cp_async_commit();
     umma::cp_async_wait<0>();
     __syncthreads();
+    // the next tile's dO, where dM was (the raw b, where there is one per channel, reaches there)
+    const int ne = hd + 1 < D ? e_item : e_item + (int)gridDim.x, nhd = hd + 1 < D ? hd + 1 : 0;
+    const bool more = ne < units && (SC || next_strong_s == 0);
+    staged_dO = more && bC == 1;
+    if (staged_dO) {
+      int nb, nh, nc;
+      place(ne, nhd, nb, nh, nc);
+      stage_dO(sl.at(5), a.d_out, ((size_t)nb * g.L + nc * C) * g.Hv * g.V + (size_t)nh * vr, dO_pitch, g.L - nc * C < C ? g.L - nc * C : C, NH == 2 ? 16 : vr / 8, qdt);
+    }
     // ---- combination, a row per lane, 32 channels per warp.  d q_n, d k_n and dLambda wait in the columns just read for the
     //      row sums of the l2norm adjoint.
     {
@@ -1167,9 +1219,8 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       return (guard ? graw < -1e-6f : graw <= 0.f) ? d : 0.f;               // through min(min(g, 0), -1e-6)
     };
     // the next tile's first operands, where the raw rows were (asked for by a warp that has little left to do)
-    const int ne = hd + 1 < D ? e_item : e_item + (int)gridDim.x;
-    loaded = ne < units && (SC || next_strong_s == 0);
-    auto load_next = [&] { if (loaded) load_first(tile_of(ne, hd + 1 < D ? hd + 1 : 0), 480); };
+    loaded = more;
+    auto load_next = [&] { if (loaded) load_first(tile_of(ne, nhd), 480); };
     if constexpr (SC) {
       __syncthreads();
       load_next();
