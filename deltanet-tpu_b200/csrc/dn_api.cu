@@ -222,15 +222,6 @@ int dn_prepass_fwd(const dn_shape* s, const void* q, const void* k, const void* 
                             scratch_bytes / sizeof(float), (cudaStream_t)stream);
 }
 
-// The forward chain of a checked call.  follows: launched right behind the prepass that it takes its tiles from.
-static int run_state_fwd(const Geo& g, const dn_residuals& res, const int32_t* seg, const float* init_state, void* out, float* final_state,
-                         bool follows, cudaStream_t st) {
-  StateArgs a{};
-  a.g = g; a.res = res; a.seg = seg; a.init_state = (g.flags & DN_HAS_INIT) ? init_state : nullptr;
-  a.out = out; a.final_state = final_state; a.states = res.states; a.early = follows;
-  return launch_state_fwd(a, st);
-}
-
 int dn_state_fwd(const dn_shape* s, const dn_residuals* res, const int32_t* seg,
                  const float* init_state, void* out, float* final_state, void* stream) {
   Geo g;
@@ -240,7 +231,10 @@ int dn_state_fwd(const dn_shape* s, const dn_residuals* res, const int32_t* seg,
   if (!res || (!out && !final_state && !res->states)) return DN_ERR_NULL_POINTER;
   if ((g.flags & DN_HAS_INIT) && !init_state) return DN_ERR_NULL_POINTER;
   if (!images_aligned(g, *res) || (g.img && !aligned16({out}))) return DN_ERR_MISALIGNED;
-  return run_state_fwd(g, *res, seg, init_state, out, final_state, false, (cudaStream_t)stream);
+  StateArgs a{};
+  a.g = g; a.res = *res; a.seg = seg; a.init_state = (g.flags & DN_HAS_INIT) ? init_state : nullptr;
+  a.out = out; a.final_state = final_state; a.states = res->states;
+  return launch_state_fwd(a, (cudaStream_t)stream);
 }
 
 int dn_recompute_states(const dn_shape* s, const dn_residuals* res, const int32_t* seg,
@@ -408,7 +402,7 @@ int dn_chunk_fwd(const dn_shape* s, const void* q, const void* k, const void* v,
     return launch_state_fwd_tc(a, st);
   }
   if ((rc = dn_prepass_fwd(s, q, k, v, g_, b, w, seg, res, p, (size_t)(end - p), stream))) return rc;
-  return run_state_fwd(g, *res, seg, init_state, out, final_state, true, (cudaStream_t)stream);
+  return dn_state_fwd(s, res, seg, init_state, out, final_state, stream);
 }
 
 int dn_chunk_bwd(const dn_shape* s, const void* q, const void* k, const void* v,

@@ -36,7 +36,6 @@ struct StateArgs {
   int c_begin, c_end;
   float* carry;
   int* err;                  // error word (bounded waits report here); set by the launchers
-  bool early;                // the launch may begin while the one before it in the stream, the forward prepass, ends (small jobs)
   int parts;                 // walks the range may be cut into at document boundaries (tensor-core path; set by the launcher)
   // Sequence-sharded use.  P_out (B,H,K,K): the forward launch carries K extra "value" columns per
   // (batch, head) that start from the identity with U = 0 and end as the shard's transition matrix

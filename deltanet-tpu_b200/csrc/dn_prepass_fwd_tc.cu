@@ -227,8 +227,6 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
 __device__ __forceinline__ umma::Ctx setup(uint64_t* bar, uint32_t* base, int* err) {
   if (threadIdx.x == 0) { umma::mbar_init(bar, 1); umma::fence_mbar_init(); }
   if (threadIdx.x < 32) umma::tmem_alloc(base, 256);
-  umma::wait_for_previous();
-  umma::let_next_begin();
   umma::tc_fence_before();
   __syncthreads();
   umma::tc_fence_after();
@@ -982,9 +980,7 @@ int launch_prepass_fwd_tc(const Geo& g, const void* q, const void* k, const void
   int* err = device_error_ptr();
   auto go = [&](auto kernel) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    // (a job of one item per SM at most, in one piece: it may move in while the launch before it, the chain of the call before, ends)
-    if (a.items <= sm_count() && a.c_begin == 0 && a.c_end == g.NC) umma::launch_early(kernel, dim3(grid), NT, SMEM_BYTES, st, a, err);
-    else kernel<<<grid, NT, SMEM_BYTES, st>>>(a, err);
+    kernel<<<grid, NT, SMEM_BYTES, st>>>(a, err);
   };
   auto pick = [&](auto vw) {
     constexpr int VW = decltype(vw)::value;

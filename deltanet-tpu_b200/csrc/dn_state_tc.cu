@@ -219,10 +219,6 @@ __global__ void __launch_bounds__(Plan<VS, false>::NT, 1) state_fwd_tc_kernel(co
     stop_s = ce;
   }
   if (warp == 0) umma::tmem_alloc(&tmem_base, PL::TMEM);
-  if (!CUT) {
-    umma::wait_for_previous();
-    umma::let_next_begin();
-  }
   umma::tc_fence_before();
   __syncthreads();
   // the first chunk behind which nothing depends on the state that this launch starts from
@@ -744,11 +740,7 @@ int launch_fwd(const StateArgs& a, cudaStream_t st) {
   using PL = Plan<VS, false>;
   const dim3 grid((a.g.Vw + (a.P_out ? a.g.K : 0)) / VS, a.g.H, a.g.B * a.parts);
   cudaFuncSetAttribute(state_fwd_tc_kernel<VS, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL::SMEM);
-  if (!CUT && a.early && a.g.B * a.g.H * a.g.NC + (int)(grid.x * grid.y * grid.z) <= sm_count()) {
-    umma::launch_early(state_fwd_tc_kernel<VS, CUT>, grid, PL::NT, PL::SMEM, st, a);
-  } else {
-    state_fwd_tc_kernel<VS, CUT><<<grid, PL::NT, PL::SMEM, st>>>(a);
-  }
+  state_fwd_tc_kernel<VS, CUT><<<grid, PL::NT, PL::SMEM, st>>>(a);
   return launch_status();
 }
 template <int VS, bool CUT>
