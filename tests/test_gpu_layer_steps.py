@@ -152,3 +152,30 @@ def test_layer_core_matches_qwen3_5_torch_reference(dn):
     assert O.rel_l2(od.cpu(), o_ref) < 2e-4
     assert O.rel_l2(sd.cpu(), s_ref) < 2e-4
     assert O.rel_l2(yd.cpu(), y_ref) < 2e-4
+
+
+@pytest.mark.parametrize("W", [4, 2])
+@pytest.mark.parametrize("L", [1, 3, 4, 5, 63, 66, 259, 517])
+def test_producer_batches(dn, W, L):
+    """Rows are worked on in batches of four, whole ones without tests: lengths either side of a batch and of a run, and document
+    boundaries at each place of a batch, against 64 bits.  fp32: three sums of at most L terms each, their order free."""
+    B, Hk, Hv, K, V = 2, 1, 1, 64, 64
+    D = 2 * Hk * K + Hv * V
+    gen = torch.Generator().manual_seed(1000 * W + L)
+    seg = torch.zeros(B, L, dtype=torch.int32)
+    for i, t in enumerate((8, 21, 34, 47, 48, 61, 256, 261)):      # at offsets 0, 1, 2, 3, 0, 1 of a batch, and around a run's start
+        seg[0, t:] = i + 1
+    mixed, dy = torch.randn(B, L, D, generator=gen), torch.randn(B, L, D, generator=gen)
+    w, bias = torch.randn(D, 1, W, generator=gen) * 0.5, torch.randn(D, generator=gen) * 0.1
+    ref_in = [t.double().requires_grad_() for t in (mixed, w, bias)]
+    xp = F.pad(ref_in[0], (0, 0, W - 1, 0))
+    ids = F.pad(seg, (W - 1, 0), value=-1)
+    pre = ref_in[2] + sum(xp[:, j:j + L] * ref_in[1][:, 0, j] * (ids[:, j:j + L] == seg)[..., None] for j in range(W))
+    ref = F.silu(pre)
+    g_ref = torch.autograd.grad((ref * dy).sum(), ref_in)
+    dev = [t.cuda().requires_grad_() for t in (mixed, w, bias)]
+    parts = dn.gdn_qkv_producer(*dev, num_k_heads=Hk, num_v_heads=Hv, head_k_dim=K, head_v_dim=V, segment_ids=seg.cuda())
+    got = torch.cat([t.reshape(B, L, -1) for t in parts], -1)
+    g_dev = torch.autograd.grad((got * dy.cuda()).sum(), dev)
+    for a, r in zip((got,) + g_dev, (ref,) + g_ref):
+        assert O.rel_l2(a.detach().double().cpu(), r.detach()) < 1e-5
