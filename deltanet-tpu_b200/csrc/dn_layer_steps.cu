@@ -22,8 +22,8 @@ namespace {
 
 constexpr int CG = 8;            // channels per thread (one 16-byte bf16 vector)
 constexpr int PT = 128;          // threads per CTA of the producer kernels (= 1024 channels)
-constexpr int TT_FWD = 64;       // tokens per thread run, forward
-constexpr int TT_BWD = 256;      // tokens per thread run, backward (also the tile of the weight-gradient partials)
+constexpr int TT_FWD = 64;       // longest run of tokens of a thread, forward
+constexpr int TT_BWD = 256;      // the same, backward (a run is also a tile of the weight-gradient partials)
 constexpr int MAXW = 4;
 
 __device__ __forceinline__ float silu(float x) { return x * __frcp_rn(1.f + __expf(-x)); }
@@ -40,6 +40,7 @@ struct ProducerArgs {
   const int32_t* seg;            // (B,L) or null: taps from another document read as zero
   int B, L, D, W, dt;
   int qk_dim, Hk_K;              // Hk*K: channels [0,HkK) -> q, [HkK, 2HkK) -> k, rest -> v
+  int run;                       // tokens per thread run, a multiple of 4
   void *q, *k, *v;               // forward outputs / backward: their cotangents
   void* d_mixed;                 // backward
   float* part;                   // backward: (tiles, D, W+1) partial sums of d w | d bias
@@ -199,8 +200,9 @@ template <int W, int NB> __device__ __forceinline__ bool one_document(const int*
 // of ids and ends (nearly every batch does); both instances add in the same order.  Measured at 2 x 4001 tokens of 8192
 // channels, bf16, W = 4: 62.2 us with a test per tap and scalar arithmetic, 58.2 without the tests, 54.5 with packed arithmetic
 // besides (4.8 TB/s); 4 x 4096 tokens 109.8, 103.6, 96.8.
-template <int W, bool BF16>
+template <int W, bool BF16, bool LONG>
 __global__ void __launch_bounds__(PT, 4) producer_fwd_kernel(ProducerArgs a) {
+  const int run = LONG ? TT_FWD : a.run;
   constexpr int NB = 4, NS = BF16 ? 4 : 2;           // rows per batch, batches in the ring (32 KB either way)
   constexpr int ES = BF16 ? 2 : 4, NP = CG * ES / 16;  // element size; 16-byte copies per row and thread
   __shared__ __align__(16) uint8_t ring[NS * NB * NP * PT * 16];
@@ -208,10 +210,10 @@ __global__ void __launch_bounds__(PT, 4) producer_fwd_kernel(ProducerArgs a) {
   const int tid = threadIdx.x;
   const bool active = (blockIdx.y * PT + tid) * CG < a.D;
   const int c0 = active ? (blockIdx.y * PT + tid) * CG : 0;
-  const int tiles_per_row = (a.L + TT_FWD - 1) / TT_FWD;
-  const int b = blockIdx.x / tiles_per_row, t0 = (blockIdx.x % tiles_per_row) * TT_FWD;
+  const int tiles_per_row = (a.L + run - 1) / run;
+  const int b = blockIdx.x / tiles_per_row, t0 = (blockIdx.x % tiles_per_row) * run;
   const size_t row0 = (size_t)b * a.L;
-  const int t_end = min(t0 + TT_FWD, a.L);
+  const int t_end = min(t0 + run, a.L);
   const int nbatch = (t_end - t0 + NB - 1) / NB;
   const char* src = reinterpret_cast<const char*>(a.mixed);
   const char* first = src + ((row0 + t0) * a.D + c0) * ES;
@@ -229,7 +231,7 @@ __global__ void __launch_bounds__(PT, 4) producer_fwd_kernel(ProducerArgs a) {
   };
 #pragma unroll
   for (int bi = 0; bi < NS - 1; ++bi) fetch(bi);
-  for (int i = tid; i < TT_FWD + W - 1; i += PT) {
+  for (int i = tid; i < run + W - 1; i += PT) {
     const int t = t0 - (W - 1) + i;
     seg_sm[i] = t < 0 ? -1 : (a.seg ? __ldg(a.seg + row0 + min(t, a.L - 1)) : 0);
   }
@@ -296,7 +298,7 @@ __global__ void __launch_bounds__(PT, 4) producer_fwd_kernel(ProducerArgs a) {
   umma::cp_async_wait<0>();
 }
 
-// Backward of the producer over one run of TT_BWD tokens: with pre[u] the conv output of token u and
+// Backward of the producer over one run of tokens: with pre[u] the conv output of token u and
 // dpre[u] = dy[u] * silu'(pre[u]),
 //   d x[s]    = sum_j w[j] * dpre[s + (W-1-j)]      (taps inside the same document)
 //   d w[j]   += dpre[u] * x[u - (W-1) + j],   d bias += dpre[u]    (u inside this run)
@@ -308,8 +310,9 @@ __global__ void __launch_bounds__(PT, 4) producer_fwd_kernel(ProducerArgs a) {
 // 123.4 us with a test per tap and scalar arithmetic, 118.3 without the tests, 94.5 with packed arithmetic besides (4.2 TB/s;
 // packed arithmetic under the tests was slower, 137); 4 x 4096 tokens 210.8, 200.0, 157.7.
 constexpr int CB = 4;
-template <int W, bool BF16>
+template <int W, bool BF16, bool LONG>
 __global__ void __launch_bounds__(PT, 4) producer_bwd_kernel(ProducerArgs a) {
+  const int run = LONG ? TT_BWD : a.run;
   constexpr int NB = 4, NS = BF16 ? 4 : 2;
   constexpr int ES = BF16 ? 2 : 4, RB = CB * ES;     // bytes per row, thread and tensor: 8 or 16
   __shared__ __align__(16) uint8_t ring[NS * NB * 2 * PT * RB];       // x rows | cotangent rows
@@ -317,10 +320,10 @@ __global__ void __launch_bounds__(PT, 4) producer_bwd_kernel(ProducerArgs a) {
   const int tid = threadIdx.x;
   const bool active = (blockIdx.y * PT + tid) * CB < a.D;
   const int c0 = active ? (blockIdx.y * PT + tid) * CB : 0;
-  const int tiles_per_row = (a.L + TT_BWD - 1) / TT_BWD;
-  const int b = blockIdx.x / tiles_per_row, t0 = (blockIdx.x % tiles_per_row) * TT_BWD;
+  const int tiles_per_row = (a.L + run - 1) / run;
+  const int b = blockIdx.x / tiles_per_row, t0 = (blockIdx.x % tiles_per_row) * run;
   const size_t row0 = (size_t)b * a.L;
-  const int t_end = min(t0 + TT_BWD, a.L);
+  const int t_end = min(t0 + run, a.L);
   const int u_end = t_end + W - 1;                   // look-ahead rows; rows >= L contribute nothing
   const int nbatch = (u_end - t0 + NB - 1) / NB;
   const int HkK = a.Hk_K, Dv = a.D - 2 * HkK;
@@ -344,7 +347,7 @@ __global__ void __launch_bounds__(PT, 4) producer_bwd_kernel(ProducerArgs a) {
   };
 #pragma unroll
   for (int bi = 0; bi < NS - 1; ++bi) fetch(bi);
-  for (int i = tid; i < TT_BWD + 2 * MAXW; i += PT) {
+  for (int i = tid; i < run + 2 * MAXW; i += PT) {
     const int t = t0 - (W - 1) + i;
     seg_sm[i] = t < 0 ? -1 : (t >= a.L ? -2 : (a.seg ? __ldg(a.seg + row0 + t) : 0));
   }
@@ -691,11 +694,27 @@ template <typename KernelT> int resident_ctas(KernelT kernel) {
 
 using namespace dn;
 
+// Length of the producer's runs.  A run is walked row by row, so a small call takes as long as one run does: runs are halved
+// while all CTAs, at half the length, still fit the chip together: four per SM in the backward (its runs are long); one in the
+// forward, where more only add halo rows and the set-up of taps.  Backward, D channels and L tokens: D = 2048, L = 301
+// 37.6 -> 9.1 us (runs of 32), D = 3072, L = 1501 37.9 -> 12.5 (32), D = 1024, L = 9001 37.5 -> 20.7 (32).  Forward, at D = 2048, L = 301
+// 11.9 -> 6.3 (16); up to four per SM, D = 1024, L = 9001 had gone from 13.8 to 17.9.  The longest run keeps an instance with its length
+// known (with the length in a register: 94.7 -> 95.9 us at 2 x 4001 tokens of 8192 channels).  The length is a function of the sizes
+// alone (148 SMs): the scratch is sized by it, and the order of the weight gradient's sum must not depend on the device.
+static int producer_run(int B, int L, int D, bool bwd) {
+  const int per_cta = PT * (bwd ? CB : CG), shortest = bwd ? 32 : 16, room = (bwd ? 4 : 1) * 148;
+  const int64_t cols = (D + per_cta - 1) / per_cta;
+  int run = bwd ? TT_BWD : TT_FWD;
+  while (run > shortest && B * cols * ((L + run / 2 - 1) / (run / 2)) <= room) run /= 2;
+  return run;
+}
+
 extern "C" {
 
 size_t dn_gdn_producer_scratch_bytes(int32_t B, int32_t L, int32_t D, int32_t W) {
   if (B < 1 || L < 1 || D < 1 || W < 2 || W > 4) return 0;
-  const size_t tiles = (size_t)B * ((L + TT_BWD - 1) / TT_BWD);
+  const int run = producer_run(B, L, D, true);
+  const size_t tiles = (size_t)B * ((L + run - 1) / run);
   return tiles * D * (W + 1) * sizeof(float);
 }
 
@@ -717,12 +736,19 @@ int dn_gdn_producer_fwd(const void* mixed, const float* conv_w, const float* con
   if (rc) return rc;
   if (!q || !k || !v) return DN_ERR_NULL_POINTER;
   a.q = q; a.k = k; a.v = v;
-  dim3 grid(B * ((L + TT_FWD - 1) / TT_FWD), (a.D / CG + PT - 1) / PT);
+  a.run = producer_run(B, L, a.D, false);
+  dim3 grid(B * ((L + a.run - 1) / a.run), (a.D / CG + PT - 1) / PT);
   cudaStream_t st = (cudaStream_t)stream;
   const bool bf = dtype == DN_BF16;
-#define DN_GO(WW) (bf ? producer_fwd_kernel<WW, true><<<grid, PT, 0, st>>>(a) : producer_fwd_kernel<WW, false><<<grid, PT, 0, st>>>(a))
-  if (W == 4) DN_GO(4); else if (W == 3) DN_GO(3); else DN_GO(2);
-#undef DN_GO
+  auto go = [&](auto width, auto is_long) {
+    constexpr int WW = decltype(width)::value;
+    constexpr bool LONG = decltype(is_long)::value;
+    if (bf) producer_fwd_kernel<WW, true, LONG><<<grid, PT, 0, st>>>(a); else producer_fwd_kernel<WW, false, LONG><<<grid, PT, 0, st>>>(a);
+  };
+  auto pick = [&](auto width) { if (a.run == TT_FWD) go(width, std::true_type{}); else go(width, std::false_type{}); };
+  if (W == 4) pick(std::integral_constant<int, 4>{});
+  else if (W == 3) pick(std::integral_constant<int, 3>{});
+  else pick(std::integral_constant<int, 2>{});
   return launch_status();
 }
 
@@ -737,13 +763,20 @@ int dn_gdn_producer_bwd(const void* mixed, const float* conv_w, const float* con
   if (scratch_bytes < dn_gdn_producer_scratch_bytes(B, L, a.D, W)) return DN_ERR_SCRATCH_TOO_SMALL;
   a.q = const_cast<void*>(dq); a.k = const_cast<void*>(dk); a.v = const_cast<void*>(dv);
   a.d_mixed = d_mixed; a.part = reinterpret_cast<float*>(scratch);
-  const int tiles = B * ((L + TT_BWD - 1) / TT_BWD);
+  a.run = producer_run(B, L, a.D, true);
+  const int tiles = B * ((L + a.run - 1) / a.run);
   dim3 grid(tiles, (a.D / CB + PT - 1) / PT);
   cudaStream_t st = (cudaStream_t)stream;
   const bool bf = dtype == DN_BF16;
-#define DN_GO(WW) (bf ? producer_bwd_kernel<WW, true><<<grid, PT, 0, st>>>(a) : producer_bwd_kernel<WW, false><<<grid, PT, 0, st>>>(a))
-  if (W == 4) DN_GO(4); else if (W == 3) DN_GO(3); else DN_GO(2);
-#undef DN_GO
+  auto go = [&](auto width, auto is_long) {
+    constexpr int WW = decltype(width)::value;
+    constexpr bool LONG = decltype(is_long)::value;
+    if (bf) producer_bwd_kernel<WW, true, LONG><<<grid, PT, 0, st>>>(a); else producer_bwd_kernel<WW, false, LONG><<<grid, PT, 0, st>>>(a);
+  };
+  auto pick = [&](auto width) { if (a.run == TT_BWD) go(width, std::true_type{}); else go(width, std::false_type{}); };
+  if (W == 4) pick(std::integral_constant<int, 4>{});
+  else if (W == 3) pick(std::integral_constant<int, 3>{});
+  else pick(std::integral_constant<int, 2>{});
   if ((rc = launch_status())) return rc;
   const size_t n = (size_t)a.D * (W + 1);
   tile_sum_kernel<<<(unsigned)((n + 31) / 32), 256, 0, st>>>(a.part, tiles, n, d_conv_w, d_conv_b, W);
