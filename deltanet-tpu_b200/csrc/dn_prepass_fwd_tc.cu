@@ -129,8 +129,11 @@ __device__ __forceinline__ void prefetch_kq(const PrepassFwdArgs& a, int e_item)
 
 // T = (I + A)^-1, then W = T X and U = T (w v).  X image and A visible to all threads on entry.
 // others(): run by warps that wait for the substitution (tri::invert); ahead(): run by all as soon as the products have read their
-// operands (the images of X and T are free then).
-template <int VW, class OTHERS, class AHEAD>
+// operands (the images of X and T are free then).  ONE_ROW: a thread takes four pieces of one row of v and w instead of two pieces of two
+// rows.  That is twice the lookups, but one address: with write gates per column or of a type known at run time, whose rows a thread
+// addresses as well, the other mapping spilled up to 290 bytes more a thread (64 registers).  Ten launches of 256 columns, L = 20011: 798 -> 769 us;
+// fused prologue, L = 4000, 32 heads: 222 -> 204; 64-wide heads, 16 of them: 177 -> 162.
+template <int VW, bool ONE_ROW, class OTHERS, class AHEAD>
 __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm, const PrepassFwdArgs& a, int h, int b, int t0,
                                                      size_t ibase, int qdt, int gdt, int wC, bool fuse, OTHERS others, AHEAD ahead) {
   constexpr int NH = VW / 128;
@@ -143,39 +146,58 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
   uint4* Wimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.W) + ibase * C * K);
   uint4* Uimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.U) + ibase * C * VW);
   const int vr = g.G * g.V, vsh = g.V == 128 ? 7 : 6;   // value columns that exist
+  constexpr int YP = ONE_ROW ? PP : PQ;                   // panels of Y
   uint4 vraw[4];                                          // a half's pieces of v (bf16) and scalar write gates, requested ahead of use
-  uint32_t w1[4];
-  auto row_at = [&](int it) { const int x = row8_of(tid, it); return (size_t)b * g.L + (t0 + x < g.L ? t0 + x : t0); };
+  [[maybe_unused]] uint32_t w1[4];
+  auto row_of_it = [&](int it) { return ONE_ROW ? row_of(tid) : row8_of(tid, it); };
+  auto piece_of_it = [&](int it) { return ONE_ROW ? it * 4 + piece_of(tid) : piece8_of(tid, it); };
+  [[maybe_unused]] auto row_at = [&](int it) { const int x = row_of_it(it); return (size_t)b * g.L + (t0 + x < g.L ? t0 + x : t0); };
+  // ONE_ROW: the thread's row and its elements of v
+  const bool live0 = t0 + row_of(tid) < g.L;
+  const size_t tok0 = (size_t)b * g.L + (live0 ? t0 + row_of(tid) : t0);
+  const uint8_t* vrow = reinterpret_cast<const uint8_t*>(a.v) + (tok0 * g.Hv * g.V + (size_t)h * vr) * dt_size(qdt);
   auto request_v = [&](int half) {
+    if constexpr (ONE_ROW) {
+      if (qdt == DN_BF16) {
 #pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int col0 = half * 128 + 8 * piece8_of(tid, it), cc = col0 < vr ? col0 : 0;
-      const size_t tok = row_at(it);
-      if (wC == 1) w1[it] = ldbits_ro(a.w, tok * g.wH + g.w_of(h * g.G + (cc >> vsh)), gdt);
-      if (qdt == DN_BF16)
-        vraw[it] = col0 < vr ? __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.v) + tok * g.Hv * g.V + (size_t)h * vr + col0)) : make_uint4(0, 0, 0, 0);
+        for (int it = 0; it < 4; ++it)
+          vraw[it] = half * 128 + 32 * it < vr ? __ldg(reinterpret_cast<const uint4*>(vrow) + half * 16 + it * 4 + piece_of(tid)) : make_uint4(0, 0, 0, 0);
+      }
+    } else {
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int col0 = half * 128 + 8 * piece_of_it(it), cc = col0 < vr ? col0 : 0;
+        const size_t tok = row_at(it);
+        if (wC == 1) w1[it] = ldbits_ro(a.w, tok * g.wH + g.w_of(h * g.G + (cc >> vsh)), gdt);
+        if (qdt == DN_BF16)
+          vraw[it] = col0 < vr ? __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.v) + tok * g.Hv * g.V + (size_t)h * vr + col0)) : make_uint4(0, 0, 0, 0);
+      }
     }
   };
   auto build_y = [&](uint4* Y, int half) {              // Y = w v of the half's columns
 #pragma unroll
     for (int it = 0; it < 4; ++it) {
-      const int x = row8_of(tid, it), p = piece8_of(tid, it);
+      const int x = row_of_it(it), p = piece_of_it(it);
       const int col0 = half * 128 + 8 * p, cv = col0 & (g.V - 1);
-      if (col0 >= vr) { Y[p * PQ + x] = make_uint4(0, 0, 0, 0); continue; }
-      const size_t tok = row_at(it);
+      if (col0 >= vr) { Y[p * YP + x] = make_uint4(0, 0, 0, 0); continue; }
+      const size_t tok = ONE_ROW ? tok0 : row_at(it);
       float vv[8], ww[8];
       if (wC == 1) {
+        float w_row;
+        if constexpr (ONE_ROW) w_row = ldf_ro(a.w, tok * g.wH + g.w_of(h * g.G + (col0 >> vsh)), gdt);
+        else w_row = bits_value(w1[it], gdt);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) ww[i] = bits_value(w1[it], gdt);
+        for (int i = 0; i < 8; ++i) ww[i] = w_row;
       } else {
         load8(a.w, (tok * g.wH + g.w_of(h * g.G + (col0 >> vsh))) * wC + cv, gdt, ww);
       }
       if (qdt == DN_BF16) umma::unpack8(vraw[it], vv);
+      else if (ONE_ROW) { const Raw8 r = ldraw(vrow, half * 16 + p, qdt); cvraw(r, qdt, vv); }
       else load8(a.v, tok * g.Hv * g.V + (size_t)h * vr + col0, qdt, vv);
-      const bool live = t0 + x < g.L;
+      const bool live = ONE_ROW ? live0 : t0 + x < g.L;
 #pragma unroll
       for (int i = 0; i < 8; ++i) vv[i] = live ? (fuse ? sigmoid_fast(ww[i]) : ww[i]) * vv[i] : 0.f;
-      Y[p * PQ + x] = umma::pack8(vv);
+      Y[p * YP + x] = umma::pack8(vv);
     }
   };
   tri::invert(Tp, reinterpret_cast<float*>(TI), others);
@@ -185,7 +207,7 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
   build_y(Y0, 0);
   umma::pre_issue_sync();
   umma::issue_pitched<128, false, true>(cx, TI, 2048, XI, PB, C, 0, false);
-  umma::issue_pitched<128, false, true>(cx, TI, 2048, Y0, PQB, C, 128, false);
+  umma::issue_pitched<128, false, true>(cx, TI, 2048, Y0, 16 * YP, C, 128, false);
   umma::commit(cx);
   if (NH == 2) request_v(1);
   if (a.res.T) {                                        // the image of T, for the backward
@@ -206,7 +228,7 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
   if (NH == 2) {                                        // the second half goes where W was
     __syncthreads();
     umma::tc_fence_after();
-    umma::issue_pitched<128, false, true>(cx, TI, 2048, XI, PQB, C, 0, false);
+    umma::issue_pitched<128, false, true>(cx, TI, 2048, XI, 16 * YP, C, 0, false);
     umma::commit(cx);
   }
   umma::drain<NT, 128>(cx, 128, [&](int row, int col, const float (&v)[16]) {
@@ -417,7 +439,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_scalar_kernel(const __grid_
     }
     __syncthreads();
     const int next = e_item + gridDim.x;
-    inverse_and_products<VW>(cx, sm, a, h, b, t0, ibase, DN_BF16, g.gate_dt, g.wC, false, [&]() {
+    inverse_and_products<VW, false>(cx, sm, a, h, b, t0, ibase, DN_BF16, g.gate_dt, g.wC, false, [&]() {
       // (the requests: 779 -> 741 us at B=4 L=8192 Hv=32.  With decay per channel they cost more than they hide,
       // 761 -> 819 us at L=20011: that kernel reads q, k, b, g in groups and has other tiles to switch to.)
       if (warp < 8) prefetch_vw(a, h, b, t0);
@@ -731,23 +753,20 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
     const uint8_t* grow = reinterpret_cast<const uint8_t*>(a.gg) +
         (((size_t)b * g.L + t0 + (warp * 8 < rows ? warp * 8 : 0)) * g.gH + g.g_head(h)) * gC * ges + (gC == 1 ? 0 : lane) * ges;
     float gv[8];
-    uint32_t graw[8];
-    const uint32_t off_bits = gdt == DN_BF16 ? 0xff80u : 0xff800000u;      // -infinity
     auto load_g = [&](int grp) {
       const bool cin = gC == 1 || CF::fixed || 32 * grp < gC;
       const uint8_t* gp = grow + (gC == 1 ? 0 : 32 * grp * ges);
       if (rows == C && cin) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) graw[i] = ldbits_ro(gp + i * gpitch, 0, gdt);
+        for (int i = 0; i < 8; ++i) gv[i] = ldf_ro(gp + i * gpitch, 0, gdt);
       } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) graw[i] = cin && warp * 8 + i < rows ? ldbits_ro(gp + i * gpitch, 0, gdt) : (fuse ? off_bits : 0u);
+        for (int i = 0; i < 8; ++i) gv[i] = cin && warp * 8 + i < rows ? ldf_ro(gp + i * gpitch, 0, gdt) : (fuse ? -INFINITY : 0.f);
       }
     };
     auto act_g = [&]() {                                // the activated decay (rows past the end: 0)
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        gv[i] = bits_value(graw[i], gdt);
         if (fuse) { const bool off = gv[i] == -INFINITY; gv[i] = off ? 0.f : -umma::ex2_fast(fminf(gv[i], 5.f) * DN_LOG2E); if (guard && !off) gv[i] = fminf(gv[i], -1e-6f); }
         else { gv[i] = gv[i] <= 0.f ? gv[i] : 0.f; if (guard && warp * 8 + i < rows) gv[i] = fminf(gv[i], -1e-6f); }
       }
@@ -957,7 +976,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       drain_am(cx, reinterpret_cast<float*>(sm + OFF_T), Mimg, ds_s[(warp & 3) * 32 + lane], [](int, float (&)[16], float (&)[16]) {});
       __syncthreads();
     }
-    inverse_and_products<VW>(cx, sm, a, h, b, t0, ibase, qdt, gdt, wC, fuse, [] {}, [] {});
+    inverse_and_products<VW, !CF::scalar_bw>(cx, sm, a, h, b, t0, ibase, qdt, gdt, wC, fuse, [] {}, [] {});
   }
   teardown(tbase);
 }
