@@ -490,11 +490,8 @@ int dn_sp_transition(const dn_shape* s, const dn_residuals* res, const int32_t* 
   if (peek_device_error()) return DN_ERR_DEVICE_WAIT;
   if (!res || !identity || !P) return DN_ERR_NULL_POINTER;
   if (!images_aligned(g, *res)) return DN_ERR_MISALIGNED;
-  Geo t = g;                       // same chunks and heads, value width K, one "value head" per exec head
-  t.Hv = g.H; t.G = 1; t.V = g.K; t.Vw = g.Kt; t.qk_div = 1;
-  t.flags |= DN_HAS_INIT;
   StateArgs a{};
-  a.g = t; a.res = *res; a.res.U = nullptr; a.res.states = nullptr; a.seg = seg;
+  a.g = transition_geo(g); a.res = *res; a.res.U = nullptr; a.res.states = nullptr; a.seg = seg;
   a.init_state = identity; a.final_state = P;
   return launch_state_fwd(a, (cudaStream_t)stream);
 }

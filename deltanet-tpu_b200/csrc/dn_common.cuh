@@ -56,6 +56,11 @@ struct Geo {
   // [(col / 8) * 128 + row] where they stand: another layout means editing each of them.
   bool img;
   FastDiv by_BH, by_H, by_q, by_g, by_b, by_w;           // B H, H, qk_div; exec heads per head of g and b, value heads per head of w
+  // whoever sets or changes a head count calls this last
+  __host__ void set_divisors() {
+    by_BH.set(B * H); by_H.set(H); by_q.set(qk_div);
+    by_g.set(H / gH); by_b.set(H / bH); by_w.set(Hv / wH);
+  }
   // tile `e` of the chunks from c_begin on, in the order chunk, batch, head
   __host__ __device__ __forceinline__ void tile(int e, int c_begin, int& b, int& h, int& c) const {
     int bh;
@@ -126,9 +131,18 @@ inline int make_geo(const dn_shape* s, Geo* g) {
   g->pre_dt = s->precision == DN_PREC_BF16 ? DN_BF16 : DN_F32;
   g->flags = s->flags; g->scale = s->scale;
   g->img = tc;
-  g->by_BH.set(g->B * g->H); g->by_H.set(g->H); g->by_q.set(g->qk_div);
-  g->by_g.set(g->H / g->gH); g->by_b.set(g->H / g->bH); g->by_w.set(g->Hv / g->wH);
+  g->set_divisors();
   return DN_OK;
+}
+
+// The geometry of a shard's transition matrix: the chunks and exec heads of `g`, K value columns, one value head per exec
+// head (the gates of v have been applied where there is no v: w counts as one head).
+inline Geo transition_geo(const Geo& g) {
+  Geo t = g;
+  t.Hv = g.H; t.G = 1; t.V = g.K; t.Vw = g.Kt; t.qk_div = 1; t.wH = 1;
+  t.flags |= DN_HAS_INIT;
+  t.set_divisors();
+  return t;
 }
 
 // On the image path three more arrays are kept as bf16 operand images, [col / 8][128 rows][8]:
