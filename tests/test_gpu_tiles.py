@@ -160,7 +160,6 @@ def test_tiles_after_the_first(dn, form):
 
     whole, apart = call(slice(None)), zip(*[call(slice(r, r + 1)) for r in range(B)])
     for i, (x, y) in enumerate(zip(whole, (torch.cat(t) for t in apart))):
-        print(form, i, (x != y).sum().item(), O.rel_l2(x.float(), y.float()))
         assert torch.equal(x, y), (i, O.rel_l2(x.float(), y.float()))
 
 
