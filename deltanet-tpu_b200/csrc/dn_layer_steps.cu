@@ -494,19 +494,22 @@ __global__ void __launch_bounds__(256) gates_fwd_kernel(const void* a_, const vo
 // da, db element-wise; dA_log[h] = sum dg * g, d dt_bias[h] = sum dg * dg/d(a).  A cluster of 8 CTAs takes 4 heads (so that a
 // thread's neighbours read next to it) and adds its partial sums in a fixed order through distributed shared memory:
 // 52 us -> 17 us at 8002 tokens x 32 heads, where one CTA per head walked the tokens alone.  A thread's tokens are a chain of loads and
-// special functions, four tokens in flight: with 512 threads instead of 256 17.6 -> 11.4 us there and 28.2 -> 15.9 at 16384 tokens (33 tokens:
-// 3.3 -> 3.6); 1024 threads leave 64 registers, which spill with four in flight: 9.7 and 13.7 with two, and 4.3 at 33 tokens.
-constexpr int GB_CTAS = 8, GB_HEADS = 4, GB_THREADS = 512;
-__global__ void __cluster_dims__(GB_CTAS, 1, 1) __launch_bounds__(GB_THREADS, 1)
+// special functions, four tokens in flight: with THREADS = 512 instead of 256 17.6 -> 11.4 us there and 28.2 -> 15.9 at 16384 tokens; 1024
+// threads leave 64 registers, which spill with four in flight: 9.7 and 13.7 with two.  Up to 512 tokens the threads of 256 have one token
+// each and 512 would only lengthen the sum over threads: both directions together 5.4 us against 5.8 at 128 and 301 tokens, 5.9 and 5.9 at 600.
+constexpr int GB_CTAS = 8, GB_HEADS = 4;
+inline bool gates_bwd_narrow(size_t tokens) { return tokens <= (size_t)GB_CTAS * (256 / GB_HEADS); }
+template <int THREADS>
+__global__ void __cluster_dims__(GB_CTAS, 1, 1) __launch_bounds__(THREADS, 1)
     gates_bwd_kernel(const void* a_, const void* b_, int dt, const float* A_log, const float* dt_bias, const float* dg, const float* dbeta,
                      size_t tokens, int Hv, void* da, void* db, float* dA_log, float* d_dt_bias) {
-  __shared__ float red[2][GB_THREADS], sums[2][GB_HEADS];
+  __shared__ float red[2][THREADS], sums[2][GB_HEADS];
   const int rank = blockIdx.x % GB_CTAS, tid = threadIdx.x, hl = tid % GB_HEADS, h = blockIdx.x / GB_CTAS * GB_HEADS + hl;
   float sA = 0.f, sB = 0.f;
   if (h < Hv) {
     const float Ae = -expf(A_log[h]), bias = dt_bias[h];
 #pragma unroll 4
-    for (size_t t = rank * (GB_THREADS / GB_HEADS) + tid / GB_HEADS; t < tokens; t += GB_CTAS * (GB_THREADS / GB_HEADS)) {
+    for (size_t t = rank * (THREADS / GB_HEADS) + tid / GB_HEADS; t < tokens; t += GB_CTAS * (THREADS / GB_HEADS)) {
       const size_t e = t * Hv + h;
       const float x = ldf_ro(a_, e, dt) + bias, braw = ldf_ro(b_, e, dt), d = __ldg(dg + e), dbe = __ldg(dbeta + e);
       const float sp = softplus(x), sg = 1.f / (1.f + expf(-x));
@@ -521,7 +524,7 @@ __global__ void __cluster_dims__(GB_CTAS, 1, 1) __launch_bounds__(GB_THREADS, 1)
   red[0][tid] = sA;
   red[1][tid] = sB;
   __syncthreads();
-  for (int o = GB_THREADS / 2; o >= GB_HEADS; o >>= 1) {
+  for (int o = THREADS / 2; o >= GB_HEADS; o >>= 1) {
     if (tid < o) { red[0][tid] += red[0][tid + o]; red[1][tid] += red[1][tid + o]; }
     __syncthreads();
   }
@@ -801,8 +804,11 @@ int dn_gdn_gates_bwd(const void* a, const void* b, const float* A_log, const flo
   if (!a || !b || !A_log || !dt_bias || !dg || !dbeta || !da || !db || !dA_log || !d_dt_bias) return DN_ERR_NULL_POINTER;
   if (B < 1 || L < 1 || Hv < 1) return DN_ERR_BAD_SHAPE;
   if (dtype != DN_F32 && dtype != DN_BF16) return DN_ERR_BAD_DTYPE;
-  gates_bwd_kernel<<<(Hv + GB_HEADS - 1) / GB_HEADS * GB_CTAS, GB_THREADS, 0, (cudaStream_t)stream>>>(a, b, dtype, A_log, dt_bias, dg, dbeta, (size_t)B * L, Hv, da, db,
-                                                         dA_log, d_dt_bias);
+  const unsigned grid = (Hv + GB_HEADS - 1) / GB_HEADS * GB_CTAS;
+  const size_t tokens = (size_t)B * L;
+  auto go = [&](auto kernel, int threads) { kernel<<<grid, threads, 0, (cudaStream_t)stream>>>(a, b, dtype, A_log, dt_bias, dg, dbeta, tokens, Hv, da, db, dA_log, d_dt_bias); };
+  if (gates_bwd_narrow(tokens)) go(gates_bwd_kernel<256>, 256);
+  else go(gates_bwd_kernel<512>, 512);
   return launch_status();
 }
 

@@ -252,6 +252,26 @@ def test_gate_gradients(dn, B, L, Hv):
         assert O.rel_l2(x.cpu(), y) < 4e-5
 
 
+# ---- either side of the line between the two CTA widths, one token a thread and several rounds of four and a remainder, against 64 bits.  A head's sum
+# adds at most 6 tokens a thread, 7 levels of threads and 8 CTAs, and its terms have either sign, so that partial sums are as large as the
+# whole: 21 roundings of 2^-24, and 2 for the exponentials of each term, 1.4e-6 if all went one way; asserted at 4e-6.  Elements are rounded to their type.
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,L,Hv", [(1, 512, 5), (1, 513, 5), (2, 2600, 5)])
+def test_gate_gradients_of_many_tokens(dn, B, L, Hv, dtype):
+    gen = torch.Generator().manual_seed(72)
+    rn = lambda *s: torch.randn(*s, generator=gen)
+    ins = [rn(B, L, Hv).to(dtype), rn(B, L, Hv).to(dtype), rn(Hv), rn(Hv)]
+    cot = [rn(B, L, Hv), rn(B, L, Hv)]
+    ref_in = [t.double().requires_grad_() for t in ins]
+    a, b, A_log, dt = ref_in
+    r = torch.autograd.grad((-A_log.exp() * torch.nn.functional.softplus(a + dt), torch.sigmoid(b)), ref_in, [c.double() for c in cot])
+    dev = [t.cuda().requires_grad_() for t in ins]
+    s = torch.autograd.grad(dn.gdn_gates(*dev), dev, [c.cuda() for c in cot])
+    elements = 4e-6 if dtype == torch.float32 else 2.0 ** -8
+    for x, y, tol in zip(s, r, (elements, elements, 4e-6, 4e-6)):
+        assert O.rel_l2(x.cpu().double(), y) < tol
+
+
 # ---- the operators' native host path and the general one launch the same kernels
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_host_paths_agree(dn, dtype):
