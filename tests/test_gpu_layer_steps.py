@@ -181,3 +181,37 @@ def test_producer_batches(dn, W, B, L, heads):
     g_dev = torch.autograd.grad((got * dy).sum(), dev)
     for a, r in zip((got,) + g_dev, (ref,) + g_ref):
         assert O.rel_l2(a.detach().double(), r.detach()) < 1.1e-5
+
+
+@pytest.mark.parametrize("W,with_bias,with_seg", [(4, False, True), (4, True, False), (3, True, True), (2, False, True)])
+@pytest.mark.parametrize("B,L,heads", [(2, 66, 1), (2, 517, 1), (60, 517, 4)])
+@pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 3e-3), (torch.float32, 1.1e-5)])
+def test_producer_runs(dn, dtype, tol, B, L, heads, W, with_bias, with_seg):
+    """The kernels of both run lengths in both types against 64 bits, with a boundary at each place of a batch of four rows and around a long
+    run's start.  bf16: each result is rounded once, 2^-9 at most, and tanh.approx adds 2^-11 of x / 2; fp32 as in test_producer_batches."""
+    from deltanet_b200 import _lib
+    Hk, Hv, K, V = heads, 2 * heads, 64, 64
+    D = 2 * Hk * K + Hv * V
+    longest = B == 60                                     # runs of 256 tokens backward, by the scratch; of 64 forward, since 60 x 17 CTAs
+    tiles = B * (-(-L // 256))                            #   of half that length are more than one per SM
+    assert (_lib.lib().dn_gdn_producer_scratch_bytes(B, L, D, W) == tiles * D * (W + 1) * 4) == longest
+    gen = torch.Generator().manual_seed(2000 * W + L)
+    seg = torch.zeros(B, L, dtype=torch.int32, device="cuda")
+    for i, t in enumerate((8, 21, 34, 47, 48, 61, 256, 261)):
+        seg[0, t:] = i + 1
+        seg[-1, t + 1:] = i + 1
+    if not with_seg: seg.zero_()
+    mixed, dy = torch.randn(B, L, D, generator=gen).to(dtype).cuda(), torch.randn(B, L, D, generator=gen).to(dtype).cuda()
+    w, bias = (torch.randn(D, 1, W, generator=gen) * 0.5).cuda(), (torch.randn(D, generator=gen) * 0.1).cuda()
+    leaves = [mixed, w] + ([bias] if with_bias else [])
+    ref_in = [t.double().requires_grad_() for t in leaves]
+    xp, ids = F.pad(ref_in[0], (0, 0, W - 1, 0)), F.pad(seg, (W - 1, 0), value=-1)
+    pre = sum(xp[:, j:j + L] * ref_in[1][:, 0, j] * (ids[:, j:j + L] == seg)[..., None] for j in range(W))
+    ref = F.silu(pre + ref_in[2] if with_bias else pre)
+    g_ref = torch.autograd.grad(ref, ref_in, dy.double())
+    dev = [t.requires_grad_() for t in leaves]
+    parts = dn.gdn_qkv_producer(*dev, num_k_heads=Hk, num_v_heads=Hv, head_k_dim=K, head_v_dim=V, segment_ids=seg if with_seg else None)
+    got = torch.cat([t.reshape(B, L, -1) for t in parts], -1)
+    g_dev = torch.autograd.grad(got, dev, dy)
+    for a, r in zip((got,) + g_dev, (ref,) + g_ref):
+        assert O.rel_l2(a.detach().double(), r.detach()) < tol
