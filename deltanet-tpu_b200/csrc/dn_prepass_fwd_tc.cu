@@ -132,7 +132,7 @@ __device__ __forceinline__ void prefetch_kq(const PrepassFwdArgs& a, int e_item)
 // operands (the images of X and T are free then).  ONE_ROW: a thread takes four pieces of one row of v and w instead of two pieces of two
 // rows.  That is twice the lookups, but one address: with write gates per column or of a type known at run time, whose rows a thread
 // addresses as well, the other mapping spilled up to 290 bytes more a thread (64 registers).  Ten launches of 256 columns, L = 20011: 798 -> 769 us;
-// fused prologue, L = 4000, 32 heads: 222 -> 204; 64-wide heads, 16 of them: 177 -> 162.
+// fused prologue, L = 4000, 32 heads: 222 -> 204; 64-wide heads, 16 of them: 177 -> 162.  The instances with two rows have bf16 v only.
 template <int VW, bool ONE_ROW, class OTHERS, class AHEAD>
 __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm, const PrepassFwdArgs& a, int h, int b, int t0,
                                                      size_t ibase, int qdt, int gdt, int wC, bool fuse, OTHERS others, AHEAD ahead) {
@@ -169,8 +169,7 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
         const int col0 = half * 128 + 8 * piece_of_it(it), cc = col0 < vr ? col0 : 0;
         const size_t tok = row_at(it);
         if (wC == 1) w1[it] = ldbits_ro(a.w, tok * g.wH + g.w_of(h * g.G + (cc >> vsh)), gdt);
-        if (qdt == DN_BF16)
-          vraw[it] = col0 < vr ? __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.v) + tok * g.Hv * g.V + (size_t)h * vr + col0)) : make_uint4(0, 0, 0, 0);
+        vraw[it] = col0 < vr ? __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.v) + tok * g.Hv * g.V + (size_t)h * vr + col0)) : make_uint4(0, 0, 0, 0);
       }
     }
   };
@@ -191,9 +190,8 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
       } else {
         load8(a.w, (tok * g.wH + g.w_of(h * g.G + (col0 >> vsh))) * wC + cv, gdt, ww);
       }
-      if (qdt == DN_BF16) umma::unpack8(vraw[it], vv);
-      else if (ONE_ROW) { const Raw8 r = ldraw(vrow, half * 16 + p, qdt); cvraw(r, qdt, vv); }
-      else load8(a.v, tok * g.Hv * g.V + (size_t)h * vr + col0, qdt, vv);
+      if (!ONE_ROW || qdt == DN_BF16) umma::unpack8(vraw[it], vv);
+      else { const Raw8 r = ldraw(vrow, half * 16 + p, qdt); cvraw(r, qdt, vv); }
       const bool live = ONE_ROW ? live0 : t0 + x < g.L;
 #pragma unroll
       for (int i = 0; i < 8; ++i) vv[i] = live ? (fuse ? sigmoid_fast(ww[i]) : ww[i]) * vv[i] : 0.f;
