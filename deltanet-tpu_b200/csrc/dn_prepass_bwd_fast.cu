@@ -3,8 +3,15 @@
 // 750-762) and of the fused prologue (558-575).  Tiles whose channel-wise decay is strong (marked by the forward
 // prepass in the unused half of T's slot) are left to dn_prepass_bwd_tc.cu, launched behind this kernel.
 //
+// With W = T X, U = T Y, V_new = U - W S, and dV the cotangent of V_new:
+//     dY = T^T dV,   dX = T^T dW = -T^T dV S^T = -dY S^T,   dA = -(dX W^T + dY U^T) = -dY (U - W S)^T = -dY V_new^T,   dM = dO V_new^T
+// (dA, dM masked): dW is not needed, nor W and U beyond V_new, and dM, dA, dX come from one batch of products.  A tile is bound by its
+// chain of products and drains; through dW, with both terms of dA, the value width took five rounds of them, now three: 2 x 4001 tokens
+// of 16 x 32 heads, scalar gates, 433 -> 390 us; 4 x 2048 tokens of 16 heads of 64 266 -> 227; 6001 tokens of 12 x 24 heads, 256 columns, 294 -> 276;
+// 131072 tokens of 32 heads, KDA, 8.40 -> 8.12 ms.
+//
 // With f_i = e^{Lam_i - mid} (mid: the document's midpoint; f = 1 and a decay f_ij applied per entry when the decay is one
-// scalar per token), dA = -(dX W^T + dY U^T), dM = dO V_new^T (masked):
+// scalar per token):
 //     T1 = dA (k / f)   + [first doc] e^{Lam} / f  dX         d beta = f T1
 //     T2 = dM (k / f)   + [first doc] e^{Lam} / f  dqe        d q    = f T2   (+ dM_ii k_i)
 //     T3 = dA^T (beta f) + dM^T (q f) + [last doc] e^{Lam_end - Lam} f  dke       d k    = T3 / f (+ dM_ii q_i + d beta b)
@@ -296,7 +303,7 @@ struct Piece {                                          // eight elements as loa
 // dv = dY w_act, dw = dY v (+ sigmoid adjoint; summed over a value head's columns when w is one scalar per head, SW) of 128
 // columns, dY from its image.  Bound by the latency of the rows of v and w (2.2 to 3.2 k cycles with every SM here at once), so
 // all of them are requested together; one function per type, because only code that runs takes instruction cache.
-// low (LOW): the second part of dY, an image in global memory.
+// low: the second part of dY, a padded image in shared memory (LOW = 1) or one in the CTA's scratch (LOW = 2).
 template <bool QBF, bool GBF, bool SW>
 struct VRows {
   Piece<QBF> v[4];
@@ -315,9 +322,9 @@ struct VRows {
     }
   }
 };
-template <bool QBF, bool GBF, bool SW, bool LOW>
+template <bool QBF, bool GBF, bool SW, int LOW>
 __device__ __forceinline__ void v_body(const VRows<QBF, GBF, SW>& in, const PrepassBwdArgs& a, const uint4* img, int half, int h, size_t tok0, int rows, bool fuse,
-                                       const float4* low) {
+                                       const void* low) {
   const Geo& g = a.g;
   const int rx = threadIdx.x >> 2, rp = threadIdx.x & 3, vr = g.G * g.V, vsh = g.V == 128 ? 7 : 6;
   const bool live = rx < rows;
@@ -337,7 +344,7 @@ __device__ __forceinline__ void v_body(const VRows<QBF, GBF, SW>& in, const Prep
     umma::unpack8(img[p * PP + rx], dy);
     if (LOW) {
       float lo[8];
-      umma::unpack8(keep_piece(low + p * 128 + rx), lo);
+      umma::unpack8(LOW == 1 ? reinterpret_cast<const uint4*>(low)[p * PP + rx] : keep_piece(reinterpret_cast<const float4*>(low) + p * 128 + rx), lo);
 #pragma unroll
       for (int i = 0; i < 8; ++i) dy[i] += lo[i];
     }
@@ -361,8 +368,8 @@ __device__ __forceinline__ void v_body(const VRows<QBF, GBF, SW>& in, const Prep
     }
   }
 }
-template <bool QBF, bool GBF, bool SW, bool LOW>
-__device__ __noinline__ void v_phase(const PrepassBwdArgs& a, const uint4* img, int half, int h, size_t tok0, int rows, bool fuse, const float4* low) {
+template <bool QBF, bool GBF, bool SW, int LOW>
+__device__ __noinline__ void v_phase(const PrepassBwdArgs& a, const uint4* img, int half, int h, size_t tok0, int rows, bool fuse, const void* low) {
   VRows<QBF, GBF, SW> in;
   in.request(a, half, h, tok0, rows);
   v_body<QBF, GBF, SW, LOW>(in, a, img, half, h, tok0, rows, fuse, low);
@@ -435,10 +442,11 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     return (size_t)(b * g.H + h) * g.NC + c;
   };
   const __nv_bfloat16* states = states_img(g, a.res.states);
-  auto load_first = [&](size_t ib, int who) {           // what the first product and its drain take
-    sl.load(0, reinterpret_cast<const __nv_bfloat16*>(a.res.W) + ib * C * K, who);
-    sl.load(1, states + ib * K * VW, who);
-    sl.load(2, reinterpret_cast<const __nv_bfloat16*>(a.res.U) + ib * C * VW, who);
+  auto load_first = [&](size_t ib, int who) {           // what the first products take
+    const __nv_bfloat16* dVt = reinterpret_cast<const __nv_bfloat16*>(a.dV) + ib * C * VW;
+    sl.load(0, reinterpret_cast<const __nv_bfloat16*>(a.res.T + ib * C * C), who);
+    sl.load(1, dVt, who);
+    sl.load(2, NH == 1 ? states + ib * K * VW : dVt + C * 128, who);
   };
   bool loaded = false, staged_dO = false;               // load_first, stage_dO have been done during the tile before
   for (int e_item = blockIdx.x, hd = 0; e_item < units; (hd = hd + 1 < D ? hd + 1 : 0) == 0 ? e_item += gridDim.x : 0) {
@@ -455,8 +463,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     const __nv_bfloat16* Ug = reinterpret_cast<const __nv_bfloat16*>(a.res.U) + ibase * C * VW;
     const __nv_bfloat16* Sg = states + ibase * K * VW;
     const __nv_bfloat16* dHg = reinterpret_cast<const __nv_bfloat16*>(a.dH) + ibase * K * VW;
-    const __nv_bfloat16* dVg = reinterpret_cast<const __nv_bfloat16*>(a.dV) + ibase * C * VW;
-    const __nv_bfloat16* Tg = reinterpret_cast<const __nv_bfloat16*>(a.res.T + ibase * C * C);
     const size_t dO_off = tok0 * g.Hv * g.V + (size_t)h * vr, dO_pitch = (size_t)g.Hv * g.V;
     constexpr int HN = C * 128;                         // elements of one half's image
     // One half, bf16 v and one fp32 write gate per head: the rows are few enough to wait in registers, and are asked for two products
@@ -465,29 +471,57 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     const bool v_ahead = V_AHEAD && qdt == DN_BF16 && gdt == DN_F32 && wC == 1;
     VRows<true, false, true> vrows;
 
-    // ---- products over the value width
+    // ---- products over the value width.  A slot's operands, in order (one half / two halves of the value columns):
+    //        0: T                    / T, U0 -> V0           3: W, dH       / W, U1 -> V1
+    //        1: dV -> dY             / dV0 -> dY0, dO0, dH1  4: U -> V_new  / S0, dH0
+    //        2: S, then dA           / dV1 -> dY1, dO1, dA   5: dO, then dM / S1, then dM
+    sl.load(3, Wg);
     if (NH == 1) {
-      sl.load(3, dVg);
-      sl.load(4, dHg);
+      sl.load(4, Ug);
       if (!staged_dO) stage_dO(sl.at(5), a.d_out, dO_off, dO_pitch, rows, vr / 8, qdt);
     } else {
-      sl.load(3, Sg + HN);
-      sl.load(4, Ug + HN);
-      if (!staged_dO) stage_dO(sl.at(5), a.d_out, dO_off, dO_pitch, rows, 16, qdt);
+      sl.load(4, Sg);
+      sl.load(5, Sg + HN);
     }
     // V_new = U - W S, in the place of U; dM masked (scalar gates: decayed), its diagonal apart
     auto vnew = [&](int slot, uint32_t col) { drain_sub(cx.dead, tb + col, sl.at(slot), row, group); };
-    auto drain_dM = [&](int slot) {
-      drain_masked(cx.dead, tb + T_TMP, sl.at(slot), row, group, 1.f, seg_s, SC ? lam_s : nullptr, dmi_s);
+    auto drain_dM = [&] {
+      drain_masked(cx.dead, tb + T_K, sl.at(5), row, group, 1.f, seg_s, SC ? lam_s : nullptr, dmi_s);
       if constexpr (FINE)
-        drain_masked_low(cx.dead, tb + T_TMP, row, group, 1.f, seg_s, SC ? lam_s : nullptr, 0.f, [&](int p, uint4 v) { keep_piece(low_M + p * 128 + row, v); }, [](int, uint4) {});
+        drain_masked_low(cx.dead, tb + T_K, row, group, 1.f, seg_s, SC ? lam_s : nullptr, 0.f, [&](int p, uint4 v) { keep_piece(low_M + p * 128 + row, v); }, [](int, uint4) {});
     };
-    auto drain_neg = [&](int slot, uint32_t col) { drain_plain(cx.dead, tb + col, sl.at(slot), 128, row, group, -1.f); };
+    // dY as operand image; FINE: its second part too (trunc: dY has one part), where there is one half into slot 0, else into scratch
+    auto drain_dY = [&](int slot, uint32_t col, int half) {
+      drain_plain(cx.dead, tb + col, sl.at(slot), PP, row, group, 1.f);
+      if constexpr (FINE)
+        drain_low(cx.dead, tb + col, group, [&](int p, uint4 v) {
+          if (trunc) v = make_uint4(0, 0, 0, 0);
+          if (NH == 1) sl.at(0)[p * PP + row] = v;
+          else keep_piece(low_Y + half * 2048 + p * 128 + row, v);
+        });
+    };
+    auto vphase = [&](int slot, int half) {
+      auto go = [&](auto qbf, auto gbf, auto scalar) {
+        v_phase<decltype(qbf)::value, decltype(gbf)::value, decltype(scalar)::value, FINE ? NH : 0>(a, sl.at(slot), half, h, tok0, rows, fuse, NH == 1 ? (const void*)sl.at(0) : low_Y + half * 2048);
+      };
+      constexpr std::true_type yes{};
+      constexpr std::false_type no{};
+      if (qdt == DN_BF16) {
+        if (gdt == DN_BF16) { if (wC == 1) go(yes, yes, yes); else go(yes, yes, no); }
+        else { if (wC == 1) go(yes, no, yes); else go(yes, no, no); }
+      } else {
+        if (gdt == DN_BF16) { if (wC == 1) go(no, yes, yes); else go(no, yes, no); }
+        else { if (wC == 1) go(no, no, yes); else go(no, no, no); }
+      }
+    };
     sl.wait(0);
     sl.wait(1);
+    if (NH == 2) sl.wait(2);
     umma::tc_fence_after();
-    product<128, false, true>(cx, sl.at(0), 2048, sl.at(1), 2048, K, T_TMP, false);                        // W S
-    // (beside the first product, which warp 0 issues)
+    product<128, true, true>(cx, sl.at(0), 2048, sl.at(1), 2048, C, T_B, false);                           // dY = T^T dV
+    if (NH == 2) product<128, true, true>(cx, sl.at(0), 2048, sl.at(2), 2048, C, T_K, false);
+    if (NH == 2) commit(cx);
+    // (beside the first products, which warp 0 issues)
     if (const int x = tid - 256; x >= 0 && x < C) {
       bool is_new, all_same;
       chunk_flags(a.seg, g, b, c_idx, is_new, all_same);
@@ -529,190 +563,117 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         bet_s[x] = bv;
       }
     }
-    if (NH == 2) {
+    auto issue_WS = [&] {
       sl.wait(3);
-      product<128, false, true>(cx, sl.at(0), 2048, sl.at(3), 2048, K, T_B, false);
-    }
-    commit(cx);
-    sl.wait(2);
-    umma::cp_async_wait<0>();                           // dO
-    finish(cx);
+      sl.wait(NH == 1 ? 2 : 4);
+      product<128, false, true>(cx, sl.at(3), 2048, sl.at(NH == 1 ? 2 : 4), 2048, K, T_TMP, false);        // W S
+      if (NH == 2) {
+        sl.wait(5);
+        product<128, false, true>(cx, sl.at(3), 2048, sl.at(5), 2048, K, T_Q, false);
+      }
+      commit(cx);
+    };
     if constexpr (NH == 1) {
-      sl.load(0, Tg);
-      vnew(2, T_TMP);
-      sl.wait(3);
+      issue_WS();
+      umma::cp_async_wait<0>();                         // dO
+      umma::fence_async_smem();
+      finish(cx);
+      sl.load(3, dHg);
+      product<128, false, false>(cx, sl.at(5), PB, sl.at(2), 2048, 128, T_Q, false);                       // dqe = dO S^T, beside the drains
       sl.wait(4);
-      umma::pre_issue_sync();
-      product<128, false, false>(cx, sl.at(5), PB, sl.at(2), 2048, 128, T_TMP, false); // dM  = dO V_new^T
-      product<128, false, false>(cx, sl.at(5), PB, sl.at(1), 2048, 128, T_Q, false);   // dqe = dO S^T
-      commit(cx);
-      finish(cx);
-      product<128, false, false>(cx, sl.at(3), 2048, sl.at(1), 2048, 128, T_B, false);                     // -dW = dV S^T
-      product<128, false, false>(cx, sl.at(2), 2048, sl.at(4), 2048, 128, T_K, false);                     // dke = V_new dH^T
-      commit(cx);
-      drain_dM(5);
-      finish(cx);
-      sl.load(2, Wg);
-      sl.load(4, Ug);
-      drain_neg(1, T_B);                                // dW
-      sl.wait(0);
-      umma::pre_issue_sync();
-      product<128, true, true>(cx, sl.at(0), 2048, sl.at(1), 2048, C, T_B, false);                         // dX = T^T dW
-      product<128, true, true>(cx, sl.at(0), 2048, sl.at(3), 2048, C, T_TMP, false);                       // dY = T^T dV
-      commit(cx);
+      vnew(4, T_TMP);
+      drain_dY(1, T_B, 0);
       if (v_ahead) vrows.request(a, 0, h, tok0, rows);
-      finish(cx);
-    } else {
-      sl.load(0, dVg);
-      sl.wait(4);
-      vnew(2, T_TMP);
-      vnew(4, T_B);
       umma::pre_issue_sync();
-      product<128, false, false>(cx, sl.at(5), PB, sl.at(2), 2048, 128, T_TMP, false); // dM, dqe: first half
-      product<128, false, false>(cx, sl.at(5), PB, sl.at(1), 2048, 128, T_Q, false);
-      commit(cx);
-      finish(cx);
-      stage_dO(sl.at(5), a.d_out, dO_off + 128, dO_pitch, rows, vr / 8 - 16, qdt);
-      sl.wait(0);
-      product<128, false, false>(cx, sl.at(0), 2048, sl.at(1), 2048, 128, T_B, false);                     // -dW: first half
-      commit(cx);
-      umma::cp_async_wait<0>();
-      finish(cx);
-      sl.load(0, dVg + HN);
-      sl.load(1, dHg);
-      umma::pre_issue_sync();
-      product<128, false, false>(cx, sl.at(5), PB, sl.at(4), 2048, 128, T_TMP, true);  // second half
-      product<128, false, false>(cx, sl.at(5), PB, sl.at(3), 2048, 128, T_Q, true);
-      commit(cx);
-      finish(cx);
-      sl.wait(0);
-      sl.wait(1);
-      product<128, false, false>(cx, sl.at(0), 2048, sl.at(3), 2048, 128, T_B, true);
-      product<128, false, false>(cx, sl.at(2), 2048, sl.at(1), 2048, 128, T_K, false);                     // dke: first half
-      commit(cx);
-      drain_dM(5);
-      finish(cx);
-      sl.load(1, dHg + HN);                             // (slot 0 keeps the second half of dV)
-      sl.load(2, Tg);
-      drain_neg(3, T_B);                                // dW
-      sl.wait(1);
-      sl.wait(2);
-      umma::pre_issue_sync();
-      product<128, false, false>(cx, sl.at(4), 2048, sl.at(1), 2048, 128, T_K, true);                      // dke: second half
-      product<128, true, true>(cx, sl.at(2), 2048, sl.at(3), 2048, C, T_B, false);                         // dX = T^T dW
-      product<128, true, true>(cx, sl.at(2), 2048, sl.at(0), 2048, C, T_TMP, false);                       // dY: second half
-      commit(cx);
-      finish(cx);
-    }
-    auto drain_dX = [&](int slot) {                     // as operand image; the accumulator itself stays for T1
-      if (trunc) {
-#pragma unroll 1
-        for (int j = 0; j < 4; ++j) {
-          float v[8];
-          ld8(cx.dead, tb + T_B + 8 * j, v);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = bf16r(v[i]);
-          umma::tmem_st8(tb + T_B + 8 * j, v);
-        }
-        umma::tmem_wait_st();
+      product<128, false, false>(cx, sl.at(5), PB, sl.at(4), 2048, 128, T_K, false);                       // dM = dO V_new^T
+      product<128, false, false>(cx, sl.at(1), PB, sl.at(4), 2048, 128, T_TMP, false);                     // -dA = dY V_new^T
+      product<128, false, false>(cx, sl.at(1), PB, sl.at(2), 2048, 128, T_B, false);                       // -dX = dY S^T
+      if constexpr (FINE) {
+        product<128, false, false>(cx, sl.at(0), PB, sl.at(4), 2048, 128, T_TMP, true);
+        product<128, false, false>(cx, sl.at(0), PB, sl.at(2), 2048, 128, T_B, true);
       }
-      drain_plain(cx.dead, tb + T_B, sl.at(slot), 128, row, group, 1.f);
-    };
-    auto drain_dY = [&](int slot, int half) {
-      drain_plain(cx.dead, tb + T_TMP, sl.at(slot), PP, row, group, 1.f);
-      if constexpr (FINE)                               // (trunc: dY has one part)
-        drain_low(cx.dead, tb + T_TMP, group, [&](int p, uint4 v) { keep_piece(low_Y + half * 2048 + p * 128 + row, trunc ? make_uint4(0, 0, 0, 0) : v); });
-    };
-    // (the calls below put a barrier behind these; a thread reads back what it wrote)
-    auto low_dX = [&](int slot) { drain_low(cx.dead, tb + T_B, group, [&](int p, uint4 v) { sl.at(slot)[p * 128 + row] = v; }); };
-    auto low_dY = [&](int slot, int half) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) sl.at(slot)[(4 * group + j) * 128 + row] = keep_piece(low_Y + half * 2048 + (4 * group + j) * 128 + row);
-    };
-    auto vphase = [&](int slot, int half) {
-      auto go = [&](auto qbf, auto gbf, auto scalar) {
-        v_phase<decltype(qbf)::value, decltype(gbf)::value, decltype(scalar)::value, FINE>(a, sl.at(slot), half, h, tok0, rows, fuse, low_Y + half * 2048);
-      };
-      constexpr std::true_type yes{};
-      constexpr std::false_type no{};
-      if (qdt == DN_BF16) {
-        if (gdt == DN_BF16) { if (wC == 1) go(yes, yes, yes); else go(yes, yes, no); }
-        else { if (wC == 1) go(yes, no, yes); else go(yes, no, no); }
-      } else {
-        if (gdt == DN_BF16) { if (wC == 1) go(no, yes, yes); else go(no, yes, no); }
-        else { if (wC == 1) go(no, no, yes); else go(no, no, no); }
-      }
-    };
-    if constexpr (NH == 1) {
-      drain_dX(0);
-      drain_dY(1, 0);
-      if constexpr (FINE) low_dY(3, 0);
-      sl.wait(2);
-      sl.wait(4);
-      umma::pre_issue_sync();
-      product<128, false, false>(cx, sl.at(0), 2048, sl.at(2), 2048, 128, T_TMP, false);                   // -dA = dX W^T + dY U^T
-      product<128, false, false>(cx, sl.at(1), PB, sl.at(4), 2048, 128, T_TMP, true);
-      if constexpr (FINE) product<128, false, false>(cx, sl.at(3), 2048, sl.at(4), 2048, 128, T_TMP, true);
       commit(cx);
-      if (v_ahead) v_body<true, false, true, FINE>(vrows, a, sl.at(1), 0, h, tok0, rows, fuse, low_Y);
+      if (v_ahead) v_body<true, false, true, FINE ? NH : 0>(vrows, a, sl.at(1), 0, h, tok0, rows, fuse, sl.at(0));
       else vphase(1, 0);
       finish(cx);
-      if constexpr (FINE) {
-        low_dX(0);
-        umma::pre_issue_sync();
-        product<128, false, false>(cx, sl.at(0), 2048, sl.at(2), 2048, 128, T_TMP, true);
-        commit(cx);
-        finish(cx);
-      }
     } else {
-      sl.load(0, dVg);
-      sl.load(1, Wg);
-      drain_dX(3);
-      drain_dY(4, 1);
-      sl.wait(0);
-      umma::pre_issue_sync();
-      product<128, true, true>(cx, sl.at(2), 2048, sl.at(0), 2048, C, T_TMP, false);                       // dY: first half
-      commit(cx);
       finish(cx);
       sl.load(0, Ug);
-      drain_dY(2, 0);
+      issue_WS();                                       // beside the drains
+      drain_dY(1, T_B, 0);
+      drain_dY(2, T_K, 1);
+      finish(cx);
+      sl.load(3, Ug + HN);
       sl.wait(0);
-      sl.wait(1);
+      vnew(0, T_TMP);
+      sl.wait(3);
+      vnew(3, T_Q);
       umma::pre_issue_sync();
-      product<128, false, false>(cx, sl.at(3), 2048, sl.at(1), 2048, 128, T_TMP, false);                   // -dA = dX W^T + dY U^T
-      product<128, false, false>(cx, sl.at(2), PB, sl.at(0), 2048, 128, T_TMP, true);
+      product<128, false, false>(cx, sl.at(1), PB, sl.at(4), 2048, 128, T_B, false);                       // -dX = dY S^T
+      product<128, false, false>(cx, sl.at(2), PB, sl.at(5), 2048, 128, T_B, true);
+      product<128, false, false>(cx, sl.at(1), PB, sl.at(0), 2048, 128, T_TMP, false);                     // -dA = dY V_new^T
+      product<128, false, false>(cx, sl.at(2), PB, sl.at(3), 2048, 128, T_TMP, true);
+      commit(cx);
+      vphase(1, 0);
+      finish(cx);
+      if constexpr (!FINE) stage_dO(sl.at(1), a.d_out, dO_off, dO_pitch, rows, 16, qdt);
+      vphase(2, 1);
+      if constexpr (FINE) {                             // second parts of dY
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {                   // (a thread reads back what it wrote)
+          const int p = 4 * group + j;
+          sl.at(1)[p * PP + row] = keep_piece(low_Y + p * 128 + row);
+          sl.at(2)[p * PP + row] = keep_piece(low_Y + 2048 + p * 128 + row);
+        }
+        umma::pre_issue_sync();
+        product<128, false, false>(cx, sl.at(1), PB, sl.at(4), 2048, 128, T_B, true);
+        product<128, false, false>(cx, sl.at(2), PB, sl.at(5), 2048, 128, T_B, true);
+        product<128, false, false>(cx, sl.at(1), PB, sl.at(0), 2048, 128, T_TMP, true);
+        product<128, false, false>(cx, sl.at(2), PB, sl.at(3), 2048, 128, T_TMP, true);
+        commit(cx);
+        finish(cx);
+        stage_dO(sl.at(1), a.d_out, dO_off, dO_pitch, rows, 16, qdt);
+      }
+      umma::cp_async_wait<0>();
+      umma::pre_issue_sync();                           // (every thread is done with dY1)
+      product<128, false, false>(cx, sl.at(1), PB, sl.at(0), 2048, 128, T_K, false);                       // dM = dO V_new^T
+      product<128, false, false>(cx, sl.at(1), PB, sl.at(4), 2048, 128, T_Q, false);                       // dqe = dO S^T
+      commit(cx);
+      stage_dO(sl.at(2), a.d_out, dO_off + 128, dO_pitch, rows, vr / 8 - 16, qdt);
+      finish(cx);
+      sl.load(1, dHg + HN);
+      sl.load(4, dHg);
+      umma::cp_async_wait<0>();
+      umma::pre_issue_sync();
+      product<128, false, false>(cx, sl.at(2), PB, sl.at(3), 2048, 128, T_K, true);
+      product<128, false, false>(cx, sl.at(2), PB, sl.at(5), 2048, 128, T_Q, true);
       commit(cx);
       finish(cx);
-      if constexpr (FINE) {
-        low_dX(3);
-        umma::pre_issue_sync();
-        product<128, false, false>(cx, sl.at(3), 2048, sl.at(1), 2048, 128, T_TMP, true);
-        commit(cx);
-        finish(cx);
-        low_dY(1, 0);
-        umma::pre_issue_sync();
-        product<128, false, false>(cx, sl.at(1), 2048, sl.at(0), 2048, 128, T_TMP, true);
-        commit(cx);
-        finish(cx);
-      }
-      sl.load(0, Ug + HN);
-      vphase(2, 0);
-      sl.wait(0);
-      product<128, false, false>(cx, sl.at(4), PB, sl.at(0), 2048, 128, T_TMP, true);
-      commit(cx);
-      vphase(4, 1);
-      finish(cx);
-      if constexpr (FINE) {
-        low_dY(1, 1);
-        umma::pre_issue_sync();
-        product<128, false, false>(cx, sl.at(1), 2048, sl.at(0), 2048, 128, T_TMP, true);
-        commit(cx);
-        finish(cx);
-      }
     }
-    // ---- dA (dM is in slot 5); everything else is free
-    uint4 *const dAi = sl.region(4), *const dMi = sl.at(5), *const dAb = SC ? sl.region(2) : nullptr;
-    if constexpr (!SC) drain_masked(cx.dead, tb + T_TMP, dAi, row, group, -1.f, seg_s, nullptr, nullptr);
+    // ---- dM and dA as operand images; dke, whose accumulator held dM, beside what follows
+    uint4 *const dAi = sl.at(2), *const dMi = sl.at(5), *const dAb = SC ? sl.region(2) : nullptr;
+    auto issue_dke = [&] {
+      if (NH == 1) {
+        sl.wait(3);
+      } else {
+        sl.wait(1);
+        sl.wait(4);
+      }
+      umma::pre_issue_sync();
+      if (NH == 1) {
+        product<128, false, false>(cx, sl.at(4), 2048, sl.at(3), 2048, 128, T_K, false);                   // dke = V_new dH^T
+      } else {
+        product<128, false, false>(cx, sl.at(0), 2048, sl.at(4), 2048, 128, T_K, false);
+        product<128, false, false>(cx, sl.at(3), 2048, sl.at(1), 2048, 128, T_K, true);
+      }
+      commit(cx);
+    };
+    if constexpr (!SC) {
+      drain_dM();
+      drain_masked(cx.dead, tb + T_TMP, dAi, row, group, -1.f, seg_s, nullptr, nullptr);
+      issue_dke();
+    }
 
     // ---- key side: rows of q, k, b in the row mapping
     const bool live = rx < rows;
@@ -788,6 +749,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       const uint32_t cuts = __ballot_sync(0xffffffffu, x0 + lane > 0 && seg_s[x0 + lane] != seg_s[x0 + lane - (x0 + lane > 0)]);
       float run = 0.f;
       float* lp = LAM + x0 * LPF + c;
+      finish(cx);                                       // dke: its operands lie where Lambda goes
 #pragma unroll 1
       for (int j = 0; j < 32 / GB; ++j) {
         float v[GB];
@@ -831,7 +793,11 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         kraw4[it] = ld16_now(krow + 16 * pc);
         qraw4[it] = ld16_now(qrow + 16 * pc);
       }
+      drain_dM();
+      issue_dke();
+      if (NH == 2) finish(cx);                          // (an operand of dke lies where the rows of dA times beta go)
       drain_masked(cx.dead, tb + T_TMP, dAi, row, group, -1.f, seg_s, lam_s, nullptr, dAb, bet_s[row]);
+      if (NH == 1) finish(cx);
 #pragma unroll
       for (int it = 0; it < 4; ++it) {
         const int p = it * 4 + rp;
@@ -870,7 +836,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         for (int i = 0; i < 8; ++i) {
           const float e1 = SC ? el : (first ? EDGE[c0 + i] : 0.f);
           v[i] *= e1;
-          w[i] *= e1;
+          w[i] = (trunc ? bf16r(w[i]) : w[i]) * -e1;    // (the accumulator holds -dX)
           if (!SC) {
             kh[i] *= rkr;
             if (round_in) kh[i] = bf16r(kh[i]);
@@ -1017,11 +983,11 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
     // the next tile's dO, where dM was (the raw b, where there is one per channel, reaches there)
     const int ne = hd + 1 < D ? e_item : e_item + (int)gridDim.x, nhd = hd + 1 < D ? hd + 1 : 0;
     const bool more = ne < units && (SC || next_strong_s == 0);
-    staged_dO = more && bC == 1;
+    staged_dO = NH == 1 && more && bC == 1;
     if (staged_dO) {
       int nb, nh, nc;
       place(ne, nhd, nb, nh, nc);
-      stage_dO(sl.at(5), a.d_out, ((size_t)nb * g.L + nc * C) * g.Hv * g.V + (size_t)nh * vr, dO_pitch, g.L - nc * C < C ? g.L - nc * C : C, NH == 2 ? 16 : vr / 8, qdt);
+      stage_dO(sl.at(5), a.d_out, ((size_t)nb * g.L + nc * C) * g.Hv * g.V + (size_t)nh * vr, dO_pitch, g.L - nc * C < C ? g.L - nc * C : C, vr / 8, qdt);
     }
     // ---- combination, a row per lane, 32 channels per warp.  d q_n, d k_n and dLambda wait in the columns just read for the
     //      row sums of the l2norm adjoint.

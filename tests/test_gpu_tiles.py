@@ -133,12 +133,13 @@ def test_shared_key_heads(dn, B, L):
 # ---- a CTA's second and third tile: what a tile does for the next one (decay scanned, rows of q, k and dO and first operands copied ahead, or
 # not, where the next tile's decay is strong), against the same call row by row, where every CTA has one tile.  13 rows x 6 tiles x 8 heads are
 # 624 tiles for at most 296 CTAs forward and 148 backward (scalar gates: 312 pairs of heads), the last of a row partial.
-@pytest.mark.parametrize("form", ["gdn", "gdn_wide", "gdn_64", "kda", "kda_strong", "kda_fp32", "gdn2", "fused_bf16"])
+@pytest.mark.parametrize("form", ["gdn", "gdn_wide", "gdn_64", "kda", "kda_strong", "kda_fp32", "gdn2", "fused_bf16",
+                                  "gdn_64_wide", "gdn2_64_wide"])
 def test_tiles_after_the_first(dn, form):
-    B, L, H, K = 13, 700, 8, 64 if form == "gdn_64" else 128
+    B, L, H, K = 13, 700, 8, 64 if "_64" in form else 128
     gen = torch.Generator().manual_seed(57)
     rn = lambda *s: torch.randn(*s, generator=gen)
-    scalar, Hv = form.startswith("gdn") and form != "gdn2", 16 if form in ("gdn_wide", "gdn2") else H
+    scalar, Hv = form.startswith("gdn") and not form.startswith("gdn2"), 16 if form in ("gdn_wide", "gdn2") else 32 if form.endswith("64_wide") else H
     Hk = 4 if form in ("gdn", "gdn_64") else H
     g_heads = H
     kw = dict(precision="bf16", qk_l2norm=True, output_final_state=True, fuse_prologue=form == "fused_bf16")
@@ -147,8 +148,8 @@ def test_tiles_after_the_first(dn, form):
     g, b = -torch.exp(0.39 * rn(B, L, g_heads, *([] if scalar else [K])) - 1.0), torch.sigmoid(rn(B, L, g_heads))
     if form == "kda_strong": g[torch.rand(B, L // 100 + 1, generator=gen).repeat_interleave(100, 1)[:, :L] < 0.3] *= 12.0
     ins += [g, b, b]
-    if form in ("gdn2", "fused_bf16"): ins[3:] = [rn(B, L, H, K) - 1.0, rn(B, L, H, K), rn(B, L, Hv, K)]
-    if form == "gdn2": ins[3:] = [-torch.exp(0.39 * ins[3]), torch.sigmoid(ins[4]), torch.sigmoid(ins[5])]
+    if form in ("gdn2", "fused_bf16", "gdn2_64_wide"): ins[3:] = [rn(B, L, H, K) - 1.0, rn(B, L, H, K), rn(B, L, Hv, K)]
+    if form.startswith("gdn2"): ins[3:] = [-torch.exp(0.39 * ins[3]), torch.sigmoid(ins[4]), torch.sigmoid(ins[5])]
     if form == "fused_bf16": ins[3:] = [t.bfloat16() for t in ins[3:]]
     seg = (torch.rand(B, L, generator=gen) < 0.01).int().cumsum(1).int().cuda()
     cot, cot_s = rn(B, L, Hv, K).to(ins[2].dtype).cuda(), (rn(B, Hv, K, K) * 0.1).cuda()
