@@ -185,10 +185,35 @@ __device__ __forceinline__ float ldf_ro(const void* p, size_t i, int dt) {
   return dt == DN_BF16 ? __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(p) + i))
                        : __ldg(reinterpret_cast<const float*>(p) + i);
 }
-// The same in two steps, bits and value, where the type is known at run time only and several loads are to be in flight together: the
-// conversion of a bf16 element waits for its load, whichever type the call turns out to have.
+// The same in two steps, bits and value: the conversion waits for its load.  (With a type that is known at run time only the load waits
+// as well, at the join of the two paths, and so does a pair of predicated loads of one register: kernels that want several
+// in flight are instantiated by type.)
 __device__ __forceinline__ uint32_t ldbits_ro(const void* p, size_t i, int dt) {
   return dt == DN_BF16 ? (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(p) + i) : __ldg(reinterpret_cast<const uint32_t*>(p) + i);
+}
+// without a branch and zero where `on` is false
+__device__ __forceinline__ uint32_t ldbits_ro_or_zero(const void* p, size_t i, int dt, bool on) {
+  uint32_t u;
+  if (dt == DN_BF16)
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.b32 %0, 0;\n\t@q ld.global.nc.u16 %0, [%1];\n\t}"
+                 : "=r"(u) : "l"(reinterpret_cast<const unsigned short*>(p) + i), "r"((int)on));
+  else
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.b32 %0, 0;\n\t@q ld.global.nc.u32 %0, [%1];\n\t}"
+                 : "=r"(u) : "l"(reinterpret_cast<const uint32_t*>(p) + i), "r"((int)on));
+  return u;
+}
+// 16 bytes of an input tensor, issued where it stands (an ordinary load may be moved down to its use, past the branches between), or zeros
+__device__ __forceinline__ uint4 ld16_now(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 ld16_now_or_zero(const void* p, bool on) {
+  uint4 v;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
+               "@q ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];\n\t}"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "r"((int)on));
+  return v;
 }
 __device__ __forceinline__ float bits_value(uint32_t u, int dt) { return __uint_as_float(dt == DN_BF16 ? u << 16 : u); }
 __device__ __forceinline__ void stf(void* p, size_t i, float v, int dt) {

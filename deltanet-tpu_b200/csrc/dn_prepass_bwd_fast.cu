@@ -234,12 +234,6 @@ __device__ __forceinline__ void stage_dO(uint4* dst, const void* d_out, size_t o
   umma::cp_async_commit();
 }
 
-// 16 bytes of an input tensor, issued where it stands: an ordinary load may be moved down to its use, past the branches between
-__device__ __forceinline__ uint4 ld16_now(const void* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
-}
 // a piece of an image in the CTA's scratch
 __device__ __forceinline__ uint4 keep_piece(const float4* p) {
   const float4 t = umma::ld_keep4(p);
@@ -416,7 +410,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
 
   const bool l2 = g.flags & DN_QK_L2NORM, trunc = g.flags & DN_TRUNC_DT_BF16;
   const bool fuse = CF::fixed || SC ? false : (g.flags & DN_FUSE_PROLOGUE) != 0, guard = CF::fixed ? false : (g.flags & DN_STABILITY_GUARD) != 0;
-  const int qdt = SC ? DN_BF16 : (CF::fixed ? CF::qkv_dt : g.qkv_dt), gdt = CF::fixed ? DN_F32 : g.gate_dt;
+  const int qdt = SC ? DN_BF16 : (CF::typed ? CF::qkv_dt : g.qkv_dt), gdt = CF::typed ? CF::gate_dt : g.gate_dt;
   const bool round_in = !fuse && qdt == DN_BF16;
   const int kp = CF::fixed && !SC ? 16 : g.K / 8, gC = SC ? 1 : (CF::fixed ? K : g.gC), bC = SC ? 1 : (CF::fixed ? (CF::scalar_bw ? 1 : K) : g.bC);
   const int wC = CF::fixed && !SC ? (CF::scalar_bw ? 1 : g.V) : g.wC;
@@ -542,9 +536,9 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         const int sp = x ? seg_at(a.seg, b, t0 + x - 1, g.L) : sg;
         float gv = 0.f, bv = 0.f;
         if (x < rows) {
-          const uint32_t gu = ldbits_ro(a.gg, (tok0 + x) * g.gH + g.g_head(h), g.gate_dt), bu = ldbits_ro(a.b, (tok0 + x) * g.bH + g.b_head(h), g.gate_dt);
-          gv = bits_value(gu, g.gate_dt);
-          bv = bits_value(bu, g.gate_dt);
+          const uint32_t gu = ldbits_ro(a.gg, (tok0 + x) * g.gH + g.g_head(h), gdt), bu = ldbits_ro(a.b, (tok0 + x) * g.bH + g.b_head(h), gdt);
+          gv = bits_value(gu, gdt);
+          bv = bits_value(bu, gdt);
           gv = gv <= 0.f ? gv : 0.f;
           if (guard) { bv = fmaxf(bv, 0.f); gv = fminf(gv, -1e-6f); }
         }
@@ -738,7 +732,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       const uint32_t gpitch = (uint32_t)(g.gH * gC) * ges;
       const bool cin = gC == 1 || c < gC;
       const uint8_t* gp = reinterpret_cast<const uint8_t*>(a.gg) + (tok0 * g.gH + g.g_head(h)) * gC * ges + (gC == 1 || !cin ? 0 : c) * ges;
-      constexpr int GB = MODE == 2 ? 8 : 32;            // rows requested together (code size against latency)
+      constexpr int GB = CF::fixed ? 32 : 8;            // rows requested together (code size against latency)
       uint32_t nx[GB];
       auto load_g = [&](int j) {                        // (rows past the end: row 0, dropped below)
         const int x = x0 + GB * j;
@@ -1331,14 +1325,21 @@ int launch_prepass_bwd_fast(const PrepassBwdArgs& args, cudaStream_t st) {
   };
   auto pick = [&](auto vw) {
     constexpr int VW = decltype(vw)::value;
+    const int mode = typed_mode(g);
     if (prepass_bwd_scalar_route(g)) {
-      if (g.fine) go(prepass_bwd_fast_kernel<VW, 2, true, true>); else go(prepass_bwd_fast_kernel<VW, 2, true>);
+      // (two parts: 227 us by run-time types, 225 typed; one part, which loads two gates a row once, is slower typed: 385 -> 396 at 2 x 4096
+      // tokens of 16 x 32 heads)
+      if (!g.fine) go(prepass_bwd_fast_kernel<VW, 2, true>);
+      else if (mode == 5) go(prepass_bwd_fast_kernel<VW, 5, true, true>);
+      else go(prepass_bwd_fast_kernel<VW, 2, true, true>);
       return;
     }
-    switch (input_mode(g)) {
+    switch (mode) {
       case 0: go(prepass_bwd_fast_kernel<VW, 0, false>); break;
       case 1: go(prepass_bwd_fast_kernel<VW, 1, false>); break;
+      case 3: go(prepass_bwd_fast_kernel<VW, 3, false>); break;
       case 4: go(prepass_bwd_fast_kernel<VW, 4, false>); break;
+      case 5: if (g.fine) go(prepass_bwd_fast_kernel<VW, 5, false, true>); else go(prepass_bwd_fast_kernel<VW, 5, false>); break;
       default: if (g.fine) go(prepass_bwd_fast_kernel<VW, 2, false, true>); else go(prepass_bwd_fast_kernel<VW, 2, false>); break;
     }
   };

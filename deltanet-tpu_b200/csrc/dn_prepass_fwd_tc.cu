@@ -161,15 +161,15 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
       if (qdt == DN_BF16) {
 #pragma unroll
         for (int it = 0; it < 4; ++it)
-          vraw[it] = half * 128 + 32 * it < vr ? __ldg(reinterpret_cast<const uint4*>(vrow) + half * 16 + it * 4 + piece_of(tid)) : make_uint4(0, 0, 0, 0);
+          vraw[it] = ld16_now_or_zero(reinterpret_cast<const uint4*>(vrow) + half * 16 + it * 4 + piece_of(tid), half * 128 + 32 * it < vr);
       }
     } else {
 #pragma unroll
       for (int it = 0; it < 4; ++it) {
         const int col0 = half * 128 + 8 * piece_of_it(it), cc = col0 < vr ? col0 : 0;
         const size_t tok = row_at(it);
-        if (wC == 1) w1[it] = ldbits_ro(a.w, tok * g.wH + g.w_of(h * g.G + (cc >> vsh)), gdt);
-        vraw[it] = col0 < vr ? __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.v) + tok * g.Hv * g.V + (size_t)h * vr + col0)) : make_uint4(0, 0, 0, 0);
+        w1[it] = ldbits_ro_or_zero(a.w, tok * g.wH + g.w_of(h * g.G + (cc >> vsh)), gdt, wC == 1);
+        vraw[it] = ld16_now_or_zero(reinterpret_cast<const __nv_bfloat16*>(a.v) + tok * g.Hv * g.V + (size_t)h * vr + col0, col0 < vr);
       }
     }
   };
@@ -265,6 +265,7 @@ struct alignas(16) ScalarRows {
   float lam[C], bet[C];
   uint8_t ds[C];
 };
+template <int GDT>
 __device__ __forceinline__ void scan_scalar(const PrepassFwdArgs& a, int e_item, int t, ScalarRows& out, float* tot_s, int* rst_s) {
   const Geo& g = a.g;
   int b, h, c;
@@ -276,9 +277,9 @@ __device__ __forceinline__ void scan_scalar(const PrepassFwdArgs& a, int e_item,
   const int sg = seg_at(a.seg, b, t0 + t, g.L), sp = t ? seg_at(a.seg, b, t0 + t - 1, g.L) : sg;
   float gv = 0.f, bv = 0.f;
   if (t0 + t < g.L) {
-    const uint32_t gu = ldbits_ro(a.gg, tok * g.gH + g.g_head(h), g.gate_dt), bu = ldbits_ro(a.b, tok * g.bH + g.b_head(h), g.gate_dt);
-    gv = bits_value(gu, g.gate_dt);
-    bv = bits_value(bu, g.gate_dt);
+    const uint32_t gu = ldbits_ro(a.gg, tok * g.gH + g.g_head(h), GDT), bu = ldbits_ro(a.b, tok * g.bH + g.b_head(h), GDT);
+    gv = bits_value(gu, GDT);
+    bv = bits_value(bu, GDT);
     gv = gv <= 0.f ? gv : 0.f;
     if (guard) { bv = fmaxf(bv, 0.f); gv = fminf(gv, -1e-6f); }
   }
@@ -303,8 +304,9 @@ __device__ __forceinline__ void scan_scalar(const PrepassFwdArgs& a, int e_item,
 // q and k are read once, eight lanes a row; qe, ke and X come from the images of q_hat and k_hat, a row per lane, so that the
 // stores of a warp are 512 contiguous bytes.  What an item waits for is taken off its path: the next item's decay is scanned by warps
 // 8 to 11 beside the substitution (its loads come from HBM: 1 to 2 k cycles), its rows of k and q are asked into L2 there and into
-// shared memory beside the last drains.
-template <int VW>
+// shared memory beside the last drains.  GDT: the type of the gates (known at run time only, the four write gates a thread
+// loads for its rows waited for one another, 700 cycles each: 4 x 8192 tokens of 32 heads 692 -> 669 us, one tile 17.2 -> 16.0).
+template <int VW, int GDT>
 __global__ void __launch_bounds__(NT, 2) prepass_fwd_scalar_kernel(const __grid_constant__ PrepassFwdArgs a, int* err) {
   extern __shared__ __align__(128) uint8_t sm[];
   __shared__ uint64_t bar;
@@ -334,7 +336,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_scalar_kernel(const __grid_
     umma::cp_async_commit();
   };
   load_kq(blockIdx.x);
-  if (tid < C) scan_scalar(a, blockIdx.x, tid, rows_s[0], tot_s, rst_s);
+  if (tid < C) scan_scalar<GDT>(a, blockIdx.x, tid, rows_s[0], tot_s, rst_s);
 
   int set = 0;
   for (int e_item = blockIdx.x; e_item < a.items; e_item += gridDim.x, set ^= 1) {
@@ -437,12 +439,12 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_scalar_kernel(const __grid_
     }
     __syncthreads();
     const int next = e_item + gridDim.x;
-    inverse_and_products<VW, false>(cx, sm, a, h, b, t0, ibase, DN_BF16, g.gate_dt, g.wC, false, [&]() {
+    inverse_and_products<VW, false>(cx, sm, a, h, b, t0, ibase, DN_BF16, GDT, g.wC, false, [&]() {
       // (the requests: 779 -> 741 us at B=4 L=8192 Hv=32.  With decay per channel they cost more than they hide,
       // 761 -> 819 us at L=20011: that kernel reads q, k, b, g in groups and has other tiles to switch to.)
       if (warp < 8) prefetch_vw(a, h, b, t0);
       else if (warp >= 12) prefetch_kq(a, next);
-      else if (next < a.items) scan_scalar(a, next, tid - 256, rows_s[set ^ 1], tot_s, rst_s);
+      else if (next < a.items) scan_scalar<GDT>(a, next, tid - 256, rows_s[set ^ 1], tot_s, rst_s);
     }, [&]() { load_kq(next); });
   }
   teardown(tbase);
@@ -728,7 +730,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
   };
   const bool fuse = CF::fixed ? false : (g.flags & DN_FUSE_PROLOGUE) != 0, guard = CF::fixed ? false : (g.flags & DN_STABILITY_GUARD) != 0;
   const bool l2 = g.flags & DN_QK_L2NORM;
-  const int qdt = CF::fixed ? CF::qkv_dt : g.qkv_dt, gdt = CF::fixed ? DN_F32 : g.gate_dt;
+  const int qdt = CF::typed ? CF::qkv_dt : g.qkv_dt, gdt = CF::typed ? CF::gate_dt : g.gate_dt;
   const bool round_in = !fuse && qdt == DN_BF16;
   const int kp = CF::fixed ? 16 : g.K / 8, gC = CF::fixed ? K : g.gC, bC = CF::fixed ? (CF::scalar_bw ? 1 : K) : g.bC;
   const int wC = CF::fixed ? (CF::scalar_bw ? 1 : g.V) : g.wC;
@@ -1001,11 +1003,16 @@ int launch_prepass_fwd_tc(const Geo& g, const void* q, const void* k, const void
   };
   auto pick = [&](auto vw) {
     constexpr int VW = decltype(vw)::value;
-    if (scalar) { go(prepass_fwd_scalar_kernel<VW>); return; }
-    switch (input_mode(g)) {
+    if (scalar) {
+      if (g.gate_dt == DN_BF16) go(prepass_fwd_scalar_kernel<VW, DN_BF16>); else go(prepass_fwd_scalar_kernel<VW, DN_F32>);
+      return;
+    }
+    switch (typed_mode(g)) {
       case 0: go(prepass_fwd_channel_kernel<VW, 0>); break;
       case 1: go(prepass_fwd_channel_kernel<VW, 1>); break;
+      case 3: go(prepass_fwd_channel_kernel<VW, 3>); break;
       case 4: go(prepass_fwd_channel_kernel<VW, 4>); break;
+      case 5: if (g.fine) go(prepass_fwd_channel_kernel<VW, 5, true>); else go(prepass_fwd_channel_kernel<VW, 5>); break;
       default: if (g.fine) go(prepass_fwd_channel_kernel<VW, 2, true>); else go(prepass_fwd_channel_kernel<VW, 2>); break;
     }
   };

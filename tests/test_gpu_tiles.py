@@ -337,3 +337,26 @@ def test_narrow_heads_gate_forms(dn, gates, K, V, Hk, Hv):
     if gates == "fused_scalar": ins[3:] = [t[..., 0].contiguous() for t in ins[3:]]
     seg = docs(1, 200, 70, 130)
     compare(lambda t, i: dn.chunk_gdn2(*t, segment_ids=seg.cuda(), **kw), lambda t, i: O.chunk_gdn2(*t, segment_ids=seg, **kw), ins, tol=BF16_TOL)
+
+
+# ---- the same gate values in bf16 and in fp32: kernels instantiated by type and by what is known of the widths, the same results
+@pytest.mark.parametrize("form", ["fused", "guard", "scalar", "scalar_b"])
+@pytest.mark.parametrize("L,G", [(1, 1), (300, 2)])
+def test_gate_types_agree(dn, form, L, G):
+    gen = torch.Generator().manual_seed(71)
+    rn = lambda *s: torch.randn(*s, generator=gen)
+    H, K = 2, 128
+    kw = dict(precision="bf16", qk_l2norm=True, output_final_state=True, fuse_prologue=form == "fused", stability_guard=form == "guard")
+    ins = [t.bfloat16() for t in (rn(1, L, H, K), rn(1, L, H, K), rn(1, L, G * H, K))]
+    cols, b_cols = ([] if form == "scalar" else [K]), ([] if form.startswith("scalar") else [K])
+    gates = [rn(1, L, H, *cols) - 1.0, rn(1, L, H, *b_cols), rn(1, L, G * H, *b_cols)]
+    if form != "fused": gates = [-torch.exp(0.39 * gates[0]), torch.sigmoid(gates[1]), torch.sigmoid(gates[2])]
+    cot = rn(1, L, G * H, K).bfloat16().cuda()
+
+    def call(dtype):
+        leaves = [t.cuda().requires_grad_() for t in ins] + [t.bfloat16().to(dtype).cuda().requires_grad_() for t in gates]
+        o, s = dn.chunk_gdn2(*leaves, **kw)
+        return [o.detach(), s.detach()] + [t.bfloat16() for t in torch.autograd.grad(o, leaves, cot)]
+
+    for i, (x, y) in enumerate(zip(call(torch.bfloat16), call(torch.float32))):
+        assert torch.equal(x, y), (i, O.rel_l2(x.float(), y.float()))
