@@ -19,13 +19,13 @@ constexpr int LP = 132;                // row pitch (floats) of the shared-memor
 // the same with q/k/v in fp32; MODE 2: nothing (dtypes, gate widths and the prologue are run-time
 // properties, every load sits behind a branch and both activation paths are compiled in);
 // MODE 4: bf16 q/k/v, fp32 activated gates, the decay per channel and ONE erase / write gate value per head
-// (the KDA layout); MODE 3 and 5: MODE 2 with the types known, q/k/v in bf16 and the gates in bf16 (3) or fp32 (5).
+// (the KDA layout); MODE 3, 5, 6: MODE 2 with types known, q/k/v in bf16 and the gates in bf16 (3) or fp32 (5), q/k/v in fp32 (6).
 template <int MODE>
 struct InCfg {
-  static constexpr bool typed = MODE != 2;           // the types are known, ...
-  static constexpr bool fixed = typed && MODE != 3 && MODE != 5;      // ... and the widths and the activation
+  static constexpr bool fixed = MODE == 0 || MODE == 1 || MODE == 4;  // types, widths and the activation are known
+  static constexpr bool qkv_typed = MODE != 2, gate_typed = MODE != 2 && MODE != 6;
   static constexpr bool scalar_bw = MODE == 4;       // b and w are one scalar per (token, head)
-  static constexpr int qkv_dt = MODE == 1 ? DN_F32 : DN_BF16;
+  static constexpr int qkv_dt = MODE == 1 || MODE == 6 ? DN_F32 : DN_BF16;
   static constexpr int gate_dt = MODE == 3 ? DN_BF16 : DN_F32;
 };
 inline int input_mode(const Geo& g) {
@@ -34,14 +34,14 @@ inline int input_mode(const Geo& g) {
   if (g.gC == g.K && g.bC == 1 && g.wC == 1 && g.qkv_dt == DN_BF16) return 4;
   return 2;
 }
-// The same for kernels that have the typed instances as well (bf16 gates in two parts have none; fp32 q/k/v stay with mode 2).  With
+// The same for kernels that have the typed instances in MODE 2's place.  With
 // types known at run time each load ends in a branch whose paths join behind it, and waits there: rows asked for one after the other,
 // a latency each.  6001 tokens of 12 x 24 heads, fused prologue, bf16 gates: forward 159 -> 134 us, backward 276 -> 251; 4 x 2048 tokens of 16
-// heads of 64, gates per channel: 237 -> 210 and 381 -> 357.
+// heads of 64, gates per channel: 237 -> 209 and 381 -> 357; fp32 q/k/v, fused prologue: 126 -> 105 and 218 -> 202.
 inline int typed_mode(const Geo& g) {
   const int mode = input_mode(g);
-  if (mode != 2 || g.qkv_dt != DN_BF16) return mode;
-  return g.gate_dt == DN_F32 ? 5 : (g.fine ? 2 : 3);
+  if (mode != 2) return mode;
+  return g.qkv_dt != DN_BF16 ? 6 : g.gate_dt == DN_F32 ? 5 : 3;
 }
 
 // Where one (batch, exec head, chunk) reads its rows from.
@@ -81,8 +81,15 @@ struct Raw8 { uint4 a, b; };
 __device__ __forceinline__ Raw8 ldraw(const uint8_t* row, int p, int dt) {
   Raw8 r;
   r.b = make_uint4(0, 0, 0, 0);
-  if (dt == DN_BF16) r.a = __ldg(reinterpret_cast<const uint4*>(row) + p);
-  else { r.a = __ldg(reinterpret_cast<const uint4*>(row) + 2 * p); r.b = __ldg(reinterpret_cast<const uint4*>(row) + 2 * p + 1); }
+  if (dt == DN_BF16) r.a = ld16_now(reinterpret_cast<const uint4*>(row) + p);
+  else { r.a = ld16_now(reinterpret_cast<const uint4*>(row) + 2 * p); r.b = ld16_now(reinterpret_cast<const uint4*>(row) + 2 * p + 1); }
+  return r;
+}
+__device__ __forceinline__ Raw8 ldraw_or_zero(const uint8_t* row, int p, int dt, bool on) {
+  Raw8 r;
+  r.b = make_uint4(0, 0, 0, 0);
+  if (dt == DN_BF16) r.a = ld16_now_or_zero(reinterpret_cast<const uint4*>(row) + p, on);
+  else { r.a = ld16_now_or_zero(reinterpret_cast<const uint4*>(row) + 2 * p, on); r.b = ld16_now_or_zero(reinterpret_cast<const uint4*>(row) + 2 * p + 1, on); }
   return r;
 }
 __device__ __forceinline__ void cvraw(const Raw8& r, int dt, float (&x)[8]) {
@@ -285,8 +292,8 @@ __device__ __forceinline__ Rows make_rows(const Geo& g, const void* q, const voi
                                           int bidx, int h, int t0, const float* rq, const float* rk) {
   Rows r;
   r.q = q; r.k = k; r.gg = gg; r.b = b;
-  r.qkv_dt = CF::typed ? CF::qkv_dt : g.qkv_dt;
-  r.gate_dt = CF::typed ? CF::gate_dt : g.gate_dt;
+  r.qkv_dt = CF::qkv_typed ? CF::qkv_dt : g.qkv_dt;
+  r.gate_dt = CF::gate_typed ? CF::gate_dt : g.gate_dt;
   const size_t tok0 = (size_t)bidx * g.L + t0;
   r.qk_pitch = (size_t)g.Hk * g.K;
   r.qk_row0 = tok0 * r.qk_pitch + (size_t)g.qk_head(h) * g.K;

@@ -185,24 +185,24 @@ __device__ __forceinline__ float ldf_ro(const void* p, size_t i, int dt) {
   return dt == DN_BF16 ? __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(p) + i))
                        : __ldg(reinterpret_cast<const float*>(p) + i);
 }
-// The same in two steps, bits and value: the conversion waits for its load.  (With a type that is known at run time only the load waits
-// as well, at the join of the two paths, and so does a pair of predicated loads of one register: kernels that want several
-// in flight are instantiated by type.)
+// The same in two steps, bits and value: the conversion waits for its load.
+// A load behind a branch is waited for where the paths join (whether the branch is the type's, a tail's or an option's), so that loads behind
+// branches take a latency each.  Where several are to be in flight the type is known to the instance, rows past the end read
+// another row, and what depends on a condition is a predicated load over a given value.  These are issued where they stand; an
+// ordinary load may be moved down to its use.
 __device__ __forceinline__ uint32_t ldbits_ro(const void* p, size_t i, int dt) {
   return dt == DN_BF16 ? (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(p) + i) : __ldg(reinterpret_cast<const uint32_t*>(p) + i);
 }
-// without a branch and zero where `on` is false
-__device__ __forceinline__ uint32_t ldbits_ro_or_zero(const void* p, size_t i, int dt, bool on) {
+__device__ __forceinline__ uint32_t ldbits_or(const void* p, size_t i, int dt, bool on, uint32_t other) {
   uint32_t u;
   if (dt == DN_BF16)
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.b32 %0, 0;\n\t@q ld.global.nc.u16 %0, [%1];\n\t}"
-                 : "=r"(u) : "l"(reinterpret_cast<const unsigned short*>(p) + i), "r"((int)on));
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.b32 %0, %3;\n\t@q ld.global.nc.u16 %0, [%1];\n\t}"
+                 : "=&r"(u) : "l"(reinterpret_cast<const unsigned short*>(p) + i), "r"((int)on), "r"(other));
   else
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.b32 %0, 0;\n\t@q ld.global.nc.u32 %0, [%1];\n\t}"
-                 : "=r"(u) : "l"(reinterpret_cast<const uint32_t*>(p) + i), "r"((int)on));
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.b32 %0, %3;\n\t@q ld.global.nc.u32 %0, [%1];\n\t}"
+                 : "=&r"(u) : "l"(reinterpret_cast<const uint32_t*>(p) + i), "r"((int)on), "r"(other));
   return u;
 }
-// 16 bytes of an input tensor, issued where it stands (an ordinary load may be moved down to its use, past the branches between), or zeros
 __device__ __forceinline__ uint4 ld16_now(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
@@ -212,8 +212,12 @@ __device__ __forceinline__ uint4 ld16_now_or_zero(const void* p, bool on) {
   uint4 v;
   asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
                "@q ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];\n\t}"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "r"((int)on));
+               : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"((int)on));
   return v;
+}
+// seg_at without a branch
+__device__ __forceinline__ int seg_now(const int32_t* seg, int b, int t, int L) {
+  return (int)ldbits_or(seg, (size_t)b * L + (t < L ? t : L - 1), DN_F32, seg != nullptr, 0u);
 }
 __device__ __forceinline__ float bits_value(uint32_t u, int dt) { return __uint_as_float(dt == DN_BF16 ? u << 16 : u); }
 __device__ __forceinline__ void stf(void* p, size_t i, float v, int dt) {

@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
 
   const bool l2 = g.flags & DN_QK_L2NORM, trunc = g.flags & DN_TRUNC_DT_BF16;
   const bool fuse = CF::fixed || SC ? false : (g.flags & DN_FUSE_PROLOGUE) != 0, guard = CF::fixed ? false : (g.flags & DN_STABILITY_GUARD) != 0;
-  const int qdt = SC ? DN_BF16 : (CF::typed ? CF::qkv_dt : g.qkv_dt), gdt = CF::typed ? CF::gate_dt : g.gate_dt;
+  const int qdt = SC ? DN_BF16 : (CF::qkv_typed ? CF::qkv_dt : g.qkv_dt), gdt = CF::gate_typed ? CF::gate_dt : g.gate_dt;
   const bool round_in = !fuse && qdt == DN_BF16;
   const int kp = CF::fixed && !SC ? 16 : g.K / 8, gC = SC ? 1 : (CF::fixed ? K : g.gC), bC = SC ? 1 : (CF::fixed ? (CF::scalar_bw ? 1 : K) : g.bC);
   const int wC = CF::fixed && !SC ? (CF::scalar_bw ? 1 : g.V) : g.wC;
@@ -1331,16 +1331,16 @@ int launch_prepass_bwd_fast(const PrepassBwdArgs& args, cudaStream_t st) {
       // tokens of 16 x 32 heads)
       if (!g.fine) go(prepass_bwd_fast_kernel<VW, 2, true>);
       else if (mode == 5) go(prepass_bwd_fast_kernel<VW, 5, true, true>);
-      else go(prepass_bwd_fast_kernel<VW, 2, true, true>);
+      else go(prepass_bwd_fast_kernel<VW, 3, true, true>);
       return;
     }
     switch (mode) {
       case 0: go(prepass_bwd_fast_kernel<VW, 0, false>); break;
       case 1: go(prepass_bwd_fast_kernel<VW, 1, false>); break;
-      case 3: go(prepass_bwd_fast_kernel<VW, 3, false>); break;
+      case 3: if (g.fine) go(prepass_bwd_fast_kernel<VW, 3, false, true>); else go(prepass_bwd_fast_kernel<VW, 3, false>); break;
       case 4: go(prepass_bwd_fast_kernel<VW, 4, false>); break;
       case 5: if (g.fine) go(prepass_bwd_fast_kernel<VW, 5, false, true>); else go(prepass_bwd_fast_kernel<VW, 5, false>); break;
-      default: if (g.fine) go(prepass_bwd_fast_kernel<VW, 2, false, true>); else go(prepass_bwd_fast_kernel<VW, 2, false>); break;
+      default: if (g.fine) go(prepass_bwd_fast_kernel<VW, 6, false, true>); else go(prepass_bwd_fast_kernel<VW, 6, false>); break;
     }
   };
   if (g.Vw == 256) pick(std::integral_constant<int, 256>{});

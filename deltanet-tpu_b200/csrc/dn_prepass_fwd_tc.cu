@@ -147,6 +147,7 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
   uint4* Uimg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.res.U) + ibase * C * VW);
   const int vr = g.G * g.V, vsh = g.V == 128 ? 7 : 6;   // value columns that exist
   constexpr int YP = ONE_ROW ? PP : PQ;                   // panels of Y
+  constexpr int W_STEP = ONE_ROW ? 2 : 4;
   uint4 vraw[4];                                          // a half's pieces of v (bf16) and scalar write gates, requested ahead of use
   [[maybe_unused]] uint32_t w1[4];
   auto row_of_it = [&](int it) { return ONE_ROW ? row_of(tid) : row8_of(tid, it); };
@@ -158,7 +159,7 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
   const uint8_t* vrow = reinterpret_cast<const uint8_t*>(a.v) + (tok0 * g.Hv * g.V + (size_t)h * vr) * dt_size(qdt);
   auto request_v = [&](int half) {
     if constexpr (ONE_ROW) {
-      if (qdt == DN_BF16) {
+      if (qdt == DN_BF16) {                             // (or in build_y)
 #pragma unroll
         for (int it = 0; it < 4; ++it)
           vraw[it] = ld16_now_or_zero(reinterpret_cast<const uint4*>(vrow) + half * 16 + it * 4 + piece_of(tid), half * 128 + 32 * it < vr);
@@ -168,34 +169,46 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
       for (int it = 0; it < 4; ++it) {
         const int col0 = half * 128 + 8 * piece_of_it(it), cc = col0 < vr ? col0 : 0;
         const size_t tok = row_at(it);
-        w1[it] = ldbits_ro_or_zero(a.w, tok * g.wH + g.w_of(h * g.G + (cc >> vsh)), gdt, wC == 1);
+        w1[it] = ldbits_or(a.w, tok * g.wH + g.w_of(h * g.G + (cc >> vsh)), gdt, wC == 1, 0u);
         vraw[it] = ld16_now_or_zero(reinterpret_cast<const __nv_bfloat16*>(a.v) + tok * g.Hv * g.V + (size_t)h * vr + col0, col0 < vr);
       }
     }
   };
   auto build_y = [&](uint4* Y, int half) {              // Y = w v of the half's columns
 #pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int x = row_of_it(it), p = piece_of_it(it);
-      const int col0 = half * 128 + 8 * p, cv = col0 & (g.V - 1);
-      if (col0 >= vr) { Y[p * YP + x] = make_uint4(0, 0, 0, 0); continue; }
-      const size_t tok = ONE_ROW ? tok0 : row_at(it);
-      float vv[8], ww[8];
-      if (wC == 1) {
-        float w_row;
-        if constexpr (ONE_ROW) w_row = ldf_ro(a.w, tok * g.wH + g.w_of(h * g.G + (col0 >> vsh)), gdt);
-        else w_row = bits_value(w1[it], gdt);
+    for (int u = 0; u < 4; u += W_STEP) {
+      [[maybe_unused]] Raw8 wr[W_STEP], vr8[W_STEP];    // one row a thread: two pieces of w together, and of v in fp32 (four: 231 -> 238)
+      if constexpr (ONE_ROW) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) ww[i] = w_row;
-      } else {
-        load8(a.w, (tok * g.wH + g.w_of(h * g.G + (col0 >> vsh))) * wC + cv, gdt, ww);
+        for (int it = 0; it < W_STEP; ++it) {
+          const int col0 = half * 128 + 8 * piece_of_it(u + it), cc = col0 < vr ? col0 : 0;
+          const size_t at = tok0 * g.wH + g.w_of(h * g.G + (cc >> vsh));
+          wr[it] = ldraw_or_zero(reinterpret_cast<const uint8_t*>(a.w) + (at * wC + (cc & (g.V - 1))) * dt_size(gdt), 0, gdt, wC != 1);
+          w1[u + it] = ldbits_or(a.w, at, gdt, wC == 1, 0u);
+          if (qdt != DN_BF16) vr8[it] = ldraw(vrow, cc >> 3, qdt);
+        }
       }
-      if (!ONE_ROW || qdt == DN_BF16) umma::unpack8(vraw[it], vv);
-      else { const Raw8 r = ldraw(vrow, half * 16 + p, qdt); cvraw(r, qdt, vv); }
-      const bool live = ONE_ROW ? live0 : t0 + x < g.L;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) vv[i] = live ? (fuse ? sigmoid_fast(ww[i]) : ww[i]) * vv[i] : 0.f;
-      Y[p * YP + x] = umma::pack8(vv);
+      for (int it = 0; it < W_STEP; ++it) {
+        const int x = row_of_it(u + it), p = piece_of_it(u + it);
+        const int col0 = half * 128 + 8 * p, cv = col0 & (g.V - 1);
+        float vv[8], ww[8];
+        if (wC == 1) {
+          const float w_row = bits_value(w1[u + it], gdt);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) ww[i] = w_row;
+        } else if constexpr (ONE_ROW) {
+          cvraw(wr[it], gdt, ww);
+        } else {
+          load8(a.w, (row_at(u + it) * g.wH + g.w_of(h * g.G + ((col0 < vr ? col0 : 0) >> vsh))) * wC + cv, gdt, ww);
+        }
+        if (!ONE_ROW || qdt == DN_BF16) umma::unpack8(vraw[u + it], vv);
+        else cvraw(vr8[it], qdt, vv);
+        const bool live = col0 < vr && (ONE_ROW ? live0 : t0 + x < g.L);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) vv[i] = live ? (fuse ? sigmoid_fast(ww[i]) : ww[i]) * vv[i] : 0.f;
+        Y[p * YP + x] = umma::pack8(vv);
+      }
     }
   };
   tri::invert(Tp, reinterpret_cast<float*>(TI), others);
@@ -730,7 +743,8 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
   };
   const bool fuse = CF::fixed ? false : (g.flags & DN_FUSE_PROLOGUE) != 0, guard = CF::fixed ? false : (g.flags & DN_STABILITY_GUARD) != 0;
   const bool l2 = g.flags & DN_QK_L2NORM;
-  const int qdt = CF::typed ? CF::qkv_dt : g.qkv_dt, gdt = CF::typed ? CF::gate_dt : g.gate_dt;
+  constexpr int qdt = CF::qkv_dt;
+  const int gdt = CF::gate_typed ? CF::gate_dt : g.gate_dt;
   const bool round_in = !fuse && qdt == DN_BF16;
   const int kp = CF::fixed ? 16 : g.K / 8, gC = CF::fixed ? K : g.gC, bC = CF::fixed ? (CF::scalar_bw ? 1 : K) : g.bC;
   const int wC = CF::fixed ? (CF::scalar_bw ? 1 : g.V) : g.wC;
@@ -743,6 +757,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
     const int t0 = c_idx * C;
     const size_t ibase = ((size_t)b * g.H + h) * g.NC + c_idx;
     const int rows = g.L - t0 < C ? g.L - t0 : C;
+    constexpr int NORM_STEP = 2;                        // pieces of q and of k in flight
     const bool live = x < rows;                         // rows past the end read row 0 and are zeroed
     const size_t tok = (size_t)b * g.L + t0 + (live ? x : 0);
     const uint8_t* krow = reinterpret_cast<const uint8_t*>(a.k) + (tok * g.Hk + g.qk_head(h)) * g.K * qes;
@@ -756,37 +771,46 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
     auto load_g = [&](int grp) {
       const bool cin = gC == 1 || CF::fixed || 32 * grp < gC;
       const uint8_t* gp = grow + (gC == 1 ? 0 : 32 * grp * ges);
-      if (rows == C && cin) {
+      const uint32_t none = fuse ? 0xff800000u : 0u;    // (-infinity; as the bits of a bf16: below)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) gv[i] = ldf_ro(gp + i * gpitch, 0, gdt);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) gv[i] = cin && warp * 8 + i < rows ? ldf_ro(gp + i * gpitch, 0, gdt) : (fuse ? -INFINITY : 0.f);
-      }
+      for (int i = 0; i < 8; ++i)
+        gv[i] = __uint_as_float(ldbits_or(gp + i * gpitch, 0, gdt, cin && warp * 8 + i < rows, gdt == DN_BF16 ? none >> 16 : none));
     };
-    auto act_g = [&]() {                                // the activated decay (rows past the end: 0)
+    auto act_g = [&]() {                                // the activated decay (rows past the end: 0) from its bits
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
+        gv[i] = bits_value(__float_as_uint(gv[i]), gdt);
         if (fuse) { const bool off = gv[i] == -INFINITY; gv[i] = off ? 0.f : -umma::ex2_fast(fminf(gv[i], 5.f) * DN_LOG2E); if (guard && !off) gv[i] = fminf(gv[i], -1e-6f); }
         else { gv[i] = gv[i] <= 0.f ? gv[i] : 0.f; if (guard && warp * 8 + i < rows) gv[i] = fminf(gv[i], -1e-6f); }
       }
     };
+    // No load of an item's head, of a group or of w and v (build_y) stands behind a branch (see ldbits_or), and the head's are asked for before
+    // the first use of one: KDA, 16384 tokens of 32 heads, 631 -> 622 us; headline step 87.5 -> 84.7; fused prologue 133.5 -> 131 (fp32 gates
+    // 155 -> 140).  All four pieces of q and k or of w at once are too many for 64 registers: 84.7 -> 88.
     load_g(0);
-    if (tid < C) seg_s[tid] = seg_at(a.seg, b, t0 + tid, g.L);
+    const int seg_x = seg_now(a.seg, b, t0 + (tid & (C - 1)), g.L);
     float rq = 1.f, rk = 1.f;
     if (l2) {
       float sq = 0.f, sk = 0.f;
 #pragma unroll
-      for (int it = 0; it < 4; ++it) {
-        const int p = it * 4 + lgrp;
-        if (CF::fixed || p < kp) {
+      for (int u = 0; u < 4; u += NORM_STEP) {
+        Raw8 qn[NORM_STEP], kn[NORM_STEP];
+#pragma unroll
+        for (int it = 0; it < NORM_STEP; ++it) {
+          const int p = (u + it) * 4 + lgrp, pc = CF::fixed || p < kp ? p : 0;
+          qn[it] = ldraw(qrow, pc, qdt);
+          kn[it] = ldraw(krow, pc, qdt);
+        }
+#pragma unroll
+        for (int it = 0; it < NORM_STEP; ++it) {
+          const bool on = CF::fixed || (u + it) * 4 + lgrp < kp;
           float f[8];
-          cvraw(ldraw(qrow, p, qdt), qdt, f);
+          cvraw(qn[it], qdt, f);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) sq = fmaf(f[i], f[i], sq);
-          cvraw(ldraw(krow, p, qdt), qdt, f);
+          for (int i = 0; i < 8; ++i) sq = on ? fmaf(f[i], f[i], sq) : sq;
+          cvraw(kn[it], qdt, f);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) sk = fmaf(f[i], f[i], sk);
+          for (int i = 0; i < 8; ++i) sk = on ? fmaf(f[i], f[i], sk) : sk;
         }
       }
       sq += __shfl_xor_sync(0xffffffffu, sq, 1);  sk += __shfl_xor_sync(0xffffffffu, sk, 1);
@@ -794,6 +818,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       rq = rsqrtf(sq + 1e-6f);
       rk = rsqrtf(sk + 1e-6f);
     }
+    if (tid < C) seg_s[tid] = seg_x;
     const float rqs = rq * g.scale;
     if (lgrp == 0) { rq_s[x] = rq; rk_s[x] = rk; }      // (for the hierarchical route and the backward)
     Raw8 kr, qr, br;                                    // this thread's piece of the group about to be built
@@ -802,10 +827,11 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       const int p = grp * 4 + lgrp, pc = CF::fixed || p < kp ? p : 0;
       kr = ldraw(krow, pc, qdt);
       qr = ldraw(qrow, pc, qdt);
-      if (bC != 1) br = ldraw(brow, pc, gdt);
+      if (CF::fixed) { if (bC != 1) br = ldraw(brow, pc, gdt); }
+      else br = ldraw_or_zero(brow, pc, gdt, bC != 1);
     };
     load_kqb(0);
-    if (bC == 1) b1 = ldf_ro(brow, 0, gdt);
+    b1 = bits_value(ldbits_or(brow, 0, gdt, bC == 1, 0u), gdt);
     __syncthreads();
     if (tid < C) {                                      // seg_s is non-decreasing: binary searches
       const int sx = seg_s[tid];
@@ -1010,10 +1036,10 @@ int launch_prepass_fwd_tc(const Geo& g, const void* q, const void* k, const void
     switch (typed_mode(g)) {
       case 0: go(prepass_fwd_channel_kernel<VW, 0>); break;
       case 1: go(prepass_fwd_channel_kernel<VW, 1>); break;
-      case 3: go(prepass_fwd_channel_kernel<VW, 3>); break;
+      case 3: if (g.fine) go(prepass_fwd_channel_kernel<VW, 3, true>); else go(prepass_fwd_channel_kernel<VW, 3>); break;
       case 4: go(prepass_fwd_channel_kernel<VW, 4>); break;
       case 5: if (g.fine) go(prepass_fwd_channel_kernel<VW, 5, true>); else go(prepass_fwd_channel_kernel<VW, 5>); break;
-      default: if (g.fine) go(prepass_fwd_channel_kernel<VW, 2, true>); else go(prepass_fwd_channel_kernel<VW, 2>); break;
+      default: if (g.fine) go(prepass_fwd_channel_kernel<VW, 6, true>); else go(prepass_fwd_channel_kernel<VW, 6>); break;
     }
   };
   if (g.Vw == 256) pick(std::integral_constant<int, 256>{});
