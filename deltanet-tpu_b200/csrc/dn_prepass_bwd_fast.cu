@@ -663,12 +663,6 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       }
       commit(cx);
     };
-    if constexpr (!SC) {
-      drain_dM();
-      drain_masked(cx.dead, tb + T_TMP, dAi, row, group, -1.f, seg_s, nullptr, nullptr);
-      issue_dke();
-    }
-
     // ---- key side: rows of q, k, b in the row mapping
     const bool live = rx < rows;
     const size_t tokx = tok0 + (live ? rx : 0);
@@ -691,23 +685,22 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       rawq = ldraw(qrow, pc, qdt);
       if (bC != 1) rawb = ldraw(brow, pc, gdt);
     };
-    auto pieces = [&](int p, float (&kh)[8], float (&qh)[8], float (&be)[8]) {
+    auto hat = [&](const Raw8& raw, int p, float by, float (&x)[8]) {
       const bool on = live && p < kp;
-      cvraw(rawk, qdt, kh);
-      cvraw(rawq, qdt, qh);
-      const float rqs = rq * g.scale;
+      cvraw(raw, qdt, x);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) { kh[i] = on ? kh[i] * rk : 0.f; qh[i] = on ? qh[i] * rqs : 0.f; }
+      for (int i = 0; i < 8; ++i) x[i] = on ? x[i] * by : 0.f;
       if (round_in) {
-        const uint4 pk = umma::pack8(kh), pq = umma::pack8(qh);
-        umma::unpack8(pk, kh);
-        umma::unpack8(pq, qh);
+        const uint4 u = umma::pack8(x);
+        umma::unpack8(u, x);
       }
+    };
+    auto beta = [&](const Raw8& raw, const float (&kh)[8], float (&be)[8]) {
       if (bC == 1) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) be[i] = b1 * kh[i];
       } else {
-        cvraw(rawb, gdt, be);
+        cvraw(raw, gdt, be);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           if (fuse) be[i] = sigmoid_fast(be[i]); else if (guard) be[i] = fmaxf(be[i], 0.f);
@@ -715,7 +708,30 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         }
       }
     };
+    auto pieces = [&](int p, float (&kh)[8], float (&qh)[8], float (&be)[8]) {
+      hat(rawk, p, rk, kh);
+      hat(rawq, p, rq * g.scale, qh);
+      beta(rawb, kh, be);
+    };
+    // The thread's pieces of k and q stay in registers until the combination wants the raw rows, where the type is known to be bf16.  (Scalar gates:
+    // reading them three times, once a row per lane, took 3 k cycles of a tile's 63.)  Decay per channel: they are asked for ahead of the scan of the decay, and
+    // wait in the regions of KF and of QF and BF, k for the column sums as well, which take it a row per lane.
+    constexpr bool HOLD = !SC && CF::fixed && CF::qkv_dt == DN_BF16;
+    uint4 kraw4[SC || HOLD ? 4 : 1], qraw4[SC || HOLD ? 4 : 1];
+    auto request_kq = [&] {
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int p = it * 4 + rp, pc = p < kp ? p : 0;
+        kraw4[SC || HOLD ? it : 0] = ld16_now(krow + 16 * pc);
+        qraw4[SC || HOLD ? it : 0] = ld16_now(qrow + 16 * pc);
+      }
+    };
 
+    if constexpr (!SC) {
+      drain_dM();
+      drain_masked(cx.dead, tb + T_TMP, dAi, row, group, -1.f, seg_s, nullptr, nullptr);
+      issue_dke();
+    }
     uint32_t gpass = 0;                                 // which of the thread's 32 rows pass the gradient of g
     // ---- the decay of all channels: thread (channel, 32 rows), scanned in registers, restarting at document changes
     if constexpr (!SC) {
@@ -744,6 +760,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       float run = 0.f;
       float* lp = LAM + x0 * LPF + c;
       finish(cx);                                       // dke: its operands lie where Lambda goes
+      if constexpr (HOLD) request_kq();                 // (ahead of a call these loads would be waited for at the call)
 #pragma unroll 1
       for (int j = 0; j < 32 / GB; ++j) {
         float v[GB];
@@ -776,17 +793,16 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         EDGE[tid] = umma::ex2_fast(0.5f * (LAM[tid] + LAM[de_s[0] * LPF + tid]));
         EDGE[128 + tid] = umma::ex2_fast(0.5f * (LAM[(C - 1) * LPF + tid] - LAM[ds_s[C - 1] * LPF + tid]));
       }
-    }
-    // Scalar gates: the thread's pieces of k and q stay in registers until the combination wants the raw rows (reading them
-    // three times, once a row per lane, took 3 k cycles of a tile's 63)
-    uint4 kraw4[SC ? 4 : 1], qraw4[SC ? 4 : 1];
-    if constexpr (SC) {
+      if constexpr (HOLD) {
 #pragma unroll
-      for (int it = 0; it < 4; ++it) {
-        const int p = it * 4 + rp, pc = p < kp ? p : 0;
-        kraw4[it] = ld16_now(krow + 16 * pc);
-        qraw4[it] = ld16_now(qrow + 16 * pc);
+        for (int it = 0; it < 4; ++it) {
+          sl.region(2)[(it * 4 + rp) * PP + rx] = kraw4[it];
+          sl.region(3)[(it * 4 + rp) * PP + rx] = qraw4[it];
+        }
       }
+    }
+    if constexpr (SC) {
+      request_kq();
       drain_dM();
       issue_dke();
       if (NH == 2) finish(cx);                          // (an operand of dke lies where the rows of dA times beta go)
@@ -813,31 +829,45 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       const uint8_t* kr = reinterpret_cast<const uint8_t*>(a.k) + ((tok0 + (row < rows ? row : 0)) * g.Hk + g.qk_head(h)) * g.K * qes;
       const float rkr = rk_s[row];
       Raw8 knext;
-      if (!SC) knext = ldraw(kr, group * 4 < kp ? group * 4 : 0, qdt);
+      if (!SC && !HOLD) knext = ldraw(kr, group * 4 < kp ? group * 4 : 0, qdt);
       float pk = 0.f;
 #pragma unroll 1
       for (int j = 0; j < 4; ++j) {
         const int p = group * 4 + j, c0 = group * 32 + 8 * j;
         float v[8], w[8], x[8], kh[8], od[8];
         const Raw8 kraw = knext;
-        if (!SC && j < 3) knext = ldraw(kr, p + 1 < kp ? p + 1 : 0, qdt);
-        ld8(cx.dead, tb + T_Q + 8 * j, v);
-        ld8(cx.dead, tb + T_B + 8 * j, w);
-        ld8(cx.dead, tb + T_K + 8 * j, x);
+        if (!SC && !HOLD) knext = ldraw(kr, p + 1 < kp ? p + 1 : 0, qdt);
+        if (!cx.dead) umma::tmem_ld8x3(tb + T_Q + 8 * j, tb + T_B + 8 * j, tb + T_K + 8 * j, v, w, x);
+        else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] = w[i] = x[i] = 0.f;
+        }
         if constexpr (SC) umma::unpack8(sl.region(0)[p * PP + row], kh);
+        else if constexpr (HOLD) umma::unpack8(sl.region(2)[p * PP + row], kh);
         else cvraw(kraw, qdt, kh);
+        float e1[8], e2[8], dl[8];
+        if constexpr (!SC) {
+#pragma unroll
+          for (int i = 0; i < 8; i += 4) {
+            const float4 u = *reinterpret_cast<const float4*>(EDGE + c0 + i), t = *reinterpret_cast<const float4*>(EDGE + 128 + c0 + i);
+            const float4 l9 = *reinterpret_cast<const float4*>(LAM + (C - 1) * LPF + c0 + i), l = *reinterpret_cast<const float4*>(LAM + row * LPF + c0 + i);
+            e1[i] = first ? u.x : 0.f; e1[i + 1] = first ? u.y : 0.f; e1[i + 2] = first ? u.z : 0.f; e1[i + 3] = first ? u.w : 0.f;
+            e2[i] = last ? t.x : 0.f; e2[i + 1] = last ? t.y : 0.f; e2[i + 2] = last ? t.z : 0.f; e2[i + 3] = last ? t.w : 0.f;
+            dl[i] = l9.x - l.x; dl[i + 1] = l9.y - l.y; dl[i + 2] = l9.z - l.z; dl[i + 3] = l9.w - l.w;
+          }
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const float e1 = SC ? el : (first ? EDGE[c0 + i] : 0.f);
-          v[i] *= e1;
-          w[i] = (trunc ? bf16r(w[i]) : w[i]) * -e1;    // (the accumulator holds -dX)
+          const float f1 = SC ? el : e1[i];
+          v[i] *= f1;
+          w[i] = (trunc ? bf16r(w[i]) : w[i]) * -f1;    // (the accumulator holds -dX)
           if (!SC) {
             kh[i] *= rkr;
             if (round_in) kh[i] = bf16r(kh[i]);
           }
-          const float e = SC ? eks : umma::ex2_fast(fminf(LAM[(C - 1) * LPF + c0 + i] - LAM[row * LPF + c0 + i], 0.f));
+          const float e = SC ? eks : umma::ex2_fast(fminf(dl[i], 0.f));
           od[i] = on && p < kp ? x[i] * (kh[i] * e) : 0.f;
-          x[i] *= SC ? (last ? eks : 0.f) : (last ? EDGE[128 + c0 + i] : 0.f);
+          x[i] *= SC ? (last ? eks : 0.f) : e2[i];
         }
         umma::tmem_st8(tb + T_Q + 8 * j, v);
         umma::tmem_st8(tb + T_B + 8 * j, w);
@@ -884,8 +914,85 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         commit(cx);
         finish(cx);
       }
+    } else if constexpr (HOLD) {
+      // k / f of all channels in region 2, then beta f and q f of 64 channels in region 3 beside the first two products, and of the others in
+      // region 2 beside the next two.  In two rounds of 64 channels (below), each behind the other's products, this took 10.0 k cycles of a KDA tile, now
+      // 8.4; with k and q loaded once and the column sums' rows by 16 bytes (7.6 k cycles -> 5.2): 16384 tokens of 32 heads 1016 -> 985 us, 8000
+      // tokens of 16 x 32 heads, gates per channel, 422 -> 412.  (Unrolled like this with types, widths and activation known at run time the
+      // kernel outgrows the instruction cache: fused prologue 251 -> 257.)
+      uint4 *const KF = sl.region(2), *const Q0 = sl.region(3);
+      auto log_f = [&](int p, float (&d)[8]) {
+        const float* lx = LAM + rx * LPF + 8 * p;
+        const float* ls = LAM + ds_s[rx] * LPF + 8 * p;
+        const float* le = LAM + de_s[rx] * LPF + 8 * p;
+#pragma unroll
+        for (int i = 0; i < 8; i += 4) {
+          const float4 u0 = *reinterpret_cast<const float4*>(lx + i), u1 = *reinterpret_cast<const float4*>(ls + i), u2 = *reinterpret_cast<const float4*>(le + i);
+          d[i] = fmaf(-0.5f, u1.x + u2.x, u0.x); d[i + 1] = fmaf(-0.5f, u1.y + u2.y, u0.y);
+          d[i + 2] = fmaf(-0.5f, u1.z + u2.z, u0.z); d[i + 3] = fmaf(-0.5f, u1.w + u2.w, u0.w);
+        }
+      };
+      Raw8 rb[2];
+      auto request_b = [&](int it0) {
+        if (bC != 1)
+#pragma unroll
+          for (int u = 0; u < 2; ++u) rb[u] = ldraw(brow, (it0 + u) * 4 + rp, gdt);
+      };
+      auto raw = [](uint4 u) { Raw8 r; r.a = u; return r; };
+      request_b(0);
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        kraw4[it] = KF[(it * 4 + rp) * PP + rx];
+        qraw4[it] = Q0[(it * 4 + rp) * PP + rx];
+      }
+      __syncthreads();                                  // (the column sums have read k)
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int p = it * 4 + rp;
+        float d[8], kh[8];
+        log_f(p, d);
+        hat(raw(kraw4[it]), p, rk, kh);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) kh[i] *= umma::ex2_fast(-d[i]);
+        KF[p * PP + rx] = umma::pack8(kh);
+      }
+      umma::pre_issue_sync();
+      product<128, false, true>(cx, dAi, 2048, KF, PB, C, T_B, true);                  // dA (k / f)
+      product<128, false, true>(cx, dMi, 2048, KF, PB, C, T_Q, true);                  // dM (k / f)
+      commit(cx);
+#pragma unroll
+      for (int rnd = 0; rnd < 2; ++rnd) {
+        uint4 *const QF = rnd ? KF : Q0, *const BF = QF + 8 * PP;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int it = 2 * rnd + u, p = it * 4 + rp, o = (u * 4 + rp) * PP + rx;
+          float d[8], kh[8], qh[8], be[8];
+          log_f(p, d);
+          hat(raw(kraw4[it]), p, rk, kh);
+          hat(raw(qraw4[it]), p, rq * g.scale, qh);
+          beta(rb[u], kh, be);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float f = umma::ex2_fast(d[i]);
+            qh[i] *= f;
+            be[i] *= f;
+          }
+          QF[o] = umma::pack8(qh);
+          BF[o] = umma::pack8(be);
+        }
+        if (rnd == 0) {
+          request_b(2);
+          umma::fence_async_smem();
+          umma::tc_fence_before();
+          finish(cx);                                   // k / f has been read
+        } else umma::pre_issue_sync();
+        product<64, true, true>(cx, dAi, 2048, BF, PB, C, T_K + 64 * rnd, true);        // dA^T (beta f)
+        product<64, true, true>(cx, dMi, 2048, QF, PB, C, T_K + 64 * rnd, true);        // dM^T (q f)
+      }
+      commit(cx);
+      finish(cx);
     } else {
-      // Two rounds of 64 channels: what the images take beside Lambda, dA and dM.  (Four rounds of 32 with two sets of images
+      // Rounds of 64 channels: what the images of all three take beside Lambda, dA and dM.  (Four rounds of 32 with two sets of images
       // overlapped building and products, but at 32 columns an MMA costs 46 cycles and at 64 it costs 48: 18.7 k cycles
       // per tile against 11 k.)
       uint4* KF = reinterpret_cast<uint4*>(sm + OFF_GI);
@@ -952,7 +1059,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
 #pragma unroll
       for (int it = 0; it < 4; ++it) {
         const int p = it * 4 + rp;
-        if constexpr (SC) {
+        if constexpr (SC || HOLD) {
           const bool on = live && p < kp;
           RK[p * PP + rx] = on ? kraw4[it] : make_uint4(0, 0, 0, 0);
           RQ[p * PP + rx] = on ? qraw4[it] : make_uint4(0, 0, 0, 0);
