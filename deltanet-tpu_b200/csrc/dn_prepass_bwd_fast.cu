@@ -30,6 +30,7 @@
 
 #include "dn_chunkprep.cuh"
 #include "dn_kernels.cuh"
+#include "dn_rows.cuh"
 
 namespace dn {
 namespace {
@@ -373,7 +374,7 @@ __device__ __noinline__ void v_phase(const PrepassBwdArgs& a, const uint4* img, 
 // k_hat and q_hat of scalar gates have one).  Three rounds of products for two: B=4 L=2048, 16 heads of 64, a training step 798 us against
 // 696 (gdn2), 493 against 428 (DeltaNet); with the hierarchical kernels in this one's place, which have an exact diagonal, 1684.
 template <int VW, int MODE, bool SC, bool FINE = false>
-__global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_constant__ PrepassBwdArgs a) {
+__global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_constant__ PrepassBwdArgs a, const __grid_constant__ RowMaps maps) {
   using CF = InCfg<MODE>;
   constexpr int NH = VW / 128;
   extern __shared__ __align__(128) uint8_t sm[];
@@ -573,6 +574,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
       umma::fence_async_smem();
       finish(cx);
       sl.load(3, dHg);
+      if (tid == NT - 1) prefetch_rows(maps, g, ROWS_V | ROWS_W, b, h, t0);      // (see row_maps)
       product<128, false, false>(cx, sl.at(5), PB, sl.at(2), 2048, 128, T_Q, false);                       // dqe = dO S^T, beside the drains
       sl.wait(4);
       vnew(4, T_TMP);
@@ -587,6 +589,7 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
         product<128, false, false>(cx, sl.at(0), PB, sl.at(2), 2048, 128, T_B, true);
       }
       commit(cx);
+      if (tid == NT - 1) prefetch_rows(maps, g, ROWS_Q | ROWS_K | ROWS_G | ROWS_B, b, h, t0);
       if (v_ahead) v_body<true, false, true, FINE ? NH : 0>(vrows, a, sl.at(1), 0, h, tok0, rows, fuse, sl.at(0));
       else vphase(1, 0);
       finish(cx);
@@ -1426,9 +1429,10 @@ int launch_prepass_bwd_fast(const PrepassBwdArgs& args, cudaStream_t st) {
   a.by_HG.set(g.H / D);
   a.by_BHG.set(g.B * (g.H / D));
   const int grid = units < sm_count() ? units : sm_count();
+  const RowMaps maps = row_maps(g, g.Vw == 128 && g.qkv_dt == DN_BF16 ? ~0u : 0u, a.q, a.k, a.v, a.gg, a.b, a.w);
   auto go = [&](auto kernel) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    kernel<<<grid, NT, SMEM_BYTES, st>>>(a);
+    kernel<<<grid, NT, SMEM_BYTES, st>>>(a, maps);
   };
   auto pick = [&](auto vw) {
     constexpr int VW = decltype(vw)::value;

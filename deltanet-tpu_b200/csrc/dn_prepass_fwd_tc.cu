@@ -20,6 +20,7 @@
 
 #include "dn_chunkprep.cuh"
 #include "dn_kernels.cuh"
+#include "dn_rows.cuh"
 #include "dn_tri_inverse.cuh"
 
 namespace dn {
@@ -716,7 +717,7 @@ __device__ __noinline__ void strong_route(const PrepassFwdArgs& a, int b, int h,
 // FINE (see make_geo): the three factors in two bf16 parts, in the two sets of images, so that a group's products (first x first,
 // second x first, first x second) are waited for by the next group.
 template <int VW, int MODE, bool FINE = false>
-__global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid_constant__ PrepassFwdArgs a, int* err) {
+__global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid_constant__ PrepassFwdArgs a, const __grid_constant__ RowMaps maps, int* err) {
   using CF = InCfg<MODE>;
   extern __shared__ __align__(128) uint8_t sm[];
   __shared__ uint64_t bar, gbar[2];                     // one barrier per set of group images: a barrier must not run two phases ahead of its waiters
@@ -1002,7 +1003,14 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
       drain_am(cx, reinterpret_cast<float*>(sm + OFF_T), Mimg, ds_s[(warp & 3) * 32 + lane], [](int, float (&)[16], float (&)[16]) {});
       __syncthreads();
     }
-    inverse_and_products<VW, !CF::scalar_bw>(cx, sm, a, h, b, t0, ibase, qdt, gdt, wC, fuse, [] {}, [] {});
+    inverse_and_products<VW, !CF::scalar_bw>(cx, sm, a, h, b, t0, ibase, qdt, gdt, wC, fuse, [&] {
+      const int next = e_item + gridDim.x;              // (the next item's head and groups: see row_maps)
+      if (VW == 128 && tid == NT - 1 && next < a.items) {
+        int nb, nh, nc;
+        g.tile(next, a.c_begin, nb, nh, nc);
+        prefetch_rows(maps, g, ROWS_Q | ROWS_K | ROWS_G | ROWS_B, nb, nh, nc * C);
+      }
+    }, [] {});
   }
   teardown(tbase);
 }
@@ -1023,9 +1031,9 @@ int launch_prepass_fwd_tc(const Geo& g, const void* q, const void* k, const void
   const bool scalar = g.gC == 1 && g.bC == 1 && g.qkv_dt == DN_BF16 && !(g.flags & DN_FUSE_PROLOGUE);
   const int grid = a.items < 2 * sm_count() ? a.items : 2 * sm_count();
   int* err = device_error_ptr();
-  auto go = [&](auto kernel) {
+  auto go = [&](auto kernel, const auto&... maps) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    kernel<<<grid, NT, SMEM_BYTES, st>>>(a, err);
+    kernel<<<grid, NT, SMEM_BYTES, st>>>(a, maps..., err);
   };
   auto pick = [&](auto vw) {
     constexpr int VW = decltype(vw)::value;
@@ -1033,13 +1041,14 @@ int launch_prepass_fwd_tc(const Geo& g, const void* q, const void* k, const void
       if (g.gate_dt == DN_BF16) go(prepass_fwd_scalar_kernel<VW, DN_BF16>); else go(prepass_fwd_scalar_kernel<VW, DN_F32>);
       return;
     }
+    const RowMaps maps = row_maps(g, VW == 128 && a.items > grid ? ROWS_Q | ROWS_K | ROWS_G | ROWS_B : 0, q, k, v, gg, b, w);
     switch (typed_mode(g)) {
-      case 0: go(prepass_fwd_channel_kernel<VW, 0>); break;
-      case 1: go(prepass_fwd_channel_kernel<VW, 1>); break;
-      case 3: if (g.fine) go(prepass_fwd_channel_kernel<VW, 3, true>); else go(prepass_fwd_channel_kernel<VW, 3>); break;
-      case 4: go(prepass_fwd_channel_kernel<VW, 4>); break;
-      case 5: if (g.fine) go(prepass_fwd_channel_kernel<VW, 5, true>); else go(prepass_fwd_channel_kernel<VW, 5>); break;
-      default: if (g.fine) go(prepass_fwd_channel_kernel<VW, 6, true>); else go(prepass_fwd_channel_kernel<VW, 6>); break;
+      case 0: go(prepass_fwd_channel_kernel<VW, 0>, maps); break;
+      case 1: go(prepass_fwd_channel_kernel<VW, 1>, maps); break;
+      case 3: if (g.fine) go(prepass_fwd_channel_kernel<VW, 3, true>, maps); else go(prepass_fwd_channel_kernel<VW, 3>, maps); break;
+      case 4: go(prepass_fwd_channel_kernel<VW, 4>, maps); break;
+      case 5: if (g.fine) go(prepass_fwd_channel_kernel<VW, 5, true>, maps); else go(prepass_fwd_channel_kernel<VW, 5>, maps); break;
+      default: if (g.fine) go(prepass_fwd_channel_kernel<VW, 6, true>, maps); else go(prepass_fwd_channel_kernel<VW, 6>, maps); break;
     }
   };
   if (g.Vw == 256) pick(std::integral_constant<int, 256>{});

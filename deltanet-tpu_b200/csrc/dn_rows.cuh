@@ -1,0 +1,79 @@
+// Rows of the operator's tensors asked into L2 ahead of their use, by one thread and one instruction for a tile's 128 rows x 128 columns
+// (cp.async.bulk.prefetch.tensor): tensor maps of the (B L) x (heads width) matrices that q, k, v and the gates are.
+//
+// What it is for: the phases of the chunk-parallel kernels run in step on all SMs, so each tensor's rows are wanted everywhere at the same time,
+// and a phase that reads them waits for HBM, which idles in the others.  Requests per line by the threads cost as much as they hid (32
+// lookups each: decay per channel, forward, 761 -> 819 us).  When to ask matters as much: what is asked for at an item's start delays the
+// loads that the start itself waits for.  So the forward kernel asks for the next item's q, k and gates beside the inverse (KDA, 16384 tokens of 32 heads,
+// 618 -> 592 us), the backward for v and w behind the first products and for the rest beside the second batch (983 -> 950; scalar gates, 2 x 4001
+// tokens of 16 x 32 heads, 381 -> 375).  Tiles of 256 value columns have twice the bytes to bring and gain nothing: forward 228 -> 235 us and more,
+// backward 412 -> 418, wherever it was asked for; nor does the backward of fp32 q/k/v (255 -> 261); nor does the forward kernel of scalar gates, which asks per line while it waits for the substitution (664 -> 682).
+#pragma once
+#include <cuda.h>
+
+#include "dn_common.cuh"
+
+namespace dn {
+
+struct RowMap {
+  alignas(64) CUtensorMap map;
+};
+struct RowMaps {
+  RowMap q, k, v, g, b, w;
+  uint32_t on;                                          // which of them there are, in this order
+};
+enum : uint32_t { ROWS_Q = 1, ROWS_K = 2, ROWS_V = 4, ROWS_G = 8, ROWS_B = 16, ROWS_W = 32 };
+
+// Maps of those of a shape's tensors that are wanted, gates of one value per head apart (a row of them is a few bytes).  Nothing where the driver has no encoder, or for a
+// tensor that it refuses: the kernels then read without.
+inline RowMaps row_maps(const Geo& g, uint32_t wanted, const void* q, const void* k, const void* v, const void* gg, const void* b, const void* w) {
+  RowMaps m;
+  m.on = 0;
+  if (!wanted) return m;
+  using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                              CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode encode = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) p = nullptr;
+    return reinterpret_cast<Encode>(p);
+  }();
+  if (!encode) return m;
+  auto add = [&](RowMap& out, uint32_t bit, const void* p, int heads, int width, int dt) {
+    if (!(wanted & bit) || !p || width % 64) return;
+    const cuuint64_t dim[2] = {(cuuint64_t)heads * width, (cuuint64_t)g.B * g.L}, pitch[1] = {dim[0] * dt_size(dt)};
+    const cuuint32_t box[2] = {dim[0] < 128 ? 64u : 128u, 128}, step[2] = {1, 1};
+    if (encode(&out.map, dt == DN_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(p), dim, pitch, box, step,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
+      m.on |= bit;
+  };
+  add(m.q, ROWS_Q, q, g.Hk, g.K, g.qkv_dt);
+  add(m.k, ROWS_K, k, g.Hk, g.K, g.qkv_dt);
+  add(m.v, ROWS_V, v, g.Hv, g.V, g.qkv_dt);
+  if (g.gC > 1) add(m.g, ROWS_G, gg, g.gH, g.gC, g.gate_dt);
+  if (g.bC > 1) add(m.b, ROWS_B, b, g.bH, g.bC, g.gate_dt);
+  if (g.wC > 1) add(m.w, ROWS_W, w, g.wH, g.wC, g.gate_dt);
+  return m;
+}
+
+// 128 rows from token `row` of (B L) on, `cols` columns from `col` on (a multiple of 64); by one thread
+__device__ __forceinline__ void prefetch_rows(const RowMap& m, int col, int cols, int row) {
+  for (int c = 0; c < cols; c += 128)
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(&m.map), "r"(col + c), "r"(row) : "memory");
+}
+// a tile's rows of some of the tensors: of exec head h of batch row b from token t0 on.  (A call: expanded, it cost the forward kernels registers.)
+static __device__ __noinline__ void prefetch_rows(const RowMaps& m, const Geo& g, uint32_t which, int b, int h, int t0) {
+  which &= m.on;
+  const int row = b * g.L + t0, hk = g.qk_head(h);
+  if (which & ROWS_Q) prefetch_rows(m.q, hk * g.K, g.K, row);
+  if (which & ROWS_K) prefetch_rows(m.k, hk * g.K, g.K, row);
+  if (which & ROWS_G) prefetch_rows(m.g, g.g_head(h) * g.gC, g.gC, row);
+  if (which & ROWS_B) prefetch_rows(m.b, g.b_head(h) * g.bC, g.bC, row);
+  if (which & ROWS_V) prefetch_rows(m.v, h * g.G * g.V, g.G * g.V, row);
+  if (which & ROWS_W) {
+    if (g.wH == g.Hv) prefetch_rows(m.w, h * g.G * g.V, g.G * g.V, row);
+    else prefetch_rows(m.w, g.w_of(h * g.G) * g.V, g.V, row);           // (one for all heads, or the key head's)
+  }
+}
+
+}  // namespace dn
