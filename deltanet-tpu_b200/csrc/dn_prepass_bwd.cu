@@ -9,7 +9,8 @@
 //
 // Formulation notes (same result up to rounding):
 //  * dA = -T^T dT T^T with dT = dW X^T + dU Y^T collapses to dA = -(dX W^T + dY U^T) with
-//    dX = T^T dW, dY = T^T dU, because W = T X and U = T Y; dT is never formed.
+//    dX = T^T dW, dY = T^T dU, because W = T X and U = T Y; and with dU = dV, dW = -dV S^T to
+//    dX = -dY S^T, dA = -dY V_new^T: neither dT nor dW is formed.
 //  * the adjoints of A and M are evaluated pair by pair with exact exponents, and
 //    dLambda = beta*dbeta' + q*dq' - k*dk' (primes: the parts coming through A and M) plus the
 //    terms through X, qe, ke and Lambda_end; dg is the within-document reverse cumulative sum.
@@ -43,8 +44,8 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
   const size_t CK = (size_t)C * K, CV = (size_t)C * Vw, CC = (size_t)C * C;
   float* sc = a.scratch + (size_t)(blockIdx.x / ranks) * a.scratch_per_cta;
   float* QH = sc;            float* KH = QH + CK;      float* LAM = KH + CK;
-  float* GB = LAM + CK;      float* BA = GB + CK;      float* DW = BA + CK;
-  float* DQE = DW + CK;      float* DKE = DQE + CK;    float* DX = DKE + CK;
+  float* GB = LAM + CK;      float* BA = GB + CK;
+  float* DQE = BA + CK;      float* DKE = DQE + CK;    float* DX = DKE + CK;
   float* DBP = DX + CK;      float* DQP = DBP + CK;    float* DKP = DQP + CK;
   float* DLAM = DKP + CK;    float* VN = DLAM + CK;    float* DY = VN + CV;
   float* DM = DY + CV;       float* DA = DM + CC;
@@ -149,11 +150,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
       const int t = t0 + i;
       return t < g.L ? ldf(a.d_out, ((size_t)b * g.L + t) * g.Hv * g.V + (size_t)h * Vw + j, g.qkv_dt) : 0.f;
     };
-    // ---- dW = -dV S^T, dqe = dO S^T, dY = T^T dV, then dke = V_new dH^T, dM = dO V_new^T
-    cta_gemm<true, false, GN>(C, K, Vw,
-        [&](int i, int kk) { float x = dV[(size_t)i * Vw + kk]; return sbf ? bf16r(x) : x; },
-        [&](int kk, int j) { float s = S[(size_t)j * Vw + kk]; return sbf ? bf16r(s) : s; },
-        [&](int i, int j, float acc) { DW[i * K + j] = -acc; }, tile, team);
+    // ---- dqe = dO S^T, dY = T^T dV, then dke = V_new dH^T, dM = dO V_new^T, dX = -dY S^T and dA = -dY V_new^T (strictly lower, same document)
     cta_gemm<true, false, GN>(C, K, Vw,
         [&](int i, int kk) { float x = dO_at(i, kk); return sbf ? bf16r(x) : x; },
         [&](int kk, int j) { float s = S[(size_t)j * Vw + kk]; return sbf ? bf16r(s) : s; },
@@ -171,19 +168,13 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
         [&](int i, int kk) { float x = dO_at(i, kk); return ibf ? bf16r(x) : x; },
         [&](int kk, int j) { float x = VN[j * Vw + kk]; return ibf ? bf16r(x) : x; },
         [&](int i, int j, float acc) { DM[i * C + j] = (i >= j && seg_s[i] == seg_s[j]) ? acc : 0.f; }, tile, team);
-    // ---- dX = T^T dW
-    cta_gemm<false, true, GN>(C, K, C,
-        [&](int i, int kk) { float t = T[(size_t)kk * C + i]; return ibf ? bf16r(t) : t; },
-        [&](int kk, int j) { float x = DW[kk * K + j]; return ibf ? bf16r(x) : x; },
-        [&](int i, int j, float acc) { DX[i * K + j] = trunc ? bf16r(acc) : acc; }, tile, team);
-    if (SPLIT) team.sync();
-    // ---- dA = -(dX W^T + dY U^T), strictly lower and same document
-    cta_gemm<true, false, GN>(C, C, K + Vw,
-        [&](int i, int kk) { return kk < K ? DX[i * K + kk] : DY[i * Vw + (kk - K)]; },
-        [&](int kk, int j) {
-          return kk < K ? ldf(a.res.W, bW + (size_t)j * K + kk, pre)
-                        : ldf(a.res.U, bU + (size_t)j * Vw + kk - K, pre);
-        },
+    cta_gemm<true, false, GN>(C, K, Vw,
+        [&](int i, int kk) { return DY[i * Vw + kk]; },
+        [&](int kk, int j) { float s = S[(size_t)j * Vw + kk]; return sbf ? bf16r(s) : s; },
+        [&](int i, int j, float acc) { DX[i * K + j] = trunc ? bf16r(-acc) : -acc; }, tile, team);
+    cta_gemm<true, false, GN>(C, C, Vw,
+        [&](int i, int kk) { return DY[i * Vw + kk]; },
+        [&](int kk, int j) { return VN[j * Vw + kk]; },
         [&](int i, int j, float acc) { DA[i * C + j] = (i > j && seg_s[i] == seg_s[j]) ? -acc : 0.f; }, tile, team);
 
     if (SPLIT) team.sync();
@@ -348,7 +339,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1) prepass_bwd_kernel(PrepassBwdAr
 }
 
 size_t prepass_bwd_scratch_per_cta(const Geo& g) {
-  return (size_t)13 * g.C * g.K + (size_t)2 * g.C * g.Vw + (size_t)2 * g.C * g.C;
+  return (size_t)12 * g.C * g.K + (size_t)2 * g.C * g.Vw + (size_t)2 * g.C * g.C;
 }
 
 bool prepass_bwd_tc_eligible(const Geo& g) { return g.img && !(g.flags & DN_STATE_FP32_MM); }
