@@ -121,7 +121,12 @@ inline int make_geo(const dn_shape* s, Geo* g) {
   // 1.35e-2 with one part).  So the shapes that are new to these tiles take their factors and cotangents in two parts.  K = 128
   // with 128 or 256 value columns has had one part from the beginning.
   g->fine = tc && (s->K == 64 || (g->G * s->V != 128 && g->G * s->V != 256));
-  g->C = tc ? 128 : s->chunk;
+  // fp32 precision runs a request for chunk 128 in chunks of 64, the same regrouping the other way: what a chunk costs beside its
+  // share of the state (pairs of rows, inverse, products of T) grows with the square of its rows, its factors fit shared memory, and
+  // its items keep more of the chip busy.  fp32 forward and backward, us at chunk 128 -> 64: 60 tokens of 2 x 4 heads of 64 215 -> 94, 2 x 1000 of
+  // 4 x 8 704 -> 444, 2048 of 4 heads 761 -> 558; heads of 128: 400 -> 150, 1820 -> 918, 2057 -> 1003.
+  // Errors against 64-bit results are half as large.  (With bf16 factors, state_fp32_matmul, they would be 0.3 % larger: twice the roundings.)
+  g->C = tc ? 128 : s->precision == DN_PREC_FP32 ? 64 : s->chunk;
   g->Kt = tc ? 128 : s->K;
   if (tc) g->Vw = g->Vw <= 128 ? 128 : 256;
   g->NC = (s->L + g->C - 1) / g->C;

@@ -442,13 +442,13 @@ static int launch_bwd(const StateArgs& a, cudaStream_t st) {
   return launch_status();
 }
 
-// fp32 residuals and products, room for a chunk's factors (all but 128 x 128), and factors that 16-byte copies can fetch.
+// fp32 residuals and products, and factors that 16-byte copies can fetch.
 static bool staged(const StateArgs& a) {
   const Geo& g = a.g;
   uintptr_t bits = 0;
   for (const void* p : {(const void*)a.res.W, (const void*)a.res.qe, (const void*)a.res.ke, (const void*)a.res.M, (const void*)a.res.lam_end})
     bits |= reinterpret_cast<uintptr_t>(p);
-  return g.pre_dt == DN_F32 && !g.state_bf16() && !g.bf16_mode() && !(g.C == 128 && g.K == 128) && (bits & 15) == 0;
+  return g.pre_dt == DN_F32 && !g.state_bf16() && !g.bf16_mode() && (bits & 15) == 0;
 }
 template <int C, int K>
 static int launch_staged(const StateArgs& a, bool bwd, cudaStream_t st) {
@@ -459,7 +459,6 @@ static int launch_staged(const StateArgs& a, bool bwd, cudaStream_t st) {
   return launch_status();
 }
 static int launch_staged(const StateArgs& a, bool bwd, cudaStream_t st) {
-  if (a.g.C == 128) return launch_staged<128, 64>(a, bwd, st);
   return a.g.K == 128 ? launch_staged<64, 128>(a, bwd, st) : launch_staged<64, 64>(a, bwd, st);
 }
 

@@ -102,11 +102,11 @@ typedef struct dn_exec {
                                   exec head, chunks */
   int32_t pre_dtype;           /* dtype of W,U,M,qe,ke: bf16 in bf16 precision else f32 (gdn2.py:1247) */
   int32_t chunk;               /* rows per tile the kernels use, the C of every layout below.  Equal to
-                                  dn_shape.chunk except on the tensor-core path (bf16 precision without
-                                  DN_STATE_FP32_MM): there tiles are 128 rows, the M of a tcgen05.mma, and a
-                                  request for 64 runs with pairs of requested chunks merged into one tile
-                                  (the chunked form regroups the token recurrence exactly; only the points
-                                  where the state is rounded to bf16 move).  NC = ceil(L / chunk).          */
+                                  dn_shape.chunk in bf16 precision with DN_STATE_FP32_MM, else whatever
+                                  that asks for: 128, the M of a tcgen05.mma, on the tensor-core
+                                  path (bf16 precision without DN_STATE_FP32_MM), 64 in fp32 precision.
+                                  The chunked form regroups the token recurrence exactly; only the points
+                                  where values are rounded move.  NC = ceil(L / chunk).                     */
 } dn_exec;
 int dn_exec_view(const dn_shape* s, dn_exec* out);
 
