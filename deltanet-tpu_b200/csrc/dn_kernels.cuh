@@ -14,6 +14,9 @@ struct PrepassFwdArgs {
   int items;
   int smem_tile_off;
   int c_begin, c_end;          // chunk range [c_begin, c_end) of every (batch, head); tensor-core path only
+  // A call of one chunk from a zero state (prepass_fwd_single): the kernel goes on to what the chain would make of the chunk
+  void* out;                   // (B,L,Hv,V) qkv dtype
+  float* final_state;          // (B,Hv,K,V) or null
 };
 
 struct StateArgs {
@@ -87,7 +90,8 @@ int launch_prepass_fwd(const Geo& g, const void* q, const void* k, const void* v
 bool prepass_fwd_tc_eligible(const Geo& g);
 int launch_prepass_fwd_tc(const Geo& g, const void* q, const void* k, const void* v, const void* gg,
                           const void* b, const void* w, const int32_t* seg, const dn_residuals& res,
-                          cudaStream_t st, int c_begin = 0, int c_end = -1);
+                          cudaStream_t st, int c_begin = 0, int c_end = -1, void* out = nullptr, float* final_state = nullptr);
+bool prepass_fwd_single(const Geo& g);            // one chunk, zero state, nothing kept: launch_prepass_fwd_tc takes out and final_state
 int launch_state_fwd(const StateArgs& a, cudaStream_t st);
 // tensor-core (tcgen05) variants of the chain kernels, used when state_tc_eligible()
 bool state_tc_eligible(const Geo& g);

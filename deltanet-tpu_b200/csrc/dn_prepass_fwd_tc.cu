@@ -128,15 +128,83 @@ __device__ __forceinline__ void prefetch_kq(const PrepassFwdArgs& a, int e_item)
   prefetch_row(reinterpret_cast<const uint8_t*>(a.q) + qk * qe, g.K * qe);
 }
 
+// One chunk from a zero state, 128 value columns: V_new = U (columns 128 of tensor memory), O = M U, S = ke^T U.  Operands and roundings are the
+// chain's, so that the results are its bits; so are its products with the zero state, 0 or not a number: `zq`, the
+// thread's share of 0 qe (row tid & 127), and `bad`, whether W has a value that is not finite.
+// Everything of the item but M and ke is consumed: U goes where X was, M where Y was, ke where T was.  What bounds such a call is latency, one
+// tile a CTA and a launch behind the other: 75 tokens of 32 heads 26.7 -> 23.6 us a call, 128 tokens of 4 x 32 heads 34.4 -> 23.6 us of
+// kernels.  (Tiles of 256 columns, one half after the other, against the chain's four CTAs a head: 28.3 -> 36.8; they keep the chain.)
+__device__ __noinline__ void single_chunk(umma::Ctx& cx, uint8_t* sm, const PrepassFwdArgs& a, int h, int b, int t0, size_t ibase, float zq, bool bad) {
+  const Geo& g = a.g;
+  const int tid = threadIdx.x, vr = g.G * g.V;
+  uint4 *const UI = reinterpret_cast<uint4*>(sm + OFF_X), *const MI = reinterpret_cast<uint4*>(sm + OFF_T), *const KE = reinterpret_cast<uint4*>(sm + OFF_TI);
+  uint8_t* zs = sm + OFF_TI + 32768;                    // 4 x 128, behind ke
+  const uint4* Mg = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.res.M) + ibase * C * C);
+  const uint4* Kg = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.res.ke) + ibase * C * K);
+  {
+    uint4 m[4], k[4];
+#pragma unroll
+    for (int it = 0; it < 4; ++it) { m[it] = Mg[it * NT + tid]; k[it] = Kg[it * NT + tid]; }             // (written by this CTA: no read-only loads)
+#pragma unroll
+    for (int it = 0; it < 4; ++it) { MI[it * NT + tid] = m[it]; KE[it * NT + tid] = k[it]; }
+    zs[tid] = zq != 0.f;                                // (0 or not a number)
+  }
+  umma::drain<NT, 128>(cx, 128, [&](int row, int col, const float (&v)[16]) {
+    const uint4 nan = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
+    UI[(col / 8) * 128 + row] = bad ? nan : umma::pack8p(v);
+    UI[(col / 8 + 1) * 128 + row] = bad ? nan : umma::pack8p(v + 8);
+  });
+  umma::pre_issue_sync();
+  umma::issue_pitched<128, false, true>(cx, MI, 2048, UI, 2048, C, 0, false);
+  if (a.final_state) umma::issue_pitched<128, true, true>(cx, KE, 2048, UI, 2048, C, 128, false);
+  umma::commit(cx);
+  umma::commit_wait_cta(cx);
+  // Through shared memory (the operands are consumed), so that rows are written by neighbouring lanes: a row per lane, 16 bytes at a time, O and S
+  // took 8 us of a 24 us launch, so 6 of 22.
+  uint4* const OS = reinterpret_cast<uint4*>(sm + OFF_X);               // rows of 17 pieces
+  float* const SS = reinterpret_cast<float*>(sm + OFF_T + 2048);        // rows of 132
+  static_assert(OFF_X + 128 * 17 * 16 <= OFF_T + 2048 && OFF_T + 2048 + 128 * 132 * 4 <= OFF_TI + 32768 && OFF_TI + 32768 + 512 <= SMEM_BYTES, "staging");
+  umma::drain<NT, 128>(cx, 0, [&](int row, int c, float (&v)[16]) {
+    const float z = zs[row] | zs[128 + row] | zs[256 + row] | zs[384 + row] ? __int_as_float(0x7fffffff) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] += z;
+    OS[row * 17 + c / 8] = umma::pack8p(v);
+    OS[row * 17 + c / 8 + 1] = umma::pack8p(v + 8);
+  });
+  if (a.final_state)
+    umma::drain<NT, 128>(cx, 128, [&](int row, int c, const float (&v)[16]) {
+#pragma unroll
+      for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(SS + row * 132 + c + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    });
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int e = it * NT + tid, row = e >> 4, p = e & 15;
+    if (t0 + row < g.L && 8 * p < vr)
+      reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.out) + ((size_t)b * g.L + t0 + row) * g.Hv * g.V + (size_t)h * vr)[p] = OS[row * 17 + p];
+  }
+  if (!a.final_state) return;
+  const bool aligned = (reinterpret_cast<uintptr_t>(a.final_state) & 15) == 0;
+#pragma unroll
+  for (int it = 0; it < 8; ++it) {
+    const int e = it * NT + tid, row = e >> 5, c = 4 * (e & 31);
+    if (row >= g.K || c >= vr) continue;
+    const float4 v = *reinterpret_cast<const float4*>(SS + row * 132 + c);
+    float* d = a.final_state + (((size_t)b * g.Hv + h * g.G + c / g.V) * g.K + row) * g.V + (c & (g.V - 1));
+    if (aligned) *reinterpret_cast<float4*>(d) = v;
+    else { d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w; }
+  }
+}
+
 // T = (I + A)^-1, then W = T X and U = T (w v).  X image and A visible to all threads on entry.
 // others(): run by warps that wait for the substitution (tri::invert); ahead(): run by all as soon as the products have read their
 // operands (the images of X and T are free then).  ONE_ROW: a thread takes four pieces of one row of v and w instead of two pieces of two
 // rows.  That is twice the lookups, but one address: with write gates per column or of a type known at run time, whose rows a thread
 // addresses as well, the other mapping spilled up to 290 bytes more a thread (64 registers).  Ten launches of 256 columns, L = 20011: 798 -> 769 us;
 // fused prologue, L = 4000, 32 heads: 222 -> 204; 64-wide heads, 16 of them: 177 -> 162.  The instances with two rows have bf16 v only.
-template <int VW, bool ONE_ROW, class OTHERS, class AHEAD>
+template <int VW, bool ONE_ROW, bool SINGLE = false, class OTHERS, class AHEAD>
 __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm, const PrepassFwdArgs& a, int h, int b, int t0,
-                                                     size_t ibase, int qdt, int gdt, int wC, bool fuse, OTHERS others, AHEAD ahead) {
+                                                     size_t ibase, int qdt, int gdt, int wC, bool fuse, OTHERS others, AHEAD ahead, float zq = 0.f) {
   constexpr int NH = VW / 128;
   const Geo& g = a.g;
   const int tid = threadIdx.x;
@@ -228,10 +296,25 @@ __device__ __forceinline__ void inverse_and_products(umma::Ctx& cx, uint8_t* sm,
     for (int it = 0; it < 4; ++it) Tg[it * NT + tid] = TI[it * NT + tid];
   }
   umma::commit_wait_cta(cx);
-  if (NH == 1) ahead();
+  if (NH == 1 && !SINGLE) ahead();
   if (NH == 2) {                                        // X has been consumed
     build_y(XI, 1);
     umma::fence_async_smem();                           // (ahead of the stores below: it would wait for them)
+  }
+  if constexpr (SINGLE) {                                // (one half)
+    float z = 0.f;                                      // 0 W
+    umma::drain<NT, 128>(cx, 0, [&](int, int, const float (&v)[16]) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) z = fmaf(v[i], 0.f, z);
+    });
+    const bool bad = __syncthreads_or(z != 0.f) != 0;
+    umma::Ctx c2 = cx;
+    single_chunk(c2, sm, a, h, b, t0, ibase, zq, bad);
+    cx.phase = c2.phase;
+    cx.dead = c2.dead;
+    __syncthreads();
+    ahead();
+    return;
   }
   umma::drain<NT, 128>(cx, 0, [&](int row, int col, const float (&v)[16]) {
     Wimg[(col / 8) * 128 + row] = umma::pack8p(v);
@@ -320,7 +403,7 @@ __device__ __forceinline__ void scan_scalar(const PrepassFwdArgs& a, int e_item,
 // 8 to 11 beside the substitution (its loads come from HBM: 1 to 2 k cycles), its rows of k and q are asked into L2 there and into
 // shared memory beside the last drains.  GDT: the type of the gates (known at run time only, the four write gates a thread
 // loads for its rows waited for one another, 700 cycles each: 4 x 8192 tokens of 32 heads 692 -> 669 us, one tile 17.2 -> 16.0).
-template <int VW, int GDT>
+template <int VW, int GDT, bool SINGLE>
 __global__ void __launch_bounds__(NT, 2) prepass_fwd_scalar_kernel(const __grid_constant__ PrepassFwdArgs a, int* err) {
   extern __shared__ __align__(128) uint8_t sm[];
   __shared__ uint64_t bar;
@@ -407,6 +490,7 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_scalar_kernel(const __grid_
     umma::issue_pitched<128, false, false>(cx, QI, PQB, KI, PQB, K, 128, false);         // q_hat k_hat^T
     umma::commit(cx);
     uint4 xr[4];                                        // X = [first document] beta e^lam k_hat
+    [[maybe_unused]] float zq = 0.f;                    // 0 qe (see single_chunk)
     {                                                   // qe, ke while the products run
       const float lam = R.lam[row], lend = R.lam[C - 1], el = umma::exp_neg(fminf(lam, 0.f)), bx = R.bet[row];
       const bool first = R.ds[row] == 0, last = R.ds[row] == R.ds[C - 1];
@@ -420,6 +504,10 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_scalar_kernel(const __grid_
         umma::unpack8(QI[p * PQ + row], f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] *= fq;
+        if (SINGLE) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) zq = fmaf(f[i], 0.f, zq);
+        }
         QE[p * 128 + row] = umma::pack8(f);
         umma::unpack8(KI[p * PQ + row], f);
 #pragma unroll
@@ -453,13 +541,13 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_scalar_kernel(const __grid_
     }
     __syncthreads();
     const int next = e_item + gridDim.x;
-    inverse_and_products<VW, false>(cx, sm, a, h, b, t0, ibase, DN_BF16, GDT, g.wC, false, [&]() {
+    inverse_and_products<VW, false, SINGLE>(cx, sm, a, h, b, t0, ibase, DN_BF16, GDT, g.wC, false, [&]() {
       // (the requests: 779 -> 741 us at B=4 L=8192 Hv=32.  With decay per channel they cost more than they hide,
       // 761 -> 819 us at L=20011: that kernel reads q, k, b, g in groups and has other tiles to switch to.)
       if (warp < 8) prefetch_vw(a, h, b, t0);
       else if (warp >= 12) prefetch_kq(a, next);
       else if (next < a.items) scan_scalar<GDT>(a, next, tid - 256, rows_s[set ^ 1], tot_s, rst_s);
-    }, [&]() { load_kq(next); });
+    }, [&]() { load_kq(next); }, zq);
   }
   teardown(tbase);
 }
@@ -1018,17 +1106,20 @@ __global__ void __launch_bounds__(NT, 2) prepass_fwd_channel_kernel(const __grid
 }  // namespace
 
 bool prepass_fwd_tc_eligible(const Geo& g) { return g.img; }
+static bool scalar_route(const Geo& g) { return g.gC == 1 && g.bC == 1 && g.qkv_dt == DN_BF16 && !(g.flags & DN_FUSE_PROLOGUE); }
+bool prepass_fwd_single(const Geo& g) { return g.img && g.NC == 1 && g.Vw == 128 && !(g.flags & DN_HAS_INIT) && scalar_route(g); }
 
 int launch_prepass_fwd_tc(const Geo& g, const void* q, const void* k, const void* v, const void* gg,
                           const void* b, const void* w, const int32_t* seg, const dn_residuals& res,
-                          cudaStream_t st, int c_begin, int c_end) {
+                          cudaStream_t st, int c_begin, int c_end, void* out, float* final_state) {
   PrepassFwdArgs a{};
+  a.out = out; a.final_state = final_state;
   a.g = g; a.q = q; a.k = k; a.v = v; a.gg = gg; a.b = b; a.w = w; a.seg = seg; a.res = res;
   a.c_begin = c_begin; a.c_end = c_end < 0 ? g.NC : c_end;
   a.items = g.B * g.H * (a.c_end - a.c_begin);
   if (a.items <= 0) return DN_OK;
   // k_hat and q_hat are rounded to bf16 ahead of their use here, which the fused prologue does not do
-  const bool scalar = g.gC == 1 && g.bC == 1 && g.qkv_dt == DN_BF16 && !(g.flags & DN_FUSE_PROLOGUE);
+  const bool scalar = scalar_route(g);
   const int grid = a.items < 2 * sm_count() ? a.items : 2 * sm_count();
   int* err = device_error_ptr();
   auto go = [&](auto kernel, const auto&... maps) {
@@ -1038,7 +1129,8 @@ int launch_prepass_fwd_tc(const Geo& g, const void* q, const void* k, const void
   auto pick = [&](auto vw) {
     constexpr int VW = decltype(vw)::value;
     if (scalar) {
-      if (g.gate_dt == DN_BF16) go(prepass_fwd_scalar_kernel<VW, DN_BF16>); else go(prepass_fwd_scalar_kernel<VW, DN_F32>);
+      if (VW == 128 && out) { if (g.gate_dt == DN_BF16) go(prepass_fwd_scalar_kernel<128, DN_BF16, true>); else go(prepass_fwd_scalar_kernel<128, DN_F32, true>); }
+      else { if (g.gate_dt == DN_BF16) go(prepass_fwd_scalar_kernel<VW, DN_BF16, false>); else go(prepass_fwd_scalar_kernel<VW, DN_F32, false>); }
       return;
     }
     const RowMaps maps = row_maps(g, VW == 128 && a.items > grid ? ROWS_Q | ROWS_K | ROWS_G | ROWS_B : 0, q, k, v, gg, b, w);

@@ -360,3 +360,27 @@ def test_gate_types_agree(dn, form, L, G):
 
     for i, (x, y) in enumerate(zip(call(torch.bfloat16), call(torch.float32))):
         assert torch.equal(x, y), (i, O.rel_l2(x.float(), y.float()))
+
+
+# ---- prompts of one chunk from a zero state go through one launch: the bits that prepass and chain give, which a call with a state of zeros takes,
+# and the same values that are not finite.  80 x 4 heads: more items than CTAs.
+@pytest.mark.parametrize("B,L,Hk,Hv,K,V,gates", [(1, 1, 2, 2, 128, 128, torch.float32), (2, 75, 2, 4, 128, 128, torch.float32), (1, 128, 1, 2, 128, 128, torch.bfloat16),
+                                                 (80, 33, 4, 4, 128, 128, torch.float32), (80, 127, 4, 8, 64, 128, torch.float32), (2, 100, 2, 4, 64, 64, torch.bfloat16)])
+@pytest.mark.parametrize("heads", ["key", "value"])
+@pytest.mark.parametrize("bad", [None, "q", "k", "v", "b"])
+def test_single_chunk(dn, B, L, Hk, Hv, K, V, gates, heads, bad):
+    gen = torch.Generator().manual_seed(83)
+    rn = lambda *s: torch.randn(*s, generator=gen)
+    H = Hk if heads == "key" else Hv
+    ins = dict(q=rn(B, L, Hk, K).bfloat16(), k=rn(B, L, Hk, K).bfloat16(), v=rn(B, L, Hv, V).bfloat16(), g=(-torch.exp(0.5 * rn(B, L, H))).to(gates),
+               b=torch.sigmoid(rn(B, L, H)).to(gates), w=torch.sigmoid(rn(B, L, Hv)).to(gates))
+    if bad: ins[bad].view(-1)[ins[bad].numel() // 2] = float("inf")
+    seg = (torch.rand(B, L, generator=gen) < 0.03).int().cumsum(1).int().cuda()
+    seg = (seg - seg[:, :1]).contiguous()
+    t = [x.cuda() for x in ins.values()]
+    for l2 in (True, False):
+        kw = dict(segment_ids=seg, precision="bf16", qk_l2norm=l2, output_final_state=True, is_inference=True)
+        one, two = dn.chunk_gdn2(*t, **kw), dn.chunk_gdn2(*t, initial_state=torch.zeros(B, Hv, K, V, device="cuda"), **kw)
+        for x, y in zip(one, two):
+            assert torch.equal(x.isfinite(), y.isfinite()) and torch.equal(x[x.isfinite()], y[y.isfinite()])
+        assert torch.equal(dn.chunk_gdn2(*t, **dict(kw, output_final_state=False)).nan_to_num(7.0, 7.0, 7.0), one[0].nan_to_num(7.0, 7.0, 7.0))
