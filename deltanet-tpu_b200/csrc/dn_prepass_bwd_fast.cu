@@ -156,10 +156,12 @@ __device__ __noinline__ void drain_sub(bool dead, uint32_t addr, uint4* img, int
   }
 }
 // strictly lower triangle inside a document, times the scalar decay when lam is given; the diagonal apart when diag is; a second
-// image, of the first one's rows times `by`, when there is one
+// image, of the first one's rows times `by`, when there is one.  Pieces of 16 columns below the diagonal of a tile of one document have nothing to
+// mask: 2 x 4001 tokens of 16 x 32 heads, scalar gates, 376 -> 367.5 us, 4 x 2048 of 16 heads of 64 221 -> 217.
 __device__ __noinline__ void drain_masked(bool dead, uint32_t addr, uint4* img, int row, int group, float sign, const int* seg, const float* lam, float* diag,
                                            uint4* img2 = nullptr, float by = 0.f) {
   const int sr = seg[row];
+  const bool one = seg[0] == seg[C - 1];
   const float lr = lam ? lam[row] * DN_LOG2E : 0.f;
   img += 4 * group * 128 + row;
   if (img2) img2 += 4 * group * 128 + row;
@@ -178,11 +180,21 @@ __device__ __noinline__ void drain_masked(bool dead, uint32_t addr, uint4* img, 
       for (int i = 0; i < 16; ++i)
         if (c0 + i == row) diag[row] = v[i];
     }
+    if (one && c0 + 15 < (row & ~31)) {                 // (uniform) nothing to mask
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = c0 + i < row && sr == seg[c0 + i] ? sign * v[i] : 0.f;
+      for (int i = 0; i < 16; ++i) v[i] *= sign;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = c0 + i < row && sr == seg[c0 + i] ? sign * v[i] : 0.f;
+    }
     if (lam) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] *= umma::ex2_fast(fminf(lr - lam[c0 + i] * DN_LOG2E, 0.f));
+      for (int i = 0; i < 16; i += 4) {
+        const float4 l4 = *reinterpret_cast<const float4*>(lam + c0 + i);
+        const float l[4] = {l4.x, l4.y, l4.z, l4.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[i + u] *= umma::ex2_fast(fminf(lr - l[u] * DN_LOG2E, 0.f));
+      }
     }
     const uint4 lo = umma::pack8p(v), hi = umma::pack8p(v + 8);
     img[0] = lo;
@@ -385,7 +397,8 @@ __global__ void __launch_bounds__(NT, 1) prepass_bwd_fast_kernel(const __grid_co
   __shared__ int next_strong_s;
   __shared__ uint8_t ds_s[C], de_s[C];                  // first / last row of each row's document inside the tile
   __shared__ float rq_s[C], rk_s[C], dmi_s[C], dlend_s[C];
-  __shared__ float lam_s[C], bet_s[C];                  // scalar gates
+  __shared__ alignas(16) float lam_s[C];                // scalar gates
+  __shared__ float bet_s[C];
   const Geo& g = a.g;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int quarter = warp & 3, group = warp >> 2, row = quarter * 32 + lane;     // tensor-memory mapping
